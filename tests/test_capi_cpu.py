@@ -5,6 +5,7 @@ import os
 import re
 
 import numpy as np
+import pytest
 
 import triebwerk_b200 as tq
 from triebwerk_b200._lib import ModelShape
