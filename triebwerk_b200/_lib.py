@@ -136,6 +136,24 @@ def lib() -> C.CDLL:
     return L
 
 
+class _HostCall:
+    """The functions of the ``_hostcall`` extension (csrc/hostcall.cpp): library calls on tensors and torch's current
+    stream, at a fraction of what ctypes costs per call.  Loaded on first use, so that the package can be imported
+    before it is built."""
+
+    def __getattr__(self, name):
+        lib()  # the plain message when nothing is built
+        from . import _hostcall
+        self.__dict__.update({k: v for k, v in vars(_hostcall).items() if not k.startswith("_")})
+        try:
+            return self.__dict__[name]
+        except KeyError:
+            raise AttributeError(name) from None
+
+
+hostcall = _HostCall()
+
+
 class TqError(RuntimeError):
     def __init__(self, status: int, where: str):
         self.status = status

@@ -16,7 +16,7 @@ from typing import Optional, Sequence
 
 import torch
 
-from ._lib import ModelShape, StepProducer, check, lib
+from ._lib import ModelShape, StepProducer, TqError, check, hostcall, lib
 
 QWEN3_0_6B = dict(num_layers=28, num_heads=16, num_kv_heads=8, head_dim=128)
 QWEN3_8B = dict(num_layers=36, num_heads=32, num_kv_heads=8, head_dim=128)
@@ -28,6 +28,7 @@ class Engine:
         self._h = C.c_void_p()
         self.shape = ModelShape(num_layers, num_heads, num_kv_heads, head_dim)
         check(lib().tq_engine_create(C.byref(self.shape), max_seq_len, kv_bits, C.byref(self._h)), "Engine()")
+        self._handle = self._h.value  # as a plain number, for hostcall
         self.max_seq_len = max_seq_len
         self._arena_ref = None
         self.G = 0
@@ -128,10 +129,9 @@ class Engine:
         """Append k/v [G, kv_dim] at the current positions of `layer`, then attend with q [G, q_dim]."""
         if out is None:
             out = torch.empty_like(q)
-        for t in (q, k, v, out):
-            assert t.is_cuda and t.is_contiguous() and t.dtype == torch.float16
-        check(lib().tq_engine_decode_layer(self._h, layer, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                           self._stream()), "decode_layer")
+        st = hostcall.tq_engine_decode_layer(self._handle, layer, q, k, v, out)
+        if st:
+            raise TqError(st, "decode_layer")
         return out
 
     def attend_layer(self, layer: int, out: torch.Tensor) -> torch.Tensor:
@@ -146,10 +146,9 @@ class Engine:
 
     def decode_step(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """All layers of one decode step on device buffers [layers, G, dim]."""
-        for t in (q, k, v, out):
-            assert t.is_cuda and t.is_contiguous() and t.dtype == torch.float16
-        check(lib().tq_engine_decode_step(self._h, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                          self._stream()), "decode_step")
+        st = hostcall.tq_engine_decode_step(self._handle, q, k, v, out)
+        if st:
+            raise TqError(st, "decode_step")
         return out
 
     def decode_step_produce(self, q_raw, k_raw, v, out, q_norm_weight, k_norm_weight, rope_cos, rope_sin, rope_dim=128,
@@ -218,29 +217,28 @@ class Engine:
     def prefill_layer(self, layer: int, seq: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor = None):
         """One layer of a prompt's prefill (reference engine/engine.cpp:2110-2146): k/v [T, kv_dim] into positions 0..T-1 of
         the sequence's slot, then causal attention of q [T, q_stride] over them; returns out [T, q_stride]."""
-        for t in (q, k, v):
-            assert t.is_cuda and t.is_contiguous() and t.dtype == torch.float16
         if out is None:
             out = torch.empty_like(q)
-        check(lib().tq_engine_prefill_layer(self._h, layer, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                            k.shape[0], q.shape[1], self._stream()), "prefill_layer")
+        st = hostcall.tq_engine_prefill_layer(self._handle, layer, seq, q, k, v, out, k.shape[0], q.shape[1])
+        if st:
+            raise TqError(st, "prefill_layer")
         return out
 
     def prefill_layer_batch(self, layer: int, first_seq: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor = None):
         """prefill_layer for the prompts of several sequences at once: q [n, T, q_stride], k/v [n, T, kv_dim]."""
-        for t in (q, k, v):
-            assert t.is_cuda and t.is_contiguous() and t.dtype == torch.float16 and t.dim() == 3
+        assert q.dim() == 3 and k.dim() == 3 and v.dim() == 3
         if out is None:
             out = torch.empty_like(q)
-        check(lib().tq_engine_prefill_layer_batch(self._h, layer, first_seq, k.shape[0], q.data_ptr(), k.data_ptr(), v.data_ptr(),
-                                                  out.data_ptr(), k.shape[1], q.shape[2], self._stream()), "prefill_layer_batch")
+        st = hostcall.tq_engine_prefill_layer_batch(self._handle, layer, first_seq, k.shape[0], q, k, v, out, k.shape[1], q.shape[2])
+        if st:
+            raise TqError(st, "prefill_layer_batch")
         return out
 
     def prefill_append(self, layer: int, seq: int, k: torch.Tensor, v: torch.Tensor, first_pos: int = 0) -> None:
         """Token-form append of k/v [T, kv_dim] for one sequence (reference engine/engine.cpp:2121-2130)."""
-        assert k.is_cuda and v.is_cuda and k.is_contiguous() and v.is_contiguous()
-        check(lib().tq_engine_prefill_append(self._h, layer, seq, k.data_ptr(), v.data_ptr(), first_pos, k.shape[0],
-                                             self._stream()), "prefill_append")
+        st = hostcall.tq_engine_prefill_append(self._handle, layer, seq, k, v, first_pos, k.shape[0])
+        if st:
+            raise TqError(st, "prefill_append")
 
     def prefill_shared(self, layer: int, first_seq: int, n_seq: int, k: torch.Tensor, v: torch.Tensor) -> None:
         """One prompt k/v [T, kv_dim] for the sequences first_seq .. first_seq + n_seq - 1: its whole tiles are stored once
@@ -251,9 +249,10 @@ class Engine:
 
     def prefill_append_batch(self, layer: int, first_seq: int, k: torch.Tensor, v: torch.Tensor, first_pos: int = 0) -> None:
         """Token-form append of k/v [n_seq, T, kv_dim] for the sequences first_seq .. first_seq + n_seq - 1 in one launch."""
-        assert k.is_cuda and v.is_cuda and k.is_contiguous() and v.is_contiguous() and k.dim() == 3 and k.shape == v.shape
-        check(lib().tq_engine_prefill_append_batch(self._h, layer, first_seq, k.shape[0], k.data_ptr(), v.data_ptr(), first_pos,
-                                                   k.shape[1], self._stream()), "prefill_append_batch")
+        assert k.dim() == 3 and k.shape == v.shape
+        st = hostcall.tq_engine_prefill_append_batch(self._handle, layer, first_seq, k.shape[0], k, v, first_pos, k.shape[1])
+        if st:
+            raise TqError(st, "prefill_append_batch")
 
     def decode_step_host(self, q_host: torch.Tensor, k_host: torch.Tensor, v_host: torch.Tensor,
                          out_host: torch.Tensor) -> torch.Tensor:

@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from ._lib import TqError, check, lib
+from ._lib import TqError, check, hostcall, lib
 
 
 def _ptr(t):
@@ -22,76 +22,75 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
-def _raise_compat(where):
-    st = lib().tq_last_compat_status()
-    if st != 0:
-        raise TqError(st, where)
-
-
 def launch_turbo_kv_quantize(cache_q, cache_norms, kv_buf, rotation, positions, max_seq_len, num_tokens,
                              num_kv_heads, head_dim, kv_dim, bits):
-    lib().launch_turbo_kv_quantize(_ptr(cache_q), _ptr(cache_norms), _ptr(kv_buf), _ptr(rotation), _ptr(positions),
-                                   max_seq_len, num_tokens, num_kv_heads, head_dim, kv_dim, bits, _stream())
-    _raise_compat("launch_turbo_kv_quantize")
+    st = hostcall.launch_turbo_kv_quantize(cache_q, cache_norms, kv_buf, rotation, positions, max_seq_len, num_tokens,
+                                           num_kv_heads, head_dim, kv_dim, bits)
+    if st:
+        raise TqError(st, "launch_turbo_kv_quantize")
 
 
 def launch_turbo_kv_quantize_batch(cache_q, cache_norms, kv_buf, rotation, positions, max_seq_len, G, num_kv_heads,
                                    head_dim, kv_dim, bits):
-    lib().launch_turbo_kv_quantize_batch(_ptr(cache_q), _ptr(cache_norms), _ptr(kv_buf), _ptr(rotation),
-                                         _ptr(positions), max_seq_len, G, num_kv_heads, head_dim, kv_dim, bits,
-                                         _stream())
-    _raise_compat("launch_turbo_kv_quantize_batch")
+    st = hostcall.launch_turbo_kv_quantize_batch(cache_q, cache_norms, kv_buf, rotation, positions, max_seq_len, G,
+                                                 num_kv_heads, head_dim, kv_dim, bits)
+    if st:
+        raise TqError(st, "launch_turbo_kv_quantize_batch")
 
 
 def launch_turbo_gqa_attention_batch(out, q, ck_q, cv_q, k_norms, v_norms, rotation, attn_scratch, pos, msl, G,
                                      num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits):
-    lib().launch_turbo_gqa_attention_batch(_ptr(out), _ptr(q), _ptr(ck_q), _ptr(cv_q), _ptr(k_norms), _ptr(v_norms),
-                                           _ptr(rotation), _ptr(attn_scratch), _ptr(pos), msl, G, num_heads,
-                                           num_kv_heads, head_dim, q_dim, kv_dim, bits, _stream())
-    _raise_compat("launch_turbo_gqa_attention_batch")
+    st = hostcall.launch_turbo_gqa_attention_batch(out, q, ck_q, cv_q, k_norms, v_norms, rotation, attn_scratch, pos,
+                                                   msl, G, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits)
+    if st:
+        raise TqError(st, "launch_turbo_gqa_attention_batch")
 
 
 def launch_turbo_gqa_attention(q, ck_q, cv_q, k_norms, v_norms, rotation, output, attn_scratch, pos, msl, num_heads,
                                num_kv_heads, head_dim, bits):
-    lib().launch_turbo_gqa_attention(_ptr(q), _ptr(ck_q), _ptr(cv_q), _ptr(k_norms), _ptr(v_norms), _ptr(rotation),
-                                     _ptr(output), _ptr(attn_scratch), int(pos), msl, num_heads, num_kv_heads,
-                                     head_dim, bits, _stream())
-    _raise_compat("launch_turbo_gqa_attention")
+    st = hostcall.launch_turbo_gqa_attention(q, ck_q, cv_q, k_norms, v_norms, rotation, output, attn_scratch, pos, msl,
+                                             num_heads, num_kv_heads, head_dim, bits)
+    if st:
+        raise TqError(st, "launch_turbo_gqa_attention")
 
 
 def launch_turbo_gqa_prefill_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, attn_scratch, T, msl,
                                        num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits):
-    lib().launch_turbo_gqa_prefill_attention(_ptr(out), _ptr(q), _ptr(ck_q), _ptr(cv_q), _ptr(k_norms),
-                                             _ptr(v_norms), _ptr(rotation), _ptr(attn_scratch), T, msl, num_heads,
-                                             num_kv_heads, head_dim, q_dim, kv_dim, bits, _stream())
-    _raise_compat("launch_turbo_gqa_prefill_attention")
+    st = hostcall.launch_turbo_gqa_prefill_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, attn_scratch, T,
+                                                     msl, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits)
+    if st:
+        raise TqError(st, "launch_turbo_gqa_prefill_attention")
 
 
 def launch_kv_cache_write_batch(ck, cv, k, v, pos, msl, G, kv_dim):
-    lib().launch_kv_cache_write_batch(_ptr(ck), _ptr(cv), _ptr(k), _ptr(v), _ptr(pos), msl, G, kv_dim, _stream())
-    _raise_compat("launch_kv_cache_write_batch")
+    st = hostcall.launch_kv_cache_write_batch(ck, cv, k, v, pos, msl, G, kv_dim)
+    if st:
+        raise TqError(st, "launch_kv_cache_write_batch")
 
 
 def launch_gqa_attention_batch(out, q, ck, cv, attn_scratch, pos, msl, G, num_heads, num_kv_heads, head_dim, q_dim,
                                kv_dim):
-    lib().launch_gqa_attention_batch(_ptr(out), _ptr(q), _ptr(ck), _ptr(cv), _ptr(attn_scratch), _ptr(pos), msl, G,
-                                     num_heads, num_kv_heads, head_dim, q_dim, kv_dim, _stream())
-    _raise_compat("launch_gqa_attention_batch")
+    st = hostcall.launch_gqa_attention_batch(out, q, ck, cv, attn_scratch, pos, msl, G, num_heads, num_kv_heads,
+                                             head_dim, q_dim, kv_dim)
+    if st:
+        raise TqError(st, "launch_gqa_attention_batch")
 
 
 def launch_gqa_attention(q, k_cache, v_cache, output, attn_scratch, pos, max_seq_len, num_heads, num_kv_heads,
                          head_dim):
-    lib().launch_gqa_attention(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(output), _ptr(attn_scratch), int(pos),
-                               max_seq_len, num_heads, num_kv_heads, head_dim, _stream())
-    _raise_compat("launch_gqa_attention")
+    st = hostcall.launch_gqa_attention(q, k_cache, v_cache, output, attn_scratch, pos, max_seq_len, num_heads,
+                                       num_kv_heads, head_dim)
+    if st:
+        raise TqError(st, "launch_gqa_attention")
 
 
 # ---- native entry points ---------------------------------------------------------------------------------------------
 def launch_gqa_prefill_attention(out, q, ck, cv, attn_scratch, T, msl, num_heads, num_kv_heads, head_dim, q_dim, kv_dim):
     """Causal prefill attention over an fp16 cache (reference engine/kernels.cu:1359-1362)."""
-    lib().launch_gqa_prefill_attention(_ptr(out), _ptr(q), _ptr(ck), _ptr(cv), _ptr(attn_scratch), T, msl, num_heads,
-                                       num_kv_heads, head_dim, q_dim, kv_dim, _stream())
-    _raise_compat("launch_gqa_prefill_attention")
+    st = hostcall.launch_gqa_prefill_attention(out, q, ck, cv, attn_scratch, T, msl, num_heads, num_kv_heads, head_dim,
+                                               q_dim, kv_dim)
+    if st:
+        raise TqError(st, "launch_gqa_prefill_attention")
 
 
 def rotation_matrix(seed: int = 42) -> torch.Tensor:
