@@ -1,0 +1,97 @@
+"""The cluster form of the decode step (csrc/tq_decode_cluster.cuh) and the one-vector append where they can go wrong: edges
+of 16- and 32-token tiles, clusters of 1 to 16 CTAs with and without a CTA for the new token, more than 8 query heads per KV
+head, against the oracle; and the suites that the cluster form serves by default, once more with the streaming forms."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+import triebwerk_b200 as tq
+from triebwerk_b200 import ops
+from oracle import tqo
+from tests import helpers as hp
+
+pytestmark = pytest.mark.gpu
+gu = pytest.importorskip("tests.gpu_util")
+D = 128
+
+
+# capacity and batch set the cluster size: at most one CTA per SM, a 16-token block per warp
+@pytest.mark.parametrize("bits,H,Hkv,msl,lengths", [
+    (4, 16, 8, 64, [1, 16, 17, 33, 64]),               # one CTA per cluster, 32-token tiles
+    (2, 32, 8, 256, [1, 2, 128, 255]),                 # 2 CTAs
+    (4, 16, 4, 512, [1, 31, 449, 512]),                # 4 CTAs, one of them for the new token
+    (2, 8, 1, 2048, [1, 15, 16, 17, 1900]),            # 16 CTAs, 16-token tiles
+    (4, 16, 8, 2112, [1801]),                          # 16 CTAs, several tiles per warp
+    (4, 24, 2, 320, [97, 320]),                        # 12 query heads per KV head: two clusters share a KV head
+    (2, 20, 1, 96, [95]),                              # 20: three
+    (0, 40, 8, 384, [1, 16, 383]),                     # fp16 rows
+    (0, 12, 4, 1024, [1000]),
+])
+def test_decode_layer_cluster_form(bits, H, Hkv, msl, lengths):
+    rng = np.random.default_rng(1000 + 7 * bits + H + msl)
+    G, kv_dim = len(lengths), Hkv * D
+    R = ops.rotation_matrix().numpy()
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(G, msl)
+    eng.reset()
+    ks = [rng.standard_normal((n, kv_dim), dtype=np.float32).astype(np.float16) for n in lengths]
+    vs = [rng.standard_normal((n, kv_dim), dtype=np.float32).astype(np.float16) for n in lengths]
+    ks[0][-1], vs[-1][-1, :D] = 0, 0  # a new token on a quantiser bound everywhere
+    for g, n in enumerate(lengths):
+        if n > 1:
+            eng.prefill_append(0, g, gu.dev(ks[g][:-1]), gu.dev(vs[g][:-1]), 0)
+    eng.set_positions([n - 1 for n in lengths])
+    q = rng.standard_normal((G, H * D), dtype=np.float32).astype(np.float16)
+    k1, v1 = np.stack([k[-1] for k in ks]), np.stack([v[-1] for v in vs])
+    out = gu.host(eng.decode_layer(0, gu.dev(q), gu.dev(k1), gu.dev(v1)))
+    again = gu.host(eng.decode_layer(0, gu.dev(q), gu.dev(k1), gu.dev(v1)))  # chained: old rows are read early
+    assert eng.status() == 0
+    assert (out.view(np.uint16) == again.view(np.uint16)).all()
+    if bits == 0:
+        ck, cv, _, _ = (None if t is None else gu.host(t) for t in eng.layer_cache(0))
+        for g, n in enumerate(lengths):
+            assert (ck[g * msl + n - 1] == k1[g]).all() and (cv[g * msl + n - 1] == v1[g]).all()
+        ref, _ = tqo.fp16_attention_batch(q, ck, cv, np.array(lengths, np.int32) - 1, msl, H, Hkv, D)
+        hp.assert_attention_close(out, ref, H, D, f"fp16 {H}/{Hkv}")
+        return
+    gk, gv, gkn, gvn = (gu.host(t) for t in eng.layer_cache(0))
+    for g, n in enumerate(lengths):
+        r = g * msl + n - 1
+        for got, norms, x in ((gk, gkn, k1), (gv, gvn, v1)):  # the stored bytes are the launcher's (the exact chain everywhere)
+            cq, cn = gu.gpu_append_tokens(x[g:g + 1], R, [0], 1, Hkv, D, bits)
+            assert (got[r] == cq[0]).all() and (norms[r].view(np.uint16) == cn[0].view(np.uint16)).all()
+        sl = slice(g * msl, g * msl + n)
+        ref, _ = tqo.attention_single(q[g], gk[sl], gv[sl], gkn[sl], gvn[sl], R, n - 1, n, H, Hkv, D, bits)
+        hp.assert_attention_close(out[g][None], ref[None], H, D, f"tq{bits} {H}/{Hkv} seq {g}")
+
+
+@pytest.mark.parametrize("bits", [4, 2])
+@pytest.mark.parametrize("G,Hkv", [(1, 1), (3, 8), (148, 8)])
+def test_one_vector_append_vs_oracle(bits, G, Hkv):
+    """148 x 8 vectors: the last launch of one CTA per vector on a 148-SM GPU."""
+    rng = np.random.default_rng(2000 + bits + G)
+    R = ops.rotation_matrix().numpy()
+    x = rng.standard_normal((G, Hkv * D), dtype=np.float32).astype(np.float16)
+    pos = rng.integers(0, 8, G).astype(np.int32)
+    got, gn = gu.gpu_append_batch(x, R, pos, 8, Hkv, D, bits)
+    want, wn = tqo.alloc_cache(G, 8, Hkv, D, bits)
+    tqo.append_batch(want, wn, x, R, pos, 8, Hkv, D, bits)
+    # rsqrt.approx against a correctly rounded 1/sqrt: a coordinate on a bound may fall to the other side (test_append_gpu.py)
+    assert int((hp.unpack_codes(got, bits) != hp.unpack_codes(want, bits)).sum()) <= 2 + G * Hkv * D // 50000
+    assert np.abs(gn.view(np.uint16).astype(np.int32) - wn.view(np.uint16).astype(np.int32)).max() <= 1
+
+
+def test_streaming_forms_in_a_child_process():
+    """TQ_CLUSTER=0 (read once per process) keeps the streaming kernels for small batches too."""
+    if os.environ.get("TQ_CLUSTER") == "0":
+        pytest.skip("already the child")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-m", "pytest", "tests/test_attention_gpu.py", "tests/test_fp16_gpu.py", "tests/test_engine_gpu.py",
+                        "-q", "-x", "-m", "gpu", "-k", "not child and not prefill", "-p", "no:cacheprovider"],
+                       cwd=root, env=dict(os.environ, TQ_CLUSTER="0"), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    assert " passed" in r.stdout

@@ -333,4 +333,60 @@ __global__ void __launch_bounds__(APPEND_THREADS) append_rotate_kernel(const App
     }
 }
 
+// One head vector per CTA of 128 threads, for launches that fit the GPU in one wave: thread d owns output coordinate d and
+// row d of R, which goes from L2 straight into its registers (64 of them, every load in flight at once, under the input's
+// round trip) -- staging R in shared memory, as append_rotate_kernel does to reuse it, costs a small launch two more
+// barriers and a round trip.  The chain is the reference's; bound by latency (launch, one round trip, 128 dependent FMAs).
+constexpr int APPEND_VECTOR_MAX_PER_SM = 8;
+template <int BITS>
+__global__ void __launch_bounds__(HEAD_DIM) append_vector_kernel(const AppendParams p) {
+    __shared__ __align__(16) float xs[HEAD_DIM];
+    __shared__ float warp_part[4];
+    const int d = threadIdx.x, lane = d & 31, wid = d >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int nk = p.k_buf ? p.Hkv : 0, per_src = nk + (p.v_buf ? p.Hkv : 0);
+    const int src = blockIdx.x / per_src, w = blockIdx.x - src * per_src;
+    const bool is_k = w < nk;
+    const int head = is_k ? w : w - nk;
+    const float val = __half2float((is_k ? p.k_buf : p.v_buf)[(size_t)src * p.kv_dim + (size_t)head * HEAD_DIM + d]);
+    uint4 r[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = *(reinterpret_cast<const uint4*>(p.rotation + (size_t)d * HEAD_DIM) + i);
+    const int pos = p.positions ? p.positions[src] : (p.token_mode ? p.pos_value + src : p.pos_value);
+    const int cap = p.seq_capacity && !p.token_mode ? p.seq_capacity[src] : p.capacity_rows;
+    const bool ok = pos >= 0 && (cap <= 0 || pos < cap);
+    const long long row = (p.token_mode ? p.token_row0 : (p.row_base ? p.row_base[src] : (long long)src * p.max_seq_len)) + pos;
+
+    float sq = mul_ftz(val, val);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sq = add_ftz(sq, __shfl_down_sync(0xffffffffu, sq, off));
+    if (lane == 0) warp_part[wid] = sq;
+    __syncthreads();
+    const float t = add_ftz(add_ftz(add_ftz(warp_part[0], warp_part[2]), add_ftz(warp_part[1], warp_part[3])), 1e-12f);
+    xs[d] = mul_ftz(val, rsqrt_approx_ftz(t));
+    __syncthreads();
+    float acc = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float4 x0 = *reinterpret_cast<const float4*>(&xs[8 * i]), x1 = *reinterpret_cast<const float4*>(&xs[8 * i + 4]);
+        const __half2* h2 = reinterpret_cast<const __half2*>(&r[i]);
+        const float2 f0 = __half22float2(h2[0]), f1 = __half22float2(h2[1]), f2 = __half22float2(h2[2]), f3 = __half22float2(h2[3]);
+        acc = fma_ftz(f0.x, x0.x, acc); acc = fma_ftz(f0.y, x0.y, acc); acc = fma_ftz(f1.x, x0.z, acc); acc = fma_ftz(f1.y, x0.w, acc);
+        acc = fma_ftz(f2.x, x1.x, acc); acc = fma_ftz(f2.y, x1.y, acc); acc = fma_ftz(f3.x, x1.z, acc); acc = fma_ftz(f3.y, x1.w, acc);
+    }
+    // codes of 8 (16) neighbouring lanes into one 32-bit word of the row
+    uint32_t v = (uint32_t)quantize_code(acc, BITS);
+#pragma unroll
+    for (int o = 1; o * BITS < 32; o <<= 1) v |= __shfl_down_sync(0xffffffffu, v, o) << (o * BITS);
+    if (!ok) {
+        if (d == 0) atomicMax(p.status, ST_BAD_POSITION);
+        return;
+    }
+    constexpr int PER_WORD = 32 / BITS, BPH = HEAD_DIM * BITS / 8;
+    if (d % PER_WORD == 0)
+        *reinterpret_cast<uint32_t*>((is_k ? p.ck : p.cv) + ((size_t)row * p.Hkv + head) * BPH + 4 * (d / PER_WORD)) = v;
+    if (d == 0) (is_k ? p.kn : p.vn)[(size_t)row * p.Hkv + head] = __float2half_rn(sqrt_approx_ftz(t));
+}
+
 }  // namespace tq

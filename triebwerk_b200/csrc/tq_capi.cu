@@ -17,6 +17,23 @@ static inline bool use_pdl() {
     return on;
 }
 
+// The cluster kernel (tq_decode_cluster.cuh) moves 16 bytes at a time and takes one grid row per KV head and sequence.
+static inline bool cluster_shape(const void* q, const void* out, const void* ck, const void* cv, const void* rotation, int G, int H, int Hkv,
+                                 int q_dim) {
+    const int grp = H / Hkv;
+    return ((((uintptr_t)q | (uintptr_t)ck | (uintptr_t)cv | (uintptr_t)rotation) & 15u) | ((uintptr_t)out & 3u)) == 0 && q_dim % 8 == 0 &&
+           G <= 65535 && (long long)Hkv * ((grp + CD_HEADS - 1) / CD_HEADS) <= 65535;
+}
+// Small batches go to it where the streaming kernels serve the layout too: rows of a layer's slots x KV heads (its time goes
+// by those, not by bytes) up to where the two forms cross.  Measured per layer, 8 KV heads, cluster / streaming form:
+// 4-bit 16 heads 4 x 1024 8.4 / 22 us, 16 x 1024 13 / 23, 4 x 4096 19 / 27, 64 x 1024 38 / 35; 2-bit the same within 10 %;
+// with 32 heads the lines cross near 64 x 1024; fp16 16 x 1024 20 / 25, 4 x 4096 27 / 25, 16 x 4096 66 / 61.
+// TQ_CLUSTER=0 keeps the streaming kernels for every layout they serve.
+static inline bool cluster_size(int bits, long long rows, int Hkv) {
+    static const bool on = !(getenv("TQ_CLUSTER") && atoi(getenv("TQ_CLUSTER")) == 0);
+    return on && rows * Hkv <= (bits == 0 ? 131072 : 393216);
+}
+
 extern "C" {
 
 const char* tq_status_string(int status) {
@@ -527,7 +544,7 @@ void launch_turbo_kv_quantize(uint8_t* cache_q, void* cache_norms, const void* k
     if (r == TQ_OK)
         r = append_impl(cache_q, cache_norms, nullptr, nullptr, kv_buf, nullptr, nullptr, rotation, positions, 0,
                         nullptr, 1, 0, max_seq_len, num_tokens, 0, num_kv_heads, head_dim, 0, kv_dim,
-                        bits == 4 ? 4 : 2, ws, need, false, cs(s));
+                        bits == 4 ? 4 : 2, ws, need, false, cs(s), use_pdl());
     g_compat_status = r;
 }
 
@@ -541,8 +558,20 @@ void launch_turbo_kv_quantize_batch(uint8_t* cache_q, void* cache_norms, const v
     if (r == TQ_OK)
         r = append_impl(cache_q, cache_norms, nullptr, nullptr, kv_buf, nullptr, nullptr, rotation, positions, 0,
                         nullptr, 0, 0, max_seq_len, G, 0, num_kv_heads, head_dim, 0, kv_dim, bits == 4 ? 4 : 2, ws,
-                        need, false, cs(s));
+                        need, false, cs(s), use_pdl());
     g_compat_status = r;
+}
+
+// The launchers' small batches and layouts outside the streaming kernels': the cluster form.  bits 0: fp16 rows.
+static int compat_cluster_attention(void* out, const void* q, const void* ck, const void* cv, const void* k_norms, const void* v_norms,
+                                    const void* rotation, const int* pos, int pos_value, int msl, int G, int H, int Hkv, int q_dim,
+                                    int bits, cudaStream_t s) {
+    ClusterDecodeParams p{};
+    p.ck = (const uint8_t*)ck; p.cv = (const uint8_t*)cv; p.kn = (const __half*)k_norms; p.vn = (const __half*)v_norms;
+    p.q = (const __half*)q; p.rotation = (const __half*)rotation; p.out = (__half*)out;
+    p.positions = pos; p.pos_value = pos_value; p.max_seq_len = msl; p.capacity_rows = msl;
+    p.H = H; p.Hkv = Hkv; p.q_dim = q_dim; p.head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
+    return launch_cluster_decode(bits, p, G, pos ? msl : pos_value + 1, s, use_pdl());
 }
 
 void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* ck_q, const uint8_t* cv_q,
@@ -553,6 +582,15 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
     (void)as;
     bits = bits == 4 ? 4 : 2;  // the reference treats anything that is not 4 as 2-bit
     int r = check_shape(G, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits, true);
+    static const bool one_launch = !(getenv("TQ_FUSED") && atoi(getenv("TQ_FUSED")) == 0);
+    if (r == TQ_OK && one_launch && cluster_shape(q, out, ck_q, cv_q, rotation, G, num_heads, num_kv_heads, q_dim) &&
+        (!fast_shape(num_heads, num_kv_heads, true) || cluster_size(bits, (long long)G * msl, num_kv_heads))) {
+        const bool args = out && q && ck_q && cv_q && k_norms && v_norms && rotation && pos;
+        g_compat_status = args ? compat_cluster_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, pos, -1, msl, G, num_heads,
+                                                          num_kv_heads, q_dim, bits, cs(s))
+                               : TQ_ERR_ARG;
+        return;
+    }
     if (r == TQ_OK && !fast_shape(num_heads, num_kv_heads, true)) {
         g_compat_status = pos ? generic_packed_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, pos, -1, nullptr, msl, G,
                                                          num_heads, num_kv_heads, q_dim, bits, cs(s))
@@ -565,7 +603,6 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
         need = carve_full(nullptr, G, num_heads).bytes;
         r = compat_workspace(need, &ws, cs(s));
     }
-    static const bool one_launch = !(getenv("TQ_FUSED") && atoi(getenv("TQ_FUSED")) == 0);
     if (r == TQ_OK && one_launch && G <= FUSED_MAX_G && pos) {
         // one launch: the attention kernel builds its tile table and rotates the queries itself (its fused form without
         // an append); only the transpose of R for the merge precedes it
@@ -606,6 +643,14 @@ void launch_turbo_gqa_attention(const void* q, const uint8_t* ck_q, const uint8_
     const int q_dim = num_heads * head_dim, kv_dim = num_kv_heads * head_dim;
     int r = check_shape(1, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits, true);
     if (r == TQ_OK && (pos < 0 || pos >= msl)) r = TQ_ERR_CAPACITY;
+    if (r == TQ_OK && cluster_shape(q, output, ck_q, cv_q, rotation, 1, num_heads, num_kv_heads, q_dim) &&
+        (!fast_shape(num_heads, num_kv_heads, true) || cluster_size(bits, pos + 1, num_kv_heads))) {
+        const bool args = output && q && ck_q && cv_q && k_norms && v_norms && rotation;
+        g_compat_status = args ? compat_cluster_attention(output, q, ck_q, cv_q, k_norms, v_norms, rotation, nullptr, pos, msl, 1, num_heads,
+                                                          num_kv_heads, q_dim, bits, cs(s))
+                               : TQ_ERR_ARG;
+        return;
+    }
     if (r == TQ_OK && !fast_shape(num_heads, num_kv_heads, true)) {
         g_compat_status = generic_packed_attention(output, q, ck_q, cv_q, k_norms, v_norms, rotation, nullptr, pos, nullptr, msl, 1,
                                                    num_heads, num_kv_heads, q_dim, bits, cs(s));
@@ -749,6 +794,12 @@ void launch_gqa_attention_batch(void* out, const void* q, const void* ck, const 
     (void)as;
     void* ws = nullptr;
     int r = check_shape(G, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, 0, false);
+    if (r == TQ_OK && out && q && ck && cv && pos && cluster_shape(q, out, ck, cv, nullptr, G, num_heads, num_kv_heads, q_dim) &&
+        (!fast_shape(num_heads, num_kv_heads, false) || cluster_size(0, (long long)G * msl, num_kv_heads))) {
+        g_compat_status = compat_cluster_attention(out, q, ck, cv, nullptr, nullptr, nullptr, pos, -1, msl, G, num_heads, num_kv_heads, q_dim,
+                                                   0, cs(s));
+        return;
+    }
     size_t need = 0;
     if (r == TQ_OK) {
         need = fp16_workspace_bytes(G, num_heads, num_kv_heads, msl);
@@ -768,6 +819,12 @@ void launch_gqa_attention(const void* q, const void* k_cache, const void* v_cach
     void* ws = nullptr;
     int r = check_shape(1, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, 0, false);
     if (r == TQ_OK && (pos < 0 || pos >= max_seq_len)) r = TQ_ERR_CAPACITY;
+    if (r == TQ_OK && q && output && k_cache && v_cache && cluster_shape(q, output, k_cache, v_cache, nullptr, 1, num_heads, num_kv_heads, q_dim) &&
+        (!fast_shape(num_heads, num_kv_heads, false) || cluster_size(0, pos + 1, num_kv_heads))) {
+        g_compat_status = compat_cluster_attention(output, q, k_cache, v_cache, nullptr, nullptr, nullptr, nullptr, pos, max_seq_len, 1,
+                                                   num_heads, num_kv_heads, q_dim, 0, cs(stream));
+        return;
+    }
     size_t need = 0;
     if (r == TQ_OK) {
         need = fp16_workspace_bytes(1, num_heads, num_kv_heads, max_seq_len);
@@ -1352,6 +1409,16 @@ int tq_engine_read_output_f32(tq_engine* e, float* host_out, int first_layer, in
     return cuda_status(cudaStreamSynchronize(cs(s)));
 }
 
+// May a fused decode launch on `s` read positions and old cache rows before the previous kernel of the stream has finished?
+// Only when that kernel is this engine's own fused launch (`chained`), and never in a launch that is being captured into a
+// graph: it is replayed after whatever the caller puts in front of the graph.
+static bool engine_reads_early(const tq_engine* e, bool chained, cudaStream_t s) {
+    static const bool early_on = !(getenv("TQ_FUSED_EARLY") && atoi(getenv("TQ_FUSED_EARLY")) == 0);
+    if (!early_on || !use_pdl() || !chained || e->chain_stream != s) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k, const void* v, void* out,
                            tq_stream_t s) {
     if (!e || layer < 0 || layer >= e->shape.num_layers || !q || !k || !v || !out) return TQ_ERR_ARG;
@@ -1361,6 +1428,26 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     const tq_engine::Layer& L = e->layers[layer];
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, D = e->shape.head_dim;
     float* const f32 = e->out_f32 ? e->out_f32 + (size_t)layer * e->G * H * HEAD_DIM : nullptr;
+    // Head layouts outside the streaming kernels', and small batches of any layout: the cluster form, one launch.
+    const bool streaming = fast_shape(H, Hkv, e->kv_bits != 0);
+    if (e->fused && cluster_shape(q, out, L.k, L.v, e->d_rotation, e->G, H, Hkv, e->q_dim()) &&
+        (((uintptr_t)k | (uintptr_t)v) & 15u) == 0 && (!streaming || cluster_size(e->kv_bits, e->total_rows, Hkv))) {
+        ClusterDecodeParams p{};
+        p.ck = (const uint8_t*)L.k; p.cv = (const uint8_t*)L.v; p.kn = (const __half*)L.kn; p.vn = (const __half*)L.vn;
+        p.q = (const __half*)q; p.new_k = (const __half*)k; p.new_v = (const __half*)v;
+        p.rotation = (const __half*)e->d_rotation; p.out = (__half*)out; p.out_f32 = f32;
+        p.positions = e->d_positions; p.row_base = e->rb(); p.seq_capacity = e->caps();
+        if (e->shared_active) { p.prefix_base = e->d_prefix_base; p.prefix_tiles = e->d_prefix_tiles; }
+        p.status = (int*)e->workspace;
+        p.max_seq_len = e->msl; p.capacity_rows = e->msl;
+        p.H = H; p.Hkv = Hkv; p.q_dim = e->q_dim(); p.head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
+        p.early = engine_reads_early(e, chained, cs(s)) ? 1 : 0;
+        p.static_rotation = 1;
+        const int r = launch_cluster_decode(e->kv_bits, p, e->G, e->msl, cs(s), use_pdl());
+        e->chain_ok = r == TQ_OK;
+        e->chain_stream = cs(s);
+        return r;
+    }
     if (e->kv_bits == 0) {
         fp16_cache_write_kernel<<<e->G, 128, 0, cs(s)>>>((__half*)L.k, (__half*)L.v, (const __half*)k, (const __half*)v,
                                                          e->d_positions, e->rb(), e->msl, e->msl, e->G,
@@ -1382,12 +1469,7 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     }
     // One launch per layer when the batch fits the kernel's shared-memory tile table (tq_engine_set_fused).
     if (e->fused && e->G <= FUSED_MAX_G) {
-        static const bool early_on = !(getenv("TQ_FUSED_EARLY") && atoi(getenv("TQ_FUSED_EARLY")) == 0);
-        // (a launch that is being captured into a graph is replayed after whatever the caller puts in front of the
-        // graph: it never reads early)
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(cs(s), &cap) != cudaSuccess) cap = cudaStreamCaptureStatusActive;
-        const int early = (early_on && use_pdl() && chained && e->chain_stream == cs(s) && cap == cudaStreamCaptureStatusNone) ? 1 : 0;
+        const int early = engine_reads_early(e, chained, cs(s)) ? 1 : 0;
         FusedInputs in{q, k, v, e->d_rotation_rep, ROT_COPIES, early, e->caps()};
         const int r = attention_impl(out, L.tmK, L.tmV, L.k, L.v, L.kn, L.vn, e->d_rotation_t, e->d_positions, -1, e->rb(),
                                      e->total_rows, e->msl, e->G, H, Hkv, e->q_dim(), e->kv_bits, e->workspace, e->ws_bytes,

@@ -19,6 +19,7 @@
 #include "tq_prefill_tc.cuh"
 #include "tq_attention.cuh"
 #include "tq_common.cuh"
+#include "tq_decode_cluster.cuh"
 #include "tq_fp16.cuh"
 #include "tq_fp16_tc.cuh"
 #include "tq_qrot.cuh"
@@ -218,7 +219,7 @@ inline int launch_kernel(Kernel kernel, dim3 grid, dim3 block, size_t smem, cuda
 constexpr size_t APPEND_SMEM = (size_t)HEAD_DIM * HEAD_DIM * sizeof(float);  // R as fp32
 
 // Opt-in to large dynamic shared memory, once per (device, kernel); safe to call from several host threads.
-inline int ensure_dynamic_smem(const void* func, size_t bytes) {
+inline int ensure_dynamic_smem(const void* func, size_t bytes, bool big_clusters = false) {
     static std::mutex mu;
     static std::map<std::pair<int, const void*>, bool> done;
     int dev = 0;
@@ -227,6 +228,7 @@ inline int ensure_dynamic_smem(const void* func, size_t bytes) {
     bool& d = done[std::make_pair(dev, func)];
     if (!d) {
         TQ_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        if (big_clusters) TQ_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         d = true;
     }
     return TQ_OK;
@@ -236,7 +238,7 @@ template <int NV>
 inline int launch_append_t(const AppendParams& p, dim3 grid, cudaStream_t s, bool pdl) {
     int r = ensure_dynamic_smem((const void*)append_rotate_kernel<NV>, APPEND_SMEM);
     if (r != TQ_OK) return r;
-    return launch_kernel(append_rotate_kernel<NV>, grid, dim3(APPEND_THREADS), APPEND_SMEM, s, pdl, p);
+    return launch_kernel(append_rotate_kernel<NV>, grid, dim3(APPEND_THREADS), APPEND_SMEM, s, pdl && p.rot_prep, p);  // (it reads a caller's R before the wait)
 }
 
 // Whole prompts (token form, K and/or V, no queries) go to the tensor-core kernel; TQ_PREFILL_TC=0 keeps them on
@@ -311,6 +313,11 @@ inline int launch_append(const AppendParams& p, cudaStream_t s, bool pdl = false
     const bool tables = p.tile_start != nullptr && !p.token_mode;
     if (total <= 0 && !tables) return TQ_OK;
     if (total >= (1ll << 31)) return TQ_ERR_CAPACITY;
+    // A few vectors and nothing else to do: one CTA each (16-byte loads of R's rows, 4-byte stores of code words).
+    if (!p.q && !tables && total <= (long long)APPEND_VECTOR_MAX_PER_SM * device_props().sm_count && (((uintptr_t)p.rotation & 15u) == 0) &&
+        ((((uintptr_t)p.ck | (uintptr_t)p.cv) & 3u) == 0))
+        return p.bits == 4 ? launch_kernel(append_vector_kernel<4>, dim3((unsigned)total), dim3(HEAD_DIM), 0, s, pdl, p)
+                           : launch_kernel(append_vector_kernel<2>, dim3((unsigned)total), dim3(HEAD_DIM), 0, s, pdl, p);
     // One CTA per SM at most.  As few vectors per group as still fit the whole launch into that one wave: short
     // dependent chains when the batch is small, amortised staging of R when it is large (then the CTAs loop).
     const long long slots = (long long)device_props().sm_count - 1;
@@ -369,6 +376,40 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
     if (mode == 1) { TQ_ATTN_DISPATCH(1) }
     TQ_ATTN_DISPATCH(0)
 #undef TQ_ATTN_DISPATCH
+}
+
+// One cluster per (sequence, KV head, block of 8 query heads): tq_decode_cluster.cuh.  `max_tokens`: rows a sequence may hold.
+template <int BITS, int MB>
+inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int G, cudaStream_t s, bool pdl) {
+    const void* kernel = (const void*)cluster_decode_kernel<BITS, MB>;
+    int r = ensure_dynamic_smem(kernel, cd_smem_bytes(BITS, CD_HEADS), true);
+    if (r != TQ_OK) return r;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)S, (unsigned)(p.Hkv * p.head_blocks), (unsigned)G);
+    cfg.blockDim = dim3(CD_THREADS);
+    cfg.dynamicSmemBytes = cd_smem_bytes(BITS, std::min(CD_HEADS, p.H / p.Hkv));
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)S;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB>, p));
+}
+inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int G, int max_tokens, cudaStream_t s, bool pdl) {
+    // As many CTAs per cluster as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch (two
+    // share the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue: 8 sequences x 1023
+    // tokens through the launchers 24 us a layer with two, 19 with one).
+    const long long clusters = (long long)G * p.Hkv * p.head_blocks, blocks = (max_tokens + 15) / 16;
+    int S = 1;
+    while (S < CD_MAX_CLUSTER && (long long)S * CD_WARPS < blocks && clusters * S * 2 <= device_props().sm_count) S *= 2;
+    if (bits == 0) return launch_cluster_decode_t<0, 1>(p, S, G, s, pdl);
+    const bool one = (long long)S * CD_WARPS >= blocks;  // a single 16-token tile per warp
+    if (bits == 4) return one ? launch_cluster_decode_t<4, 1>(p, S, G, s, pdl) : launch_cluster_decode_t<4, 2>(p, S, G, s, pdl);
+    return one ? launch_cluster_decode_t<2, 1>(p, S, G, s, pdl) : launch_cluster_decode_t<2, 2>(p, S, G, s, pdl);
 }
 
 __global__ void transpose_rotation_kernel(__half* dst, const __half* src, int* tickets = nullptr, int n_tickets = 0) {
