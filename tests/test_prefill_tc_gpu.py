@@ -1,0 +1,64 @@
+"""The tcgen05 prefill attention (csrc/tq_prefill_fa.cuh) where it can go wrong: edges of its 128-row tiles and query blocks, one
+and two query blocks per CTA, any number of query heads per KV head, prompts that go through the scratch in groups.  Against the
+oracle on the engine's own cache bytes."""
+import numpy as np
+import pytest
+import torch
+
+import triebwerk_b200 as tq
+from oracle import tqo
+from tests import helpers as hp
+
+pytestmark = pytest.mark.gpu
+gu = pytest.importorskip("tests.gpu_util")
+D = 128
+
+
+@pytest.mark.parametrize("bits,H,Hkv,n,T,msl", [
+    # few blocks: one query block per CTA, even and odd tiles in its two slots
+    (4, 16, 8, 1, 1, 32), (4, 16, 8, 1, 127, 128), (2, 16, 8, 1, 128, 160), (0, 16, 8, 1, 129, 160), (4, 32, 8, 2, 257, 288),
+    (0, 8, 8, 1, 385, 416), (2, 40, 8, 1, 150, 160), (4, 24, 2, 1, 140, 160), (0, 40, 8, 1, 51, 64), (4, 96, 1, 1, 130, 160),
+    # many: two query blocks per CTA (8 KV heads x 8 prompts x 3 pairs of blocks), the last pair with one block or none at the end
+    (4, 16, 8, 8, 300, 320), (2, 16, 8, 8, 257, 288), (0, 16, 8, 8, 321, 352), (4, 40, 8, 8, 160, 160), (0, 16, 8, 13, 129, 160),
+])
+def test_prefill_attention_edges(bits, H, Hkv, n, T, msl):
+    rng = np.random.default_rng(4000 + 17 * bits + H + T)
+    kv_dim = Hkv * D
+    R = tq.ops.rotation_matrix().numpy()
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(n, msl)
+    for t in eng.layer_cache(0):  # rows past the prompts: codes of any kind, norms and fp16 values that are not numbers
+        if t is not None:
+            t.view(torch.int16).fill_(0x7E00)
+    k, v = (rng.standard_normal((n, T, kv_dim), dtype=np.float32).astype(np.float16) for _ in range(2))
+    q = rng.standard_normal((n, T, H * D), dtype=np.float32).astype(np.float16)
+    got = gu.host(eng.prefill_layer_batch(0, 0, gu.dev(q), gu.dev(k), gu.dev(v)))
+    assert eng.status() == 0
+    assert np.isfinite(got.astype(np.float32)).all()
+    cache = [None if t is None else gu.host(t) for t in eng.layer_cache(0)]
+    for i in {0, n // 2, n - 1}:
+        sl = slice(i * msl, i * msl + T)
+        if bits == 0:
+            toks = sorted({0, 1, 24, 25, 63, 64, 127, 128, T // 2, T - 2, T - 1} & set(range(T)))
+            ref = np.stack([tqo.fp16_attention_single(q[i, t], k[i], v[i], t, T, H, Hkv, D)[0] for t in toks])
+            hp.assert_attention_close(got[i][toks], ref, H, D, f"fp16 {H}/{Hkv} T={T} prompt {i}")
+        else:
+            ck, cv, kn, vn = (t[sl] for t in cache)
+            ref, _ = tqo.prefill_attention(q[i], ck, cv, kn, vn, R, T, H, Hkv, D, bits)
+            hp.assert_attention_close(got[i], ref, H, D, f"tq{bits} {H}/{Hkv} T={T} prompt {i}")
+
+
+def test_prompts_pass_through_the_scratch_in_groups():
+    """20 prompts of 1000 tokens: more than the 16384 tokens that fit the fp16 scratch at a time."""
+    H, Hkv, n, T = 8, 4, 20, 1000
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    k, v = (torch.randn(n, T, Hkv * D, generator=gen, device="cuda").half() for _ in range(2))
+    q = torch.randn(n, T, H * D, generator=gen, device="cuda").half()
+    eng = tq.Engine(1024, 4, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(n, 1024)
+    together = eng.prefill_layer_batch(0, 0, q, k, v)
+    for i in (0, 15, 16, 19):
+        one = eng.prefill_layer(0, i, q[i], k[i], v[i])
+        # (one prompt alone has one query block per CTA, the batch two: another order of summation)
+        assert torch.allclose(together[i].float(), one.float(), atol=1e-3, rtol=2e-3)
+    assert eng.status() == 0

@@ -90,10 +90,6 @@ struct AttnParams {
     int early;                 // 1: positions and this layer's cache tiles may be read before the previous kernel in the
                                // stream has finished (the caller knows it writes neither): table, slice and first copies
                                // then run under that kernel's tail
-    // prefill form: a "sequence" of the launch is a group of qg consecutive query tokens of ONE cache (row base 0); its
-    // H = qg * (real heads) rows are ordered (kv head, token in group, head of the kv head); token t attends to rows 0..t
-    int qg;                    // 0 or 1: plain decode
-    int qg_tokens;             // number of query tokens (the last group may be partial)
     int l2_ahead;              // tiles prefetched into L2 beyond the shared-memory ring
     // whole-step form (MODE 2): ONE launch streams the layers [layer0, layer0 + n_layers) back to back -- every worker
     // walks its slice of the tile list once per layer, its ring of stages never drains in between -- rotates the
@@ -981,14 +977,6 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         const long long seg_end = hi < ts_g1 ? hi : ts_g1;
         const int pos = p.positions ? p.positions[g] : p.pos_value;
         const int L = (pos < 0 ? 0 : pos) + 1;
-        // causal limit of this lane's score row (row gl) and of the group's first token; equal to L outside the prefill form
-        const int qg = FUSED ? 0 : p.qg;  // the fused form is a decode step: no token groups
-        const int grp_real = qg > 1 ? grp / qg : grp;
-        // (this lane's score columns are the heads 2*t4 and 2*t4 + 1 of its KV head)
-        const int Lcol0 = qg > 1 ? min(L, g * qg + (2 * t4) / grp_real + 1) : L;
-        const int Lcol1 = qg > 1 ? min(L, g * qg + (2 * t4 + 1) / grp_real + 1) : L;
-        const int Lmin = qg > 1 ? min(L, g * qg + 1) : L;
-
         TQ_STAMP(8);   // loop tail + publishing of the previous segment + this segment's table / position reads
         // query fragments (B operand of the score product): lane (gl, t4) holds coordinates 32*t4 .. 32*t4+31 of head
         // head*grp + gl as fp16
@@ -1126,7 +1114,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 
         for (; tile < seg_end; ++tile) {
             const int t0 = (int)(tile - ts_g) * TILE_TOKENS;
-            const bool full = t0 + TILE_TOKENS <= Lmin;  // warp-uniform: no token of the tile is masked for any row
+            const bool full = t0 + TILE_TOKENS <= L;  // warp-uniform: no token of the tile is masked
             const int s = BITS == 2 ? s_idx : (consumed & (S - 1));
             const uint32_t parity = BITS == 2 ? s_par : ((uint32_t)(consumed >> s_log) & 1u);
             // the tile that takes this stage's place (warp-uniform; every warp of the worker advances the cursor in step)
@@ -1237,8 +1225,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #pragma unroll
                     for (int blk = 0; blk < 4; ++blk) {
                         const int tok = t0 + 8 * blk + (int)tauK;
-                        if (tok >= Lcol0) sv[blk][0] = -1e30f;
-                        if (tok >= Lcol1) sv[blk][1] = -1e30f;
+                        if (tok >= L) sv[blk][0] = sv[blk][1] = -1e30f;
                     }
                 }
                 float mx0 = fmaxf(fmaxf(sv[0][0], sv[1][0]), fmaxf(sv[2][0], sv[3][0]));
@@ -1272,8 +1259,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #pragma unroll
                     for (int blk = 0; blk < 4; ++blk) {
                         const int tok = t0 + 8 * blk + (int)tauK;
-                        if (tok >= Lcol0) pv[blk][0] = 0.0f;
-                        if (tok >= Lcol1) pv[blk][1] = 0.0f;
+                        if (tok >= L) pv[blk][0] = pv[blk][1] = 0.0f;
                     }
                 }
                 l_run[0] += (pv[0][0] + pv[1][0]) + (pv[2][0] + pv[3][0]);
@@ -1440,15 +1426,11 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             // where row vh of this sequence's output goes (null: nowhere)
             auto out_row = [&](int vh) -> __half* {
                 if (vh >= H) return nullptr;
-                if (qg <= 1) return p.out + (size_t)g * p.q_dim + (size_t)vh * HEAD_DIM;
-                const int kvh = vh / grp, r = vh - kvh * grp, qi = r / grp_real, hq = r - qi * grp_real;
-                const int token = g * qg + qi;
-                if (token >= p.qg_tokens) return nullptr;
-                return p.out + (size_t)token * p.q_dim + (size_t)(kvh * grp_real + hq) * HEAD_DIM;
+                return p.out + (size_t)g * p.q_dim + (size_t)vh * HEAD_DIM;
             };
-            // optional copy of the results before their rounding to fp16 (decode form only)
+            // optional copy of the results before their rounding to fp16
             auto out_row_f32 = [&](int vh) -> float* {
-                if (!p.out_f32 || vh >= H || qg > 1) return nullptr;
+                if (!p.out_f32 || vh >= H) return nullptr;
                 return p.out_f32 + ((size_t)g * H + (size_t)vh) * HEAD_DIM;
             };
             merge_sequence<Hkv>(p.partials + (size_t)(first_w + g) * H * PART_STRIDE, parts, H, merge_s, p.rotation_t, head, lane,

@@ -245,7 +245,7 @@ static int append_impl(uint8_t* ck_q, void* k_norms, uint8_t* cv_q, void* v_norm
                        const long long* row_base, int token_mode, long long token_row0, int max_seq_len, int n_src,
                        int num_heads, int num_kv_heads, int head_dim, int q_dim, int kv_dim, int bits, void* workspace,
                        size_t workspace_bytes, bool build_tiles, cudaStream_t s, bool pdl = false,
-                       const float* rot_prep = nullptr, int qg = 0, const int* seq_capacity = nullptr) {
+                       const float* rot_prep = nullptr, const int* seq_capacity = nullptr) {
     if (head_dim != HEAD_DIM) return TQ_ERR_UNSUPPORTED;
     if (bits != 2 && bits != 4) return TQ_ERR_ARG;
     if (n_src <= 0 || num_kv_heads <= 0 || kv_dim != num_kv_heads * head_dim || !rotation) return TQ_ERR_ARG;
@@ -272,7 +272,6 @@ static int append_impl(uint8_t* ck_q, void* k_norms, uint8_t* cv_q, void* v_norm
     p.max_seq_len = max_seq_len; p.capacity_rows = max_seq_len;
     p.n_src = n_src; p.H = num_heads; p.Hkv = num_kv_heads; p.q_dim = q_dim; p.kv_dim = kv_dim; p.bits = bits;
     p.pos_value = pos_value;
-    p.qg = qg;
     p.seq_capacity = seq_capacity;
     return launch_append(p, s, pdl);
 }
@@ -303,7 +302,7 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
                           const void* rotation_t, const int* positions, int pos_value, const long long* row_base,
                           long long total_rows, int max_seq_len, int G, int num_heads, int num_kv_heads, int q_dim,
                           int bits, void* workspace, size_t workspace_bytes, cudaStream_t s, bool pdl = false,
-                          const FusedInputs* fused = nullptr, int qg = 0, int qg_tokens = 0, float* out_f32 = nullptr,
+                          const FusedInputs* fused = nullptr, float* out_f32 = nullptr,
                           const long long* prefix_base = nullptr, const int* prefix_tiles = nullptr) {
     FullWorkspace fw = carve_full(workspace, G, num_heads);
     if (fw.bytes > workspace_bytes) return TQ_ERR_WORKSPACE;
@@ -322,11 +321,6 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
     p.total_rows = total_rows;
     p.pos_value = pos_value; p.max_seq_len = max_seq_len;
     p.G = G; p.H = num_heads; p.Hkv = num_kv_heads; p.q_dim = q_dim;
-    p.qg = qg; p.qg_tokens = qg_tokens;
-    if (qg > 1) {  // groups of query tokens are short sequences: what each costs beside its tiles, in tiles (measured)
-        static const int seq_weight = getenv("TQ_PREFILL_SEQ_WEIGHT") ? atoi(getenv("TQ_PREFILL_SEQ_WEIGHT")) : 10;
-        p.app_weight = seq_weight < 0 ? 0 : seq_weight;
-    }
 #ifdef TQ_TIMING_SWITCHES
     static const int debug_mode = getenv("TQ_ATTN_DEBUG") ? atoi(getenv("TQ_ATTN_DEBUG")) : 0;
     p.debug = debug_mode;
@@ -387,17 +381,16 @@ __global__ void causal_rows_kernel(int* pos, long long* rows, int n) {
 }
 
 // Any head layout: one CTA per (sequence, query head), see tq_generic.cuh.
-static int generic_packed_attention(void* out, const void* q, const void* ck_q, const void* cv_q, const void* k_norms,
-                                    const void* v_norms, const void* rotation, const int* positions, int pos_value,
-                                    const long long* row_base, int max_seq_len, int G, int H, int Hkv, int q_dim, int bits,
-                                    cudaStream_t s) {
-    if (!out || !q || !ck_q || !cv_q || !k_norms || !v_norms || !rotation) return TQ_ERR_ARG;
+static int generic_attention(void* out, const void* q, const void* ck, const void* cv, const void* k_norms, const void* v_norms,
+                             const void* rotation, const int* positions, int pos_value, const long long* row_base, int max_seq_len,
+                             int G, int H, int Hkv, int q_dim, int bits, cudaStream_t s) {
+    if (!out || !q || !ck || !cv || (bits != 0 && (!k_norms || !v_norms || !rotation))) return TQ_ERR_ARG;
     GenericAttnParams p{};
-    p.ck = (const uint8_t*)ck_q; p.cv = (const uint8_t*)cv_q; p.kn = (const __half*)k_norms; p.vn = (const __half*)v_norms;
+    p.ck = (const uint8_t*)ck; p.cv = (const uint8_t*)cv; p.kn = (const __half*)k_norms; p.vn = (const __half*)v_norms;
     p.q = (const __half*)q; p.rotation = (const __half*)rotation; p.out = (__half*)out;
     p.positions = positions; p.row_base = row_base; p.pos_value = pos_value; p.max_seq_len = max_seq_len;
     p.G = G; p.H = H; p.Hkv = Hkv; p.q_dim = q_dim; p.bits = bits;
-    return launch_generic_attention(p, false, s);
+    return launch_generic_attention(p, bits == 0, s);
 }
 
 // ---- allocation-free decode attention -----------------------------------------------------------------------------------
@@ -489,11 +482,8 @@ int tq_fp16_decode_attention(void* out, const void* q, const void* ck, const voi
     if (!out || !q || !ck || !cv) return TQ_ERR_ARG;
     if (!positions && pos_value < 0) return TQ_ERR_ARG;
     if (!fast_shape(num_heads, num_kv_heads, false)) {  // 3, 5, 6, 7 or more than 8 query heads per KV head
-        GenericAttnParams gp{};
-        gp.ck = (const uint8_t*)ck; gp.cv = (const uint8_t*)cv; gp.q = (const __half*)q; gp.out = (__half*)out;
-        gp.positions = positions; gp.row_base = row_base; gp.pos_value = pos_value; gp.max_seq_len = max_seq_len;
-        gp.G = G; gp.H = num_heads; gp.Hkv = num_kv_heads; gp.q_dim = q_dim; gp.bits = 0;
-        return launch_generic_attention(gp, true, cs(s));
+        return generic_attention(out, q, ck, cv, nullptr, nullptr, nullptr, positions, pos_value, row_base, max_seq_len, G, num_heads,
+                                 num_kv_heads, q_dim, 0, cs(s));
     }
     if (!workspace) return TQ_ERR_WORKSPACE;
     // fp16 layout of the workspace: [0,256) header, tickets int[G*H] (one per sequence and virtual KV head, at most H), partials
@@ -592,7 +582,7 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
         return;
     }
     if (r == TQ_OK && !fast_shape(num_heads, num_kv_heads, true)) {
-        g_compat_status = pos ? generic_packed_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, pos, -1, nullptr, msl, G,
+        g_compat_status = pos ? generic_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, pos, -1, nullptr, msl, G,
                                                          num_heads, num_kv_heads, q_dim, bits, cs(s))
                               : TQ_ERR_ARG;
         return;
@@ -652,7 +642,7 @@ void launch_turbo_gqa_attention(const void* q, const uint8_t* ck_q, const uint8_
         return;
     }
     if (r == TQ_OK && !fast_shape(num_heads, num_kv_heads, true)) {
-        g_compat_status = generic_packed_attention(output, q, ck_q, cv_q, k_norms, v_norms, rotation, nullptr, pos, nullptr, msl, 1,
+        g_compat_status = generic_attention(output, q, ck_q, cv_q, k_norms, v_norms, rotation, nullptr, pos, nullptr, msl, 1,
                                                    num_heads, num_kv_heads, q_dim, bits, cs(s));
         return;
     }
@@ -671,114 +661,47 @@ void launch_turbo_gqa_attention(const void* q, const uint8_t* ck_q, const uint8_
     g_compat_status = r;
 }
 
+// The causal prefill attention of one prompt behind both launchers: the tensor-core kernel, or, for what it does not take (arrays
+// off a 16-byte boundary, more than 128 query heads per KV head), every query token as a "sequence" of its own (position t,
+// row base 0) through the generic kernel.  bits 0: fp16 rows.
+static int compat_prefill_attention(void* out, const void* q, const void* ck, const void* cv, const void* k_norms, const void* v_norms,
+                                    const void* rotation, int T, int msl, int H, int Hkv, int q_dim, int bits, cudaStream_t s) {
+    if (!out || !q || !ck || !cv || (bits != 0 && (!k_norms || !v_norms || !rotation))) return TQ_ERR_ARG;
+    if (T > msl) return TQ_ERR_CAPACITY;
+    void* ws = nullptr;
+    const bool aligned = (((uintptr_t)q | (uintptr_t)out | (uintptr_t)ck | (uintptr_t)cv | (uintptr_t)rotation) & 15u) == 0 && q_dim % 8 == 0;
+    if (aligned && prefill_attn_shape(H, Hkv)) {
+        const size_t scratch = bits ? prefill_scratch_bytes(T, Hkv) : 0;
+        int r = compat_workspace(256 + scratch, &ws, s);
+        if (r != TQ_OK) return r;
+        PrefillAttnParams p{};
+        p.q = (const __half*)q; p.q_tok_stride = q_dim;
+        p.ck = (const uint8_t*)ck; p.cv = (const uint8_t*)cv; p.kn = (const __half*)k_norms; p.vn = (const __half*)v_norms;
+        p.rotation = (const __half*)rotation; p.out = (__half*)out; p.q_dim = q_dim;
+        p.status = (int*)ws;
+        p.T = T; p.H = H; p.Hkv = Hkv;
+        return launch_prefill_attention(bits, p, msl, (char*)ws + 256, scratch, s);
+    }
+    int r = compat_workspace(align_up((size_t)T * sizeof(int), 256) + (size_t)T * sizeof(long long), &ws, s);
+    if (r != TQ_OK) return r;
+    int* pos = (int*)ws;
+    long long* rows = (long long*)((char*)ws + align_up((size_t)T * sizeof(int), 256));
+    causal_rows_kernel<<<(T + 127) / 128, 128, 0, s>>>(pos, rows, T);
+    r = cuda_status(cudaGetLastError());
+    if (r != TQ_OK) return r;
+    return generic_attention(out, q, ck, cv, k_norms, v_norms, rotation, pos, -1, rows, msl, T, H, Hkv, q_dim, bits, s);
+}
+
 void launch_turbo_gqa_prefill_attention(void* out, const void* q, const uint8_t* ck_q, const uint8_t* cv_q,
                                         const void* k_norms, const void* v_norms, const void* rotation, float* as,
                                         int T, int msl, int num_heads, int num_kv_heads, int head_dim, int q_dim,
                                         int kv_dim, int bits, tq_stream_t s) {
     std::lock_guard<std::recursive_mutex> compat_lock(compat_mutex());  // per-device compat state, see tq_host.cuh
     (void)as;
-    // Query t attends to rows 0..t of ONE sequence.  The decode kernel serves up to 8 score rows per KV head at the
-    // price of one: groups of qg = 8 / (heads per KV head) consecutive query tokens become the "sequences" of the launch,
-    // their rows ordered (kv head, token in group, head), each row with its own causal limit.  Every cache tile is then
-    // fetched and dequantised once per group instead of once per token.
     bits = bits == 4 ? 4 : 2;
     int r = check_shape(T, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits, true);
-    if (r == TQ_OK && T > msl) r = TQ_ERR_CAPACITY;
-    if (r == TQ_OK && !fast_shape(num_heads, num_kv_heads, true)) {
-        // every query token as a "sequence" of its own: position t, row base 0
-        void* gws = nullptr;
-        const size_t gneed = align_up((size_t)T * sizeof(int), 256) + align_up((size_t)T * sizeof(long long), 256);
-        r = compat_workspace(gneed, &gws, cs(s));
-        if (r == TQ_OK) {
-            int* gpos = (int*)gws;
-            long long* grows = (long long*)((char*)gws + align_up((size_t)T * sizeof(int), 256));
-            causal_rows_kernel<<<(T + 127) / 128, 128, 0, cs(s)>>>(gpos, grows, T);
-            r = cuda_status(cudaGetLastError());
-            if (r == TQ_OK)
-                r = generic_packed_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, gpos, -1, grows, msl, T, num_heads,
-                                             num_kv_heads, q_dim, bits, cs(s));
-        }
-        g_compat_status = r;
-        return;
-    }
-    static const bool dedicated = !(getenv("TQ_PREFILL_ATTN") && atoi(getenv("TQ_PREFILL_ATTN")) == 0);
-    if (r == TQ_OK && dedicated && prefill_attn_shape(num_heads, num_kv_heads)) {
-        // the kernel with the query tokens in the M dimension: one launch (it rotates its queries, attends, normalises and
-        // applies R^T)
-        PrefillAttnParams ap{};
-        ap.q = (const __half*)q;
-        ap.q_tok_stride = q_dim;
-        ap.ck = ck_q;
-        ap.cv = cv_q;
-        ap.kn = (const __half*)k_norms;
-        ap.vn = (const __half*)v_norms;
-        ap.rotation = (const __half*)rotation;
-        {  // the tcgen05 form wants R^T as well: 32 KB of the launchers' workspace, written by a small launch
-            void* pws = nullptr;
-            r = compat_workspace((size_t)HEAD_DIM * HEAD_DIM * sizeof(__half) + 256, &pws, cs(s));
-            if (r == TQ_OK) {
-                ap.status = (int*)pws;
-                ap.rotation_t = (const __half*)((char*)pws + 256);
-                transpose_rotation_kernel<<<16, 256, 0, cs(s)>>>((__half*)((char*)pws + 256), (const __half*)rotation);
-                r = cuda_status(cudaGetLastError());
-            }
-            if (r != TQ_OK) {
-                g_compat_status = r;
-                return;
-            }
-        }
-        ap.out = (__half*)out;
-        ap.q_dim = q_dim;
-        ap.T = T;
-        ap.rows = msl;
-        ap.H = num_heads;
-        ap.Hkv = num_kv_heads;
-        ap.score_scale = 1.0f;
-        r = launch_prefill_attention(bits, ap, cs(s));
-        g_compat_status = r;
-        return;
-    }
-    void* ws = nullptr;
-    size_t need = 0;
-    int qg = 1, groups = T, vheads = num_heads;
-    if (r == TQ_OK) {
-        const int grp = num_heads / num_kv_heads;
-        static const bool grouped = !(getenv("TQ_PREFILL_QG") && atoi(getenv("TQ_PREFILL_QG")) == 0);
-        qg = grouped ? 8 / grp : 1;
-        if (qg < 1) qg = 1;
-        groups = (T + qg - 1) / qg;
-        vheads = num_heads * qg;
-        need = std::max(carve_full(nullptr, groups, vheads).bytes, carve_full(nullptr, T, num_heads).bytes);
-        r = compat_workspace(need, &ws, cs(s));
-    }
-    if (r == TQ_OK) {
-        FullWorkspace fw = carve_full(ws, groups, vheads);
-        // rotated queries of all T tokens (positions play no part in that), written in the grouped row order
-        r = append_impl(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, q, rotation, nullptr, 0, nullptr, 0, 0, msl, T,
-                        num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits, ws, need, false, cs(s), false, nullptr, qg);
-        // the tile table of the groups: group j ends at token min((j + 1) * qg, T) - 1; every group starts at row 0
-        if (r == TQ_OK) {
-            group_rows_kernel<<<(groups + 127) / 128, 128, 0, cs(s)>>>(fw.aux_pos, fw.aux_rows, groups, qg, T);
-            r = cuda_status(cudaGetLastError());
-        }
-        if (r == TQ_OK)
-            r = append_impl(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, rotation, fw.aux_pos, 0, fw.aux_rows,
-                            0, 0, msl, groups, vheads, num_kv_heads, head_dim, vheads * head_dim, kv_dim, bits, ws, need, true,
-                            cs(s));
-        if (r == TQ_OK) {
-            CUtensorMap tmK, tmV;
-            const int kvp = num_kv_heads * (bits == 4 ? 64 : 32);
-            r = cached_code_map(&tmK, ck_q, msl, kvp);
-            if (r == TQ_OK) r = cached_code_map(&tmV, cv_q, msl, kvp);
-            if (r == TQ_OK) {
-                transpose_rotation_kernel<<<16, 256, 0, cs(s)>>>(fw.rot_t, (const __half*)rotation);
-                r = cuda_status(cudaGetLastError());
-            }
-            if (r == TQ_OK)
-                r = attention_impl(out, tmK, tmV, ck_q, cv_q, k_norms, v_norms, fw.rot_t, fw.aux_pos, -1, fw.aux_rows, msl, msl,
-                                   groups, vheads, num_kv_heads, q_dim, bits, ws, need, cs(s), false, nullptr, qg, T);
-        }
-    }
+    if (r == TQ_OK)
+        r = compat_prefill_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, T, msl, num_heads, num_kv_heads, q_dim, bits, cs(s));
     g_compat_status = r;
 }
 
@@ -836,48 +759,12 @@ void launch_gqa_attention(const void* q, const void* k_cache, const void* v_cach
     g_compat_status = r;
 }
 
-// Causal prefill attention over an fp16 cache (kv_bits = 0), replaces launch_gqa_prefill_attention
-// (engine/kernels.cu:1071-1158, 1359-1362): query token t of ONE sequence attends to cache rows 0 .. t.  Served by the
-// fp16 decode kernel with every query token as a "sequence" of its own (position t, row base 0): no O(T^2) score scratch.
 void launch_gqa_prefill_attention(void* out, const void* q, const void* ck, const void* cv, float* as, int T, int msl,
                                   int num_heads, int num_kv_heads, int head_dim, int q_dim, int kv_dim, tq_stream_t s) {
     std::lock_guard<std::recursive_mutex> compat_lock(compat_mutex());  // per-device compat state, see tq_host.cuh
     (void)as;
     int r = check_shape(T, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, 0, false);
-    if (r == TQ_OK && T > msl) r = TQ_ERR_CAPACITY;
-    static const bool dedicated = !(getenv("TQ_PREFILL_ATTN") && atoi(getenv("TQ_PREFILL_ATTN")) == 0);
-    if (r == TQ_OK && dedicated && prefill_attn_shape(num_heads, num_kv_heads) && kv_dim == num_kv_heads * HEAD_DIM) {
-        PrefillAttnParams ap{};
-        ap.q = (const __half*)q;
-        ap.q_tok_stride = q_dim;
-        ap.ck = (const uint8_t*)ck;
-        ap.cv = (const uint8_t*)cv;
-        ap.out = (__half*)out;
-        ap.q_dim = q_dim;
-        ap.T = T;
-        ap.rows = msl;
-        ap.H = num_heads;
-        ap.Hkv = num_kv_heads;
-        ap.score_scale = 0.12751743074602467f;  // log2(e) / sqrt(128)
-        g_compat_status = launch_prefill_attention(0, ap, cs(s));
-        return;
-    }
-    void* ws = nullptr;
-    size_t attn_bytes = 0, need = 0;
-    if (r == TQ_OK) {
-        attn_bytes = align_up(fp16_workspace_bytes(T, num_heads, num_kv_heads, msl), 256);
-        need = attn_bytes + align_up((size_t)T * sizeof(int), 256) + align_up((size_t)T * sizeof(long long), 256);
-        r = compat_workspace(need, &ws, cs(s));
-    }
-    if (r == TQ_OK) {
-        int* pos = (int*)((char*)ws + attn_bytes);
-        long long* rows = (long long*)((char*)pos + align_up((size_t)T * sizeof(int), 256));
-        causal_rows_kernel<<<(T + 127) / 128, 128, 0, cs(s)>>>(pos, rows, T);
-        r = cuda_status(cudaGetLastError());
-        if (r == TQ_OK)
-            r = tq_fp16_decode_attention(out, q, ck, cv, pos, -1, rows, msl, msl, T, num_heads, num_kv_heads, head_dim, q_dim,
-                                         kv_dim, ws, attn_bytes, s);
-    }
+    if (r == TQ_OK) r = compat_prefill_attention(out, q, ck, cv, nullptr, nullptr, nullptr, T, msl, num_heads, num_kv_heads, q_dim, 0, cs(s));
     g_compat_status = r;
 }
 
@@ -955,6 +842,8 @@ static void engine_release_arena(tq_engine* e) {
     e->step_table = nullptr;
     e->step_qrot = nullptr;
     e->step_kpost = nullptr;
+    e->prefill_scratch = nullptr;
+    e->prefill_scratch_bytes = 0;
     e->workspace = nullptr;
     for (auto& l : e->layers) l = tq_engine::Layer();
 }
@@ -1039,7 +928,13 @@ static size_t engine_carve(tq_engine* e, char* base, int G, int msl, long long r
     const size_t qb = (size_t)e->shape.num_layers * G * e->q_dim() * 2;
     const size_t kb = (size_t)e->shape.num_layers * G * e->kv_dim() * 2;
     size_t oq = bump(off, qb), okk = bump(off, kb), ovv = bump(off, kb), oo = bump(off, qb);
+    // prompts on their way through the prefill attention as fp16 rows: one full slot, or several up to 16384 tokens together
+    const size_t pf_tokens = std::max<size_t>((size_t)msl, std::min<size_t>((size_t)rows, 16384));
+    const size_t pf_bytes = e->kv_bits ? prefill_scratch_bytes((int)pf_tokens, e->shape.num_kv_heads) : 0;
+    size_t opf = bump(off, pf_bytes);
     if (assign) {
+        e->prefill_scratch = e->kv_bits ? base + opf : nullptr;
+        e->prefill_scratch_bytes = pf_bytes;
         e->d_positions = (int*)(base + opos);
         e->d_capacities = (int*)(base + ocap);
         e->d_row_base = (long long*)(base + orb);
@@ -1462,9 +1357,9 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
         if (e->shared_active) return TQ_ERR_UNSUPPORTED;
         int r = append_impl((uint8_t*)L.k, L.kn, (uint8_t*)L.v, L.vn, k, v, nullptr, e->d_rotation, e->d_positions, 0, e->rb(), 0, 0,
                             e->msl, e->G, H, Hkv, D, e->q_dim(), e->kv_dim(), e->kv_bits, e->workspace, e->ws_bytes, false, cs(s),
-                            false, e->d_rotation_prep, 0, e->caps());
+                            false, e->d_rotation_prep, e->caps());
         if (r != TQ_OK) return r;
-        return generic_packed_attention(out, q, L.k, L.v, L.kn, L.vn, e->d_rotation, e->d_positions, -1, e->rb(), e->msl, e->G, H,
+        return generic_attention(out, q, L.k, L.v, L.kn, L.vn, e->d_rotation, e->d_positions, -1, e->rb(), e->msl, e->G, H,
                                         Hkv, e->q_dim(), e->kv_bits, cs(s));
     }
     // One launch per layer when the batch fits the kernel's shared-memory tile table (tq_engine_set_fused).
@@ -1473,7 +1368,7 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
         FusedInputs in{q, k, v, e->d_rotation_rep, ROT_COPIES, early, e->caps()};
         const int r = attention_impl(out, L.tmK, L.tmV, L.k, L.v, L.kn, L.vn, e->d_rotation_t, e->d_positions, -1, e->rb(),
                                      e->total_rows, e->msl, e->G, H, Hkv, e->q_dim(), e->kv_bits, e->workspace, e->ws_bytes,
-                                     cs(s), use_pdl(), &in, 0, 0, f32, e->shared_active ? e->d_prefix_base : nullptr,
+                                     cs(s), use_pdl(), &in, f32, e->shared_active ? e->d_prefix_base : nullptr,
                                      e->shared_active ? e->d_prefix_tiles : nullptr);
         e->chain_ok = r == TQ_OK;
         e->chain_stream = cs(s);
@@ -1481,10 +1376,10 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     }
     int r = append_impl((uint8_t*)L.k, L.kn, (uint8_t*)L.v, L.vn, k, v, q, e->d_rotation, e->d_positions, 0,
                         e->rb(), 0, 0, e->msl, e->G, H, Hkv, D, e->q_dim(), e->kv_dim(), e->kv_bits, e->workspace,
-                        e->ws_bytes, true, cs(s), use_pdl(), e->d_rotation_prep, 0, e->caps());
+                        e->ws_bytes, true, cs(s), use_pdl(), e->d_rotation_prep, e->caps());
     if (r != TQ_OK) return r;
     return attention_impl(out, L.tmK, L.tmV, L.k, L.v, L.kn, L.vn, e->d_rotation_t, e->d_positions, -1, e->rb(), e->total_rows,
-                          e->msl, e->G, H, Hkv, e->q_dim(), e->kv_bits, e->workspace, e->ws_bytes, cs(s), use_pdl(), nullptr, 0, 0, f32,
+                          e->msl, e->G, H, Hkv, e->q_dim(), e->kv_bits, e->workspace, e->ws_bytes, cs(s), use_pdl(), nullptr, f32,
                           e->shared_active ? e->d_prefix_base : nullptr, e->shared_active ? e->d_prefix_tiles : nullptr);
 }
 
@@ -1501,7 +1396,7 @@ int tq_engine_attend_layer(tq_engine* e, int layer, void* out, tq_stream_t s) {
     if (r != TQ_OK) return r;
     return attention_impl(out, L.tmK, L.tmV, L.k, L.v, L.kn, L.vn, e->d_rotation_t, e->d_positions, -1, e->rb(), e->total_rows,
                           e->msl, e->G, e->shape.num_heads, e->shape.num_kv_heads, e->q_dim(), e->kv_bits, e->workspace,
-                          e->ws_bytes, cs(s), use_pdl(), nullptr, 0, 0, nullptr, e->shared_active ? e->d_prefix_base : nullptr,
+                          e->ws_bytes, cs(s), use_pdl(), nullptr, nullptr, e->shared_active ? e->d_prefix_base : nullptr,
                           e->shared_active ? e->d_prefix_tiles : nullptr);
 }
 
@@ -1867,7 +1762,7 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
     }
     const tq_engine::Layer& L = e->layers[layer];
     const size_t row_bytes = e->code_row_bytes();
-    if (!prefill_attn_shape(H, Hkv)) {   // layouts outside the tiled kernel: the compat launchers' generic path, prompt by prompt
+    if (!prefill_attn_shape(H, Hkv) || (((uintptr_t)q | (uintptr_t)out) & 15u) != 0) {  // what the tiled kernel does not take, prompt by prompt
         std::lock_guard<std::recursive_mutex> compat_lock(compat_mutex());
         for (int i = 0; i < n_seq && r == TQ_OK; ++i) {
             const long long row0 = e->row0_eff(first_seq + i);
@@ -1890,7 +1785,6 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
     ap.out = (__half*)out;
     ap.q_dim = q_stride;
     ap.T = T;
-    ap.rows = cap;
     ap.H = H;
     ap.Hkv = Hkv;
     ap.n_seq = n_seq;
@@ -1899,17 +1793,13 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
     const long long row0 = ap.row_base ? 0 : e->row0_eff(first_seq);   // dense slots: first_seq * max_seq_len
     ap.ck = (const uint8_t*)L.k + (size_t)row0 * row_bytes;
     ap.cv = (const uint8_t*)L.v + (size_t)row0 * row_bytes;
-    if (e->kv_bits == 0) {
-        ap.score_scale = 0.12751743074602467f;
-    } else {
+    if (e->kv_bits != 0) {
         ap.kn = (const __half*)L.kn + (size_t)row0 * Hkv;
         ap.vn = (const __half*)L.vn + (size_t)row0 * Hkv;
         ap.rotation = (const __half*)e->d_rotation;
-        ap.rotation_t = (const __half*)e->d_rotation_t;
-        ap.score_scale = 1.0f;
     }
     ap.status = (int*)e->workspace;
-    return launch_prefill_attention(e->kv_bits, ap, cs(s));
+    return launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s));
 }
 
 int tq_engine_prefill_layer(tq_engine* e, int layer, int seq, const void* q, const void* k, const void* v, void* out, int T,

@@ -24,8 +24,7 @@
 #include "tq_fp16_tc.cuh"
 #include "tq_qrot.cuh"
 #include "tq_generic.cuh"
-#include "tq_prefill_attn.cuh"
-#include "tq_prefill_attn_tc.cuh"
+#include "tq_prefill_fa.cuh"
 
 namespace tq {
 
@@ -142,12 +141,9 @@ inline int make_append_input_map(CUtensorMap* m, const void* base, long long tok
 }
 
 // ---- workspace ------------------------------------------------------------------------------------------------------
-// The carve of tq_common.cuh plus two helper arrays used by the prefill form (positions 0..T-1 and a
-// constant row base) and the fp16 twin's ticket/partial area, which aliases the packed path's partials.
+// The carve of tq_common.cuh plus the transposed rotation; the fp16 twin's ticket/partial area aliases the packed path's partials.
 struct FullWorkspace {
     Workspace w;
-    int* aux_pos;          // [G]
-    long long* aux_rows;   // [G]
     __half* rot_t;         // [128][128] transposed rotation (for callers that only hand over R)
     size_t bytes;
 };
@@ -157,10 +153,6 @@ inline FullWorkspace carve_full(void* base, int G, int H) {
     f.w = carve_workspace(base, G, H);
     size_t off = f.w.bytes;
     char* p = (char*)base;
-    f.aux_pos = (int*)(p + off);
-    off += align_up((size_t)G * sizeof(int), 256);
-    f.aux_rows = (long long*)(p + off);
-    off += align_up((size_t)G * sizeof(long long), 256);
     f.rot_t = (__half*)(p + off);
     off += (size_t)HEAD_DIM * HEAD_DIM * sizeof(__half);
     f.bytes = off;
@@ -441,52 +433,128 @@ inline int launch_fp16_tc_attention(const CUtensorMap& tmK, const CUtensorMap& t
     }
 }
 
-// Causal prefill attention with the query tokens in the M dimension (tq_prefill_attn.cuh); bits 0 = fp16 cache.
-inline bool prefill_attn_shape(int H, int Hkv) {
-    const int grp = Hkv > 0 ? H / Hkv : 0;
-    return Hkv > 0 && Hkv <= 65535 && H == grp * Hkv && (grp == 1 || grp == 2 || grp == 4 || grp == 8 || grp == 16);
+// What the causal prefill attention (tq_prefill_fa.cuh) serves: a slot holds at least one token's query heads.
+inline bool prefill_attn_shape(int H, int Hkv) { return Hkv > 0 && H % Hkv == 0 && H / Hkv <= PFT_ROWS; }
+// fp16 K or V array [rows][kv_dim] viewed as bytes for prefill_attention_fa_kernel: box = one head's 256 bytes (two 128-byte
+// blocks) x 128 rows, 128-byte swizzle.
+inline int make_prefill_rows_map(CUtensorMap* m, const void* base, long long rows, int kv_dim) {
+    auto fn = encode_fn();
+    if (!fn) return TQ_ERR_UNSUPPORTED;
+    const long long row_bytes = (long long)kv_dim * 2;
+    if (((uintptr_t)base & 15u) != 0 || rows <= 0 || rows >= (1ll << 31)) return TQ_ERR_ARG;
+    cuuint64_t dims[3] = {128u, (cuuint64_t)rows, (cuuint64_t)(row_bytes / 128)};
+    cuuint64_t strides[2] = {(cuuint64_t)row_bytes, 128u};
+    cuuint32_t box[3] = {128u, (cuuint32_t)PFT_KT, 2u};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? TQ_OK : TQ_ERR_ARG;
 }
-inline int launch_prefill_attention(int bits, PrefillAttnParams p, cudaStream_t s) {
-    const int grp = p.H / p.Hkv;
-    p.grp_shift = 0;
-    while ((1 << p.grp_shift) < grp) ++p.grp_shift;
-    const int qt = PFA_ROWS >> p.grp_shift;
+// Queries [tokens][q_stride] halves: box = one half (128 bytes) of the coordinates of `grp` heads of `qt` tokens, landing as
+// [token][head][128 B] with the 128-byte swizzle = the rows of a query operand tile.
+inline int make_prefill_query_map(CUtensorMap* m, const void* base, long long tokens, int H, int grp, int qt, long long q_stride) {
+    auto fn = encode_fn();
+    if (!fn) return TQ_ERR_UNSUPPORTED;
+    if (((uintptr_t)base & 15u) != 0 || q_stride % 8 != 0 || tokens <= 0 || tokens >= (1ll << 31)) return TQ_ERR_ARG;
+    cuuint64_t dims[4] = {128u, (cuuint64_t)H, (cuuint64_t)tokens, 2u};
+    cuuint64_t strides[3] = {256u, (cuuint64_t)q_stride * 2u, 128u};
+    cuuint32_t box[4] = {128u, (cuuint32_t)grp, (cuuint32_t)qt, 1u};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? TQ_OK : TQ_ERR_ARG;
+}
+template <bool PACKED, int MT>
+inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ, const CUtensorMap& tmR, const PrefillAttnParams& p,
+                               dim3 grid, cudaStream_t s) {
+    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT>, PftSmem::BYTES);
+    if (r != TQ_OK) return r;
+    // the register split inside the kernel draws on what the launch brings: never launch with less
+    static const int regs = [] {
+        cudaFuncAttributes a{};
+        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT>) == cudaSuccess ? a.numRegs : 0;
+    }();
+    if (regs < PFT_REGS_LAUNCH) return TQ_ERR_UNSUPPORTED;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(PFT_THREADS);
+    cfg.dynamicSmemBytes = PftSmem::BYTES;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT>, tmK, tmV, tmQ, tmR, p));
+}
+// Bytes of scratch a packed prompt of T tokens needs: fp16 centroids of K and V, fp32 norms.
+inline int prefill_t_pad(int T) { return (T + PFT_KT - 1) / PFT_KT * PFT_KT; }
+inline size_t prefill_scratch_bytes(int T, int Hkv) {
+    return 2 * align_up((size_t)T * Hkv * HEAD_DIM * sizeof(__half), 256) + align_up((size_t)2 * Hkv * prefill_t_pad(T) * sizeof(float), 256);
+}
+// Causal prefill attention.  `total_rows`: rows of the arrays ck and cv point into (from where they point); `scratch`: packed
+// modes, device memory for at least one prompt (prompts go through it in groups).
+inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long total_rows, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+    p.grp = p.H / p.Hkv;
     if (p.n_seq <= 0) p.n_seq = 1;
-    if ((long long)p.Hkv * p.n_seq > 2147483647ll || (p.T + qt - 1) / qt > 65535) return TQ_ERR_CAPACITY;
-    dim3 grid((unsigned)(p.Hkv * p.n_seq), (unsigned)((p.T + qt - 1) / qt));
     if (p.T <= 0) return TQ_OK;
-    int ar;
-    // tcgen05 form (default; TQ_PREFILL_ATTN_TC=0 selects the mma.sync form); the packed modes need R^T as well
-    static const bool tc = !(getenv("TQ_PREFILL_ATTN_TC") && atoi(getenv("TQ_PREFILL_ATTN_TC")) == 0);
-    if (tc && ((bits != 0 && p.rotation_t) || bits == 0)) {
-        if (bits == 4) {
-            if ((ar = ensure_dynamic_smem((const void*)prefill_attention_tc_kernel<4>, PTC_DYN_SMEM)) != TQ_OK) return ar;
-            prefill_attention_tc_kernel<4><<<grid, PTC_THREADS, PTC_DYN_SMEM, s>>>(p);
-        } else if (bits == 2) {
-            if ((ar = ensure_dynamic_smem((const void*)prefill_attention_tc_kernel<2>, PTC_DYN_SMEM)) != TQ_OK) return ar;
-            prefill_attention_tc_kernel<2><<<grid, PTC_THREADS, PTC_DYN_SMEM, s>>>(p);
+    const int qt = PFT_ROWS / p.grp, kv_dim = p.Hkv * HEAD_DIM;
+    int group = p.n_seq;  // prompts per launch (fp16 caches: all of them)
+    if (bits != 0) {
+        const size_t one = prefill_scratch_bytes(p.T, p.Hkv);
+        if (!scratch || scratch_bytes < one) return TQ_ERR_WORKSPACE;
+        group = (int)std::min<long long>(p.n_seq, (long long)(scratch_bytes / one));
+    }
+    for (int s0 = 0; s0 < p.n_seq; s0 += group) {
+        PrefillAttnParams a = p;
+        a.n_seq = std::min(group, p.n_seq - s0);
+        a.q = p.q + (size_t)s0 * p.T * p.q_tok_stride;
+        a.out = p.out + (size_t)s0 * p.T * p.q_dim;
+        CUtensorMap tmK{}, tmV{}, tmQ{}, tmR{};
+        int r = make_prefill_query_map(&tmQ, a.q, (long long)a.n_seq * p.T, p.H, p.grp, qt, p.q_tok_stride);
+        if (r != TQ_OK) return r;
+        if (bits == 0) {
+            r = make_prefill_rows_map(&tmK, p.ck, total_rows, kv_dim);
+            if (r == TQ_OK) r = make_prefill_rows_map(&tmV, p.cv, total_rows, kv_dim);
         } else {
-            if ((ar = ensure_dynamic_smem((const void*)prefill_attention_tc_kernel<0>, PTC_DYN_SMEM)) != TQ_OK) return ar;
-            prefill_attention_tc_kernel<0><<<grid, PTC_THREADS, PTC_DYN_SMEM, s>>>(p);
+            DequantParams d{};
+            d.ck = p.ck; d.cv = p.cv; d.kn = p.kn; d.vn = p.vn;
+            d.row_base = p.row_base ? p.row_base + s0 : nullptr;
+            d.seq_rows = p.seq_rows; d.T = p.T; d.t_pad = prefill_t_pad(p.T); d.Hkv = p.Hkv;
+            if (!p.row_base) {
+                const size_t skip = (size_t)s0 * p.seq_rows;
+                d.ck += skip * kv_dim / (bits == 4 ? 2 : 4); d.cv += skip * kv_dim / (bits == 4 ? 2 : 4);
+                d.kn += skip * p.Hkv; d.vn += skip * p.Hkv;
+            }
+            const size_t rows16 = align_up((size_t)a.n_seq * p.T * kv_dim * sizeof(__half), 256);
+            d.k16 = (__half*)scratch; d.v16 = (__half*)((char*)scratch + rows16); d.norms = (float*)((char*)scratch + 2 * rows16);
+            const long long pieces = 2ll * p.T * p.Hkv * 16;
+            const dim3 grid((unsigned)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count), (unsigned)a.n_seq);
+            r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4>, grid, dim3(256), 0, s, true, d)
+                          : launch_kernel(dequantize_rows_kernel<2>, grid, dim3(256), 0, s, true, d);
+            a.ck = (const uint8_t*)d.k16; a.cv = (const uint8_t*)d.v16; a.norms = d.norms; a.t_pad = d.t_pad;
+            a.row_base = nullptr;
+            a.seq_rows = p.T;
+            if (r == TQ_OK) r = make_prefill_rows_map(&tmR, p.rotation, HEAD_DIM, HEAD_DIM);
+            if (r == TQ_OK) r = make_prefill_rows_map(&tmK, d.k16, (long long)a.n_seq * p.T, kv_dim);
+            if (r == TQ_OK) r = make_prefill_rows_map(&tmV, d.v16, (long long)a.n_seq * p.T, kv_dim);
         }
-        return cuda_status(cudaGetLastError());
+        if (r != TQ_OK) return r;
+        // Two query blocks per CTA, which share every tile, once there are enough of them for the GPU; below that twice the CTAs
+        // with one block each, whose two slots take the even and the odd tiles.  Per layer, one block / two (8 KV heads, 4-bit):
+        // 2048 tokens 16 heads (128 pairs of blocks) 70 / 83 us, 32 heads (256) 117 / 104, 8192 tokens 16 heads (512) 449 / 439.
+        const long long blocks2 = (p.T + 2 * qt - 1) / (2 * qt), cols = (long long)p.Hkv * a.n_seq;
+        const int mt = 4 * blocks2 * cols >= 5ll * device_props().sm_count ? 2 : 1;
+        const long long blocks = mt == 2 ? blocks2 : (p.T + qt - 1) / qt;
+        if (cols > 2147483647ll || blocks > 65535) return TQ_ERR_CAPACITY;
+        dim3 grid((unsigned)cols, (unsigned)blocks);
+        if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
+        else r = mt == 2 ? launch_prefill_fa_t<false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
+        if (r != TQ_OK) return r;
     }
-    switch (bits) {
-        case 4:
-            if ((ar = ensure_dynamic_smem((const void*)prefill_attention_kernel<4>, PfaSmem::BYTES)) != TQ_OK) return ar;
-            prefill_attention_kernel<4><<<grid, PFA_THREADS, PfaSmem::BYTES, s>>>(p);
-            break;
-        case 2:
-            if ((ar = ensure_dynamic_smem((const void*)prefill_attention_kernel<2>, PfaSmem::BYTES)) != TQ_OK) return ar;
-            prefill_attention_kernel<2><<<grid, PFA_THREADS, PfaSmem::BYTES, s>>>(p);
-            break;
-        case 0:
-            if ((ar = ensure_dynamic_smem((const void*)prefill_attention_kernel<0>, PfaSmem::BYTES)) != TQ_OK) return ar;
-            prefill_attention_kernel<0><<<grid, PFA_THREADS, PfaSmem::BYTES, s>>>(p);
-            break;
-        default: return TQ_ERR_UNSUPPORTED;
-    }
-    return cuda_status(cudaGetLastError());
+    return TQ_OK;
 }
 
 inline int launch_fp16_attention(const Fp16AttnParams& p_in, cudaStream_t s) {
@@ -506,24 +574,6 @@ inline int launch_fp16_attention(const Fp16AttnParams& p_in, cudaStream_t s) {
         default: return TQ_ERR_UNSUPPORTED;
     }
     return cuda_status(cudaGetLastError());
-}
-
-__global__ void iota_rows_kernel(int* pos, long long* rows, int n, long long row0) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        pos[i] = i;
-        rows[i] = row0;
-    }
-}
-
-// positions and row bases of the prefill form's token groups: group j ends at token min((j + 1) * qg, T) - 1, row base 0
-__global__ void group_rows_kernel(int* pos, long long* rows, int groups, int qg, int T) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < groups) {
-        const int last = (j + 1) * qg;
-        pos[j] = (last < T ? last : T) - 1;
-        rows[j] = 0;
-    }
 }
 
 // ---- per-device workspace of the compat launchers + descriptor cache ----------------------------------------------------------
@@ -667,6 +717,8 @@ struct tq_engine {
     int* step_table = nullptr;         // [G + 4]
     void* step_qrot = nullptr;         // [layers][G][H][128] fp16: pre-rotated, pre-scaled queries
     void* step_kpost = nullptr;        // [layers][G][kv_dim] fp16: K after QK-norm and rotary embedding (producer form)
+    void* prefill_scratch = nullptr;   // packed modes: fp16 rows and fp32 norms of prompts (launch_prefill_attention)
+    size_t prefill_scratch_bytes = 0;
     bool whole_step = !(getenv("TQ_WHOLE_STEP") && atoi(getenv("TQ_WHOLE_STEP")) == 0);
     float* out_f32 = nullptr;          // optional [layers][G][H][128]: results before the fp16 rounding (outside the arena)
     cudaEvent_t ev_attn[2] = {nullptr, nullptr};  // optional: recorded around the attention launch of the whole-step form
