@@ -209,46 +209,48 @@ __device__ __forceinline__ float ldsp_h2f(uint32_t addr) {  // one fp16 from sha
 template <int NW, typename OutRow, typename OutRowF32>
 __device__ __forceinline__ void merge_sequence(const float* part0, int parts, int H, uint32_t merge_s, const __half* rotation_t,
                                                int head, int lane, int bar_group, int nthreads, OutRow out_row,
-                                               OutRowF32 out_row_f32, bool rotated_out = false) {
+                                               OutRowF32 out_row_f32, int hb_begin, int hb_end, bool rotated_out = false) {
     const int gl = lane >> 2, t4 = lane & 3;
-    for (int hb = 0; hb < H; hb += 16) {
+    constexpr int RH = NW >= 16 ? 1 : 2, FLIGHT = 16 / RH;  // heads per warp at a time, parts whose loads are in flight together
+    for (int hb = hb_begin; hb < hb_end; hb += 16) {
         // ---- phase A: heads hb .. hb+15, two heads per warp at a time with all their loads in flight
         //      together: combine the parts, normalise, split into fp16 high + low, store as the A operand
         //      [16][MERGE_ROW]
-        for (int hh0 = head; hh0 < 16; hh0 += 2 * NW) {
-            float4 a[2];
-            a[0] = a[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-            const size_t pstride = (size_t)H * PART_STRIDE;
-            if (parts <= 8) {
-                // common case: one round trip for everything, weights afterwards
-                float4 v[2][8];
-                float2 ml[2];
+        for (int hh0 = head; hh0 < 16; hh0 += RH * NW) {
+            float4 a[RH];
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
+            for (int r = 0; r < RH; ++r) a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const size_t pstride = (size_t)H * PART_STRIDE;
+            if (parts <= FLIGHT) {
+                // common case: one round trip for everything, weights afterwards
+                float4 v[RH][FLIGHT];
+                float2 ml[RH];
+#pragma unroll
+                for (int r = 0; r < RH; ++r) {
                     const int hq = hb + hh0 + r * NW;
                     const float* base = part0 + (size_t)hq * PART_STRIDE;
                     const bool on = hq < H && hh0 + r * NW < 16;
                     ml[r] = make_float2(-1e30f, 0.0f);
                     if (on && lane < parts) ml[r] = __ldcg(reinterpret_cast<const float2*>(base + lane * pstride + HEAD_DIM));
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
+                    for (int j = 0; j < FLIGHT; ++j)
                         v[r][j] = (on && j < parts) ? __ldcg(reinterpret_cast<const float4*>(base + j * pstride) + lane)
                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
+                for (int r = 0; r < RH; ++r) {
                     float M = ml[r].x;
 #pragma unroll
-                    for (int o = 4; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+                    for (int o = FLIGHT / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
                     M = __shfl_sync(0xffffffffu, M, 0);
                     const float e = lane < parts ? ex2_approx(ml[r].x - M) : 0.0f;
                     float Z = ml[r].y * e;
 #pragma unroll
-                    for (int o = 4; o > 0; o >>= 1) Z += __shfl_xor_sync(0xffffffffu, Z, o);
+                    for (int o = FLIGHT / 2; o > 0; o >>= 1) Z += __shfl_xor_sync(0xffffffffu, Z, o);
                     Z = __shfl_sync(0xffffffffu, Z, 0);
                     const float sc = e / (Z + 1e-8f);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < FLIGHT; ++j) {
                         const float wj = __shfl_sync(0xffffffffu, sc, j);
                         a[r].x = fmaf(wj, v[r][j].x, a[r].x); a[r].y = fmaf(wj, v[r][j].y, a[r].y);
                         a[r].z = fmaf(wj, v[r][j].z, a[r].z); a[r].w = fmaf(wj, v[r][j].w, a[r].w);
@@ -257,7 +259,7 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
             } else {
                 // many parts: one round trip for all (max, sum) pairs, then the vectors 16 at a time
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
+                for (int r = 0; r < RH; ++r) {
                     const int hq = hb + hh0 + r * NW;
                     if (hq >= H || hh0 + r * NW >= 16) continue;
                     const float* base = part0 + (size_t)hq * PART_STRIDE;
@@ -301,7 +303,7 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
             if (rotated_out) {
                 // the consumer's weights carry R^T (tq_fold_rotation_into_projection): the normalised sums leave as they are
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
+                for (int r = 0; r < RH; ++r) {
                     const int hh = hh0 + r * NW;
                     if (hh >= 16) continue;
                     if (__half* o = out_row(hb + hh)) {
@@ -313,7 +315,7 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
                 continue;
             }
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
+            for (int r = 0; r < RH; ++r) {
                 const int hh = hh0 + r * NW;
                 if (hh >= 16) continue;
                 __half2 h01 = __floats2half2_rn(a[r].x, a[r].y), h23 = __floats2half2_rn(a[r].z, a[r].w);
@@ -329,10 +331,10 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
         // ---- phase B: out[h][d] = sum_k a[h][k] * R[k][d]  ==  A(16 x 128) * B with B[k][n=d] = rotation_t[d][k].
         //      Two column blocks of 8 per warp and pass; their B fragments are fetched before the barrier so that
         //      the round trip overlaps the other warps' phase A.
-        for (int nb0 = head; nb0 < 16; nb0 += 2 * NW) {
-            uint32_t bfrag[2][8][2];
+        for (int nb0 = head; nb0 < 16; nb0 += RH * NW) {
+            uint32_t bfrag[RH][8][2];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < RH; ++i) {
                 const int nb = nb0 + i * NW;
                 const __half* rt = rotation_t + (size_t)(8 * (nb < 16 ? nb : 0) + gl) * HEAD_DIM + 2 * t4;
 #pragma unroll
@@ -343,7 +345,7 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
             }
             if (nb0 == head) group_barrier(bar_group, nthreads);  // phase A of every warp is in shared memory
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < RH; ++i) {
                 const int nb = nb0 + i * NW;
                 if (nb >= 16) continue;
                 float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -370,7 +372,8 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
 }
 
 // MODE 0: queries pre-rotated and tile table built by append_rotate_kernel; 1: the kernel builds its table, rotates the
-// queries, optionally appends the step's token (one launch per layer and step); 2: whole-step form, see AttnParams.
+// queries, optionally appends the step's token (one launch per layer and step); 2: whole-step form, see AttnParams; 3: as 1,
+// but the partials are only published (merge_partials_kernel<16> follows).
 template <int BITS, int HKV, int MODE>
 __global__ void __launch_bounds__(ATTN_GROUPS * 32 * HKV, 1)
 decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -378,6 +381,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     using Geo = AttnGeom<BITS>;
     constexpr bool FUSED = MODE >= 1;
     constexpr bool PERSIST = MODE == 2;
+    constexpr bool SEPARATE = MODE == 3;
     extern __shared__ __align__(1024) uint8_t dyn_smem[];
 
     const int tid = threadIdx.x;
@@ -500,7 +504,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         }
         if (tid == 0) ts_s[G] = carry;
         ts = ts_s;
-        if constexpr (PERSIST) {
+        if constexpr (PERSIST) {  // (never early)
             if (blockIdx.x == 0) {  // the merge kernel reads the table from global memory
                 __syncthreads();
                 for (int i = tid; i <= G; i += (int)blockDim.x) p.table_out[i] = ts_s[i];
@@ -685,6 +689,15 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             pdl_launch_dependents();
         } else if (fill_before) {
             fill_ring();
+        }
+        if constexpr (SEPARATE) {  // the table for the merge kernel (behind the wait: the previous layer's merge has read its own)
+            if (wid == 0) {  // (worker 0 always takes part)
+                for (int i = gtid; i <= G; i += gthreads) p.table_out[i] = ts[i];
+                if (gtid == 0) {
+                    p.table_out[G + 1] = W;
+                    p.table_out[G + 2] = (int)N;
+                }
+            }
         }
         if (have_app) {
             constexpr float APPEND_MARGIN = 1.6e-5f;  // twice the worst-case rounding of a 128-term fp32 sum with sum|r x| <= 1
@@ -981,22 +994,13 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         // query fragments (B operand of the score product): lane (gl, t4) holds coordinates 32*t4 .. 32*t4+31 of head
         // head*grp + gl as fp16
         uint32_t qb[8][2];
-        if constexpr (PERSIST) {
-            uint32_t ok = (dead || !loads_on) ? 1u : 0u;
-            for (uint32_t it = 0; it < (1u << 14) && !ok; ++it) ok = mbar_try_wait_hint(qbar, q_par, 20000u);
-            if (!ok) {
-                dead = true;
-                if (lane == 0) atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
-            }
-            dead = __any_sync(0xffffffffu, dead);
-            q_par ^= 1u;
-            TQ_STAMP(9);   // wait for the query block
-            // lane (gl, t4): the 32 coordinates 32*t4 .. of head head*grp + gl, 64 bytes
+        // lane (gl, t4): the 32 coordinates 32*t4 .. of head head*grp + gl from the merge area, rows `pitch` bytes apart
+        auto take_fragments = [&](uint32_t pitch) {
             uint4 qw[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 qw[i] = make_uint4(0u, 0u, 0u, 0u);
-                if (gl < grp && !dead) qw[i] = ldsv128(merge_s + (uint32_t)((head * grp + gl) * HEAD_DIM + 32 * t4 + 8 * i) * 2u);
+                if (gl < grp && !dead) qw[i] = ldsv128(merge_s + (uint32_t)(head * grp + gl) * pitch + (uint32_t)(32 * t4 + 8 * i) * 2u);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -1010,6 +1014,18 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                     qb[2 * i + h2][1] = BITS == 2 ? prmt(a, b, 0x7632u) : b;
                 }
             }
+        };
+        if constexpr (PERSIST) {
+            uint32_t ok = (dead || !loads_on) ? 1u : 0u;
+            for (uint32_t it = 0; it < (1u << 14) && !ok; ++it) ok = mbar_try_wait_hint(qbar, q_par, 20000u);
+            if (!ok) {
+                dead = true;
+                if (lane == 0) atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
+            }
+            dead = __any_sync(0xffffffffu, dead);
+            q_par ^= 1u;
+            TQ_STAMP(9);   // wait for the query block
+            take_fragments((uint32_t)HEAD_DIM * 2u);
             TQ_STAMP(10);  // fragments
             group_barrier(group, gthreads);  // every warp holds its fragments: the area may take the next block
             TQ_STAMP(11);  // barrier of the worker's warps
@@ -1018,6 +1034,63 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 if (seg_end < hi) issue_queries(layer, g + 1);
                 else if (layer + 1 < n_layers) issue_queries(layer + 1, g_lo);
             }
+        } else if constexpr (SEPARATE) {
+            // Rotate this sequence's queries here: rot[h][d] = sum_k q[h][k] * R[d][k] on the tensor cores, all heads in one
+            // round through the merge area: fp16 in ([H][MERGE_ROW], padded), fp16 out, scaled by log2(e) / sqrt(128).  The
+            // loads of R and of the queries are in flight together.  (In rounds of 16 heads, with fp32 results, this took 5.5 us
+            // of a layer's 84 at 32 heads.)  B fragments straight from R, 16 contiguous bytes per lane and load; the contraction
+            // index is permuted the same way on both sides: step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3.
+            uint4 bq[16 / Hkv][4];
+#pragma unroll
+            for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
+                const int nb = head + nbi * Hkv;
+                const uint4* rr = reinterpret_cast<const uint4*>(p.rotation + (size_t)(wid % p.rot_copies) * (HEAD_DIM * HEAD_DIM) +
+                                                                 (size_t)(8 * nb + gl) * HEAD_DIM) + t4;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) bq[nbi][m] = __ldg(rr + 4 * m);
+            }
+            if (tile != lo) group_barrier(group, gthreads);  // every warp has taken the previous sequence's fragments
+            const uint4* const q_src = reinterpret_cast<const uint4*>(p.new_q + (size_t)g * p.q_dim);
+            for (int i = gtid; i < p.H * 16; i += gthreads) {
+                const uint4 u = __ldg(q_src + i);
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(merge_s + (uint32_t)((i >> 4) * MERGE_ROW) * 2u + (uint32_t)(i & 15) * 16u),
+                             "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w) : "memory");
+            }
+            group_barrier(group, gthreads);
+            float rc[2][16 / Hkv][4];
+#pragma unroll
+            for (int hb = 0; hb < 2; ++hb) {
+                if (16 * hb >= p.H) break;
+                // (rows at or past H hold whatever the area held: their results are not stored)
+#pragma unroll
+                for (int nbi = 0; nbi < 16 / Hkv; ++nbi) rc[hb][nbi][0] = rc[hb][nbi][1] = rc[hb][nbi][2] = rc[hb][nbi][3] = 0.0f;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const uint32_t at = merge_s + (uint32_t)((16 * hb + gl) * MERGE_ROW + 32 * m + 8 * t4) * 2u;
+                    const uint4 a_lo = ldsv128(at), a_hi = ldsv128(at + 8u * MERGE_ROW * 2u);
+#pragma unroll
+                    for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
+                        mma16816(rc[hb][nbi], a_lo.x, a_hi.x, a_lo.y, a_hi.y, bq[nbi][m].x, bq[nbi][m].y);
+                        mma16816(rc[hb][nbi], a_lo.z, a_hi.z, a_lo.w, a_hi.w, bq[nbi][m].z, bq[nbi][m].w);
+                    }
+                }
+            }
+            group_barrier(group, gthreads);
+#pragma unroll
+            for (int hb = 0; hb < 2; ++hb) {
+                if (16 * hb >= p.H) break;
+                const float sc = 0.12751743074602467f;
+#pragma unroll
+                for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
+                    const uint32_t at = merge_s + (uint32_t)((16 * hb + gl) * MERGE_ROW + 8 * (head + nbi * Hkv) + 2 * t4) * 2u;
+                    if (16 * hb + gl < p.H)
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(pack_half2(rc[hb][nbi][0] * sc, rc[hb][nbi][1] * sc)) : "memory");
+                    if (16 * hb + gl + 8 < p.H)
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + 8u * MERGE_ROW * 2u), "r"(pack_half2(rc[hb][nbi][2] * sc, rc[hb][nbi][3] * sc)) : "memory");
+                }
+            }
+            group_barrier(group, gthreads);
+            take_fragments((uint32_t)MERGE_ROW * 2u);
         } else {
             float qv[32];
             if constexpr (FUSED) {
@@ -1397,7 +1470,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             }
         }
         if (TQ_DBG(4)) { ++g; continue; }
-        if constexpr (PERSIST) {  // the partials of all layers are merged by merge_partials_kernel
+        if constexpr (PERSIST || SEPARATE) {  // the partials are merged by merge_partials_kernel
             ++g;
             continue;
         }
@@ -1434,7 +1507,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 return p.out_f32 + ((size_t)g * H + (size_t)vh) * HEAD_DIM;
             };
             merge_sequence<Hkv>(p.partials + (size_t)(first_w + g) * H * PART_STRIDE, parts, H, merge_s, p.rotation_t, head, lane,
-                                group, gthreads, out_row, out_row_f32);
+                                group, gthreads, out_row, out_row_f32, 0, H);
         }
         ++g;
     }
@@ -1457,7 +1530,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     }
 }
 
-// ---- whole-step form: merge of the published partials --------------------------------------------------------------
+// ---- merge of the partials that modes 2 and 3 publish -----------------------------------------------------------------
 struct MergeParams {
     const float* partials;       // [layers][workers + G][H][PART_STRIDE]
     const int* table;            // tile table [G + 1], then {workers that took part, total tiles}
@@ -1467,23 +1540,27 @@ struct MergeParams {
     long long part_layer_stride; // floats
     long long q_layer_stride;    // halves
     int G, H, q_dim;
+    int app_weight;              // as in AttnParams: what a sequence weighs beside its tiles in the cut of the work list
     int rotated_out;             // 1: leave the results in rotated space (the consumer's weights carry R^T)
 };
-constexpr int MERGE_WARPS = 8;
 
-// One CTA per (sequence, layer): the merge that decode_attention_kernel's last-arriving worker does in the one-launch
-// forms, here as a launch of its own after the whole-step kernel, spread over the whole GPU.
-__global__ void __launch_bounds__(MERGE_WARPS * 32) merge_partials_kernel(const MergeParams p) {
+// The merge that mode 1's last-arriving worker does, as a launch of its own spread over the whole GPU.  One CTA per (sequence,
+// layer): WARPS = 8, two heads per warp, for the many short merges of a whole step; WARPS = 16, a CTA per 16 heads too, a head
+// per warp with up to 16 parts' loads in flight, where one layer's merge is the tail of a layer.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) merge_partials_kernel(const MergeParams p) {
     __shared__ __align__(16) uint8_t merge_buf[RegionA::MERGE_GROUP_BYTES];
+    if (WARPS == 16) pdl_launch_dependents();
     pdl_wait();  // the partials and the table come from the previous kernel in the stream
-    const int g = blockIdx.x, layer = blockIdx.y;
+    const int g = blockIdx.x, layer = blockIdx.y, hb = 16 * (int)blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long ts_g = p.table[g], ts_g1 = p.table[g + 1];
-    const long long W = p.table[p.G + 1], N = p.table[p.G + 2];
-    if (N <= 0 || W <= 0) return;
-    // owners of the sequence's first and last tile: worker w holds the tiles [w * N / W, (w + 1) * N / W)
-    const int first_w = (int)(((ts_g + 1) * W - 1) / N);
-    const int last_w = (int)((ts_g1 * W - 1) / N);
+    const long long A = p.app_weight;
+    const long long u0 = p.table[g] + g * A, u1 = p.table[g + 1] + g * A;  // the units its first tile starts and its last one ends at
+    const long long W = p.table[p.G + 1], U = p.table[p.G + 2] + p.G * A;
+    if (U <= 0 || W <= 0) return;
+    // owners of the sequence's first and last tile: worker w holds the units [w * U / W, (w + 1) * U / W)
+    const int first_w = (int)(((u0 + 1) * W - 1) / U);
+    const int last_w = (int)((u1 * W - 1) / U);
     const int parts = last_w - first_w + 1;
     const int H = p.H;
     auto out_row = [&](int vh) -> __half* {
@@ -1494,9 +1571,9 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_partials_kernel(const 
         if (!p.out_f32 || vh >= H) return nullptr;
         return p.out_f32 + (((size_t)layer * p.G + (size_t)g) * H + (size_t)vh) * HEAD_DIM;
     };
-    merge_sequence<MERGE_WARPS>(p.partials + (size_t)layer * (size_t)p.part_layer_stride + (size_t)(first_w + g) * H * PART_STRIDE,
-                                parts, H, smem_u32(merge_buf), p.rotation_t, warp, lane, 0, MERGE_WARPS * 32, out_row, out_row_f32,
-                                p.rotated_out != 0);
+    merge_sequence<WARPS>(p.partials + (size_t)layer * (size_t)p.part_layer_stride + (size_t)(first_w + g) * H * PART_STRIDE,
+                          parts, H, smem_u32(merge_buf), p.rotation_t, warp, lane, 0, WARPS * 32, out_row, out_row_f32,
+                          WARPS == 16 ? hb : 0, WARPS == 16 ? min(hb + 16, H) : H, p.rotated_out != 0);
 }
 
 }  // namespace tq

@@ -338,7 +338,20 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
         p.kv_dim = num_kv_heads * HEAD_DIM; p.capacity_rows = max_seq_len;
         p.seq_capacity = fused->seq_capacity;
     }
-    return launch_attention(bits, tmK, tmV, p, attention_ctas(G, max_seq_len), s, pdl, fused != nullptr ? 1 : 0);
+    const int ctas = attention_ctas(G, max_seq_len);
+    if (!fused) return launch_attention(bits, tmK, tmV, p, ctas, s, pdl, 0);
+    // The merge inside the kernel (by the last worker to arrive at a sequence, under the others' last tiles and the next layer's
+    // start) or as a launch of its own: with more than 16 heads (two rounds) or few sequences, cut into many parts, that
+    // worker is a layer's tail of ten microseconds and more.  Measured per layer, in the kernel / as a launch: 4-bit 16 heads
+    // 64 x 4096 80 / 84 us, 32 heads 88 / 87, 16 x 4096 43 / 34, 4 x 16384 61 / 42; 16 heads 1 x 16384 38 / 30.
+    const bool separate = num_heads > 16 || ctas * ATTN_GROUPS > 16 * G;
+    p.table_out = fw.w.tile_start;
+    const int r = launch_attention(bits, tmK, tmV, p, ctas, s, pdl, separate ? 3 : 1);
+    if (r != TQ_OK || !separate) return r;
+    MergeParams m{};
+    m.partials = p.partials; m.table = p.table_out; m.rotation_t = p.rotation_t; m.out = p.out; m.out_f32 = out_f32;
+    m.G = G; m.H = num_heads; m.q_dim = q_dim; m.app_weight = p.app_weight;
+    return launch_kernel(merge_partials_kernel<16>, dim3((unsigned)G, 1u, (unsigned)((num_heads + 15) / 16)), dim3(512), 0, s, use_pdl(), m);
 }
 
 int tq_decode_attention(void* out, const uint8_t* ck_q, const uint8_t* cv_q, const void* k_norms, const void* v_norms,
@@ -560,8 +573,8 @@ static int compat_cluster_attention(void* out, const void* q, const void* ck, co
     p.ck = (const uint8_t*)ck; p.cv = (const uint8_t*)cv; p.kn = (const __half*)k_norms; p.vn = (const __half*)v_norms;
     p.q = (const __half*)q; p.rotation = (const __half*)rotation; p.out = (__half*)out;
     p.positions = pos; p.pos_value = pos_value; p.max_seq_len = msl; p.capacity_rows = msl;
-    p.H = H; p.Hkv = Hkv; p.q_dim = q_dim; p.head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
-    return launch_cluster_decode(bits, p, G, pos ? msl : pos_value + 1, s, use_pdl());
+    p.G = G; p.H = H; p.Hkv = Hkv; p.q_dim = q_dim; p.head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
+    return launch_cluster_decode(bits, p, 1, 1, pos ? msl : pos_value + 1, s, use_pdl());
 }
 
 void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* ck_q, const uint8_t* cv_q,
@@ -1034,6 +1047,10 @@ int tq_engine_alloc_batch(tq_engine* e, int G, int max_seq_len, const int* capac
         int ur = engine_upload_rotation(e, nullptr);
         if (ur != TQ_OK) return ur;
     }
+    // every layer is carved alike, so consecutive layers' arrays lie a constant distance apart
+    const int NL = e->shape.num_layers;
+    e->code_layer_stride = NL > 1 ? (size_t)((char*)e->layers[1].k - (char*)e->layers[0].k) : (size_t)rows * e->code_row_bytes();
+    e->norm_layer_stride = e->kv_bits == 0 ? 0 : (NL > 1 ? (size_t)((char*)e->layers[1].kn - (char*)e->layers[0].kn) : (size_t)rows * e->shape.num_kv_heads * 2);
     if (e->kv_bits != 0 && fast_shape(e->shape.num_heads, e->shape.num_kv_heads, true)) {
         // (other head layouts take the generic kernel, which reads the cache with plain loads: no descriptors)
         const int kvp = e->kv_dim() / e->vpb();
@@ -1043,10 +1060,6 @@ int tq_engine_alloc_batch(tq_engine* e, int G, int max_seq_len, const int* capac
             r = make_code_map(&L.tmV, L.v, rows, kvp);
             if (r != TQ_OK) return r;
         }
-        // every layer is carved alike, so consecutive layers' arrays lie a constant distance apart
-        const int NL = e->shape.num_layers;
-        e->code_layer_stride = NL > 1 ? (size_t)((char*)e->layers[1].k - (char*)e->layers[0].k) : (size_t)rows * kvp;
-        e->norm_layer_stride = NL > 1 ? (size_t)((char*)e->layers[1].kn - (char*)e->layers[0].kn) : (size_t)rows * e->shape.num_kv_heads * 2;
         r = make_code_map_layers(&e->tmK4, e->layers[0].k, rows, kvp, NL, e->code_layer_stride);
         if (r != TQ_OK) return r;
         r = make_code_map_layers(&e->tmV4, e->layers[0].v, rows, kvp, NL, e->code_layer_stride);
@@ -1314,6 +1327,38 @@ static bool engine_reads_early(const tq_engine* e, bool chained, cudaStream_t s)
     return cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
+static bool engine_cluster_ok(const tq_engine* e, const void* q, const void* k, const void* v, const void* out) {
+    return e->fused && (((uintptr_t)k | (uintptr_t)v) & 15u) == 0 &&
+           cluster_shape(q, out, e->layers[0].k, e->layers[0].v, e->d_rotation, e->G, e->shape.num_heads, e->shape.num_kv_heads, e->q_dim());
+}
+
+// The layers l0 .. l0 + n - 1 of a step in one launch of the cluster form; q, k, v, out point at layer l0's [G][dim] blocks.
+static int engine_cluster_layers(tq_engine* e, int l0, int n, int split_layers, const void* q, const void* k, const void* v, void* out, bool chained,
+                                 cudaStream_t s) {
+    const tq_engine::Layer& L = e->layers[l0];
+    const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
+    ClusterDecodeParams p{};
+    p.ck = (const uint8_t*)L.k; p.cv = (const uint8_t*)L.v; p.kn = (const __half*)L.kn; p.vn = (const __half*)L.vn;
+    p.q = (const __half*)q; p.new_k = (const __half*)k; p.new_v = (const __half*)v;
+    p.rotation = (const __half*)e->d_rotation; p.out = (__half*)out;
+    p.out_f32 = e->out_f32 ? e->out_f32 + (size_t)l0 * e->G * H * HEAD_DIM : nullptr;
+    p.positions = e->d_positions; p.row_base = e->rb(); p.seq_capacity = e->caps();
+    if (e->shared_active) { p.prefix_base = e->d_prefix_base; p.prefix_tiles = e->d_prefix_tiles; }
+    p.status = (int*)e->workspace;
+    p.max_seq_len = e->msl; p.capacity_rows = e->msl;
+    p.G = e->G; p.H = H; p.Hkv = Hkv; p.q_dim = e->q_dim(); p.head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
+    p.code_layer_stride = (long long)e->code_layer_stride; p.norm_layer_stride = (long long)(e->norm_layer_stride / 2);
+    p.q_layer_stride = (long long)e->G * e->q_dim(); p.kv_layer_stride = (long long)e->G * e->kv_dim();
+    p.early = engine_reads_early(e, chained, s) ? 1 : 0;
+    p.static_rotation = 1;
+    if (split_layers > 1 && e->ev_attn[0]) cudaEventRecord(e->ev_attn[0], s);
+    const int r = launch_cluster_decode(e->kv_bits, p, n, split_layers, e->msl, s, use_pdl() && !(split_layers > 1 && e->ev_attn[0]));
+    if (split_layers > 1 && e->ev_attn[0]) cudaEventRecord(e->ev_attn[1], s);
+    e->chain_ok = r == TQ_OK;
+    e->chain_stream = s;
+    return r;
+}
+
 int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k, const void* v, void* out,
                            tq_stream_t s) {
     if (!e || layer < 0 || layer >= e->shape.num_layers || !q || !k || !v || !out) return TQ_ERR_ARG;
@@ -1324,25 +1369,9 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, D = e->shape.head_dim;
     float* const f32 = e->out_f32 ? e->out_f32 + (size_t)layer * e->G * H * HEAD_DIM : nullptr;
     // Head layouts outside the streaming kernels', and small batches of any layout: the cluster form, one launch.
-    const bool streaming = fast_shape(H, Hkv, e->kv_bits != 0);
-    if (e->fused && cluster_shape(q, out, L.k, L.v, e->d_rotation, e->G, H, Hkv, e->q_dim()) &&
-        (((uintptr_t)k | (uintptr_t)v) & 15u) == 0 && (!streaming || cluster_size(e->kv_bits, e->total_rows, Hkv))) {
-        ClusterDecodeParams p{};
-        p.ck = (const uint8_t*)L.k; p.cv = (const uint8_t*)L.v; p.kn = (const __half*)L.kn; p.vn = (const __half*)L.vn;
-        p.q = (const __half*)q; p.new_k = (const __half*)k; p.new_v = (const __half*)v;
-        p.rotation = (const __half*)e->d_rotation; p.out = (__half*)out; p.out_f32 = f32;
-        p.positions = e->d_positions; p.row_base = e->rb(); p.seq_capacity = e->caps();
-        if (e->shared_active) { p.prefix_base = e->d_prefix_base; p.prefix_tiles = e->d_prefix_tiles; }
-        p.status = (int*)e->workspace;
-        p.max_seq_len = e->msl; p.capacity_rows = e->msl;
-        p.H = H; p.Hkv = Hkv; p.q_dim = e->q_dim(); p.head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
-        p.early = engine_reads_early(e, chained, cs(s)) ? 1 : 0;
-        p.static_rotation = 1;
-        const int r = launch_cluster_decode(e->kv_bits, p, e->G, e->msl, cs(s), use_pdl());
-        e->chain_ok = r == TQ_OK;
-        e->chain_stream = cs(s);
-        return r;
-    }
+    if (engine_cluster_ok(e, q, k, v, out) &&
+        (!fast_shape(H, Hkv, e->kv_bits != 0) || cluster_size(e->kv_bits, e->total_rows, Hkv)))
+        return engine_cluster_layers(e, layer, 1, 1, q, k, v, out, chained, cs(s));
     if (e->kv_bits == 0) {
         fp16_cache_write_kernel<<<e->G, 128, 0, cs(s)>>>((__half*)L.k, (__half*)L.v, (const __half*)k, (const __half*)v,
                                                          e->d_positions, e->rb(), e->msl, e->msl, e->G,
@@ -1425,9 +1454,42 @@ static bool engine_whole_step_ok(const tq_engine* e, const void* q, const void* 
 
 static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* out, cudaStream_t s, const tq_step_producer* prod);
 
+// Is a whole step of this engine's batch faster as one launch of the cluster form over all layers than in the whole-step form's
+// four launches?  Both times fit a line, in ns: a cluster (sequence, KV head, 8 query heads, layer) costs 24.5 and a cached row
+// and KV head 0.0346 in the one, a layer 3600, a sequence 1000 and a cached row and KV head 0.030 in the other, whose launches,
+// table and merges take 35 us at least (28 layers of 1 x 256 tokens 9 / 137 us, 4 x 4096 186 / 311, 16 x 1024 222 / 240, 16 x
+// 4096 647 / 595, 64 x 64 352 / 195).  fp16 caches have no whole-step form; up to 4 M rows and KV heads the one launch beats one
+// per layer (28 layers of 16 x 1024 338 / 596 us), above that the chunks of the streaming kernel balance better.
+// It depends on the engine's batch alone: every call that runs a step, or part of one, takes the same form and gives the same bits.
+static bool engine_step_small(const tq_engine* e) {
+    if (!e->fused || !e->whole_step || e->G > 65535) return false;
+    const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, NL = e->shape.num_layers;
+    if (!fast_shape(H, Hkv, e->kv_bits != 0)) return true;
+    static const bool on = !(getenv("TQ_CLUSTER") && atoi(getenv("TQ_CLUSTER")) == 0);
+    const double rows = (double)e->total_rows * Hkv * NL;
+    if (e->kv_bits == 0) return on && rows <= 4e6;
+    const double clusters = (double)e->G * Hkv * NL * ((H / Hkv + CD_HEADS - 1) / CD_HEADS);
+    return on && 24.5 * clusters + 0.0046 * rows < 35000.0 + 3600.0 * NL + 1000.0 * e->G;
+}
+
+// The layers l0 .. l0 + n - 1 of such a step; q, k, v, out point at layer l0's [G][dim] blocks.
+static int engine_cluster_step(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s) {
+    const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
+    const int chunk = std::min(n, 65535 / e->G);  // layers per launch: the grid's third dimension
+    for (int i = 0; i < n; i += chunk) {
+        const bool chained = e->chain_ok;
+        e->chain_ok = false;
+        int r = engine_cluster_layers(e, l0 + i, std::min(chunk, n - i), e->shape.num_layers, (const char*)q + qb * i, (const char*)k + kb * i,
+                                      (const char*)v + kb * i, (char*)out + qb * i, chained, s);
+        if (r != TQ_OK) return r;
+    }
+    return TQ_OK;
+}
+
 // launches 1 and 1b of the whole-step form for the layers [l0, l0 + n): the append and the query rotation
+// (raw_q, producer form: the produced queries are stored as they are, not rotated)
 static int engine_step_prepare(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, cudaStream_t s,
-                               const tq_step_producer* prod) {
+                               const tq_step_producer* prod, bool raw_q = false) {
     e->chain_ok = false;
     const tq_engine::Layer& L = e->layers[l0];
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, G = e->G;
@@ -1458,6 +1520,7 @@ static int engine_step_prepare(tq_engine* e, int l0, int n, const void* q, const
         if (prod) {
             qr.norm_w = (const __half*)prod->q_norm_weight + (size_t)l0 * HEAD_DIM;
             qr.rope_cos = (const __half*)prod->rope_cos; qr.rope_sin = (const __half*)prod->rope_sin;
+            qr.raw = raw_q ? 1 : 0;
             qr.positions = e->d_positions; qr.G = G; qr.rope_dim = prod->rope_dim; qr.eps = prod->eps; qr.biased = prod->biased;
             rotate_queries_kernel<true><<<(unsigned)blocks, QROT_WARPS * 32, 0, s>>>(qr);
         } else {
@@ -1471,6 +1534,12 @@ static int engine_step_prepare(tq_engine* e, int l0, int n, const void* q, const
 
 static int engine_step_layers(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s,
                               const tq_step_producer* prod = nullptr) {
+    // A small step: the produced queries and keys, then the cluster form.  (It stores the new token's bytes once more, the same.)
+    const size_t qo = (size_t)l0 * e->G * e->q_dim() * 2, ko = (size_t)l0 * e->G * e->kv_dim() * 2;
+    if (prod && !prod->rotated_output && engine_step_small(e) && engine_cluster_ok(e, (char*)e->step_qrot + qo, (char*)e->step_kpost + ko, v, out)) {
+        int r = engine_step_prepare(e, l0, n, q, k, v, s, prod, true);
+        return r != TQ_OK ? r : engine_cluster_step(e, l0, n, (char*)e->step_qrot + qo, (char*)e->step_kpost + ko, v, out, s);
+    }
     int r = engine_step_prepare(e, l0, n, q, k, v, s, prod);
     if (r != TQ_OK) return r;
     return engine_step_attend(e, l0, n, q, out, s, prod);
@@ -1535,7 +1604,7 @@ static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* 
                 n, h[0] / w, h[1] / w, h[2] / w, h[3] / w, h[4] / w, h[5] / w, h[6] / w, h[8] / w, h[9] / w, h[10] / w, h[11] / w, h[12] / w, w);
     }
 #endif
-    return launch_kernel(merge_partials_kernel, dim3(G, n), dim3(MERGE_WARPS * 32), 0, s, use_pdl(), m);
+    return launch_kernel(merge_partials_kernel<8>, dim3(G, n), dim3(256), 0, s, use_pdl(), m);
 }
 
 int tq_engine_time_attention(tq_engine* e, int enable) {
@@ -1564,6 +1633,13 @@ int tq_engine_step_prepare(tq_engine* e, const void* q, const void* k, const voi
     if (!e || !q || !k || !v) return TQ_ERR_ARG;
     if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     if (!engine_whole_step_ok(e, q, k, v, q)) return TQ_ERR_UNSUPPORTED;
+    if (engine_step_small(e) && engine_cluster_ok(e, e->stage_q, e->stage_k, e->stage_v, q)) {
+        // the second phase runs the cluster form, on copies of the step's inputs
+        const size_t qb = (size_t)e->shape.num_layers * e->G * e->q_dim() * 2, kb = (size_t)e->shape.num_layers * e->G * e->kv_dim() * 2;
+        TQ_CUDA(cudaMemcpyAsync(e->stage_q, q, qb, cudaMemcpyDeviceToDevice, cs(s)));
+        TQ_CUDA(cudaMemcpyAsync(e->stage_k, k, kb, cudaMemcpyDeviceToDevice, cs(s)));
+        TQ_CUDA(cudaMemcpyAsync(e->stage_v, v, kb, cudaMemcpyDeviceToDevice, cs(s)));
+    }
     return engine_step_prepare(e, 0, e->shape.num_layers, q, k, v, cs(s), nullptr);
 }
 
@@ -1571,7 +1647,23 @@ int tq_engine_step_attend_layers(tq_engine* e, int first_layer, int n_layers, vo
     if (!e || !out_first || first_layer < 0 || n_layers <= 0 || first_layer + n_layers > e->shape.num_layers) return TQ_ERR_ARG;
     if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     if (!engine_whole_step_ok(e, out_first, out_first, out_first, out_first)) return TQ_ERR_UNSUPPORTED;
+    const size_t qo = (size_t)first_layer * e->G * e->q_dim() * 2, ko = (size_t)first_layer * e->G * e->kv_dim() * 2;
+    if (engine_step_small(e) && engine_cluster_ok(e, e->stage_q, e->stage_k, e->stage_v, out_first))
+        return engine_cluster_step(e, first_layer, n_layers, (char*)e->stage_q + qo, (char*)e->stage_k + ko, (char*)e->stage_v + ko, out_first, cs(s));
     return engine_step_attend(e, first_layer, n_layers, nullptr, out_first, cs(s), nullptr);
+}
+
+// The layers l0 .. l0 + n - 1 of a step whose inputs are all there, in the form that is fastest for the whole step's size.
+static int engine_decode_range(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s) {
+    const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
+    if (engine_step_small(e) && engine_cluster_ok(e, q, k, v, out)) return engine_cluster_step(e, l0, n, q, k, v, out, s);
+    if (engine_whole_step_ok(e, q, k, v, out)) return engine_step_layers(e, l0, n, q, k, v, out, s);
+    for (int i = 0; i < n; ++i) {
+        int r = tq_engine_decode_layer(e, l0 + i, (const char*)q + qb * i, (const char*)k + kb * i, (const char*)v + kb * i, (char*)out + qb * i,
+                                       (tq_stream_t)s);
+        if (r != TQ_OK) return r;
+    }
+    return TQ_OK;
 }
 
 int tq_engine_decode_layers(tq_engine* e, int first_layer, int n_layers, const void* q, const void* k, const void* v, void* out,
@@ -1579,14 +1671,7 @@ int tq_engine_decode_layers(tq_engine* e, int first_layer, int n_layers, const v
     if (!e || !q || !k || !v || !out || first_layer < 0 || n_layers <= 0 || first_layer + n_layers > e->shape.num_layers)
         return TQ_ERR_ARG;
     if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
-    if (engine_whole_step_ok(e, q, k, v, out)) return engine_step_layers(e, first_layer, n_layers, q, k, v, out, cs(s));
-    const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
-    for (int i = 0; i < n_layers; ++i) {
-        int r = tq_engine_decode_layer(e, first_layer + i, (const char*)q + qb * i, (const char*)k + kb * i, (const char*)v + kb * i,
-                                       (char*)out + qb * i, s);
-        if (r != TQ_OK) return r;
-    }
-    return TQ_OK;
+    return engine_decode_range(e, first_layer, n_layers, q, k, v, out, cs(s));
 }
 
 int tq_engine_decode_step(tq_engine* e, const void* q, const void* k, const void* v, void* out, tq_stream_t s) {
@@ -1852,22 +1937,12 @@ int tq_engine_decode_step_host(tq_engine* e, const void* q_host, const void* k_h
     for (int c = 0; c < chunks; ++c) {
         const int l0 = first_layer(c), l1 = first_layer(c + 1);
         TQ_CUDA(cudaStreamWaitEvent(cs(s), e->ev_in[c], 0));
-        const bool whole = engine_whole_step_ok(e, e->stage_q, e->stage_k, e->stage_v, e->stage_out) && ((qb | kb) & 15u) == 0;
-        for (int l = l0; l < l1; ++l) {
-            int r;
-            if (whole) {  // the chunk's layers in one whole-step pass
-                r = engine_step_layers(e, l0, l1 - l0, (char*)e->stage_q + qb * l0, (char*)e->stage_k + kb * l0,
-                                       (char*)e->stage_v + kb * l0, (char*)e->stage_out + qb * l0, cs(s));
-                l = l1;
-            } else {
-                r = tq_engine_decode_layer(e, l, (char*)e->stage_q + qb * l, (char*)e->stage_k + kb * l,
-                                           (char*)e->stage_v + kb * l, (char*)e->stage_out + qb * l, s);
-            }
-            if (r != TQ_OK) {
-                cudaStreamSynchronize(e->st_in);
-                cudaStreamSynchronize(cs(s));
-                return r;
-            }
+        const int r = engine_decode_range(e, l0, l1 - l0, (char*)e->stage_q + qb * l0, (char*)e->stage_k + kb * l0, (char*)e->stage_v + kb * l0,
+                                          (char*)e->stage_out + qb * l0, cs(s));
+        if (r != TQ_OK) {
+            cudaStreamSynchronize(e->st_in);
+            cudaStreamSynchronize(cs(s));
+            return r;
         }
         TQ_CUDA(cudaEventRecord(e->ev_out[c], cs(s)));
         TQ_CUDA(cudaStreamWaitEvent(e->st_out, e->ev_out[c], 0));

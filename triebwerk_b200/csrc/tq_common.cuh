@@ -34,7 +34,7 @@ enum : int {
 // ---- workspace layout ---------------------------------------------------------------------------------------
 // [0,256)                       header: int status; int total_tiles; ...
 // q_rot      float [G][H][128]  pre-rotated queries, already multiplied by log2(e)/sqrt(128)
-// tile_start int   [G+1]        exclusive prefix of ceil(L_g / TILE_TOKENS)
+// tile_start int   [G+4]        exclusive prefix of ceil(L_g / TILE_TOKENS); one-launch form: then workers, total tiles
 // tickets    int   [G]          arrivals per sequence (zeroed by the append/rotate kernel)
 // worker_g   int   [MAX_WORKERS] first sequence of each attention worker's slice
 // partials   float [W+G][H][PART_STRIDE]  acc[128], m, l, pad
@@ -64,7 +64,7 @@ __host__ inline Workspace carve_workspace(void* base, int G, int H) {
     w.q_rot = (float*)(p + off);
     off += align_up((size_t)G * H * HEAD_DIM * sizeof(float), 256);
     w.tile_start = (int*)(p + off);
-    off += align_up((size_t)(G + 1) * sizeof(int), 256);
+    off += align_up((size_t)(G + 4) * sizeof(int), 256);
     w.tickets = (int*)(p + off);
     off += align_up((size_t)G * sizeof(int), 256);
     w.worker_g = (int*)(p + off);

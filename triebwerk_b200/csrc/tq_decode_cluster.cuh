@@ -57,7 +57,10 @@ struct ClusterDecodeParams {
     const int* prefix_tiles;
     int* status;                 // or null
     int pos_value, max_seq_len, capacity_rows;
-    int H, Hkv, q_dim;
+    int G, H, Hkv, q_dim;
+    // Several layers in one launch (a decode step that has all layers' queries, keys and values at once): grid.z = layers * G,
+    // the pointers above are the first layer's, the others lie these strides behind (bytes of the code arrays, halves elsewhere).
+    long long code_layer_stride, norm_layer_stride, q_layer_stride, kv_layer_stride;
     int head_blocks;             // clusters per KV head: ceil(query heads per KV head / 8)
     int early;                   // as in AttnParams: positions and old rows may be read before the previous kernel has finished
     int static_rotation;         // R is not written by any kernel of the stream: staged before the wait
@@ -141,15 +144,23 @@ inline size_t cd_smem_bytes(int bits, int heads) {
 
 // MB: 16-token blocks per tile (2 for throughput, 1 where every warp gets a single tile anyway and its latency counts)
 template <int BITS, int MB>
-__global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const ClusterDecodeParams p) {
+__global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const ClusterDecodeParams p_in) {
     extern __shared__ __align__(1024) uint8_t cd_smem[];
+    ClusterDecodeParams p = p_in;
     constexpr int BPH = BITS == 0 ? 256 : (BITS == 4 ? 64 : 32);  // bytes of a head's row
     constexpr int TT = 16 * MB;                                   // tokens per tile
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gl = lane >> 2, t4 = lane & 3;
     const uint32_t rank = cluster_ctarank(), S = cluster_nctarank();
     const int kvh = blockIdx.y / p.head_blocks, hblk = blockIdx.y - kvh * p.head_blocks;
-    const int g = blockIdx.z;
+    const int layer = (int)blockIdx.z / p.G, g = (int)blockIdx.z - layer * p.G;
+    if (layer > 0) {
+        p.ck += layer * p.code_layer_stride; p.cv += layer * p.code_layer_stride;
+        p.kn += layer * p.norm_layer_stride; p.vn += layer * p.norm_layer_stride;
+        p.q += layer * p.q_layer_stride; p.out += layer * p.q_layer_stride;
+        p.new_k += layer * p.kv_layer_stride; p.new_v += layer * p.kv_layer_stride;
+        if (p.out_f32) p.out_f32 += (long long)layer * p.G * p.H * HEAD_DIM;
+    }
     const int grp = p.H / p.Hkv;
     const int nh = min(CD_HEADS, grp - CD_HEADS * hblk);  // query heads of this cluster
     const int head0 = kvh * grp + CD_HEADS * hblk;

@@ -354,7 +354,8 @@ inline int launch_attention_t(const CUtensorMap& tmK, const CUtensorMap& tmV, co
 }
 
 // mode 0: after append_rotate_kernel (rotated queries and tile table in the workspace); 1: one launch per layer and step
-// (table, query rotation, optional append and merge in the kernel); 2: whole-step form over AttnParams::n_layers layers.
+// (table, query rotation, optional append and merge in the kernel); 2: whole-step form over AttnParams::n_layers layers; 3: as 1
+// with the merge left to merge_partials_kernel.
 inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnParams& p, int ctas,
                             cudaStream_t s, bool pdl = false, int mode = 0) {
     if (p.Hkv != 8 && p.Hkv != 4) return TQ_ERR_UNSUPPORTED;
@@ -365,6 +366,7 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
     return bits == 4 ? launch_attention_t<4, 4, MODE>(tmK, tmV, p, ctas, s, pdl)                                \
                      : launch_attention_t<2, 4, MODE>(tmK, tmV, p, ctas, s, pdl);
     if (mode == 2) { TQ_ATTN_DISPATCH(2) }
+    if (mode == 3) { TQ_ATTN_DISPATCH(3) }
     if (mode == 1) { TQ_ATTN_DISPATCH(1) }
     TQ_ATTN_DISPATCH(0)
 #undef TQ_ATTN_DISPATCH
@@ -372,12 +374,12 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
 
 // One cluster per (sequence, KV head, block of 8 query heads): tq_decode_cluster.cuh.  `max_tokens`: rows a sequence may hold.
 template <int BITS, int MB>
-inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int G, cudaStream_t s, bool pdl) {
+inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int layers, cudaStream_t s, bool pdl) {
     const void* kernel = (const void*)cluster_decode_kernel<BITS, MB>;
     int r = ensure_dynamic_smem(kernel, cd_smem_bytes(BITS, CD_HEADS), true);
     if (r != TQ_OK) return r;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)S, (unsigned)(p.Hkv * p.head_blocks), (unsigned)G);
+    cfg.gridDim = dim3((unsigned)S, (unsigned)(p.Hkv * p.head_blocks), (unsigned)(p.G * layers));
     cfg.blockDim = dim3(CD_THREADS);
     cfg.dynamicSmemBytes = cd_smem_bytes(BITS, std::min(CD_HEADS, p.H / p.Hkv));
     cfg.stream = s;
@@ -391,17 +393,18 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int G, c
     cfg.numAttrs = pdl ? 2 : 1;
     return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB>, p));
 }
-inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int G, int max_tokens, cudaStream_t s, bool pdl) {
+// split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
+inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
     // As many CTAs per cluster as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch (two
     // share the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue: 8 sequences x 1023
     // tokens through the launchers 24 us a layer with two, 19 with one).
-    const long long clusters = (long long)G * p.Hkv * p.head_blocks, blocks = (max_tokens + 15) / 16;
+    const long long clusters = (long long)p.G * split_layers * p.Hkv * p.head_blocks, blocks = (max_tokens + 15) / 16;
     int S = 1;
     while (S < CD_MAX_CLUSTER && (long long)S * CD_WARPS < blocks && clusters * S * 2 <= device_props().sm_count) S *= 2;
-    if (bits == 0) return launch_cluster_decode_t<0, 1>(p, S, G, s, pdl);
+    if (bits == 0) return launch_cluster_decode_t<0, 1>(p, S, layers, s, pdl);
     const bool one = (long long)S * CD_WARPS >= blocks;  // a single 16-token tile per warp
-    if (bits == 4) return one ? launch_cluster_decode_t<4, 1>(p, S, G, s, pdl) : launch_cluster_decode_t<4, 2>(p, S, G, s, pdl);
-    return one ? launch_cluster_decode_t<2, 1>(p, S, G, s, pdl) : launch_cluster_decode_t<2, 2>(p, S, G, s, pdl);
+    if (bits == 4) return one ? launch_cluster_decode_t<4, 1>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2>(p, S, layers, s, pdl);
+    return one ? launch_cluster_decode_t<2, 1>(p, S, layers, s, pdl) : launch_cluster_decode_t<2, 2>(p, S, layers, s, pdl);
 }
 
 __global__ void transpose_rotation_kernel(__half* dst, const __half* src, int* tickets = nullptr, int n_tickets = 0) {

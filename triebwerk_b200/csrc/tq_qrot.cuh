@@ -31,6 +31,7 @@ struct QRotParams {
     int rope_dim;            // 64 or 128
     float eps;
     int biased;              // weights are stored minus one (the reference's `biased` flag)
+    int raw;                 // 1: store the produced vectors as they are (for a consumer that rotates them itself)
 };
 
 // RMS norm + rotary embedding of one head vector spread over the four lanes of a row: lane t4 holds, for m = 0 .. 3,
@@ -143,6 +144,16 @@ __global__ void __launch_bounds__(QROT_WARPS * 32) rotate_queries_kernel(const Q
             const size_t pa = (size_t)p.positions[(int)(lga % p.G)] * half_rope, pb = (size_t)p.positions[(int)(lgb % p.G)] * half_rope;
             qk_norm_rope_row(a_lo, p.norm_w + (size_t)(lga / p.G) * HEAD_DIM, p.rope_cos + pa, p.rope_sin + pa, p.rope_dim, p.eps, p.biased, t4);
             qk_norm_rope_row(a_hi, p.norm_w + (size_t)(lgb / p.G) * HEAD_DIM, p.rope_cos + pb, p.rope_sin + pb, p.rope_dim, p.eps, p.biased, t4);
+            if (p.raw) {
+                if (warp == 0) {  // (every warp has produced all 16 vectors)
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        if (va < p.n_vec) *(reinterpret_cast<uint4*>(p.q_rot + (size_t)va * HEAD_DIM + 32 * m) + t4) = a_lo[m];
+                        if (vb < p.n_vec) *(reinterpret_cast<uint4*>(p.q_rot + (size_t)vb * HEAD_DIM + 32 * m) + t4) = a_hi[m];
+                    }
+                }
+                continue;
+            }
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
