@@ -1496,6 +1496,7 @@ static int engine_step_prepare(tq_engine* e, int l0, int n, const void* q, const
     PrefillTcParams t{};
     t.ck = (uint8_t*)L.k; t.kn = (__half*)L.kn; t.cv = (uint8_t*)L.v; t.vn = (__half*)L.vn;
     t.k_buf = (const __half*)k; t.v_buf = (const __half*)v; t.rotation = (const __half*)e->d_rotation;
+    t.static_rotation = 1;
     t.positions = e->d_positions; t.status = (int*)e->workspace;
     t.token_row0 = 0; t.seq_stride_rows = e->msl; t.row_base = e->rb();
     t.capacity_rows = e->msl; t.seq_capacity = e->caps();
@@ -1507,7 +1508,7 @@ static int engine_step_prepare(tq_engine* e, int l0, int n, const void* q, const
         t.rope_dim = prod->rope_dim; t.eps = prod->eps; t.biased = prod->biased;
         t.k_post = (__half*)e->step_kpost + (size_t)l0 * G * e->kv_dim();
     }
-    int r = launch_prefill_tc_params(t, s, prod != nullptr);
+    int r = launch_prefill_tc_params(t, s, use_pdl(), prod != nullptr);
     if (r != TQ_OK) return r;
     {   // all query heads of the n layers, rotated and scaled, as fp16 (producer form: normed and rope'd first)
         QRotParams qr{};
@@ -1759,10 +1760,10 @@ static int engine_prefill_impl(tq_engine* e, int layer, int first_seq, int n_seq
     p.max_seq_len = e->msl; p.capacity_rows = cap;
     p.n_src = T; p.H = e->shape.num_heads; p.Hkv = e->shape.num_kv_heads; p.q_dim = e->q_dim(); p.kv_dim = e->kv_dim();
     p.bits = e->kv_bits; p.pos_value = first_pos;
-    if (n_seq == 1) return launch_append(p, cs(s));
+    if (n_seq == 1) return launch_append(p, cs(s), use_pdl());
     if ((long long)n_seq * T * p.Hkv >= (1ll << 31)) return TQ_ERR_CAPACITY;
     // several sequences: the tensor-core kernel takes them in one launch (whatever their number of head vectors)
-    return launch_prefill_tc(p, cs(s), n_seq, e->msl, e->rb() ? e->rb() + first_seq : nullptr);
+    return launch_prefill_tc(p, cs(s), use_pdl(), n_seq, e->msl, e->rb() ? e->rb() + first_seq : nullptr);
 }
 
 // A prompt of T tokens shared by the sequences first_seq .. first_seq + n_seq - 1 (rollouts of one prompt: the

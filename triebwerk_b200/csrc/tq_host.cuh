@@ -236,7 +236,7 @@ inline int launch_append_t(const AppendParams& p, dim3 grid, cudaStream_t s, boo
 // Whole prompts (token form, K and/or V, no queries) go to the tensor-core kernel; TQ_PREFILL_TC=0 keeps them on
 // the fp32-chain kernel.  Both store the same bytes.
 // producer: the form that applies QK-norm and rotary embedding to the K vectors on the way in (PrefillTcParams)
-inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bool producer = false) {
+inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bool pdl, bool producer = false) {
     const long long tokens = (long long)t.n_seq * t.T;
     const long long tiles = ((tokens * t.Hkv + TC_TILE - 1) / TC_TILE) * ((t.k_buf ? 1 : 0) + (t.v_buf ? 1 : 0));
     long long grid = (long long)(producer ? 2 : TC_CTAS_PER_SM) * device_props().sm_count;
@@ -262,9 +262,21 @@ inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bo
         ts.stamps = d_stamps;
     }
 #endif
-    if (producer) prefill_append_tc_kernel<true, false><<<(unsigned)grid, TC_THREADS, TC_DYN_SMEM, s>>>(tmk, tmv, ts);
-    else if (tma) prefill_append_tc_kernel<false, true><<<(unsigned)grid, TC_THREADS, TC_DYN_SMEM, s>>>(tmk, tmv, ts);
-    else prefill_append_tc_kernel<false, false><<<(unsigned)grid, TC_THREADS, TC_DYN_SMEM, s>>>(tmk, tmv, ts);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = TC_DYN_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaError_t le;
+    if (producer) le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<true, false>, tmk, tmv, ts);
+    else if (tma) le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<false, true>, tmk, tmv, ts);
+    else le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<false, false>, tmk, tmv, ts);
+    if (le != cudaSuccess) return (int)le;
 #ifdef TQ_TIMING_SWITCHES
     if (ts.stamps && ++stamp_calls == 40) {
         unsigned long long h[32];
@@ -282,7 +294,7 @@ inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bo
     return cuda_status(cudaGetLastError());
 }
 
-inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, int n_seq = 1, long long seq_stride_rows = 0,
+inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, bool pdl, int n_seq = 1, long long seq_stride_rows = 0,
                              const long long* seq_row_base = nullptr) {
     PrefillTcParams t{};
     t.ck = p.ck; t.kn = p.kn; t.cv = p.cv; t.vn = p.vn;
@@ -290,7 +302,8 @@ inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, int n_seq = 
     t.token_row0 = p.token_row0; t.capacity_rows = p.capacity_rows;
     t.seq_stride_rows = seq_stride_rows; t.row_base = seq_row_base; t.n_seq = n_seq;
     t.T = p.n_src; t.Hkv = p.Hkv; t.kv_dim = p.kv_dim; t.bits = p.bits;
-    return launch_prefill_tc_params(t, s);
+    t.static_rotation = p.rot_prep ? 1 : 0;  // (the engine's own R)
+    return launch_prefill_tc_params(t, s, pdl);
 }
 
 inline int launch_append(const AppendParams& p, cudaStream_t s, bool pdl = false) {
@@ -299,7 +312,7 @@ inline int launch_append(const AppendParams& p, cudaStream_t s, bool pdl = false
     const uintptr_t align_or = (uintptr_t)p.k_buf | (uintptr_t)p.v_buf | (uintptr_t)p.ck | (uintptr_t)p.cv | (uintptr_t)p.rotation;
     if (prefill_tc && p.token_mode && !p.q && (p.k_buf || p.v_buf) && (align_or & 15u) == 0 &&
         p.kv_dim == p.Hkv * HEAD_DIM && (long long)p.n_src * p.Hkv >= 4 * TC_TILE && (long long)p.n_src * p.Hkv < (1ll << 31))
-        return launch_prefill_tc(p, s);
+        return launch_prefill_tc(p, s, pdl);
     const int nk = p.k_buf ? p.Hkv : 0, nv = p.v_buf ? p.Hkv : 0, nq = p.q ? p.H : 0;
     const long long total = (long long)p.n_src * (nk + nv + nq);
     const bool tables = p.tile_start != nullptr && !p.token_mode;

@@ -3,7 +3,7 @@
 // Query token t of a prompt attends to cache rows 0 .. t (reference engine/kernels.cu:1874-1960 packed, :1071-1158 fp16).
 // One CTA has two SLOTS that work in turn, so that the tensor core always has a product of one slot while the softmax of the
 // other runs.  A slot = 128 score rows (128 / GRP query tokens x the GRP query heads of one KV head) = the M dimension,
-// a warpgroup of softmax threads (one thread per row), 128 columns of tensor memory for S and 128 for O:
+// eight softmax warps (16 rows each, four threads per row), 128 columns of tensor memory for S and 128 for O:
 //   * long prompts (MT = 2): the slots are two consecutive query blocks that share every K and V tile;
 //   * short ones (MT = 1): both slots hold the same query block and take the even and the odd tiles; their results are
 //     combined at the end.  Twice the CTAs and half the chain when there are not enough blocks for the GPU.
@@ -14,17 +14,19 @@
 // this kernel the table look-ups and operand stores took as much of the shared-memory pipe as the products themselves (8192
 // tokens, 16/8 heads, 4-bit: 617 us against 439).  P (times the V norm, fp16) replaces S in tensor memory and is read from
 // there as the A operand.
-//   warps 0-7    softmax of slots 0 and 1: S -> registers, K norm, causal limit, exponentials, P -> tensor memory.  The
+//   warps 0-15   softmax of slots 0 and 1: S -> registers (16x256b loads: a thread holds two rows' column pairs as in an mma
+//                fragment, so a row's maximum is two shuffles), K norm, causal limit, exponentials, P -> tensor memory.  The
 //                exponentials' reference point follows the row maximum only when that has grown by more than PFT_SLACK (in
 //                powers of two): weights stay below 2^PFT_SLACK and O is rescaled in place in the first tiles only.
-//   warp 8       issues the copies; warp 9 issues every product, in the order P(i) V -> S(i + 1) per slot, slots alternating: the
+//   warp 16      issues the copies; warp 17 issues every product, in the order P(i) V -> S(i + 1) per slot, slots alternating: the
 //                products of one thread execute in order, so S(i + 1) may overwrite the P(i) that the one before it reads.
 // Packed forms: Q R^T at the start and (O / l) R at the end (fp16 high + low parts) are tcgen05 products too.
 // Every wait on a barrier is bounded; a wait that runs out raises the status word and the kernel runs to its end.
 // Bound by the softmax threads (exponentials, tensor-memory loads) against the tensor core at long prompts, by the chain copy ->
 // S -> softmax -> O of a single block at short ones.  Per layer, 8 KV heads, cache write included, the one-block kernel with V
-// transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 530 us (1040 TFLOP/s of causal arithmetic), 777
-// tokens 59 -> 31; 4-bit 8192 tokens 16 heads 763 -> 379 us, 777 tokens 43.7 -> 34.2.
+// transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 508 us (1080 TFLOP/s of causal arithmetic), 777
+// tokens 59 -> 29; 4-bit 8192 tokens 16 heads 763 -> 350 us, 777 tokens 43.7 -> 32.2.  (With one thread per row, eight softmax
+// warps, S read twice: 530, 31, 379, 34.2.)
 #pragma once
 
 #include "tq_prefill_tc.cuh"
@@ -37,11 +39,12 @@ constexpr float PFT_SLACK = 4.0f;
 constexpr float PFT_SCALE = 0.12751743074602467f;  // log2(e) / sqrt(128); packed forms: carried by the rotated queries
 constexpr uint32_t PFT_TILE = 32768u;  // an operand tile: [2 halves of the coordinates][128 rows][128 B]
 
-constexpr int PFT_THREADS = 384;  // 8 softmax warps, one for the copies, one for the products, two idle (a full warpgroup)
-// Registers per thread of the softmax and the other warpgroup after the split.  The launch must bring at least their sum (the
-// host checks what the kernel was built with): 384 x 168 >= 256 x 200 + 128 x 88.
-constexpr int PFT_REGS_SOFT = 200, PFT_REGS_REST = 88;
-constexpr int PFT_REGS_LAUNCH = (256 * PFT_REGS_SOFT + 128 * PFT_REGS_REST + PFT_THREADS - 1) / PFT_THREADS;
+constexpr int PFT_SOFT_WARPS = 16;
+constexpr int PFT_THREADS = 32 * PFT_SOFT_WARPS + 128;  // softmax, then one warp for the copies, one for the products, two idle (a full warpgroup)
+// Registers per thread of the softmax warpgroups and of the last one after the split.  The launch must bring at least their sum
+// (the host checks what the kernel was built with): 640 x 96 = 512 x 104 + 128 x 64.
+constexpr int PFT_REGS_SOFT = 104, PFT_REGS_REST = 64;
+constexpr int PFT_REGS_LAUNCH = (32 * PFT_SOFT_WARPS * PFT_REGS_SOFT + 128 * PFT_REGS_REST + PFT_THREADS - 1) / PFT_THREADS;
 
 struct PrefillAttnParams {
     const __half* q;          // queries [n_seq][T][q_tok_stride] as the model makes them
@@ -131,24 +134,29 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
     }
 }
 
-// 32 lanes x 32 consecutive 32-bit columns, registers -> tensor memory (the counterpart of tmem_ld32)
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
-        "r"(r[31])
-        : "memory");
+// 16 lanes x 32 (64) consecutive 32-bit columns.  Thread (g = lane / 4, t = lane % 4) holds of column block j (8 columns) the
+// columns 8 j + 2 t, + 1 of row g in r[4 j], r[4 j + 1] and of row g + 8 in r[4 j + 2], r[4 j + 3].
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
+__device__ __forceinline__ void tmem_ld_frag64(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_frag32(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+// 16 lanes x 32 columns of words that pack two halves each: of word block j (4 words) word 4 j + t of row g in r[2 j], of row g + 8
+// in r[2 j + 1] -- what the two values of a fragment pack to
+__device__ __forceinline__ void tmem_st_pack32(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // The same products with the descriptors as their low words; the high word is common to all operand tiles of this kernel (groups
@@ -208,7 +216,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         if (threadIdx.x == 0 && p.status) atomicMax(p.status, ST_SMEM_LAYOUT);
         return;
     }
-    constexpr int MMA_WARP = 9;
+    constexpr int COPY_WARP = PFT_SOFT_WARPS, MMA_WARP = PFT_SOFT_WARPS + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int GRP = p.grp, QT = PFT_ROWS / GRP;
     const int qb = (int)gridDim.y - 1 - (int)blockIdx.y;  // the longest causal prefixes of all heads and prompts first
@@ -248,7 +256,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             mbar_init(bar_kfree + 8u * i, 1);
             mbar_init(bar_vfree + 8u * i, 1);
             mbar_init(bar_sfull + 8u * i, 1);
-            mbar_init(bar_pfull + 8u * i, PFT_ROWS);
+            mbar_init(bar_pfull + 8u * i, 16 * PFT_SOFT_WARPS);
         }
         mbar_init(bar_rot, 1);
         mbar_init(bar_done, 1);
@@ -261,9 +269,10 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     __syncthreads();
     tc_fence_after();
     pdl_wait();
+    pdl_launch_dependents();  // (the next launch waits for this one's end before it reads or writes anything of the caller's)
     // this block's queries, row (token, head), and R: one copy each (rows behind GRP * QT and tokens past the prompt: whatever comes
     // -- a row's garbage stays in that row and is never stored)
-    if (tid == 256) {
+    if (tid == 32 * COPY_WARP) {
         mbar_arrive_expect_tx(bar_q, (uint32_t)(MT * QT * GRP) * 256u + (PACKED ? PFT_TILE : 0u));
         for (int m = 0; m < MT; ++m) {  // a box narrower than the tile: the coordinate halves separately
             tma_load_4d(sb + PftSmem::Q + m * PFT_TILE, &tmQ, bar_q, 0, kvh * GRP, seq * p.T + q0 + m * QT, 0);
@@ -272,12 +281,20 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         if (PACKED) tma_load_3d(sb + PftSmem::R, &tmR, bar_q, 0, 0, 0);
     }
     const uint32_t tmem = *tmem_slot;
-    // softmax threads: slot, score row = tensor-memory lane, the row's token and query head
-    const int slot = warp >> 2, srow = (warp & 3) * 32 + lane;
-    const int my_t = srow / GRP, my_first = q0 + (MT == 2 ? slot * QT : 0);
-    const int my_tok = my_t < QT ? my_first + my_t : p.T;  // (p.T: a row of no query)
-    const int my_head = kvh * GRP + (srow - my_t * GRP);
-    const uint32_t my_lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    // softmax warps: slot, 16 score rows (= tensor-memory lanes) row0 ..; a thread's rows row0 + g and row0 + g + 8
+    const int slot = (warp >> 2) & 1, row0 = 32 * (warp & 3) + 16 * (warp >> 3), g = lane >> 2, t4 = lane & 3;
+    const int my_first = q0 + (MT == 2 ? slot * QT : 0);
+    auto token_of = [&](int row) { return row / GRP < QT ? my_first + row / GRP : p.T; };  // (p.T: a row of no query)
+    const uint32_t my_lanes = tmem + ((uint32_t)row0 << 16);
+    // a pair of columns (c, c + 1) of a row of an operand tile
+    auto put_pair = [&](uint32_t tile, int row, int c, float x, float y) {
+        *reinterpret_cast<uint32_t*>(gb + tile + pft_chunk(row, c >> 3) + (uint32_t)(c & 7) * 2u) = pack_half2(x, y);
+    };
+    // in the products before and after the tiles a warp takes 128 columns of its slot's rows, or with one query block, whose rows
+    // both slots' warps share, 64
+    constexpr int PCOLS = MT == 2 ? 128 : 64;
+    const int pcol0 = MT == 2 ? 0 : 64 * slot;
+    const uint32_t pslot = MT == 2 ? (uint32_t)slot : 0u;
 
     if (PACKED) {
         // ---- q_rot = Q . R^T (reference engine/kernels.cu:1896-1903), scaled by log2(e) / sqrt(128), back into the Q tiles ----
@@ -290,38 +307,33 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     umma_lo(tmem + 128u * m, pft_lo_k(sb + PftSmem::Q + m * PFT_TILE) + pft_kstep(ks), pft_lo_k(sb + PftSmem::R) + pft_kstep(ks), PFT_IDESC_K, ks != 0);
             umma_commit(bar_rot);
         }
-        if (warp < 4 * MT) {
+        if (warp < PFT_SOFT_WARPS) {
             wait_bar(bar_rot, 0u);
             tc_fence_after();
 #pragma unroll 1
-            for (int c2 = 0; c2 < 4; ++c2) {
-                uint32_t r[32];
-                tmem_ld32(my_lanes + 128u * slot + 32u * c2, r);
+            for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 32) {
+                uint32_t r[16];
+                tmem_ld_frag32(my_lanes + 128u * pslot + (uint32_t)c0, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float sc = PFT_SCALE;
-                    uint4 u;
-                    u.x = pack_half2(__uint_as_float(r[8 * i]) * sc, __uint_as_float(r[8 * i + 1]) * sc);
-                    u.y = pack_half2(__uint_as_float(r[8 * i + 2]) * sc, __uint_as_float(r[8 * i + 3]) * sc);
-                    u.z = pack_half2(__uint_as_float(r[8 * i + 4]) * sc, __uint_as_float(r[8 * i + 5]) * sc);
-                    u.w = pack_half2(__uint_as_float(r[8 * i + 6]) * sc, __uint_as_float(r[8 * i + 7]) * sc);
-                    *reinterpret_cast<uint4*>(gb + PftSmem::Q + slot * PFT_TILE + pft_chunk(srow, 4 * c2 + i)) = u;
-                }
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        put_pair(PftSmem::Q + pslot * PFT_TILE, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, __uint_as_float(r[4 * j + 2 * h]) * PFT_SCALE,
+                                 __uint_as_float(r[4 * j + 2 * h + 1]) * PFT_SCALE);
             }
         }
-        if (warp < 8 || warp == MMA_WARP) {  // the rotated queries are in place (the copies of the first tiles are on their way already)
+        if (warp < PFT_SOFT_WARPS || warp == MMA_WARP) {  // the rotated queries are in place (the copies of the first tiles are on their way already)
             fence_proxy_async_smem();
             tc_fence_before();
-            named_barrier(1, 288);
+            named_barrier(1, 32 * PFT_SOFT_WARPS + 32);
             tc_fence_after();
         }
     }
 
-    float m_run = -1e30f, l_run = 0.0f;
-    if (warp >= 8) {
+    if (warp >= PFT_SOFT_WARPS) {
       regs_dec<PFT_REGS_REST>();
-      if (warp == 8) {
+      if (warp == COPY_WARP) {
         // ================= the copies of every tile =================
         // (fp16 caches, the prompt's last tile: rows past the prompt may hold anything, and 0 x NaN is NaN, so its V rows are blanked)
         const int x_row = (int)seq_row0;
@@ -400,7 +412,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         __syncwarp();
         if (PACKED) {
             // out[d] = sum_k R[k][d] * acc[k] (reference engine/kernels.cu:1957): the results' high and low parts times R
-            named_barrier(1, 288);
+            named_barrier(1, 32 * PFT_SOFT_WARPS + 32);
             tc_fence_after();
             if (lane == 0 && !dead) {
 #pragma unroll
@@ -417,197 +429,203 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         }
       }
     } else {
-        // ================= softmax of slot `slot`, row `srow` =================
+        // ================= softmax of slot `slot`, rows row0 + g and row0 + g + 8 =================
         regs_inc<PFT_REGS_SOFT>();
         const uint32_t s_col = my_lanes + 128u * slot, o_col = my_lanes + 256u + 128u * slot;
         const int nt = slot ? n1 : n0;
+        const int tok0 = token_of(row0 + g), tok1 = token_of(row0 + g + 8);
+        float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};  // (sums: of this thread's columns)
         for (int i = 0; i < nt; ++i) {
             const int j = tile_of(slot, i), st = j & 1, col0 = j * PFT_KT;
             if (PACKED) wait_bar(bar_vfull + 8u * st, (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
             wait_bar(bar_sfull + 8u * slot, (uint32_t)(i & 1));
             tc_fence_after();
             const bool diagonal = col0 + PFT_KT - 1 > my_first;  // (uniform for the slot)
-            const int lim = my_tok - col0;                        // columns up to here count
-            const float4* const nrm = reinterpret_cast<const float4*>(gb + PftSmem::NORM + (uint32_t)st * 1024u);
-            // S comes out of tensor memory twice, 64 columns at a time: once for the row maximum, once for the weights.  Holding
-            // all 128 columns in between would save four loads and cost an unrolled body of several thousand instructions, which a
-            // short prompt spends its time fetching (777 tokens, 16/8 heads, 4-bit: 38.9 us a layer that way, 35.2 this way).
-            auto load64 = [&](int c, float2 (&x)[32]) {  // 64 scores, scaled (packed: by the K norms), masked
-                uint32_t r[2][32];
-                tmem_ld32(s_col + 64u * c, r[0]);
-                tmem_ld32(s_col + 64u * c + 32u, r[1]);
-                tmem_ld_wait();
+            const float2* const nrm = reinterpret_cast<const float2*>(gb + PftSmem::NORM + (uint32_t)st * 1024u) + t4;
+            // ---- scores, scaled (packed: by the K norms), masked; row maxima ----
+            uint32_t sr[2][32];
+            tmem_ld_frag64(s_col, sr[0]);
+            tmem_ld_frag64(s_col + 64u, sr[1]);
+            tmem_ld_wait();
+            float2 x[2][16];  // [row][column block]
+            float mx[2] = {-1e30f, -1e30f};
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    const uint32_t* w = &r[e >> 4][2 * (e & 15)];
-                    x[e] = make_float2(__uint_as_float(w[0]), __uint_as_float(w[1]));
-                    x[e + 1] = make_float2(__uint_as_float(w[2]), __uint_as_float(w[3]));
-                    if constexpr (PACKED) {
-                        const float4 k4 = nrm[16 * c + (e >> 1)];
-                        x[e] = mul2(x[e], make_float2(k4.x, k4.y));
-                        x[e + 1] = mul2(x[e + 1], make_float2(k4.z, k4.w));
+            for (int b = 0; b < 16; ++b) {
+                float2 k2;
+                if constexpr (PACKED) k2 = nrm[4 * b];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    x[h][b] = make_float2(__uint_as_float(sr[b >> 3][4 * (b & 7) + 2 * h]), __uint_as_float(sr[b >> 3][4 * (b & 7) + 2 * h + 1]));
+                    if constexpr (PACKED) x[h][b] = mul2(x[h][b], k2);
+                }
+            }
+            if (diagonal) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int lim = (h ? tok1 : tok0) - col0 - 2 * t4;  // columns up to here count
+#pragma unroll
+                    for (int b = 0; b < 16; ++b) {
+                        if (8 * b > lim) x[h][b].x = -1e30f;
+                        if (8 * b + 1 > lim) x[h][b].y = -1e30f;
                     }
                 }
-                if (diagonal) {
+            }
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) {
-                        if (64 * c + 2 * e > lim) x[e].x = -1e30f;
-                        if (64 * c + 2 * e + 1 > lim) x[e].y = -1e30f;
-                    }
-                }
-            };
-            float mx = -1e30f;
-#pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
-                float2 x[32];
-                load64(c, x);
+            for (int h = 0; h < 2; ++h) {
                 float m2 = -1e30f;
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    mx = fmaxf(mx, fmaxf(x[e].x, x[e].y));
-                    m2 = fmaxf(m2, fmaxf(x[e + 1].x, x[e + 1].y));
+                for (int b = 0; b < 16; b += 2) {
+                    mx[h] = fmaxf(mx[h], fmaxf(x[h][b].x, x[h][b].y));
+                    m2 = fmaxf(m2, fmaxf(x[h][b + 1].x, x[h][b + 1].y));
                 }
-                mx = fmaxf(mx, m2);
+                mx[h] = fmaxf(mx[h], m2);
+                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+                if (!PACKED) mx[h] *= mx[h] <= -1e30f ? 1.0f : PFT_SCALE;
             }
-            if (!PACKED) mx *= mx <= -1e30f ? 1.0f : PFT_SCALE;
-            const bool grew = mx > m_run + PFT_SLACK;
-            const float mn = grew ? mx : m_run;
-            const float corr = ex2_approx(m_run - mn);
-            m_run = mn;
-            if (i > 0 && __any_sync(0xffffffffu, grew)) {  // S(i) is there, so P(i - 1) V has finished: O is at rest
+            const bool grew0 = mx[0] > m_run[0] + PFT_SLACK, grew1 = mx[1] > m_run[1] + PFT_SLACK;
+            if (__any_sync(0xffffffffu, grew0 || grew1)) {
+                const float mn0 = grew0 ? mx[0] : m_run[0], mn1 = grew1 ? mx[1] : m_run[1];
+                const float corr0 = ex2_approx(m_run[0] - mn0), corr1 = ex2_approx(m_run[1] - mn1);
+                m_run[0] = mn0; m_run[1] = mn1;
+                l_run[0] *= corr0; l_run[1] *= corr1;
+                if (i > 0) {  // S(i) is there, so P(i - 1) V has finished: O is at rest
 #pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t r[32];
-                    tmem_ld32(o_col + 32u * c, r);
-                    tmem_ld_wait();
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t r[16];
+                        tmem_ld_frag32(o_col + 32u * c, r);
+                        tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * corr);
-                    tmem_st32(o_col + 32u * c, r);
-                }
-            }
-            // ---- P (times the V norm) as fp16 over S: the columns a store covers have been read by then ----
-            float2 lsum2 = make_float2(0.0f, 0.0f);
-            const float2 sc2 = make_float2(PFT_SCALE, PFT_SCALE);
-            const float2 minus = mn <= -1e29f ? make_float2(0.0f, 0.0f) : make_float2(-mn, -mn);  // (no column counts yet: all weights 0)
-#pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
-                float2 x[32];
-                load64(c, x);
-                uint32_t pr[2][16];
-#pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    float4 v4;
-                    if constexpr (PACKED) v4 = nrm[32 + 16 * c + (e >> 1)];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        float2 a = PACKED ? add2(x[e + h], minus) : fma2(x[e + h], sc2, minus);
-                        a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-                        lsum2 = add2(lsum2, a);
-                        if constexpr (PACKED) a = mul2(a, h ? make_float2(v4.z, v4.w) : make_float2(v4.x, v4.y));
-                        pr[e >> 4][(e & 15) + h] = pack_half2(a.x, a.y);
+                        for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * ((e & 2) ? corr1 : corr0));
+                        tmem_st_frag32(o_col + 32u * c, r);
                     }
                 }
-                tmem_st16(s_col + 32u * c, pr[0]);
-                tmem_st16(s_col + 32u * c + 16u, pr[1]);
             }
-            l_run = l_run * corr + (lsum2.x + lsum2.y);
+            // ---- P (times the V norm) as fp16 over S ----
+            float2 lsum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+            float2 minus[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)  // (no column counts yet: all weights 0)
+                minus[h] = m_run[h] <= -1e29f ? make_float2(0.0f, 0.0f) : make_float2(-m_run[h], -m_run[h]);
+            const float2 sc2 = make_float2(PFT_SCALE, PFT_SCALE);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                uint32_t pr[16];
+#pragma unroll
+                for (int b = 0; b < 8; ++b) {
+                    float2 v2;
+                    if constexpr (PACKED) v2 = nrm[64 + 32 * c + 4 * b];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float2 a = PACKED ? add2(x[h][8 * c + b], minus[h]) : fma2(x[h][8 * c + b], sc2, minus[h]);
+                        a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+                        lsum[h] = add2(lsum[h], a);
+                        if constexpr (PACKED) a = mul2(a, v2);
+                        pr[2 * b + h] = pack_half2(a.x, a.y);
+                    }
+                }
+                tmem_st_pack32(s_col + 32u * c, pr);
+            }
+            l_run[0] += lsum[0].x + lsum[0].y;
+            l_run[1] += lsum[1].x + lsum[1].y;
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(bar_pfull + 8u * slot);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
+            l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
         }
         wait_bar(bar_done, 0u);  // every product has completed (and nobody reads the norms any more)
         tc_fence_after();
 
         // ================= results =================
-        // MT = 2: a slot's rows are its own.  MT = 1: the slots' sums over the same rows meet; slot s finishes the coordinate half s.
-        float inv, w0 = 0.0f, w1 = 0.0f;
+        // MT = 2: a slot's rows are its own.  MT = 1: the slots' sums over the same rows meet; slot s finishes the columns 64 s ..
+        float w0[2], w1[2] = {0.0f, 0.0f};  // by row: weights of the slots' sums, normalised (MT = 2: of its own)
         if constexpr (MT == 1) {
             float2* const xch = reinterpret_cast<float2*>(gb + PftSmem::NORM);
-            xch[slot * 128 + srow] = make_float2(m_run, l_run);
-            named_barrier(2, 256);
-            const float2 a = xch[srow], b = xch[128 + srow];
-            const float M = fmaxf(a.x, b.x), e0 = ex2_approx(a.x - M), e1 = n1 > 0 ? ex2_approx(b.x - M) : 0.0f;
-            inv = 1.0f / (a.y * e0 + b.y * e1 + 1e-8f);
-            w0 = e0 * inv;
-            w1 = e1 * inv;
+            if (t4 == 0) {
+                xch[slot * 128 + row0 + g] = make_float2(m_run[0], l_run[0]);
+                xch[slot * 128 + row0 + g + 8] = make_float2(m_run[1], l_run[1]);
+            }
+            named_barrier(2, 32 * PFT_SOFT_WARPS);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 a = xch[row0 + g + 8 * h], b = xch[128 + row0 + g + 8 * h];
+                const float M = fmaxf(a.x, b.x), e0 = ex2_approx(a.x - M), e1 = n1 > 0 ? ex2_approx(b.x - M) : 0.0f;
+                const float inv = 1.0f / (a.y * e0 + b.y * e1 + 1e-8f);
+                w0[h] = e0 * inv;
+                w1[h] = e1 * inv;
+            }
         } else {
-            inv = 1.0f / (l_run + 1e-8f);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) w0[h] = 1.0f / (l_run[h] + 1e-8f);
         }
-        auto result = [&](int c2, float (&x)[32]) {  // this row's columns 32 c2 .., normalised
-            uint32_t r[32];
-            tmem_ld32(MT == 2 ? o_col + 32u * c2 : my_lanes + 256u + 32u * c2, r);
+        const bool has_rows = MT == 1 || nt > 0;
+        auto result = [&](int c0, float (&y)[16]) {  // columns c0 .. c0 + 31, normalised, in fragment order
+            uint32_t r[16];
+            tmem_ld_frag32((MT == 2 ? o_col : my_lanes + 256u) + (uint32_t)c0, r);
             tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 32; ++e) x[e] = __uint_as_float(r[e]) * (MT == 2 ? inv : w0);
+            for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(r[e]) * w0[(e >> 1) & 1];
             if (MT == 1 && n1 > 0) {
-                tmem_ld32(my_lanes + 384u + 32u * c2, r);
+                tmem_ld_frag32(my_lanes + 384u + (uint32_t)c0, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 32; ++e) x[e] = fmaf(__uint_as_float(r[e]), w1, x[e]);
+                for (int e = 0; e < 16; ++e) y[e] = fmaf(__uint_as_float(r[e]), w1[(e >> 1) & 1], y[e]);
             }
         };
-        const int c_begin = MT == 2 ? 0 : 2 * slot, c_end = MT == 2 ? 4 : 2 * slot + 2;
-        __half* const dst = out_seq + (size_t)my_tok * p.q_dim + (size_t)my_head * HEAD_DIM;
-        const bool has_rows = MT == 1 || nt > 0, stores = my_tok < p.T;
-        auto store32 = [&](int c2, const float (&x)[32]) {
+        auto put_frag = [&](uint32_t tile, int c0, const float (&y)[16]) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint4 u;
-                u.x = pack_half2(x[8 * i], x[8 * i + 1]); u.y = pack_half2(x[8 * i + 2], x[8 * i + 3]);
-                u.z = pack_half2(x[8 * i + 4], x[8 * i + 5]); u.w = pack_half2(x[8 * i + 6], x[8 * i + 7]);
-                *reinterpret_cast<uint4*>(dst + 32 * c2 + 8 * i) = u;
-            }
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) put_pair(tile, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, y[4 * j + 2 * h], y[4 * j + 2 * h + 1]);
         };
-        if constexpr (!PACKED) {
+        const uint32_t qtile = PftSmem::Q + pslot * PFT_TILE, ktile = PftSmem::K + pslot * PFT_TILE;
+        if constexpr (PACKED) {
+            // out[d] = sum_k R[k][d] * acc[k]: the normalised rows, split into fp16 high and low parts, over the Q and K tiles
             if (has_rows) {
 #pragma unroll 1
-                for (int c2 = c_begin; c2 < c_end; ++c2) {
-                    float x[32];
-                    result(c2, x);
-                    if (stores) store32(c2, x);
-                }
-            }
-        } else {
-            // the normalised rows, split into fp16 high and low parts, over the Q and K tiles
-            const int m = MT == 2 ? slot : 0;
-            if (has_rows) {
-#pragma unroll 1
-                for (int c2 = c_begin; c2 < c_end; ++c2) {
-                    float x[32];
-                    result(c2, x);
+                for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 32) {
+                    float y[16];
+                    result(c0, y);
+                    put_frag(qtile, c0, y);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        uint4 uh, ul;
-                        uint32_t* ph = &uh.x;
-                        uint32_t* pl = &ul.x;
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float x0 = x[8 * i + 2 * e], x1 = x[8 * i + 2 * e + 1];
-                            const __half2 h = __floats2half2_rn(x0, x1);
-                            const float2 f = __half22float2(h);
-                            ph[e] = *reinterpret_cast<const uint32_t*>(&h);
-                            pl[e] = pack_half2(x0 - f.x, x1 - f.y);
-                        }
-                        *reinterpret_cast<uint4*>(gb + PftSmem::Q + m * PFT_TILE + pft_chunk(srow, 4 * c2 + i)) = uh;
-                        *reinterpret_cast<uint4*>(gb + PftSmem::K + m * PFT_TILE + pft_chunk(srow, 4 * c2 + i)) = ul;
-                    }
+                    for (int e = 0; e < 16; ++e) y[e] -= __half2float(__float2half_rn(y[e]));
+                    put_frag(ktile, c0, y);
                 }
             }
             fence_proxy_async_smem();
             tc_fence_before();
-            named_barrier(1, 288);
+            named_barrier(1, 32 * PFT_SOFT_WARPS + 32);
             wait_bar(bar_rot, 1u);
             tc_fence_after();
-            if (has_rows) {
+        }
+        if (has_rows) {
+            // the finished values as fp16 through the (consumed) query tile, so that 16 lanes store 256 contiguous bytes of a row
 #pragma unroll 1
-                for (int c2 = c_begin; c2 < c_end; ++c2) {
-                    uint32_t r[32];
-                    float x[32];
-                    tmem_ld32(my_lanes + 128u * m + 32u * c2, r);
+            for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 32) {
+                float y[16];
+                if constexpr (PACKED) {
+                    uint32_t r[16];
+                    tmem_ld_frag32(my_lanes + 128u * pslot + (uint32_t)c0, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) x[e] = __uint_as_float(r[e]);
-                    if (stores) store32(c2, x);
+                    for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(r[e]);
+                } else {
+                    result(c0, y);
+                }
+                put_frag(qtile, c0, y);
+            }
+            __syncwarp();
+            constexpr int CH = PCOLS / 8;  // 16-byte pieces per row
+#pragma unroll
+            for (int k = 0; k < CH / 2; ++k) {
+                const int at = 32 * k + lane, row = row0 + at / CH, ch = (pcol0 >> 3) + at % CH, tok = token_of(row);
+                if (tok < p.T) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(gb + qtile + pft_chunk(row, ch));
+                    *(reinterpret_cast<uint4*>(out_seq + (size_t)tok * p.q_dim + (size_t)(kvh * GRP + row % GRP) * HEAD_DIM) + ch) = u;
                 }
             }
         }

@@ -82,6 +82,7 @@ struct PrefillTcParams {
     const __half* k_buf;       // [T][kv_dim], either may be null
     const __half* v_buf;
     const __half* rotation;    // [128][128] row-major
+    int static_rotation;       // no kernel of the stream writes R: it is staged before the wait for the previous kernel
     const int* positions;      // [T] device, or null: token t goes to position pos_value + t
     int pos_value;
     int* status;
@@ -314,11 +315,21 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         mbar_init(bar_ld, 1);
         fence_mbar_init();
     }
-    for (int c = tid; c < 2048; c += TC_THREADS) {  // R as the B operand: row d, 16-byte chunk j
-        const int d = c >> 4, j = c & 15;
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p.rotation + (size_t)d * HEAD_DIM) + j);
-        *reinterpret_cast<uint4*>(gbase + (tc_operand_addr(base + TcSmem::B_R, d, 8 * j) - base)) = u;
-    }
+    auto stage_rotation = [&]() {  // R as the B operand: row d, 16-byte chunk j
+        uint4 u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = tid + i * TC_THREADS;
+            if (c < 2048) asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u[i].x), "=r"(u[i].y), "=r"(u[i].z), "=r"(u[i].w)
+                                       : "l"(reinterpret_cast<const uint4*>(p.rotation) + c));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = tid + i * TC_THREADS;
+            if (c < 2048) *reinterpret_cast<uint4*>(gbase + (tc_operand_addr(base + TcSmem::B_R, c >> 4, 8 * (c & 15)) - base)) = u[i];
+        }
+    };
+    if (p.static_rotation) stage_rotation();
     for (int i = tid; i < TC_BUCKETS; i += TC_THREADS) {
         // Bucket table over the rotated coordinate x.  The epilogue forms k = rne(4 x / w) in the low mantissa bits of
         // fma(x, 1 / w, 1.5 * 2^21) and takes bucket k >> 2 (modulo 256): bucket n holds x in [(n - 0.125) w, (n + 0.875) w],
@@ -351,6 +362,14 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctrl[2];
+    // (everything above is shared and tensor memory, and R where no kernel writes it: under the previous kernel's tail)
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!p.static_rotation) {
+        stage_rotation();
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
 
     const int vec_per_seq = p.T * p.Hkv;
     const int vec_per_kind = p.n_seq * vec_per_seq;
