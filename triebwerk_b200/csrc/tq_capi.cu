@@ -1334,7 +1334,7 @@ static bool engine_cluster_ok(const tq_engine* e, const void* q, const void* k, 
 
 // The layers l0 .. l0 + n - 1 of a step in one launch of the cluster form; q, k, v, out point at layer l0's [G][dim] blocks.
 static int engine_cluster_layers(tq_engine* e, int l0, int n, int split_layers, const void* q, const void* k, const void* v, void* out, bool chained,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, bool host_inputs = false) {
     const tq_engine::Layer& L = e->layers[l0];
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
     ClusterDecodeParams p{};
@@ -1352,7 +1352,9 @@ static int engine_cluster_layers(tq_engine* e, int l0, int n, int split_layers, 
     p.early = engine_reads_early(e, chained, s) ? 1 : 0;
     p.static_rotation = 1;
     if (split_layers > 1 && e->ev_attn[0]) cudaEventRecord(e->ev_attn[0], s);
-    const int r = launch_cluster_decode(e->kv_bits, p, n, split_layers, e->msl, s, use_pdl() && !(split_layers > 1 && e->ev_attn[0]));
+    const bool pdl = use_pdl() && !(split_layers > 1 && e->ev_attn[0]);
+    const int r = host_inputs ? launch_cluster_decode<true>(e->kv_bits, p, n, split_layers, e->msl, s, pdl)
+                              : launch_cluster_decode(e->kv_bits, p, n, split_layers, e->msl, s, pdl);
     if (split_layers > 1 && e->ev_attn[0]) cudaEventRecord(e->ev_attn[1], s);
     e->chain_ok = r == TQ_OK;
     e->chain_stream = s;
@@ -1473,14 +1475,15 @@ static bool engine_step_small(const tq_engine* e) {
 }
 
 // The layers l0 .. l0 + n - 1 of such a step; q, k, v, out point at layer l0's [G][dim] blocks.
-static int engine_cluster_step(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s) {
+static int engine_cluster_step(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s,
+                               bool host_inputs = false) {
     const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
     const int chunk = std::min(n, 65535 / e->G);  // layers per launch: the grid's third dimension
     for (int i = 0; i < n; i += chunk) {
         const bool chained = e->chain_ok;
         e->chain_ok = false;
         int r = engine_cluster_layers(e, l0 + i, std::min(chunk, n - i), e->shape.num_layers, (const char*)q + qb * i, (const char*)k + kb * i,
-                                      (const char*)v + kb * i, (char*)out + qb * i, chained, s);
+                                      (const char*)v + kb * i, (char*)out + qb * i, chained, s, host_inputs);
         if (r != TQ_OK) return r;
     }
     return TQ_OK;
@@ -1735,6 +1738,16 @@ static int engine_prefill_impl(tq_engine* e, int layer, int first_seq, int n_seq
     if (first_pos + T > cap) return TQ_ERR_CAPACITY;
     const tq_engine::Layer& L = e->layers[layer];
     if (e->kv_bits == 0) {
+        if (((((uintptr_t)k | (uintptr_t)v) & 15u)) == 0 && n_seq <= 65535) {
+            Fp16PromptParams p{};
+            p.ck = (__half*)L.k; p.cv = (__half*)L.v; p.k = (const __half*)k; p.v = (const __half*)v;
+            p.row_base = e->rb() ? e->rb() + first_seq : nullptr;
+            p.row0 = e->row0_eff(first_seq); p.seq_rows = e->msl;
+            p.first_pos = first_pos; p.T = T; p.kv_dim = e->kv_dim();
+            const long long pieces = (long long)T * e->kv_dim() / 8;
+            const dim3 grid((unsigned)std::min<long long>((pieces + 511) / 512, std::max(1, 8 * device_props().sm_count / n_seq)), (unsigned)n_seq);
+            return launch_kernel(fp16_prompt_write_kernel, grid, dim3(256), 0, cs(s), use_pdl(), p);
+        }
         const size_t row_bytes = (size_t)e->kv_dim() * 2;
         for (int i = 0; i < n_seq; ++i) {
             const long long row0 = e->row0_eff(first_seq + i);
@@ -1899,6 +1912,26 @@ int tq_engine_decode_step_host(tq_engine* e, const void* q_host, const void* k_h
     if (e->asleep || !e->arena || e->G == 0) return TQ_ERR_STATE;
     const int NL = e->shape.num_layers;
     const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
+    // A small step straight on the host buffers, where the device can reach them (pinned memory): every CTA fetches its 0.5 to
+    // 2.5 KB of inputs over the bus itself and writes its results there.  Copies cost 10 us of latency each, 40 us before the
+    // first kernel can start, and the launches of the groups that overlap them 15 % of the GPU (28 layers, 16 sequences x 2019
+    // tokens, 16/8 heads: 521 / 415 us; 1 x 300 tokens 264 / 38).
+    if (engine_step_small(e)) {
+        void* d[4] = {nullptr, nullptr, nullptr, nullptr};
+        const void* h[4] = {q_host, k_host, v_host, out_host};
+        bool reach = true;
+        for (int i = 0; i < 4 && reach; ++i) {
+            cudaPointerAttributes a{};
+            reach = cudaPointerGetAttributes(&a, h[i]) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer != nullptr;
+            d[i] = a.devicePointer;
+        }
+        if (!reach) cudaGetLastError();
+        if (reach && engine_cluster_ok(e, d[0], d[1], d[2], d[3])) {
+            const int r = engine_cluster_step(e, 0, NL, d[0], d[1], d[2], d[3], cs(s), true);
+            if (r != TQ_OK) return r;
+            return cuda_status(cudaStreamSynchronize(cs(s)));
+        }
+    }
     // The layers go in a few groups: the inputs of group c+1 are copied in (and the outputs of group c-1 copied out)
     // on two copy streams while the kernels of group c run on the caller's stream.
     constexpr int NC = tq_engine::HOST_STEP_CHUNKS;

@@ -91,6 +91,7 @@ __device__ __forceinline__ void st_async_f32x2(uint32_t addr, float a, float b, 
 }
 
 // Loads that stay behind griddepcontrol.wait (volatile: never moved across it), zero where `on` is 0.
+__device__ __forceinline__ uint4 lds128_if(uint32_t addr, bool on) { return on ? lds128(addr) : make_uint4(0u, 0u, 0u, 0u); }
 __device__ __forceinline__ uint4 ldg128_if(const void* src, bool on) {
     uint4 r;
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
@@ -143,7 +144,8 @@ inline size_t cd_smem_bytes(int bits, int heads) {
 }
 
 // MB: 16-token blocks per tile (2 for throughput, 1 where every warp gets a single tile anyway and its latency counts)
-template <int BITS, int MB>
+// HOST: q, new_k, new_v (and out) are pinned host memory: every byte of them is fetched once per CTA, not once per warp
+template <int BITS, int MB, bool HOST>
 __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const ClusterDecodeParams p_in) {
     extern __shared__ __align__(1024) uint8_t cd_smem[];
     ClusterDecodeParams p = p_in;
@@ -330,20 +332,42 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
     // ---- queries ----
     uint32_t qb[8][2];  // B fragments of the score product: lane (gl, t4) holds head gl, step j coordinates 32 t4 + 4 j ..
     uint4 qw[4];
+    const size_t new_at = ((size_t)g * p.Hkv + kvh) * HEAD_DIM;
+    const uint32_t in_s = warps_s;  // host inputs: [nh] queries, K, V, 256 bytes each, where the warps' results will be
+    if constexpr (HOST) {
+        const uint4* const q_src = reinterpret_cast<const uint4*>(p.q + (size_t)g * p.q_dim + (size_t)head0 * HEAD_DIM);
+        for (int i = tid; i < (nh + (owner ? 2 : 0)) * 16; i += CD_THREADS) {
+            const int r = i >> 4;
+            const uint4* src = r < nh ? q_src + i : reinterpret_cast<const uint4*>((r == nh ? p.new_k : p.new_v) + new_at) + (i & 15);
+            const uint4 u = ldg128_if(src, true);
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(in_s + (uint32_t)i * 16u), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w) : "memory");
+        }
+        __syncthreads();
+    }
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
+        const int c = BITS == 0 ? 4 * t4 + m : 4 * m + t4;
         const __half* src = p.q + (size_t)g * p.q_dim + (size_t)(head0 + gl) * HEAD_DIM;
-        qw[m] = ldg128_if(src + 8 * (BITS == 0 ? 4 * t4 + m : 4 * m + t4), gl < nh);
+        qw[m] = HOST ? lds128_if(in_s + (uint32_t)(gl * 256 + 16 * c), gl < nh) : ldg128_if(src + 8 * c, gl < nh);
     }
     // the CTA that owns the sequence's last tile also takes the new token: K and V are rows 8 and 9 of the rotation's A operand
     const int vec = tid >> 7, d = tid & 127;
-    const size_t new_at = ((size_t)g * p.Hkv + kvh) * HEAD_DIM;
     uint4 nw[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m)
-        nw[m] = ldg128_if((gl == 0 ? p.new_k : p.new_v) + new_at + 8 * (4 * m + t4), BITS != 0 && owner && gl < 2);
+    for (int m = 0; m < 4; ++m) {
+        const bool on = BITS != 0 && owner && gl < 2;
+        nw[m] = HOST ? lds128_if(in_s + (uint32_t)((nh + gl) * 256 + 16 * (4 * m + t4)), on)
+                              : ldg128_if((gl == 0 ? p.new_k : p.new_v) + new_at + 8 * (4 * m + t4), on);
+    }
     if (owner) {
-        const __half xh = ldg_half_if((vec == 0 ? p.new_k : p.new_v) + new_at + d, true);
+        __half xh;
+        if constexpr (HOST) {
+            unsigned short u;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(in_s + (uint32_t)((nh + vec) * 256 + 2 * d)));
+            xh = __ushort_as_half(u);
+        } else {
+            xh = ldg_half_if((vec == 0 ? p.new_k : p.new_v) + new_at + d, true);
+        }
         asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + CdSmem::RAW_OFF + 2u * (uint32_t)tid), "h"(__half_as_ushort(xh)) : "memory");
         if (!pos_ok && tid == 0 && p.status) atomicMax(p.status, ST_BAD_POSITION);
         if constexpr (BITS != 0) {  // sum of squares in the reference's order (tq_append.cuh)

@@ -386,9 +386,9 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
 }
 
 // One cluster per (sequence, KV head, block of 8 query heads): tq_decode_cluster.cuh.  `max_tokens`: rows a sequence may hold.
-template <int BITS, int MB>
+template <int BITS, int MB, bool HOST>
 inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int layers, cudaStream_t s, bool pdl) {
-    const void* kernel = (const void*)cluster_decode_kernel<BITS, MB>;
+    const void* kernel = (const void*)cluster_decode_kernel<BITS, MB, HOST>;
     int r = ensure_dynamic_smem(kernel, cd_smem_bytes(BITS, CD_HEADS), true);
     if (r != TQ_OK) return r;
     cudaLaunchConfig_t cfg{};
@@ -404,9 +404,10 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB>, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB, HOST>, p));
 }
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
+template <bool HOST = false>
 inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
     // As many CTAs per cluster as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch (two
     // share the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue: 8 sequences x 1023
@@ -414,10 +415,10 @@ inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int lay
     const long long clusters = (long long)p.G * split_layers * p.Hkv * p.head_blocks, blocks = (max_tokens + 15) / 16;
     int S = 1;
     while (S < CD_MAX_CLUSTER && (long long)S * CD_WARPS < blocks && clusters * S * 2 <= device_props().sm_count) S *= 2;
-    if (bits == 0) return launch_cluster_decode_t<0, 1>(p, S, layers, s, pdl);
+    if (bits == 0) return launch_cluster_decode_t<0, 1, HOST>(p, S, layers, s, pdl);
     const bool one = (long long)S * CD_WARPS >= blocks;  // a single 16-token tile per warp
-    if (bits == 4) return one ? launch_cluster_decode_t<4, 1>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2>(p, S, layers, s, pdl);
-    return one ? launch_cluster_decode_t<2, 1>(p, S, layers, s, pdl) : launch_cluster_decode_t<2, 2>(p, S, layers, s, pdl);
+    if (bits == 4) return one ? launch_cluster_decode_t<4, 1, HOST>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2, HOST>(p, S, layers, s, pdl);
+    return one ? launch_cluster_decode_t<2, 1, HOST>(p, S, layers, s, pdl) : launch_cluster_decode_t<2, 2, HOST>(p, S, layers, s, pdl);
 }
 
 __global__ void transpose_rotation_kernel(__half* dst, const __half* src, int* tickets = nullptr, int n_tickets = 0) {
