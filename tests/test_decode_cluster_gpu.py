@@ -26,6 +26,8 @@ D = 128
     (4, 16, 4, 512, [1, 31, 449, 512]),                # 4 CTAs, one of them for the new token
     (2, 8, 1, 2048, [1, 15, 16, 17, 1900]),            # 16 CTAs, 16-token tiles
     (4, 16, 8, 2112, [1801]),                          # 16 CTAs, several tiles per warp
+    (4, 16, 4, 1600, [1] * 17 + [17, 700, 1600]),      # 2 CTAs, two on an SM
+    (0, 16, 4, 640, [1] * 18 + [639, 640]),            # the same, fp16
     (4, 24, 2, 320, [97, 320]),                        # 12 query heads per KV head: two clusters share a KV head
     (2, 20, 1, 96, [95]),                              # 20: three
     (0, 40, 8, 384, [1, 16, 383]),                     # fp16 rows

@@ -24,14 +24,16 @@ static inline bool cluster_shape(const void* q, const void* out, const void* ck,
     return ((((uintptr_t)q | (uintptr_t)ck | (uintptr_t)cv | (uintptr_t)rotation) & 15u) | ((uintptr_t)out & 3u)) == 0 && q_dim % 8 == 0 &&
            G <= 65535 && (long long)Hkv * ((grp + CD_HEADS - 1) / CD_HEADS) <= 65535;
 }
-// Small batches go to it where the streaming kernels serve the layout too: rows of a layer's slots x KV heads (its time goes
-// by those, not by bytes) up to where the two forms cross.  Measured per layer, 8 KV heads, cluster / streaming form:
-// 4-bit 16 heads 4 x 1024 8.4 / 22 us, 16 x 1024 13 / 23, 4 x 4096 19 / 27, 64 x 1024 38 / 35; 2-bit the same within 10 %;
-// with 32 heads the lines cross near 64 x 1024; fp16 16 x 1024 20 / 25, 4 x 4096 27 / 25, 16 x 4096 66 / 61.
-// TQ_CLUSTER=0 keeps the streaming kernels for every layout they serve.
-static inline bool cluster_size(int bits, long long rows, int Hkv) {
+// Layers that are faster in it go to it where the streaming kernels serve the layout too (cluster_layer_faster).  TQ_CLUSTER=0
+// keeps the streaming kernels for every layout they serve.
+static inline bool cluster_on() {
     static const bool on = !(getenv("TQ_CLUSTER") && atoi(getenv("TQ_CLUSTER")) == 0);
-    return on && rows * Hkv <= (bits == 0 ? 131072 : 393216);
+    return on;
+}
+// Calls without an engine: the streaming kernels' rotated queries, table and clears are launches of their own there (packed 9 us,
+// fp16 3).
+static inline bool compat_cluster_size(int bits, int G, int H, int Hkv, int max_tokens) {
+    return cluster_on() && cluster_layer_faster(bits, G, Hkv, H / Hkv, (long long)G * max_tokens, max_tokens, bits ? 9.0 : 3.0);
 }
 
 extern "C" {
@@ -343,8 +345,9 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
     // The merge inside the kernel (by the last worker to arrive at a sequence, under the others' last tiles and the next layer's
     // start) or as a launch of its own: with more than 16 heads (two rounds) or few sequences, cut into many parts, that
     // worker is a layer's tail of ten microseconds and more.  Measured per layer, in the kernel / as a launch: 4-bit 16 heads
-    // 64 x 4096 80 / 84 us, 32 heads 88 / 87, 16 x 4096 43 / 34, 4 x 16384 61 / 42; 16 heads 1 x 16384 38 / 30.
-    const bool separate = num_heads > 16 || ctas * ATTN_GROUPS > 16 * G;
+    // 64 x 4096 80 / 84 us, 4 x 16384 61 / 42, 1 x 16384 38 / 30, 18 ragged x 6395 28 / 30; 32 heads 16 x 1500 34 / 26, 64 x 1500 41 / 40,
+    // 96 x 1500 61 / 64; over 4 KV heads, whose workers have four warps for the merge, 16 x 1500 38 / 22, 128 x 1500 62 / 59.
+    const bool separate = num_heads > 16 ? num_kv_heads == 4 || 2 * ctas * ATTN_GROUPS > 7 * G : ctas * ATTN_GROUPS > 36 * G;
     p.table_out = fw.w.tile_start;
     const int r = launch_attention(bits, tmK, tmV, p, ctas, s, pdl, separate ? 3 : 1);
     if (r != TQ_OK || !separate) return r;
@@ -587,7 +590,7 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
     int r = check_shape(G, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits, true);
     static const bool one_launch = !(getenv("TQ_FUSED") && atoi(getenv("TQ_FUSED")) == 0);
     if (r == TQ_OK && one_launch && cluster_shape(q, out, ck_q, cv_q, rotation, G, num_heads, num_kv_heads, q_dim) &&
-        (!fast_shape(num_heads, num_kv_heads, true) || cluster_size(bits, (long long)G * msl, num_kv_heads))) {
+        (!fast_shape(num_heads, num_kv_heads, true) || compat_cluster_size(bits, G, num_heads, num_kv_heads, msl))) {
         const bool args = out && q && ck_q && cv_q && k_norms && v_norms && rotation && pos;
         g_compat_status = args ? compat_cluster_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, pos, -1, msl, G, num_heads,
                                                           num_kv_heads, q_dim, bits, cs(s))
@@ -647,7 +650,7 @@ void launch_turbo_gqa_attention(const void* q, const uint8_t* ck_q, const uint8_
     int r = check_shape(1, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, bits, true);
     if (r == TQ_OK && (pos < 0 || pos >= msl)) r = TQ_ERR_CAPACITY;
     if (r == TQ_OK && cluster_shape(q, output, ck_q, cv_q, rotation, 1, num_heads, num_kv_heads, q_dim) &&
-        (!fast_shape(num_heads, num_kv_heads, true) || cluster_size(bits, pos + 1, num_kv_heads))) {
+        (!fast_shape(num_heads, num_kv_heads, true) || compat_cluster_size(bits, 1, num_heads, num_kv_heads, pos + 1))) {
         const bool args = output && q && ck_q && cv_q && k_norms && v_norms && rotation;
         g_compat_status = args ? compat_cluster_attention(output, q, ck_q, cv_q, k_norms, v_norms, rotation, nullptr, pos, msl, 1, num_heads,
                                                           num_kv_heads, q_dim, bits, cs(s))
@@ -731,7 +734,7 @@ void launch_gqa_attention_batch(void* out, const void* q, const void* ck, const 
     void* ws = nullptr;
     int r = check_shape(G, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, 0, false);
     if (r == TQ_OK && out && q && ck && cv && pos && cluster_shape(q, out, ck, cv, nullptr, G, num_heads, num_kv_heads, q_dim) &&
-        (!fast_shape(num_heads, num_kv_heads, false) || cluster_size(0, (long long)G * msl, num_kv_heads))) {
+        (!fast_shape(num_heads, num_kv_heads, false) || compat_cluster_size(0, G, num_heads, num_kv_heads, msl))) {
         g_compat_status = compat_cluster_attention(out, q, ck, cv, nullptr, nullptr, nullptr, pos, -1, msl, G, num_heads, num_kv_heads, q_dim,
                                                    0, cs(s));
         return;
@@ -756,7 +759,7 @@ void launch_gqa_attention(const void* q, const void* k_cache, const void* v_cach
     int r = check_shape(1, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, 0, false);
     if (r == TQ_OK && (pos < 0 || pos >= max_seq_len)) r = TQ_ERR_CAPACITY;
     if (r == TQ_OK && q && output && k_cache && v_cache && cluster_shape(q, output, k_cache, v_cache, nullptr, 1, num_heads, num_kv_heads, q_dim) &&
-        (!fast_shape(num_heads, num_kv_heads, false) || cluster_size(0, pos + 1, num_kv_heads))) {
+        (!fast_shape(num_heads, num_kv_heads, false) || compat_cluster_size(0, 1, num_heads, num_kv_heads, pos + 1))) {
         g_compat_status = compat_cluster_attention(output, q, k_cache, v_cache, nullptr, nullptr, nullptr, nullptr, pos, max_seq_len, 1,
                                                    num_heads, num_kv_heads, q_dim, 0, cs(stream));
         return;
@@ -1372,7 +1375,7 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     float* const f32 = e->out_f32 ? e->out_f32 + (size_t)layer * e->G * H * HEAD_DIM : nullptr;
     // Head layouts outside the streaming kernels', and small batches of any layout: the cluster form, one launch.
     if (engine_cluster_ok(e, q, k, v, out) &&
-        (!fast_shape(H, Hkv, e->kv_bits != 0) || cluster_size(e->kv_bits, e->total_rows, Hkv)))
+        (!fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, 0.0))))
         return engine_cluster_layers(e, layer, 1, 1, q, k, v, out, chained, cs(s));
     if (e->kv_bits == 0) {
         fp16_cache_write_kernel<<<e->G, 128, 0, cs(s)>>>((__half*)L.k, (__half*)L.v, (const __half*)k, (const __half*)v,
@@ -1457,21 +1460,23 @@ static bool engine_whole_step_ok(const tq_engine* e, const void* q, const void* 
 static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* out, cudaStream_t s, const tq_step_producer* prod);
 
 // Is a whole step of this engine's batch faster as one launch of the cluster form over all layers than in the whole-step form's
-// four launches?  Both times fit a line, in ns: a cluster (sequence, KV head, 8 query heads, layer) costs 24.5 and a cached row
-// and KV head 0.0346 in the one, a layer 3600, a sequence 1000 and a cached row and KV head 0.030 in the other, whose launches,
-// table and merges take 35 us at least (28 layers of 1 x 256 tokens 9 / 137 us, 4 x 4096 186 / 311, 16 x 1024 222 / 240, 16 x
-// 4096 647 / 595, 64 x 64 352 / 195).  fp16 caches have no whole-step form; up to 4 M rows and KV heads the one launch beats one
-// per layer (28 layers of 16 x 1024 338 / 596 us), above that the chunks of the streaming kernel balance better.
+// four launches?  Both times, in ns, are lines in what bounds them (1500 steps of 1 to 128 sequences x 64 to 16384 tokens, equal
+// and ragged, 4 to 36 layers): the one launch 2500 + 18 per cluster (sequence, KV head, layer; with 8 query heads 32, 15 in 2-bit,
+// whose tables are smaller) + 300 per tile of its longest warp + 0.038 per row and KV head, the four 22000 + 3500 per layer +
+// 0.032 per row and KV head (0.038 with 8 query heads in 2-bit).  28 layers of 1 x 256 tokens 9 / 137 us, 4 x 4096 186 / 311, 16 x
+// 1024 222 / 240, 16 x 4096 647 / 595, 64 x 64 352 / 195; 8 ragged layers of 95 x 6..433 187 / 140.  fp16 caches have no whole-step
+// form: the one launch saves 10 us a layer; a tile of its longest warp costs it 600 ns, a cached row and KV head 2 ps more.
 // It depends on the engine's batch alone: every call that runs a step, or part of one, takes the same form and gives the same bits.
 static bool engine_step_small(const tq_engine* e) {
     if (!e->fused || !e->whole_step || e->G > 65535) return false;
-    const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, NL = e->shape.num_layers;
+    const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, NL = e->shape.num_layers, heads = H / Hkv;
     if (!fast_shape(H, Hkv, e->kv_bits != 0)) return true;
-    static const bool on = !(getenv("TQ_CLUSTER") && atoi(getenv("TQ_CLUSTER")) == 0);
-    const double rows = (double)e->total_rows * Hkv * NL;
-    if (e->kv_bits == 0) return on && rows <= 4e6;
-    const double clusters = (double)e->G * Hkv * NL * ((H / Hkv + CD_HEADS - 1) / CD_HEADS);
-    return on && 24.5 * clusters + 0.0046 * rows < 35000.0 + 3600.0 * NL + 1000.0 * e->G;
+    if (!cluster_on()) return false;
+    const long long clusters = (long long)e->G * Hkv * NL;
+    const double tiles = ((e->msl + 15) / 16) / (double)(CD_WARPS * cluster_split(e->kv_bits, clusters, heads, e->msl));
+    if (e->kv_bits == 0) return 600.0 * tiles + 2.0 * clusters + 0.002 * (double)e->total_rows * Hkv * NL < 2000.0 + 10000.0 * NL;
+    const double per_cluster = heads <= 4 ? 18.0 : e->kv_bits == 4 ? 32.0 : 15.0, per_row = heads > 4 && e->kv_bits == 2 ? 0.0 : 0.006;
+    return per_cluster * clusters + per_row * (double)e->total_rows * Hkv * NL + 300.0 * tiles < 20000.0 + 3500.0 * NL;
 }
 
 // The layers l0 .. l0 + n - 1 of such a step; q, k, v, out point at layer l0's [G][dim] blocks.

@@ -406,17 +406,45 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
     cfg.numAttrs = pdl ? 2 : 1;
     return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB, HOST>, p));
 }
+// CTAs per cluster.  As many as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch: two share
+// the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue (8 sequences x 1023 tokens through
+// the launchers 24 us a layer with two, 19 with one).  Clusters of 4 and more leave some of a processing cluster's SMs over (136
+// of 148 serve fours, 128 eights): one cluster more than fits waits for a whole turn (72 clusters of 4 at two CTAs per SM 1.5
+// times the time of 72 of 2).  Where a warp goes through many tiles, more than the launch's fixed part costs, a second CTA per SM
+// hides the latency of the first one's loads: above 12 tiles 0.6 to 0.95 of the time (4 x 8192 tokens, 8 KV heads, 44 -> 28 us),
+// above 4 for fp16, whose rows are four times as long.  Not with more than 4 query heads per cluster in a packed mode: the warps'
+// partial results leave room for one CTA per SM there.
+inline int cluster_split(int bits, long long clusters, int heads, int max_tokens) {
+    const long long sms = device_props().sm_count, blocks = (max_tokens + 15) / 16;
+    auto fit = [&](int n) { return sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
+    int S = 1;
+    while (S < CD_MAX_CLUSTER && (long long)S * CD_WARPS < blocks && clusters * S * 2 <= fit(2 * S)) S *= 2;
+    if (S <= 4 && clusters * S * 8 <= 7 * sms && clusters * S * 2 <= 2 * fit(2 * S) && blocks > (bits ? 12 : 4) * CD_WARPS * S &&
+        (heads <= 4 || bits == 0))
+        S *= 2;
+    return S;
+}
+// Is one layer faster in the cluster form than in the streaming one?  Both times, in us, are lines in what bounds them, measured
+// over 1 to 128 sequences of 64 to 16384 tokens, equal and ragged, and 8 KV heads of 2 and 4 query heads, 4 of 8.  Packed: the
+// cluster form 4.6 + 0.4 per tile of its longest warp + 0.3 more per turn of the SMs + 0.023 per 1000 rows and KV heads + 0.007 to
+// 0.009 per cluster, the streaming form 17.7 + 0.030 per 1000 rows and KV heads + 0.4 per 1000 tokens of the longest sequence;
+// where the two are within 3 us it is the streaming form.  fp16: a tile costs the cluster form 1 us more than the streaming form's
+// share of it where there is one turn, less with more turns and with 8 query heads,
+// and that form starts 7 us later.  `extra`: us the streaming form's launches cost on top.
+inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, double extra) {
+    const long long clusters = (long long)G * Hkv, sms = device_props().sm_count;
+    const int S = cluster_split(bits, clusters, heads, max_tokens);
+    const double chain = ((max_tokens + 15) / 16) / (double)(S * CD_WARPS), turns = (double)((clusters * S + sms - 1) / sms);
+    if (bits == 0) return (heads > 4 ? 0.5 : 1.0) * chain < 7.0 + 1.5 * turns + extra;
+    return 0.4 * chain + 0.3 * chain * turns + 0.009 * clusters < 10.0 + 7e-6 * (double)rows * Hkv + 0.0004 * max_tokens + extra;
+}
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
 template <bool HOST = false>
 inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
-    // As many CTAs per cluster as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch (two
-    // share the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue: 8 sequences x 1023
-    // tokens through the launchers 24 us a layer with two, 19 with one).
-    const long long clusters = (long long)p.G * split_layers * p.Hkv * p.head_blocks, blocks = (max_tokens + 15) / 16;
-    int S = 1;
-    while (S < CD_MAX_CLUSTER && (long long)S * CD_WARPS < blocks && clusters * S * 2 <= device_props().sm_count) S *= 2;
+    const int blocks = (max_tokens + 15) / 16;
+    const int S = cluster_split(bits, (long long)p.G * split_layers * p.Hkv * p.head_blocks, std::min(CD_HEADS, p.H / p.Hkv), max_tokens);
     if (bits == 0) return launch_cluster_decode_t<0, 1, HOST>(p, S, layers, s, pdl);
-    const bool one = (long long)S * CD_WARPS >= blocks;  // a single 16-token tile per warp
+    const bool one = S * CD_WARPS >= blocks;  // a single 16-token tile per warp
     if (bits == 4) return one ? launch_cluster_decode_t<4, 1, HOST>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2, HOST>(p, S, layers, s, pdl);
     return one ? launch_cluster_decode_t<2, 1, HOST>(p, S, layers, s, pdl) : launch_cluster_decode_t<2, 2, HOST>(p, S, layers, s, pdl);
 }
