@@ -49,16 +49,34 @@ def test_prefill_attention_edges(bits, H, Hkv, n, T, msl):
 
 
 def test_prompts_pass_through_the_scratch_in_groups():
-    """20 prompts of 1000 tokens: more than the 16384 tokens that fit the fp16 scratch at a time."""
-    H, Hkv, n, T = 8, 4, 20, 1000
+    """40 prompts of 1000 tokens x 4 KV heads: more than the 131072 rows of one KV head that fit the fp16 scratch at a time."""
+    H, Hkv, n, T = 8, 4, 40, 1000
     gen = torch.Generator(device="cuda").manual_seed(5)
     k, v = (torch.randn(n, T, Hkv * D, generator=gen, device="cuda").half() for _ in range(2))
     q = torch.randn(n, T, H * D, generator=gen, device="cuda").half()
     eng = tq.Engine(1024, 4, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
     eng.alloc_batch(n, 1024)
     together = eng.prefill_layer_batch(0, 0, q, k, v)
-    for i in (0, 15, 16, 19):
+    for i in (0, 31, 32, 39):
         one = eng.prefill_layer(0, i, q[i], k[i], v[i])
         # (one prompt alone has one query block per CTA, the batch two: another order of summation)
         assert torch.allclose(together[i].float(), one.float(), atol=1e-3, rtol=2e-3)
     assert eng.status() == 0
+
+
+@pytest.mark.parametrize("bits", [4, 2])
+def test_long_prompt_passes_through_the_scratch_by_kv_heads(bits):
+    """16500 tokens x 8 KV heads do not fit the scratch as a whole: 4 heads, then 4.  The launcher, whose scratch holds the prompt,
+    computes every column in the same order: the same bits."""
+    H, Hkv, T, msl = 16, 8, 16500, 16512
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    k, v = (torch.randn(T, Hkv * D, generator=gen, device="cuda").half() for _ in range(2))
+    q = torch.randn(T, H * D, generator=gen, device="cuda").half()
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(2, msl)
+    got = eng.prefill_layer(0, 1, q, k, v)
+    ck, cv, kn, vn = (t[msl:] for t in eng.layer_cache(0))
+    want = torch.empty_like(q)
+    tq.ops.launch_turbo_gqa_prefill_attention(want, q, ck, cv, kn, vn, tq.ops.rotation_matrix().cuda(), None, T, msl, H, Hkv, D, H * D, Hkv * D, bits)
+    assert eng.status() == 0
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))

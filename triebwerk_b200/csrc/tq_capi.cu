@@ -944,9 +944,9 @@ static size_t engine_carve(tq_engine* e, char* base, int G, int msl, long long r
     const size_t qb = (size_t)e->shape.num_layers * G * e->q_dim() * 2;
     const size_t kb = (size_t)e->shape.num_layers * G * e->kv_dim() * 2;
     size_t oq = bump(off, qb), okk = bump(off, kb), ovv = bump(off, kb), oo = bump(off, qb);
-    // prompts on their way through the prefill attention as fp16 rows: one full slot, or several up to 16384 tokens together
-    const size_t pf_tokens = std::max<size_t>((size_t)msl, std::min<size_t>((size_t)rows, 16384));
-    const size_t pf_bytes = e->kv_bits ? prefill_scratch_bytes((int)pf_tokens, e->shape.num_kv_heads) : 0;
+    // prompts on their way through the prefill attention as fp16 rows: 16384 tokens of 8 KV heads whatever the slots hold (64 MiB:
+    // half of L2, where the attention reads them again); longer prompts pass through it some KV heads at a time
+    const size_t pf_bytes = e->kv_bits ? prefill_scratch_bytes(131072, 1) : 0;
     size_t opf = bump(off, pf_bytes);
     if (assign) {
         e->prefill_scratch = e->kv_bits ? base + opf : nullptr;
@@ -1903,6 +1903,12 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
         ap.rotation = (const __half*)e->d_rotation;
     }
     ap.status = (int*)e->workspace;
+    if (e->kv_bits != 0 && prefill_scratch_bytes(T, 1) > e->prefill_scratch_bytes) {  // not even one KV head of such a prompt fits
+        std::lock_guard<std::recursive_mutex> compat_lock(compat_mutex());
+        void* ws = nullptr;
+        r = compat_workspace(prefill_scratch_bytes(T, 1), &ws, cs(s));
+        return r != TQ_OK ? r : launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, ws, prefill_scratch_bytes(T, 1), cs(s));
+    }
     return launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s));
 }
 

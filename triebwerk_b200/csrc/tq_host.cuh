@@ -540,64 +540,72 @@ inline size_t prefill_scratch_bytes(int T, int Hkv) {
     return 2 * align_up((size_t)T * Hkv * HEAD_DIM * sizeof(__half), 256) + align_up((size_t)2 * Hkv * prefill_t_pad(T) * sizeof(float), 256);
 }
 // Causal prefill attention.  `total_rows`: rows of the arrays ck and cv point into (from where they point); `scratch`: packed
-// modes, device memory for at least one prompt (prompts go through it in groups).
+// modes, device memory for at least one KV head of one prompt (prompts go through it in groups; one that is too long for it as a
+// whole, some of its KV heads at a time).
 inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long total_rows, void* scratch, size_t scratch_bytes, cudaStream_t s) {
     p.grp = p.H / p.Hkv;
     if (p.n_seq <= 0) p.n_seq = 1;
     if (p.T <= 0) return TQ_OK;
-    const int qt = PFT_ROWS / p.grp, kv_dim = p.Hkv * HEAD_DIM;
-    int group = p.n_seq;  // prompts per launch (fp16 caches: all of them)
+    const int qt = PFT_ROWS / p.grp;
+    int group = p.n_seq, heads = p.Hkv;  // prompts and KV heads per launch (fp16 caches: all of them)
     if (bits != 0) {
-        const size_t one = prefill_scratch_bytes(p.T, p.Hkv);
-        if (!scratch || scratch_bytes < one) return TQ_ERR_WORKSPACE;
-        group = (int)std::min<long long>(p.n_seq, (long long)(scratch_bytes / one));
+        if (!scratch) return TQ_ERR_WORKSPACE;
+        while (heads > 0 && prefill_scratch_bytes(p.T, heads) > scratch_bytes) --heads;
+        if (heads == 0) return TQ_ERR_WORKSPACE;
+        const int passes = (p.Hkv + heads - 1) / heads;
+        heads = (p.Hkv + passes - 1) / passes;  // of about the same size
+        group = (int)std::min<long long>(p.n_seq, (long long)(scratch_bytes / prefill_scratch_bytes(p.T, heads)));
     }
     for (int s0 = 0; s0 < p.n_seq; s0 += group) {
-        PrefillAttnParams a = p;
-        a.n_seq = std::min(group, p.n_seq - s0);
-        a.q = p.q + (size_t)s0 * p.T * p.q_tok_stride;
-        a.out = p.out + (size_t)s0 * p.T * p.q_dim;
-        CUtensorMap tmK{}, tmV{}, tmQ{}, tmR{};
-        int r = make_prefill_query_map(&tmQ, a.q, (long long)a.n_seq * p.T, p.H, p.grp, qt, p.q_tok_stride);
-        if (r != TQ_OK) return r;
-        if (bits == 0) {
-            r = make_prefill_rows_map(&tmK, p.ck, total_rows, kv_dim);
-            if (r == TQ_OK) r = make_prefill_rows_map(&tmV, p.cv, total_rows, kv_dim);
-        } else {
-            DequantParams d{};
-            d.ck = p.ck; d.cv = p.cv; d.kn = p.kn; d.vn = p.vn;
-            d.row_base = p.row_base ? p.row_base + s0 : nullptr;
-            d.seq_rows = p.seq_rows; d.T = p.T; d.t_pad = prefill_t_pad(p.T); d.Hkv = p.Hkv;
-            if (!p.row_base) {
-                const size_t skip = (size_t)s0 * p.seq_rows;
-                d.ck += skip * kv_dim / (bits == 4 ? 2 : 4); d.cv += skip * kv_dim / (bits == 4 ? 2 : 4);
-                d.kn += skip * p.Hkv; d.vn += skip * p.Hkv;
+        for (int h0 = 0; h0 < p.Hkv; h0 += heads) {
+            PrefillAttnParams a = p;
+            a.n_seq = std::min(group, p.n_seq - s0);
+            a.Hkv = std::min(heads, p.Hkv - h0);
+            a.H = a.Hkv * p.grp;
+            const size_t col = (size_t)h0 * p.grp * HEAD_DIM;
+            const int kv_dim = a.Hkv * HEAD_DIM;
+            a.q = p.q + (size_t)s0 * p.T * p.q_tok_stride + col;
+            a.out = p.out + (size_t)s0 * p.T * p.q_dim + col;
+            CUtensorMap tmK{}, tmV{}, tmQ{}, tmR{};
+            int r = make_prefill_query_map(&tmQ, a.q, (long long)a.n_seq * p.T, a.H, p.grp, qt, p.q_tok_stride);
+            if (r != TQ_OK) return r;
+            if (bits == 0) {
+                r = make_prefill_rows_map(&tmK, p.ck, total_rows, kv_dim);
+                if (r == TQ_OK) r = make_prefill_rows_map(&tmV, p.cv, total_rows, kv_dim);
+            } else {
+                DequantParams d{};
+                const size_t rows = p.row_base ? 0 : (size_t)s0 * p.seq_rows, head_bytes = bits == 4 ? 64 : 32;
+                d.ck = p.ck + (rows * p.Hkv + h0) * head_bytes; d.cv = p.cv + (rows * p.Hkv + h0) * head_bytes;
+                d.kn = p.kn + rows * p.Hkv + h0; d.vn = p.vn + rows * p.Hkv + h0;
+                d.row_base = p.row_base ? p.row_base + s0 : nullptr;
+                d.seq_rows = p.seq_rows; d.T = p.T; d.t_pad = prefill_t_pad(p.T); d.Hkv = a.Hkv; d.row_heads = p.Hkv;
+                const size_t rows16 = align_up((size_t)a.n_seq * p.T * kv_dim * sizeof(__half), 256);
+                d.k16 = (__half*)scratch; d.v16 = (__half*)((char*)scratch + rows16); d.norms = (float*)((char*)scratch + 2 * rows16);
+                const long long pieces = 2ll * p.T * a.Hkv * 16;
+                const dim3 grid((unsigned)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count), (unsigned)a.n_seq);
+                r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4>, grid, dim3(256), 0, s, true, d)
+                              : launch_kernel(dequantize_rows_kernel<2>, grid, dim3(256), 0, s, true, d);
+                a.ck = (const uint8_t*)d.k16; a.cv = (const uint8_t*)d.v16; a.norms = d.norms; a.t_pad = d.t_pad;
+                a.row_base = nullptr;
+                a.seq_rows = p.T;
+                if (r == TQ_OK) r = make_prefill_rows_map(&tmR, p.rotation, HEAD_DIM, HEAD_DIM);
+                if (r == TQ_OK) r = make_prefill_rows_map(&tmK, d.k16, (long long)a.n_seq * p.T, kv_dim);
+                if (r == TQ_OK) r = make_prefill_rows_map(&tmV, d.v16, (long long)a.n_seq * p.T, kv_dim);
             }
-            const size_t rows16 = align_up((size_t)a.n_seq * p.T * kv_dim * sizeof(__half), 256);
-            d.k16 = (__half*)scratch; d.v16 = (__half*)((char*)scratch + rows16); d.norms = (float*)((char*)scratch + 2 * rows16);
-            const long long pieces = 2ll * p.T * p.Hkv * 16;
-            const dim3 grid((unsigned)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count), (unsigned)a.n_seq);
-            r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4>, grid, dim3(256), 0, s, true, d)
-                          : launch_kernel(dequantize_rows_kernel<2>, grid, dim3(256), 0, s, true, d);
-            a.ck = (const uint8_t*)d.k16; a.cv = (const uint8_t*)d.v16; a.norms = d.norms; a.t_pad = d.t_pad;
-            a.row_base = nullptr;
-            a.seq_rows = p.T;
-            if (r == TQ_OK) r = make_prefill_rows_map(&tmR, p.rotation, HEAD_DIM, HEAD_DIM);
-            if (r == TQ_OK) r = make_prefill_rows_map(&tmK, d.k16, (long long)a.n_seq * p.T, kv_dim);
-            if (r == TQ_OK) r = make_prefill_rows_map(&tmV, d.v16, (long long)a.n_seq * p.T, kv_dim);
+            if (r != TQ_OK) return r;
+            // Two query blocks per CTA, which share every tile, once there are enough of them for the GPU; below that twice the
+            // CTAs with one block each, whose two slots take the even and the odd tiles.  Per layer, one block / two (8 KV heads,
+            // 4-bit): 2048 tokens 16 heads (128 pairs of blocks) 70 / 83 us, 32 heads (256) 117 / 104, 8192 tokens 16 heads (512)
+            // 449 / 439.
+            const long long blocks2 = (p.T + 2 * qt - 1) / (2 * qt), cols = (long long)a.Hkv * a.n_seq;
+            const int mt = 4 * blocks2 * cols >= 5ll * device_props().sm_count ? 2 : 1;
+            const long long blocks = mt == 2 ? blocks2 : (p.T + qt - 1) / qt;
+            if (cols > 2147483647ll || blocks > 65535) return TQ_ERR_CAPACITY;
+            dim3 grid((unsigned)cols, (unsigned)blocks);
+            if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
+            else r = mt == 2 ? launch_prefill_fa_t<false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
+            if (r != TQ_OK) return r;
         }
-        if (r != TQ_OK) return r;
-        // Two query blocks per CTA, which share every tile, once there are enough of them for the GPU; below that twice the CTAs
-        // with one block each, whose two slots take the even and the odd tiles.  Per layer, one block / two (8 KV heads, 4-bit):
-        // 2048 tokens 16 heads (128 pairs of blocks) 70 / 83 us, 32 heads (256) 117 / 104, 8192 tokens 16 heads (512) 449 / 439.
-        const long long blocks2 = (p.T + 2 * qt - 1) / (2 * qt), cols = (long long)p.Hkv * a.n_seq;
-        const int mt = 4 * blocks2 * cols >= 5ll * device_props().sm_count ? 2 : 1;
-        const long long blocks = mt == 2 ? blocks2 : (p.T + qt - 1) / qt;
-        if (cols > 2147483647ll || blocks > 65535) return TQ_ERR_CAPACITY;
-        dim3 grid((unsigned)cols, (unsigned)blocks);
-        if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
-        else r = mt == 2 ? launch_prefill_fa_t<false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
-        if (r != TQ_OK) return r;
     }
     return TQ_OK;
 }

@@ -90,7 +90,8 @@ struct DequantParams {
     __half* k16;
     __half* v16;
     float* norms;
-    int T, t_pad, Hkv;
+    int T, t_pad, Hkv;           // Hkv: heads of this pass; ck, cv, kn, vn point at the first one's
+    int row_heads;               // heads per row of the cache
 };
 template <int BITS>
 __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParams p) {
@@ -112,13 +113,14 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * n; i += (long long)gridDim.x * 256) {
         const bool is_v = i >= n;
         const long long w = is_v ? i - n : i;
+        const long long at = row0 * (p.row_heads * 16) + (p.row_heads == p.Hkv ? w : w / words * (p.row_heads * 16) + w % words);
         uint4 u;
         if (BITS == 4) {
-            const uint32_t c = *(reinterpret_cast<const uint32_t*>(is_v ? p.cv : p.ck) + row0 * words + w);
+            const uint32_t c = *(reinterpret_cast<const uint32_t*>(is_v ? p.cv : p.ck) + at);
             u.x = lut[(c & 0xffu) * 8 + copy]; u.y = lut[((c >> 8) & 0xffu) * 8 + copy];
             u.z = lut[((c >> 16) & 0xffu) * 8 + copy]; u.w = lut[(c >> 24) * 8 + copy];
         } else {
-            const uint32_t c = *(reinterpret_cast<const unsigned short*>(is_v ? p.cv : p.ck) + row0 * words + w);
+            const uint32_t c = *(reinterpret_cast<const unsigned short*>(is_v ? p.cv : p.ck) + at);
             u.x = lut[(c & 0xfu) * 8 + copy]; u.y = lut[((c >> 4) & 0xfu) * 8 + copy];
             u.z = lut[((c >> 8) & 0xfu) * 8 + copy]; u.w = lut[(c >> 12) * 8 + copy];
         }
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
         const bool is_v = i >= m;
         const long long w = is_v ? i - m : i;
         const int t = (int)(w / p.Hkv), h = (int)(w - (long long)t * p.Hkv);
-        const float x = t < p.T ? __half2float((is_v ? p.vn : p.kn)[(row0 + t) * p.Hkv + h]) : 0.0f;
+        const float x = t < p.T ? __half2float((is_v ? p.vn : p.kn)[(row0 + t) * p.row_heads + h]) : 0.0f;
         p.norms[(((long long)seq * p.Hkv + h) * 2 + (is_v ? 1 : 0)) * p.t_pad + t] = x;
     }
 }
