@@ -20,7 +20,9 @@
 //     contiguous bulk copies; completion on one mbarrier per stage.  (An optional cp.async.bulk.prefetch.L2 of tiles
 //     further ahead exists, TQ_ATTN_L2_AHEAD; it is off by default because it did not pay on B200.)  The last warp of the
 //     worker to finish a stage (one shared-memory atomic per warp and tile) re-arms it: nobody waits for a slower
-//     warp.  With the swizzle, and with the eight tokens of a score block taken in the order 0,5,2,7,4,1,6,3, every
+//     warp.  In the whole-step form a copy warp does, which the warps tell through a barrier per part: without the list's
+//     cursor, the atomics and the fences 664 -> 630 warp instructions per warp and tile (28 layers of 64 x 4096 tokens
+//     2007 -> 1863 us, ragged 128 sequences 2319 -> 2135; shared memory 74 % busy, issue slots 64 %).  With the swizzle, and with the eight tokens of a score block taken in the order 0,5,2,7,4,1,6,3, every
 //     16-, 8- and 4-byte read of packed codes is free of bank conflicts.
 //   * Codes are turned into fp16 centroids one BYTE at a time (2 codes for 4-bit, 4 for 2-bit) through a
 //     shared-memory table with one private column per lane (bank-conflict free); the table sits at shared
@@ -374,8 +376,13 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
 // MODE 0: queries pre-rotated and tile table built by append_rotate_kernel; 1: the kernel builds its table, rotates the
 // queries, optionally appends the step's token (one launch per layer and step); 2: whole-step form, see AttnParams; 3: as 1,
 // but the partials are only published (merge_partials_kernel<16> follows).
+// The whole-step form has one warp more, which issues the copies of both workers.  With 16 warps at work it is a warpgroup more:
+// the launch brings 640 x 96 registers, of which the workers' warps take 112 each and the copy warps keep 32.
+template <int HKV, int MODE>
+constexpr int attn_threads() { return ATTN_GROUPS * 32 * HKV + (MODE == 2 ? (HKV == 8 ? 128 : 32) : 0); }
+constexpr int ATTN_REGS_WORK = 112, ATTN_REGS_COPY = 32;
 template <int BITS, int HKV, int MODE>
-__global__ void __launch_bounds__(ATTN_GROUPS * 32 * HKV, 1)
+__global__ void __launch_bounds__(attn_threads<HKV, MODE>(), 1)
 decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const AttnParams p) {
     using Geo = AttnGeom<BITS>;
@@ -388,7 +395,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     const int lane = tid & 31;
     const int warp = tid >> 5;
     constexpr int Hkv = HKV;  // compile time: row pitches, tile sizes and norm strides fold into immediates
-    const int group = warp / Hkv;        // worker within the CTA
+    // whole-step form: lane 0 (1) of the copy warp keeps the ring of worker 0 (1) filled
+    const bool copier = PERSIST && warp >= ATTN_GROUPS * Hkv;
+    const int group = copier ? (lane & 1) : warp / Hkv;  // worker within the CTA
     const int head = warp - group * Hkv; // KV head of this warp
     const int gl = lane >> 2;            // mma "group id": token (K side), coordinate row (V side), head (S layout)
     const int t4 = lane & 3;             // mma "thread in group"
@@ -426,6 +435,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     // and handed back separately, so that a stage's K half is on its way again while its V half is still being read
     const uint32_t bar0 = a_base + RegionA::BAR_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 16u);
     const uint32_t cnt0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 8u);
+    const uint32_t ebar0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 16u);  // whole-step form: "part handed back" barriers
     const uint32_t ctrl_s = a_base + RegionA::CTRL_OFF + (uint32_t)group * 16u;
     const uint32_t merge_s = a_base + RegionA::MERGE_OFF + (uint32_t)group * RegionA::MERGE_GROUP_BYTES;
 
@@ -457,7 +467,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     if (gtid == 0) {
         for (int s = 0; s < 2 * ATTN_MAX_STAGES; ++s) {
             mbar_init(bar0 + 8u * s, 1);
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(cnt0 + 4u * s), "r"(0u) : "memory");
+            if (PERSIST) mbar_init(ebar0 + 8u * s, Hkv);
+            else asm volatile("st.shared.u32 [%0], %1;" ::"r"(cnt0 + 4u * s), "r"(0u) : "memory");
         }
         if (PERSIST) mbar_init(a_base + 320u + 8u * (uint32_t)group, 1);
         fence_mbar_init();
@@ -526,7 +537,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         p.table_out[G + 1] = W;
         p.table_out[G + 2] = (int)N;
     }
-    if (wid >= W) return;  // uniform for the worker; no CTA-wide barrier follows
+    if (wid >= W && !copier) return;  // uniform for the worker; no CTA-wide barrier follows
     // The flat list is cut in UNITS: a tile is one unit, except the last tile of a sequence, which counts 1 + A units
     // for what a sequence costs beside its tiles (A = p.app_weight, in tiles): in the fused form its owner also appends
     // the sequence's new token; in the prefill form sequences are short and their partials and merges weigh as much
@@ -550,7 +561,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         int g_hi;
         lo = tiles_before((long long)wid * U / W, &g);
         hi = tiles_before((long long)(wid + 1) * U / W, &g_hi);
-        if (lo >= hi) return;  // the worker's units all lie inside an append's share: nothing to do
+        if (lo >= hi && !copier) return;  // the worker's units all lie inside an append's share: nothing to do
     } else {
         lo = (long long)wid * N / W;
         hi = (long long)(wid + 1) * N / W;
@@ -567,6 +578,10 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         }
     }
 
+    if (copier && (lane >= ATTN_GROUPS || wid >= W || lo >= hi)) {  // nothing to copy (it returns further down)
+        g = 0;
+        lo = hi = 0;
+    }
     // ---- load cursor over the flat tile list (warp-uniform, advanced in step by every warp of the worker) ----
     // Tile counts and row numbers fit 32 bits (the host refuses caches of 2^31 rows or more).
     const int lo_i = (int)lo, hi_i = (int)hi;
@@ -670,8 +685,45 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             }
         }
     };
-    if (PERSIST && gtid == 0 && loads_on) issue_queries(0, g);
-    if constexpr (FUSED) {
+    if constexpr (PERSIST) {
+        if (copier) {
+            // One thread per worker walks the worker's list and re-arms every part as soon as all its warps have handed it back.
+            // (When the last warp to hand a part back did this itself, the cursor over the list, the counter's atomic and the
+            // fences were in all 16 warps' instruction streams.)  Its own wait is bounded like theirs, and it leaves only when
+            // the copies it issued have landed.
+            if constexpr (HKV == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ATTN_REGS_COPY));
+            if (warp > ATTN_GROUPS * Hkv || lo >= hi) return;
+            int n = 0;
+            bool stuck = false;
+            for (; cursor_more() && loads_on && !stuck; ++n, cursor_advance()) {
+                const int st = n % S;
+                const uint32_t par = ((uint32_t)(n / S) & 1u) ^ 1u;  // of the hand-back that this tile's copies wait for
+                for (int part = 0; part < 2 && !stuck; ++part) {
+                    if (n >= S) {
+                        uint32_t ok = 0;
+                        for (uint32_t it = 0; it < (1u << 23) && !ok; ++it) {
+                            ok = mbar_test_wait(ebar0 + 16u * (uint32_t)st + 8u * (uint32_t)part, par);
+                            if (!ok) __nanosleep(64);
+                        }
+                        if (!ok) {
+                            stuck = true;
+                            atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
+                            break;
+                        }
+                    }
+                    issue_part(cl_row, st, part, cl_layer);
+                }
+                if (!stuck) prefetch_ahead(cl_row, cl_tile, cl_gend);
+            }
+            for (int m = n > S ? n - S : 0; m < n; ++m) {
+                mbar_wait_bounded(bar0 + 16u * (uint32_t)(m % S), (uint32_t)(m / S) & 1u, 1u << 16);
+                mbar_wait_bounded(bar0 + 16u * (uint32_t)(m % S) + 8u, (uint32_t)(m / S) & 1u, 1u << 16);
+            }
+            return;
+        }
+        if constexpr (HKV == 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ATTN_REGS_WORK));
+        if (gtid == 0 && loads_on) issue_queries(0, g);
+    } else if constexpr (FUSED) {
         // The new token of a sequence is appended by the worker that owns the sequence's last tile (the only tile the
         // row can be in), before that tile is fetched.  The rotation of the sequence's 2 * Hkv head vectors runs on the
         // tensor cores (16 rows x 128 x 128, fp16 hi/lo operands as in the prefill kernel); a coordinate within
@@ -981,13 +1033,13 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     long long stamp_last = clock64();
 #endif
     for (int layer = 0; layer < n_layers; ++layer) {  // (one pass unless this is the whole-step form)
-    long long tile = lo;
+    int tile = lo_i;
     g = g_lo;
-    while (tile < hi) {
+    while (tile < hi_i) {
         // ================= one segment: tiles [tile, seg_end) of sequence g =================
-        const long long ts_g = ts[g];
-        const long long ts_g1 = ts[g + 1];
-        const long long seg_end = hi < ts_g1 ? hi : ts_g1;
+        const int ts_g = ts[g];
+        const int ts_g1 = ts[g + 1];
+        const int seg_end = hi_i < ts_g1 ? hi_i : ts_g1;
         const int pos = p.positions ? p.positions[g] : p.pos_value;
         const int L = (pos < 0 ? 0 : pos) + 1;
         TQ_STAMP(8);   // loop tail + publishing of the previous segment + this segment's table / position reads
@@ -1031,7 +1083,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             TQ_STAMP(11);  // barrier of the worker's warps
             if (gtid == 0 && !dead && loads_on) {
                 fence_proxy_async_smem();
-                if (seg_end < hi) issue_queries(layer, g + 1);
+                if (seg_end < hi_i) issue_queries(layer, g + 1);
                 else if (layer + 1 < n_layers) issue_queries(layer + 1, g_lo);
             }
         } else if constexpr (SEPARATE) {
@@ -1049,7 +1101,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #pragma unroll
                 for (int m = 0; m < 4; ++m) bq[nbi][m] = __ldg(rr + 4 * m);
             }
-            if (tile != lo) group_barrier(group, gthreads);  // every warp has taken the previous sequence's fragments
+            if (tile != lo_i) group_barrier(group, gthreads);  // every warp has taken the previous sequence's fragments
             const uint4* const q_src = reinterpret_cast<const uint4*>(p.new_q + (size_t)g * p.q_dim);
             for (int i = gtid; i < p.H * 16; i += gthreads) {
                 const uint4 u = __ldg(q_src + i);
@@ -1186,13 +1238,13 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         for (int b = 0; b < 8; ++b) { acc[b][0] = acc[b][1] = acc[b][2] = acc[b][3] = 0.0f; }
 
         for (; tile < seg_end; ++tile) {
-            const int t0 = (int)(tile - ts_g) * TILE_TOKENS;
+            const int t0 = (tile - ts_g) * TILE_TOKENS;
             const bool full = t0 + TILE_TOKENS <= L;  // warp-uniform: no token of the tile is masked
             const int s = BITS == 2 ? s_idx : (consumed & (S - 1));
             const uint32_t parity = BITS == 2 ? s_par : ((uint32_t)(consumed >> s_log) & 1u);
             // the tile that takes this stage's place (warp-uniform; every warp of the worker advances the cursor in step)
             const int next_row = cl_row, next_tile = cl_tile, next_gend = cl_gend, next_layer = cl_layer;
-            const bool more = cursor_more();
+            const bool more = !PERSIST && cursor_more();
             if (more) cursor_advance();
             // Wait for one part (0: K codes and norms, 1: V codes and norms) of the stage.  Returns 0 at run time, as a
             // value PRODUCED by the wait: the part's loads take it into their address and so cannot move above the wait.
@@ -1200,13 +1252,16 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 uint32_t token = 0;
                 if (!dead && loads_on) {
                     const uint32_t bar = bar0 + 16u * s + 8u * part;
-                    uint32_t ok = 0;
-                    for (uint32_t it = 0; it < (1u << 14) && !ok; ++it) ok = mbar_try_wait_hint(bar, parity, 20000u);
+                    uint32_t ok = mbar_try_wait_hint(bar, parity, 20000u);
                     if (!ok) {
-                        dead = true;
-                        if (lane == 0) atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
+                        for (uint32_t it = 0; it < (1u << 14) && !ok; ++it) ok = mbar_try_wait_hint(bar, parity, 20000u);
+                        if (!ok) {  // (lane by lane: one that gave up computes on, on whatever is there, and waits for nothing more)
+                            dead = true;
+                            atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
+                            ok = 1u;
+                        }
                     }
-                    dead = __any_sync(0xffffffffu, dead);
+                    __syncwarp();
                     token = ok ^ 1u;
                 }
                 return token;
@@ -1215,6 +1270,10 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             // last warp of the worker to get here re-arms the part with the same part of the tile S ahead; nobody waits.
             auto release_part = [&](int part) {
                 __syncwarp();
+                if constexpr (PERSIST) {
+                    if (lane == 0) mbar_arrive(ebar0 + 16u * (uint32_t)s + 8u * (uint32_t)part);
+                    return;
+                }
                 if (lane == 0 && more && !dead && loads_on) {
                     __threadfence_block();  // this warp's reads of the part are ordered before the hand-over below
                     const uint32_t cnt = cnt0 + 8u * s + 4u * part;
@@ -1235,7 +1294,6 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 TQ_STAMP(0);
                 const uint32_t tokK = wait_part(0);
                 TQ_STAMP(1);
-                if (dead) return;
                 const uint32_t kt = stage_addr(s) + tokK;
                 const uint32_t kns = kt + 2u * code_tile + (uint32_t)head * 2u;
 
@@ -1303,13 +1361,14 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 }
                 float mx0 = fmaxf(fmaxf(sv[0][0], sv[1][0]), fmaxf(sv[2][0], sv[3][0]));
                 float mx1 = fmaxf(fmaxf(sv[0][1], sv[1][1]), fmaxf(sv[2][1], sv[3][1]));
+                // (the maximum over the row lanes is only looked for in the few tiles that hold a new one)
+                if (__any_sync(0xffffffffu, mx0 > m_run[0] || mx1 > m_run[1])) {
 #pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-                }
-                const float mn0 = fmaxf(m_run[0], mx0), mn1 = fmaxf(m_run[1], mx1);
-                if (__any_sync(0xffffffffu, mn0 > m_run[0] || mn1 > m_run[1])) {
+                    for (int o = 4; o < 32; o <<= 1) {
+                        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+                        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+                    }
+                    const float mn0 = fmaxf(m_run[0], mx0), mn1 = fmaxf(m_run[1], mx1);
                     // 1 when unchanged, 0 at the first tile; the accumulators of heads 2*t4, 2*t4 + 1 live in this very lane
                     const float c0 = ex2_approx(m_run[0] - mn0), c1 = ex2_approx(m_run[1] - mn1);
                     l_run[0] *= c0;
@@ -1342,7 +1401,6 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 TQ_STAMP(3);
                 const uint32_t tokV = wait_part(1);
                 TQ_STAMP(4);
-                if (dead) return;
                 const uint32_t vt = stage_addr(s) + code_tile + tokV;
                 const uint32_t vns = stage_addr(s) + tokV + 2u * code_tile + norm_tile + (uint32_t)head * 2u;
                 // weights times V norms as fp16 pairs (heads 2*t4, 2*t4 + 1) of this lane's token rows, then transposed
@@ -1412,7 +1470,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                     }
                 }
             };
-            if (!dead && !TQ_DBG(1)) {
+            if (!TQ_DBG(1)) {
                 if (full) tile_body(std::true_type{});
                 else tile_body(std::false_type{});
             }
@@ -1522,7 +1580,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #endif
     // A warp that gave up on a wait may still have copies in flight: give them a bounded chance to land
     // before the CTA (and its shared memory) goes away.
-    if (dead) {
+    if (!PERSIST && dead) {
         for (int n = consumed; n < consumed + S && n < (int)(hi - lo) * n_layers; ++n) {
             mbar_wait_bounded(bar0 + 16u * (uint32_t)(n % S), (uint32_t)(n / S) & 1u, 1u << 16);
             mbar_wait_bounded(bar0 + 16u * (uint32_t)(n % S) + 8u, (uint32_t)(n / S) & 1u, 1u << 16);

@@ -353,9 +353,17 @@ inline int launch_attention_t(const CUtensorMap& tmK, const CUtensorMap& tmV, co
                               bool pdl) {
     int ar = ensure_dynamic_smem((const void*)decode_attention_kernel<BITS, HKV, MODE>, ATTN_DYN_SMEM);
     if (ar != TQ_OK) return ar;
+    if constexpr (MODE == 2 && HKV == 8) {
+        // the register split inside the kernel draws on what the launch brings: never launch with less
+        static const int regs = [] {
+            cudaFuncAttributes f{};
+            return cudaFuncGetAttributes(&f, (const void*)decode_attention_kernel<BITS, HKV, MODE>) == cudaSuccess ? f.numRegs : 0;
+        }();
+        if (regs * attn_threads<HKV, MODE>() < 32 * (ATTN_GROUPS * HKV * ATTN_REGS_WORK + 4 * ATTN_REGS_COPY)) return TQ_ERR_UNSUPPORTED;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(ATTN_GROUPS * 32 * HKV);
+    cfg.blockDim = dim3(attn_threads<HKV, MODE>());
     cfg.dynamicSmemBytes = ATTN_DYN_SMEM;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
