@@ -392,6 +392,12 @@ def run_append_only(args, w, rank, world, local_rank):
     print(json.dumps(line))
 
 
+def prefill_launches(bits, batch, T, Hkv):
+    """Kernels per layer: (cache write +) attention, a packed prompt's rows as fp16 before it; 131072 rows of a KV head at a time."""
+    groups = 1 if bits == 0 or not batch else -(-batch // max(1, 131072 // (T * Hkv)))
+    return (1 if batch else 0) + groups * (1 if bits == 0 else 2)
+
+
 def run_prefill_attention(args, w, rank, world, local_rank):
     """Prefill attention of whole prompts through the reference's launcher symbol (launch_turbo_gqa_prefill_attention):
     one step = every layer's causal attention of the prompt over its own packed cache."""
@@ -459,13 +465,13 @@ def run_prefill_attention(args, w, rank, world, local_rank):
     line = {
         "metric": METRIC, "value": bytes_step / (ms * 1e-3) / 1e9, "unit": "GB/s", "n_gpus": 1, "steps": steps,
         "warmup": max(3, args.warmup), "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "u8 codes -> f16 tiles, f16 mma.sync, f32 accumulate", "data": "synthetic",
+        "dtype": "u8 codes -> f16 rows, f16 tcgen05.mma, f32 accumulate", "data": "synthetic",
         "config": {"workload": w["desc"], "kv_bits": bits, "l2": "each step reads every layer's cache and queries again (one prompt fits L2: compute bound)"},
         "us_per_layer": ms * 1e3 / NL, "us_per_prompt_and_layer": ms * 1e3 / NL / NP, "causal_tflops": tfs,
-        "gpu_launches": steps * NL * (2 if B else 1),   # (cache write +) attention, one launch each per layer
-        "roofline": {"kernel": f"prefill_attention_kernel<{bits}> (mma.sync)", "bound": "tensor",
+        "gpu_launches": steps * NL * prefill_launches(bits, B, T, Hkv),
+        "roofline": {"kernel": "prefill_attention_fa_kernel (tcgen05)", "bound": "tensor",
                      "achieved": tfs, "peak": tf_peak, "unit": "TFLOP/s", "frac": tfs / tf_peak,
-                     "peak_kind": "measured cuBLAS bf16 (tcgen05); this kernel issues mma.sync", "traffic": None},
+                     "peak_kind": "measured cuBLAS bf16 (tcgen05)", "traffic": None},
         "clocks": clocks,
     }
     print(json.dumps(line))

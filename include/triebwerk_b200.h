@@ -293,9 +293,10 @@ int tq_engine_attend_step(tq_engine* e, void* out, tq_stream_t s);
 
 /* Every layer of a decode step on DEVICE buffers: q/out [layers][G][q_dim], k/v [layers][G][kv_dim]; the layers'
  * append + attention of forward_layer_batch (engine/engine.cpp:1979-2006) for callers that hold all layers' q/k/v
- * at once.  Packed modes run it as four launches whatever the number of layers (one append of every layer's new
- * token, one rotation of all queries, one attention launch that streams the layers back to back, one merge); set TQ_WHOLE_STEP=0 in the
- * environment to get one launch per layer instead. */
+ * at once.  A small step is one launch over all layers (a thread-block cluster per sequence, KV head and layer); a larger one of
+ * the packed modes four, whatever the number of layers (one append of every layer's new token, one rotation of all queries, one
+ * attention launch that streams the layers back to back, one merge).  TQ_WHOLE_STEP=0 in the environment gives one call per
+ * layer instead, TQ_CLUSTER=0 the four launches for small steps too. */
 int tq_engine_decode_step(tq_engine* e, const void* q, const void* k, const void* v, void* out, tq_stream_t s);
 
 /* The step's producer and consumer folded into it.  In the reference the projections' outputs pass through two more
