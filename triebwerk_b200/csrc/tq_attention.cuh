@@ -22,7 +22,9 @@
 //     worker to finish a stage (one shared-memory atomic per warp and tile) re-arms it: nobody waits for a slower
 //     warp.  In the whole-step form a copy warp does, which the warps tell through a barrier per part: without the list's
 //     cursor, the atomics and the fences 664 -> 630 warp instructions per warp and tile (28 layers of 64 x 4096 tokens
-//     2007 -> 1863 us, ragged 128 sequences 2319 -> 2135; shared memory 74 % busy, issue slots 64 %).  With the swizzle, and with the eight tokens of a score block taken in the order 0,5,2,7,4,1,6,3, every
+//     2007 -> 1863 us, ragged 128 sequences 2319 -> 2135; shared memory 74 % busy, issue slots 64 %, and
+//     with two stages the time from hand-back to copy counts: a thread that polls and sleeps 64 ns, 8 layers 2-bit 64 x 3000
+//     198 us, one suspended in the wait 180).  With the swizzle, and with the eight tokens of a score block taken in the order 0,5,2,7,4,1,6,3, every
 //     16-, 8- and 4-byte read of packed codes is free of bank conflicts.
 //   * Codes are turned into fp16 centroids one BYTE at a time (2 codes for 4-bit, 4 for 2-bit) through a
 //     shared-memory table with one private column per lane (bank-conflict free); the table sits at shared
@@ -376,10 +378,10 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
 // MODE 0: queries pre-rotated and tile table built by append_rotate_kernel; 1: the kernel builds its table, rotates the
 // queries, optionally appends the step's token (one launch per layer and step); 2: whole-step form, see AttnParams; 3: as 1,
 // but the partials are only published (merge_partials_kernel<16> follows).
-// The whole-step form has one warp more, which issues the copies of both workers.  With 16 warps at work it is a warpgroup more:
+// The whole-step form has two warps more, which issue the copies of one worker each.  With 16 warps at work it is a warpgroup more:
 // the launch brings 640 x 96 registers, of which the workers' warps take 112 each and the copy warps keep 32.
 template <int HKV, int MODE>
-constexpr int attn_threads() { return ATTN_GROUPS * 32 * HKV + (MODE == 2 ? (HKV == 8 ? 128 : 32) : 0); }
+constexpr int attn_threads() { return ATTN_GROUPS * 32 * HKV + (MODE == 2 ? (HKV == 8 ? 128 : 64) : 0); }
 constexpr int ATTN_REGS_WORK = 112, ATTN_REGS_COPY = 32;
 template <int BITS, int HKV, int MODE>
 __global__ void __launch_bounds__(attn_threads<HKV, MODE>(), 1)
@@ -395,9 +397,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     const int lane = tid & 31;
     const int warp = tid >> 5;
     constexpr int Hkv = HKV;  // compile time: row pitches, tile sizes and norm strides fold into immediates
-    // whole-step form: lane 0 (1) of the copy warp keeps the ring of worker 0 (1) filled
+    // whole-step form: lane 0 of each worker's copy warp keeps its ring filled
     const bool copier = PERSIST && warp >= ATTN_GROUPS * Hkv;
-    const int group = copier ? (lane & 1) : warp / Hkv;  // worker within the CTA
+    const int group = copier ? ((warp - ATTN_GROUPS * Hkv) & 1) : warp / Hkv;  // worker within the CTA
     const int head = warp - group * Hkv; // KV head of this warp
     const int gl = lane >> 2;            // mma "group id": token (K side), coordinate row (V side), head (S layout)
     const int t4 = lane & 3;             // mma "thread in group"
@@ -578,7 +580,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         }
     }
 
-    if (copier && (lane >= ATTN_GROUPS || wid >= W || lo >= hi)) {  // nothing to copy (it returns further down)
+    if (copier && (lane > 0 || wid >= W || lo >= hi)) {  // nothing to copy (it returns further down)
         g = 0;
         lo = hi = 0;
     }
@@ -692,7 +694,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             // fences were in all 16 warps' instruction streams.)  Its own wait is bounded like theirs, and it leaves only when
             // the copies it issued have landed.
             if constexpr (HKV == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ATTN_REGS_COPY));
-            if (warp > ATTN_GROUPS * Hkv || lo >= hi) return;
+            if (warp >= ATTN_GROUPS * (Hkv + 1) || lo >= hi) return;
             int n = 0;
             bool stuck = false;
             for (; cursor_more() && loads_on && !stuck; ++n, cursor_advance()) {
@@ -701,10 +703,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 for (int part = 0; part < 2 && !stuck; ++part) {
                     if (n >= S) {
                         uint32_t ok = 0;
-                        for (uint32_t it = 0; it < (1u << 23) && !ok; ++it) {
-                            ok = mbar_test_wait(ebar0 + 16u * (uint32_t)st + 8u * (uint32_t)part, par);
-                            if (!ok) __nanosleep(64);
-                        }
+                        for (uint32_t it = 0; it < (1u << 15) && !ok; ++it)
+                            ok = mbar_try_wait_hint(ebar0 + 16u * (uint32_t)st + 8u * (uint32_t)part, par, 20000u);
                         if (!ok) {
                             stuck = true;
                             atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
