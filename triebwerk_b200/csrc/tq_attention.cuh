@@ -23,7 +23,7 @@
 //     warp.  In the whole-step form a copy warp does, which the warps tell through a barrier per part: without the list's
 //     cursor, the atomics and the fences 664 -> 630 warp instructions per warp and tile (28 layers of 64 x 4096 tokens
 //     2007 -> 1863 us, ragged 128 sequences 2319 -> 2135; shared memory 74 % busy, issue slots 64 %, and
-//     with two stages the time from hand-back to copy counts: a thread that polls and sleeps 64 ns, 8 layers 2-bit 64 x 3000
+//     with two stages the time from hand-back to copy counts: a thread that polls and sleeps 64 ns, 4 layers 2-bit 64 x 3000
 //     198 us, one suspended in the wait 180).  With the swizzle, and with the eight tokens of a score block taken in the order 0,5,2,7,4,1,6,3, every
 //     16-, 8- and 4-byte read of packed codes is free of bank conflicts.
 //   * Codes are turned into fp16 centroids one BYTE at a time (2 codes for 4-bit, 4 for 2-bit) through a
