@@ -48,6 +48,29 @@ def test_prefill_attention_edges(bits, H, Hkv, n, T, msl):
             hp.assert_attention_close(got[i], ref, H, D, f"tq{bits} {H}/{Hkv} T={T} prompt {i}")
 
 
+@pytest.mark.parametrize("bits,n", [(4, 1), (2, 1), (4, 8)])  # one and two query blocks per CTA
+def test_a_norm_that_is_not_finite_reaches_no_earlier_query(bits, n):
+    """128 values of 6000 have a norm beyond fp16.  Query token t reads rows 0 .. t: such a V vector at row 70 (KV head 0) and
+    such a K vector at row 200 (KV head 1) must not show in the results of the queries before them."""
+    H, Hkv, T, msl = 16, 8, 300, 320
+    rng = np.random.default_rng(4500 + bits + n)
+    R = tq.ops.rotation_matrix().numpy()
+    k, v = (rng.standard_normal((n, T, Hkv * D), dtype=np.float32).astype(np.float16) for _ in range(2))
+    v[:, 70, :D], k[:, 200, D:2 * D] = 6000, 6000
+    q = rng.standard_normal((n, T, H * D), dtype=np.float32).astype(np.float16)
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(n, msl)
+    got = gu.host(eng.prefill_layer_batch(0, 0, gu.dev(q), gu.dev(k), gu.dev(v)))
+    ck, cv, kn, vn = (gu.host(t) for t in eng.layer_cache(0))
+    for i in {0, n - 1}:
+        at = i * msl
+        assert np.isinf(vn[at + 70, 0]) and np.isinf(kn[at + 200, 1])
+        for heads, rows in ((slice(0, 2), 70), (slice(2, 4), 200), (slice(4, 16), T)):  # 2 query heads per KV head
+            ref, _ = tqo.prefill_attention(q[i, :rows], ck[at:], cv[at:], kn[at:], vn[at:], R, msl, H, Hkv, D, bits)
+            sl = slice(heads.start * D, heads.stop * D)
+            hp.assert_attention_close(got[i, :rows, sl], ref[:, sl], heads.stop - heads.start, D, f"tq{bits} heads {heads}")
+
+
 def test_prompts_pass_through_the_scratch_in_groups():
     """40 prompts of 1000 tokens x 4 KV heads: more than the 131072 rows of one KV head that fit the fp16 scratch at a time."""
     H, Hkv, n, T = 8, 4, 40, 1000

@@ -543,9 +543,9 @@ inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, c
     return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT>, tmK, tmV, tmQ, tmR, p));
 }
 // Bytes of scratch a packed prompt of T tokens needs: fp16 centroids of K and V, fp32 norms.
-inline int prefill_t_pad(int T) { return (T + PFT_KT - 1) / PFT_KT * PFT_KT; }
+inline int prefill_tiles(int T) { return (T + PFT_KT - 1) / PFT_KT; }
 inline size_t prefill_scratch_bytes(int T, int Hkv) {
-    return 2 * align_up((size_t)T * Hkv * HEAD_DIM * sizeof(__half), 256) + align_up((size_t)2 * Hkv * prefill_t_pad(T) * sizeof(float), 256);
+    return 2 * align_up((size_t)T * Hkv * HEAD_DIM * sizeof(__half), 256) + align_up((size_t)Hkv * prefill_tiles(T) * PFT_NORM_BYTES, 256);
 }
 // Causal prefill attention.  `total_rows`: rows of the arrays ck and cv point into (from where they point); `scratch`: packed
 // modes, device memory for at least one KV head of one prompt (prompts go through it in groups; one that is too long for it as a
@@ -586,14 +586,16 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
                 d.ck = p.ck + (rows * p.Hkv + h0) * head_bytes; d.cv = p.cv + (rows * p.Hkv + h0) * head_bytes;
                 d.kn = p.kn + rows * p.Hkv + h0; d.vn = p.vn + rows * p.Hkv + h0;
                 d.row_base = p.row_base ? p.row_base + s0 : nullptr;
-                d.seq_rows = p.seq_rows; d.T = p.T; d.t_pad = prefill_t_pad(p.T); d.Hkv = a.Hkv; d.row_heads = p.Hkv;
+                d.seq_rows = p.seq_rows; d.T = p.T; d.tiles = prefill_tiles(p.T); d.Hkv = a.Hkv; d.row_heads = p.Hkv;
                 const size_t rows16 = align_up((size_t)a.n_seq * p.T * kv_dim * sizeof(__half), 256);
                 d.k16 = (__half*)scratch; d.v16 = (__half*)((char*)scratch + rows16); d.norms = (float*)((char*)scratch + 2 * rows16);
                 const long long pieces = 2ll * p.T * a.Hkv * 16;
-                const dim3 grid((unsigned)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count), (unsigned)a.n_seq);
+                d.code_blocks = (int)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count);
+                const int norm_blocks = (int)std::min<long long>(((long long)a.Hkv * d.tiles + 7) / 8, device_props().sm_count);
+                const dim3 grid((unsigned)(d.code_blocks + norm_blocks), (unsigned)a.n_seq);
                 r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4>, grid, dim3(256), 0, s, true, d)
                               : launch_kernel(dequantize_rows_kernel<2>, grid, dim3(256), 0, s, true, d);
-                a.ck = (const uint8_t*)d.k16; a.cv = (const uint8_t*)d.v16; a.norms = d.norms; a.t_pad = d.t_pad;
+                a.ck = (const uint8_t*)d.k16; a.cv = (const uint8_t*)d.v16; a.norms = d.norms; a.tiles = d.tiles;
                 a.row_base = nullptr;
                 a.seq_rows = p.T;
                 if (r == TQ_OK) r = make_prefill_rows_map(&tmR, p.rotation, HEAD_DIM, HEAD_DIM);

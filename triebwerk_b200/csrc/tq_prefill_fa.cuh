@@ -38,6 +38,8 @@ constexpr int PFT_KT = 128;       // cache rows per tile
 constexpr float PFT_SLACK = 4.0f;
 constexpr float PFT_SCALE = 0.12751743074602467f;  // log2(e) / sqrt(128); packed forms: carried by the rotated queries
 constexpr uint32_t PFT_TILE = 32768u;  // an operand tile: [2 halves of the coordinates][128 rows][128 B]
+constexpr int PFT_NORMS = 2 * PFT_KT + 4;  // floats per tile of a packed cache: K norms, V norms, the largest V norm, padding to 16 bytes
+constexpr uint32_t PFT_NORM_BYTES = PFT_NORMS * 4u;
 
 constexpr int PFT_SOFT_WARPS = 16;
 constexpr int PFT_THREADS = 32 * PFT_SOFT_WARPS + 128;  // softmax, then one warp for the copies, one for the products, two idle (a full warpgroup)
@@ -54,8 +56,8 @@ struct PrefillAttnParams {
     const __half* kn;         // (host) [rows][Hkv], packed caches
     const __half* vn;
     const __half* rotation;   // packed: R row-major [128][128]
-    const float* norms;       // packed: fp32 [n_seq][Hkv][K, V][t_pad] (dequantize_rows_kernel)
-    int t_pad;
+    const float* norms;       // packed: fp32 [n_seq][Hkv][tiles][PFT_NORMS] (dequantize_rows_kernel)
+    int tiles;                // of PFT_KT cache rows per prompt
     int* status;              // optional device status word (a bounded wait that gave up raises it)
     __half* out;              // [n_seq][T][q_dim]
     int q_dim;
@@ -73,13 +75,13 @@ struct PftSmem {
     static constexpr uint32_t K = 2 * PFT_TILE;         // 2 stages; at the end: low parts
     static constexpr uint32_t V = K + 2 * PFT_TILE;     // 2 stages
     static constexpr uint32_t R = V + 2 * PFT_TILE;     // packed: R [row][column]
-    static constexpr uint32_t NORM = R + PFT_TILE;      // [2 stages][K, V][128] floats; MT = 1, at the end: [2 slots][128][maximum, sum]
-    static constexpr uint32_t CTRL = NORM + 2048u;      // mbarriers, tensor-memory base
+    static constexpr uint32_t NORM = R + PFT_TILE;      // [2 stages][PFT_NORMS] floats; MT = 1, at the end: [2 slots][128][maximum, sum]
+    static constexpr uint32_t CTRL = NORM + 2u * PFT_NORM_BYTES;  // mbarriers, tensor-memory base
     static constexpr uint32_t BYTES = CTRL + 256u;
 };
 
 // Packed prompts for the kernel below: rows first_row .. of one KV cache array pair as fp16 centroids [n_seq][T][kv_dim] and fp32
-// norms [n_seq][Hkv][K, V][t_pad] (zero behind the prompt).  One thread per 8 codes; bound by HBM / L2 writes of the fp16 rows.
+// norms [n_seq][Hkv][tiles][PFT_NORMS] (zero behind the prompt).  One thread per 8 codes; bound by HBM / L2 writes of the fp16 rows.
 struct DequantParams {
     const uint8_t* ck;
     const uint8_t* cv;
@@ -90,8 +92,9 @@ struct DequantParams {
     __half* k16;
     __half* v16;
     float* norms;
-    int T, t_pad, Hkv;           // Hkv: heads of this pass; ck, cv, kn, vn point at the first one's
+    int T, tiles, Hkv;           // Hkv: heads of this pass; ck, cv, kn, vn point at the first one's
     int row_heads;               // heads per row of the cache
+    int code_blocks;             // CTAs (per prompt) for the codes; those behind them take the norms, a warp per tile and KV head
 };
 template <int BITS>
 __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParams p) {
@@ -107,10 +110,30 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
     pdl_wait();  // the rows come from the append before this launch
     const int seq = blockIdx.y;
     const long long row0 = p.row_base ? p.row_base[seq] : (long long)seq * p.seq_rows;
+    if ((int)blockIdx.x >= p.code_blocks) {
+        const int lane = threadIdx.x & 31, blocks = (int)gridDim.x - p.code_blocks;
+        for (int w = ((int)blockIdx.x - p.code_blocks) * 8 + (threadIdx.x >> 5); w < p.Hkv * p.tiles; w += blocks * 8) {
+            const int h = w / p.tiles, tile = w - h * p.tiles;
+            float* const dst = p.norms + (((long long)seq * p.Hkv + h) * p.tiles + tile) * PFT_NORMS;
+            uint32_t top = 0u;  // of the V norms' words: they order as the values do, and what is not a number lies above them all
+#pragma unroll
+            for (int i = 0; i < PFT_KT; i += 32) {
+                const int t = tile * PFT_KT + i + lane;
+                const long long at = (row0 + t) * p.row_heads + h;
+                const float kn = t < p.T ? __half2float(p.kn[at]) : 0.0f, vn = t < p.T ? __half2float(p.vn[at]) : 0.0f;
+                dst[i + lane] = kn;
+                dst[PFT_KT + i + lane] = vn;
+                top = max(top, __float_as_uint(vn));
+            }
+            top = __reduce_max_sync(0xffffffffu, top);
+            if (lane == 0) dst[2 * PFT_KT] = __uint_as_float(top);
+        }
+        return;
+    }
     const int words = p.Hkv * 16;  // 8-code pieces per row
     const long long n = (long long)p.T * words;
     const int copy = threadIdx.x & 7;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * n; i += (long long)gridDim.x * 256) {
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * n; i += (long long)p.code_blocks * 256) {
         const bool is_v = i >= n;
         const long long w = is_v ? i - n : i;
         const long long at = row0 * (p.row_heads * 16) + (p.row_heads == p.Hkv ? w : w / words * (p.row_heads * 16) + w % words);
@@ -125,14 +148,6 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
             u.z = lut[((c >> 8) & 0xfu) * 8 + copy]; u.w = lut[(c >> 12) * 8 + copy];
         }
         *(reinterpret_cast<uint4*>(is_v ? p.v16 : p.k16) + (long long)seq * n + w) = u;
-    }
-    const long long m = (long long)p.t_pad * p.Hkv;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * m; i += (long long)gridDim.x * 256) {
-        const bool is_v = i >= m;
-        const long long w = is_v ? i - m : i;
-        const int t = (int)(w / p.Hkv), h = (int)(w - (long long)t * p.Hkv);
-        const float x = t < p.T ? __half2float((is_v ? p.vn : p.kn)[(row0 + t) * p.row_heads + h]) : 0.0f;
-        p.norms[(((long long)seq * p.Hkv + h) * 2 + (is_v ? 1 : 0)) * p.t_pad + t] = x;
     }
 }
 
@@ -339,7 +354,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         // ================= the copies of every tile =================
         // (fp16 caches, the prompt's last tile: rows past the prompt may hold anything, and 0 x NaN is NaN, so its V rows are blanked)
         const int x_row = (int)seq_row0;
-        const float* const norms = PACKED ? p.norms + ((size_t)seq * p.Hkv + kvh) * 2 * p.t_pad : nullptr;
+        const float* const norms = PACKED ? p.norms + ((size_t)seq * p.Hkv + kvh) * p.tiles * PFT_NORMS : nullptr;
         for (int j = 0; j < n_tiles; ++j) {
             const int st = j & 1;
             const uint32_t again = (uint32_t)(((j >> 1) - 1) & 1);
@@ -354,11 +369,8 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             const bool tail = !PACKED && valid < PFT_KT;
             const uint32_t bar = tail ? bar_tail : bar_vfull + 8u * st;
             if (lane == 0 && !dead) {
-                mbar_arrive_expect_tx(bar, PFT_TILE + (PACKED ? 1024u : 0u));
-                if (PACKED) {
-                    bulk_load(sb + PftSmem::NORM + st * 1024u, norms + j * PFT_KT, 512u, bar);
-                    bulk_load(sb + PftSmem::NORM + st * 1024u + 512u, norms + p.t_pad + j * PFT_KT, 512u, bar);
-                }
+                mbar_arrive_expect_tx(bar, PFT_TILE + (PACKED ? PFT_NORM_BYTES : 0u));
+                if (PACKED) bulk_load(sb + PftSmem::NORM + st * PFT_NORM_BYTES, norms + (size_t)j * PFT_NORMS, PFT_NORM_BYTES, bar);
                 tma_load_3d(sb + PftSmem::V + st * PFT_TILE, &tmV, bar, 0, x_row + j * PFT_KT, 2 * kvh);
             }
             if (tail) {
@@ -443,7 +455,8 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             wait_bar(bar_sfull + 8u * slot, (uint32_t)(i & 1));
             tc_fence_after();
             const bool diagonal = col0 + PFT_KT - 1 > my_first;  // (uniform for the slot)
-            const float2* const nrm = reinterpret_cast<const float2*>(gb + PftSmem::NORM + (uint32_t)st * 1024u) + t4;
+            const float2* const nrm = reinterpret_cast<const float2*>(gb + PftSmem::NORM + (uint32_t)st * PFT_NORM_BYTES) + t4;
+            const float v_top = PACKED ? *reinterpret_cast<const float*>(gb + PftSmem::NORM + (uint32_t)st * PFT_NORM_BYTES + 8u * PFT_KT) : 0.0f;
             // ---- scores, scaled (packed: by the K norms), masked; row maxima ----
             uint32_t sr[2][32];
             tmem_ld_frag64(s_col, sr[0]);
@@ -510,24 +523,33 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             for (int h = 0; h < 2; ++h)  // (no column counts yet: all weights 0)
                 minus[h] = m_run[h] <= -1e29f ? make_float2(0.0f, 0.0f) : make_float2(-m_run[h], -m_run[h]);
             const float2 sc2 = make_float2(PFT_SCALE, PFT_SCALE);
+            auto weights = [&](auto masked_is_zero) {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint32_t pr[16];
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t pr[16];
 #pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    float2 v2;
-                    if constexpr (PACKED) v2 = nrm[64 + 32 * c + 4 * b];
+                    for (int b = 0; b < 8; ++b) {
+                        float2 v2;
+                        if constexpr (PACKED) v2 = nrm[64 + 32 * c + 4 * b];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        float2 a = PACKED ? add2(x[h][8 * c + b], minus[h]) : fma2(x[h][8 * c + b], sc2, minus[h]);
-                        a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-                        lsum[h] = add2(lsum[h], a);
-                        if constexpr (PACKED) a = mul2(a, v2);
-                        pr[2 * b + h] = pack_half2(a.x, a.y);
+                        for (int h = 0; h < 2; ++h) {
+                            float2 a = PACKED ? add2(x[h][8 * c + b], minus[h]) : fma2(x[h][8 * c + b], sc2, minus[h]);
+                            a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+                            lsum[h] = add2(lsum[h], a);
+                            if constexpr (PACKED && decltype(masked_is_zero)::value) {
+                                a = make_float2(x[h][8 * c + b].x <= -1e30f ? 0.0f : a.x * v2.x, x[h][8 * c + b].y <= -1e30f ? 0.0f : a.y * v2.y);
+                            } else if constexpr (PACKED) {
+                                a = mul2(a, v2);
+                            }
+                            pr[2 * b + h] = pack_half2(a.x, a.y);
+                        }
                     }
+                    tmem_st_pack32(s_col + 32u * c, pr);
                 }
-                tmem_st_pack32(s_col + 32u * c, pr);
-            }
+            };
+            // a masked weight is 0, and 0 times a V norm that is not finite is not: a tile with such a norm selects instead
+            if (PACKED && diagonal && !(v_top < INFINITY)) weights(std::true_type{});
+            else weights(std::false_type{});
             l_run[0] += lsum[0].x + lsum[0].y;
             l_run[1] += lsum[1].x + lsum[1].y;
             tmem_st_wait();
