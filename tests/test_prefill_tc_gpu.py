@@ -71,6 +71,31 @@ def test_a_norm_that_is_not_finite_reaches_no_earlier_query(bits, n):
             hp.assert_attention_close(got[i, :rows, sl], ref[:, sl], heads.stop - heads.start, D, f"tq{bits} heads {heads}")
 
 
+@pytest.mark.parametrize("bits,n", [(4, 1), (2, 1), (4, 8)])  # one and two query blocks per CTA
+def test_weights_times_large_norms_stay_finite(bits, n):
+    """V norms of about 1e4 and scores that rise by 3.4 powers of two in the second and third tile: a weight of 2^3.4 over a
+    reference point of the first tile, times such a norm, is beyond fp16."""
+    H, Hkv, T, msl = 16, 8, 300, 320
+    rng = np.random.default_rng(4600 + bits + n)
+    R = tq.ops.rotation_matrix().numpy()
+    u = rng.standard_normal(D).astype(np.float32)
+    rise = 3.4 / (float(u @ u) * 1.4426950 / np.sqrt(D))
+    k = 0.001 * rng.standard_normal((n, T, Hkv, D)).astype(np.float32)
+    k[:, 130], k[:, 260] = rise * u, rise * u
+    k = k.reshape(n, T, Hkv * D).astype(np.float16)
+    v = (900 * rng.standard_normal((n, T, Hkv * D), dtype=np.float32)).astype(np.float16)
+    q = np.broadcast_to(u.astype(np.float16), (n, T, H, D)).reshape(n, T, H * D).copy()
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(n, msl)
+    got = gu.host(eng.prefill_layer_batch(0, 0, gu.dev(q), gu.dev(k), gu.dev(v))).astype(np.float32)
+    ck, cv, kn, vn = (gu.host(t) for t in eng.layer_cache(0))
+    for i in {0, n - 1}:
+        _, ref = tqo.prefill_attention(q[i], ck[i * msl:], cv[i * msl:], kn[i * msl:], vn[i * msl:], R, msl, H, Hkv, D, bits)
+        # fp16 roundings (2^-11 at most) of weights, centroids, queries' share of the scores and results
+        err = np.linalg.norm(got[i].reshape(T, H, D) - ref, axis=-1) / np.linalg.norm(ref, axis=-1)
+        assert err.max() <= 4 * 2.0 ** -11, f"relative error {err.max():.2e}"
+
+
 def test_prompts_pass_through_the_scratch_in_groups():
     """40 prompts of 1000 tokens x 4 KV heads: more than the 131072 rows of one KV head that fit the fp16 scratch at a time."""
     H, Hkv, n, T = 8, 4, 40, 1000

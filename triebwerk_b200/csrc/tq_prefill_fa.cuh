@@ -17,7 +17,8 @@
 //   warps 0-15   softmax of slots 0 and 1: S -> registers (16x256b loads: a thread holds two rows' column pairs as in an mma
 //                fragment, so a row's maximum is two shuffles), K norm, causal limit, exponentials, P -> tensor memory.  The
 //                exponentials' reference point follows the row maximum only when that has grown by more than PFT_SLACK (in
-//                powers of two): weights stay below 2^PFT_SLACK and O is rescaled in place in the first tiles only.
+//                powers of two; packed tiles with very large V norms: at all): weights stay below 2^PFT_SLACK and O is rescaled in
+//                place in the first tiles only.
 //   warp 16      issues the copies; warp 17 issues every product, in the order P(i) V -> S(i + 1) per slot, slots alternating: the
 //                products of one thread execute in order, so S(i + 1) may overwrite the P(i) that the one before it reads.
 // Packed forms: Q R^T at the start and (O / l) R at the end (fp16 high + low parts) are tcgen05 products too.
@@ -498,7 +499,9 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
                 if (!PACKED) mx[h] *= mx[h] <= -1e30f ? 1.0f : PFT_SCALE;
             }
-            const bool grew0 = mx[0] > m_run[0] + PFT_SLACK, grew1 = mx[1] > m_run[1] + PFT_SLACK;
+            // (weights of up to 2^PFT_SLACK times a norm of 4094 still fit fp16; a tile with a larger one keeps its weights below 1)
+            const float slack = !PACKED || v_top <= 65504.0f / (float)(1 << (int)PFT_SLACK) ? PFT_SLACK : 0.0f;
+            const bool grew0 = mx[0] > m_run[0] + slack, grew1 = mx[1] > m_run[1] + slack;
             if (__any_sync(0xffffffffu, grew0 || grew1)) {
                 const float mn0 = grew0 ? mx[0] : m_run[0], mn1 = grew1 ? mx[1] : m_run[1];
                 const float corr0 = ex2_approx(m_run[0] - mn0), corr1 = ex2_approx(m_run[1] - mn1);
