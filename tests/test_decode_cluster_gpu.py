@@ -71,6 +71,51 @@ def test_decode_layer_cluster_form(bits, H, Hkv, msl, lengths):
         hp.assert_attention_close(out[g][None], ref[None], H, D, f"tq{bits} {H}/{Hkv} seq {g}")
 
 
+# layouts that only the cluster form serves: through decode_layer, whole steps on device and on host buffers, the launchers
+@pytest.mark.parametrize("bits,H,Hkv,msl,lengths", [
+    (4, 40, 8, 640, [1, 16, 33, 639]), (2, 20, 1, 96, [95]), (4, 64, 4, 512, [449, 512]), (2, 6, 2, 320, [17, 300, 320]), (2, 40, 8, 64, [64] * 3),
+    (0, 40, 8, 384, [1, 16, 383]), (0, 12, 4, 1024, [1000]), (0, 20, 1, 320, [97, 320]),
+])
+def test_other_layouts_are_off_by_their_rounding_to_fp16_only(bits, H, Hkv, msl, lengths):
+    """They used to run with fp32 queries, centroids and weights: the results' distance from the oracle's fp32 ones is that of
+    these ones' own rounding to fp16 (3 % for the order of sums and the exponentials)."""
+    rng = np.random.default_rng(3000 + bits + H + msl)
+    NL, G, kv_dim = 2, len(lengths), Hkv * D
+    R = ops.rotation_matrix().numpy()
+    eng = tq.Engine(msl, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(G, msl)
+    pos = [n - 1 for n in lengths]
+    for layer in range(NL):
+        for g, n in enumerate(pos):
+            if n:
+                eng.prefill_append(layer, g, *(gu.dev(rng.standard_normal((n, kv_dim), dtype=np.float32).astype(np.float16)) for _ in range(2)))
+    eng.set_positions(pos)
+    q, k, v = (rng.standard_normal((NL, G, d), dtype=np.float32).astype(np.float16) for d in (H * D, kv_dim, kv_dim))
+    dq, dk, dv = gu.dev(q), gu.dev(k), gu.dev(v)
+    outs = {"layers": gu.host(torch.stack([eng.decode_layer(i, dq[i], dk[i], dv[i]) for i in range(NL)])),
+            "step": gu.host(eng.decode_step(dq, dk, dv, torch.empty_like(dq))),
+            "host": eng.decode_step_host(*(t.cpu().pin_memory() for t in (dq, dk, dv)), torch.empty(dq.shape, dtype=torch.float16, pin_memory=True)).numpy()}
+    outs["launcher"] = np.empty_like(q)
+    ref = np.empty((NL, G, H, D), np.float32)
+    for i in range(NL):
+        cache = eng.layer_cache(i)
+        ck, cv, kn, vn = (None if t is None else gu.host(t) for t in cache)
+        o = torch.empty_like(dq[i])
+        p = gu.dev(np.array(pos, np.int32))
+        if bits == 0:
+            ops.launch_gqa_attention_batch(o, dq[i], cache[0], cache[1], None, p, msl, G, H, Hkv, D, H * D, kv_dim)
+            ref[i] = tqo.fp16_attention_batch(q[i], ck, cv, np.array(pos, np.int32), msl, H, Hkv, D)[1].reshape(G, H, D)
+        else:
+            ops.launch_turbo_gqa_attention_batch(o, dq[i], *cache, gu.dev(R), None, p, msl, G, H, Hkv, D, H * D, kv_dim, bits)
+            ref[i] = tqo.attention_batch(q[i], ck, cv, kn, vn, R, np.array(pos, np.int32), msl, H, Hkv, D, bits)[1].reshape(G, H, D)
+        outs["launcher"][i] = gu.host(o)
+    assert eng.status() == 0
+    rounding = np.linalg.norm(ref.astype(np.float16).astype(np.float32) - ref)
+    for name, out in outs.items():
+        err = np.linalg.norm(out.astype(np.float32).reshape(ref.shape) - ref)
+        assert err <= 1.03 * rounding, f"{name}: {err / rounding:.2f} times the rounding to fp16"
+
+
 @pytest.mark.parametrize("bits", [4, 2])
 @pytest.mark.parametrize("G,Hkv", [(1, 1), (3, 8), (148, 8)])
 def test_one_vector_append_vs_oracle(bits, G, Hkv):

@@ -22,6 +22,9 @@
 //     low parts) and sends every other CTA its share of the output coordinates with asynchronous stores into that CTA's
 //     shared memory, counted by that CTA's mbarrier; a CTA adds up its share, weighted, when all of it has arrived.  (A
 //     cluster barrier in that place costs 0.8 us more: its release waits for the remote stores to be acknowledged.)
+//   * Head layouts that the streaming kernels do not serve took a kernel with fp32 queries, centroids and weights.  Here they are
+//     fp16 high + low parts (EXACT: three products for one, a second table): the results' error is that kernel's.  With the high
+//     parts alone it was 2.9 (4-bit), 3.8 (2-bit) and 1.12 (fp16 rows) times as large.
 // Bound by latency: one round trip for the inputs, the rotation, one tile, three CTA barriers, one trip across the cluster.
 #pragma once
 
@@ -118,6 +121,11 @@ __device__ __forceinline__ __half ldg_half_if(const __half* src, bool on) {
     return __ushort_as_half(r);
 }
 
+// What is left of two floats behind their halves, as halves
+__device__ __forceinline__ uint32_t pack_low_half2(float a, float b) {
+    return pack_half2(a - __half2float(__float2half_rn(a)), b - __half2float(__float2half_rn(b)));
+}
+
 // Shared memory of a CTA below the table, from the dynamic base: the small arrays and, when they fit, the warps' partial
 // results (otherwise those lie behind table and R).
 struct CdSmem {
@@ -133,20 +141,24 @@ struct CdSmem {
     static constexpr uint32_t MZ_OFF = CP_OFF + CD_HEADS * HEAD_DIM * 4; // [CTA][head] maximum and sum
     static constexpr uint32_t WARP_OFF = MZ_OFF + CD_MAX_CLUSTER * CD_HEADS * 8;  // the warps' partial results [8][heads][PART_STRIDE] fp32
 };
-__host__ __device__ constexpr uint32_t cd_table_bytes(int bits) { return bits == 4 ? 0x10000u : (bits == 2 ? 0x1000u + 0x8000u : 0u); }  // with R
+__host__ __device__ constexpr uint32_t cd_low_table(int bits) { return bits == 4 ? 0x10000u : 0x1000u + 0x8000u; }  // the low parts' table, from the first one
+__host__ __device__ constexpr uint32_t cd_table_bytes(int bits, bool exact) {                                       // with R
+    return bits == 0 ? 0u : cd_low_table(bits) + (!exact ? 0u : bits == 4 ? 0x10000u : 0x1000u);
+}
 // (the host: bytes of dynamic shared memory for `heads` query heads per cluster, counted from address 0: what the driver
 // reserves at the start is slack)
-inline size_t cd_smem_bytes(int bits, int heads) {
+inline size_t cd_smem_bytes(int bits, int heads, bool exact) {
     const uint32_t warps = (uint32_t)CD_WARPS * heads * PART_STRIDE * 4u;
-    uint32_t top = CD_LUT_ABS + cd_table_bytes(bits);
+    uint32_t top = CD_LUT_ABS + cd_table_bytes(bits, exact);
     if (CD_MAX_BASE + CdSmem::WARP_OFF + warps > CD_LUT_ABS) top += warps;
     return (size_t)top;
 }
 
 // MB: 16-token blocks per tile (2 for throughput, 1 where every warp gets a single tile anyway and its latency counts)
 // HOST: q, new_k, new_v (and out) are pinned host memory: every byte of them is fetched once per CTA, not once per warp
-template <int BITS, int MB, bool HOST>
-__global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const ClusterDecodeParams p_in) {
+// EXACT: rotated queries, centroids and weights as fp16 high + low parts (see above)
+template <int BITS, int MB, bool HOST, bool EXACT>
+__global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluster_decode_kernel(const ClusterDecodeParams p_in) {
     extern __shared__ __align__(1024) uint8_t cd_smem[];
     ClusterDecodeParams p = p_in;
     constexpr int BPH = BITS == 0 ? 256 : (BITS == 4 ? 64 : 32);  // bytes of a head's row
@@ -174,7 +186,7 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
     const uint32_t lut_s = window + CD_LUT_ABS;
     const uint32_t warps_low = base + CdSmem::WARP_OFF;
     const uint32_t warp_bytes = (uint32_t)(CD_WARPS * nh * PART_STRIDE * 4);
-    const uint32_t warps_s = warps_low + warp_bytes <= lut_s ? warps_low : lut_s + cd_table_bytes(BITS);
+    const uint32_t warps_s = warps_low + warp_bytes <= lut_s ? warps_low : lut_s + cd_table_bytes(BITS, EXACT);
     if (base - window > CD_MAX_BASE) {  // the dynamic part does not start where cd_smem_bytes counts on: no CTA of the launch goes on
         if (tid == 0 && p.status) atomicMax(p.status, ST_SMEM_LAYOUT);
         return;
@@ -201,18 +213,18 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
         const float bound = tid == 0 ? -3.4e38f : (tid > NBND ? 3.4e38f : (BITS == 4 ? kBnd4[(tid - 1) & 15] : kBnd2[(tid - 1) & 3]));
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::BND_OFF + 4u * (uint32_t)tid), "f"(bound) : "memory");
     }
+    constexpr uint32_t LOW = cd_low_table(BITS);
+    auto table_entry = [&](uint32_t at, float c0, float c1) {  // four lanes' copies of two centroids
+        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(pack_half2(c0, c1)) : "memory");
+        if (EXACT) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + LOW), "r"(pack_low_half2(c0, c1)) : "memory");
+    };
     if constexpr (BITS == 4) {
         const float lo = kCent4[(tid >> 3) & 15];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {  // entry (tid >> 3) + 32 i, lanes 4 (tid & 7) .. + 3
-            const uint32_t val = pack_half2(lo, kCent4[(tid >> 7) + 2 * i]);
-            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(lut_s + (uint32_t)((tid >> 3) + 32 * i) * 256u + (uint32_t)(tid & 7) * 16u),
-                         "r"(val) : "memory");
-        }
+        for (int i = 0; i < 8; ++i)  // entry (tid >> 3) + 32 i, lanes 4 (tid & 7) .. + 3
+            table_entry(lut_s + (uint32_t)((tid >> 3) + 32 * i) * 256u + (uint32_t)(tid & 7) * 16u, lo, kCent4[(tid >> 7) + 2 * i]);
     } else if constexpr (BITS == 2) {
-        if (tid < 128)
-            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(lut_s + (uint32_t)(tid >> 3) * 256u + (uint32_t)(tid & 7) * 16u),
-                         "r"(pack_half2(kCent2[(tid >> 3) & 3], kCent2[tid >> 5])) : "memory");
+        if (tid < 128) table_entry(lut_s + (uint32_t)(tid >> 3) * 256u + (uint32_t)(tid & 7) * 16u, kCent2[(tid >> 3) & 3], kCent2[tid >> 5]);
     }
     auto stage_rotation = [&]() {
         uint4 u[8];
@@ -331,6 +343,7 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
 
     // ---- queries ----
     uint32_t qb[8][2];  // B fragments of the score product: lane (gl, t4) holds head gl, step j coordinates 32 t4 + 4 j ..
+    uint32_t ql[EXACT && BITS != 0 ? 8 : 1][2];  // their low parts
     uint4 qw[4];
     const size_t new_at = ((size_t)g * p.Hkv + kvh) * HEAD_DIM;
     const uint32_t in_s = warps_s;  // host inputs: [nh] queries, K, V, 256 bytes each, where the warps' results will be
@@ -395,8 +408,10 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
 #pragma unroll
             for (int e = 0; e < 4; ++e) c[e] += c2[e];
             const float sc = 0.12751743074602467f;  // log2(e) / sqrt(128)
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + CdSmem::Q_OFF + (uint32_t)(gl * MERGE_ROW + 8 * nb + 2 * t4) * 2u),
-                         "r"(pack_half2(c[0] * sc, c[1] * sc)) : "memory");
+            const uint32_t q_at = base + CdSmem::Q_OFF + (uint32_t)(gl * MERGE_ROW + 8 * nb + 2 * t4) * 2u;
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(q_at), "r"(pack_half2(c[0] * sc, c[1] * sc)) : "memory");
+            if (EXACT)
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(q_at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), "r"(pack_low_half2(c[0] * sc, c[1] * sc)) : "memory");
             nc[2 * i] = c[2];
             nc[2 * i + 1] = c[3];
         }
@@ -463,6 +478,11 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
             const uint4 w = gl < nh ? lds128(qa + 16u * i) : make_uint4(0u, 0u, 0u, 0u);
             qb[2 * i][0] = w.x; qb[2 * i][1] = w.y;
             qb[2 * i + 1][0] = w.z; qb[2 * i + 1][1] = w.w;
+            if constexpr (EXACT) {
+                const uint4 l = gl < nh ? lds128(qa + (CdSmem::LO_OFF - CdSmem::Q_OFF) + 16u * i) : make_uint4(0u, 0u, 0u, 0u);
+                ql[2 * i][0] = l.x; ql[2 * i][1] = l.y;
+                ql[2 * i + 1][0] = l.z; ql[2 * i + 1][1] = l.w;
+            }
         }
     } else {
 #pragma unroll
@@ -478,6 +498,11 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
     auto lut = [&](uint32_t w, int byte) -> uint32_t {  // the table's entry for a byte of w: two halves
         uint32_t r;
         asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS));
+        return r;
+    };
+    auto lut_low = [&](uint32_t w, int byte) -> uint32_t {  // EXACT: the low parts
+        uint32_t r;
+        asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS + LOW));
         return r;
     };
     float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};
@@ -526,24 +551,32 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
             }
         }
         // ---- scores: rows gl and gl + 8 of each block, heads 2 t4 and 2 t4 + 1 ----
-        float c[MB][4];
+        float c[MB][4], ce[MB][4];  // ce, EXACT: the products with one low part
 #pragma unroll
-        for (int b = 0; b < MB; ++b) c[b][0] = c[b][1] = c[b][2] = c[b][3] = 0.0f;
+        for (int b = 0; b < MB; ++b) c[b][0] = c[b][1] = c[b][2] = c[b][3] = ce[b][0] = ce[b][1] = ce[b][2] = ce[b][3] = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
 #pragma unroll
             for (int b = 0; b < MB; ++b) {
                 uint32_t a0, a1, a2, a3;
+                auto low_product = [&](uint32_t wlo, int blo, uint32_t whi, int bhi, uint32_t wlo2, int blo2, uint32_t whi2, int bhi2) {
+                    if constexpr (EXACT && BITS != 0) {
+                        mma16816(ce[b], a0, a1, a2, a3, ql[j][0], ql[j][1]);
+                        mma16816(ce[b], lut_low(wlo, blo), lut_low(whi, bhi), lut_low(wlo2, blo2), lut_low(whi2, bhi2), qb[j][0], qb[j][1]);
+                    }
+                };
                 if constexpr (BITS == 4) {
                     const uint4 lo4 = kw[b][0][0], hi4 = kw[b][1][0];
                     const uint32_t lo = j < 2 ? lo4.x : (j < 4 ? lo4.y : (j < 6 ? lo4.z : lo4.w)), hi = j < 2 ? hi4.x : (j < 4 ? hi4.y : (j < 6 ? hi4.z : hi4.w));
                     a0 = lut(lo, 2 * (j & 1)); a1 = lut(hi, 2 * (j & 1));
                     a2 = lut(lo, 2 * (j & 1) + 1); a3 = lut(hi, 2 * (j & 1) + 1);
+                    low_product(lo, 2 * (j & 1), hi, 2 * (j & 1), lo, 2 * (j & 1) + 1, hi, 2 * (j & 1) + 1);
                 } else if constexpr (BITS == 2) {
                     // byte j & 3 of the word: low nibble coordinates 4 j, 4 j + 1, high nibble 4 j + 2, 4 j + 3
                     const uint32_t lo = j < 4 ? kw[b][0][0].x : kw[b][0][0].y, hi = j < 4 ? kw[b][1][0].x : kw[b][1][0].y;
                     a0 = lut(lo & 0x0f0f0f0fu, j & 3); a1 = lut(hi & 0x0f0f0f0fu, j & 3);
                     a2 = lut((lo >> 4) & 0x0f0f0f0fu, j & 3); a3 = lut((hi >> 4) & 0x0f0f0f0fu, j & 3);
+                    low_product(lo & 0x0f0f0f0fu, j & 3, hi & 0x0f0f0f0fu, j & 3, (lo >> 4) & 0x0f0f0f0fu, j & 3, (hi >> 4) & 0x0f0f0f0fu, j & 3);
                 } else {
                     const uint4 lo = kw[b][0][j >> 1], hi = kw[b][1][j >> 1];
                     a0 = (j & 1) ? lo.z : lo.x; a1 = (j & 1) ? hi.z : hi.x;
@@ -551,6 +584,12 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
                 }
                 mma16816(c[b], a0, a1, a2, a3, qb[j][0], qb[j][1]);
             }
+        if (EXACT && BITS != 0) {
+#pragma unroll
+            for (int b = 0; b < MB; ++b)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[b][e] += ce[b][e];
+        }
         float sv[2 * MB][2];
 #pragma unroll
         for (int b = 0; b < MB; ++b)
@@ -588,7 +627,7 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
             m_run[0] = mn0;
             m_run[1] = mn1;
         }
-        uint32_t pb[2 * MB];
+        uint32_t pb[2 * MB], pl[EXACT ? 2 * MB : 1];  // weights times norms, their low parts
 #pragma unroll
         for (int i = 0; i < 2 * MB; ++i) {
             const int t = t0 + 16 * (i >> 1) + 8 * (i & 1) + gl;
@@ -598,11 +637,20 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
             l_run[1] += p1;
             const float n = BITS == 0 ? 1.0f : (on ? __half2float(vn_h[i >> 1][i & 1]) : 0.0f);
             pb[i] = movmatrix_trans(pack_half2(p0 * n, p1 * n));
+            if constexpr (EXACT) pl[i] = movmatrix_trans(pack_low_half2(p0 * n, p1 * n));
         }
         // ---- values ----
 #pragma unroll
         for (int b = 0; b < MB; ++b) {
-            const uint32_t pb0 = pb[2 * b], pb1 = pb[2 * b + 1];
+            const uint32_t pb0 = pb[2 * b], pb1 = pb[2 * b + 1], pl0 = EXACT ? pl[2 * b] : 0u, pl1 = EXACT ? pl[2 * b + 1] : 0u;
+            auto value_product = [&](float (&d)[4], uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int byte) {
+                const uint32_t a0 = lut(w0, byte), a1 = lut(w1, byte), a2 = lut(w2, byte), a3 = lut(w3, byte);
+                mma16816(d, a0, a1, a2, a3, pb0, pb1);
+                if constexpr (EXACT) {
+                    mma16816(d, a0, a1, a2, a3, pl0, pl1);
+                    mma16816(d, lut_low(w0, byte), lut_low(w1, byte), lut_low(w2, byte), lut_low(w3, byte), pb0, pb1);
+                }
+            };
             if constexpr (BITS == 4) {
                 const uint32_t wa[2] = {vw[b][0][0].x, vw[b][0][0].y}, wb[2] = {vw[b][1][0].x, vw[b][1][0].y};
                 const uint32_t wc[2] = {vw[b][2][0].x, vw[b][2][0].y}, wd[2] = {vw[b][3][0].x, vw[b][3][0].y};
@@ -613,8 +661,7 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
                     const uint32_t ev_cd = (wc[w2] & 0x0f0f0f0fu) | ((wd[w2] << 4) & 0xf0f0f0f0u);
                     const uint32_t od_cd = ((wc[w2] >> 4) & 0x0f0f0f0fu) | (wd[w2] & 0xf0f0f0f0u);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        mma16816(acc[4 * w2 + i], lut(ev_ab, i), lut(od_ab, i), lut(ev_cd, i), lut(od_cd, i), pb0, pb1);
+                    for (int i = 0; i < 4; ++i) value_product(acc[4 * w2 + i], ev_ab, od_ab, ev_cd, od_cd, i);
                 }
             } else if constexpr (BITS == 2) {
                 const uint32_t wa = vw[b][0][0].x, wb = vw[b][1][0].x, wc = vw[b][2][0].x, wd = vw[b][3][0].x;
@@ -623,7 +670,7 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {  // coordinates 2 i, 2 i + 1 of the lane's 16: nibble i of `ev`, `od`
                     auto nib = [&](uint32_t w) { return ((i & 1) ? w >> 4 : w) & 0x0f0f0f0fu; };
-                    mma16816(acc[i], lut(nib(ev_ab), i >> 1), lut(nib(od_ab), i >> 1), lut(nib(ev_cd), i >> 1), lut(nib(od_cd), i >> 1), pb0, pb1);
+                    value_product(acc[i], nib(ev_ab), nib(od_ab), nib(ev_cd), nib(od_cd), i >> 1);
                 }
             } else {
 #pragma unroll
@@ -632,8 +679,10 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cluster_decode_kernel(const Clu
                         const uint4 u = vw[b][r][i >> 2];
                         return (i & 3) == 0 ? u.x : ((i & 3) == 1 ? u.y : ((i & 3) == 2 ? u.z : u.w));
                     };
-                    mma16816(acc[i], prmt(word(0), word(1), 0x5410u), prmt(word(0), word(1), 0x7632u), prmt(word(2), word(3), 0x5410u),
-                             prmt(word(2), word(3), 0x7632u), pb0, pb1);
+                    const uint32_t a0 = prmt(word(0), word(1), 0x5410u), a1 = prmt(word(0), word(1), 0x7632u);
+                    const uint32_t a2 = prmt(word(2), word(3), 0x5410u), a3 = prmt(word(2), word(3), 0x7632u);
+                    mma16816(acc[i], a0, a1, a2, a3, pb0, pb1);
+                    if (EXACT) mma16816(acc[i], a0, a1, a2, a3, pl0, pl1);
                 }
             }
         }

@@ -394,15 +394,15 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
 }
 
 // One cluster per (sequence, KV head, block of 8 query heads): tq_decode_cluster.cuh.  `max_tokens`: rows a sequence may hold.
-template <int BITS, int MB, bool HOST>
+template <int BITS, int MB, bool HOST, bool EXACT>
 inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int layers, cudaStream_t s, bool pdl) {
-    const void* kernel = (const void*)cluster_decode_kernel<BITS, MB, HOST>;
-    int r = ensure_dynamic_smem(kernel, cd_smem_bytes(BITS, CD_HEADS), true);
+    const void* kernel = (const void*)cluster_decode_kernel<BITS, MB, HOST, EXACT>;
+    int r = ensure_dynamic_smem(kernel, cd_smem_bytes(BITS, CD_HEADS, EXACT), true);
     if (r != TQ_OK) return r;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)S, (unsigned)(p.Hkv * p.head_blocks), (unsigned)(p.G * layers));
     cfg.blockDim = dim3(CD_THREADS);
-    cfg.dynamicSmemBytes = cd_smem_bytes(BITS, std::min(CD_HEADS, p.H / p.Hkv));
+    cfg.dynamicSmemBytes = cd_smem_bytes(BITS, std::min(CD_HEADS, p.H / p.Hkv), EXACT);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -412,7 +412,7 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB, HOST>, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, cluster_decode_kernel<BITS, MB, HOST, EXACT>, p));
 }
 // CTAs per cluster.  As many as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch: two share
 // the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue (8 sequences x 1023 tokens through
@@ -447,14 +447,20 @@ inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long 
     return 0.4 * chain + 0.3 * chain * turns + 0.009 * clusters < 10.0 + 7e-6 * (double)rows * Hkv + 0.0004 * max_tokens + extra;
 }
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
+template <bool HOST, bool EXACT>
+inline int launch_cluster_decode_e(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
+    const int blocks = (max_tokens + 15) / 16;
+    const int heads = EXACT && bits != 0 ? CD_HEADS : std::min(CD_HEADS, p.H / p.Hkv);  // (EXACT, packed: one CTA per SM, as with 8 heads)
+    const int S = cluster_split(bits, (long long)p.G * split_layers * p.Hkv * p.head_blocks, heads, max_tokens);
+    if (bits == 0) return launch_cluster_decode_t<0, 1, HOST, EXACT>(p, S, layers, s, pdl);
+    const bool one = S * CD_WARPS >= blocks;  // a single 16-token tile per warp
+    if (bits == 4) return one ? launch_cluster_decode_t<4, 1, HOST, EXACT>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2, HOST, EXACT>(p, S, layers, s, pdl);
+    return one ? launch_cluster_decode_t<2, 1, HOST, EXACT>(p, S, layers, s, pdl) : launch_cluster_decode_t<2, 2, HOST, EXACT>(p, S, layers, s, pdl);
+}
 template <bool HOST = false>
 inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
-    const int blocks = (max_tokens + 15) / 16;
-    const int S = cluster_split(bits, (long long)p.G * split_layers * p.Hkv * p.head_blocks, std::min(CD_HEADS, p.H / p.Hkv), max_tokens);
-    if (bits == 0) return launch_cluster_decode_t<0, 1, HOST>(p, S, layers, s, pdl);
-    const bool one = S * CD_WARPS >= blocks;  // a single 16-token tile per warp
-    if (bits == 4) return one ? launch_cluster_decode_t<4, 1, HOST>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2, HOST>(p, S, layers, s, pdl);
-    return one ? launch_cluster_decode_t<2, 1, HOST>(p, S, layers, s, pdl) : launch_cluster_decode_t<2, 2, HOST>(p, S, layers, s, pdl);
+    return fast_shape(p.H, p.Hkv, bits != 0) ? launch_cluster_decode_e<HOST, false>(bits, p, layers, split_layers, max_tokens, s, pdl)
+                                             : launch_cluster_decode_e<HOST, true>(bits, p, layers, split_layers, max_tokens, s, pdl);
 }
 
 __global__ void transpose_rotation_kernel(__half* dst, const __half* src, int* tickets = nullptr, int n_tickets = 0) {
