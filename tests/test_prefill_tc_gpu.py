@@ -96,6 +96,34 @@ def test_weights_times_large_norms_stay_finite(bits, n):
         assert err.max() <= 4 * 2.0 ** -11, f"relative error {err.max():.2e}"
 
 
+@pytest.mark.parametrize("bits,H,Hkv,n,T,msl", [
+    (4, 40, 8, 1, 1, 32), (2, 40, 8, 1, 129, 160), (4, 20, 1, 1, 300, 320), (2, 6, 2, 2, 127, 128), (4, 40, 8, 8, 160, 160),
+    (0, 40, 8, 1, 129, 160), (0, 12, 4, 1, 257, 288), (0, 24, 8, 13, 129, 160), (0, 20, 1, 2, 300, 320),
+])
+def test_other_layouts_are_off_by_their_rounding_to_fp16_only(bits, H, Hkv, n, T, msl):
+    """Numbers of query heads per KV head that used to run with fp32 queries, centroids and weights: the results' distance from the
+    oracle's fp32 ones is that of these ones' own rounding to fp16 (3 % for the order of sums and the exponentials)."""
+    rng = np.random.default_rng(4700 + bits + H + T)
+    R = tq.ops.rotation_matrix().numpy()
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(n, msl)
+    k, v = (rng.standard_normal((n, T, Hkv * D), dtype=np.float32).astype(np.float16) for _ in range(2))
+    q = rng.standard_normal((n, T, H * D), dtype=np.float32).astype(np.float16)
+    got = gu.host(eng.prefill_layer_batch(0, 0, gu.dev(q), gu.dev(k), gu.dev(v))).astype(np.float32)
+    assert eng.status() == 0
+    cache = [None if t is None else gu.host(t) for t in eng.layer_cache(0)]
+    for i in {0, n - 1}:
+        if bits == 0:
+            toks = np.unique(np.linspace(0, T - 1, 40).astype(int))
+            ref = np.stack([tqo.fp16_attention_single(q[i, t], k[i], v[i], t, T, H, Hkv, D)[1] for t in toks])
+        else:
+            toks = np.arange(T)
+            _, ref = tqo.prefill_attention(q[i], *(t[i * msl:] for t in cache), R, msl, H, Hkv, D, bits)
+        ref = ref.reshape(len(toks), H * D)
+        err, rounding = np.linalg.norm(got[i, toks] - ref), np.linalg.norm(ref.astype(np.float16).astype(np.float32) - ref)
+        assert err <= 1.03 * rounding, f"prompt {i}: {err / rounding:.2f} times the rounding to fp16"
+
+
 def test_prompts_pass_through_the_scratch_in_groups():
     """40 prompts of 1000 tokens x 4 KV heads: more than the 131072 rows of one KV head that fit the fp16 scratch at a time."""
     H, Hkv, n, T = 8, 4, 40, 1000

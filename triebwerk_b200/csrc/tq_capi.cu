@@ -687,7 +687,7 @@ static int compat_prefill_attention(void* out, const void* q, const void* ck, co
     void* ws = nullptr;
     const bool aligned = (((uintptr_t)q | (uintptr_t)out | (uintptr_t)ck | (uintptr_t)cv | (uintptr_t)rotation) & 15u) == 0 && q_dim % 8 == 0;
     if (aligned && prefill_attn_shape(H, Hkv)) {
-        const size_t scratch = bits ? prefill_scratch_bytes(T, Hkv) : 0;
+        const size_t scratch = bits ? prefill_scratch_bytes(T, Hkv, prefill_exact(bits, H, Hkv)) : 0;
         int r = compat_workspace(256 + scratch, &ws, s);
         if (r != TQ_OK) return r;
         PrefillAttnParams p{};
@@ -946,7 +946,7 @@ static size_t engine_carve(tq_engine* e, char* base, int G, int msl, long long r
     size_t oq = bump(off, qb), okk = bump(off, kb), ovv = bump(off, kb), oo = bump(off, qb);
     // prompts on their way through the prefill attention as fp16 rows: 16384 tokens of 8 KV heads whatever the slots hold (64 MiB:
     // half of L2, where the attention reads them again); longer prompts pass through it some KV heads at a time
-    const size_t pf_bytes = e->kv_bits ? prefill_scratch_bytes(131072, 1) : 0;
+    const size_t pf_bytes = e->kv_bits ? prefill_scratch_bytes(131072, 1, false) : 0;
     size_t opf = bump(off, pf_bytes);
     if (assign) {
         e->prefill_scratch = e->kv_bits ? base + opf : nullptr;
@@ -1903,11 +1903,12 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
         ap.rotation = (const __half*)e->d_rotation;
     }
     ap.status = (int*)e->workspace;
-    if (e->kv_bits != 0 && prefill_scratch_bytes(T, 1) > e->prefill_scratch_bytes) {  // not even one KV head of such a prompt fits
+    const size_t least = e->kv_bits ? prefill_scratch_bytes(T, 1, prefill_exact(e->kv_bits, H, Hkv)) : 0;
+    if (least > e->prefill_scratch_bytes) {  // not even one KV head of such a prompt fits
         std::lock_guard<std::recursive_mutex> compat_lock(compat_mutex());
         void* ws = nullptr;
-        r = compat_workspace(prefill_scratch_bytes(T, 1), &ws, cs(s));
-        return r != TQ_OK ? r : launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, ws, prefill_scratch_bytes(T, 1), cs(s));
+        r = compat_workspace(least, &ws, cs(s));
+        return r != TQ_OK ? r : launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, ws, least, cs(s));
     }
     return launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s));
 }

@@ -145,6 +145,9 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
 }
+// What a float's rounding to fp16 leaves over, and two floats' rest as halves
+__device__ __forceinline__ float low_part(float x) { return x - __half2float(__float2half_rn(x)); }
+__device__ __forceinline__ uint32_t pack_low_half2(float lo, float hi) { return pack_half2(low_part(lo), low_part(hi)); }
 
 // D += A(16x16, row) * B(16x8, col), fp16 inputs, fp32 accumulate.
 // Four 8x8 fp16 matrices from shared memory as mma fragments: lane l supplies the address of row l % 8 of matrix l / 8;

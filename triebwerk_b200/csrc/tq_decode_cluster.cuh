@@ -121,11 +121,6 @@ __device__ __forceinline__ __half ldg_half_if(const __half* src, bool on) {
     return __ushort_as_half(r);
 }
 
-// What is left of two floats behind their halves, as halves
-__device__ __forceinline__ uint32_t pack_low_half2(float a, float b) {
-    return pack_half2(a - __half2float(__float2half_rn(a)), b - __half2float(__float2half_rn(b)));
-}
-
 // Shared memory of a CTA below the table, from the dynamic base: the small arrays and, when they fit, the warps' partial
 // results (otherwise those lie behind table and R).
 struct CdSmem {

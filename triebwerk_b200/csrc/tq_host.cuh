@@ -525,15 +525,15 @@ inline int make_prefill_query_map(CUtensorMap* m, const void* base, long long to
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TQ_OK : TQ_ERR_ARG;
 }
-template <bool PACKED, int MT>
+template <bool PACKED, int MT, bool EXACT = false>
 inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ, const CUtensorMap& tmR, const PrefillAttnParams& p,
                                dim3 grid, cudaStream_t s) {
-    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT>, PftSmem::BYTES);
+    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT>, PftSmem::BYTES);
     if (r != TQ_OK) return r;
     // the register split inside the kernel draws on what the launch brings: never launch with less
     static const int regs = [] {
         cudaFuncAttributes a{};
-        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT>) == cudaSuccess ? a.numRegs : 0;
+        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT>) == cudaSuccess ? a.numRegs : 0;
     }();
     if (regs < PFT_REGS_LAUNCH) return TQ_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg{};
@@ -546,29 +546,35 @@ inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT>, tmK, tmV, tmQ, tmR, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT, EXACT>, tmK, tmV, tmQ, tmR, p));
 }
-// Bytes of scratch a packed prompt of T tokens needs: fp16 centroids of K and V, fp32 norms.
+// Which layouts keep fp32's precision (tq_prefill_fa.cuh): those that neither this kernel's predecessor nor the streaming kernels took.
+inline bool prefill_exact(int bits, int H, int Hkv) {
+    const int grp = H / Hkv;
+    return !(grp == 1 || grp == 2 || grp == 4 || grp == 8 || grp == 16) && !fast_shape(H, Hkv, bits != 0);
+}
+// Bytes of scratch a packed prompt of T tokens needs: fp16 centroids of K and V (exact: high and low parts), fp32 norms.
 inline int prefill_tiles(int T) { return (T + PFT_KT - 1) / PFT_KT; }
-inline size_t prefill_scratch_bytes(int T, int Hkv) {
-    return 2 * align_up((size_t)T * Hkv * HEAD_DIM * sizeof(__half), 256) + align_up((size_t)Hkv * prefill_tiles(T) * PFT_NORM_BYTES, 256);
+inline size_t prefill_scratch_bytes(int T, int Hkv, bool exact) {
+    return 2 * align_up((size_t)(exact ? 2 : 1) * T * Hkv * HEAD_DIM * sizeof(__half), 256) + align_up((size_t)Hkv * prefill_tiles(T) * PFT_NORM_BYTES, 256);
 }
 // Causal prefill attention.  `total_rows`: rows of the arrays ck and cv point into (from where they point); `scratch`: packed
 // modes, device memory for at least one KV head of one prompt (prompts go through it in groups; one that is too long for it as a
 // whole, some of its KV heads at a time).
 inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long total_rows, void* scratch, size_t scratch_bytes, cudaStream_t s) {
     p.grp = p.H / p.Hkv;
+    const bool exact = prefill_exact(bits, p.H, p.Hkv), low = exact && bits != 0;
     if (p.n_seq <= 0) p.n_seq = 1;
     if (p.T <= 0) return TQ_OK;
     const int qt = PFT_ROWS / p.grp;
     int group = p.n_seq, heads = p.Hkv;  // prompts and KV heads per launch (fp16 caches: all of them)
     if (bits != 0) {
         if (!scratch) return TQ_ERR_WORKSPACE;
-        while (heads > 0 && prefill_scratch_bytes(p.T, heads) > scratch_bytes) --heads;
+        while (heads > 0 && prefill_scratch_bytes(p.T, heads, exact) > scratch_bytes) --heads;
         if (heads == 0) return TQ_ERR_WORKSPACE;
         const int passes = (p.Hkv + heads - 1) / heads;
         heads = (p.Hkv + passes - 1) / passes;  // of about the same size
-        group = (int)std::min<long long>(p.n_seq, (long long)(scratch_bytes / prefill_scratch_bytes(p.T, heads)));
+        group = (int)std::min<long long>(p.n_seq, (long long)(scratch_bytes / prefill_scratch_bytes(p.T, heads, exact)));
     }
     for (int s0 = 0; s0 < p.n_seq; s0 += group) {
         for (int h0 = 0; h0 < p.Hkv; h0 += heads) {
@@ -593,20 +599,25 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
                 d.kn = p.kn + rows * p.Hkv + h0; d.vn = p.vn + rows * p.Hkv + h0;
                 d.row_base = p.row_base ? p.row_base + s0 : nullptr;
                 d.seq_rows = p.seq_rows; d.T = p.T; d.tiles = prefill_tiles(p.T); d.Hkv = a.Hkv; d.row_heads = p.Hkv;
-                const size_t rows16 = align_up((size_t)a.n_seq * p.T * kv_dim * sizeof(__half), 256);
+                const long long rows_hi = (long long)a.n_seq * p.T, rows_all = low ? 2 * rows_hi : rows_hi;  // the low parts behind the high ones
+                const size_t rows16 = align_up((size_t)rows_all * kv_dim * sizeof(__half), 256);
+                d.low = rows_hi * kv_dim;
                 d.k16 = (__half*)scratch; d.v16 = (__half*)((char*)scratch + rows16); d.norms = (float*)((char*)scratch + 2 * rows16);
                 const long long pieces = 2ll * p.T * a.Hkv * 16;
                 d.code_blocks = (int)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count);
                 const int norm_blocks = (int)std::min<long long>(((long long)a.Hkv * d.tiles + 7) / 8, device_props().sm_count);
                 const dim3 grid((unsigned)(d.code_blocks + norm_blocks), (unsigned)a.n_seq);
-                r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4>, grid, dim3(256), 0, s, true, d)
-                              : launch_kernel(dequantize_rows_kernel<2>, grid, dim3(256), 0, s, true, d);
+                if (low) r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4, true>, grid, dim3(256), 0, s, true, d)
+                                       : launch_kernel(dequantize_rows_kernel<2, true>, grid, dim3(256), 0, s, true, d);
+                else r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4, false>, grid, dim3(256), 0, s, true, d)
+                                   : launch_kernel(dequantize_rows_kernel<2, false>, grid, dim3(256), 0, s, true, d);
                 a.ck = (const uint8_t*)d.k16; a.cv = (const uint8_t*)d.v16; a.norms = d.norms; a.tiles = d.tiles;
                 a.row_base = nullptr;
                 a.seq_rows = p.T;
+                a.low_row = (int)rows_hi;
                 if (r == TQ_OK) r = make_prefill_rows_map(&tmR, p.rotation, HEAD_DIM, HEAD_DIM);
-                if (r == TQ_OK) r = make_prefill_rows_map(&tmK, d.k16, (long long)a.n_seq * p.T, kv_dim);
-                if (r == TQ_OK) r = make_prefill_rows_map(&tmV, d.v16, (long long)a.n_seq * p.T, kv_dim);
+                if (r == TQ_OK) r = make_prefill_rows_map(&tmK, d.k16, rows_all, kv_dim);
+                if (r == TQ_OK) r = make_prefill_rows_map(&tmV, d.v16, rows_all, kv_dim);
             }
             if (r != TQ_OK) return r;
             // Two query blocks per CTA, which share every tile, once there are enough of them for the GPU; below that twice the
@@ -618,11 +629,13 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
             // 4/3 of one with one: 12 prompts of 70 tokens 32.4 / 29.6 us, of 163 38.8 / 45.4, 16 of 250 63.5 / 55.2.
             const long long sms = device_props().sm_count, blocks1 = (p.T + qt - 1) / qt;
             const long long turns1 = (blocks1 * cols + sms - 1) / sms, turns2 = (blocks2 * cols + sms - 1) / sms;
-            const int mt = (p.T <= 2 * PFT_KT ? 3 * turns1 >= 4 * turns2 : 4 * blocks2 * cols >= 5 * sms) ? 2 : 1;
+            const int mt = low ? 1 : (p.T <= 2 * PFT_KT ? 3 * turns1 >= 4 * turns2 : 4 * blocks2 * cols >= 5 * sms) ? 2 : 1;
             const long long blocks = mt == 2 ? blocks2 : blocks1;
             if (cols > 2147483647ll || blocks > 65535) return TQ_ERR_CAPACITY;
             dim3 grid((unsigned)cols, (unsigned)blocks);
-            if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
+            if (low) r = launch_prefill_fa_t<true, 1, true>(tmK, tmV, tmQ, tmR, a, grid, s);
+            else if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
+            else if (exact) r = mt == 2 ? launch_prefill_fa_t<false, 2, true>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1, true>(tmK, tmV, tmQ, tmR, a, grid, s);
             else r = mt == 2 ? launch_prefill_fa_t<false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
             if (r != TQ_OK) return r;
         }

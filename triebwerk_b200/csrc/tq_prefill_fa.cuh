@@ -21,6 +21,9 @@
 //                place in the first tiles only.
 //   warp 16      issues the copies; warp 17 issues every product, in the order P(i) V -> S(i + 1) per slot, slots alternating: the
 //                products of one thread execute in order, so S(i + 1) may overwrite the P(i) that the one before it reads.
+// Numbers of query heads per KV head other than 1, 2, 4, 8 and 16 took a kernel with fp32 queries, centroids and weights.  Here they
+// are fp16 high + low parts (EXACT: three products for one, two for fp16 caches): the results' error is that kernel's.  With the high
+// parts alone it was 2.4 (4-bit), 2.9 (2-bit) and 1.2 (fp16) times as large.
 // Packed forms: Q R^T at the start and (O / l) R at the end (fp16 high + low parts) are tcgen05 products too.
 // Every wait on a barrier is bounded; a wait that runs out raises the status word and the kernel runs to its end.
 // Bound by the softmax threads (exponentials, tensor-memory loads) against the tensor core at long prompts, by the chain copy ->
@@ -57,6 +60,7 @@ struct PrefillAttnParams {
     const __half* kn;         // (host) [rows][Hkv], packed caches
     const __half* vn;
     const __half* rotation;   // packed: R row-major [128][128]
+    int low_row;              // packed, EXACT: rows from the high parts to the low parts of ck, cv
     const float* norms;       // packed: fp32 [n_seq][Hkv][tiles][PFT_NORMS] (dequantize_rows_kernel)
     int tiles;                // of PFT_KT cache rows per prompt
     int* status;              // optional device status word (a bounded wait that gave up raises it)
@@ -95,16 +99,19 @@ struct DequantParams {
     float* norms;
     int T, tiles, Hkv;           // Hkv: heads of this pass; ck, cv, kn, vn point at the first one's
     int row_heads;               // heads per row of the cache
+    long long low;               // EXACT: halves from a value's high part to its low part
     int code_blocks;             // CTAs (per prompt) for the codes; those behind them take the norms, a warp per tile and KV head
 };
-template <int BITS>
+template <int BITS, bool EXACT>
 __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParams p) {
     // byte (4-bit) or nibble (2-bit) -> two centroids; eight copies, so that at most four lanes of a warp share a bank
     constexpr int ENTRIES = BITS == 4 ? 256 : 16;
-    __shared__ uint32_t lut[ENTRIES * 8];
+    __shared__ uint32_t luts[(EXACT ? 2 : 1) * ENTRIES * 8];  // EXACT: then their low parts
     for (int i = threadIdx.x; i < ENTRIES * 8; i += 256) {
         const int e = i >> 3;
-        lut[i] = BITS == 4 ? pack_half2(kCent4[e & 15], kCent4[e >> 4]) : pack_half2(kCent2[e & 3], kCent2[(e >> 2) & 3]);
+        const float c0 = BITS == 4 ? kCent4[e & 15] : kCent2[e & 3], c1 = BITS == 4 ? kCent4[e >> 4] : kCent2[(e >> 2) & 3];
+        luts[i] = pack_half2(c0, c1);
+        if (EXACT) luts[ENTRIES * 8 + i] = pack_low_half2(c0, c1);
     }
     __syncthreads();
     pdl_launch_dependents();
@@ -138,17 +145,22 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
         const bool is_v = i >= n;
         const long long w = is_v ? i - n : i;
         const long long at = row0 * (p.row_heads * 16) + (p.row_heads == p.Hkv ? w : w / words * (p.row_heads * 16) + w % words);
-        uint4 u;
-        if (BITS == 4) {
-            const uint32_t c = *(reinterpret_cast<const uint32_t*>(is_v ? p.cv : p.ck) + at);
-            u.x = lut[(c & 0xffu) * 8 + copy]; u.y = lut[((c >> 8) & 0xffu) * 8 + copy];
-            u.z = lut[((c >> 16) & 0xffu) * 8 + copy]; u.w = lut[(c >> 24) * 8 + copy];
-        } else {
-            const uint32_t c = *(reinterpret_cast<const unsigned short*>(is_v ? p.cv : p.ck) + at);
-            u.x = lut[(c & 0xfu) * 8 + copy]; u.y = lut[((c >> 4) & 0xfu) * 8 + copy];
-            u.z = lut[((c >> 8) & 0xfu) * 8 + copy]; u.w = lut[(c >> 12) * 8 + copy];
+        const uint32_t c = BITS == 4 ? *(reinterpret_cast<const uint32_t*>(is_v ? p.cv : p.ck) + at)
+                                     : (uint32_t)*(reinterpret_cast<const unsigned short*>(is_v ? p.cv : p.ck) + at);
+        uint4* const dst = reinterpret_cast<uint4*>(is_v ? p.v16 : p.k16) + (long long)seq * n + w;
+#pragma unroll
+        for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
+            const uint32_t* const lut = luts + part * ENTRIES * 8;
+            uint4 u;
+            if (BITS == 4) {
+                u.x = lut[(c & 0xffu) * 8 + copy]; u.y = lut[((c >> 8) & 0xffu) * 8 + copy];
+                u.z = lut[((c >> 16) & 0xffu) * 8 + copy]; u.w = lut[(c >> 24) * 8 + copy];
+            } else {
+                u.x = lut[(c & 0xfu) * 8 + copy]; u.y = lut[((c >> 4) & 0xfu) * 8 + copy];
+                u.z = lut[((c >> 8) & 0xfu) * 8 + copy]; u.w = lut[(c >> 12) * 8 + copy];
+            }
+            dst[part ? p.low / 8 : 0] = u;
         }
-        *(reinterpret_cast<uint4*>(is_v ? p.v16 : p.k16) + (long long)seq * n + w) = u;
     }
 }
 
@@ -223,7 +235,9 @@ template <int N>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // PACKED: ck, cv are the fp16 centroids [n_seq * T][kv_dim] of dequantize_rows_kernel (seq_rows = T, no row_base), p.norms its norms
-template <bool PACKED, int MT>
+// EXACT: queries, centroids and weights as fp16 high + low parts; packed with MT = 1 only: one stage of K and V, the low parts in
+// the other one's place, the queries' in the second query tile's
+template <bool PACKED, int MT, bool EXACT>
 __global__ void __launch_bounds__(PFT_THREADS, 1)
 prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ,
                             const __grid_constant__ CUtensorMap tmR, const PrefillAttnParams p) {
@@ -235,6 +249,11 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         return;
     }
     constexpr int COPY_WARP = PFT_SOFT_WARPS, MMA_WARP = PFT_SOFT_WARPS + 1;
+    constexpr bool LOW = PACKED && EXACT;  // low parts of the operands in shared memory
+    static_assert(!LOW || MT == 1, "the second query block's places hold the low parts");
+    // tile j's data are in stage j % STAGES; its barriers are number j & 1 also where there is one stage (a slot waits for every other
+    // tile only, so that it must not meet the one between them on the same barrier)
+    constexpr int STAGES = LOW ? 1 : 2;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int GRP = p.grp, QT = PFT_ROWS / GRP;
     const int qb = (int)gridDim.y - 1 - (int)blockIdx.y;  // the longest causal prefixes of all heads and prompts first
@@ -336,9 +355,12 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        put_pair(PftSmem::Q + pslot * PFT_TILE, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, __uint_as_float(r[4 * j + 2 * h]) * PFT_SCALE,
-                                 __uint_as_float(r[4 * j + 2 * h + 1]) * PFT_SCALE);
+                    for (int h = 0; h < 2; ++h) {
+                        const float q0 = __uint_as_float(r[4 * j + 2 * h]) * PFT_SCALE, q1 = __uint_as_float(r[4 * j + 2 * h + 1]) * PFT_SCALE;
+                        put_pair(PftSmem::Q + pslot * PFT_TILE, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, q0, q1);
+                        if (LOW)
+                            put_pair(PftSmem::Q + PFT_TILE, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, low_part(q0), low_part(q1));
+                    }
             }
         }
         if (warp < PFT_SOFT_WARPS || warp == MMA_WARP) {  // the rotated queries are in place (the copies of the first tiles are on their way already)
@@ -357,22 +379,23 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         const int x_row = (int)seq_row0;
         const float* const norms = PACKED ? p.norms + ((size_t)seq * p.Hkv + kvh) * p.tiles * PFT_NORMS : nullptr;
         for (int j = 0; j < n_tiles; ++j) {
-            const int st = j & 1;
-            const uint32_t again = (uint32_t)(((j >> 1) - 1) & 1);
-            if (j > 1) wait_bar(bar_kfree + 8u * st, again);
+            const int st = j % STAGES, b = j & 1, last = j - STAGES;  // last: the tile that was in this stage
+            if (last >= 0) wait_bar(bar_kfree + 8u * (last & 1), (uint32_t)((last >> 1) & 1));
             if (lane == 0 && !dead) {
-                mbar_arrive_expect_tx(bar_kfull + 8u * st, PFT_TILE);
-                tma_load_3d(sb + PftSmem::K + st * PFT_TILE, &tmK, bar_kfull + 8u * st, 0, x_row + j * PFT_KT, 2 * kvh);
+                mbar_arrive_expect_tx(bar_kfull + 8u * b, (LOW ? 2u : 1u) * PFT_TILE);
+                tma_load_3d(sb + PftSmem::K + st * PFT_TILE, &tmK, bar_kfull + 8u * b, 0, x_row + j * PFT_KT, 2 * kvh);
+                if (LOW) tma_load_3d(sb + PftSmem::K + PFT_TILE, &tmK, bar_kfull + 8u * b, 0, p.low_row + x_row + j * PFT_KT, 2 * kvh);
             }
-            // (V free: the value products of the tile two back are done, hence its softmax has read its norms)
-            if (j > 1) wait_bar(bar_vfree + 8u * st, again);
+            // (V free: the value products of that tile are done, hence its softmax has read its norms)
+            if (last >= 0) wait_bar(bar_vfree + 8u * (last & 1), (uint32_t)((last >> 1) & 1));
             const int valid = p.T - j * PFT_KT;
             const bool tail = !PACKED && valid < PFT_KT;
-            const uint32_t bar = tail ? bar_tail : bar_vfull + 8u * st;
+            const uint32_t bar = tail ? bar_tail : bar_vfull + 8u * b;
             if (lane == 0 && !dead) {
-                mbar_arrive_expect_tx(bar, PFT_TILE + (PACKED ? PFT_NORM_BYTES : 0u));
+                mbar_arrive_expect_tx(bar, (LOW ? 2u : 1u) * PFT_TILE + (PACKED ? PFT_NORM_BYTES : 0u));
                 if (PACKED) bulk_load(sb + PftSmem::NORM + st * PFT_NORM_BYTES, norms + (size_t)j * PFT_NORMS, PFT_NORM_BYTES, bar);
                 tma_load_3d(sb + PftSmem::V + st * PFT_TILE, &tmV, bar, 0, x_row + j * PFT_KT, 2 * kvh);
+                if (LOW) tma_load_3d(sb + PftSmem::V + PFT_TILE, &tmV, bar, 0, p.low_row + x_row + j * PFT_KT, 2 * kvh);
             }
             if (tail) {
                 wait_bar(bar_tail, 0u);
@@ -380,26 +403,33 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     *reinterpret_cast<uint4*>(gb + PftSmem::V + st * PFT_TILE + pft_chunk(valid + (i >> 4), i & 15)) = make_uint4(0u, 0u, 0u, 0u);
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_vfull + 8u * st);
+                if (lane == 0) mbar_arrive(bar_vfull + 8u * b);
             }
         }
       } else if (warp == MMA_WARP) {
         // ================= one thread issues every product =================
         if (lane == 0) {
             auto issue_scores = [&](int s, int i) {
-                const int j = tile_of(s, i), st = j & 1;
-                wait_bar(bar_kfull + 8u * st, (uint32_t)((j >> 1) & 1));
+                const int j = tile_of(s, i), st = j % STAGES;
+                wait_bar(bar_kfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
                 tc_fence_after();
                 if (dead) return;
                 const uint32_t a = pft_lo_k(sb + PftSmem::Q + (MT == 2 ? s * PFT_TILE : 0u)), b = pft_lo_k(sb + PftSmem::K + st * PFT_TILE);
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) umma_lo(tmem + 128u * s, a + pft_kstep(ks), b + pft_kstep(ks), PFT_IDESC_K, ks != 0);
+                if (LOW) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks) {
+                        umma_lo(tmem + 128u * s, a + PFT_TILE / 16u + pft_kstep(ks), b + pft_kstep(ks), PFT_IDESC_K, 1u);
+                        umma_lo(tmem + 128u * s, a + pft_kstep(ks), b + PFT_TILE / 16u + pft_kstep(ks), PFT_IDESC_K, 1u);
+                    }
+                }
                 umma_commit(bar_sfull + 8u * s);
-                if (MT == 1 || s == (j < n1 ? 1 : 0)) umma_commit(bar_kfree + 8u * st);  // its last reader
+                if (MT == 1 || s == (j < n1 ? 1 : 0)) umma_commit(bar_kfree + 8u * (j & 1));  // its last reader
             };
             auto issue_values = [&](int s, int i) {
-                const int j = tile_of(s, i), st = j & 1;
-                wait_bar(bar_vfull + 8u * st, (uint32_t)((j >> 1) & 1));
+                const int j = tile_of(s, i), st = j % STAGES;
+                wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
                 wait_bar(bar_pfull + 8u * s, (uint32_t)(i & 1));
                 tc_fence_after();
                 if (dead) return;
@@ -407,7 +437,14 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks)
                     umma_lo_ta(tmem + 256u + 128u * s, tmem + 128u * s + 8u * ks, b + 128u * ks, PFT_IDESC_MN, ks == 0 ? (uint32_t)(i != 0) : 1u);
-                if (MT == 1 || s == (j < n1 ? 1 : 0)) umma_commit(bar_vfree + 8u * st);
+                if (EXACT) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks) {
+                        umma_lo_ta(tmem + 256u + 128u * s, tmem + 128u * s + 64u + 8u * ks, b + 128u * ks, PFT_IDESC_MN, 1u);
+                        if (LOW) umma_lo_ta(tmem + 256u + 128u * s, tmem + 128u * s + 8u * ks, b + PFT_TILE / 16u + 128u * ks, PFT_IDESC_MN, 1u);
+                    }
+                }
+                if (MT == 1 || s == (j < n1 ? 1 : 0)) umma_commit(bar_vfree + 8u * (j & 1));
             };
             if (!PACKED) wait_bar(bar_q, 0u);
             if (n0 > 0) issue_scores(0, 0);
@@ -451,8 +488,8 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         const int tok0 = token_of(row0 + g), tok1 = token_of(row0 + g + 8);
         float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};  // (sums: of this thread's columns)
         for (int i = 0; i < nt; ++i) {
-            const int j = tile_of(slot, i), st = j & 1, col0 = j * PFT_KT;
-            if (PACKED) wait_bar(bar_vfull + 8u * st, (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
+            const int j = tile_of(slot, i), st = j % STAGES, col0 = j * PFT_KT;
+            if (PACKED) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
             wait_bar(bar_sfull + 8u * slot, (uint32_t)(i & 1));
             tc_fence_after();
             const bool diagonal = col0 + PFT_KT - 1 > my_first;  // (uniform for the slot)
@@ -529,7 +566,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             auto weights = [&](auto masked_is_zero) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
-                    uint32_t pr[16];
+                    uint32_t pr[16], pl[EXACT ? 16 : 1];  // EXACT: the low parts behind the high ones, columns 64 ..
 #pragma unroll
                     for (int b = 0; b < 8; ++b) {
                         float2 v2;
@@ -545,9 +582,11 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                                 a = mul2(a, v2);
                             }
                             pr[2 * b + h] = pack_half2(a.x, a.y);
+                            if constexpr (EXACT) pl[2 * b + h] = pack_low_half2(a.x, a.y);
                         }
                     }
                     tmem_st_pack32(s_col + 32u * c, pr);
+                    if constexpr (EXACT) tmem_st_pack32(s_col + 64u + 32u * c, pl);
                 }
             };
             // a masked weight is 0, and 0 times a V norm that is not finite is not: a tile with such a norm selects instead
@@ -619,7 +658,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     result(c0, y);
                     put_frag(qtile, c0, y);
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) y[e] -= __half2float(__float2half_rn(y[e]));
+                    for (int e = 0; e < 16; ++e) y[e] = low_part(y[e]);
                     put_frag(ktile, c0, y);
                 }
             }
