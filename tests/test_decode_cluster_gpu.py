@@ -132,6 +132,35 @@ def test_one_vector_append_vs_oracle(bits, G, Hkv):
     assert np.abs(gn.view(np.uint16).astype(np.int32) - wn.view(np.uint16).astype(np.int32)).max() <= 1
 
 
+@pytest.mark.parametrize("bits,msl", [(4, 288), (4, 320), (2, 288)])
+def test_whole_steps_with_and_without_copy_warps(bits, msl):
+    """128 sequences, too many for the cluster form: 4-bit slots of 36864 rows in all run without the copy warps on 148 SMs, of
+    40960 with them (the line is four tiles per worker: 37888 rows)."""
+    H, Hkv, NL, G = 16, 8, 2, 128
+    rng = np.random.default_rng(3500 + bits + msl)
+    R = ops.rotation_matrix().numpy()
+    lengths = [int(n) for n in rng.integers(1, 289, G)]
+    lengths[:6] = [1, 32, 33, 64, 287, 288]
+    eng = tq.Engine(msl, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(G, msl)
+    pool = gu.dev(rng.standard_normal((2, 512, Hkv * D), dtype=np.float32).astype(np.float16))
+    for layer in range(NL):
+        for g, n in enumerate(lengths):
+            if n > 1:
+                at = (37 * g + 11 * layer) % 224
+                eng.prefill_append(layer, g, pool[0, at:at + n - 1], pool[1, at:at + n - 1])
+    eng.set_positions([n - 1 for n in lengths])
+    q, k, v = (gu.dev(rng.standard_normal((NL, G, d), dtype=np.float32).astype(np.float16)) for d in (H * D, Hkv * D, Hkv * D))
+    out = gu.host(eng.decode_step(q, k, v, torch.empty_like(q)))
+    assert eng.status() == 0
+    for layer in range(NL):
+        ck, cv, kn, vn = (gu.host(t) for t in eng.layer_cache(layer))
+        for g in (0, 1, 2, 3, 4, 5, 64, 127):
+            sl = slice(g * msl, g * msl + lengths[g])
+            ref, _ = tqo.attention_single(gu.host(q)[layer, g], ck[sl], cv[sl], kn[sl], vn[sl], R, lengths[g] - 1, lengths[g], H, Hkv, D, bits)
+            hp.assert_attention_close(out[layer, g][None], ref[None], H, D, f"tq{bits} layer {layer} sequence {g}")
+
+
 def test_streaming_forms_in_a_child_process():
     """TQ_CLUSTER=0 (read once per process) keeps the streaming kernels for small batches too."""
     if os.environ.get("TQ_CLUSTER") == "0":

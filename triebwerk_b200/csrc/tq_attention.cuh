@@ -377,7 +377,7 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
 
 // MODE 0: queries pre-rotated and tile table built by append_rotate_kernel; 1: the kernel builds its table, rotates the
 // queries, optionally appends the step's token (one launch per layer and step); 2: whole-step form, see AttnParams; 3: as 1,
-// but the partials are only published (merge_partials_kernel<16> follows).
+// but the partials are only published (merge_partials_kernel<16> follows); 4: as 2 without the copy warps.
 // The whole-step form has two warps more, which issue the copies of one worker each.  With 16 warps at work it is a warpgroup more:
 // the launch brings 640 x 96 registers, of which the workers' warps take 112 each and the copy warps keep 32.
 template <int HKV, int MODE>
@@ -389,7 +389,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                         const AttnParams p) {
     using Geo = AttnGeom<BITS>;
     constexpr bool FUSED = MODE >= 1;
-    constexpr bool PERSIST = MODE == 2;
+    constexpr bool PERSIST = MODE == 2 || MODE == 4;
+    constexpr bool COPIER = MODE == 2;
     constexpr bool SEPARATE = MODE == 3;
     extern __shared__ __align__(1024) uint8_t dyn_smem[];
 
@@ -398,7 +399,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     const int warp = tid >> 5;
     constexpr int Hkv = HKV;  // compile time: row pitches, tile sizes and norm strides fold into immediates
     // whole-step form: lane 0 of each worker's copy warp keeps its ring filled
-    const bool copier = PERSIST && warp >= ATTN_GROUPS * Hkv;
+    const bool copier = COPIER && warp >= ATTN_GROUPS * Hkv;
     const int group = copier ? ((warp - ATTN_GROUPS * Hkv) & 1) : warp / Hkv;  // worker within the CTA
     const int head = warp - group * Hkv; // KV head of this warp
     const int gl = lane >> 2;            // mma "group id": token (K side), coordinate row (V side), head (S layout)
@@ -469,7 +470,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     if (gtid == 0) {
         for (int s = 0; s < 2 * ATTN_MAX_STAGES; ++s) {
             mbar_init(bar0 + 8u * s, 1);
-            if (PERSIST) mbar_init(ebar0 + 8u * s, Hkv);
+            if (COPIER) mbar_init(ebar0 + 8u * s, Hkv);
             else asm volatile("st.shared.u32 [%0], %1;" ::"r"(cnt0 + 4u * s), "r"(0u) : "memory");
         }
         if (PERSIST) mbar_init(a_base + 320u + 8u * (uint32_t)group, 1);
@@ -687,7 +688,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             }
         }
     };
-    if constexpr (PERSIST) {
+    if (PERSIST && !COPIER && gtid == 0 && loads_on) issue_queries(0, g);
+    if constexpr (COPIER) {
         if (copier) {
             // One thread per worker walks the worker's list and re-arms every part as soon as all its warps have handed it back.
             // (When the last warp to hand a part back did this itself, the cursor over the list, the counter's atomic and the
@@ -1244,7 +1246,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             const uint32_t parity = BITS == 2 ? s_par : ((uint32_t)(consumed >> s_log) & 1u);
             // the tile that takes this stage's place (warp-uniform; every warp of the worker advances the cursor in step)
             const int next_row = cl_row, next_tile = cl_tile, next_gend = cl_gend, next_layer = cl_layer;
-            const bool more = !PERSIST && cursor_more();
+            const bool more = !COPIER && cursor_more();
             if (more) cursor_advance();
             // Wait for one part (0: K codes and norms, 1: V codes and norms) of the stage.  Returns 0 at run time, as a
             // value PRODUCED by the wait: the part's loads take it into their address and so cannot move above the wait.
@@ -1270,7 +1272,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             // last warp of the worker to get here re-arms the part with the same part of the tile S ahead; nobody waits.
             auto release_part = [&](int part) {
                 __syncwarp();
-                if constexpr (PERSIST) {
+                if constexpr (COPIER) {
                     if (lane == 0) mbar_arrive(ebar0 + 16u * (uint32_t)s + 8u * (uint32_t)part);
                     return;
                 }
@@ -1580,7 +1582,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #endif
     // A warp that gave up on a wait may still have copies in flight: give them a bounded chance to land
     // before the CTA (and its shared memory) goes away.
-    if (!PERSIST && dead) {
+    if (!COPIER && dead) {
         for (int n = consumed; n < consumed + S && n < (int)(hi - lo) * n_layers; ++n) {
             mbar_wait_bounded(bar0 + 16u * (uint32_t)(n % S), (uint32_t)(n / S) & 1u, 1u << 16);
             mbar_wait_bounded(bar0 + 16u * (uint32_t)(n % S) + 8u, (uint32_t)(n / S) & 1u, 1u << 16);
