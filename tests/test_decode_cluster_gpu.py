@@ -132,15 +132,15 @@ def test_one_vector_append_vs_oracle(bits, G, Hkv):
     assert np.abs(gn.view(np.uint16).astype(np.int32) - wn.view(np.uint16).astype(np.int32)).max() <= 1
 
 
-@pytest.mark.parametrize("bits,msl", [(4, 288), (4, 320), (2, 288)])
+@pytest.mark.parametrize("bits,msl", [(4, 288), (4, 320), (2, 64), (2, 96)])
 def test_whole_steps_with_and_without_copy_warps(bits, msl):
     """128 sequences, too many for the cluster form: 4-bit slots of 36864 rows in all run without the copy warps on 148 SMs, of
-    40960 with them (the line is four tiles per worker: 37888 rows)."""
+    40960 with them (the line is four tiles per worker: 37888 rows); 2-bit ones of 8192 and 12288 (one tile: 9472)."""
     H, Hkv, NL, G = 16, 8, 2, 128
     rng = np.random.default_rng(3500 + bits + msl)
     R = ops.rotation_matrix().numpy()
-    lengths = [int(n) for n in rng.integers(1, 289, G)]
-    lengths[:6] = [1, 32, 33, 64, 287, 288]
+    lengths = [int(n) for n in rng.integers(1, min(msl, 288) + 1, G)]
+    lengths[:6] = [1, 32, 33, 64, min(msl, 288) - 1, min(msl, 288)]
     eng = tq.Engine(msl, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
     eng.alloc_batch(G, msl)
     pool = gu.dev(rng.standard_normal((2, 512, Hkv * D), dtype=np.float32).astype(np.float16))

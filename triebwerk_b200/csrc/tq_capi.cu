@@ -1595,9 +1595,9 @@ static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* 
     // With 8 KV heads the copy warps leave a worker's warps 112 registers instead of 128: a layer of a few tiles per worker, which is
     // one chain of segment starts and ends, is slower for it, from about four tiles on the freed instructions win.  4-bit, 28
     // layers, attention alone, with / without: 64 x 64 tokens 138 / 113 us, 64 x 256 219 / 200, 64 x 500 305 / 310, 32 heads
-    // 328 / 322, 64 x 4096 1740 / 1880.  In 2-bit they differ by 2 % at one tile and the copy warps win from two on (64 x 256 187 / 189).
+    // 328 / 322, 64 x 4096 1740 / 1880.  In 2-bit the line is at one tile: 64 x 64 110.7 / 108.7, 64 x 256 187 / 189.
     const int ctas = attention_ctas(G, e->msl);
-    const bool few = e->kv_bits == 4 && Hkv == 8 && e->total_rows <= 4ll * TILE_TOKENS * ctas * ATTN_GROUPS;
+    const bool few = Hkv == 8 && e->total_rows <= (e->kv_bits == 4 ? 4ll : 1ll) * TILE_TOKENS * ctas * ATTN_GROUPS;
     r = launch_attention(e->kv_bits, e->tmK4, e->tmV4, p, ctas, s, use_pdl() && !e->ev_attn[0], few ? 4 : 2);
     if (e->ev_attn[0]) cudaEventRecord(e->ev_attn[1], s);
     if (r != TQ_OK) return r;

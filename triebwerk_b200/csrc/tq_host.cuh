@@ -376,7 +376,7 @@ inline int launch_attention_t(const CUtensorMap& tmK, const CUtensorMap& tmV, co
 
 // mode 0: after append_rotate_kernel (rotated queries and tile table in the workspace); 1: one launch per layer and step
 // (table, query rotation, optional append and merge in the kernel); 2: whole-step form over AttnParams::n_layers layers; 3: as 1
-// with the merge left to merge_partials_kernel; 4: as 2 without the copy warps (4-bit, 8 KV heads only).
+// with the merge left to merge_partials_kernel; 4: as 2 without the copy warps (8 KV heads only).
 inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnParams& p, int ctas,
                             cudaStream_t s, bool pdl = false, int mode = 0) {
     if (p.Hkv != 8 && p.Hkv != 4) return TQ_ERR_UNSUPPORTED;
@@ -386,7 +386,7 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
                          : launch_attention_t<2, 8, MODE>(tmK, tmV, p, ctas, s, pdl);                           \
     return bits == 4 ? launch_attention_t<4, 4, MODE>(tmK, tmV, p, ctas, s, pdl)                                \
                      : launch_attention_t<2, 4, MODE>(tmK, tmV, p, ctas, s, pdl);
-    if (mode == 4) return launch_attention_t<4, 8, 4>(tmK, tmV, p, ctas, s, pdl);
+    if (mode == 4) return bits == 4 ? launch_attention_t<4, 8, 4>(tmK, tmV, p, ctas, s, pdl) : launch_attention_t<2, 8, 4>(tmK, tmV, p, ctas, s, pdl);
     if (mode == 2) { TQ_ATTN_DISPATCH(2) }
     if (mode == 3) { TQ_ATTN_DISPATCH(3) }
     if (mode == 1) { TQ_ATTN_DISPATCH(1) }
