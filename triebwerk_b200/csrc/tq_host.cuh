@@ -439,13 +439,17 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
 // 0.009 per cluster, the streaming form 17.7 + 0.030 per 1000 rows and KV heads + 0.4 per 1000 tokens of the longest sequence;
 // where the two are within 3 us it is the streaming form.  fp16: a tile costs the cluster form 1 us more than the streaming form's
 // share of it where there is one turn, less with more turns and with 8 query heads,
-// and that form starts 7 us later.  `extra`: us the streaming form's launches cost on top.
+// and that form starts 7 us later.  Above 640 clusters their number counts for more than in the lines fitted below it (128 x 64
+// tokens, 16/8 heads, 4-bit 25.7 / 19.7 us, 96 x 64 19.8 / 19.0, 64 x 64 13.5 / 17.2; 32/8 heads 128 x 64 26.8 / 24.9, 96 x 64 20 / 23;
+// fp16 128 x 300 43.0 / 39.1, 96 x 300 32.6 / 33.2).
+// `extra`: us the streaming form's launches cost on top.
 inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, double extra) {
     const long long clusters = (long long)G * Hkv, sms = device_props().sm_count;
     const int S = cluster_split(bits, clusters, heads, max_tokens);
     const double chain = ((max_tokens + 15) / 16) / (double)(S * CD_WARPS), turns = (double)((clusters * S + sms - 1) / sms);
-    if (bits == 0) return (heads > 4 ? 0.5 : 1.0) * chain < 7.0 + 1.5 * turns + extra;
-    return 0.4 * chain + 0.3 * chain * turns + 0.009 * clusters < 10.0 + 7e-6 * (double)rows * Hkv + 0.0004 * max_tokens + extra;
+    if (bits == 0) return (heads > 4 ? 0.5 : 1.0) * chain < 7.0 + 1.5 * turns + extra && !(clusters > 768 && chain > 2.0);
+    const double many = heads > 2 ? 0.0015 * std::max(0ll, clusters - 800) : 0.02 * std::max(0ll, clusters - 640);
+    return 0.4 * chain + 0.3 * chain * turns + 0.009 * clusters + many < 10.0 + 7e-6 * (double)rows * Hkv + 0.0004 * max_tokens + extra;
 }
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
 template <bool HOST, bool EXACT>
