@@ -161,6 +161,40 @@ def test_whole_steps_with_and_without_copy_warps(bits, msl):
             hp.assert_attention_close(out[layer, g][None], ref[None], H, D, f"tq{bits} layer {layer} sequence {g}")
 
 
+@pytest.mark.parametrize("bits,H,Hkv,NL,G,T", [
+    (4, 16, 8, 28, 16, 1000),  # plain and host-buffer steps as one launch, the others as four
+    (2, 32, 4, 28, 16, 2000),  # host-buffer steps only
+    (4, 16, 8, 4, 64, 64),     # all but the produced ones
+    (4, 16, 8, 4, 128, 300),   # none
+])
+def test_steps_agree_whatever_form_their_inputs_choose(bits, H, Hkv, NL, G, T):
+    """Plain, produced (unit norm weights on normed inputs, no rotation), two-phase and host-buffer steps of one batch choose between
+    one launch and four by different lines; results agree to the order of sums."""
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    eng = tq.Engine(T, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(G, T)
+    k, v = (torch.randn(G, T - 1, Hkv * D, generator=gen, device="cuda").half() for _ in range(2))
+    for layer in range(NL):
+        eng.prefill_append_batch(layer, 0, k, v)
+    eng.set_positions([T - 1] * G)
+    q, k, v = (torch.randn(NL, G, d, generator=gen, device="cuda").half() for d in (H * D, Hkv * D, Hkv * D))
+    want = eng.decode_step(q, k, v, torch.empty_like(q))
+    cache = [t.clone() for t in eng.layer_cache(NL - 1)]
+    two, rest = torch.empty_like(q), NL // 2 + 1
+    assert eng.step_prepare(q, k, v)
+    eng.step_attend_layers(0, rest, two)
+    eng.step_attend_layers(rest, NL - rest, two)
+    host = eng.decode_step_host(*(t.cpu().pin_memory() for t in (q, k, v)), torch.empty(q.shape, dtype=torch.float16, pin_memory=True)).cuda()
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(cache, eng.layer_cache(NL - 1)))
+    ones, cos, sin = torch.ones(NL, D, device="cuda").half(), torch.ones(T, 64, device="cuda").half(), torch.zeros(T, 64, device="cuda").half()
+    qn, kn = ((t.view(-1, D).float() * torch.rsqrt(t.view(-1, D).float().pow(2).mean(-1, keepdim=True) + 1e-6)).half().view(t.shape) for t in (q, k))
+    produced = eng.decode_step_produce(q, k, v, torch.empty_like(q), ones, ones, cos, sin)
+    plain = eng.decode_step(qn, kn, v, torch.empty_like(q))
+    assert eng.status() == 0
+    for name, got, ref in (("two phases", two, want), ("host", host, want), ("produced", produced, plain)):
+        hp.assert_attention_close(gu.host(got).reshape(-1, H * D), gu.host(ref).reshape(-1, H * D), H, D, name)
+
+
 def test_streaming_forms_in_a_child_process():
     """TQ_CLUSTER=0 (read once per process) keeps the streaming kernels for small batches too."""
     if os.environ.get("TQ_CLUSTER") == "0":

@@ -2,6 +2,7 @@
 // The whole library is this one translation unit; kernels live in the .cuh files it includes.
 
 #include <algorithm>
+#include <cmath>
 
 #include "tq_host.cuh"
 
@@ -1459,24 +1460,46 @@ static bool engine_whole_step_ok(const tq_engine* e, const void* q, const void* 
 
 static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* out, cudaStream_t s, const tq_step_producer* prod);
 
+// How a step's inputs reach the cluster form.  Plain: device buffers.  Produced: a launch that appends and one that produces the
+// queries come first all the same.  TwoPhase: the same, and the layers follow in groups.  Host: pinned host buffers.
+enum class StepInputs { Plain, Produced, TwoPhase, Host };
+
 // Is a whole step of this engine's batch faster as one launch of the cluster form over all layers than in the whole-step form's
-// four launches?  Both times, in ns, are lines in what bounds them (1500 steps of 1 to 128 sequences x 64 to 16384 tokens, equal
-// and ragged, 4 to 36 layers): the one launch 2500 + 18 per cluster (sequence, KV head, layer; with 8 query heads 32, 15 in 2-bit,
-// whose tables are smaller) + 300 per tile of its longest warp + 0.038 per row and KV head, the four 22000 + 3500 per layer +
-// 0.032 per row and KV head (0.038 with 8 query heads in 2-bit).  28 layers of 1 x 256 tokens 9 / 137 us, 4 x 4096 186 / 311, 16 x
-// 1024 222 / 240, 16 x 4096 647 / 595, 64 x 64 352 / 195; 8 ragged layers of 95 x 6..433 187 / 140.  fp16 caches have no whole-step
-// form: the one launch saves 10 us a layer; a tile of its longest warp costs it 600 ns, a cached row and KV head 2 ps more.
-// It depends on the engine's batch alone: every call that runs a step, or part of one, takes the same form and gives the same bits.
-static bool engine_step_small(const tq_engine* e) {
+// four launches?  Both times, in us, as lines in what bounds them, fitted to 336 steps of 4 to 128 sequences x 64 to 4000 tokens, 4
+// and 28 layers, in both forms (average loss against the better form 0.3 %, largest 19 %):
+//   the one launch   3.5 + per CTA a fixed part and one per round of its warps through 32 tokens each
+//   four launches    26 + per layer, more with 8 KV heads and per query head, + a share per cached row and KV head
+// 28 layers, 16/8 heads, 4-bit, one launch / four: 8 x 1000 tokens 121 / 197, 24 x 300 191 / 159, 16 x 2000 358 / 336, 64 x 64 341 / 177.
+// Produced inputs cost the one launch 10 us more than the four (16 x 300 tokens 163 / 170, 16 x 1000 253 / 234); two phases with four
+// groups of layers a last round per group, and the four launches one more per group (28 layers 16 x 2000 444 / 385, 4 layers 32 x
+// 300 61 / 93).  From host buffers the four launches run in groups of layers under the copies of others, 60 us and more of latency
+// on top; the one launch reads over the bus as it goes (16 x 2000 404 / 510, 24 x 2000 579 / 609, 64 x 300 612 / 592).
+// fp16 caches have no whole-step form: the one launch saves 10 us a layer; a tile of its longest warp costs it 600 ns, a cached row
+// and KV head 2 ps more.  It depends on the engine's batch alone: every call that runs a part of a step takes the form of the whole.
+static bool engine_step_small(const tq_engine* e, StepInputs inputs) {
     if (!e->fused || !e->whole_step || e->G > 65535) return false;
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads, NL = e->shape.num_layers, heads = H / Hkv;
     if (!fast_shape(H, Hkv, e->kv_bits != 0)) return true;
     if (!cluster_on()) return false;
     const long long clusters = (long long)e->G * Hkv * NL;
-    const double tiles = ((e->msl + 15) / 16) / (double)(CD_WARPS * cluster_split(e->kv_bits, clusters, heads, e->msl));
-    if (e->kv_bits == 0) return 600.0 * tiles + 2.0 * clusters + 0.002 * (double)e->total_rows * Hkv * NL < 2000.0 + 10000.0 * NL;
-    const double per_cluster = heads <= 4 ? 18.0 : e->kv_bits == 4 ? 32.0 : 15.0, per_row = heads > 4 && e->kv_bits == 2 ? 0.0 : 0.006;
-    return per_cluster * clusters + per_row * (double)e->total_rows * Hkv * NL + 300.0 * tiles < 20000.0 + 3500.0 * NL;
+    const int S = cluster_split(e->kv_bits, clusters, heads, e->msl);
+    if (e->kv_bits == 0) {
+        const double tiles = ((e->msl + 15) / 16) / (double)(CD_WARPS * S);
+        return 600.0 * tiles + 2.0 * clusters + 0.002 * (double)e->total_rows * Hkv * NL < 2000.0 + 10000.0 * NL;
+    }
+    const bool b4 = e->kv_bits == 4, wide = heads > 4;
+    auto rounds = [&](double tokens) { return tokens <= 16.0 * CD_WARPS * S ? 0.5 : std::ceil(tokens / (32.0 * CD_WARPS * S)); };
+    const double fixed = !wide ? 0.016 : (b4 ? 0.030 : 0.018), round = !wide ? (b4 ? 0.0103 : 0.0092) : (b4 ? 0.0156 : 0.0101);
+    double one = 3.5 + (double)clusters * S * (fixed + round * rounds((double)e->total_rows / e->G)) + 0.5 * rounds(e->msl);
+    const double per_row = Hkv == 8 ? (b4 ? 32e-6 : 26e-6) : (b4 ? 40e-6 : 35e-6);
+    double four = 26.0 + NL * ((Hkv == 8 ? 3.0 : 1.7) + 0.0375 * H) + 0.0008 * e->G * H * NL + per_row * (double)e->total_rows * Hkv * NL;
+    switch (inputs) {
+        case StepInputs::Plain: break;
+        case StepInputs::Produced: one += 10.0; break;
+        case StepInputs::TwoPhase: one += 2.0 * rounds(e->msl) + 0.5 * NL - 20.0; four *= 0.9; break;
+        case StepInputs::Host: four = 1.05 * four + 60.0; break;
+    }
+    return one < four;
 }
 
 // The layers l0 .. l0 + n - 1 of such a step; q, k, v, out point at layer l0's [G][dim] blocks.
@@ -1545,7 +1568,7 @@ static int engine_step_layers(tq_engine* e, int l0, int n, const void* q, const 
                               const tq_step_producer* prod = nullptr) {
     // A small step: the produced queries and keys, then the cluster form.  (It stores the new token's bytes once more, the same.)
     const size_t qo = (size_t)l0 * e->G * e->q_dim() * 2, ko = (size_t)l0 * e->G * e->kv_dim() * 2;
-    if (prod && !prod->rotated_output && engine_step_small(e) && engine_cluster_ok(e, (char*)e->step_qrot + qo, (char*)e->step_kpost + ko, v, out)) {
+    if (prod && !prod->rotated_output && engine_step_small(e, StepInputs::Produced) && engine_cluster_ok(e, (char*)e->step_qrot + qo, (char*)e->step_kpost + ko, v, out)) {
         int r = engine_step_prepare(e, l0, n, q, k, v, s, prod, true);
         return r != TQ_OK ? r : engine_cluster_step(e, l0, n, (char*)e->step_qrot + qo, (char*)e->step_kpost + ko, v, out, s);
     }
@@ -1648,7 +1671,7 @@ int tq_engine_step_prepare(tq_engine* e, const void* q, const void* k, const voi
     if (!e || !q || !k || !v) return TQ_ERR_ARG;
     if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     if (!engine_whole_step_ok(e, q, k, v, q)) return TQ_ERR_UNSUPPORTED;
-    if (engine_step_small(e) && engine_cluster_ok(e, e->stage_q, e->stage_k, e->stage_v, q)) {
+    if (engine_step_small(e, StepInputs::TwoPhase) && engine_cluster_ok(e, e->stage_q, e->stage_k, e->stage_v, q)) {
         // the second phase runs the cluster form, on copies of the step's inputs
         const size_t qb = (size_t)e->shape.num_layers * e->G * e->q_dim() * 2, kb = (size_t)e->shape.num_layers * e->G * e->kv_dim() * 2;
         TQ_CUDA(cudaMemcpyAsync(e->stage_q, q, qb, cudaMemcpyDeviceToDevice, cs(s)));
@@ -1663,7 +1686,7 @@ int tq_engine_step_attend_layers(tq_engine* e, int first_layer, int n_layers, vo
     if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     if (!engine_whole_step_ok(e, out_first, out_first, out_first, out_first)) return TQ_ERR_UNSUPPORTED;
     const size_t qo = (size_t)first_layer * e->G * e->q_dim() * 2, ko = (size_t)first_layer * e->G * e->kv_dim() * 2;
-    if (engine_step_small(e) && engine_cluster_ok(e, e->stage_q, e->stage_k, e->stage_v, out_first))
+    if (engine_step_small(e, StepInputs::TwoPhase) && engine_cluster_ok(e, e->stage_q, e->stage_k, e->stage_v, out_first))
         return engine_cluster_step(e, first_layer, n_layers, (char*)e->stage_q + qo, (char*)e->stage_k + ko, (char*)e->stage_v + ko, out_first, cs(s));
     return engine_step_attend(e, first_layer, n_layers, nullptr, out_first, cs(s), nullptr);
 }
@@ -1671,7 +1694,7 @@ int tq_engine_step_attend_layers(tq_engine* e, int first_layer, int n_layers, vo
 // The layers l0 .. l0 + n - 1 of a step whose inputs are all there, in the form that is fastest for the whole step's size.
 static int engine_decode_range(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s) {
     const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
-    if (engine_step_small(e) && engine_cluster_ok(e, q, k, v, out)) return engine_cluster_step(e, l0, n, q, k, v, out, s);
+    if (engine_step_small(e, StepInputs::Plain) && engine_cluster_ok(e, q, k, v, out)) return engine_cluster_step(e, l0, n, q, k, v, out, s);
     if (engine_whole_step_ok(e, q, k, v, out)) return engine_step_layers(e, l0, n, q, k, v, out, s);
     for (int i = 0; i < n; ++i) {
         int r = tq_engine_decode_layer(e, l0 + i, (const char*)q + qb * i, (const char*)k + kb * i, (const char*)v + kb * i, (char*)out + qb * i,
@@ -1934,7 +1957,7 @@ int tq_engine_decode_step_host(tq_engine* e, const void* q_host, const void* k_h
     // 2.5 KB of inputs over the bus itself and writes its results there.  Copies cost 10 us of latency each, 40 us before the
     // first kernel can start, and the launches of the groups that overlap them 15 % of the GPU (28 layers, 16 sequences x 2019
     // tokens, 16/8 heads: 521 / 415 us; 1 x 300 tokens 264 / 38).
-    if (engine_step_small(e)) {
+    if (engine_step_small(e, StepInputs::Host)) {
         void* d[4] = {nullptr, nullptr, nullptr, nullptr};
         const void* h[4] = {q_host, k_host, v_host, out_host};
         bool reach = true;
