@@ -3,9 +3,12 @@ host-only entry points (rotation generator, sizing, argument checks) behave.  No
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
+import torch
 
 import triebwerk_b200 as tq
 from triebwerk_b200._lib import ModelShape
@@ -160,3 +163,17 @@ def test_reference_engine_links_against_this_library_for_the_path():
     hdr_text = open(os.path.join(ROOT, "include", "triebwerk_b200.h")).read()
     for name in sorted(path):
         assert params(ref_text, name) == params(hdr_text, name), name
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="what a machine without a GPU does")
+@pytest.mark.parametrize("call", [
+    "tq.ops.launch_kv_cache_write_batch(None, None, None, None, None, 1, 1, 128)",  # there is no current stream
+    "with FakeTensorMode():\n    t = torch.empty(1, 128, dtype=torch.float16, device='cuda')\n"
+    "    tq.ops.launch_kv_cache_write_batch(t, t, t, t, t, 1, 1, 128)",             # there is no data pointer
+])
+def test_what_torch_throws_is_a_python_error(call):
+    """... and not the end of the process: in a child, which would be gone."""
+    src = ("import torch, triebwerk_b200 as tq\nfrom torch._subclasses.fake_tensor import FakeTensorMode\n"
+           "try:\n" + "".join(f"    {line}\n" for line in call.split("\n")) + "except RuntimeError as e:\n    print('caught', type(e).__name__)")
+    r = subprocess.run([sys.executable, "-c", src], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "caught" in r.stdout, f"{r.returncode}: {r.stderr[-600:]}"

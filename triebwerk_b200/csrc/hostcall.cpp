@@ -8,7 +8,7 @@
 //
 // Every function is made by one template from the declaration in triebwerk_b200.h: pointer parameters take a tensor
 // (CUDA, contiguous), None or an address, int parameters a number; a trailing tq_stream_t is torch's current stream.
-// They return the status (launchers: that of tq_last_compat_status()).
+// They return the status (launchers: that of tq_last_compat_status()).  No C++ exception leaves them.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -16,6 +16,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <exception>
+#include <tuple>
 #include <type_traits>
 #include <utility>
 
@@ -66,15 +68,24 @@ struct Call<Fn, need> {
     template <size_t... I>
     static PyObject* go(PyObject* const* args, std::index_sequence<I...>) {
         std::tuple<std::decay_t<A>...> v{};
-        if (!(convert(args[I], need, &std::get<I>(v)) && ...)) return nullptr;
-        std::get<N>(v) = (tq_stream_t)c10::cuda::getCurrentCUDAStream().stream();
+        try {
+            if (!(convert(args[I], need, &std::get<I>(v)) && ...)) return nullptr;
+            std::get<N>(v) = (tq_stream_t)c10::cuda::getCurrentCUDAStream().stream();
+        } catch (const std::exception& e) {  // torch throws: a machine without a GPU, a tensor without memory of its own
+            PyErr_SetString(PyExc_RuntimeError, e.what());
+            return nullptr;
+        }
         int status = 0;
         Py_BEGIN_ALLOW_THREADS
-        if constexpr (std::is_void_v<R>) {
-            std::apply(Fn, v);
-            status = tq_last_compat_status();
-        } else {
-            status = std::apply(Fn, v);
+        try {
+            if constexpr (std::is_void_v<R>) {
+                std::apply(Fn, v);
+                status = tq_last_compat_status();
+            } else {
+                status = std::apply(Fn, v);
+            }
+        } catch (const std::exception&) {  // (the library's own containers)
+            status = TQ_ERR_NOMEM;
         }
         Py_END_ALLOW_THREADS
         return PyLong_FromLong(status);
