@@ -177,3 +177,24 @@ def test_what_torch_throws_is_a_python_error(call):
            "try:\n" + "".join(f"    {line}\n" for line in call.split("\n")) + "except RuntimeError as e:\n    print('caught', type(e).__name__)")
     r = subprocess.run([sys.executable, "-c", src], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "caught" in r.stdout, f"{r.returncode}: {r.stderr[-600:]}"
+
+
+def test_positions_are_taken_as_any_number():
+    """The single-sequence launchers take the position as Python, numpy and torch make it, as int() does."""
+    for name in ("launch_turbo_gqa_attention", "launch_gqa_attention"):
+        seen = []
+        old = tq._lib.hostcall.__dict__.get(name)
+        tq._lib.hostcall.__dict__[name] = lambda *a: seen.append(a) or 0
+        try:
+            n = 14 if name == "launch_turbo_gqa_attention" else 10
+            at = 8 if name == "launch_turbo_gqa_attention" else 5
+            for pos in (3, 3.0, np.int64(3), np.float32(3), torch.tensor(3), torch.tensor(3.0)):
+                args = [None] * n
+                args[at] = pos
+                getattr(tq.ops, name)(*args)
+        finally:
+            if old is None:
+                del tq._lib.hostcall.__dict__[name]
+            else:
+                tq._lib.hostcall.__dict__[name] = old
+        assert [type(a[at]) for a in seen] == [int] * 6 and {a[at] for a in seen} == {3}

@@ -48,7 +48,7 @@ def launch_turbo_gqa_attention_batch(out, q, ck_q, cv_q, k_norms, v_norms, rotat
 
 def launch_turbo_gqa_attention(q, ck_q, cv_q, k_norms, v_norms, rotation, output, attn_scratch, pos, msl, num_heads,
                                num_kv_heads, head_dim, bits):
-    st = hostcall.launch_turbo_gqa_attention(q, ck_q, cv_q, k_norms, v_norms, rotation, output, attn_scratch, pos, msl,
+    st = hostcall.launch_turbo_gqa_attention(q, ck_q, cv_q, k_norms, v_norms, rotation, output, attn_scratch, int(pos), msl,
                                              num_heads, num_kv_heads, head_dim, bits)
     if st:
         raise TqError(st, "launch_turbo_gqa_attention")
@@ -78,7 +78,7 @@ def launch_gqa_attention_batch(out, q, ck, cv, attn_scratch, pos, msl, G, num_he
 
 def launch_gqa_attention(q, k_cache, v_cache, output, attn_scratch, pos, max_seq_len, num_heads, num_kv_heads,
                          head_dim):
-    st = hostcall.launch_gqa_attention(q, k_cache, v_cache, output, attn_scratch, pos, max_seq_len, num_heads,
+    st = hostcall.launch_gqa_attention(q, k_cache, v_cache, output, attn_scratch, int(pos), max_seq_len, num_heads,
                                        num_kv_heads, head_dim)
     if st:
         raise TqError(st, "launch_gqa_attention")
