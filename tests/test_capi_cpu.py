@@ -198,3 +198,20 @@ def test_positions_are_taken_as_any_number():
             else:
                 tq._lib.hostcall.__dict__[name] = old
         assert [type(a[at]) for a in seen] == [int] * 6 and {a[at] for a in seen} == {3}
+
+
+def test_engine_calls_that_launch_kernels_check_the_device():
+    """An engine's pointers belong to one device: with another one current its kernels would read memory that is not theirs.  There is
+    one device at most to test on, so the source is read: every call with a stream that does more than copy begins with the check,
+    or hands over to one that does."""
+    src = open(os.path.join(ROOT, "triebwerk_b200", "csrc", "tq_capi.cu")).read()
+    copies = {"tq_engine_reset", "tq_engine_status", "tq_engine_set_positions", "tq_engine_set_rotation", "tq_engine_read_output_f32"}
+    bodies = {m.group(1): m.group(2) for m in re.finditer(r"^(?:static )?int (\w+)\([^{;]*?\) \{\n(.*?)^\}", src, re.S | re.M)}
+    calls = [n for n in re.findall(r"^int (tq_engine_\w+)\([^)]*tq_stream_t[^)]*\) \{", src, re.M) if n not in copies]
+    assert len(calls) >= 16
+
+    def checks(name):
+        first = re.search(r"engine_on_its_device|((?:tq_)?engine_\w+)\(e,", bodies[name])  # whichever comes first
+        return first and (first.group(1) is None or first.group(1) in bodies and checks(first.group(1)))
+
+    assert not [n for n in calls if not checks(n)]

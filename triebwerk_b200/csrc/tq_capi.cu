@@ -1266,7 +1266,7 @@ __global__ void advance_positions_kernel(int* pos, int n) {
 
 int tq_engine_advance(tq_engine* e, tq_stream_t s) {
     if (e) e->chain_ok = false;  // not a fused decode launch: the next one reads nothing early
-    if (!e || !e->arena || e->G == 0) return TQ_ERR_STATE;
+    if (!e || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     advance_positions_kernel<<<(e->G + 127) / 128, 128, 0, cs(s)>>>(e->d_positions, e->G);
     return cuda_status(cudaGetLastError());
 }
@@ -1421,7 +1421,7 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
 int tq_engine_attend_layer(tq_engine* e, int layer, void* out, tq_stream_t s) {
     if (e) e->chain_ok = false;  // not a fused decode launch: the next one reads nothing early
     if (!e || layer < 0 || layer >= e->shape.num_layers || !out) return TQ_ERR_ARG;
-    if (e->asleep || !e->arena || e->G == 0) return TQ_ERR_STATE;
+    if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     if (e->kv_bits == 0 || !fast_shape(e->shape.num_heads, e->shape.num_kv_heads, true)) return TQ_ERR_UNSUPPORTED;
     const tq_engine::Layer& L = e->layers[layer];
     // the tile table of the current positions (a launch of the append kernel without vectors), then the attention
@@ -1950,7 +1950,7 @@ int tq_engine_prefill_layer(tq_engine* e, int layer, int seq, const void* q, con
 int tq_engine_decode_step_host(tq_engine* e, const void* q_host, const void* k_host, const void* v_host, void* out_host,
                                tq_stream_t s) {
     if (!e || !q_host || !k_host || !v_host || !out_host) return TQ_ERR_ARG;
-    if (e->asleep || !e->arena || e->G == 0) return TQ_ERR_STATE;
+    if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
     const int NL = e->shape.num_layers;
     const size_t qb = (size_t)e->G * e->q_dim() * 2, kb = (size_t)e->G * e->kv_dim() * 2;
     // A small step straight on the host buffers, where the device can reach them (pinned memory): every CTA fetches its 0.5 to
