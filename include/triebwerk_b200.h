@@ -369,7 +369,9 @@ int tq_engine_prefill_append_batch(tq_engine* e, int layer, int first_seq, int n
 /* One layer of a prompt's prefill (engine/engine.cpp:2110-2146: the cache write of all T tokens, then the causal
  * self-attention): k/v [T][kv_dim] of sequence `seq` go to positions 0 .. T-1 of its slot, and query token t of
  * q [T][q_stride] attends to rows 0 .. t; out [T][q_stride] (the reference passes one stride, Q_PROJ_DIM, for both).
- * Packed modes and kv_bits = 0; sequences behind a shared prefix are refused (TQ_ERR_STATE). */
+ * Packed modes and kv_bits = 0; sequences behind a shared prefix are refused (TQ_ERR_STATE).  Prompts may come on several
+ * streams: packed ones, whose rows pass through one scratch of the engine, take turns there.  (Captured calls are not ordered
+ * against others: a graph's replay must not overlap another prompt of the engine.) */
 int tq_engine_prefill_layer(tq_engine* e, int layer, int seq, const void* q, const void* k, const void* v, void* out, int T,
                             int q_stride, tq_stream_t s);
 /* The same for the n_seq prompts of T tokens of the sequences first_seq .. : q and out [n_seq][T][q_stride], k/v

@@ -140,6 +140,32 @@ def test_prompts_pass_through_the_scratch_in_groups():
     assert eng.status() == 0
 
 
+def test_prompts_on_two_streams_share_the_scratch_in_turn():
+    """Prompts of two sequences, layer by layer on a stream each: their fp16 rows go through one scratch, whose second user waits for
+    the first one's kernels."""
+    H, Hkv, T, NL, msl = 16, 8, 777, 16, 1024
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (torch.randn(2, NL, T, d, generator=gen, device="cuda").half() for d in (H * D, Hkv * D, Hkv * D))
+    eng = tq.Engine(msl, 4, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(2, msl)
+    want = torch.stack([torch.stack([eng.prefill_layer(i, s, q[s, i], k[s, i], v[s, i]) for i in range(NL)]) for s in range(2)])
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for delay in range(0, 60000, 3000):  # (cycles by which one stream is late: its conversions meet the other's products)
+        got = torch.zeros_like(want)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[1]):
+            torch.cuda._sleep(200000 + delay)
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(200000)
+        for i in range(NL):
+            for s in range(2):
+                with torch.cuda.stream(streams[s]):
+                    eng.prefill_layer(i, s, q[s, i], k[s, i], v[s, i], got[s, i])
+        torch.cuda.synchronize()
+        assert eng.status() == 0
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("bits", [4, 2])
 def test_long_prompt_passes_through_the_scratch_by_kv_heads(bits):
     """16500 tokens x 8 KV heads do not fit the scratch as a whole: 4 heads, then 4.  The launcher, whose scratch holds the prompt,

@@ -878,6 +878,7 @@ void tq_engine_destroy(tq_engine* e) {
     if (e->d_rotation_prep) cudaFree(e->d_rotation_prep);
     if (e->d_rotation_rep) cudaFree(e->d_rotation_rep);
     if (e->out_f32) cudaFree(e->out_f32);
+    if (e->ev_prefill) cudaEventDestroy(e->ev_prefill);
     if (e->st_in) {
         cudaStreamDestroy(e->st_in);
         cudaStreamDestroy(e->st_out);
@@ -1939,7 +1940,23 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
         r = compat_workspace(least, &ws, cs(s));
         return r != TQ_OK ? r : launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, ws, least, cs(s));
     }
-    return launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s));
+    if (e->kv_bits == 0) return launch_prefill_attention(0, ap, e->total_rows - row0, nullptr, 0, cs(s));
+    std::lock_guard<std::mutex> lock(e->prefill_mutex);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TQ_CUDA(cudaStreamIsCapturing(cs(s), &capture));
+    const bool ordered = capture == cudaStreamCaptureStatusNone;  // (a captured call runs when its graph does: the caller orders that)
+    unsigned long long id = 0;
+    if (ordered) {
+        TQ_CUDA(cudaStreamGetId(cs(s), &id));
+        if (!e->ev_prefill) TQ_CUDA(cudaEventCreateWithFlags(&e->ev_prefill, cudaEventDisableTiming));
+        if (e->prefill_stream_id != 0 && e->prefill_stream_id != id) TQ_CUDA(cudaStreamWaitEvent(cs(s), e->ev_prefill, 0));
+    }
+    r = launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s));
+    if (ordered) {
+        TQ_CUDA(cudaEventRecord(e->ev_prefill, cs(s)));
+        e->prefill_stream_id = id;
+    }
+    return r;
 }
 
 int tq_engine_prefill_layer(tq_engine* e, int layer, int seq, const void* q, const void* k, const void* v, void* out, int T,

@@ -810,6 +810,10 @@ struct tq_engine {
     void* step_kpost = nullptr;        // [layers][G][kv_dim] fp16: K after QK-norm and rotary embedding (producer form)
     void* prefill_scratch = nullptr;   // packed modes: fp16 rows and fp32 norms of prompts (launch_prefill_attention)
     size_t prefill_scratch_bytes = 0;
+    // Its users are calls on any stream of any host thread: a call on another stream than the last one's waits for that one's kernels.
+    std::mutex prefill_mutex;
+    cudaEvent_t ev_prefill = nullptr;           // behind the last use
+    unsigned long long prefill_stream_id = 0;   // whose stream it was (0: none yet)
     bool whole_step = !(getenv("TQ_WHOLE_STEP") && atoi(getenv("TQ_WHOLE_STEP")) == 0);
     float* out_f32 = nullptr;          // optional [layers][G][H][128]: results before the fp16 rounding (outside the arena)
     cudaEvent_t ev_attn[2] = {nullptr, nullptr};  // optional: recorded around the attention launch of the whole-step form
