@@ -215,3 +215,17 @@ def test_engine_calls_that_launch_kernels_check_the_device():
         return first and (first.group(1) is None or first.group(1) in bodies and checks(first.group(1)))
 
     assert not [n for n in calls if not checks(n)]
+
+
+@pytest.mark.parametrize("G,msl", [(1, 512), (1, 1536), (4, 256)])
+def test_arena_of_a_small_engine_stays_in_proportion(G, msl):
+    """The 64 MiB for prompts as fp16 rows are for batches that can use them; an engine whose slots fit 16 MiB takes those."""
+    arena = {n: tq.Engine(msl, 4, num_layers=n, num_heads=16, num_kv_heads=8, head_dim=128).arena_bytes(G, msl) for n in (1, 2)}
+    one_layer = arena[2] - arena[1]  # cache, partial results, staging of a layer
+    assert arena[1] - one_layer <= (17 << 20) + (10 << 20)  # (10 MiB: the decode workspace)
+
+
+def test_arena_holds_slots_longer_than_the_given_length():
+    """Slots of capacities beyond max_seq_len (rounded up to 32 rows, or given so): what arena_bytes says is what alloc_batch carves."""
+    e = tq.Engine(100, 4, num_layers=2, num_heads=16, num_kv_heads=8, head_dim=128)
+    assert e.arena_bytes(2, 100, [100, 4000]) == e.arena_bytes(2, 4000, [100, 4000])

@@ -946,9 +946,14 @@ static size_t engine_carve(tq_engine* e, char* base, int G, int msl, long long r
     const size_t qb = (size_t)e->shape.num_layers * G * e->q_dim() * 2;
     const size_t kb = (size_t)e->shape.num_layers * G * e->kv_dim() * 2;
     size_t oq = bump(off, qb), okk = bump(off, kb), ovv = bump(off, kb), oo = bump(off, qb);
-    // prompts on their way through the prefill attention as fp16 rows: 16384 tokens of 8 KV heads whatever the slots hold (64 MiB:
-    // half of L2, where the attention reads them again); longer prompts pass through it some KV heads at a time
-    const size_t pf_bytes = e->kv_bits ? prefill_scratch_bytes(131072, 1, false) : 0;
+    // prompts on their way through the prefill attention as fp16 rows: 16384 tokens of 8 KV heads (64 MiB: half of L2, where the
+    // attention reads them again; more pass through it some prompts or KV heads at a time), or 16 MiB where all slots together fit
+    size_t pf_bytes = 0;
+    if (e->kv_bits) {
+        const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
+        const size_t all = (size_t)G * prefill_scratch_bytes(msl, Hkv, prefill_exact(e->kv_bits, H, Hkv)), small = prefill_scratch_bytes(32768, 1, false);
+        pf_bytes = all <= small ? small : prefill_scratch_bytes(131072, 1, false);
+    }
     size_t opf = bump(off, pf_bytes);
     if (assign) {
         e->prefill_scratch = e->kv_bits ? base + opf : nullptr;
@@ -975,8 +980,11 @@ static size_t engine_carve(tq_engine* e, char* base, int G, int msl, long long r
 
 size_t tq_engine_arena_bytes(const tq_engine* e, int G, int max_seq_len, const int* capacities) {
     if (!e || G <= 0 || max_seq_len <= 0) return 0;
-    long long rows = plan_rows(G, max_seq_len, capacities, nullptr, nullptr);
-    return engine_carve(const_cast<tq_engine*>(e), nullptr, G, max_seq_len, rows, capacities != nullptr, false);
+    std::vector<int> caps;
+    long long rows = plan_rows(G, max_seq_len, capacities, &caps, nullptr);
+    int msl = max_seq_len;  // as tq_engine_alloc_batch sees it: a slot may be longer
+    for (int c : caps) msl = c > msl ? c : msl;
+    return engine_carve(const_cast<tq_engine*>(e), nullptr, G, msl, rows, capacities != nullptr, false);
 }
 
 int tq_engine_set_arena(tq_engine* e, void* device_ptr, size_t bytes) {
