@@ -1,6 +1,10 @@
 """The tcgen05 prefill attention (csrc/tq_prefill_fa.cuh) where it can go wrong: edges of its 128-row tiles and query blocks, one
 and two query blocks per CTA, any number of query heads per KV head, prompts that go through the scratch in groups.  Against the
 oracle on the engine's own cache bytes."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -168,8 +172,8 @@ def test_prompts_on_two_streams_share_the_scratch_in_turn():
 
 @pytest.mark.parametrize("bits", [4, 2])
 def test_long_prompt_passes_through_the_scratch_by_kv_heads(bits):
-    """16500 tokens x 8 KV heads do not fit the scratch as a whole: 4 heads, then 4.  The launcher, whose scratch holds the prompt,
-    computes every column in the same order: the same bits."""
+    """16500 tokens x 8 KV heads do not fit the scratch as a whole: 4 heads, then 4.  The launcher, given those two halves' heads as
+    caches of their own, which fit, computes every column in the same order: the same bits; given the prompt as a whole, too."""
     H, Hkv, T, msl = 16, 8, 16500, 16512
     gen = torch.Generator(device="cuda").manual_seed(6)
     k, v = (torch.randn(T, Hkv * D, generator=gen, device="cuda").half() for _ in range(2))
@@ -182,3 +186,39 @@ def test_long_prompt_passes_through_the_scratch_by_kv_heads(bits):
     tq.ops.launch_turbo_gqa_prefill_attention(want, q, ck, cv, kn, vn, tq.ops.rotation_matrix().cuda(), None, T, msl, H, Hkv, D, H * D, Hkv * D, bits)
     assert eng.status() == 0
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    for half in range(2):
+        sl = slice(half * Hkv // 2, (half + 1) * Hkv // 2)
+        part = [t.view(msl, Hkv, -1)[:, sl].reshape(msl, -1).contiguous() for t in (ck, cv, kn, vn)]
+        cols = slice(half * H // 2 * D, (half + 1) * H // 2 * D)
+        o = torch.empty(T, H // 2 * D, dtype=torch.float16, device="cuda")
+        tq.ops.launch_turbo_gqa_prefill_attention(o, q[:, cols].contiguous(), *part, tq.ops.rotation_matrix().cuda(), None, T, msl, H // 2, Hkv // 2,
+                                                  D, H // 2 * D, Hkv // 2 * D, bits)
+        assert torch.equal(got[:, cols].contiguous().view(torch.int16), o.view(torch.int16))
+
+
+def test_a_long_prompt_through_the_launcher_can_be_captured():
+    """16500 tokens x 8 KV heads are 135 MB as fp16 rows; the launchers' workspace, 64 MiB after their first call, serves them some KV
+    heads at a time and need not grow, which it cannot under capture.  In a child: the workspace is the process's."""
+    src = """
+import torch, triebwerk_b200 as tq
+H, Hkv, D, T, msl = 16, 8, 128, 16500, 16512
+R = tq.ops.rotation_matrix().cuda()
+ck, cv = (torch.randint(0, 256, (msl, Hkv * 64), dtype=torch.uint8, device='cuda') for _ in range(2))
+kn, vn = (torch.rand(msl, Hkv, device='cuda').half() for _ in range(2))
+q = torch.randn(T, H * D, device='cuda').half()
+out, want = torch.zeros_like(q), torch.zeros_like(q)
+run = lambda o, t: tq.ops.launch_turbo_gqa_prefill_attention(o, q, ck, cv, kn, vn, R, None, t, msl, H, Hkv, D, H * D, Hkv * D, 4)
+run(want, 100)  # (the first call allocates)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    run(out, T)
+g.replay()
+run(want, T)
+torch.cuda.synchronize()
+assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+print('captured')
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", src], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]

@@ -688,7 +688,10 @@ static int compat_prefill_attention(void* out, const void* q, const void* ck, co
     void* ws = nullptr;
     const bool aligned = (((uintptr_t)q | (uintptr_t)out | (uintptr_t)ck | (uintptr_t)cv | (uintptr_t)rotation) & 15u) == 0 && q_dim % 8 == 0;
     if (aligned && prefill_attn_shape(H, Hkv)) {
-        const size_t scratch = bits ? prefill_scratch_bytes(T, Hkv, prefill_exact(bits, H, Hkv)) : 0;
+        // packed: room for the whole prompt as fp16 rows, or what is left of 64 MiB for some of its KV heads at a time.  That is the
+        // workspace's first size: a long prompt does not make it grow, nor fail under stream capture for having to.
+        const bool exact = prefill_exact(bits, H, Hkv);
+        const size_t scratch = !bits ? 0 : std::max(prefill_scratch_bytes(T, 1, exact), std::min(prefill_scratch_bytes(T, Hkv, exact), ((size_t)64 << 20) - 256));
         int r = compat_workspace(256 + scratch, &ws, s);
         if (r != TQ_OK) return r;
         PrefillAttnParams p{};
