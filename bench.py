@@ -393,9 +393,12 @@ def run_append_only(args, w, rank, world, local_rank):
 
 
 def prefill_launches(bits, batch, T, Hkv):
-    """Kernels per layer: (cache write +) attention, a packed prompt's rows as fp16 before it; 131072 rows of a KV head at a time."""
-    groups = 1 if bits == 0 or not batch else -(-batch // max(1, 131072 // (T * Hkv)))
-    return (1 if batch else 0) + groups * (1 if bits == 0 else 2)
+    """Kernels per layer: (cache write +) attention, the rows of a packed prompt of more than 128 tokens as fp16 before it; of those
+    131072 rows of a KV head at a time, some prompts or some KV heads of one."""
+    if bits == 0 or T <= 128:
+        return (1 if batch else 0) + 1
+    prompts = max(1, 131072 // (T * Hkv))
+    return (1 if batch else 0) + 2 * -(-(batch or 1) // prompts) * -(-T * Hkv // 131072)
 
 
 def run_prefill_attention(args, w, rank, world, local_rank):

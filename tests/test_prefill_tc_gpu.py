@@ -23,6 +23,7 @@ D = 128
     (4, 16, 8, 1, 1, 32), (4, 16, 8, 1, 127, 128), (2, 16, 8, 1, 128, 160), (0, 16, 8, 1, 129, 160), (4, 32, 8, 2, 257, 288),
     (0, 8, 8, 1, 385, 416), (2, 40, 8, 1, 150, 160), (4, 24, 2, 1, 140, 160), (0, 40, 8, 1, 51, 64), (4, 96, 1, 1, 130, 160),
     # many: two query blocks per CTA (8 KV heads x 8 prompts x 3 pairs of blocks), the last pair with one block or none at the end
+    (4, 16, 8, 13, 128, 160), (2, 16, 8, 13, 100, 128), (4, 32, 8, 13, 65, 96),  # prompts of one tile: codes converted in place
     (4, 16, 8, 8, 300, 320), (2, 16, 8, 8, 257, 288), (0, 16, 8, 8, 321, 352), (4, 40, 8, 8, 160, 160), (0, 16, 8, 13, 129, 160),
 ])
 def test_prefill_attention_edges(bits, H, Hkv, n, T, msl):

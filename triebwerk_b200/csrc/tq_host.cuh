@@ -530,15 +530,15 @@ inline int make_prefill_query_map(CUtensorMap* m, const void* base, long long to
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TQ_OK : TQ_ERR_ARG;
 }
-template <bool PACKED, int MT, bool EXACT = false>
+template <bool PACKED, int MT, bool EXACT = false, int DIRECT = 0>
 inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ, const CUtensorMap& tmR, const PrefillAttnParams& p,
                                dim3 grid, cudaStream_t s) {
-    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT>, PftSmem::BYTES);
+    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT>, PftSmem::BYTES);
     if (r != TQ_OK) return r;
     // the register split inside the kernel draws on what the launch brings: never launch with less
     static const int regs = [] {
         cudaFuncAttributes a{};
-        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT>) == cudaSuccess ? a.numRegs : 0;
+        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT>) == cudaSuccess ? a.numRegs : 0;
     }();
     if (regs < PFT_REGS_LAUNCH) return TQ_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg{};
@@ -551,7 +551,7 @@ inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT, EXACT>, tmK, tmV, tmQ, tmR, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT>, tmK, tmV, tmQ, tmR, p));
 }
 // Which layouts keep fp32's precision (tq_prefill_fa.cuh): those that neither this kernel's predecessor nor the streaming kernels took.
 inline bool prefill_exact(int bits, int H, int Hkv) {
@@ -565,7 +565,7 @@ inline size_t prefill_scratch_bytes(int T, int Hkv, bool exact) {
 }
 // Causal prefill attention.  `total_rows`: rows of the arrays ck and cv point into (from where they point); `scratch`: packed
 // modes, device memory for at least one KV head of one prompt (prompts go through it in groups; one that is too long for it as a
-// whole, some of its KV heads at a time).
+// whole, some of its KV heads at a time).  Prompts of one tile need none: their blocks convert the codes themselves.
 inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long total_rows, void* scratch, size_t scratch_bytes, cudaStream_t s) {
     p.grp = p.H / p.Hkv;
     const bool exact = prefill_exact(bits, p.H, p.Hkv), low = exact && bits != 0;
@@ -573,7 +573,8 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
     if (p.T <= 0) return TQ_OK;
     const int qt = PFT_ROWS / p.grp;
     int group = p.n_seq, heads = p.Hkv;  // prompts and KV heads per launch (fp16 caches: all of them)
-    if (bits != 0) {
+    const bool direct = bits != 0 && !exact && p.T <= PFT_KT;  // prompts of one tile: no rows in between
+    if (bits != 0 && !direct) {
         if (!scratch) return TQ_ERR_WORKSPACE;
         while (heads > 0 && prefill_scratch_bytes(p.T, heads, exact) > scratch_bytes) --heads;
         if (heads == 0) return TQ_ERR_WORKSPACE;
@@ -597,6 +598,8 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
             if (bits == 0) {
                 r = make_prefill_rows_map(&tmK, p.ck, total_rows, kv_dim);
                 if (r == TQ_OK) r = make_prefill_rows_map(&tmV, p.cv, total_rows, kv_dim);
+            } else if (direct) {
+                r = make_prefill_rows_map(&tmR, p.rotation, HEAD_DIM, HEAD_DIM);
             } else {
                 DequantParams d{};
                 const size_t rows = p.row_base ? 0 : (size_t)s0 * p.seq_rows, head_bytes = bits == 4 ? 64 : 32;
@@ -638,7 +641,9 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
             const long long blocks = mt == 2 ? blocks2 : blocks1;
             if (cols > 2147483647ll || blocks > 65535) return TQ_ERR_CAPACITY;
             dim3 grid((unsigned)cols, (unsigned)blocks);
-            if (low) r = launch_prefill_fa_t<true, 1, true>(tmK, tmV, tmQ, tmR, a, grid, s);
+            if (direct) r = bits == 4 ? (mt == 2 ? launch_prefill_fa_t<true, 2, false, 4>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1, false, 4>(tmK, tmV, tmQ, tmR, a, grid, s))
+                                      : (mt == 2 ? launch_prefill_fa_t<true, 2, false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1, false, 2>(tmK, tmV, tmQ, tmR, a, grid, s));
+            else if (low) r = launch_prefill_fa_t<true, 1, true>(tmK, tmV, tmQ, tmR, a, grid, s);
             else if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);
             else if (exact) r = mt == 2 ? launch_prefill_fa_t<false, 2, true>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1, true>(tmK, tmV, tmQ, tmR, a, grid, s);
             else r = mt == 2 ? launch_prefill_fa_t<false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<false, 1>(tmK, tmV, tmQ, tmR, a, grid, s);

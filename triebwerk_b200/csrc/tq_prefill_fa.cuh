@@ -55,9 +55,9 @@ constexpr int PFT_REGS_LAUNCH = (32 * PFT_SOFT_WARPS * PFT_REGS_SOFT + 128 * PFT
 struct PrefillAttnParams {
     const __half* q;          // queries [n_seq][T][q_tok_stride] as the model makes them
     long long q_tok_stride;   // halves between the queries of consecutive tokens
-    const uint8_t* ck;        // (host) packed codes [rows][kvp] or fp16 rows [rows][Hkv * 128]; the kernel reads through its maps
+    const uint8_t* ck;        // packed codes [rows][kvp] or fp16 rows [rows][Hkv * 128]; read through maps, but for DIRECT
     const uint8_t* cv;
-    const __half* kn;         // (host) [rows][Hkv], packed caches
+    const __half* kn;         // [rows][Hkv], packed caches (read by DIRECT)
     const __half* vn;
     const __half* rotation;   // packed: R row-major [128][128]
     int low_row;              // packed, EXACT: rows from the high parts to the low parts of ck, cv
@@ -234,10 +234,13 @@ __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.a
 template <int N>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// PACKED: ck, cv are the fp16 centroids [n_seq * T][kv_dim] of dequantize_rows_kernel (seq_rows = T, no row_base), p.norms its norms
+// PACKED: but for DIRECT, ck, cv are the fp16 centroids [n_seq * T][kv_dim] of dequantize_rows_kernel (seq_rows = T, no row_base), p.norms its norms
 // EXACT: queries, centroids and weights as fp16 high + low parts; packed with MT = 1 only: one stage of K and V, the low parts in
 // the other one's place, the queries' in the second query tile's
-template <bool PACKED, int MT, bool EXACT>
+// DIRECT (4 or 2 bits, prompts of one tile): the softmax warps turn the tile's codes into centroids themselves, while the queries arrive
+// and are rotated.  Every query block of a head repeats that, but dequantize_rows_kernel's launch is saved: a layer of 35 tokens,
+// 16/8 heads, 4-bit 20.4 -> 15.5 us, 16 prompts of 32 tokens, 2-bit 24.9 -> 19.9, 16 of 128, 4-bit 33.0 -> 25.8.
+template <bool PACKED, int MT, bool EXACT, int DIRECT>
 __global__ void __launch_bounds__(PFT_THREADS, 1)
 prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ,
                             const __grid_constant__ CUtensorMap tmR, const PrefillAttnParams p) {
@@ -251,6 +254,10 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     constexpr int COPY_WARP = PFT_SOFT_WARPS, MMA_WARP = PFT_SOFT_WARPS + 1;
     constexpr bool LOW = PACKED && EXACT;  // low parts of the operands in shared memory
     static_assert(!LOW || MT == 1, "the second query block's places hold the low parts");
+    static_assert(!DIRECT || (PACKED && !EXACT), "a packed form");
+    // DIRECT: byte (4-bit) or nibble (2-bit) -> two centroids, eight copies, in the idle second stage of K
+    constexpr int CODES = DIRECT == 4 ? 256 : 16;
+    uint32_t* const lut = reinterpret_cast<uint32_t*>(gb + PftSmem::K + PFT_TILE);
     // tile j's data are in stage j % STAGES; its barriers are number j & 1 also where there is one stage (a slot waits for every other
     // tile only, so that it must not meet the one between them on the same barrier)
     constexpr int STAGES = LOW ? 1 : 2;
@@ -301,6 +308,13 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         mbar_init(bar_q, 1);
         fence_mbar_init();
     }
+    if (DIRECT) {
+        for (int i = tid; i < CODES * 8; i += PFT_THREADS) {
+            const int e = i >> 3;
+            lut[i] = DIRECT == 4 ? pack_half2(kCent4[e & 15], kCent4[(e >> 4) & 15]) : pack_half2(kCent2[e & 3], kCent2[(e >> 2) & 3]);
+        }
+        if (tid == 0) *reinterpret_cast<uint32_t*>(gb + PftSmem::NORM + 8u * PFT_KT) = 0u;  // the largest V norm
+    }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -344,6 +358,40 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     umma_lo(tmem + 128u * m, pft_lo_k(sb + PftSmem::Q + m * PFT_TILE) + pft_kstep(ks), pft_lo_k(sb + PftSmem::R) + pft_kstep(ks), PFT_IDESC_K, ks != 0);
             umma_commit(bar_rot);
         }
+        if (DIRECT && warp < PFT_SOFT_WARPS) {
+            constexpr int PIECES = 2 * PFT_KT * 16 / (32 * PFT_SOFT_WARPS);  // of 8 codes per thread: K rows, then V rows
+            uint32_t c[PIECES];
+            const size_t head0 = ((size_t)seq_row0 * p.Hkv + kvh) * 16;
+#pragma unroll
+            for (int i = 0; i < PIECES; ++i) {
+                const int row = (tid >> 4) + 32 * (i % (PIECES / 2));
+                const size_t at = head0 + (size_t)row * p.Hkv * 16 + (tid & 15);
+                const uint8_t* const codes = i < PIECES / 2 ? p.ck : p.cv;
+                c[i] = 0u;
+                if (row < p.T) c[i] = DIRECT == 4 ? reinterpret_cast<const uint32_t*>(codes)[at] : (uint32_t)reinterpret_cast<const unsigned short*>(codes)[at];
+            }
+            if (tid < PFT_KT) {
+                const size_t at = ((size_t)seq_row0 + tid) * p.Hkv + kvh;
+                const float kn = tid < p.T ? __half2float(p.kn[at]) : 0.0f, vn = tid < p.T ? __half2float(p.vn[at]) : 0.0f;
+                float* const norms = reinterpret_cast<float*>(gb + PftSmem::NORM);
+                norms[tid] = kn;
+                norms[PFT_KT + tid] = vn;
+                const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(vn));
+                if (lane == 0) atomicMax(reinterpret_cast<uint32_t*>(norms + 2 * PFT_KT), top);
+            }
+#pragma unroll
+            for (int i = 0; i < PIECES; ++i) {
+                const int row = (tid >> 4) + 32 * (i % (PIECES / 2)), copy = tid & 7;
+                uint4 u = make_uint4(0u, 0u, 0u, 0u);  // (rows past the prompt)
+                if (row < p.T) {
+                    constexpr int W = DIRECT == 4 ? 8 : 4;
+                    constexpr uint32_t M = CODES - 1;
+                    u.x = lut[(c[i] & M) * 8 + copy]; u.y = lut[((c[i] >> W) & M) * 8 + copy];
+                    u.z = lut[((c[i] >> (2 * W)) & M) * 8 + copy]; u.w = lut[((c[i] >> (3 * W)) & M) * 8 + copy];
+                }
+                *reinterpret_cast<uint4*>(gb + (i < PIECES / 2 ? PftSmem::K : PftSmem::V) + pft_chunk(row, tid & 15)) = u;
+            }
+        }
         if (warp < PFT_SOFT_WARPS) {
             wait_bar(bar_rot, 0u);
             tc_fence_after();
@@ -378,7 +426,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         // (fp16 caches, the prompt's last tile: rows past the prompt may hold anything, and 0 x NaN is NaN, so its V rows are blanked)
         const int x_row = (int)seq_row0;
         const float* const norms = PACKED ? p.norms + ((size_t)seq * p.Hkv + kvh) * p.tiles * PFT_NORMS : nullptr;
-        for (int j = 0; j < n_tiles; ++j) {
+        for (int j = 0; j < (DIRECT ? 0 : n_tiles); ++j) {
             const int st = j % STAGES, b = j & 1, last = j - STAGES;  // last: the tile that was in this stage
             if (last >= 0) wait_bar(bar_kfree + 8u * (last & 1), (uint32_t)((last >> 1) & 1));
             if (lane == 0 && !dead) {
@@ -411,7 +459,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         if (lane == 0) {
             auto issue_scores = [&](int s, int i) {
                 const int j = tile_of(s, i), st = j % STAGES;
-                wait_bar(bar_kfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
+                if (!DIRECT) wait_bar(bar_kfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
                 tc_fence_after();
                 if (dead) return;
                 const uint32_t a = pft_lo_k(sb + PftSmem::Q + (MT == 2 ? s * PFT_TILE : 0u)), b = pft_lo_k(sb + PftSmem::K + st * PFT_TILE);
@@ -429,7 +477,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             };
             auto issue_values = [&](int s, int i) {
                 const int j = tile_of(s, i), st = j % STAGES;
-                wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
+                if (!DIRECT) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
                 wait_bar(bar_pfull + 8u * s, (uint32_t)(i & 1));
                 tc_fence_after();
                 if (dead) return;
@@ -489,7 +537,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};  // (sums: of this thread's columns)
         for (int i = 0; i < nt; ++i) {
             const int j = tile_of(slot, i), st = j % STAGES, col0 = j * PFT_KT;
-            if (PACKED) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
+            if (PACKED && !DIRECT) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
             wait_bar(bar_sfull + 8u * slot, (uint32_t)(i & 1));
             tc_fence_after();
             const bool diagonal = col0 + PFT_KT - 1 > my_first;  // (uniform for the slot)
