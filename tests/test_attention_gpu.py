@@ -305,18 +305,37 @@ def test_prefill_attention_with_query_tiles_at_ragged_sizes(bits, H, Hkv):
     hp.assert_attention_close(got_s, ref[:5], H, D, "prefill attention, 5 tokens")
 
 
-def test_prefill_attention_mma_sync_form_in_a_child_process():
-    """The tcgen05 form of the prefill attention is the default; the mma.sync form is selected by TQ_PREFILL_ATTN_TC=0, which
-    the library reads once per process: the parity tests of the prefill attention run again in a child with it set."""
-    import os
-    import subprocess
-    import sys
-    if os.environ.get("TQ_PREFILL_ATTN_TC") == "0":
-        pytest.skip("already the child")
-    env = dict(os.environ, TQ_PREFILL_ATTN_TC="0")
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-m", "pytest", "tests/test_attention_gpu.py", "tests/test_fp16_gpu.py", "tests/test_engine_gpu.py",
-                        "-q", "-x", "-m", "gpu", "-k", "prefill and not child", "-p", "no:cacheprovider"],
-                       cwd=root, env=env, capture_output=True, text=True, timeout=600)
-    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
-    assert " passed" in r.stdout
+@pytest.mark.parametrize("bits,H,Hkv,shift", [(4, 16, 8, 1), (2, 16, 8, 4), (0, 16, 8, 2), (4, 129, 1, 0), (0, 130, 1, 0)])
+def test_prefill_attention_outside_the_tiled_kernel(bits, H, Hkv, shift):
+    """Queries and results off a 16-byte boundary (by `shift` halves) and more than 128 query heads per KV head go token by token
+    through the generic kernel, from the launchers and from the engine."""
+    import triebwerk_b200 as tq
+    from triebwerk_b200 import ops
+    rng = np.random.default_rng(700 + bits + H)
+    R, _ = tqo.rotation()
+    D, T, msl = 128, 37, 64
+    kv_dim = Hkv * D
+
+    def shifted(x):
+        flat = torch.zeros(x.size + 16, dtype=torch.float16, device="cuda")
+        view = flat[shift:shift + x.size].view(x.shape)
+        view.copy_(gu.dev(x))
+        assert view.is_contiguous() and (view.data_ptr() % 16 == 0) == (shift == 0)
+        return view
+
+    k, v = (rng.standard_normal((T, kv_dim), dtype=np.float32).astype(np.float16) for _ in range(2))
+    q = shifted(rng.standard_normal((T, H * D), dtype=np.float32).astype(np.float16))
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(2, msl)
+    out = [shifted(np.zeros((T, H * D), np.float16)) for _ in range(2)]
+    eng.prefill_layer(0, 1, q, gu.dev(k), gu.dev(v), out[0])
+    assert eng.status() == 0
+    cache = [None if t is None else t[msl:] for t in eng.layer_cache(0)]
+    if bits == 0:
+        ops.launch_gqa_prefill_attention(out[1], q, cache[0], cache[1], None, T, msl, H, Hkv, D, H * D, kv_dim)
+        ref = np.stack([tqo.fp16_attention_single(gu.host(q)[t], k, v, t, T, H, Hkv, D)[0] for t in range(T)])
+    else:
+        ops.launch_turbo_gqa_prefill_attention(out[1], q, *cache, gu.dev(R), None, T, msl, H, Hkv, D, H * D, kv_dim, bits)
+        ref, _ = tqo.prefill_attention(gu.host(q), *(gu.host(t) for t in cache), R, msl, H, Hkv, D, bits)
+    for o, what in zip(out, ("engine", "launcher")):
+        hp.assert_attention_close(gu.host(o), ref, H, D, f"{what} tq{bits} {H}/{Hkv}")
