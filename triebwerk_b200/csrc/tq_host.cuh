@@ -630,11 +630,11 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
             if (r != TQ_OK) return r;
             // Two query blocks per CTA, which share every tile, once there are enough of them for the GPU; below that twice the
             // CTAs with one block each, whose two slots take the even and the odd tiles.  Per layer, one block / two (8 KV heads,
-            // 4-bit): 2048 tokens 16 heads (128 pairs of blocks) 70 / 83 us, 32 heads (256) 117 / 104, 8192 tokens 16 heads (512)
-            // 449 / 439.
+            // 4-bit): 2048 tokens 16 heads (128 pairs of blocks) 55 / 67 us, 3000 tokens (188) 88 / 85, 32 heads 2048 tokens (256)
+            // 91 / 76, 8192 tokens 16 heads (512) 381 / 352; fp16 2048 tokens 16 heads 31 / 43, 32 heads 57 / 48.
             const long long blocks2 = (p.T + 2 * qt - 1) / (2 * qt), cols = (long long)a.Hkv * a.n_seq;
             // Prompts of up to two tiles have no long CTAs, there the turns of the SMs decide, of which one with two blocks costs about
-            // 4/3 of one with one: 12 prompts of 70 tokens 32.4 / 29.6 us, of 163 38.8 / 45.4, 16 of 250 63.5 / 55.2.
+            // 4/3 of one with one: 12 prompts of 70 tokens 29.4 / 23.8 us, of 163 39.5 / 44.4, 16 of 250 62.6 / 51.6.
             const long long sms = device_props().sm_count, blocks1 = (p.T + qt - 1) / qt;
             const long long turns1 = (blocks1 * cols + sms - 1) / sms, turns2 = (blocks2 * cols + sms - 1) / sms;
             const int mt = low ? 1 : (p.T <= 2 * PFT_KT ? 3 * turns1 >= 4 * turns2 : 4 * blocks2 * cols >= 5 * sms) ? 2 : 1;

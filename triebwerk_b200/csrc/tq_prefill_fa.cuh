@@ -12,7 +12,7 @@
 // copy.  Packed caches are turned into fp16 centroids (unscaled: the same operands as ever) and fp32 norms by
 // dequantize_rows_kernel first, once per prompt and layer instead of once per query block: done by producer warps inside
 // this kernel the table look-ups and operand stores took as much of the shared-memory pipe as the products themselves (8192
-// tokens, 16/8 heads, 4-bit: 617 us against 439).  P (times the V norm, fp16) replaces S in tensor memory and is read from
+// tokens, 16/8 heads, 4-bit, eight softmax warps: 617 us against 439).  Prompts of a single tile are the exception (DIRECT).  P (times the V norm, fp16) replaces S in tensor memory and is read from
 // there as the A operand.
 //   warps 0-15   softmax of slots 0 and 1: S -> registers (16x256b loads: a thread holds two rows' column pairs as in an mma
 //                fragment, so a row's maximum is two shuffles), K norm, causal limit, exponentials, P -> tensor memory.  The
@@ -28,9 +28,9 @@
 // Every wait on a barrier is bounded; a wait that runs out raises the status word and the kernel runs to its end.
 // Bound by the softmax threads (exponentials, tensor-memory loads) against the tensor core at long prompts, by the chain copy ->
 // S -> softmax -> O of a single block at short ones.  Per layer, 8 KV heads, cache write included, the one-block kernel with V
-// transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 508 us (1080 TFLOP/s of causal arithmetic), 777
-// tokens 59 -> 29; 4-bit 8192 tokens 16 heads 763 -> 350 us, 777 tokens 43.7 -> 32.2.  (With one thread per row, eight softmax
-// warps, S read twice: 530, 31, 379, 34.2.)
+// transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 507 us in runs of a few milliseconds (1080 TFLOP/s
+// of causal arithmetic), 590 (930) under the power cap of longer ones; 4-bit 8192 tokens 16 heads 763 -> 343 to 361 us, 777 tokens
+// 43.7 -> 32.5.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
 #pragma once
 
 #include "tq_prefill_tc.cuh"
