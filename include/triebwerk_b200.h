@@ -299,6 +299,10 @@ int tq_engine_attend_step(tq_engine* e, void* out, tq_stream_t s);
  * layer instead, TQ_CLUSTER=0 the four launches for small steps too. */
 int tq_engine_decode_step(tq_engine* e, const void* q, const void* k, const void* v, void* out, tq_stream_t s);
 
+/* Which form tq_engine_decode_layer (whole_step = 0) or tq_engine_decode_step (1) take for the present batch on 16-byte aligned
+ * buffers: the CTAs per thread-block cluster, or 0 for the streaming kernels.  For tests and tuning. */
+int tq_engine_decode_form(const tq_engine* e, int whole_step);
+
 /* The step's producer and consumer folded into it.  In the reference the projections' outputs pass through two more
  * kernels before the cache write -- per-head RMS norm with weights (launch_qk_norm_batch) and rotary embedding
  * (launch_rope_batch), engine/engine.cpp:1972-1977, kernels engine/kernels.cu:880-962 -- and the attention result

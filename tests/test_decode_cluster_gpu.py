@@ -20,26 +20,28 @@ D = 128
 
 
 # capacity and batch set the cluster size: at most one CTA per SM, a 16-token block per warp
-@pytest.mark.parametrize("bits,H,Hkv,msl,lengths", [
-    (4, 16, 8, 64, [1, 16, 17, 33, 64]),               # one CTA per cluster, 32-token tiles
-    (2, 32, 8, 256, [1, 2, 128, 255]),                 # 2 CTAs
-    (4, 16, 4, 512, [1, 31, 449, 512]),                # 4 CTAs, one of them for the new token
-    (2, 8, 1, 2048, [1, 15, 16, 17, 1900]),            # 16 CTAs, 16-token tiles
-    (4, 16, 8, 2112, [1801]),                          # 16 CTAs, several tiles per warp
-    (4, 16, 4, 1600, [1] * 17 + [17, 700, 1600]),      # 2 CTAs, two on an SM
-    (0, 16, 4, 640, [1] * 18 + [639, 640]),            # the same, fp16
-    (4, 24, 2, 320, [97, 320]),                        # 12 query heads per KV head: two clusters share a KV head
-    (2, 20, 1, 96, [95]),                              # 20: three
-    (0, 40, 8, 384, [1, 16, 383]),                     # fp16 rows
-    (0, 12, 4, 1024, [1000]),
+@pytest.mark.parametrize("bits,H,Hkv,msl,lengths,ctas", [
+    (4, 16, 8, 64, [1, 16, 17, 33, 64], 1),            # one CTA per cluster, 32-token tiles
+    (2, 32, 8, 256, [1, 2, 128, 255], 2),
+    (4, 16, 4, 512, [1, 31, 449, 512], 4),             # one of them for the new token
+    (2, 8, 1, 2048, [1, 15, 16, 17, 1900], 16),        # 16-token tiles
+    (4, 16, 8, 2112, [1801], 16),                      # several tiles per warp
+    (4, 16, 4, 1600, [1] * 17 + [17, 700, 1600], 2),   # two on an SM
+    (0, 16, 4, 640, [1] * 18 + [639, 640], 2),         # the same, fp16
+    (4, 24, 2, 320, [97, 320], 4),                     # 12 query heads per KV head: two clusters share a KV head
+    (2, 20, 1, 96, [95], 1),                           # 20: three
+    (0, 40, 8, 384, [1, 16, 383], 4),                  # fp16 rows
+    (0, 12, 4, 1024, [1000], 8),
 ])
-def test_decode_layer_cluster_form(bits, H, Hkv, msl, lengths):
+def test_decode_layer_cluster_form(bits, H, Hkv, msl, lengths, ctas):
     rng = np.random.default_rng(1000 + 7 * bits + H + msl)
     G, kv_dim = len(lengths), Hkv * D
     R = ops.rotation_matrix().numpy()
     eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
     eng.alloc_batch(G, msl)
     eng.reset()
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert tq.lib().tq_engine_decode_form(eng._h, 0) == ctas
     ks = [rng.standard_normal((n, kv_dim), dtype=np.float32).astype(np.float16) for n in lengths]
     vs = [rng.standard_normal((n, kv_dim), dtype=np.float32).astype(np.float16) for n in lengths]
     ks[0][-1], vs[-1][-1, :D] = 0, 0  # a new token on a quantiser bound everywhere

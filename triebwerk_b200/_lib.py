@@ -24,7 +24,7 @@ SYMBOLS = [
     "tq_engine_alloc_batch", "tq_engine_reset", "tq_engine_sleep", "tq_engine_wake", "tq_engine_positions",
     "tq_engine_set_positions", "tq_engine_advance", "tq_engine_layer_ptrs", "tq_engine_row_base",
     "tq_engine_rotation", "tq_engine_set_rotation", "tq_engine_decode_layer", "tq_engine_prefill_append", "tq_engine_prefill_append_batch",
-    "tq_engine_decode_step_host", "tq_engine_attend_layer", "tq_engine_decode_step", "tq_engine_status", "tq_engine_attend_step",
+    "tq_engine_decode_step_host", "tq_engine_attend_layer", "tq_engine_decode_step", "tq_engine_status", "tq_engine_attend_step", "tq_engine_decode_form",
     "tq_engine_output_f32", "tq_engine_read_output_f32", "tq_engine_decode_layers", "tq_static_status", "tq_selftest_bounded_wait",
     "tq_engine_sequence_blob_bytes", "tq_engine_export_sequence", "tq_engine_import_sequence", "tq_engine_sleep_keep", "tq_engine_prefill_shared", "tq_engine_decode_step_produce", "tq_fold_rotation_into_projection",
     "tq_engine_time_attention", "tq_engine_last_attention_ms", "tq_engine_prefill_layer", "tq_engine_prefill_layer_batch", "tq_engine_step_prepare", "tq_engine_step_attend_layers",
@@ -107,6 +107,7 @@ def lib() -> C.CDLL:
     sig("tq_engine_decode_step", i, [vp, vp, vp, vp, vp, vp])
     sig("tq_engine_status", i, [vp, vp])
     sig("tq_engine_attend_step", i, [vp, vp, vp])
+    sig("tq_engine_decode_form", i, [vp, i])
     sig("tq_static_status", i, [vp])
     sig("tq_engine_decode_step_produce", i, [vp, vp, vp, vp, vp, C.POINTER(StepProducer), vp])
     sig("tq_fold_rotation_into_projection", i, [vp, vp, vp, ll, i, vp])

@@ -1514,6 +1514,14 @@ static bool engine_step_small(const tq_engine* e, StepInputs inputs) {
     return one < four;
 }
 
+int tq_engine_decode_form(const tq_engine* e, int whole_step) {
+    if (!e || !e->arena || e->G == 0) return TQ_ERR_STATE;
+    const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
+    const bool layer = !fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, 0.0));
+    if (!e->fused || !(whole_step ? engine_step_small(e, StepInputs::Plain) : layer)) return 0;
+    return cluster_launch_split(e->kv_bits, e->G, whole_step ? e->shape.num_layers : 1, H, Hkv, e->msl);
+}
+
 // The layers l0 .. l0 + n - 1 of such a step; q, k, v, out point at layer l0's [G][dim] blocks.
 static int engine_cluster_step(tq_engine* e, int l0, int n, const void* q, const void* k, const void* v, void* out, cudaStream_t s,
                                bool host_inputs = false) {

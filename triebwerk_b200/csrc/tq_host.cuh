@@ -452,11 +452,15 @@ inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long 
     return 0.4 * chain + 0.3 * chain * turns + 0.009 * clusters + many < 10.0 + 7e-6 * (double)rows * Hkv + 0.0004 * max_tokens + extra;
 }
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
+inline int cluster_launch_split(int bits, int G, int split_layers, int H, int Hkv, int max_tokens) {
+    const int head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
+    const bool one_per_sm = bits != 0 && !fast_shape(H, Hkv, true);  // (EXACT, packed: as with 8 heads)
+    return cluster_split(bits, (long long)G * split_layers * Hkv * head_blocks, one_per_sm ? CD_HEADS : std::min(CD_HEADS, H / Hkv), max_tokens);
+}
 template <bool HOST, bool EXACT>
 inline int launch_cluster_decode_e(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
     const int blocks = (max_tokens + 15) / 16;
-    const int heads = EXACT && bits != 0 ? CD_HEADS : std::min(CD_HEADS, p.H / p.Hkv);  // (EXACT, packed: one CTA per SM, as with 8 heads)
-    const int S = cluster_split(bits, (long long)p.G * split_layers * p.Hkv * p.head_blocks, heads, max_tokens);
+    const int S = cluster_launch_split(bits, p.G, split_layers, p.H, p.Hkv, max_tokens);
     if (bits == 0) return launch_cluster_decode_t<0, 1, HOST, EXACT>(p, S, layers, s, pdl);
     const bool one = S * CD_WARPS >= blocks;  // a single 16-token tile per warp
     if (bits == 4) return one ? launch_cluster_decode_t<4, 1, HOST, EXACT>(p, S, layers, s, pdl) : launch_cluster_decode_t<4, 2, HOST, EXACT>(p, S, layers, s, pdl);
