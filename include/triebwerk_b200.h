@@ -86,8 +86,8 @@ void launch_turbo_gqa_attention(const void* q, const uint8_t* ck_q, const uint8_
 
 /* engine/kernels.cu:2015-2028 (kernel :1874-1960).  Causal prefill attention over a single-sequence
  * packed cache: query row tq of q [T][q_dim] attends to positions 0..tq.  Served by a tcgen05 kernel that holds 128 score rows
- * (query tokens x heads of a KV head) in the M dimension, after a launch that turns the prompt's codes into fp16 centroids once,
- * in the library's workspace; `as` (the reference's [T][heads][T] score scratch) is accepted and ignored. */
+ * (query tokens x heads of a KV head) in the M dimension, after a launch that turns the codes of a prompt of more than 128 tokens
+ * into fp16 centroids once, in the library's workspace (64 MiB of it, some KV heads at a time); `as` (the reference's [T][heads][T] score scratch) is accepted and ignored. */
 void launch_turbo_gqa_prefill_attention(void* out, const void* q, const uint8_t* ck_q, const uint8_t* cv_q,
                                         const void* k_norms, const void* v_norms, const void* rotation,
                                         float* as, int T, int msl, int num_heads, int num_kv_heads,
