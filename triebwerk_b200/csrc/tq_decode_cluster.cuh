@@ -11,21 +11,27 @@
 //   * codes become fp16 through a shared-memory table with a private column per lane (one entry per code byte at 4-bit,
 //     per nibble at 2-bit); table and R are staged before griddepcontrol.wait, i.e. under the previous kernel's tail, and
 //     so are, in a chain of layers, the cache rows of the warp's first tile.
-//   * the step's token is quantised by the CTA that owns the sequence's last tile: its raw K and V vectors are two more
+//   * positions and R are requested first, the table is written while they are on their way; K rows of a single tile per warp are
+//     looked up there too, so that only products are left once the queries have arrived.
+//   * the step's token is quantised by the cluster's last CTA (its owner): its raw K and V vectors are two more
 //     rows of the A operand of the query rotation (rows 8 and 9, otherwise idle), scaled by 1/norm afterwards; a
 //     coordinate within CD_MARGIN of a decision bound is recomputed with the reference's exact fp32 chain, as in
-//     tq_prefill_tc.cuh, so the stored bytes are the reference's.  The last tile reads the token from shared memory; it
-//     goes to the cache at the very end, so that no barrier has to wait for a global write.  In clusters of four CTAs or
-//     more that CTA takes nothing but the new token: quantising it then costs no more time than the others' tiles.
+//     tq_prefill_tc.cuh, so the stored bytes are the reference's.  It is in no tile: its score is a dot product of one warp per
+//     head, its value row enters the CTA's sum of the warps' results, in fp32; it goes to the cache at the very end, so that no
+//     barrier has to wait for a global write.  In clusters of four CTAs or more the owner takes nothing else: quantising costs no
+//     more time than the others' tiles then.
 //   * S^T = K Q^T and O^T += V^T P^T on mma.sync with tokens / coordinates in the M dimension as in the streaming kernel.
-//     The warps' partial results meet in shared memory; every CTA normalises its own and multiplies it by R (fp16 high +
-//     low parts) and sends every other CTA its share of the output coordinates with asynchronous stores into that CTA's
+//     The warps' partial results meet in shared memory; every CTA normalises its own and multiplies it by R (fp16 high
+//     parts as rows 0-7 of the A operand, low parts as rows 8-15) and sends every other CTA its share of the output coordinates with asynchronous stores into that CTA's
 //     shared memory, counted by that CTA's mbarrier; a CTA adds up its share, weighted, when all of it has arrived.  (A
 //     cluster barrier in that place costs 0.8 us more: its release waits for the remote stores to be acknowledged.)
 //   * Head layouts that the streaming kernels do not serve took a kernel with fp32 queries, centroids and weights.  Here they are
 //     fp16 high + low parts (EXACT: three products for one, a second table): the results' error is that kernel's.  With the high
 //     parts alone it was 2.9 (4-bit), 3.8 (2-bit) and 1.12 (fp16 rows) times as large.
-// Bound by latency: one round trip for the inputs, the rotation, one tile, three CTA barriers, one trip across the cluster.
+// Bound by latency: one round trip for the inputs, the rotation, one tile, three CTA barriers, one trip across the cluster, about
+// 700 + 800 + 1500 + 600 + 900 + 900 + 1500 cycles.  With the token as a row of the last tile (its CTA 1600 cycles behind the others),
+// divisions by the cluster's size in the exchange, the low parts' products with R of their own and the look-ups behind the queries:
+// 1 layer of 4 x 612 tokens 7.05 us, now 5.84; 28 layers of 1 x 1500 187 us, now 169 (4-bit, 16/8 heads).
 #pragma once
 
 #include "tq_attention.cuh"
@@ -132,7 +138,9 @@ struct CdSmem {
     static constexpr uint32_t LO_OFF = Q_OFF + CD_HEADS * MERGE_ROW * 2; // merge operand low part
     static constexpr uint32_t BND_OFF = LO_OFF + CD_HEADS * MERGE_ROW * 2;  // decision bounds, fp32, between -inf and +inf
     static constexpr uint32_t BAR_OFF = BND_OFF + 80;                    // mbarrier of what the cluster's CTAs send
-    static constexpr uint32_t CP_OFF = BND_OFF + 96;                     // [CTA][head][this CTA's share of the coordinates] fp32, from all CTAs
+    static constexpr uint32_t CENT_OFF = BND_OFF + 96;                   // centroids, fp32
+    static constexpr uint32_t NS_OFF = CENT_OFF + 64;                    // new token: its score with each query head
+    static constexpr uint32_t CP_OFF = NS_OFF + 32;                      // [CTA][head][this CTA's share of the coordinates] fp32, from all CTAs
     static constexpr uint32_t MZ_OFF = CP_OFF + CD_HEADS * HEAD_DIM * 4; // [CTA][head] maximum and sum
     static constexpr uint32_t WARP_OFF = MZ_OFF + CD_MAX_CLUSTER * CD_HEADS * 8;  // the warps' partial results [8][heads][PART_STRIDE] fp32
 };
@@ -192,82 +200,40 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     const uint32_t r_s = lut_s + (BITS == 4 ? 128u : 0x1000u);
     auto r_piece = [&](int row, int k8) -> uint32_t { return r_s + (uint32_t)(k8 * 16 + (row >> 3)) * RS + (uint32_t)(((row + 2 * k8) & 7) << 4); };
 
-    // ---- before the wait: table, bounds, R ----
-    const uint32_t bar = base + CdSmem::BAR_OFF;
-    if (S > 1) {
-        if (tid == 0) {
-            mbar_init(bar, 1);
-            fence_mbar_init();
-            mbar_arrive_expect_tx(bar, (uint32_t)nh * (HEAD_DIM * 4u + S * 8u));
-        }
-        __syncwarp();
-        cluster_arrive();  // (the wait comes before the first store to another CTA: it has started then, its barrier is set)
-    }
-    constexpr int NBND = BITS == 4 ? 15 : 3;
-    if (BITS != 0 && tid <= NBND + 1) {
-        const float bound = tid == 0 ? -3.4e38f : (tid > NBND ? 3.4e38f : (BITS == 4 ? kBnd4[(tid - 1) & 15] : kBnd2[(tid - 1) & 3]));
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::BND_OFF + 4u * (uint32_t)tid), "f"(bound) : "memory");
-    }
-    constexpr uint32_t LOW = cd_low_table(BITS);
-    auto table_entry = [&](uint32_t at, float c0, float c1) {  // four lanes' copies of two centroids
-        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(pack_half2(c0, c1)) : "memory");
-        if (EXACT) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + LOW), "r"(pack_low_half2(c0, c1)) : "memory");
-    };
-    if constexpr (BITS == 4) {
-        const float lo = kCent4[(tid >> 3) & 15];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)  // entry (tid >> 3) + 32 i, lanes 4 (tid & 7) .. + 3
-            table_entry(lut_s + (uint32_t)((tid >> 3) + 32 * i) * 256u + (uint32_t)(tid & 7) * 16u, lo, kCent4[(tid >> 7) + 2 * i]);
-    } else if constexpr (BITS == 2) {
-        if (tid < 128) table_entry(lut_s + (uint32_t)(tid >> 3) * 256u + (uint32_t)(tid & 7) * 16u, kCent2[(tid >> 3) & 3], kCent2[tid >> 5]);
-    }
-    auto stage_rotation = [&]() {
-        uint4 u[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) u[i] = ldg128_if(reinterpret_cast<const uint4*>(p.rotation) + tid + CD_THREADS * i, true);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int at = tid + CD_THREADS * i;
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(r_piece(at >> 4, at & 15)), "r"(u[i].x), "r"(u[i].y), "r"(u[i].z), "r"(u[i].w) : "memory");
-        }
-    };
-    if (BITS != 0 && p.static_rotation) stage_rotation();
-
     // ---- positions, rows, and the cache rows of a tile ----
-    int pos = 0;
-    bool appends = false, pos_ok = false, owner = false;
+    const bool owner = p.new_k != nullptr && rank == S - 1u;  // the CTA of the new token
+    int pos = 0, cap = 0;
+    bool appends = false, pos_ok = false;
     int tile = 0, tile_end = 0, tile_step = 1;  // this warp's tiles
-    int lo = 0, hi = 0, lim = 0;                // tokens of them that count: lo .. hi - 1; rows that are read: those below lim
+    int n_act = 0;                              // warps of this CTA that have any
+    int lim = 0;                                // cached tokens: those below lim
     long long row0 = 0, prow0 = 0;
     int ptok = 0;  // tokens below ptok are read from the shared prefix
-    auto read_position = [&]() {
-        pos = p.positions ? p.positions[g] : p.pos_value;
-        const int cap = p.seq_capacity ? p.seq_capacity[g] : p.capacity_rows;
+    uint2 row0_w = make_uint2(0u, 0u), prow0_w = make_uint2(0u, 0u);
+    auto fetch_position = [&]() {  // (volatile loads, all in flight together before anything waits for one)
+        pos = (int)ldg32_if(p.positions + g, p.positions != nullptr);
+        cap = (int)ldg32_if(p.seq_capacity + g, p.seq_capacity != nullptr);
+        row0_w = ldg64_if(p.row_base + g, p.row_base != nullptr);
+        ptok = (int)ldg32_if(p.prefix_tiles + g, p.prefix_tiles != nullptr);
+        prow0_w = ldg64_if(p.prefix_base + g, p.prefix_tiles != nullptr);
+    };
+    auto use_position = [&]() {
+        if (!p.positions) pos = p.pos_value;
+        if (!p.seq_capacity) cap = p.capacity_rows;
         pos_ok = pos >= 0 && (cap <= 0 || pos < cap);
         int L = (pos < 0 ? 0 : pos) + 1;
         if (cap > 0 && L > cap) L = cap;  // a position outside its slot is reported; rows outside the slot are not read
         appends = p.new_k != nullptr && pos_ok;
         lim = appends ? L - 1 : L;        // (the row this very step writes is never read from the cache)
-        const int W = p.new_k != nullptr && S >= 4u ? (int)S - 1 : (int)S;  // CTAs that take the old tokens
-        hi = W == (int)S ? L : lim;
-        tile_end = (hi + TT - 1) / TT;
+        const int W = p.new_k != nullptr && S >= 4u ? (int)S - 1 : (int)S;  // CTAs that take the cached tokens
+        tile_end = (int)rank < W ? (lim + TT - 1) / TT : 0;
         tile = warp * W + (int)rank;
         tile_step = CD_WARPS * W;
-        if (W == (int)S) {
-            owner = p.new_k != nullptr && (tile_end - 1) % (int)S == (int)rank;
-        } else if ((int)rank == W) {      // the CTA of the new token: one tile, nothing in it but that token
-            owner = true;
-            lo = lim;
-            hi = L;
-            lim = 0;
-            tile = warp == 0 && appends ? lo / TT : 1;
-            tile_end = tile + 1 - (warp == 0 && appends ? 0 : 1);
-        }
-        row0 = p.row_base ? p.row_base[g] : (long long)g * p.max_seq_len;
-        if (p.prefix_tiles) {
-            ptok = p.prefix_tiles[g] * TILE_TOKENS;
-            prow0 = p.prefix_base[g];
-        }
+        for (int w = 0, t = (int)rank; w < CD_WARPS && t < tile_end; ++w, t += W) n_act = w + 1;
+        auto join = [](uint2 w) { return (long long)((unsigned long long)w.y << 32 | w.x); };
+        row0 = p.row_base ? join(row0_w) : (long long)g * p.max_seq_len;
+        ptok *= TILE_TOKENS;
+        prow0 = join(prow0_w);
     };
     constexpr int KV4 = BITS == 0 ? 4 : 1, VV4 = BITS == 0 ? 2 : 1;  // 16-byte pieces per lane and row
     uint4 kw[MB][2][KV4];                      // K rows gl, gl + 8 of a block: the lane's 32 coordinates 32 t4 ..
@@ -324,17 +290,107 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     };
     auto first_tile = [&]() {
-        read_position();
+        use_position();
         if (tile < tile_end) {
             load_k(tile, lim);
             load_v(tile, lim);
         }
     };
+    const bool staged = BITS == 0 || p.static_rotation != 0;  // R may be read before the wait
+    uint4 ru[8];
+    auto fetch_rotation = [&]() {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ru[i] = ldg128_if(reinterpret_cast<const uint4*>(p.rotation) + tid + CD_THREADS * i, true);
+    };
+    auto store_rotation = [&]() {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int at = tid + CD_THREADS * i;
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(r_piece(at >> 4, at & 15)), "r"(ru[i].x), "r"(ru[i].y), "r"(ru[i].z), "r"(ru[i].w) : "memory");
+        }
+    };
+
+    // ---- before the wait: positions and R on their way, table and bounds meanwhile, then the first tile ----
+    if (p.early) fetch_position();
+    if (BITS != 0 && staged) fetch_rotation();
+    const uint32_t bar = base + CdSmem::BAR_OFF;
+    if (S > 1) {
+        if (tid == 0) {
+            mbar_init(bar, 1);
+            fence_mbar_init();
+            mbar_arrive_expect_tx(bar, (uint32_t)nh * (HEAD_DIM * 4u + S * 8u));
+        }
+        __syncwarp();
+        cluster_arrive();  // (the wait comes before the first store to another CTA: it has started then, its barrier is set)
+    }
+    constexpr int NBND = BITS == 4 ? 15 : 3;
+    if (BITS != 0 && tid <= NBND + 1) {
+        const float bound = tid == 0 ? -3.4e38f : (tid > NBND ? 3.4e38f : (BITS == 4 ? kBnd4[(tid - 1) & 15] : kBnd2[(tid - 1) & 3]));
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::BND_OFF + 4u * (uint32_t)tid), "f"(bound) : "memory");
+    }
+    if (BITS != 0 && tid >= 32 && tid < 48)
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::CENT_OFF + 4u * (uint32_t)(tid - 32)), "f"(BITS == 4 ? kCent4[tid & 15] : kCent2[tid & 3]) : "memory");
+    constexpr uint32_t LOW = cd_low_table(BITS);
+    auto table_entry = [&](uint32_t at, float c0, float c1) {  // four lanes' copies of two centroids
+        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(pack_half2(c0, c1)) : "memory");
+        if (EXACT) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + LOW), "r"(pack_low_half2(c0, c1)) : "memory");
+    };
+    if constexpr (BITS == 4) {
+        const float lo = kCent4[(tid >> 3) & 15];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)  // entry (tid >> 3) + 32 i, lanes 4 (tid & 7) .. + 3
+            table_entry(lut_s + (uint32_t)((tid >> 3) + 32 * i) * 256u + (uint32_t)(tid & 7) * 16u, lo, kCent4[(tid >> 7) + 2 * i]);
+    } else if constexpr (BITS == 2) {
+        if (tid < 128) table_entry(lut_s + (uint32_t)(tid >> 3) * 256u + (uint32_t)(tid & 7) * 16u, kCent2[(tid >> 3) & 3], kCent2[tid >> 5]);
+    }
+    if (BITS != 0 && staged) store_rotation();
+    uint32_t lutlane;  // produced behind the barrier that the table waits for: the look-ups, which take it into their address, cannot move above it
+    auto after_table = [&]() { asm volatile("mov.u32 %0, %1;" : "=r"(lutlane) : "r"(window | ((uint32_t)lane << 2)) : "memory"); };
+    auto lut = [&](uint32_t w, int byte) -> uint32_t {  // the table's entry for a byte of w: two halves
+        uint32_t r;
+        asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS));
+        return r;
+    };
+    auto lut_low = [&](uint32_t w, int byte) -> uint32_t {  // EXACT: the low parts
+        uint32_t r;
+        asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS + LOW));
+        return r;
+    };
+    // One tile per warp: the K rows' operands are looked up as soon as the rows are there, in a chain of layers under the previous
+    // kernel's tail.
+    constexpr bool PRE = BITS != 0 && MB == 1 && !EXACT;
+    uint32_t ka[PRE ? 8 : 1][4];
+    auto look_up_k = [&]() {
+        auto now = [&](uint32_t w, int byte) -> uint32_t {  // (volatile: not behind the wait, where it would be on the critical path)
+            uint32_t r;
+            asm volatile("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS));
+            return r;
+        };
+#pragma unroll
+        for (int j = 0; j < (PRE ? 8 : 0); ++j) {
+            if constexpr (BITS == 4) {
+                const uint4 lo4 = kw[0][0][0], hi4 = kw[0][1][0];
+                const uint32_t lo = j < 2 ? lo4.x : (j < 4 ? lo4.y : (j < 6 ? lo4.z : lo4.w)), hi = j < 2 ? hi4.x : (j < 4 ? hi4.y : (j < 6 ? hi4.z : hi4.w));
+                ka[j][0] = now(lo, 2 * (j & 1)); ka[j][1] = now(hi, 2 * (j & 1));
+                ka[j][2] = now(lo, 2 * (j & 1) + 1); ka[j][3] = now(hi, 2 * (j & 1) + 1);
+            } else {
+                const uint32_t lo = j < 4 ? kw[0][0][0].x : kw[0][0][0].y, hi = j < 4 ? kw[0][1][0].x : kw[0][1][0].y;
+                ka[j][0] = now(lo & 0x0f0f0f0fu, j & 3); ka[j][1] = now(hi & 0x0f0f0f0fu, j & 3);
+                ka[j][2] = now((lo >> 4) & 0x0f0f0f0fu, j & 3); ka[j][3] = now((hi >> 4) & 0x0f0f0f0fu, j & 3);
+            }
+        }
+    };
     if (p.early) first_tile();
+    if (staged) {
+        __syncthreads();  // table, R: under the previous kernel's tail too
+        after_table();
+        if (PRE && p.early && tile < tile_end) look_up_k();
+    }
     pdl_wait();
     pdl_launch_dependents();
-    if (!p.early) first_tile();
-    if (BITS != 0 && !p.static_rotation) stage_rotation();
+    if (!p.early) fetch_position();
+    if (!staged) fetch_rotation();
+    if (HOST && !p.early) first_tile();  // (the inputs take longer than the rows: they come over the bus)
 
     // ---- queries ----
     uint32_t qb[8][2];  // B fragments of the score product: lane (gl, t4) holds head gl, step j coordinates 32 t4 + 4 j ..
@@ -358,7 +414,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         const __half* src = p.q + (size_t)g * p.q_dim + (size_t)(head0 + gl) * HEAD_DIM;
         qw[m] = HOST ? lds128_if(in_s + (uint32_t)(gl * 256 + 16 * c), gl < nh) : ldg128_if(src + 8 * c, gl < nh);
     }
-    // the CTA that owns the sequence's last tile also takes the new token: K and V are rows 8 and 9 of the rotation's A operand
+    // the owner takes the new token: K and V are rows 8 and 9 of the rotation's A operand
     const int vec = tid >> 7, d = tid & 127;
     uint4 nw[4];
 #pragma unroll
@@ -367,15 +423,22 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         nw[m] = HOST ? lds128_if(in_s + (uint32_t)((nh + gl) * 256 + 16 * (4 * m + t4)), on)
                               : ldg128_if((gl == 0 ? p.new_k : p.new_v) + new_at + 8 * (4 * m + t4), on);
     }
+    uint2 q4 = make_uint2(0u, 0u);  // fp16 rows: head `warp`, coordinates 4 lane .., for the new token's score
+    __half xh = __ushort_as_half((unsigned short)0);
     if (owner) {
-        __half xh;
         if constexpr (HOST) {
             unsigned short u;
             asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(in_s + (uint32_t)((nh + vec) * 256 + 2 * d)));
             xh = __ushort_as_half(u);
+            if (BITS == 0 && warp < nh) q4 = lds64(in_s + (uint32_t)(warp * 256 + 8 * lane));
         } else {
             xh = ldg_half_if((vec == 0 ? p.new_k : p.new_v) + new_at + d, true);
+            if (BITS == 0) q4 = ldg64_if(p.q + (size_t)g * p.q_dim + (size_t)(head0 + warp) * HEAD_DIM + 4 * lane, warp < nh);
         }
+    }
+    if (!staged) store_rotation();
+    if (!HOST && !p.early) first_tile();
+    if (owner) {
         asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + CdSmem::RAW_OFF + 2u * (uint32_t)tid), "h"(__half_as_ushort(xh)) : "memory");
         if (!pos_ok && tid == 0 && p.status) atomicMax(p.status, ST_BAD_POSITION);
         if constexpr (BITS != 0) {  // sum of squares in the reference's order (tq_append.cuh)
@@ -386,24 +449,34 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::WP_OFF + 4u * (uint32_t)warp), "f"(sq) : "memory");
         }
     }
-    __syncthreads();  // table, R, warp sums, raw token
+    if (owner || !staged) __syncthreads();  // warp sums, raw token; a rotation that was not staged before the wait, and the table
+    if (!staged) after_table();
     if constexpr (BITS != 0) {
         // rotated queries, rot[h][n] = sum_k q[h][k] R[n][k]: warp w takes the coordinate blocks w and w + 8
         float nc[4];  // rows 8 (lanes gl = 0: K) and 9 (gl = 1: V): coordinates 8 warp + 2 t4, + 1, and the same + 64
+        float rc[2][2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) rc[i][0][e] = rc[i][1][e] = 0.0f;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            uint4 b4[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) b4[i] = lds128(r_piece(8 * (warp + CD_WARPS * i) + gl, 4 * m + t4));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                mma16816(rc[i][0], qw[m].x, nw[m].x, qw[m].y, nw[m].y, b4[i].x, b4[i].y);
+                mma16816(rc[i][1], qw[m].z, nw[m].z, qw[m].w, nw[m].w, b4[i].z, b4[i].w);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const int nb = warp + CD_WARPS * i;
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, c2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            float c[4];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const uint4 b4 = lds128(r_piece(8 * nb + gl, 4 * m + t4));
-                mma16816(c, qw[m].x, nw[m].x, qw[m].y, nw[m].y, b4.x, b4.y);
-                mma16816(c2, qw[m].z, nw[m].z, qw[m].w, nw[m].w, b4.z, b4.w);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) c[e] += c2[e];
+            for (int e = 0; e < 4; ++e) c[e] = rc[i][0][e] + rc[i][1][e];
             const float sc = 0.12751743074602467f;  // log2(e) / sqrt(128)
-            const uint32_t q_at = base + CdSmem::Q_OFF + (uint32_t)(gl * MERGE_ROW + 8 * nb + 2 * t4) * 2u;
+            const uint32_t q_at = base + CdSmem::Q_OFF + (uint32_t)(gl * MERGE_ROW + 8 * (warp + CD_WARPS * i) + 2 * t4) * 2u;
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(q_at), "r"(pack_half2(c[0] * sc, c[1] * sc)) : "memory");
             if (EXACT)
                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(q_at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), "r"(pack_low_half2(c[0] * sc, c[1] * sc)) : "memory");
@@ -487,66 +560,53 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     }
 
+    // ---- the new token, in its owner: warp h takes its score with query head h (its weight in the CTA's result follows below) ----
+    auto lds_f32 = [&](uint32_t a) { float f; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(a)); return f; };
+    auto centroid = [&](uint32_t code) { return lds_f32(base + CdSmem::CENT_OFF + 4u * code); };
+    const bool takes_new = owner && appends;  // uniform for the CTA
+    if (takes_new && warp < nh) {
+        float q[4], k[4];
+        auto halves = [&](uint2 u, float (&f)[4]) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+        };
+        float scale = 0.12751743074602467f;
+        if constexpr (BITS == 0) {
+            halves(q4, q);
+            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
+        } else {
+            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(warp * MERGE_ROW + 4 * lane) * 2u;
+            halves(lds64(at), q);
+            if constexpr (EXACT) {
+                float ql4[4];
+                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
+            }
+            uint32_t w;
+            if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 2u * (uint32_t)lane));
+            else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + (uint32_t)lane));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) k[e] = centroid((w >> (BITS * e)) & ((1u << BITS) - 1u));
+            scale = lds_f32(base + CdSmem::NN_OFF);
+        }
+        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)warp), "f"(dot * scale) : "memory");
+    }
+
     // ---- tiles ----
-    uint32_t lutlane;  // produced behind the barriers: the look-ups, which take it into their address, cannot move above them
-    asm volatile("mov.u32 %0, %1;" : "=r"(lutlane) : "r"(window | ((uint32_t)lane << 2)) : "memory");
-    auto lut = [&](uint32_t w, int byte) -> uint32_t {  // the table's entry for a byte of w: two halves
-        uint32_t r;
-        asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS));
-        return r;
-    };
-    auto lut_low = [&](uint32_t w, int byte) -> uint32_t {  // EXACT: the low parts
-        uint32_t r;
-        asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(r) : "r"(prmt(w, lutlane, 0x7604u | ((uint32_t)byte << 4))), "n"(CD_LUT_ABS + LOW));
-        return r;
-    };
+    const bool any_tile = tile < tile_end;
+    if (PRE && !(staged && p.early) && any_tile) look_up_k();
     float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};
     float acc[8][4];
 #pragma unroll
     for (int b = 0; b < 8; ++b) acc[b][0] = acc[b][1] = acc[b][2] = acc[b][3] = 0.0f;
     for (; tile < tile_end; tile += tile_step) {
         const int t0 = tile * TT;
-        if (appends && owner && tile * TT <= pos && pos < tile * TT + TT) {  // the new token of the sequence, from shared memory
-            const uint32_t nk = base + (BITS == 0 ? CdSmem::RAW_OFF : CdSmem::NEW_OFF), nv = nk + (BITS == 0 ? 256u : 128u);
-            float nkn = 0.0f, nvn = 0.0f;
-            if (BITS != 0) {
-                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(nkn) : "r"(base + CdSmem::NN_OFF));
-                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(nvn) : "r"(base + CdSmem::NN_OFF + 4u));
-            }
-#pragma unroll
-            for (int b = 0; b < MB; ++b) {
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-                    if (t0 + 16 * b + 8 * r + gl == pos) {
-                        if constexpr (BITS == 2) {
-                            const uint2 w = lds64(nk + 8u * t4);
-                            kw[b][r][0].x = w.x; kw[b][r][0].y = w.y;
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < KV4; ++i) kw[b][r][i] = lds128(nk + 16u * (KV4 * t4 + i));
-                        }
-                        if constexpr (BITS != 0) {
-                            kn_h[b][r] = __float2half_rn(nkn);
-                            vn_h[b][r] = __float2half_rn(nvn);
-                        }
-                    }
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    if (t0 + 16 * b + 2 * t4 + (r & 1) + 8 * (r >> 1) == pos) {
-                        if constexpr (BITS == 4) {
-                            const uint2 w = lds64(nv + 8u * gl);
-                            vw[b][r][0].x = w.x; vw[b][r][0].y = w.y;
-                        } else if constexpr (BITS == 2) {
-                            vw[b][r][0].x = lds32(nv + 4u * gl);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < VV4; ++i) vw[b][r][i] = lds128(nv + 16u * (VV4 * gl + i));
-                        }
-                    }
-            }
-        }
         // ---- scores: rows gl and gl + 8 of each block, heads 2 t4 and 2 t4 + 1 ----
-        float c[MB][4], ce[MB][4];  // ce, EXACT: the products with one low part
+        float c[MB][4], ce[MB][4];  // ce: EXACT, the products with one low part; a single block: every other step, for two short chains
 #pragma unroll
         for (int b = 0; b < MB; ++b) c[b][0] = c[b][1] = c[b][2] = c[b][3] = ce[b][0] = ce[b][1] = ce[b][2] = ce[b][3] = 0.0f;
 #pragma unroll
@@ -560,7 +620,9 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                         mma16816(ce[b], lut_low(wlo, blo), lut_low(whi, bhi), lut_low(wlo2, blo2), lut_low(whi2, bhi2), qb[j][0], qb[j][1]);
                     }
                 };
-                if constexpr (BITS == 4) {
+                if constexpr (PRE) {
+                    a0 = ka[j][0]; a1 = ka[j][1]; a2 = ka[j][2]; a3 = ka[j][3];
+                } else if constexpr (BITS == 4) {
                     const uint4 lo4 = kw[b][0][0], hi4 = kw[b][1][0];
                     const uint32_t lo = j < 2 ? lo4.x : (j < 4 ? lo4.y : (j < 6 ? lo4.z : lo4.w)), hi = j < 2 ? hi4.x : (j < 4 ? hi4.y : (j < 6 ? hi4.z : hi4.w));
                     a0 = lut(lo, 2 * (j & 1)); a1 = lut(hi, 2 * (j & 1));
@@ -577,9 +639,9 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                     a0 = (j & 1) ? lo.z : lo.x; a1 = (j & 1) ? hi.z : hi.x;
                     a2 = (j & 1) ? lo.w : lo.y; a3 = (j & 1) ? hi.w : hi.y;
                 }
-                mma16816(c[b], a0, a1, a2, a3, qb[j][0], qb[j][1]);
+                mma16816(MB == 1 && !(EXACT && BITS != 0) && (j & 1) ? ce[b] : c[b], a0, a1, a2, a3, qb[j][0], qb[j][1]);
             }
-        if (EXACT && BITS != 0) {
+        if ((EXACT && BITS != 0) || MB == 1) {
 #pragma unroll
             for (int b = 0; b < MB; ++b)
 #pragma unroll
@@ -592,7 +654,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             for (int r = 0; r < 2; ++r) {
                 const float n = BITS == 0 ? 0.12751743074602467f : __half2float(kn_h[b][r]);
                 const int t = t0 + 16 * b + 8 * r + gl;
-                const bool on = t >= lo && t < hi;
+                const bool on = t < lim;
                 sv[2 * b + r][0] = on ? c[b][2 * r] * n : -1e30f;
                 sv[2 * b + r][1] = on ? c[b][2 * r + 1] * n : -1e30f;
             }
@@ -626,7 +688,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
 #pragma unroll
         for (int i = 0; i < 2 * MB; ++i) {
             const int t = t0 + 16 * (i >> 1) + 8 * (i & 1) + gl;
-            const bool on = t >= lo && t < hi;
+            const bool on = t < lim;
             const float p0 = on ? ex2_approx(sv[i][0] - m_run[0]) : 0.0f, p1 = on ? ex2_approx(sv[i][1] - m_run[1]) : 0.0f;
             l_run[0] += p0;
             l_run[1] += p1;
@@ -681,57 +743,81 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                 }
             }
         }
-        if (next < tile_end) load_v(next, lim);
+        if (next < tile_end) {
+            load_v(next, lim);
+            if (PRE) look_up_k();
+        }
     }
 
     // ---- the warps' results: acc[b]: coordinates 16 gl + 2 b (and + 1), heads 2 t4, 2 t4 + 1 ----
+    if (any_tile) {
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-        l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], o);
-        l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], o);
-    }
+        for (int o = 4; o < 32; o <<= 1) {
+            l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], o);
+            l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], o);
+        }
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int h = 2 * t4 + e;
-        if (h < nh) {
-            const uint32_t dst = warps_s + (uint32_t)((warp * nh + h) * PART_STRIDE) * 4u;
+        for (int e = 0; e < 2; ++e) {
+            const int h = 2 * t4 + e;
+            if (h < nh) {
+                const uint32_t dst = warps_s + (uint32_t)((warp * nh + h) * PART_STRIDE) * 4u;
 #pragma unroll
-            for (int b2 = 0; b2 < 4; ++b2)
-                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(16 * gl + 4 * b2) * 4u), "f"(acc[2 * b2][e]),
-                             "f"(acc[2 * b2][2 + e]), "f"(acc[2 * b2 + 1][e]), "f"(acc[2 * b2 + 1][2 + e]) : "memory");
-            if (gl == 0)
-                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst + HEAD_DIM * 4u), "f"(m_run[e]), "f"(l_run[e]) : "memory");
+                for (int b2 = 0; b2 < 4; ++b2)
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(16 * gl + 4 * b2) * 4u), "f"(acc[2 * b2][e]),
+                                 "f"(acc[2 * b2][2 + e]), "f"(acc[2 * b2 + 1][e]), "f"(acc[2 * b2 + 1][2 + e]) : "memory");
+                if (gl == 0)
+                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst + HEAD_DIM * 4u), "f"(m_run[e]), "f"(l_run[e]) : "memory");
+            }
         }
     }
     __syncthreads();
     // ---- the CTA's result, normalised: maximum and sum beside it ----
-    auto lds_f32 = [&](uint32_t a) { float f; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(a)); return f; };
     // where coordinate n of head h goes in the CTA that adds up its share: [this CTA][head][coordinate of the share]
-    const int share = HEAD_DIM / (int)S;
+    const uint32_t s_log = 31u - (uint32_t)__clz((int)S), share_log = 7u - s_log;  // (S is a power of two)
     auto send = [&](int h, int n, float v0, float v1) {  // coordinates n, n + 1
-        const int r = n / share;
-        st_async_f32x2(map_shared(base + CdSmem::CP_OFF + (uint32_t)(((int)rank * nh + h) * share + (n - r * share)) * 4u, (uint32_t)r), v0, v1,
-                       map_shared(bar, (uint32_t)r));
+        const uint32_t r = (uint32_t)n >> share_log;
+        st_async_f32x2(map_shared(base + CdSmem::CP_OFF + ((((rank * (uint32_t)nh + (uint32_t)h) << share_log) + ((uint32_t)n & ((1u << share_log) - 1u))) << 2), r), v0, v1,
+                       map_shared(bar, r));
     };
     if (S > 1) cluster_wait();  // every CTA of the cluster has started
     for (int i = tid; i < nh * HEAD_DIM; i += CD_THREADS) {  // (a warp stays within one head)
         const int h = i >> 7, k = i & 127;
         const uint32_t src = warps_s + (uint32_t)(h * PART_STRIDE) * 4u, wstride = (uint32_t)(nh * PART_STRIDE) * 4u;
-        float mw[CD_WARPS], M = -1e30f;
+        float mw[CD_WARPS], lw[CD_WARPS], aw[CD_WARPS], M = -1e30f, m_new = -1e30f, v_new = 0.0f;
+        if (takes_new) {
+            m_new = lds_f32(base + CdSmem::NS_OFF + 4u * (uint32_t)h);
+            if constexpr (BITS == 0) {
+                unsigned short u;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(base + CdSmem::RAW_OFF + 256u + 2u * (uint32_t)k));
+                v_new = __half2float(__ushort_as_half(u));
+            } else {
+                uint32_t w;
+                asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 128u + (uint32_t)(k * BITS >> 3)));
+                v_new = lds_f32(base + CdSmem::NN_OFF + 4u) * centroid((w >> (k * BITS & 7)) & ((1u << BITS) - 1u));
+            }
+            M = fmaxf(M, m_new);
+        }
 #pragma unroll
         for (int w = 0; w < CD_WARPS; ++w) {
-            mw[w] = lds_f32(src + (uint32_t)w * wstride + HEAD_DIM * 4u);
-            M = fmaxf(M, mw[w]);
+            mw[w] = -1e30f;
+            lw[w] = aw[w] = 0.0f;
+            if (w < n_act) {  // uniform for the CTA
+                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(mw[w]), "=f"(lw[w]) : "r"(src + (uint32_t)w * wstride + HEAD_DIM * 4u));
+                aw[w] = lds_f32(src + (uint32_t)w * wstride + (uint32_t)k * 4u);
+            }
         }
-        float a = 0.0f, z = 0.0f;
+#pragma unroll
+        for (int w = 0; w < CD_WARPS; ++w) M = fmaxf(M, mw[w]);
+        const float e_new = takes_new ? ex2_approx(m_new - M) : 0.0f;
+        float a = takes_new ? e_new * v_new : 0.0f, z = e_new;
 #pragma unroll
         for (int w = 0; w < CD_WARPS; ++w) {
-            const float e = ex2_approx(mw[w] - M);
-            a = fmaf(e, lds_f32(src + (uint32_t)w * wstride + (uint32_t)k * 4u), a);
-            z = fmaf(e, lds_f32(src + (uint32_t)w * wstride + (HEAD_DIM + 1) * 4u), z);
+            const float e = ex2_approx(mw[w] - M);  // (a warp without tiles: times zero)
+            a = fmaf(e, aw[w], a);
+            z = fmaf(e, lw[w], z);
         }
-        // one CTA: the reference's denominator; several: the part's own sum (none: no tile), the rest follows below
-        a = S == 1 ? a / (z + 1e-8f) : (z > 0.0f ? a / z : 0.0f);
+        // one CTA: the reference's denominator; several: the part's own sum (none: no token), the rest follows below
+        a = S == 1 ? a / (z + 1e-8f) : (z > 0.0f || z != z ? a * rcp_approx_ftz(z) : 0.0f);
         if (S > 1 && k < (int)S)
             st_async_f32x2(map_shared(base + CdSmem::MZ_OFF + (uint32_t)((int)rank * nh + h) * 8u, (uint32_t)k), M, z, map_shared(bar, (uint32_t)k));
         if constexpr (BITS == 0) {
@@ -747,31 +833,36 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     }
     if constexpr (BITS != 0) {
         __syncthreads();
-        // times R: o[h][n] = sum_k a[h][k] R[k][n], two blocks of 8 output coordinates per warp
-        uint32_t ah[4][4], al[4][4];  // rows 0-7 of two 16-k steps each (rows 8-15 of the operand are zero); rows >= nh are never read back
+        // times R: o[h][n] = sum_k a[h][k] R[k][n], two blocks of 8 output coordinates per warp.  The high parts are rows 0-7 of the A
+        // operand, the low parts rows 8-15 (rows >= nh are never read back)
+        uint32_t ah[4][4], al[4][4];  // two 16-k steps each
         const uint32_t a_at = base + CdSmem::Q_OFF + (uint32_t)((lane & 7) * MERGE_ROW + 8 * (lane >> 3)) * 2u;
 #pragma unroll
         for (int j2 = 0; j2 < 4; ++j2) {
             ldmatrix_x4(ah[j2], a_at + 64u * j2);
             ldmatrix_x4(al[j2], a_at + (CdSmem::LO_OFF - CdSmem::Q_OFF) + 64u * j2);
         }
+        float oc[2][2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) oc[i][0][e] = oc[i][1][e] = 0.0f;
+#pragma unroll
+        for (int j2 = 0; j2 < 4; ++j2) {  // two steps of 16 k each per ldmatrix
+            uint32_t b[2][4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) ldmatrix_x4_trans(b[i], r_piece(32 * j2 + lane, warp + CD_WARPS * i));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                mma16816(oc[i][0], ah[j2][0], al[j2][0], ah[j2][1], al[j2][1], b[i][0], b[i][1]);
+                mma16816(oc[i][1], ah[j2][2], al[j2][2], ah[j2][3], al[j2][3], b[i][2], b[i][3]);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int nb = warp + CD_WARPS * i;
-            float c[4][4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) c[e][0] = c[e][1] = c[e][2] = c[e][3] = 0.0f;
-#pragma unroll
-            for (int j2 = 0; j2 < 4; ++j2) {  // two steps of 16 k each per ldmatrix
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, r_piece(32 * j2 + lane, nb));
-                mma16816(c[0], ah[j2][0], 0u, ah[j2][1], 0u, b[0], b[1]);
-                mma16816(c[1], al[j2][0], 0u, al[j2][1], 0u, b[0], b[1]);
-                mma16816(c[2], ah[j2][2], 0u, ah[j2][3], 0u, b[2], b[3]);
-                mma16816(c[3], al[j2][2], 0u, al[j2][3], 0u, b[2], b[3]);
-            }
             if (gl < nh) {
-                const float o0 = (c[0][0] + c[2][0]) + (c[1][0] + c[3][0]), o1 = (c[0][1] + c[2][1]) + (c[1][1] + c[3][1]);
+                const float o0 = (oc[i][0][0] + oc[i][1][0]) + (oc[i][0][2] + oc[i][1][2]), o1 = (oc[i][0][1] + oc[i][1][1]) + (oc[i][0][3] + oc[i][1][3]);
                 if (S == 1) {
                     const size_t at = (size_t)(head0 + gl) * HEAD_DIM + 8 * nb + 2 * t4;
                     *reinterpret_cast<__half2*>(p.out + (size_t)g * p.q_dim + at) = __floats2half2_rn(o0, o1);
@@ -786,21 +877,25 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         if (!mbar_wait_bounded_hint(bar, 0u, 1u << 14, 20000u) && p.status) atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
         // ---- this CTA's share of the coordinates: one lane per (coordinate, CTA), the S lanes of a coordinate side by side ----
         for (int i = tid; i < nh * HEAD_DIM; i += CD_THREADS) {
-            const int r = i & ((int)S - 1), o = i / (int)S;       // (S is a power of two)
-            const int h = o / share, n = o - h * share;
-            const uint32_t mz = base + CdSmem::MZ_OFF + (uint32_t)(r * nh + h) * 8u;
-            const float v = lds_f32(base + CdSmem::CP_OFF + (uint32_t)((r * nh + h) * share + n) * 4u);
-            const float m = lds_f32(mz), z = lds_f32(mz + 4u);
+            const int r = i & ((int)S - 1), o = i >> s_log;
+            const int h = o >> share_log, n = o & ((1 << share_log) - 1);
+            const float v = lds_f32(base + CdSmem::CP_OFF + (uint32_t)(((r * nh + h) << share_log) + n) * 4u);
+            float m, z;
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m), "=f"(z) : "r"(base + CdSmem::MZ_OFF + (uint32_t)(r * nh + h) * 8u));
             float M = m;
-            for (int w = 1; w < (int)S; w <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, w));
+#pragma unroll
+            for (int w = 1; w < CD_MAX_CLUSTER; w <<= 1)
+                if (w < (int)S) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, w));
             float Z = ex2_approx(m - M) * z, a = Z * v;
-            for (int w = 1; w < (int)S; w <<= 1) {
-                Z += __shfl_xor_sync(0xffffffffu, Z, w);
-                a += __shfl_xor_sync(0xffffffffu, a, w);
-            }
+#pragma unroll
+            for (int w = 1; w < CD_MAX_CLUSTER; w <<= 1)
+                if (w < (int)S) {
+                    Z += __shfl_xor_sync(0xffffffffu, Z, w);
+                    a += __shfl_xor_sync(0xffffffffu, a, w);
+                }
             if (r == 0) {
-                a /= Z + 1e-8f;
-                const size_t at = (size_t)(head0 + h) * HEAD_DIM + (int)rank * share + n;
+                a = __fdividef(a, Z + 1e-8f);
+                const size_t at = (size_t)(head0 + h) * HEAD_DIM + ((int)rank << share_log) + n;
                 p.out[(size_t)g * p.q_dim + at] = __float2half_rn(a);
                 if (p.out_f32) p.out_f32[(size_t)g * p.H * HEAD_DIM + at] = a;
             }
