@@ -560,41 +560,9 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     }
 
-    // ---- the new token, in its owner: warp h takes its score with query head h (its weight in the CTA's result follows below) ----
     auto lds_f32 = [&](uint32_t a) { float f; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(a)); return f; };
     auto centroid = [&](uint32_t code) { return lds_f32(base + CdSmem::CENT_OFF + 4u * code); };
     const bool takes_new = owner && appends;  // uniform for the CTA
-    if (takes_new && warp < nh) {
-        float q[4], k[4];
-        auto halves = [&](uint2 u, float (&f)[4]) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
-        };
-        float scale = 0.12751743074602467f;
-        if constexpr (BITS == 0) {
-            halves(q4, q);
-            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
-        } else {
-            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(warp * MERGE_ROW + 4 * lane) * 2u;
-            halves(lds64(at), q);
-            if constexpr (EXACT) {
-                float ql4[4];
-                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
-            }
-            uint32_t w;
-            if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 2u * (uint32_t)lane));
-            else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + (uint32_t)lane));
-#pragma unroll
-            for (int e = 0; e < 4; ++e) k[e] = centroid((w >> (BITS * e)) & ((1u << BITS) - 1u));
-            scale = lds_f32(base + CdSmem::NN_OFF);
-        }
-        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)warp), "f"(dot * scale) : "memory");
-    }
 
     // ---- tiles ----
     const bool any_tile = tile < tile_end;
@@ -747,6 +715,39 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             load_v(next, lim);
             if (PRE) look_up_k();
         }
+    }
+
+    // ---- the new token, in its owner: warp h takes its score with query head h (its weight in the CTA's result follows below) ----
+    if (takes_new && warp < nh) {
+        float q[4], k[4];
+        auto halves = [&](uint2 u, float (&f)[4]) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+        };
+        float scale = 0.12751743074602467f;
+        if constexpr (BITS == 0) {
+            halves(q4, q);
+            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
+        } else {
+            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(warp * MERGE_ROW + 4 * lane) * 2u;
+            halves(lds64(at), q);
+            if constexpr (EXACT) {
+                float ql4[4];
+                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
+            }
+            uint32_t w;
+            if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 2u * (uint32_t)lane));
+            else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + (uint32_t)lane));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) k[e] = centroid((w >> (BITS * e)) & ((1u << BITS) - 1u));
+            scale = lds_f32(base + CdSmem::NN_OFF);
+        }
+        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)warp), "f"(dot * scale) : "memory");
     }
 
     // ---- the warps' results: acc[b]: coordinates 16 gl + 2 b (and + 1), heads 2 t4, 2 t4 + 1 ----

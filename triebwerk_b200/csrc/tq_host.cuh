@@ -395,15 +395,21 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
 }
 
 // One cluster per (sequence, KV head, block of 8 query heads): tq_decode_cluster.cuh.  `max_tokens`: rows a sequence may hold.
+constexpr size_t CD_ONE_PER_SM = 118 * 1024;  // more than half of an SM's shared memory
 template <int BITS, int MB, bool HOST, bool EXACT>
 inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int layers, cudaStream_t s, bool pdl) {
     const void* kernel = (const void*)cluster_decode_kernel<BITS, MB, HOST, EXACT>;
-    int r = ensure_dynamic_smem(kernel, cd_smem_bytes(BITS, CD_HEADS, EXACT), true);
+    int r = ensure_dynamic_smem(kernel, std::max(cd_smem_bytes(BITS, CD_HEADS, EXACT), CD_ONE_PER_SM), true);
     if (r != TQ_OK) return r;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)S, (unsigned)(p.Hkv * p.head_blocks), (unsigned)(p.G * layers));
     cfg.blockDim = dim3(CD_THREADS);
     cfg.dynamicSmemBytes = cd_smem_bytes(BITS, std::min(CD_HEADS, p.H / p.Hkv), EXACT);
+    // One CTA per SM where they fit and none starts under a launch of its own kind (its room would be needed then): small clusters come
+    // two to an SM otherwise, with SMs idle (launchers, 2-bit 32/8 heads 8 x 1023 tokens 18.5 us a layer, one per SM 17.5; 4-bit 16/8
+    // 8 x 1500 22.4 / 20.5).  Clusters of 4 and more find no room that way (4-bit 4 x 600 13.5 / 14.2, 1 x 3000 15.1 / 19.4).
+    if (S <= 2 && !p.early && !p.static_rotation && (long long)S * cfg.gridDim.y * cfg.gridDim.z <= device_props().sm_count)
+        cfg.dynamicSmemBytes = std::max(cfg.dynamicSmemBytes, CD_ONE_PER_SM);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -417,7 +423,9 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
 }
 // CTAs per cluster.  As many as give every warp a 16-token block of its own, up to one CTA per SM over the whole launch: two share
 // the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue (8 sequences x 1023 tokens through
-// the launchers 24 us a layer with two, 19 with one).  Clusters of 4 and more leave some of a processing cluster's SMs over (136
+// the launchers 24 us a layer with two, 19 with one).  16 only where 8 leave a warp two blocks and more: seven of the GPU's
+// processing clusters hold one cluster of 16 beside the previous launch's, an eighth waits (1 sequence, 8 KV heads, 4-bit: 600 tokens 5.2 us
+// with 8 and 7.9 with 16, 1500 tokens 5.5 / 6.2, 3000 tokens 7.4 / 6.8; fp16 1500 5.3 / 5.6, 3000 11.0 / 7.9).  Clusters of 4 and more leave some of a processing cluster's SMs over (136
 // of 148 serve fours, 128 eights): one cluster more than fits waits for a whole turn (72 clusters of 4 at two CTAs per SM 1.5
 // times the time of 72 of 2).  Where a warp goes through many tiles, more than the launch's fixed part costs, a second CTA per SM
 // hides the latency of the first one's loads: above 12 tiles 0.6 to 0.95 of the time (4 x 8192 tokens, 8 KV heads, 44 -> 28 us),
@@ -427,7 +435,8 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
     const long long sms = device_props().sm_count, blocks = (max_tokens + 15) / 16;
     auto fit = [&](int n) { return sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
     int S = 1;
-    while (S < CD_MAX_CLUSTER && (long long)S * CD_WARPS < blocks && clusters * S * 2 <= fit(2 * S)) S *= 2;
+    auto longer = [&](int n) { return n == 8 ? 2 * n * CD_WARPS <= blocks : n * CD_WARPS < blocks; };
+    while (S < CD_MAX_CLUSTER && longer(S) && clusters * S * 2 <= fit(2 * S)) S *= 2;
     if (S <= 4 && clusters * S * 8 <= 7 * sms && clusters * S * 2 <= 2 * fit(2 * S) && blocks > (bits ? 12 : 4) * CD_WARPS * S &&
         (heads <= 4 || bits == 0))
         S *= 2;
