@@ -392,6 +392,14 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     constexpr bool PERSIST = MODE == 2 || MODE == 4;
     constexpr bool COPIER = MODE == 2;
     constexpr bool SEPARATE = MODE == 3;
+    // Eight KV heads have at most four query heads each (ATTN_MAX_HEADS), half of a product's eight columns.  Head h takes the columns
+    // 2 h and 2 h + 1: a lane's two score columns are ONE head, so that it has half the exponentials; in the value product the even
+    // column sums the first eight tokens of a step, the odd one the other eight.
+    constexpr bool PAIR = HKV == 8;
+    constexpr int NE = PAIR ? 1 : 2;               // query heads per lane in the score layout
+    // 2-bit: a centroid is affine in its code's two bits, so the scores need no table: every bit of the code bytes, masked in place, is
+    // a plane of an integer product with 16-bit fixed-point queries (see make_planes).
+    constexpr bool PLANES = PAIR && BITS == 2;
     extern __shared__ __align__(1024) uint8_t dyn_smem[];
 
     const int tid = threadIdx.x;
@@ -1048,13 +1056,74 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         // query fragments (B operand of the score product): lane (gl, t4) holds coordinates 32*t4 .. 32*t4+31 of head
         // head*grp + gl as fp16
         uint32_t qb[8][2];
-        // lane (gl, t4): the 32 coordinates 32*t4 .. of head head*grp + gl from the merge area, rows `pitch` bytes apart
+        const int q_col = PAIR ? gl >> 1 : gl;                                       // query head of this lane's column
+        const bool q_on = q_col < grp && !(PAIR && !PLANES && (gl & 1));             // (fp16 queries: the odd columns stay zero)
+        float s_scale = 0.0f, s_zero = 0.0f;  // PLANES: score = (sum * s_scale + s_zero) * K norm, of head t4
+        // PLANES: the queries as integers Q, |Q| <= 32639, in two signed bytes: the even column of a head has the high ones, the odd
+        // column the low ones.  Code 2 b1 + b0 stands for -c3 + (c3 - c2) b0 + (c3 + c2) b1, c2 and c3 the positive centroids.  Bit b of
+        // a byte's coordinate j is worth 2^(2 j + b) where it stands: the query of that plane is divided by it (by 2^(2 (j mod 2) + b): the
+        // coordinates 0, 1 and 2, 3 have sums of their own, 16 apart).  The sum's offset is minus half the sum with all bits set.
+        // Rounding: 4e-5 of the largest coordinate at most, 1.3e-4 of a typical one where fp16 has 2e-4.
+        auto make_planes = [&](const float (&x)[32]) {
+            constexpr float C0 = 0.13351f - 0.04003f, C1 = 0.13351f + 0.04003f;
+            uint32_t top = 0u;  // of the magnitudes' bits: an infinity or a NaN comes out on top
+#pragma unroll
+            for (int i = 0; i < 32; ++i) top = max(top, __float_as_uint(x[i]) & 0x7fffffffu);
+            top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            const float mx = __uint_as_float(top);
+            const bool some = mx > 1e-30f;
+            const float k = some ? 32639.0f / (mx * C0) : 0.0f;
+            const float scale = some ? mx * (C0 / (16.0f * 32639.0f)) : (mx == mx ? 0.0f : mx);
+            const uint32_t bias = (gl & 1) ? 0u : 128u, sel = (gl & 1) ? 0x0040u : 0x0051u;
+            const float magic = 12582912.0f + (float)bias;  // 1.5 * 2^23: the sum's low bits are the rounded integer
+            uint32_t all = 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const uint32_t weight = 1u << (2 * (j & 1) + b);
+                    const float kk = k * ((b ? C1 : C0) / (float)weight);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        uint32_t u[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            u[i] = __float_as_uint(fmaf(x[16 * r + 4 * i + j], kk, magic));
+                            all += weight * u[i];
+                        }
+                        qb[2 * j + b][r] = prmt(prmt(u[0], u[1], sel), prmt(u[2], u[3], sel), 0x5410u);
+                    }
+                }
+            all -= 240u * (0x4b400000u + bias);  // 8 bytes' weights
+            all += __shfl_xor_sync(0xffffffffu, all, 1);
+            all += __shfl_xor_sync(0xffffffffu, all, 2);
+            const float zero = -8.0f * (float)(int)all * scale;
+            s_scale = __shfl_sync(0xffffffffu, scale, 8 * t4);
+            s_zero = __shfl_sync(0xffffffffu, zero, 8 * t4);
+        };
+        // lane (gl, t4): the 32 coordinates 32*t4 .. of its head from the merge area, rows `pitch` bytes apart
         auto take_fragments = [&](uint32_t pitch) {
             uint4 qw[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 qw[i] = make_uint4(0u, 0u, 0u, 0u);
-                if (gl < grp && !dead) qw[i] = ldsv128(merge_s + (uint32_t)(head * grp + gl) * pitch + (uint32_t)(32 * t4 + 8 * i) * 2u);
+                if (q_on && !dead) qw[i] = ldsv128(merge_s + (uint32_t)(head * grp + q_col) * pitch + (uint32_t)(32 * t4 + 8 * i) * 2u);
+            }
+            if constexpr (PLANES) {
+                float x[32];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const __half2* h2 = reinterpret_cast<const __half2*>(&qw[i]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __half22float2(h2[e]);
+                        x[8 * i + 2 * e] = f.x;
+                        x[8 * i + 2 * e + 1] = f.y;
+                    }
+                }
+                make_planes(x);
+                return;
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -1199,8 +1268,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                         asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(o0 + 8u * HEAD_DIM * 4u), "f"(c[2] * sc), "f"(c[3] * sc) : "memory");
                     }
                     group_barrier(group, gthreads);
-                    const int myrow = head * grp + gl - hb;
-                    if (gl < grp && myrow >= 0 && myrow < 16 && !TQ_DBG(8)) {
+                    const int myrow = head * grp + q_col - hb;
+                    if (q_on && myrow >= 0 && myrow < 16 && !TQ_DBG(8)) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             float4 f;
@@ -1211,9 +1280,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                     }
                     group_barrier(group, gthreads);
                 }
-            } else if (gl < grp && !TQ_DBG(8)) {
+            } else if (q_on && !TQ_DBG(8)) {
                 const float4* src =
-                    reinterpret_cast<const float4*>(p.q_rot + ((size_t)g * p.H + (size_t)head * grp + gl) * HEAD_DIM + 32 * t4);
+                    reinterpret_cast<const float4*>(p.q_rot + ((size_t)g * p.H + (size_t)head * grp + q_col) * HEAD_DIM + 32 * t4);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     float4 f = __ldg(src + i);
@@ -1223,8 +1292,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #pragma unroll
                 for (int i = 0; i < 32; ++i) qv[i] = 0.0f;
             }
+            if constexpr (PLANES) make_planes(qv);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < (PLANES ? 0 : 8); ++j) {
                 // the 2-bit table returns the four values of a byte as (0, 2), (1, 3)
                 const float x0 = qv[4 * j], x1 = BITS == 2 ? qv[4 * j + 2] : qv[4 * j + 1];
                 const float x2 = BITS == 2 ? qv[4 * j + 1] : qv[4 * j + 2], x3 = qv[4 * j + 3];
@@ -1233,8 +1303,10 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             }
         }
 
-        // running maximum and (per lane: over its own token rows) sum of the two score columns of this lane
-        float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};
+        // running maximum and (per lane: over its own token rows) sum of the heads of this lane's score columns
+        float m_run[NE], l_run[NE];
+#pragma unroll
+        for (int e = 0; e < NE; ++e) { m_run[e] = -1e30f; l_run[e] = 0.0f; }
         float acc[8][4];
 #pragma unroll
         for (int b = 0; b < 8; ++b) { acc[b][0] = acc[b][1] = acc[b][2] = acc[b][3] = 0.0f; }
@@ -1303,6 +1375,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 // blocks of 16 token rows.  Row r of block rb is token 16*rb + 8*(r >> 3) + tau(r & 7) of the tile; the
                 // eight 16-coordinate steps of a row block form one accumulator chain.
                 float c[2][4];
+                int t_lo[2][4], t_hi[2][4];  // PLANES: sums of the coordinates 0, 1 and 2, 3 of every byte
                 {
                     uint32_t w[4][4];
 #pragma unroll
@@ -1316,9 +1389,25 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                         }
                     }
 #pragma unroll
-                    for (int rb = 0; rb < 2; ++rb) c[rb][0] = c[rb][1] = c[rb][2] = c[rb][3] = 0.0f;
+                    for (int rb = 0; rb < 2; ++rb) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                        for (int e = 0; e < 4; ++e) {
+                            c[rb][e] = 0.0f;
+                            t_lo[rb][e] = t_hi[rb][e] = 0;
+                        }
+                    }
+                    if constexpr (PLANES) {
+#pragma unroll
+                        for (int pl = 0; pl < 4; ++pl)
+#pragma unroll
+                            for (int rb = 0; rb < 2; ++rb) {
+                                const uint32_t m = 0x01010101u << pl, n = m << 4;
+                                mma16832(t_lo[rb], w[2 * rb][0] & m, w[2 * rb + 1][0] & m, w[2 * rb][1] & m, w[2 * rb + 1][1] & m, qb[pl][0], qb[pl][1]);
+                                mma16832(t_hi[rb], w[2 * rb][0] & n, w[2 * rb + 1][0] & n, w[2 * rb][1] & n, w[2 * rb + 1][1] & n, qb[4 + pl][0], qb[4 + pl][1]);
+                            }
+                    }
+#pragma unroll
+                    for (int j = 0; j < (PLANES ? 0 : 8); ++j) {
 #pragma unroll
                         for (int rb = 0; rb < 2; ++rb) {
                             uint32_t a0, a1, a2, a3;  // rows gl / gl + 8, coordinate pairs (4j, 4j+1) / (4j+2, 4j+3) of the lane's 32
@@ -1346,58 +1435,69 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 release_part(0);
                 TQ_STAMP(2);
 
-                // ---------------- online softmax: sv[blk][e] = score of token row (block blk, tau(gl)) and head 2*t4 + e.
+                // ---------------- online softmax: sv[blk][e] = score of token row (block blk, tau(gl)) and head t4 (PAIR), 2*t4 + e.
                 // Columns of heads >= grp carry zeros and are never read.
-                float sv[4][2];
+                float sv[4][NE];
 #pragma unroll
                 for (int blk = 0; blk < 4; ++blk) {
-                    sv[blk][0] = c[blk >> 1][2 * (blk & 1)] * kn4[blk];
-                    sv[blk][1] = c[blk >> 1][2 * (blk & 1) + 1] * kn4[blk];
+                    const int rb = blk >> 1, at = 2 * (blk & 1);
+                    if constexpr (PLANES) {
+                        const int t = t_lo[rb][at] * 4096 + t_lo[rb][at + 1] * 16 + t_hi[rb][at] * 256 + t_hi[rb][at + 1];  // (below 2^30)
+                        sv[blk][0] = fmaf((float)t, s_scale, s_zero) * kn4[blk];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < NE; ++e) sv[blk][e] = c[rb][at + e] * kn4[blk];
+                    }
                 }
                 if constexpr (!FULLT) {  // rows past the position may hold anything (even NaN norms): force them out
 #pragma unroll
                     for (int blk = 0; blk < 4; ++blk) {
                         const int tok = t0 + 8 * blk + (int)tauK;
-                        if (tok >= L) sv[blk][0] = sv[blk][1] = -1e30f;
+#pragma unroll
+                        for (int e = 0; e < NE; ++e)
+                            if (tok >= L) sv[blk][e] = -1e30f;
                     }
                 }
-                float mx0 = fmaxf(fmaxf(sv[0][0], sv[1][0]), fmaxf(sv[2][0], sv[3][0]));
-                float mx1 = fmaxf(fmaxf(sv[0][1], sv[1][1]), fmaxf(sv[2][1], sv[3][1]));
+                float mx[NE];
+                bool grown = false;
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    mx[e] = fmaxf(fmaxf(sv[0][e], sv[1][e]), fmaxf(sv[2][e], sv[3][e]));
+                    grown = grown || mx[e] > m_run[e];
+                }
                 // (the maximum over the row lanes is only looked for in the few tiles that hold a new one)
-                if (__any_sync(0xffffffffu, mx0 > m_run[0] || mx1 > m_run[1])) {
+                if (__any_sync(0xffffffffu, grown)) {
+                    float cf[NE];
 #pragma unroll
-                    for (int o = 4; o < 32; o <<= 1) {
-                        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-                        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+                    for (int e = 0; e < NE; ++e) {
+#pragma unroll
+                        for (int o = 4; o < 32; o <<= 1) mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], o));
+                        const float mn = fmaxf(m_run[e], mx[e]);
+                        cf[e] = ex2_approx(m_run[e] - mn);  // 1 when unchanged, 0 at the first tile; the lane's accumulators are of its own heads
+                        l_run[e] *= cf[e];
+                        m_run[e] = mn;
                     }
-                    const float mn0 = fmaxf(m_run[0], mx0), mn1 = fmaxf(m_run[1], mx1);
-                    // 1 when unchanged, 0 at the first tile; the accumulators of heads 2*t4, 2*t4 + 1 live in this very lane
-                    const float c0 = ex2_approx(m_run[0] - mn0), c1 = ex2_approx(m_run[1] - mn1);
-                    l_run[0] *= c0;
-                    l_run[1] *= c1;
 #pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        acc[b][0] *= c0; acc[b][2] *= c0;
-                        acc[b][1] *= c1; acc[b][3] *= c1;
-                    }
-                    m_run[0] = mn0;
-                    m_run[1] = mn1;
-                }
-                float pv[4][2];
+                    for (int b = 0; b < 8; ++b)
 #pragma unroll
-                for (int blk = 0; blk < 4; ++blk) {
-                    pv[blk][0] = ex2_approx(sv[blk][0] - m_run[0]);
-                    pv[blk][1] = ex2_approx(sv[blk][1] - m_run[1]);
+                        for (int e = 0; e < 4; ++e) acc[b][e] *= cf[PAIR ? 0 : e & 1];
                 }
+                float pv[4][NE];
+#pragma unroll
+                for (int blk = 0; blk < 4; ++blk)
+#pragma unroll
+                    for (int e = 0; e < NE; ++e) pv[blk][e] = ex2_approx(sv[blk][e] - m_run[e]);
                 if constexpr (!FULLT) {
 #pragma unroll
                     for (int blk = 0; blk < 4; ++blk) {
                         const int tok = t0 + 8 * blk + (int)tauK;
-                        if (tok >= L) pv[blk][0] = pv[blk][1] = 0.0f;
+#pragma unroll
+                        for (int e = 0; e < NE; ++e)
+                            if (tok >= L) pv[blk][e] = 0.0f;
                     }
                 }
-                l_run[0] += (pv[0][0] + pv[1][0]) + (pv[2][0] + pv[3][0]);
-                l_run[1] += (pv[0][1] + pv[1][1]) + (pv[2][1] + pv[3][1]);
+#pragma unroll
+                for (int e = 0; e < NE; ++e) l_run[e] += (pv[0][e] + pv[1][e]) + (pv[2][e] + pv[3][e]);
 
                 // ---------------- values: 2 blocks of 16 tokens ----------------
                 TQ_STAMP(3);
@@ -1408,14 +1508,26 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 // weights times V norms as fp16 pairs (heads 2*t4, 2*t4 + 1) of this lane's token rows, then transposed
                 // across the warp into the B operand of the value product: lane (gl, t4) receives head gl of the token
                 // rows tau(2*t4), tau(2*t4 + 1) of every 8-row block
+                // (PAIR: the pairs are one head's rows of two blocks; the even lanes gl get the first block's, the odd ones the second's)
                 uint32_t pb[4];
+                float vn[4];
 #pragma unroll
                 for (int blk = 0; blk < 4; ++blk) {
-                    float vn = ldsp_h2f(vns + ((uint32_t)(8 * blk) + tauK) * nstride);
+                    vn[blk] = ldsp_h2f(vns + ((uint32_t)(8 * blk) + tauK) * nstride);
                     if constexpr (!FULLT) {  // 0 * NaN would poison the accumulators
-                        if (t0 + 8 * blk + (int)tauK >= L) vn = 0.0f;
+                        if (t0 + 8 * blk + (int)tauK >= L) vn[blk] = 0.0f;
                     }
-                    pb[blk] = movmatrix_trans(pack_half2(pv[blk][0] * vn, pv[blk][1] * vn));
+                }
+                if constexpr (PAIR) {
+#pragma unroll
+                    for (int gam = 0; gam < 2; ++gam) {
+                        const uint32_t t = movmatrix_trans(pack_half2(pv[2 * gam][0] * vn[2 * gam], pv[2 * gam + 1][0] * vn[2 * gam + 1]));
+                        pb[2 * gam] = (gl & 1) ? 0u : t;
+                        pb[2 * gam + 1] = (gl & 1) ? t : 0u;
+                    }
+                } else {
+#pragma unroll
+                    for (int blk = 0; blk < 4; ++blk) pb[blk] = movmatrix_trans(pack_half2(pv[blk][0] * vn[blk], pv[blk][NE - 1] * vn[blk]));
                 }
 #pragma unroll
                 for (int gam = 0; gam < 2; ++gam) {
@@ -1497,35 +1609,26 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         const int slot = wid + g;
         float* const part_base = p.partials + (PERSIST ? (size_t)layer * (size_t)p.part_layer_stride : (size_t)0);
         if (!TQ_DBG(8)) {
-            float lsum0 = l_run[0], lsum1 = l_run[1];  // per lane over its own token rows: sum over the eight row lanes
+            float lsum[NE];  // per lane over its own token rows: sum over the eight row lanes
 #pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                lsum0 += __shfl_xor_sync(0xffffffffu, lsum0, o);
-                lsum1 += __shfl_xor_sync(0xffffffffu, lsum1, o);
-            }
-            if (gl == 0) {
+            for (int e = 0; e < NE; ++e) {
+                lsum[e] = l_run[e];
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int hq = 2 * t4 + e;
-                    if (hq < grp) {
-                        float* dst = part_base + ((size_t)slot * p.H + (size_t)head * grp + hq) * PART_STRIDE;
-                        dst[HEAD_DIM] = e ? m_run[1] : m_run[0];
-                        dst[HEAD_DIM + 1] = e ? lsum1 : lsum0;
-                    }
-                }
+                for (int o = 4; o < 32; o <<= 1) lsum[e] += __shfl_xor_sync(0xffffffffu, lsum[e], o);
             }
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int hq = 2 * t4 + e;
+            for (int e = 0; e < NE; ++e) {
+                const int hq = NE * t4 + e;
                 if (hq < grp) {
-                    float* dst = part_base + ((size_t)slot * p.H + (size_t)head * grp + hq) * PART_STRIDE + 16 * gl;
-#pragma unroll
-                    for (int b2 = 0; b2 < 4; ++b2) {
-                        float4 o;
-                        o.x = acc[2 * b2][e]; o.y = acc[2 * b2][2 + e];
-                        o.z = acc[2 * b2 + 1][e]; o.w = acc[2 * b2 + 1][2 + e];
-                        *reinterpret_cast<float4*>(dst + 4 * b2) = o;
+                    float* dst = part_base + ((size_t)slot * p.H + (size_t)head * grp + hq) * PART_STRIDE;
+                    if (gl == 0) {
+                        dst[HEAD_DIM] = m_run[e];
+                        dst[HEAD_DIM + 1] = lsum[e];
                     }
+                    auto sum = [&](int b, int row) { return PAIR ? acc[b][2 * row] + acc[b][2 * row + 1] : acc[b][2 * row + e]; };
+#pragma unroll
+                    for (int b2 = 0; b2 < 4; ++b2)
+                        *reinterpret_cast<float4*>(dst + 16 * gl + 4 * b2) = make_float4(sum(2 * b2, 0), sum(2 * b2, 1), sum(2 * b2 + 1, 0), sum(2 * b2 + 1, 1));
                 }
             }
         }

@@ -175,6 +175,13 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// D += A(16x32, row) * B(32x8, col): A unsigned bytes, B signed bytes, 32-bit sums.
+__device__ __forceinline__ void mma16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---- programmatic dependent launch: a kernel launched with the programmatic-serialisation attribute may start
 // while its predecessor in the stream is still running; everything that depends on the predecessor's writes (or
 // that overwrites something the predecessor still reads) comes after pdl_wait().  No-ops otherwise.
