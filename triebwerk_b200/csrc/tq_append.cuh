@@ -328,14 +328,15 @@ __global__ void __launch_bounds__(APPEND_THREADS) append_rotate_kernel(const App
 }
 
 // One head vector per CTA of 128 threads, for launches that fit the GPU in one wave: thread d owns output coordinate d and
-// row d of R, which goes from L2 straight into its registers (64 of them, every load in flight at once, under the input's
-// round trip) -- staging R in shared memory, as append_rotate_kernel does to reuse it, costs a small launch two more
-// barriers and a round trip.  The chain is the reference's; bound by latency (launch, one round trip, 128 dependent FMAs).
-constexpr int APPEND_VECTOR_MAX_PER_SM = 8;
+// row d of R.  All of R is in flight at once, under the input's round trip, in pieces that are next to each other for a warp,
+// and changes hands in shared memory (each thread loading its own row, 256 bytes from its neighbour's, kept the load unit busy
+// for a microsecond).  The chain is the reference's; bound by latency (launch, one round trip, 128 dependent FMAs).
+constexpr int APPEND_VECTOR_MAX_PER_SM = 6;  // (shared memory)
 template <int BITS>
 __global__ void __launch_bounds__(HEAD_DIM) append_vector_kernel(const AppendParams p) {
     __shared__ __align__(16) float xs[HEAD_DIM];
     __shared__ float warp_part[4];
+    __shared__ uint4 rs[HEAD_DIM * HEAD_DIM / 8];  // R, rows of 16 pieces
     const int d = threadIdx.x, lane = d & 31, wid = d >> 5;
     pdl_launch_dependents();
     pdl_wait();
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(HEAD_DIM) append_vector_kernel(const AppendPar
     const float val = __half2float((is_k ? p.k_buf : p.v_buf)[(size_t)src * p.kv_dim + (size_t)head * HEAD_DIM + d]);
     uint4 r[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = *(reinterpret_cast<const uint4*>(p.rotation + (size_t)d * HEAD_DIM) + i);
+    for (int i = 0; i < 16; ++i) r[i] = *(reinterpret_cast<const uint4*>(p.rotation) + d + HEAD_DIM * i);
     const int pos = p.positions ? p.positions[src] : (p.token_mode ? p.pos_value + src : p.pos_value);
     const int cap = p.seq_capacity && !p.token_mode ? p.seq_capacity[src] : p.capacity_rows;
     const bool ok = pos >= 0 && (cap <= 0 || pos < cap);
@@ -356,6 +357,11 @@ __global__ void __launch_bounds__(HEAD_DIM) append_vector_kernel(const AppendPar
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) sq = add_ftz(sq, __shfl_down_sync(0xffffffffu, sq, off));
     if (lane == 0) warp_part[wid] = sq;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {  // piece (row, k / 8), turned by the row: a warp's reads of 32 rows below are free of bank conflicts
+        const int row = (d >> 4) + 8 * i, k8 = d & 15;
+        rs[row * 16 + (k8 ^ (row & 7))] = r[i];
+    }
     __syncthreads();
     const float t = add_ftz(add_ftz(add_ftz(warp_part[0], warp_part[2]), add_ftz(warp_part[1], warp_part[3])), 1e-12f);
     xs[d] = mul_ftz(val, rsqrt_approx_ftz(t));
@@ -364,7 +370,8 @@ __global__ void __launch_bounds__(HEAD_DIM) append_vector_kernel(const AppendPar
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         const float4 x0 = *reinterpret_cast<const float4*>(&xs[8 * i]), x1 = *reinterpret_cast<const float4*>(&xs[8 * i + 4]);
-        const __half2* h2 = reinterpret_cast<const __half2*>(&r[i]);
+        const uint4 ri = rs[d * 16 + (i ^ (d & 7))];
+        const __half2* h2 = reinterpret_cast<const __half2*>(&ri);
         const float2 f0 = __half22float2(h2[0]), f1 = __half22float2(h2[1]), f2 = __half22float2(h2[2]), f3 = __half22float2(h2[3]);
         acc = fma_ftz(f0.x, x0.x, acc); acc = fma_ftz(f0.y, x0.y, acc); acc = fma_ftz(f1.x, x0.z, acc); acc = fma_ftz(f1.y, x0.w, acc);
         acc = fma_ftz(f2.x, x1.x, acc); acc = fma_ftz(f2.y, x1.y, acc); acc = fma_ftz(f3.x, x1.z, acc); acc = fma_ftz(f3.y, x1.w, acc);
