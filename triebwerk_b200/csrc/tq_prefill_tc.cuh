@@ -384,6 +384,16 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
     const uint2 div_hkv = fastdiv_make((uint32_t)p.Hkv), div_T = fastdiv_make((uint32_t)p.T),
                 div_G = fastdiv_make((uint32_t)(p.step_G > 0 ? p.step_G : 1));
 
+    // One thread per vector settles it (norm out, 1/norm, where its codes go): thread v < 128, or, in the TMA form, the
+    // lane that ends up holding the vector's sum of squares.
+    const int settle_v = TMA_IN ? (lane < 16 ? 64 * (lane >> 3) + 8 * warp + (lane & 7) : -1) : (tid < TC_TILE ? tid : -1);
+    // TMA form: a tile is TPT whole tokens.  Where they lie in one prompt at positions without an array of their own, the tile's
+    // first row says where all its vectors go; the token and head of a thread's vector within the tile never change.  (With the
+    // divisions and range checks of the general case once per tile and vector, a third of a CTA's time went into bookkeeping.)
+    const int TPT = TMA_IN ? TC_TILE / p.Hkv : 0;
+    const int dtok = TMA_IN && settle_v >= 0 ? settle_v / p.Hkv : 0, dhead = TMA_IN && settle_v >= 0 ? settle_v - dtok * p.Hkv : 0;
+    const bool plain_positions = TMA_IN && p.step_G == 0 && !p.positions;
+
     const int ev = (warp & 3) * 32 + lane;    // this thread's vector in the epilogue
     const int cc0 = (warp >> 2) * 2;          // its first block of 32 coordinates (warps 0-7)
 
@@ -484,7 +494,7 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         const __half* src_buf = kind == 0 ? p.k_buf : p.v_buf;
         uint8_t* cq = kind == 0 ? p.ck : p.cv;
         __half* cn = kind == 0 ? p.kn : p.vn;
-        const int tok0 = fastdiv(vec0, div_hkv), head0 = vec0 - tok0 * p.Hkv;
+        const int tok0 = TMA_IN ? (tile - (kind == 0 || !p.k_buf ? 0 : tiles_per_kind)) * TPT : fastdiv(vec0, div_hkv), head0 = TMA_IN ? 0 : vec0 - tok0 * p.Hkv;
         const int seq0 = fastdiv(tok0, div_T), t0 = tok0 - seq0 * p.T;
         auto split_vec = [&](int v, int& tok, int& head) {  // vector vec0 + v of the tile
             if (fast_head) {
@@ -525,13 +535,14 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
             for (int i = 0; i < 4; ++i) raw_all[pass][i] = live ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
         }
         }
-        // One thread per vector settles it (norm out, 1/norm, where its codes go): thread v < 128, or, in the TMA form, the
-        // lane that ends up holding the vector's sum of squares.  Its position and row base are loads of their own: issued
-        // here, needed only once the operands are with the tensor core.
-        const int settle_v = TMA_IN ? (lane < 16 ? 64 * (lane >> 3) + 8 * warp + (lane & 7) : -1) : (tid < TC_TILE ? tid : -1);
-        long long my_row_base = 0;
-        int my_pos = -1, my_head_layer = 0;  // position in the sequence (-1: the vector is not stored), head | layer << 16
-        if (settle_v >= 0 && vec0 + settle_v < vec_per_kind) {
+        // Where the vector that this thread settles goes: byte offset of its codes, index of its norm (-1: it is not stored)
+        long long my_dst = -1, my_norm = 0;
+        const int pos0 = p.pos_value + t0;
+        if (plain_positions && t0 + TPT <= p.T && seq0 < p.n_seq && pos0 >= 0 && (p.capacity_rows <= 0 || pos0 + TPT <= p.capacity_rows)) {
+            const long long row = (p.row_base ? p.row_base[seq0] : p.token_row0 + (long long)seq0 * p.seq_stride_rows) + pos0 + dtok;
+            my_norm = row * p.Hkv + dhead;
+            my_dst = my_norm * bpv;
+        } else if (settle_v >= 0 && vec0 + settle_v < vec_per_kind) {
             int tok, head, seq, t, layer = 0;
             split_vec(settle_v, tok, head);
             split_tok(tok, seq, t);
@@ -542,10 +553,13 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                 if (p.seq_capacity) cap = p.seq_capacity[sq];
             }
             const int pos = p.step_G > 0 ? p.positions[sq] : (p.positions ? p.positions[t] : p.pos_value + t);
-            my_row_base = p.row_base ? p.row_base[sq] : p.token_row0 + (long long)sq * p.seq_stride_rows;
-            my_head_layer = head | (layer << 16);
-            if (pos >= 0 && (cap <= 0 || pos < cap)) my_pos = pos;
-            else atomicMax(p.status, ST_BAD_POSITION);
+            const long long row = (p.row_base ? p.row_base[sq] : p.token_row0 + (long long)sq * p.seq_stride_rows) + pos;
+            if (pos >= 0 && (cap <= 0 || pos < cap)) {
+                my_norm = (long long)layer * p.norm_layer_stride + row * p.Hkv + head;
+                my_dst = (long long)layer * p.code_layer_stride + row * kvp + (long long)head * bpv;
+            } else {
+                atomicMax(p.status, ST_BAD_POSITION);
+            }
         }
         if constexpr (!TMA_IN) {
         {   // the CTA's next tile (same kind or the other one) on its way into L2 while this one is worked on
@@ -738,13 +752,7 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         }
         if (settle_v >= 0) {  // settle the vector: norm out, 1/norm, where its codes go
             const bool abnormal = !(my_tt < 3.0e38f);  // an infinity or a NaN among the inputs: every coordinate is a NaN
-            long long my_dst = -1;  // byte offset of the vector's codes in the cache
-            if (my_pos >= 0) {
-                const long long row = my_row_base + my_pos;
-                const int head = my_head_layer & 65535, layer = my_head_layer >> 16;
-                my_dst = (long long)layer * p.code_layer_stride + row * kvp + (long long)head * bpv;
-                cn[(long long)layer * p.norm_layer_stride + row * p.Hkv + head] = __float2half_rn(sqrt_approx_ftz(my_tt));
-            }
+            if (my_dst >= 0) cn[my_norm] = __float2half_rn(sqrt_approx_ftz(my_tt));
             dst_s[settle_v] = my_dst;
             // (an all-zero vector -- padding, say -- has every coordinate ON the bound 0: 128 exact chains, all with the result
             //  +0; it gets its constant codes directly instead.  The sum of squares of any other fp16 vector is at least 3.6e-15.)
