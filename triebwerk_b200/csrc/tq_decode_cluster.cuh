@@ -310,8 +310,22 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     };
 
+    // Host inputs take longer than all else: they are requested first, one 16-byte piece per thread, and everything else is done while
+    // they are on the bus.  (Many CTAs follow each other on an SM; only the first could have started under a previous kernel.  Behind the
+    // first rows and the barrier, 28 layers of 16 x 2019 tokens take 420 us instead of 397.)
+    const size_t new_at = ((size_t)g * p.Hkv + kvh) * HEAD_DIM;
+    uint4 in_w = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (HOST) {
+        pdl_wait();
+        pdl_launch_dependents();
+        const int r = tid >> 4;
+        const uint4* src = r < nh ? reinterpret_cast<const uint4*>(p.q + (size_t)g * p.q_dim + (size_t)head0 * HEAD_DIM) + tid
+                                  : reinterpret_cast<const uint4*>((r == nh ? p.new_k : p.new_v) + new_at) + (tid & 15);
+        in_w = ldg128_if(src, tid < (nh + (owner ? 2 : 0)) * 16);
+    }
     // ---- before the wait: positions and R on their way, table and bounds meanwhile, then the first tile ----
-    if (p.early) fetch_position();
+    const bool early = HOST || p.early != 0;
+    if (early) fetch_position();
     if (BITS != 0 && staged) fetch_rotation();
     const uint32_t bar = base + CdSmem::BAR_OFF;
     if (S > 1) {
@@ -380,32 +394,27 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             }
         }
     };
-    if (p.early) first_tile();
+    if (early) first_tile();
     if (staged) {
         __syncthreads();  // table, R: under the previous kernel's tail too
         after_table();
-        if (PRE && p.early && tile < tile_end) look_up_k();
+        if (PRE && early && tile < tile_end) look_up_k();
     }
-    pdl_wait();
-    pdl_launch_dependents();
-    if (!p.early) fetch_position();
-    if (!staged) fetch_rotation();
-    if (HOST && !p.early) first_tile();  // (the inputs take longer than the rows: they come over the bus)
+    if constexpr (!HOST) {
+        pdl_wait();
+        pdl_launch_dependents();
+        if (!early) fetch_position();
+        if (!staged) fetch_rotation();
+    }
 
     // ---- queries ----
     uint32_t qb[8][2];  // B fragments of the score product: lane (gl, t4) holds head gl, step j coordinates 32 t4 + 4 j ..
     uint32_t ql[EXACT && BITS != 0 ? 8 : 1][2];  // their low parts
     uint4 qw[4];
-    const size_t new_at = ((size_t)g * p.Hkv + kvh) * HEAD_DIM;
     const uint32_t in_s = warps_s;  // host inputs: [nh] queries, K, V, 256 bytes each, where the warps' results will be
     if constexpr (HOST) {
-        const uint4* const q_src = reinterpret_cast<const uint4*>(p.q + (size_t)g * p.q_dim + (size_t)head0 * HEAD_DIM);
-        for (int i = tid; i < (nh + (owner ? 2 : 0)) * 16; i += CD_THREADS) {
-            const int r = i >> 4;
-            const uint4* src = r < nh ? q_src + i : reinterpret_cast<const uint4*>((r == nh ? p.new_k : p.new_v) + new_at) + (i & 15);
-            const uint4 u = ldg128_if(src, true);
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(in_s + (uint32_t)i * 16u), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w) : "memory");
-        }
+        if (tid < (nh + (owner ? 2 : 0)) * 16)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(in_s + (uint32_t)tid * 16u), "r"(in_w.x), "r"(in_w.y), "r"(in_w.z), "r"(in_w.w) : "memory");
         __syncthreads();
     }
 #pragma unroll
@@ -423,21 +432,21 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         nw[m] = HOST ? lds128_if(in_s + (uint32_t)((nh + gl) * 256 + 16 * (4 * m + t4)), on)
                               : ldg128_if((gl == 0 ? p.new_k : p.new_v) + new_at + 8 * (4 * m + t4), on);
     }
-    uint2 q4 = make_uint2(0u, 0u);  // fp16 rows: head `warp`, coordinates 4 lane .., for the new token's score
+    uint2 q4 = make_uint2(0u, 0u);  // fp16 rows: coordinates 4 lane .. of the head whose score with the new token this warp takes
     __half xh = __ushort_as_half((unsigned short)0);
     if (owner) {
         if constexpr (HOST) {
             unsigned short u;
             asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(in_s + (uint32_t)((nh + vec) * 256 + 2 * d)));
             xh = __ushort_as_half(u);
-            if (BITS == 0 && warp < nh) q4 = lds64(in_s + (uint32_t)(warp * 256 + 8 * lane));
+            if (BITS == 0 && CD_WARPS - 1 - warp < nh) q4 = lds64(in_s + (uint32_t)((CD_WARPS - 1 - warp) * 256 + 8 * lane));
         } else {
             xh = ldg_half_if((vec == 0 ? p.new_k : p.new_v) + new_at + d, true);
-            if (BITS == 0) q4 = ldg64_if(p.q + (size_t)g * p.q_dim + (size_t)(head0 + warp) * HEAD_DIM + 4 * lane, warp < nh);
+            if (BITS == 0) q4 = ldg64_if(p.q + (size_t)g * p.q_dim + (size_t)(head0 + CD_WARPS - 1 - warp) * HEAD_DIM + 4 * lane, CD_WARPS - 1 - warp < nh);
         }
     }
     if (!staged) store_rotation();
-    if (!HOST && !p.early) first_tile();
+    if (!HOST && !early) first_tile();
     if (owner) {
         asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + CdSmem::RAW_OFF + 2u * (uint32_t)tid), "h"(__half_as_ushort(xh)) : "memory");
         if (!pos_ok && tid == 0 && p.status) atomicMax(p.status, ST_BAD_POSITION);
@@ -564,9 +573,43 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     auto centroid = [&](uint32_t code) { return lds_f32(base + CdSmem::CENT_OFF + 4u * code); };
     const bool takes_new = owner && appends;  // uniform for the CTA
 
+    // ---- the new token, in its owner: one of the last warps, which have the fewest tiles, takes its score with a query head (its weight in the CTA's result follows below) ----
+    const int new_h = CD_WARPS - 1 - warp;  // this warp's query head
+    if (takes_new && new_h < nh) {
+        float q[4], k[4];
+        auto halves = [&](uint2 u, float (&f)[4]) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+        };
+        float scale = 0.12751743074602467f;
+        if constexpr (BITS == 0) {
+            halves(q4, q);
+            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
+        } else {
+            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(new_h * MERGE_ROW + 4 * lane) * 2u;
+            halves(lds64(at), q);
+            if constexpr (EXACT) {
+                float ql4[4];
+                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
+            }
+            uint32_t w;
+            if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 2u * (uint32_t)lane));
+            else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + (uint32_t)lane));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) k[e] = centroid((w >> (BITS * e)) & ((1u << BITS) - 1u));
+            scale = lds_f32(base + CdSmem::NN_OFF);
+        }
+        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)new_h), "f"(dot * scale) : "memory");
+    }
+
     // ---- tiles ----
     const bool any_tile = tile < tile_end;
-    if (PRE && !(staged && p.early) && any_tile) look_up_k();
+    if (PRE && !(staged && early) && any_tile) look_up_k();
     float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};
     float acc[8][4];
 #pragma unroll
@@ -715,39 +758,6 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             load_v(next, lim);
             if (PRE) look_up_k();
         }
-    }
-
-    // ---- the new token, in its owner: warp h takes its score with query head h (its weight in the CTA's result follows below) ----
-    if (takes_new && warp < nh) {
-        float q[4], k[4];
-        auto halves = [&](uint2 u, float (&f)[4]) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
-        };
-        float scale = 0.12751743074602467f;
-        if constexpr (BITS == 0) {
-            halves(q4, q);
-            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
-        } else {
-            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(warp * MERGE_ROW + 4 * lane) * 2u;
-            halves(lds64(at), q);
-            if constexpr (EXACT) {
-                float ql4[4];
-                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
-            }
-            uint32_t w;
-            if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 2u * (uint32_t)lane));
-            else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + (uint32_t)lane));
-#pragma unroll
-            for (int e = 0; e < 4; ++e) k[e] = centroid((w >> (BITS * e)) & ((1u << BITS) - 1u));
-            scale = lds_f32(base + CdSmem::NN_OFF);
-        }
-        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)warp), "f"(dot * scale) : "memory");
     }
 
     // ---- the warps' results: acc[b]: coordinates 16 gl + 2 b (and + 1), heads 2 t4, 2 t4 + 1 ----

@@ -141,25 +141,42 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
     const int words = p.Hkv * 16;  // 8-code pieces per row
     const long long n = (long long)p.T * words;
     const int copy = threadIdx.x & 7;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * n; i += (long long)p.code_blocks * 256) {
-        const bool is_v = i >= n;
-        const long long w = is_v ? i - n : i;
-        const long long at = row0 * (p.row_heads * 16) + (p.row_heads == p.Hkv ? w : w / words * (p.row_heads * 16) + w % words);
-        const uint32_t c = BITS == 4 ? *(reinterpret_cast<const uint32_t*>(is_v ? p.cv : p.ck) + at)
-                                     : (uint32_t)*(reinterpret_cast<const unsigned short*>(is_v ? p.cv : p.ck) + at);
-        uint4* const dst = reinterpret_cast<uint4*>(is_v ? p.v16 : p.k16) + (long long)seq * n + w;
+    // (four pieces' loads in flight at a time, not four round trips one after the other)
+    constexpr int FLIGHT = 4;
+    const long long step = (long long)p.code_blocks * 256;
+    for (long long i0 = (long long)blockIdx.x * 256 + threadIdx.x; i0 < 2 * n; i0 += FLIGHT * step) {
+        uint32_t codes[FLIGHT];
 #pragma unroll
-        for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
-            const uint32_t* const lut = luts + part * ENTRIES * 8;
-            uint4 u;
-            if (BITS == 4) {
-                u.x = lut[(c & 0xffu) * 8 + copy]; u.y = lut[((c >> 8) & 0xffu) * 8 + copy];
-                u.z = lut[((c >> 16) & 0xffu) * 8 + copy]; u.w = lut[(c >> 24) * 8 + copy];
-            } else {
-                u.x = lut[(c & 0xfu) * 8 + copy]; u.y = lut[((c >> 4) & 0xfu) * 8 + copy];
-                u.z = lut[((c >> 8) & 0xfu) * 8 + copy]; u.w = lut[(c >> 12) * 8 + copy];
+        for (int f = 0; f < FLIGHT; ++f) {
+            const long long i = i0 + f * step;
+            const bool is_v = i >= n;
+            const long long w = is_v ? i - n : i;
+            const long long at = row0 * (p.row_heads * 16) + (p.row_heads == p.Hkv ? w : w / words * (p.row_heads * 16) + w % words);
+            codes[f] = 0u;
+            if (i < 2 * n)
+                codes[f] = BITS == 4 ? *(reinterpret_cast<const uint32_t*>(is_v ? p.cv : p.ck) + at)
+                                     : (uint32_t)*(reinterpret_cast<const unsigned short*>(is_v ? p.cv : p.ck) + at);
+        }
+#pragma unroll
+        for (int f = 0; f < FLIGHT; ++f) {
+            const long long i = i0 + f * step;
+            if (i >= 2 * n) break;
+            const bool is_v = i >= n;
+            const uint32_t c = codes[f];
+            uint4* const dst = reinterpret_cast<uint4*>(is_v ? p.v16 : p.k16) + (long long)seq * n + (is_v ? i - n : i);
+#pragma unroll
+            for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
+                const uint32_t* const lut = luts + part * ENTRIES * 8;
+                uint4 u;
+                if (BITS == 4) {
+                    u.x = lut[(c & 0xffu) * 8 + copy]; u.y = lut[((c >> 8) & 0xffu) * 8 + copy];
+                    u.z = lut[((c >> 16) & 0xffu) * 8 + copy]; u.w = lut[(c >> 24) * 8 + copy];
+                } else {
+                    u.x = lut[(c & 0xfu) * 8 + copy]; u.y = lut[((c >> 4) & 0xfu) * 8 + copy];
+                    u.z = lut[((c >> 8) & 0xfu) * 8 + copy]; u.w = lut[(c >> 12) * 8 + copy];
+                }
+                dst[part ? p.low / 8 : 0] = u;
             }
-            dst[part ? p.low / 8 : 0] = u;
         }
     }
 }
