@@ -30,10 +30,17 @@
 //     shared-memory table with one private column per lane (bank-conflict free); the table sits at shared
 //     address 0x10000 so that a single PRMT builds the lookup address from the packed word.
 //   * The dot products run on the tensor cores with warp-level mma.sync.m16n8k16 (fp16 in, fp32 accumulate):
-//     scores as Q(16 x 16) * K^T(16 x 8 tokens) with the query split into an fp16 high part (rows 0-7) and
-//     low part (rows 8-15) so that no query precision is lost, and the value sum in transposed form
-//     V^T(16 coords x 16 tokens) * P^T(16 tokens x 8 heads); the token pairs the V^T fragment needs are
-//     formed by interleaving the nibbles of two tokens' words BEFORE the table lookup.  Scalar fp32 FMAs cannot
+//     scores as K(16 tokens x 16 coordinates) * Q^T(16 x 8 columns), and the value sum in transposed form
+//     V^T(16 coords x 16 tokens) * P^T(16 tokens x 8 columns); the token pairs the V^T fragment needs are
+//     formed by interleaving the nibbles of two tokens' words BEFORE the table lookup.  With eight KV heads a head
+//     has two columns (PAIR): a lane's scores are of one head, half the exponentials, and 580 instead of 622 warp
+//     instructions per warp and 4-bit tile (28 layers of 64 x 4096 tokens 1902 -> 1874 us).
+//   * 2-bit scores need no table there (PLANES): a centroid is affine in its code's two bits, so every bit of the code bytes,
+//     masked in place, is an operand of mma.sync.m16n8k32 (u8 x s8) against 16-bit fixed-point queries; one mask per four
+//     codes and plane, as many products as before.  The table look-ups of K were 64 of a tile's 176 shared-memory wavefronts: that
+//     pipe 67 -> 39 % busy, 8 layers of 64 x 4096 tokens (32/8 heads) 456 -> 423 us in the whole-step form, 32 x 8192 one launch per
+//     layer 73.5 -> 69.7 us.  What is left is instruction issue (50 %) and fetch.  V keeps the table: its operand is the weights, whose
+//     range fixed point does not cover.  Scalar fp32 FMAs cannot
 //     keep up with HBM3e on this path: 512 FMAs per 132-byte row is more than the SMs can issue.
 //   * A worker that finishes its part of a sequence writes (acc[128], m, l) per query head to the workspace
 //     and takes a ticket; the last arrival merges all parts, and multiplies by R^T on the tensor cores

@@ -1992,7 +1992,7 @@ int tq_engine_decode_step_host(tq_engine* e, const void* q_host, const void* k_h
     // A small step straight on the host buffers, where the device can reach them (pinned memory): every CTA fetches its 0.5 to
     // 2.5 KB of inputs over the bus itself and writes its results there.  Copies cost 10 us of latency each, 40 us before the
     // first kernel can start, and the launches of the groups that overlap them 15 % of the GPU (28 layers, 16 sequences x 2019
-    // tokens, 16/8 heads: 521 / 415 us; 1 x 300 tokens 264 / 38).
+    // tokens, 16/8 heads: 521 / 394 us; 1 x 300 tokens 264 / 38).
     if (engine_step_small(e, StepInputs::Host)) {
         void* d[4] = {nullptr, nullptr, nullptr, nullptr};
         const void* h[4] = {q_host, k_host, v_host, out_host};
