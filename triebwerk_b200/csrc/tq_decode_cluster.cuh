@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     };
     if (early) first_tile();
-    if (staged) {
+    if (BITS != 0 && staged) {
         __syncthreads();  // table, R: under the previous kernel's tail too
         after_table();
         if (PRE && early && tile < tile_end) look_up_k();
@@ -427,8 +427,8 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     const int vec = tid >> 7, d = tid & 127;
     uint4 nw[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const bool on = BITS != 0 && owner && gl < 2;
+    for (int m = 0; m < (BITS != 0 ? 4 : 0); ++m) {
+        const bool on = owner && gl < 2;
         nw[m] = HOST ? lds128_if(in_s + (uint32_t)((nh + gl) * 256 + 16 * (4 * m + t4)), on)
                               : ldg128_if((gl == 0 ? p.new_k : p.new_v) + new_at + 8 * (4 * m + t4), on);
     }

@@ -354,20 +354,7 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         }
         grid_s[i] = amb >= 0 ? ((__float_as_uint(ambv) & ~15u) | (uint32_t)amb) : (0x7f000000u | (uint32_t)code);
     }
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = ctrl[2];
-    // (everything above is shared and tensor memory, and R where no kernel writes it: under the previous kernel's tail)
-    pdl_wait();
-    pdl_launch_dependents();
-    if (!p.static_rotation) {
-        stage_rotation();
-        fence_proxy_async_smem();
-        __syncthreads();
-    }
-
+    // (divisions and what else depends on the parameters alone: before the wait)
     const int vec_per_seq = p.T * p.Hkv;
     const int vec_per_kind = p.n_seq * vec_per_seq;
     const int tiles_per_kind = (vec_per_kind + TC_TILE - 1) / TC_TILE;
@@ -393,6 +380,20 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
     const int TPT = TMA_IN ? TC_TILE / p.Hkv : 0;
     const int dtok = TMA_IN && settle_v >= 0 ? settle_v / p.Hkv : 0, dhead = TMA_IN && settle_v >= 0 ? settle_v - dtok * p.Hkv : 0;
     const bool plain_positions = TMA_IN && p.step_G == 0 && !p.positions;
+
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = ctrl[2];
+    // (everything above is shared and tensor memory, and R where no kernel writes it: under the previous kernel's tail)
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!p.static_rotation) {
+        stage_rotation();
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
 
     const int ev = (warp & 3) * 32 + lane;    // this thread's vector in the epilogue
     const int cc0 = (warp >> 2) * 2;          // its first block of 32 coordinates (warps 0-7)
