@@ -315,6 +315,13 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     // first rows and the barrier, 28 layers of 16 x 2019 tokens take 420 us instead of 397.)
     const size_t new_at = ((size_t)g * p.Hkv + kvh) * HEAD_DIM;
     uint4 in_w = make_uint4(0u, 0u, 0u, 0u);
+    // (fp16 rows: one place where the first rows are requested, before or after the wait -- two places cost registers that
+    // the loop needs, and a spilled value read back there comes behind the loads of the next rows: 4 layers of 16 x 1000 tokens 57 us, now 53.6)
+    constexpr bool ROWS16 = BITS == 0 && !HOST;
+    if (ROWS16 && !p.early) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     if constexpr (HOST) {
         pdl_wait();
         pdl_launch_dependents();
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         in_w = ldg128_if(src, tid < (nh + (owner ? 2 : 0)) * 16);
     }
     // ---- before the wait: positions and R on their way, table and bounds meanwhile, then the first tile ----
-    const bool early = HOST || p.early != 0;
+    const bool early = HOST || ROWS16 || p.early != 0;
     if (early) fetch_position();
     if (BITS != 0 && staged) fetch_rotation();
     const uint32_t bar = base + CdSmem::BAR_OFF;
@@ -400,7 +407,11 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         after_table();
         if (PRE && early && tile < tile_end) look_up_k();
     }
-    if constexpr (!HOST) {
+    if (ROWS16 && p.early) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+    if constexpr (!HOST && !ROWS16) {
         pdl_wait();
         pdl_launch_dependents();
         if (!early) fetch_position();
@@ -446,7 +457,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     }
     if (!staged) store_rotation();
-    if (!HOST && !early) first_tile();
+    if (!HOST && !ROWS16 && !early) first_tile();
     if (owner) {
         asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + CdSmem::RAW_OFF + 2u * (uint32_t)tid), "h"(__half_as_ushort(xh)) : "memory");
         if (!pos_ok && tid == 0 && p.status) atomicMax(p.status, ST_BAD_POSITION);
@@ -575,7 +586,8 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
 
     // ---- the new token, in its owner: one of the last warps, which have the fewest tiles, takes its score with a query head (its weight in the CTA's result follows below) ----
     const int new_h = CD_WARPS - 1 - warp;  // this warp's query head
-    if (takes_new && new_h < nh) {
+    auto new_score = [&]() {
+        if (!takes_new || new_h >= nh) return;
         float q[4], k[4];
         auto halves = [&](uint2 u, float (&f)[4]) {
             const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
@@ -605,7 +617,8 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
         if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)new_h), "f"(dot * scale) : "memory");
-    }
+    };
+    if (BITS != 0) new_score();  // (fp16: after the tiles, whose first rows fill the registers here)
 
     // ---- tiles ----
     const bool any_tile = tile < tile_end;
@@ -650,9 +663,9 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                     a0 = (j & 1) ? lo.z : lo.x; a1 = (j & 1) ? hi.z : hi.x;
                     a2 = (j & 1) ? lo.w : lo.y; a3 = (j & 1) ? hi.w : hi.y;
                 }
-                mma16816(MB == 1 && !(EXACT && BITS != 0) && (j & 1) ? ce[b] : c[b], a0, a1, a2, a3, qb[j][0], qb[j][1]);
+                mma16816(MB == 1 && BITS != 0 && !EXACT && (j & 1) ? ce[b] : c[b], a0, a1, a2, a3, qb[j][0], qb[j][1]);
             }
-        if ((EXACT && BITS != 0) || MB == 1) {
+        if (BITS != 0 && (EXACT || MB == 1)) {
 #pragma unroll
             for (int b = 0; b < MB; ++b)
 #pragma unroll
@@ -760,6 +773,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     }
 
+    if (BITS == 0) new_score();
     // ---- the warps' results: acc[b]: coordinates 16 gl + 2 b (and + 1), heads 2 t4, 2 t4 + 1 ----
     if (any_tile) {
 #pragma unroll
