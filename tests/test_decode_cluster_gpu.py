@@ -118,6 +118,29 @@ def test_other_layouts_are_off_by_their_rounding_to_fp16_only(bits, H, Hkv, msl,
         assert err <= 1.03 * rounding, f"{name}: {err / rounding:.2f} times the rounding to fp16"
 
 
+# The host form's inputs lie where the warps' results go: clusters of 2 to 16 CTAs, with one and several tiles per warp, against the
+# same steps on device buffers, which have no such area
+@pytest.mark.parametrize("bits,H,Hkv,NL,G,msl,ctas", [
+    (0, 16, 8, 2, 4, 256, 2), (0, 32, 8, 2, 2, 512, 4), (0, 16, 8, 1, 2, 1024, 8), (0, 32, 4, 2, 2, 900, 8), (0, 8, 1, 1, 2, 4096, 16),
+    (0, 40, 8, 2, 2, 640, 4), (0, 12, 4, 1, 2, 1024, 8), (4, 16, 8, 2, 4, 256, 2), (2, 32, 8, 1, 2, 1024, 8)])
+def test_host_steps_are_those_of_device_buffers(bits, H, Hkv, NL, G, msl, ctas):
+    gen = torch.Generator(device="cuda").manual_seed(11 + msl)
+    eng = tq.Engine(msl, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(G, msl)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert tq.lib().tq_engine_decode_form(eng._h, 1) == ctas
+    k, v = (torch.randn(G, msl - 1, Hkv * D, generator=gen, device="cuda").half() for _ in range(2))
+    for layer in range(NL):
+        eng.prefill_append_batch(layer, 0, k, v)
+    eng.set_positions([msl - 1 - 17 * g for g in range(G)])
+    for _ in range(20):
+        q, k, v = (torch.randn(NL, G, d, generator=gen, device="cuda").half() for d in (H * D, Hkv * D, Hkv * D))
+        want = eng.decode_step(q, k, v, torch.empty_like(q))
+        got = eng.decode_step_host(*(t.cpu().pin_memory() for t in (q, k, v)), torch.empty(q.shape, dtype=torch.float16, pin_memory=True)).cuda()
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert eng.status() == 0
+
+
 @pytest.mark.parametrize("bits", [4, 2])
 @pytest.mark.parametrize("G,Hkv", [(1, 1), (3, 8), (148, 8)])
 def test_one_vector_append_vs_oracle(bits, G, Hkv):

@@ -469,7 +469,9 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::WP_OFF + 4u * (uint32_t)warp), "f"(sq) : "memory");
         }
     }
-    if (owner || !staged) __syncthreads();  // warp sums, raw token; a rotation that was not staged before the wait, and the table
+    // warp sums, raw token; a rotation that was not staged before the wait, and the table; host inputs, which lie where the warps' results
+    // will be: in the packed modes the rotation's barrier stands between their last reads and the first result, with fp16 rows only this one
+    if (owner || !staged || (HOST && BITS == 0)) __syncthreads();
     if (!staged) after_table();
     if constexpr (BITS != 0) {
         // rotated queries, rot[h][n] = sum_k q[h][k] R[n][k]: warp w takes the coordinate blocks w and w + 8
