@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             load_v(tile, lim);
         }
     };
-    const bool staged = BITS == 0 || p.static_rotation != 0;  // R may be read before the wait
+    const bool staged = BITS == 0 || HOST || p.static_rotation != 0;  // R may be read now (HOST waits for the previous kernel before all else)
     uint4 ru[8];
     auto fetch_rotation = [&]() {
 #pragma unroll
