@@ -34,6 +34,8 @@
 // 1 layer of 4 x 612 tokens 6.9 us, now 5.9; 28 layers of 1 x 1500 187 us, now 163 with fewer CTAs (4-bit, 16/8 heads).
 #pragma once
 
+#include <type_traits>
+
 #include "tq_attention.cuh"
 
 namespace tq {
@@ -125,6 +127,19 @@ __device__ __forceinline__ __half ldg_half_if(const __half* src, bool on) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u16 %0, 0;\n\t@p ld.global.u16 %0, [%1];\n\t}"
                  : "=&h"(r) : "l"(src), "r"((uint32_t)on));
     return __ushort_as_half(r);
+}
+
+// A warp's partial result, or that of a warp without tiles: maximum, sum, one or four coordinates.
+__device__ __forceinline__ void part_if(uint32_t ml, uint32_t acc, bool on, float& m, float& l, float (&a)[4]) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %8, 0;\n\tmov.f32 %0, 0fF149F2CA;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\t"
+                 "mov.f32 %3, 0f00000000;\n\tmov.f32 %4, 0f00000000;\n\tmov.f32 %5, 0f00000000;\n\t"
+                 "@p ld.shared.v2.f32 {%0, %1}, [%6];\n\t@p ld.shared.v4.f32 {%2, %3, %4, %5}, [%7];\n\t}"
+                 : "=&f"(m), "=&f"(l), "=&f"(a[0]), "=&f"(a[1]), "=&f"(a[2]), "=&f"(a[3]) : "r"(ml), "r"(acc), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void part_if(uint32_t ml, uint32_t acc, bool on, float& m, float& l, float (&a)[1]) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.f32 %0, 0fF149F2CA;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\t"
+                 "@p ld.shared.v2.f32 {%0, %1}, [%3];\n\t@p ld.shared.f32 %2, [%4];\n\t}"
+                 : "=&f"(m), "=&f"(l), "=&f"(a[0]) : "r"(ml), "r"(acc), "r"((uint32_t)on));
 }
 
 // Shared memory of a CTA below the table, from the dynamic base: the small arrays and, when they fit, the warps' partial
@@ -583,44 +598,15 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     }
 
     auto lds_f32 = [&](uint32_t a) { float f; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(a)); return f; };
-    auto centroid = [&](uint32_t code) { return lds_f32(base + CdSmem::CENT_OFF + 4u * code); };
-    const bool takes_new = owner && appends;  // uniform for the CTA
-
-    // ---- the new token, in its owner: one of the last warps, which have the fewest tiles, takes its score with a query head (its weight in the CTA's result follows below) ----
-    const int new_h = CD_WARPS - 1 - warp;  // this warp's query head
-    auto new_score = [&]() {
-        if (!takes_new || new_h >= nh) return;
-        float q[4], k[4];
-        auto halves = [&](uint2 u, float (&f)[4]) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
-        };
-        float scale = 0.12751743074602467f;
-        if constexpr (BITS == 0) {
-            halves(q4, q);
-            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
-        } else {
-            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(new_h * MERGE_ROW + 4 * lane) * 2u;
-            halves(lds64(at), q);
-            if constexpr (EXACT) {
-                float ql4[4];
-                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
-            }
-            uint32_t w;
-            if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 2u * (uint32_t)lane));
-            else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + (uint32_t)lane));
-#pragma unroll
-            for (int e = 0; e < 4; ++e) k[e] = centroid((w >> (BITS * e)) & ((1u << BITS) - 1u));
-            scale = lds_f32(base + CdSmem::NN_OFF);
-        }
-        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)new_h), "f"(dot * scale) : "memory");
+    auto new_codes = [&](int v, int k) -> uint32_t {  // the new token's K (0) or V (1): codes of the coordinates k .. k + 3
+        const uint32_t at = base + CdSmem::NEW_OFF + 128u * (uint32_t)v + (uint32_t)(k * BITS >> 3);
+        uint32_t w;
+        if (BITS == 4) asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(w) : "r"(at));
+        else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(at));
+        return w;
     };
-    if (BITS != 0) new_score();  // (fp16: after the tiles, whose first rows fill the registers here)
+    auto centroid = [&](uint32_t w, int e) { return lds_f32(base + CdSmem::CENT_OFF + 4u * ((w >> (BITS * e)) & ((1u << BITS) - 1u))); };
+    const bool takes_new = owner && appends;  // uniform for the CTA
 
     // ---- tiles ----
     const bool any_tile = tile < tile_end;
@@ -775,7 +761,6 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         }
     }
 
-    if (BITS == 0) new_score();
     // ---- the warps' results: acc[b]: coordinates 16 gl + 2 b (and + 1), heads 2 t4, 2 t4 + 1 ----
     if (any_tile) {
 #pragma unroll
@@ -797,6 +782,38 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             }
         }
     }
+    // ---- the new token, in its owner: one of the last warps, which have the fewest tiles, takes its score with a query head (its weight
+    // in the CTA's result follows below).  (In front of the tiles it held up the launches of many CTAs.) ----
+    const int new_h = CD_WARPS - 1 - warp;  // this warp's query head
+    if (takes_new && new_h < nh) {
+        float q[4], k[4];
+        auto halves = [&](uint2 u, float (&f)[4]) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+        };
+        float scale = 0.12751743074602467f;
+        if constexpr (BITS == 0) {
+            halves(q4, q);
+            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
+        } else {
+            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(new_h * MERGE_ROW + 4 * lane) * 2u;
+            halves(lds64(at), q);
+            if constexpr (EXACT) {
+                float ql4[4];
+                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
+            }
+            const uint32_t w = new_codes(0, 4 * lane);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) k[e] = centroid(w, e);
+            scale = lds_f32(base + CdSmem::NN_OFF);
+        }
+        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)new_h), "f"(dot * scale) : "memory");
+    }
     __syncthreads();
     // ---- the CTA's result, normalised: maximum and sum beside it ----
     // where coordinate n of head h goes in the CTA that adds up its share: [this CTA][head][coordinate of the share]
@@ -807,57 +824,86 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                        map_shared(bar, r));
     };
     if (S > 1) cluster_wait();  // every CTA of the cluster has started
-    for (int i = tid; i < nh * HEAD_DIM; i += CD_THREADS) {  // (a warp stays within one head)
-        const int h = i >> 7, k = i & 127;
+    // The warps' results are added up by a warp per head, a lane per four coordinates: maxima and exponentials once for four (a lane per
+    // coordinate costs steps of many short sequences with 8 heads 5 %).  Clusters with up to two heads, whose launches wait for their
+    // longest chain, take a lane per coordinate, four warps per head.
+    auto sum_up = [&](auto c_) {
+        constexpr int C = decltype(c_)::value;
+        const int h = C == 1 ? warp >> 2 : warp, k = C == 1 ? tid & (HEAD_DIM - 1) : C * lane;
+        if (h >= nh) return;
         const uint32_t src = warps_s + (uint32_t)(h * PART_STRIDE) * 4u, wstride = (uint32_t)(nh * PART_STRIDE) * 4u;
-        float mw[CD_WARPS], lw[CD_WARPS], aw[CD_WARPS], M = -1e30f, m_new = -1e30f, v_new = 0.0f;
-        if (takes_new) {
-            m_new = lds_f32(base + CdSmem::NS_OFF + 4u * (uint32_t)h);
-            if constexpr (BITS == 0) {
-                unsigned short u;
-                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(base + CdSmem::RAW_OFF + 256u + 2u * (uint32_t)k));
-                v_new = __half2float(__ushort_as_half(u));
-            } else {
-                uint32_t w;
-                asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w) : "r"(base + CdSmem::NEW_OFF + 128u + (uint32_t)(k * BITS >> 3)));
-                v_new = lds_f32(base + CdSmem::NN_OFF + 4u) * centroid((w >> (k * BITS & 7)) & ((1u << BITS) - 1u));
-            }
-            M = fmaxf(M, m_new);
-        }
+        float mw[CD_WARPS], lw[CD_WARPS], aw[CD_WARPS][C], vn[C], M = -1e30f, m_new = -1e30f;
 #pragma unroll
         for (int w = 0; w < CD_WARPS; ++w) {
-            mw[w] = -1e30f;
-            lw[w] = aw[w] = 0.0f;
-            if (w < n_act) {  // uniform for the CTA
-                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(mw[w]), "=f"(lw[w]) : "r"(src + (uint32_t)w * wstride + HEAD_DIM * 4u));
-                aw[w] = lds_f32(src + (uint32_t)w * wstride + (uint32_t)k * 4u);
+            const uint32_t at = src + (uint32_t)w * wstride;
+            part_if(at + HEAD_DIM * 4u, at + (uint32_t)k * 4u, w < n_act, mw[w], lw[w], aw[w]);
+        }
+#pragma unroll
+        for (int i = 0; i < C; ++i) vn[i] = 0.0f;
+        if (takes_new) {
+            if constexpr (BITS == 0) {
+                const uint2 u = lds64(base + CdSmem::RAW_OFF + 256u + 2u * (uint32_t)(k & ~3));
+                const float2 v0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), v1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+                const float v[4] = {v0.x, v0.y, v1.x, v1.y};
+                if constexpr (C == 4) { vn[0] = v[0]; vn[1] = v[1]; vn[2] = v[2]; vn[3] = v[3]; }
+                else vn[0] = (k & 2) ? ((k & 1) ? v[3] : v[2]) : ((k & 1) ? v[1] : v[0]);
+            } else {
+                const uint32_t w = new_codes(1, k & ~3);
+                const float n = lds_f32(base + CdSmem::NN_OFF + 4u);
+#pragma unroll
+                for (int i = 0; i < C; ++i) vn[i] = n * centroid(w, C == 1 ? k & 3 : i);
             }
+            m_new = lds_f32(base + CdSmem::NS_OFF + 4u * (uint32_t)h);
+            M = fmaxf(M, m_new);
         }
 #pragma unroll
         for (int w = 0; w < CD_WARPS; ++w) M = fmaxf(M, mw[w]);
         const float e_new = takes_new ? ex2_approx(m_new - M) : 0.0f;
-        float a = takes_new ? e_new * v_new : 0.0f, z = e_new;
+        float a[C], z = e_new;
+#pragma unroll
+        for (int i = 0; i < C; ++i) a[i] = takes_new ? e_new * vn[i] : 0.0f;
 #pragma unroll
         for (int w = 0; w < CD_WARPS; ++w) {
             const float e = ex2_approx(mw[w] - M);  // (a warp without tiles: times zero)
-            a = fmaf(e, aw[w], a);
+#pragma unroll
+            for (int i = 0; i < C; ++i) a[i] = fmaf(e, aw[w][i], a[i]);
             z = fmaf(e, lw[w], z);
         }
-        // one CTA: the reference's denominator; several: the part's own sum (none: no token), the rest follows below
-        a = S == 1 ? a / (z + 1e-8f) : (z > 0.0f || z != z ? a * rcp_approx_ftz(z) : 0.0f);
-        if (S > 1 && k < (int)S)
-            st_async_f32x2(map_shared(base + CdSmem::MZ_OFF + (uint32_t)((int)rank * nh + h) * 8u, (uint32_t)k), M, z, map_shared(bar, (uint32_t)k));
+        // one CTA: the reference's denominator; several: the part's own sum (none: no token), the rest follows below (there, and here for
+        // several, 1 and 2 units of fp32 off a correctly rounded quotient: those cost 1 to 3 % of a small layer)
+#pragma unroll
+        for (int i = 0; i < C; ++i) a[i] = S == 1 ? a[i] / (z + 1e-8f) : (z > 0.0f || z != z ? a[i] * rcp_approx_ftz(z) : 0.0f);
+        const int r = C == 1 ? k : lane;
+        if (S > 1 && r < (int)S)
+            st_async_f32x2(map_shared(base + CdSmem::MZ_OFF + (uint32_t)((int)rank * nh + h) * 8u, (uint32_t)r), M, z, map_shared(bar, (uint32_t)r));
         if constexpr (BITS == 0) {
-            const float a1 = __shfl_down_sync(0xffffffffu, a, 1);
-            if (S == 1) p.out[(size_t)g * p.q_dim + (size_t)(head0 + h) * HEAD_DIM + k] = __float2half_rn(a);
-            else if ((k & 1) == 0) send(h, k, a, a1);
+            __half* const o = p.out + (size_t)g * p.q_dim + (size_t)(head0 + h) * HEAD_DIM + k;
+            if constexpr (C == 1) {
+                const float a1 = __shfl_down_sync(0xffffffffu, a[0], 1);
+                if (S == 1) *o = __float2half_rn(a[0]);
+                else if ((k & 1) == 0) send(h, k, a[0], a1);
+            } else if (S == 1) {
+                reinterpret_cast<__half2*>(o)[0] = __floats2half2_rn(a[0], a[1]);
+                reinterpret_cast<__half2*>(o)[1] = __floats2half2_rn(a[2], a[3]);
+            } else {
+                send(h, k, a[0], a[1]);
+                send(h, k + 2, a[2], a[3]);
+            }
         } else {
-            const __half ahi = __float2half_rn(a);
-            const uint32_t o = (uint32_t)(h * MERGE_ROW + k) * 2u;
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + CdSmem::Q_OFF + o), "h"(__half_as_ushort(ahi)) : "memory");
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + CdSmem::LO_OFF + o), "h"(__half_as_ushort(__float2half_rn(a - __half2float(ahi)))) : "memory");
+            const uint32_t o = base + CdSmem::Q_OFF + (uint32_t)(h * MERGE_ROW + k) * 2u;
+            constexpr uint32_t low = CdSmem::LO_OFF - CdSmem::Q_OFF;
+            if constexpr (C == 1) {
+                const __half ahi = __float2half_rn(a[0]);
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(o), "h"(__half_as_ushort(ahi)) : "memory");
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(o + low), "h"(__half_as_ushort(__float2half_rn(a[0] - __half2float(ahi)))) : "memory");
+            } else {
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(o), "r"(pack_half2(a[0], a[1])), "r"(pack_half2(a[2], a[3])) : "memory");
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(o + low), "r"(pack_low_half2(a[0], a[1])), "r"(pack_low_half2(a[2], a[3])) : "memory");
+            }
         }
-    }
+    };
+    if (nh <= 2) sum_up(std::integral_constant<int, 1>());
+    else sum_up(std::integral_constant<int, 4>());
     if constexpr (BITS != 0) {
         __syncthreads();
         // times R: o[h][n] = sum_k a[h][k] R[k][n], two blocks of 8 output coordinates per warp.  The high parts are rows 0-7 of the A
