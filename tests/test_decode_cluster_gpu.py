@@ -122,7 +122,10 @@ def test_other_layouts_are_off_by_their_rounding_to_fp16_only(bits, H, Hkv, msl,
 # same steps on device buffers, which have no such area
 @pytest.mark.parametrize("bits,H,Hkv,NL,G,msl,ctas", [
     (0, 16, 8, 2, 4, 256, 2), (0, 32, 8, 2, 2, 512, 4), (0, 16, 8, 1, 2, 1024, 8), (0, 32, 4, 2, 2, 900, 8), (0, 8, 1, 1, 2, 4096, 16),
-    (0, 40, 8, 2, 2, 640, 4), (0, 12, 4, 1, 2, 1024, 8), (4, 16, 8, 2, 4, 256, 2), (2, 32, 8, 1, 2, 1024, 8)])
+    (0, 40, 8, 2, 2, 640, 4), (0, 12, 4, 1, 2, 1024, 8), (4, 16, 8, 2, 4, 256, 2), (2, 32, 8, 1, 2, 1024, 8),
+    # one CTA each: results leave through shared memory, one to eight heads of a KV head, three clusters to a KV head
+    (0, 16, 8, 4, 12, 256, 1), (0, 8, 8, 4, 12, 256, 1), (0, 32, 4, 8, 12, 256, 1), (4, 16, 8, 4, 12, 256, 1), (2, 32, 4, 8, 12, 256, 1), (4, 40, 8, 4, 12, 256, 1),
+    (2, 20, 1, 16, 12, 256, 1)])
 def test_host_steps_are_those_of_device_buffers(bits, H, Hkv, NL, G, msl, ctas):
     gen = torch.Generator(device="cuda").manual_seed(11 + msl)
     eng = tq.Engine(msl, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)

@@ -823,6 +823,10 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
         st_async_f32x2(map_shared(base + CdSmem::CP_OFF + ((((rank * (uint32_t)nh + (uint32_t)h) << share_log) + ((uint32_t)n & ((1u << share_log) - 1u))) << 2), r), v0, v1,
                        map_shared(bar, r));
     };
+    // Host results of a single CTA meet in shared memory and leave in whole lines: the bus takes a write in the pieces it arrives in.  As
+    // the products leave them, 16 bytes at a time, those were what L2 happened to put together: a step of many short sequences took up to
+    // 1.7 times as long for a change of the instructions in front of them (28 layers, 2-bit 32/4 heads 16 x 300 tokens 140 or 230 us, now 137).
+    auto stage_out = [&](int at, uint32_t two) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + CdSmem::CP_OFF + 2u * (uint32_t)at), "r"(two) : "memory"); };
     if (S > 1) cluster_wait();  // every CTA of the cluster has started
     // The warps' results are added up by a warp per head, a lane per four coordinates: maxima and exponentials once for four (a lane per
     // coordinate costs steps of many short sequences with 8 heads 5 %).  Clusters with up to two heads, whose launches wait for their
@@ -882,6 +886,9 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                 const float a1 = __shfl_down_sync(0xffffffffu, a[0], 1);
                 if (S == 1) *o = __float2half_rn(a[0]);
                 else if ((k & 1) == 0) send(h, k, a[0], a1);
+            } else if (HOST && S == 1) {
+                stage_out(h * HEAD_DIM + k, pack_half2(a[0], a[1]));
+                stage_out(h * HEAD_DIM + k + 2, pack_half2(a[2], a[3]));
             } else if (S == 1) {
                 reinterpret_cast<__half2*>(o)[0] = __floats2half2_rn(a[0], a[1]);
                 reinterpret_cast<__half2*>(o)[1] = __floats2half2_rn(a[2], a[3]);
@@ -938,13 +945,19 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
                 const float o0 = (oc[i][0][0] + oc[i][1][0]) + (oc[i][0][2] + oc[i][1][2]), o1 = (oc[i][0][1] + oc[i][1][1]) + (oc[i][0][3] + oc[i][1][3]);
                 if (S == 1) {
                     const size_t at = (size_t)(head0 + gl) * HEAD_DIM + 8 * nb + 2 * t4;
-                    *reinterpret_cast<__half2*>(p.out + (size_t)g * p.q_dim + at) = __floats2half2_rn(o0, o1);
+                    if (HOST) stage_out(gl * HEAD_DIM + 8 * nb + 2 * t4, pack_half2(o0, o1));
+                    else *reinterpret_cast<__half2*>(p.out + (size_t)g * p.q_dim + at) = __floats2half2_rn(o0, o1);
                     if (p.out_f32) *reinterpret_cast<float2*>(p.out_f32 + (size_t)g * p.H * HEAD_DIM + at) = make_float2(o0, o1);
                 } else {
                     send(gl, 8 * nb + 2 * t4, o0, o1);
                 }
             }
         }
+    }
+    if (HOST && S == 1 && (BITS != 0 || nh > 2)) {
+        __syncthreads();
+        uint32_t* const o = reinterpret_cast<uint32_t*>(p.out + (size_t)g * p.q_dim + (size_t)head0 * HEAD_DIM);
+        for (int i = tid; i < nh * (HEAD_DIM / 2); i += CD_THREADS) o[i] = lds32(base + CdSmem::CP_OFF + 4u * (uint32_t)i);
     }
     if (S > 1) {
         if (!mbar_wait_bounded_hint(bar, 0u, 1u << 14, 20000u) && p.status) atomicMax(p.status, ST_TMA_WAIT_TIMEOUT);
