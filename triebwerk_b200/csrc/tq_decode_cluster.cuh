@@ -5,8 +5,8 @@
 // round trips, a 16-row append on one worker, per-sequence tickets and a merge through global memory.  Here the work is
 // cut so that the longest dependent chain is short:
 //   * a cluster of S CTAs (1 to 16, chosen by the host) owns one sequence and one KV head with up to 8 of its query heads
-//     (more query heads: further clusters).  Its 8 * S warps take the sequence's 32-token tiles in turn, first all CTAs'
-//     warp 0, then warp 1 ..., with plain 16- and 8-byte loads that land in registers in fragment order: no shared-memory
+//     (more query heads: further clusters).  Its 8 * S warps (8 * (S - 1) where a CTA is the new token's alone, see below) take the
+//     sequence's tiles of 32 tokens, or of 16 where that leaves each warp one, in turn, first all CTAs' warp 0, then warp 1 ..., with plain 16- and 8-byte loads that land in registers in fragment order: no shared-memory
 //     ring, no table of tiles, any head layout, ragged slots and shared prefixes by row arithmetic alone.
 //   * codes become fp16 through a shared-memory table with a private column per lane (one entry per code byte at 4-bit,
 //     per nibble at 2-bit); table and R are staged before griddepcontrol.wait, i.e. under the previous kernel's tail, and
