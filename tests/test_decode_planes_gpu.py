@@ -55,6 +55,41 @@ def test_streaming_decode_of_eight_kv_heads(bits, H):
             hp.assert_attention_close(o.reshape(G, H * D), ref, H, D, f"{name} {bits} bits, {H} heads, layer {layer}")
 
 
+# 2-bit queries as fixed point: one rotated coordinate far above the others, at each of a byte's four places, among ordinary ones; and
+# beyond fp16, as which the whole-step form holds them: NaN, whatever the codes (bits of 0 and 1 that an infinity leaves in the planes)
+def test_queries_with_one_large_coordinate():
+    rng = np.random.default_rng(77)
+    G, H, msl, NL = 144, 16, 96, 2
+    R = ops.rotation_matrix().numpy()
+    eng = tq.Engine(msl, 2, num_layers=NL, num_heads=H, num_kv_heads=HKV, head_dim=D)
+    eng.alloc_batch(G, msl)
+    eng.reset()
+    assert tq.lib().tq_engine_decode_form(eng._h, 0) == 0 and tq.lib().tq_engine_decode_form(eng._h, 1) == 0
+    k, v = (rng.standard_normal((NL, G, msl, HKV * D), dtype=np.float32).astype(np.float16) for _ in range(2))
+    for layer in range(NL):
+        eng.prefill_append_batch(layer, 0, gu.dev(k[layer][:, :msl - 1]), gu.dev(v[layer][:, :msl - 1]))
+    lengths = np.array([(96, 40, 1, 2)[g // 36] for g in range(G)])
+    pos = (lengths - 1).astype(np.int32)
+    eng.set_positions(pos)
+    Rf, at = R.astype(np.float32), np.arange(G)
+    q = rng.standard_normal((NL, G, H, D), dtype=np.float32)
+    q[:, :72] += 8 * Rf[at[:72] % D][:, None]
+    q[:, 72:] = 65504 * np.where(Rf[at[72:] % D] < 0, -1, 1)[:, None]   # rotated and scaled 7e4 and more
+    q = q.astype(np.float16).reshape(NL, G, H * D)
+    dq, dk, dv = gu.dev(q), gu.dev(k[:, at, pos]), gu.dev(v[:, at, pos])
+    layers = gu.host(torch.stack([eng.decode_layer(i, dq[i], dk[i], dv[i]) for i in range(NL)]))
+    step = gu.host(eng.decode_step(dq, dk, dv, torch.empty_like(dq)))
+    assert eng.status() == 0
+    beyond = np.abs((q[0, :, :D].astype(np.float32) @ Rf.T) * 0.12751743).max(1) > 65520
+    assert not beyond[:72].any() and beyond[72:].sum() >= 36
+    for layer in range(NL):
+        ck, cv, kn, vn = (gu.host(t) for t in eng.layer_cache(layer))
+        ref, _ = tqo.attention_batch(q[layer], ck, cv, kn, vn, R, pos, msl, H, HKV, D, 2)
+        hp.assert_attention_close(layers[layer, :108], ref[:108], H, D, "layers")  # (one token, or ordinary scores)
+        hp.assert_attention_close(step[layer, :72], ref[:72], H, D, "step")
+        assert np.isnan(step[layer, beyond]).all()
+
+
 # a slot that 8 CTAs serve with more than one block per warp; the launchers' clusters of one and two CTAs, one per SM
 @pytest.mark.parametrize("bits,H,msl,lengths,ctas", [(4, 16, 1536, [1500], 8), (2, 32, 2032, [2032], 8), (2, 32, 1024, [1023] * 8, 2), (4, 16, 512, [300, 512] * 8, 1)])
 def test_cluster_sizes_and_the_launchers(bits, H, msl, lengths, ctas):

@@ -1070,7 +1070,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         // column the low ones.  Code 2 b1 + b0 stands for -c3 + (c3 - c2) b0 + (c3 + c2) b1, c2 and c3 the positive centroids.  Bit b of
         // a byte's coordinate j is worth 2^(2 j + b) where it stands: the query of that plane is divided by it (by 2^(2 (j mod 2) + b): the
         // coordinates 0, 1 and 2, 3 have sums of their own, 16 apart).  The sum's offset is minus half the sum with all bits set.
-        // Rounding: 4e-5 of the largest coordinate at most, 1.3e-4 of a typical one where fp16 has 2e-4.
+        // Rounding: half a weight (1 and 4, 2 and 8) of the 32639 C_b / C0 steps to the largest coordinate: 1.5e-5 to 6.6e-5 of it at most.
+        // Queries with an infinity (rotated and scaled they do not fit fp16, in the whole-step form) give NaN.
         auto make_planes = [&](const float (&x)[32]) {
             constexpr float C0 = 0.13351f - 0.04003f, C1 = 0.13351f + 0.04003f;
             uint32_t top = 0u;  // of the magnitudes' bits: an infinity or a NaN comes out on top
@@ -1081,7 +1082,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             const float mx = __uint_as_float(top);
             const bool some = mx > 1e-30f;
             const float k = some ? 32639.0f / (mx * C0) : 0.0f;
-            const float scale = some ? mx * (C0 / (16.0f * 32639.0f)) : (mx == mx ? 0.0f : mx);
+            const float scale = top >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : some ? mx * (C0 / (16.0f * 32639.0f)) : 0.0f;
             const uint32_t bias = (gl & 1) ? 0u : 128u, sel = (gl & 1) ? 0x0040u : 0x0051u;
             const float magic = 12582912.0f + (float)bias;  // 1.5 * 2^23: the sum's low bits are the rounded integer
             uint32_t all = 0u;
