@@ -145,9 +145,9 @@ def test_host_steps_are_those_of_device_buffers(bits, H, Hkv, NL, G, msl, ctas):
 
 
 @pytest.mark.parametrize("bits", [4, 2])
-@pytest.mark.parametrize("G,Hkv", [(1, 1), (3, 8), (148, 8)])
+@pytest.mark.parametrize("G,Hkv", [(1, 1), (3, 8), (111, 8), (112, 8), (148, 8)])
 def test_one_vector_append_vs_oracle(bits, G, Hkv):
-    """148 x 8 vectors: the last launch of one CTA per vector on a 148-SM GPU."""
+    """111 x 8 vectors: the last launch of one CTA per vector on a 148-SM GPU (six per SM); 112 x 8 and 148 x 8 share R in groups."""
     rng = np.random.default_rng(2000 + bits + G)
     R = ops.rotation_matrix().numpy()
     x = rng.standard_normal((G, Hkv * D), dtype=np.float32).astype(np.float16)

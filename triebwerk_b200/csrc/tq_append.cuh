@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(APPEND_THREADS) append_rotate_kernel(const App
 // row d of R.  All of R is in flight at once, under the input's round trip, in pieces that are next to each other for a warp,
 // and changes hands in shared memory (each thread loading its own row, 256 bytes from its neighbour's, kept the load unit busy
 // for a microsecond).  The chain is the reference's; bound by latency (launch, one round trip, 128 dependent FMAs).
-constexpr int APPEND_VECTOR_MAX_PER_SM = 6;  // (shared memory)
+constexpr int APPEND_VECTOR_MAX_PER_SM = 6;  // (as many as shared memory holds; 888 vectors 5.4 us, 896 to 1088 through append_rotate_kernel 8.2)
 template <int BITS>
 __global__ void __launch_bounds__(HEAD_DIM) append_vector_kernel(const AppendParams p) {
     __shared__ __align__(16) float xs[HEAD_DIM];
