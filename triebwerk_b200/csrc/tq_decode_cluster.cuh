@@ -608,6 +608,44 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
     auto centroid = [&](uint32_t w, int e) { return lds_f32(base + CdSmem::CENT_OFF + 4u * ((w >> (BITS * e)) & ((1u << BITS) - 1u))); };
     const bool takes_new = owner && appends;  // uniform for the CTA
 
+    // ---- the new token, in its owner: one of the last warps, which have the fewest tiles, takes its score with a query head (its weight
+    // in the CTA's result follows below).  Behind the tiles: in front of them it holds up launches of many CTAs (28 layers of 32 x 128 tokens,
+    // 2-bit 32/8 heads, 178 us, behind them 168).  Not in EXACT's packed modes, whose one CTA per SM has longer tiles, which the compiler
+    // orders better without it behind them (4-bit 40/8 heads 21 x 5198 tokens, 4 layers, 158 us, in front of them 153). ----
+    const int new_h = CD_WARPS - 1 - warp;  // this warp's query head
+    auto new_score = [&]() {
+        if (!takes_new || new_h >= nh) return;
+        float q[4], k[4];
+        auto halves = [&](uint2 u, float (&f)[4]) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+        };
+        float scale = 0.12751743074602467f;
+        if constexpr (BITS == 0) {
+            halves(q4, q);
+            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
+        } else {
+            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(new_h * MERGE_ROW + 4 * lane) * 2u;
+            halves(lds64(at), q);
+            if constexpr (EXACT) {
+                float ql4[4];
+                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
+            }
+            const uint32_t w = new_codes(0, 4 * lane);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) k[e] = centroid(w, e);
+            scale = lds_f32(base + CdSmem::NN_OFF);
+        }
+        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)new_h), "f"(dot * scale) : "memory");
+    };
+    constexpr bool SCORE_FIRST = EXACT && BITS != 0;
+    if (SCORE_FIRST) new_score();
+
     // ---- tiles ----
     const bool any_tile = tile < tile_end;
     if (PRE && !(staged && early) && any_tile) look_up_k();
@@ -782,38 +820,7 @@ __global__ void __launch_bounds__(CD_THREADS, EXACT && BITS != 0 ? 1 : 2) cluste
             }
         }
     }
-    // ---- the new token, in its owner: one of the last warps, which have the fewest tiles, takes its score with a query head (its weight
-    // in the CTA's result follows below).  (In front of the tiles it held up the launches of many CTAs.) ----
-    const int new_h = CD_WARPS - 1 - warp;  // this warp's query head
-    if (takes_new && new_h < nh) {
-        float q[4], k[4];
-        auto halves = [&](uint2 u, float (&f)[4]) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
-        };
-        float scale = 0.12751743074602467f;
-        if constexpr (BITS == 0) {
-            halves(q4, q);
-            halves(lds64(base + CdSmem::RAW_OFF + 8u * (uint32_t)lane), k);
-        } else {
-            const uint32_t at = base + CdSmem::Q_OFF + (uint32_t)(new_h * MERGE_ROW + 4 * lane) * 2u;
-            halves(lds64(at), q);
-            if constexpr (EXACT) {
-                float ql4[4];
-                halves(lds64(at + (CdSmem::LO_OFF - CdSmem::Q_OFF)), ql4);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) q[e] += ql4[e];
-            }
-            const uint32_t w = new_codes(0, 4 * lane);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) k[e] = centroid(w, e);
-            scale = lds_f32(base + CdSmem::NN_OFF);
-        }
-        float dot = fmaf(q[0], k[0], q[1] * k[1]) + fmaf(q[2], k[2], q[3] * k[3]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + CdSmem::NS_OFF + 4u * (uint32_t)new_h), "f"(dot * scale) : "memory");
-    }
+    if (!SCORE_FIRST) new_score();
     __syncthreads();
     // ---- the CTA's result, normalised: maximum and sum beside it ----
     // where coordinate n of head h goes in the CTA that adds up its share: [this CTA][head][coordinate of the share]
