@@ -38,8 +38,8 @@
 //   * 2-bit scores need no table there (PLANES): a centroid is affine in its code's two bits, so every bit of the code bytes,
 //     masked in place, is an operand of mma.sync.m16n8k32 (u8 x s8) against 16-bit fixed-point queries; one mask per four
 //     codes and plane, as many products as before.  The table look-ups of K were 64 of a tile's 176 shared-memory wavefronts: that
-//     pipe 67 -> 39 % busy, 8 layers of 64 x 4096 tokens (32/8 heads) 456 -> 423 us in the whole-step form, 32 x 8192 one launch per
-//     layer 73.5 -> 69.7 us.  What is left is instruction issue (50 %) and fetch.  V keeps the table: its operand is the weights, whose
+//     pipe 67 -> 49 % busy, 550 -> 484 warp instructions, 8 layers of 64 x 4096 tokens (32/8 heads) 456 -> 423 us in the whole-step form, 32 x 8192 one launch per
+//     layer 73.5 -> 69.7 us.  What is left is instruction issue (65 %) and the ALU (56 %).  V keeps the table: its operand is the weights, whose
 //     range fixed point does not cover.  Scalar fp32 FMAs cannot
 //     keep up with HBM3e on this path: 512 FMAs per 132-byte row is more than the SMs can issue.
 //   * A worker that finishes its part of a sequence writes (acc[128], m, l) per query head to the workspace

@@ -31,7 +31,8 @@
 // Bound by latency: one round trip for the inputs, the rotation, one tile, three CTA barriers, one trip across the cluster, about
 // 700 + 800 + 1500 + 600 + 900 + 900 + 1500 cycles.  With the token as a row of the last tile (its CTA 1600 cycles behind the others),
 // divisions by the cluster's size in the exchange, the low parts' products with R of their own and the look-ups behind the queries:
-// 1 layer of 4 x 612 tokens 6.9 us, now 5.9; 28 layers of 1 x 1500 187 us, now 163 with fewer CTAs (4-bit, 16/8 heads).
+// 1 layer of 4 x 612 tokens 7.0 us, now 5.9; 28 layers of 1 x 1500 188 us, now 157 with fewer CTAs (4-bit, 16/8 heads, one call after
+// the other, caches from HBM; 8 layers, which stay in L2, 5.3 us each).
 #pragma once
 
 #include <type_traits>

@@ -425,7 +425,8 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
 // the SM's L1 and issue slots, and the CTAs of the next launch find no room for their prologue (8 sequences x 1023 tokens through
 // the launchers 24 us a layer with two, 19 with one).  16 only where 8 leave a warp two blocks and more: seven of the GPU's
 // processing clusters hold one cluster of 16 beside the previous launch's, an eighth waits (1 sequence, 8 KV heads, 4-bit: 600 tokens 5.2 us
-// with 8 and 7.9 with 16, 1500 tokens 5.5 / 6.2, 3000 tokens 7.4 / 6.8; fp16 1500 5.3 / 5.6, 3000 11.0 / 7.9).  Clusters of 4 and more leave some of a processing cluster's SMs over (136
+// with 8 and 7.9 with 16, 1500 tokens 5.5 / 6.2, 3000 tokens 7.4 / 6.8; fp16 1500 5.3 / 5.6, 3000 11.0 / 7.9; layers
+// that stay in L2.  1 and 2 sequences of 1100 to 2019 tokens, all modes and layouts, 1.0 to 1.25 times as fast as with 16, EXACT up to 2.)  Clusters of 4 and more leave some of a processing cluster's SMs over (136
 // of 148 serve fours, 128 eights): one cluster more than fits waits for a whole turn (72 clusters of 4 at two CTAs per SM 1.5
 // times the time of 72 of 2).  Where a warp goes through many tiles, more than the launch's fixed part costs, a second CTA per SM
 // hides the latency of the first one's loads: above 12 tiles 0.6 to 0.95 of the time (4 x 8192 tokens, 8 KV heads, 44 -> 28 us),
