@@ -88,31 +88,21 @@ struct AttnParams {
     int pos_value;
     int max_seq_len;
     int G, H, Hkv, q_dim;
-    // fused form (one launch per layer and step: append the new token, rotate the queries, attend)
-    const __half* new_k;       // [G][kv_dim] this step's keys, values and queries
-    const __half* new_v;
-    const __half* new_q;       // [G][q_dim]
-    const __half* rotation;    // R row-major (B operand of the query rotation); rot_copies copies back to back
-    int rot_copies;            // every worker reads copy (worker % rot_copies): 300 workers fetching the same 32 KB at once queue up in L2
-    int kv_dim;
-    int capacity_rows;         // rows a sequence may use (position check)
-    const int* seq_capacity;   // optional [G]: rows sequence g may use (ragged slots), instead of capacity_rows
-    int app_weight;            // cost of one append in tiles, for the balance of the work list
-    int early;                 // 1: positions and this layer's cache tiles may be read before the previous kernel in the
-                               // stream has finished (the caller knows it writes neither): table, slice and first copies
-                               // then run under that kernel's tail
+    // layer form (MODE 1): after layer_prep_kernel (tq_layer_prep.cuh), whose predecessors have finished when this kernel starts:
+    // positions and cache rows are read before that launch has, but for the tiles it writes the new tokens to
+    int appends;               // 1: layer_prep_kernel appends, to the last tile of every sequence
+    const float* q_rot32;      // rotated queries as fp32 [G][H][128] instead of q_rot16 (2-bit with eight KV heads, up to 16 heads)
     int l2_ahead;              // tiles prefetched into L2 beyond the shared-memory ring
     // whole-step form (MODE 2): ONE launch streams the layers [layer0, layer0 + n_layers) back to back -- every worker
-    // walks its slice of the tile list once per layer, its ring of stages never drains in between -- rotates the
-    // queries itself and only PUBLISHES its split-K partials, per layer; merge_partials_kernel finishes the step.
+    // walks its slice of the tile list once per layer, its ring of stages never drains in between -- and only PUBLISHES its
+    // split-K partials, per layer; merge_partials_kernel finishes the step.
     // ck/cv/kn/vn are the arrays of layer0, the tensor maps have the layer as their outermost coordinate.
     int layer0, n_layers;
     long long norm_layer_stride;   // halves between consecutive layers' norm arrays
-    long long q_layer_stride;      // halves between consecutive layers' queries (and outputs)
     long long part_layer_stride;   // floats between consecutive layers' partial areas
     int* table_out;                // [G + 4]: the tile table, then {workers taking part, total tiles}, for the merge kernel
-    const __half* q_rot16;         // whole-step form: pre-rotated, pre-scaled fp16 queries of layer0, [layers][G][H][128]
-                                   // (rotate_queries_kernel); a sequence's block reaches shared memory by one bulk copy
+    const __half* q_rot16;         // layer and whole-step form: pre-rotated, pre-scaled fp16 queries of layer0, [layers][G][H][128]
+                                   // (layer_prep_kernel, rotate_queries_kernel); a sequence's block reaches shared memory by one bulk copy
 #ifdef TQ_TIMING_SWITCHES
     int debug;                 // timing-experiment builds only: bit 0 = skip the math, bit 1 = skip the loads, ... (results are then wrong)
     unsigned long long* stamps;  // timing-experiment builds only: [8] summed clock deltas of the tile loop's sections
@@ -144,12 +134,10 @@ struct RegionA {
     static constexpr uint32_t MERGE_OFF = 512;   // per group: hi + lo [16][MERGE_ROW] halves
     static constexpr uint32_t MERGE_GROUP_BYTES = 2 * 16 * MERGE_ROW * 2;  // 8704
     static constexpr uint32_t BLOCKS_OFF = MERGE_OFF + ATTN_GROUPS * MERGE_GROUP_BYTES;
-    // fused form only: tile table of the launch, then per group the append's codes, partial sums and destinations
+    // layer and whole-step form: tile table of the launch
     static constexpr uint32_t FUSED_SCAN_OFF = BLOCKS_OFF;           // 32 ints of scan scratch
     static constexpr uint32_t FUSED_TS_OFF = FUSED_SCAN_OFF + 128;   // tile_start[G + 1], G <= FUSED_MAX_G
-    static constexpr uint32_t FUSED_APP_OFF = FUSED_TS_OFF + 4096;
-    static constexpr uint32_t FUSED_APP_GROUP_BYTES = 16 * 128 + 16 * 4 * 4 + 128;  // codes [16][128], 1/norm [16], spare
-    static constexpr uint32_t FUSED_BLOCKS_OFF = FUSED_APP_OFF + ATTN_GROUPS * FUSED_APP_GROUP_BYTES;
+    static constexpr uint32_t FUSED_BLOCKS_OFF = FUSED_TS_OFF + 4096;
 };
 constexpr int FUSED_MAX_G = 1023;
 
@@ -206,6 +194,12 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
     return d;
 }
+// Sixteen bytes from global memory, requested where they stand (a later griddepcontrol.wait does not pull the load behind it).
+__device__ __forceinline__ uint4 ldg128_now(const void* src) {
+    uint4 r;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(src));
+    return r;
+}
 __device__ __forceinline__ float ldsp_h2f(uint32_t addr) {  // one fp16 from shared memory as float
     unsigned short h;
     asm("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(addr));
@@ -222,7 +216,7 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
                                                int head, int lane, int bar_group, int nthreads, OutRow out_row,
                                                OutRowF32 out_row_f32, int hb_begin, int hb_end, bool rotated_out = false) {
     const int gl = lane >> 2, t4 = lane & 3;
-    constexpr int RH = NW >= 16 ? 1 : 2, FLIGHT = 16 / RH;  // heads per warp at a time, parts whose loads are in flight together
+    constexpr int RH = 2, FLIGHT = 16 / RH;  // heads per warp at a time, parts whose loads are in flight together
     for (int hb = hb_begin; hb < hb_end; hb += 16) {
         // ---- phase A: heads hb .. hb+15, two heads per warp at a time with all their loads in flight
         //      together: combine the parts, normalise, split into fp16 high + low, store as the A operand
@@ -382,23 +376,23 @@ __device__ __forceinline__ void merge_sequence(const float* part0, int parts, in
     }
 }
 
-// MODE 0: queries pre-rotated and tile table built by append_rotate_kernel; 1: the kernel builds its table, rotates the
-// queries, optionally appends the step's token (one launch per layer and step); 2: whole-step form, see AttnParams; 3: as 1,
-// but the partials are only published (merge_partials_kernel<16> follows); 4: as 2 without the copy warps.
-// The whole-step form has two warps more, which issue the copies of one worker each.  With 16 warps at work it is a warpgroup more:
+// MODE 0: queries pre-rotated and tile table built by append_rotate_kernel, merge in the kernel.  In the other modes the kernel builds
+// its table and publishes its partials, the queries are rotated and the new tokens appended already: 1: one layer, after
+// layer_prep_kernel, merge_layer_kernel follows; 2: whole-step form, see AttnParams; 4: as 2 without the copy warps.
+// Modes 1 and 2 have two warps more, which issue the copies of one worker each.  With 16 warps at work it is a warpgroup more:
 // the launch brings 640 x 96 registers, of which the workers' warps take 112 each and the copy warps keep 32.
 template <int HKV, int MODE>
-constexpr int attn_threads() { return ATTN_GROUPS * 32 * HKV + (MODE == 2 ? (HKV == 8 ? 128 : 64) : 0); }
+constexpr int attn_threads() { return ATTN_GROUPS * 32 * HKV + (MODE == 1 || MODE == 2 ? (HKV == 8 ? 128 : 64) : 0); }
 constexpr int ATTN_REGS_WORK = 112, ATTN_REGS_COPY = 32;
 template <int BITS, int HKV, int MODE>
 __global__ void __launch_bounds__(attn_threads<HKV, MODE>(), 1)
 decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const AttnParams p) {
     using Geo = AttnGeom<BITS>;
-    constexpr bool FUSED = MODE >= 1;
+    constexpr bool LAYER = MODE == 1;
     constexpr bool PERSIST = MODE == 2 || MODE == 4;
-    constexpr bool COPIER = MODE == 2;
-    constexpr bool SEPARATE = MODE == 3;
+    constexpr bool PUBLISH = LAYER || PERSIST;
+    constexpr bool COPIER = MODE == 1 || MODE == 2;
     // Eight KV heads have at most four query heads each (ATTN_MAX_HEADS), half of a product's eight columns.  Head h takes the columns
     // 2 h and 2 h + 1: a lane's two score columns are ONE head, so that it has half the exponentials; in the value product the even
     // column sums the first eight tokens of a step, the odd one the other eight.
@@ -413,7 +407,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     const int lane = tid & 31;
     const int warp = tid >> 5;
     constexpr int Hkv = HKV;  // compile time: row pitches, tile sizes and norm strides fold into immediates
-    // whole-step form: lane 0 of each worker's copy warp keeps its ring filled
+    // lane 0 of each worker's copy warp keeps its ring filled
     const bool copier = COPIER && warp >= ATTN_GROUPS * Hkv;
     const int group = copier ? ((warp - ATTN_GROUPS * Hkv) & 1) : warp / Hkv;  // worker within the CTA
     const int head = warp - group * Hkv; // KV head of this warp
@@ -431,7 +425,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     // ---- shared memory map (absolute shared addresses) ----
     const uint32_t dyn_base = smem_u32(dyn_smem);
     const uint32_t a_base = (dyn_base + 1023u) & ~1023u;
-    const uint32_t blocks_a = (a_base + (FUSED ? RegionA::FUSED_BLOCKS_OFF : RegionA::BLOCKS_OFF) + 1023u) & ~1023u;
+    const uint32_t blocks_a = (a_base + (PUBLISH ? RegionA::FUSED_BLOCKS_OFF : RegionA::BLOCKS_OFF) + 1023u) & ~1023u;
     const uint32_t n_a = blocks_a < LUT_ABS ? (LUT_ABS - blocks_a) / stage_bytes : 0u;
     const uint32_t dyn_end = dyn_base + (uint32_t)ATTN_DYN_SMEM;
     const uint32_t n_b = dyn_end > REGION_B_ABS ? (dyn_end - REGION_B_ABS) / stage_bytes : 0u;
@@ -453,32 +447,32 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     // and handed back separately, so that a stage's K half is on its way again while its V half is still being read
     const uint32_t bar0 = a_base + RegionA::BAR_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 16u);
     const uint32_t cnt0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 8u);
-    const uint32_t ebar0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 16u);  // whole-step form: "part handed back" barriers
+    const uint32_t ebar0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 16u);  // copy warps: "part handed back" barriers
     const uint32_t ctrl_s = a_base + RegionA::CTRL_OFF + (uint32_t)group * 16u;
     const uint32_t merge_s = a_base + RegionA::MERGE_OFF + (uint32_t)group * RegionA::MERGE_GROUP_BYTES;
 
-    // The fused form lets its successor start only once it has itself seen its predecessor finish (see `early`).
-    if (!FUSED) pdl_launch_dependents();
+    // (modes with a table of their own let their successor start only once they have themselves seen their predecessor finish)
+    if (!PUBLISH) pdl_launch_dependents();
     if (TQ_DBG(32)) { pdl_wait(); pdl_launch_dependents(); return; }
     const int G = p.G;
 
     // ---- byte -> centroid table, one column per lane ----
     if (TQ_DBG(16)) {
     } else if (BITS == 4) {
-        for (int idx = tid; idx < 256 * 32; idx += blockDim.x) {
-            int v = idx >> 5, l = idx & 31;
+        for (int idx = tid; idx < 256 * 8; idx += blockDim.x) {  // four lanes' columns at a time
+            int v = idx >> 3, l = idx & 7;
             uint32_t val = pack_half2(kCent4[v & 15], kCent4[v >> 4]);
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(LUT_ABS + (uint32_t)v * 256u + (uint32_t)l * 4u), "r"(val) : "memory");
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(LUT_ABS + (uint32_t)v * 256u + (uint32_t)l * 16u), "r"(val) : "memory");
         }
     } else {
-        for (int idx = tid; idx < 256 * 32; idx += blockDim.x) {
-            int v = idx >> 5, l = idx & 31;
+        for (int idx = tid; idx < 256 * 16; idx += blockDim.x) {  // two lanes' columns at a time
+            int v = idx >> 4, l = idx & 15;
             // (c0, c2), (c1, c3): the low and the high nibble each give one value to either word.  For K a byte is four
             // coordinates of one token (the query fragments are packed in the same order); for V a byte is put together
             // from the nibbles of two tokens, and either word is then one coordinate of that token pair.
             uint32_t lo2 = pack_half2(kCent2[v & 3], kCent2[(v >> 4) & 3]);
             uint32_t hi2 = pack_half2(kCent2[(v >> 2) & 3], kCent2[(v >> 6) & 3]);
-            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(LUT_ABS + (uint32_t)v * 256u + (uint32_t)l * 8u),
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %1, %2};" ::"r"(LUT_ABS + (uint32_t)v * 256u + (uint32_t)l * 16u),
                          "r"(lo2), "r"(hi2) : "memory");
         }
     }
@@ -488,20 +482,19 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             if (COPIER) mbar_init(ebar0 + 8u * s, Hkv);
             else asm volatile("st.shared.u32 [%0], %1;" ::"r"(cnt0 + 4u * s), "r"(0u) : "memory");
         }
-        if (PERSIST) mbar_init(a_base + 320u + 8u * (uint32_t)group, 1);
+        if (PUBLISH) mbar_init(a_base + 320u + 8u * (uint32_t)group, 1);
         fence_mbar_init();
         fence_proxy_async_smem();
     }
     // Everything above touches only shared memory and may overlap the tail of the previous kernel in the stream.
-    const bool early = FUSED && p.early != 0;
-    if (!early) {
+    if (!LAYER) {
         pdl_wait();
-        if (FUSED) pdl_launch_dependents();
+        if (PUBLISH) pdl_launch_dependents();
     }
-    // Tile table.  The fused form builds it here, in shared memory, from the positions (every CTA the same table);
-    // the plain form reads the one the append kernel left in the workspace.
+    // Tile table.  Built here, in shared memory, from the positions (every CTA the same table); the plain form reads the one the
+    // append kernel left in the workspace.
     const int* ts;
-    if constexpr (FUSED) {
+    if constexpr (PUBLISH) {
         int* ts_s = reinterpret_cast<int*>(dyn_smem + (a_base - dyn_base) + RegionA::FUSED_TS_OFF);
         int* scan_s = reinterpret_cast<int*>(dyn_smem + (a_base - dyn_base) + RegionA::FUSED_SCAN_OFF);
         int carry = 0;
@@ -533,7 +526,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         }
         if (tid == 0) ts_s[G] = carry;
         ts = ts_s;
-        if constexpr (PERSIST) {  // (never early)
+        if constexpr (PERSIST) {
             if (blockIdx.x == 0) {  // the merge kernel reads the table from global memory
                 __syncthreads();
                 for (int i = tid; i <= G; i += (int)blockDim.x) p.table_out[i] = ts_s[i];
@@ -556,53 +549,25 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         p.table_out[G + 2] = (int)N;
     }
     if (wid >= W && !copier) return;  // uniform for the worker; no CTA-wide barrier follows
-    // The flat list is cut in UNITS: a tile is one unit, except the last tile of a sequence, which counts 1 + A units
-    // for what a sequence costs beside its tiles (A = p.app_weight, in tiles): in the fused form its owner also appends
-    // the sequence's new token; in the prefill form sequences are short and their partials and merges weigh as much
-    // as their tiles.  Sequence g starts at unit ts[g] + g*A; a tile belongs to the worker its first unit falls to.
-    const long long A = (long long)p.app_weight;
-    const long long U = N + (long long)G * A;
-    long long lo, hi;
-    int g;
-    if (FUSED || A > 0) {
-        auto tiles_before = [&](long long x, int* gfirst) -> long long {  // tiles whose first unit is below unit x
-            if (x >= U) { *gfirst = G; return N; }
-            int a = 0, b = G;  // invariant: unit start of a <= x < unit start of b
-            while (b - a > 1) {
-                const int mid = (a + b) >> 1;
-                if ((long long)ts[mid] + mid * A <= x) a = mid; else b = mid;
-            }
-            const long long off = x - ((long long)ts[a] + a * A), n = ts[a + 1] - ts[a];
-            *gfirst = off >= n ? a + 1 : a;
-            return ts[a] + (off < n ? off : n);
-        };
-        int g_hi;
-        lo = tiles_before((long long)wid * U / W, &g);
-        hi = tiles_before((long long)(wid + 1) * U / W, &g_hi);
-        if (lo >= hi && !copier) return;  // the worker's units all lie inside an append's share: nothing to do
+    // Worker w takes the tiles [w * N / W, (w + 1) * N / W).
+    const long long lo = (long long)wid * N / W, hi = (long long)(wid + 1) * N / W;
+    int g;  // first sequence of the slice: largest g with tile_start[g] <= lo
+    if (!PUBLISH && p.worker_g && !TQ_DBG_FACTOR) {
+        g = p.worker_g[wid];
     } else {
-        lo = (long long)wid * N / W;
-        hi = (long long)(wid + 1) * N / W;
-        // first sequence of the slice: largest g with tile_start[g] <= lo
-        if (p.worker_g && !TQ_DBG_FACTOR) {
-            g = p.worker_g[wid];
-        } else {
-            int a = 0, b = G;  // invariant: tile_start[a] <= lo < tile_start[b]
-            while (b - a > 1) {
-                int mid = (a + b) >> 1;
-                if ((long long)ts[mid] <= lo) a = mid; else b = mid;
-            }
-            g = a;
+        int a = 0, b = G;  // invariant: tile_start[a] <= lo < tile_start[b]
+        while (b - a > 1) {
+            int mid = (a + b) >> 1;
+            if ((long long)ts[mid] <= lo) a = mid; else b = mid;
         }
+        g = a;
     }
 
-    if (copier && (lane > 0 || wid >= W || lo >= hi)) {  // nothing to copy (it returns further down)
-        g = 0;
-        lo = hi = 0;
-    }
+    const bool idle = copier && (lane > 0 || wid >= W);  // nothing to copy (it returns further down)
+    if (idle) g = 0;
     // ---- load cursor over the flat tile list (warp-uniform, advanced in step by every warp of the worker) ----
     // Tile counts and row numbers fit 32 bits (the host refuses caches of 2^31 rows or more).
-    const int lo_i = (int)lo, hi_i = (int)hi;
+    const int lo_i = idle ? 0 : (int)lo, hi_i = idle ? 0 : (int)hi;
     int cl_tile = lo_i;                         // next tile to load into shared memory
     int cl_g = g;
     int cl_gend = ts[g + 1];
@@ -637,15 +602,17 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         }
     };
     auto cursor_more = [&]() -> bool { return PERSIST ? cl_layer < n_layers : cl_tile < hi_i; };
-    // whole-step form: the rotated queries of a segment's sequence arrive by a bulk copy into the (otherwise idle) merge
+    // the rotated queries of a segment's sequence arrive by a bulk copy into the (otherwise idle) merge
     // area of the worker, completion on a barrier of their own; the copy for the next segment goes out as soon as every
     // warp has taken its fragments of the current one
     const uint32_t qbar = a_base + 320u + 8u * (uint32_t)group;
-    const uint32_t q_block_bytes = (uint32_t)p.H * HEAD_DIM * 2u;
+    const bool q_wide = LAYER && PLANES && p.q_rot32 != nullptr;
+    const uint32_t q_block_bytes = (uint32_t)p.H * HEAD_DIM * (q_wide ? 4u : 2u);
     uint32_t q_par = 0;
     auto issue_queries = [&](int layer, int gq) {
         mbar_arrive_expect_tx(qbar, q_block_bytes);
-        bulk_load(merge_s, p.q_rot16 + ((size_t)layer * p.G + (size_t)gq) * (size_t)p.H * HEAD_DIM, q_block_bytes, qbar);
+        const char* const src = q_wide ? reinterpret_cast<const char*>(p.q_rot32) : reinterpret_cast<const char*>(p.q_rot16);
+        bulk_load(merge_s, src + ((size_t)layer * p.G + (size_t)gq) * q_block_bytes, q_block_bytes, qbar);
     };
     int consumed = 0;
     int s_idx = 0;          // 2-bit form: stage of the tile being consumed and the parity of its barrier
@@ -711,10 +678,14 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             // fences were in all 16 warps' instruction streams.)  Its own wait is bounded like theirs, and it leaves only when
             // the copies it issued have landed.
             if constexpr (HKV == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ATTN_REGS_COPY));
-            if (warp >= ATTN_GROUPS * (Hkv + 1) || lo >= hi) return;
+            if (warp >= ATTN_GROUPS * (Hkv + 1) || lo_i >= hi_i) return;
             int n = 0;
-            bool stuck = false;
+            bool stuck = false, waited = !LAYER || !p.appends;
             for (; cursor_more() && loads_on && !stuck; ++n, cursor_advance()) {
+                if (!waited && cl_tile + 1 == cl_gend) {  // the tile of a new token: not before the launch that appends has finished
+                    pdl_wait();
+                    waited = true;
+                }
                 const int st = n % S;
                 const uint32_t par = ((uint32_t)(n / S) & 1u) ^ 1u;  // of the hand-back that this tile's copies wait for
                 for (int part = 0; part < 2 && !stuck; ++part) {
@@ -739,285 +710,11 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             return;
         }
         if constexpr (HKV == 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ATTN_REGS_WORK));
-        if (gtid == 0 && loads_on) issue_queries(0, g);
-    } else if constexpr (FUSED) {
-        // The new token of a sequence is appended by the worker that owns the sequence's last tile (the only tile the
-        // row can be in), before that tile is fetched.  The rotation of the sequence's 2 * Hkv head vectors runs on the
-        // tensor cores (16 rows x 128 x 128, fp16 hi/lo operands as in the prefill kernel); a coordinate within
-        // APPEND_MARGIN of a decision bound is recomputed with the reference's exact fp32 chain, so that the stored
-        // bytes are the reference's.  The ring is filled first unless one of its tiles is the tile being written.
-        int g_app0 = g;  // first sequence whose last tile starts at or after lo
-        while (g_app0 < G && ts[g_app0 + 1] - 1 < lo_i) ++g_app0;
-        // (without new keys and values the launch only builds its table, rotates the queries and attends)
-        const bool have_app = !PERSIST && p.new_k != nullptr && g_app0 < G && ts[g_app0 + 1] - 1 < hi_i;
-        const bool fill_before = !have_app || ts[g_app0 + 1] - 1 >= lo_i + S;
-        if (early) {
-            // none of the tiles filled here can hold a row the step is about to write
-            if (fill_before) fill_ring();
+        if (LAYER) {
             pdl_wait();
             pdl_launch_dependents();
-        } else if (fill_before) {
-            fill_ring();
         }
-        if constexpr (SEPARATE) {  // the table for the merge kernel (behind the wait: the previous layer's merge has read its own)
-            if (wid == 0) {  // (worker 0 always takes part)
-                for (int i = gtid; i <= G; i += gthreads) p.table_out[i] = ts[i];
-                if (gtid == 0) {
-                    p.table_out[G + 1] = W;
-                    p.table_out[G + 2] = (int)N;
-                }
-            }
-        }
-        if (have_app) {
-            constexpr float APPEND_MARGIN = 1.6e-5f;  // twice the worst-case rounding of a 128-term fp32 sum with sum|r x| <= 1
-            constexpr int NVEC = 2 * Hkv;              // head vectors of one token: K heads, then V heads
-            const uint32_t hi_a = merge_s, lo_a = merge_s + 16u * MERGE_ROW * 2u;  // A operands [16][MERGE_ROW] fp16 (idle merge area)
-            const uint32_t app_a = a_base + RegionA::FUSED_APP_OFF + (uint32_t)group * RegionA::FUSED_APP_GROUP_BYTES;
-            const uint32_t codes_a = app_a, inv_a = app_a + 2048u;  // codes [16][128] u8, 1/norm [16] f32
-            const uint32_t qcnt_a = app_a + 2112u, queue_a = app_a + 2128u;  // near-bound coordinates: count, [APPEND_QUEUE] items
-            constexpr uint32_t APPEND_QUEUE = 64;
-            const __half* rot_w = p.rotation + (size_t)(wid % p.rot_copies) * (HEAD_DIM * HEAD_DIM);
-            for (int ga = g_app0; ga < G && ts[ga + 1] - 1 < hi_i; ++ga) {
-                const int pos = p.positions ? p.positions[ga] : p.pos_value;
-                const int cap = p.seq_capacity ? p.seq_capacity[ga] : p.capacity_rows;
-                const bool ok = pos >= 0 && (cap <= 0 || pos < cap);
-                const long long row = (p.row_base ? p.row_base[ga] : (long long)ga * p.max_seq_len) + pos;
-                // B fragments (R), 16 bytes per lane and load, contraction index permuted as in the query rotation
-                uint4 bq[16 / Hkv][4];
-#pragma unroll
-                for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                    const uint4* rr = reinterpret_cast<const uint4*>(rot_w + (size_t)(8 * (head + nbi * Hkv) + gl) * HEAD_DIM) + t4;
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) bq[nbi][m] = __ldg(rr + 4 * m);
-                }
-                if (gtid == gthreads - 1) asm volatile("st.shared.u32 [%0], %1;" ::"r"(qcnt_a), "r"(0u) : "memory");
-                // ---- thread (vector v, 32-coordinate chunk c): sum of squares in the reference's order, norm, hi/lo ----
-                if (gtid < NVEC * 4) {
-                    const int v = gtid >> 2, c = gtid & 3;
-                    const uint4* src = reinterpret_cast<const uint4*>((v < Hkv ? p.new_k : p.new_v) + (size_t)ga * p.kv_dim +
-                                                                      (size_t)(v % Hkv) * HEAD_DIM + 32 * c);
-                    uint4 raw[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) raw[i] = __ldg(src + i);
-                    float val[32], sq[32];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const __half2* h2 = reinterpret_cast<const __half2*>(&raw[i]);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 f = __half22float2(h2[e]);
-                            val[8 * i + 2 * e] = f.x;
-                            val[8 * i + 2 * e + 1] = f.y;
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) sq[i] = mul_ftz(val[i], val[i]);
-                    // the warp-shuffle tree of the reference (offsets 16, 8, 4, 2, 1), element l taking lane l's place
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-                        for (int l = 0; l < off; ++l) sq[l] = add_ftz(sq[l], sq[l + off]);
-                    const float part = sq[0];
-                    const int l0 = lane & ~3;
-                    const float p0 = __shfl_sync(0xffffffffu, part, l0), p1 = __shfl_sync(0xffffffffu, part, l0 + 1);
-                    const float p2 = __shfl_sync(0xffffffffu, part, l0 + 2), p3 = __shfl_sync(0xffffffffu, part, l0 + 3);
-                    const float tt = add_ftz(add_ftz(add_ftz(p0, p2), add_ftz(p1, p3)), 1e-12f);
-                    const float inv = rsqrt_approx_ftz(tt);
-                    if (c == 0) {
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(inv_a + (uint32_t)v * 4u), "f"(inv) : "memory");
-                        if (ok) {
-                            __half* cn = const_cast<__half*>(v < Hkv ? p.kn : p.vn);
-                            cn[(size_t)row * Hkv + (v % Hkv)] = __float2half_rn(sqrt_approx_ftz(tt));
-                        } else if (v == 0) {
-                            atomicMax(p.status, ST_BAD_POSITION);
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {  // 8 coordinates = 16 bytes at a time
-                        uint32_t hw[4], lw[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float x0 = mul_ftz(val[8 * i + 2 * e], inv), x1 = mul_ftz(val[8 * i + 2 * e + 1], inv);
-                            const __half2 h = __floats2half2_rn(x0, x1);
-                            const float2 hf = __half22float2(h);
-                            hw[e] = *reinterpret_cast<const uint32_t*>(&h);
-                            lw[e] = pack_half2((x0 - hf.x) * 4096.0f, (x1 - hf.y) * 4096.0f);
-                        }
-                        const uint32_t o = (uint32_t)(v * MERGE_ROW + 32 * c + 8 * i) * 2u;
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(hi_a + o), "r"(hw[0]), "r"(hw[1]), "r"(hw[2]), "r"(hw[3]) : "memory");
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(lo_a + o), "r"(lw[0]), "r"(lw[1]), "r"(lw[2]), "r"(lw[3]) : "memory");
-                    }
-                } else if (NVEC < 16) {
-                    // fewer than 16 vectors: rows NVEC .. 15 of both operands are zero (16-byte pieces, 17 per row)
-                    for (int i = gtid - NVEC * 4; i < (16 - NVEC) * 17; i += gthreads - NVEC * 4) {
-                        const uint32_t o = (uint32_t)((NVEC + i / 17) * MERGE_ROW) * 2u + (uint32_t)(i % 17) * 16u;
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(hi_a + o), "r"(0u) : "memory");
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(lo_a + o), "r"(0u) : "memory");
-                    }
-                }
-                group_barrier(group, gthreads);
-                // ---- rotation on the tensor cores: two accumulators per column block (hi part, scaled lo part) ----
-                uint4 ah_lo[4], ah_hi[4], al_lo[4], al_hi[4];  // operand hi / lo, rows gl / gl + 8
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const uint32_t o0 = (uint32_t)(gl * MERGE_ROW + 32 * m + 8 * t4) * 2u, o8 = o0 + 8u * MERGE_ROW * 2u;
-                    ah_lo[m] = ldsv128(hi_a + o0);
-                    ah_hi[m] = ldsv128(hi_a + o8);
-                    al_lo[m] = ldsv128(lo_a + o0);
-                    al_hi[m] = ldsv128(lo_a + o8);
-                }
-                // the exact chain of the reference for coordinate d of vector v (R row from global, x rebuilt from the input)
-                auto exact_code = [&](int v, int d) -> int {
-                    const uint4* xs = reinterpret_cast<const uint4*>((v < Hkv ? p.new_k : p.new_v) + (size_t)ga * p.kv_dim +
-                                                                     (size_t)(v % Hkv) * HEAD_DIM);
-                    const uint4* rs = reinterpret_cast<const uint4*>(rot_w + (size_t)d * HEAD_DIM);
-                    float inv;
-                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(inv) : "r"(inv_a + (uint32_t)v * 4u) : "memory");
-                    float acc = 0.0f;
-#pragma unroll 2
-                    for (int j = 0; j < 16; ++j) {
-                        const uint4 xv = __ldg(xs + j), rv = __ldg(rs + j);
-                        const __half2* xh = reinterpret_cast<const __half2*>(&xv);
-                        const __half2* rh = reinterpret_cast<const __half2*>(&rv);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 xf = __half22float2(xh[e]), rf = __half22float2(rh[e]);
-                            acc = fma_ftz(rf.x, mul_ftz(xf.x, inv), acc);
-                            acc = fma_ftz(rf.y, mul_ftz(xf.y, inv), acc);
-                        }
-                    }
-                    return quantize_code(acc, BITS);
-                };
-#pragma unroll
-                for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                    const int nb = head + nbi * Hkv;
-                    float ch[4] = {0.0f, 0.0f, 0.0f, 0.0f}, cl[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        mma16816(ch, ah_lo[m].x, ah_hi[m].x, ah_lo[m].y, ah_hi[m].y, bq[nbi][m].x, bq[nbi][m].y);
-                        mma16816(ch, ah_lo[m].z, ah_hi[m].z, ah_lo[m].w, ah_hi[m].w, bq[nbi][m].z, bq[nbi][m].w);
-                        mma16816(cl, al_lo[m].x, al_hi[m].x, al_lo[m].y, al_hi[m].y, bq[nbi][m].x, bq[nbi][m].y);
-                        mma16816(cl, al_lo[m].z, al_hi[m].z, al_lo[m].w, al_hi[m].w, bq[nbi][m].z, bq[nbi][m].w);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {  // (row gl, col), (row gl, col + 1), (row gl + 8, col), (row gl + 8, col + 1)
-                        const int v = gl + 8 * (e >> 1), d = 8 * nb + 2 * t4 + (e & 1);
-                        const float dval = fmaf(cl[e], 1.0f / 4096.0f, ch[e]);
-                        int code = quantize_code(dval, BITS);
-                        float dist = 3.0e38f;  // distance to the nearest decision bound
-                        if (BITS == 4) {
-#pragma unroll
-                            for (int i = 0; i < 15; ++i) dist = fminf(dist, fabsf(dval - kBnd4[i]));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) dist = fminf(dist, fabsf(dval - kBnd2[i]));
-                        }
-                        if (v < NVEC) {
-                            if (dist < APPEND_MARGIN) {  // rare (about 1 coordinate in 700): queued for the exact chain below
-                                const uint32_t slot = atom_add_shared(qcnt_a, 1u);
-                                if (slot < APPEND_QUEUE)
-                                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(queue_a + 4u * slot), "r"((uint32_t)(v << 8 | d)) : "memory");
-                                else
-                                    code = exact_code(v, d);
-                            }
-                            asm volatile("st.shared.u8 [%0], %1;" ::"r"(codes_a + (uint32_t)(v * HEAD_DIM + d)), "r"(code) : "memory");
-                        }
-                    }
-                }
-                group_barrier(group, gthreads);
-                // ---- the exact chain of the reference for the queued coordinates, 8 lanes per item: lane s of a group
-                //      prepares terms k = 16 s .. 16 s + 15 (one round trip for everything), then the k-ascending chain
-                //      runs through the lanes in order, the running sum handed on by a shuffle ----
-                {
-                    uint32_t queued;
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(queued) : "r"(qcnt_a) : "memory");
-                    queued = queued < APPEND_QUEUE ? queued : APPEND_QUEUE;
-                    const int sub = lane & 7;
-                    for (uint32_t i0 = (uint32_t)head * 4u; i0 < queued; i0 += (uint32_t)Hkv * 4u) {  // warp-uniform
-                        const uint32_t i = i0 + (uint32_t)(lane >> 3);
-                        const bool live = i < queued;
-                        uint32_t item = 0u;
-                        if (live) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(item) : "r"(queue_a + 4u * i) : "memory");
-                        const int v = (int)(item >> 8), d = (int)(item & 255u);
-                        float xs[16], rr[16];
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) xs[e] = rr[e] = 0.0f;
-                        if (live) {
-                            const uint4* xsrc = reinterpret_cast<const uint4*>((v < Hkv ? p.new_k : p.new_v) + (size_t)ga * p.kv_dim +
-                                                                               (size_t)(v % Hkv) * HEAD_DIM) + 2 * sub;
-                            const uint4* rsrc = reinterpret_cast<const uint4*>(rot_w + (size_t)d * HEAD_DIM) + 2 * sub;
-                            float inv;
-                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(inv) : "r"(inv_a + (uint32_t)v * 4u) : "memory");
-#pragma unroll
-                            for (int j = 0; j < 2; ++j) {
-                                const uint4 xv = __ldg(xsrc + j), rv = __ldg(rsrc + j);
-                                const __half2* xh = reinterpret_cast<const __half2*>(&xv);
-                                const __half2* rh = reinterpret_cast<const __half2*>(&rv);
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const float2 xf = __half22float2(xh[e]), rf = __half22float2(rh[e]);
-                                    xs[8 * j + 2 * e] = mul_ftz(xf.x, inv);
-                                    xs[8 * j + 2 * e + 1] = mul_ftz(xf.y, inv);
-                                    rr[8 * j + 2 * e] = rf.x;
-                                    rr[8 * j + 2 * e + 1] = rf.y;
-                                }
-                            }
-                        }
-                        float acc = 0.0f;
-#pragma unroll
-                        for (int st = 0; st < 8; ++st) {
-                            if (sub == st) {
-#pragma unroll
-                                for (int e = 0; e < 16; ++e) acc = fma_ftz(rr[e], xs[e], acc);
-                            }
-                            acc = __shfl_sync(0xffffffffu, acc, (lane & ~7) + st);
-                        }
-                        if (live && sub == 0)
-                            asm volatile("st.shared.u8 [%0], %1;" ::"r"(codes_a + (uint32_t)(v * HEAD_DIM + d)), "r"(quantize_code(acc, BITS)) : "memory");
-                    }
-                }
-                group_barrier(group, gthreads);
-                // ---- pack: one 32-bit word (8 four-bit or 16 two-bit codes) per thread; NVEC vectors ----
-                {
-                    constexpr int words_per_vec = (int)Geo::BPH / 4;
-                    for (int wi = gtid; ok && wi < NVEC * words_per_vec; wi += gthreads) {
-                        const int vi = wi / words_per_vec, wv = wi - vi * words_per_vec;
-                        uint32_t word = 0;
-                        if (BITS == 2) {
-                            uint4 c4;  // ordered after the barrier: a volatile load, unlike the tile loop's
-                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(c4.x), "=r"(c4.y), "=r"(c4.z), "=r"(c4.w)
-                                         : "r"(codes_a + (uint32_t)(vi * HEAD_DIM + 16 * wv)) : "memory");
-                            const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-                            for (int b2 = 0; b2 < 4; ++b2) {
-                                const uint32_t x = cw[b2];
-                                const uint32_t pk = (x & 3u) | ((x >> 6) & 0xcu) | ((x >> 12) & 0x30u) | ((x >> 18) & 0xc0u);
-                                word |= pk << (8 * b2);
-                            }
-                        } else {
-                            uint2 c2;
-                            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(c2.x), "=r"(c2.y)
-                                         : "r"(codes_a + (uint32_t)(vi * HEAD_DIM + 8 * wv)) : "memory");
-                            const uint32_t cw[2] = {c2.x, c2.y};
-#pragma unroll
-                            for (int hb2 = 0; hb2 < 2; ++hb2) {
-                                const uint32_t x = cw[hb2];
-                                const uint32_t pk = (x & 0xfu) | ((x >> 4) & 0xf0u) | ((x >> 8) & 0xf00u) | ((x >> 12) & 0xf000u);
-                                word |= pk << (16 * hb2);
-                            }
-                        }
-                        uint8_t* cq = const_cast<uint8_t*>(vi < Hkv ? p.ck : p.cv);
-                        *reinterpret_cast<uint32_t*>(cq + (size_t)row * kvp + (size_t)(vi % Hkv) * Geo::BPH + 4 * wv) = word;
-                    }
-                }
-                // the row is read back by tensor-map copies (async proxy) of this worker
-                __threadfence();
-                fence_proxy_async_all();
-                group_barrier(group, gthreads);
-            }
-            if (gtid == 0) fence_proxy_async_all();
-        }
-        if (!fill_before) fill_ring();
+        if (gtid == 0 && loads_on) issue_queries(0, g);
     } else {
         fill_ring();
     }
@@ -1111,7 +808,20 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             s_zero = __shfl_sync(0xffffffffu, zero, 8 * t4);
         };
         // lane (gl, t4): the 32 coordinates 32*t4 .. of its head from the merge area, rows `pitch` bytes apart
-        auto take_fragments = [&](uint32_t pitch) {
+        auto take_fragments = [&]() {
+            constexpr uint32_t pitch = HEAD_DIM * 2u;
+            if (q_wide) {
+                float x[32];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    uint4 u = make_uint4(0u, 0u, 0u, 0u);
+                    if (q_on && !dead) u = ldsv128(merge_s + (uint32_t)(head * grp + q_col) * (HEAD_DIM * 4u) + (uint32_t)(32 * t4 + 4 * i) * 4u);
+                    x[4 * i] = __uint_as_float(u.x); x[4 * i + 1] = __uint_as_float(u.y);
+                    x[4 * i + 2] = __uint_as_float(u.z); x[4 * i + 3] = __uint_as_float(u.w);
+                }
+                make_planes(x);
+                return;
+            }
             uint4 qw[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -1146,7 +856,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 }
             }
         };
-        if constexpr (PERSIST) {
+        if constexpr (PUBLISH) {
             uint32_t ok = (dead || !loads_on) ? 1u : 0u;
             for (uint32_t it = 0; it < (1u << 14) && !ok; ++it) ok = mbar_try_wait_hint(qbar, q_par, 20000u);
             if (!ok) {
@@ -1156,7 +866,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             dead = __any_sync(0xffffffffu, dead);
             q_par ^= 1u;
             TQ_STAMP(9);   // wait for the query block
-            take_fragments((uint32_t)HEAD_DIM * 2u);
+            take_fragments();
             TQ_STAMP(10);  // fragments
             group_barrier(group, gthreads);  // every warp holds its fragments: the area may take the next block
             TQ_STAMP(11);  // barrier of the worker's warps
@@ -1165,130 +875,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 if (seg_end < hi_i) issue_queries(layer, g + 1);
                 else if (layer + 1 < n_layers) issue_queries(layer + 1, g_lo);
             }
-        } else if constexpr (SEPARATE) {
-            // Rotate this sequence's queries here: rot[h][d] = sum_k q[h][k] * R[d][k] on the tensor cores, all heads in one
-            // round through the merge area: fp16 in ([H][MERGE_ROW], padded), fp16 out, scaled by log2(e) / sqrt(128).  The
-            // loads of R and of the queries are in flight together.  (In rounds of 16 heads, with fp32 results, this took 5.5 us
-            // of a layer's 84 at 32 heads.)  B fragments straight from R, 16 contiguous bytes per lane and load; the contraction
-            // index is permuted the same way on both sides: step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3.
-            uint4 bq[16 / Hkv][4];
-#pragma unroll
-            for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                const int nb = head + nbi * Hkv;
-                const uint4* rr = reinterpret_cast<const uint4*>(p.rotation + (size_t)(wid % p.rot_copies) * (HEAD_DIM * HEAD_DIM) +
-                                                                 (size_t)(8 * nb + gl) * HEAD_DIM) + t4;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) bq[nbi][m] = __ldg(rr + 4 * m);
-            }
-            if (tile != lo_i) group_barrier(group, gthreads);  // every warp has taken the previous sequence's fragments
-            const uint4* const q_src = reinterpret_cast<const uint4*>(p.new_q + (size_t)g * p.q_dim);
-            for (int i = gtid; i < p.H * 16; i += gthreads) {
-                const uint4 u = __ldg(q_src + i);
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(merge_s + (uint32_t)((i >> 4) * MERGE_ROW) * 2u + (uint32_t)(i & 15) * 16u),
-                             "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w) : "memory");
-            }
-            group_barrier(group, gthreads);
-            float rc[2][16 / Hkv][4];
-#pragma unroll
-            for (int hb = 0; hb < 2; ++hb) {
-                if (16 * hb >= p.H) break;
-                // (rows at or past H hold whatever the area held: their results are not stored)
-#pragma unroll
-                for (int nbi = 0; nbi < 16 / Hkv; ++nbi) rc[hb][nbi][0] = rc[hb][nbi][1] = rc[hb][nbi][2] = rc[hb][nbi][3] = 0.0f;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const uint32_t at = merge_s + (uint32_t)((16 * hb + gl) * MERGE_ROW + 32 * m + 8 * t4) * 2u;
-                    const uint4 a_lo = ldsv128(at), a_hi = ldsv128(at + 8u * MERGE_ROW * 2u);
-#pragma unroll
-                    for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                        mma16816(rc[hb][nbi], a_lo.x, a_hi.x, a_lo.y, a_hi.y, bq[nbi][m].x, bq[nbi][m].y);
-                        mma16816(rc[hb][nbi], a_lo.z, a_hi.z, a_lo.w, a_hi.w, bq[nbi][m].z, bq[nbi][m].w);
-                    }
-                }
-            }
-            group_barrier(group, gthreads);
-#pragma unroll
-            for (int hb = 0; hb < 2; ++hb) {
-                if (16 * hb >= p.H) break;
-                const float sc = 0.12751743074602467f;
-#pragma unroll
-                for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                    const uint32_t at = merge_s + (uint32_t)((16 * hb + gl) * MERGE_ROW + 8 * (head + nbi * Hkv) + 2 * t4) * 2u;
-                    if (16 * hb + gl < p.H)
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(pack_half2(rc[hb][nbi][0] * sc, rc[hb][nbi][1] * sc)) : "memory");
-                    if (16 * hb + gl + 8 < p.H)
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + 8u * MERGE_ROW * 2u), "r"(pack_half2(rc[hb][nbi][2] * sc, rc[hb][nbi][3] * sc)) : "memory");
-                }
-            }
-            group_barrier(group, gthreads);
-            take_fragments((uint32_t)MERGE_ROW * 2u);
         } else {
             float qv[32];
-            if constexpr (FUSED) {
-                // Rotate this sequence's queries here: rot[h][d] = sum_k q[h][k] * R[d][k] on the tensor cores, 16 heads
-                // at a time, every warp two (Hkv = 8) or four (Hkv = 4) blocks of 8 coordinates; the result goes through
-                // shared memory (the idle merge area) to the lanes that need it, scaled by log2(e) / sqrt(128).
-                const uint32_t qs_a = merge_s;  // [16][128] fp32
-#pragma unroll
-                for (int i = 0; i < 32; ++i) qv[i] = 0.0f;
-                for (int hb = 0; hb < p.H; hb += 16) {
-                    // 16 query heads (4 KB) into shared memory with one coalesced 16-byte load per thread
-                    for (int i = gtid; i < 256; i += gthreads) {
-                        const int r = i >> 4;
-                        uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                        if (hb + r < p.H)
-                            u = __ldg(reinterpret_cast<const uint4*>(p.new_q + (PERSIST ? (size_t)layer * (size_t)p.q_layer_stride : (size_t)0) +
-                                                                     (size_t)g * p.q_dim + (size_t)(hb + r) * HEAD_DIM) + (i & 15));
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(qs_a + (uint32_t)i * 16u), "r"(u.x), "r"(u.y),
-                                     "r"(u.z), "r"(u.w) : "memory");
-                    }
-                    // B fragments straight from R (16 contiguous bytes per lane and load: whole sectors).  The contraction
-                    // index is permuted the same way on both sides: step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3.
-                    uint4 bq[16 / Hkv][4];
-#pragma unroll
-                    for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                        const int nb = head + nbi * Hkv;
-                        const uint4* rr = reinterpret_cast<const uint4*>(p.rotation + (size_t)(wid % p.rot_copies) * (HEAD_DIM * HEAD_DIM) +
-                                                                         (size_t)(8 * nb + gl) * HEAD_DIM) + t4;
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) bq[nbi][m] = __ldg(rr + 4 * m);
-                    }
-                    group_barrier(group, gthreads);
-                    uint4 a_lo[4], a_hi[4];  // rows gl and gl + 8
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        a_lo[m] = ldsv128(qs_a + (uint32_t)(gl * HEAD_DIM + 32 * m + 8 * t4) * 2u);
-                        a_hi[m] = ldsv128(qs_a + (uint32_t)((gl + 8) * HEAD_DIM + 32 * m + 8 * t4) * 2u);
-                    }
-                    group_barrier(group, gthreads);  // the staging area turns into the fp32 result area
-#pragma unroll
-                    for (int nbi = 0; nbi < 16 / Hkv; ++nbi) {
-                        const int nb = head + nbi * Hkv;
-                        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) {
-                            mma16816(c, a_lo[m].x, a_hi[m].x, a_lo[m].y, a_hi[m].y, bq[nbi][m].x, bq[nbi][m].y);
-                            mma16816(c, a_lo[m].z, a_hi[m].z, a_lo[m].w, a_hi[m].w, bq[nbi][m].z, bq[nbi][m].w);
-                        }
-                        const float sc = 0.12751743074602467f;
-                        const uint32_t o0 = qs_a + (uint32_t)(gl * HEAD_DIM + 8 * nb + 2 * t4) * 4u;
-                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(o0), "f"(c[0] * sc), "f"(c[1] * sc) : "memory");
-                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(o0 + 8u * HEAD_DIM * 4u), "f"(c[2] * sc), "f"(c[3] * sc) : "memory");
-                    }
-                    group_barrier(group, gthreads);
-                    const int myrow = head * grp + q_col - hb;
-                    if (q_on && myrow >= 0 && myrow < 16 && !TQ_DBG(8)) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            float4 f;
-                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w)
-                                         : "r"(qs_a + (uint32_t)(myrow * HEAD_DIM + 32 * t4 + 4 * i) * 4u) : "memory");
-                            qv[4 * i] = f.x; qv[4 * i + 1] = f.y; qv[4 * i + 2] = f.z; qv[4 * i + 3] = f.w;
-                        }
-                    }
-                    group_barrier(group, gthreads);
-                }
-            } else if (q_on && !TQ_DBG(8)) {
+            if (q_on && !TQ_DBG(8)) {
                 const float4* src =
                     reinterpret_cast<const float4*>(p.q_rot + ((size_t)g * p.H + (size_t)head * grp + q_col) * HEAD_DIM + 32 * t4);
 #pragma unroll
@@ -1641,14 +1230,13 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             }
         }
         if (TQ_DBG(4)) { ++g; continue; }
-        if constexpr (PERSIST || SEPARATE) {  // the partials are merged by merge_partials_kernel
+        if constexpr (PUBLISH) {  // the partials are merged by a launch of its own
             ++g;
             continue;
         }
-        // number of workers that hold a part of sequence g
-        // owners of the sequence's first and last tile (of the units those tiles start at)
-        const int first_w = (int)(((ts_g + g * A + 1) * W - 1) / U);
-        const int last_w = (int)(((ts_g1 + g * A) * W - 1) / U);
+        // number of workers that hold a part of sequence g: owners of the sequence's first and last tile
+        const int first_w = (int)(((long long)(ts_g + 1) * W - 1) / N);
+        const int last_w = (int)(((long long)ts_g1 * W - 1) / N);
         const int parts = last_w - first_w + 1;
         group_barrier(group, gthreads);  // every warp's partial is written (happens-before the fence below)
         uint32_t is_last = 1u;
@@ -1701,7 +1289,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     }
 }
 
-// ---- merge of the partials that modes 2 and 3 publish -----------------------------------------------------------------
+// ---- merge of the partials that modes 1 and 2 publish -----------------------------------------------------------------
 struct MergeParams {
     const float* partials;       // [layers][workers + G][H][PART_STRIDE]
     const int* table;            // tile table [G + 1], then {workers that took part, total tiles}
@@ -1711,27 +1299,20 @@ struct MergeParams {
     long long part_layer_stride; // floats
     long long q_layer_stride;    // halves
     int G, H, q_dim;
-    int app_weight;              // as in AttnParams: what a sequence weighs beside its tiles in the cut of the work list
     int rotated_out;             // 1: leave the results in rotated space (the consumer's weights carry R^T)
 };
 
-// The merge that mode 1's last-arriving worker does, as a launch of its own spread over the whole GPU.  One CTA per (sequence,
-// layer): WARPS = 8, two heads per warp, for the many short merges of a whole step; WARPS = 16, a CTA per 16 heads too, a head
-// per warp with up to 16 parts' loads in flight, where one layer's merge is the tail of a layer.
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) merge_partials_kernel(const MergeParams p) {
+// Merge of a whole step's partials: one CTA of 8 warps per (sequence, layer), two heads per warp.
+__global__ void __launch_bounds__(256) merge_partials_kernel(const MergeParams p) {
     __shared__ __align__(16) uint8_t merge_buf[RegionA::MERGE_GROUP_BYTES];
-    if (WARPS == 16) pdl_launch_dependents();
     pdl_wait();  // the partials and the table come from the previous kernel in the stream
-    const int g = blockIdx.x, layer = blockIdx.y, hb = 16 * (int)blockIdx.z;
+    const int g = blockIdx.x, layer = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long A = p.app_weight;
-    const long long u0 = p.table[g] + g * A, u1 = p.table[g + 1] + g * A;  // the units its first tile starts and its last one ends at
-    const long long W = p.table[p.G + 1], U = p.table[p.G + 2] + p.G * A;
-    if (U <= 0 || W <= 0) return;
-    // owners of the sequence's first and last tile: worker w holds the units [w * U / W, (w + 1) * U / W)
-    const int first_w = (int)(((u0 + 1) * W - 1) / U);
-    const int last_w = (int)((u1 * W - 1) / U);
+    const long long t0 = p.table[g], t1 = p.table[g + 1], W = p.table[p.G + 1], N = p.table[p.G + 2];
+    if (N <= 0 || W <= 0) return;
+    // owners of the sequence's first and last tile: worker w holds the tiles [w * N / W, (w + 1) * N / W)
+    const int first_w = (int)(((t0 + 1) * W - 1) / N);
+    const int last_w = (int)((t1 * W - 1) / N);
     const int parts = last_w - first_w + 1;
     const int H = p.H;
     auto out_row = [&](int vh) -> __half* {
@@ -1742,9 +1323,127 @@ __global__ void __launch_bounds__(WARPS * 32) merge_partials_kernel(const MergeP
         if (!p.out_f32 || vh >= H) return nullptr;
         return p.out_f32 + (((size_t)layer * p.G + (size_t)g) * H + (size_t)vh) * HEAD_DIM;
     };
-    merge_sequence<WARPS>(p.partials + (size_t)layer * (size_t)p.part_layer_stride + (size_t)(first_w + g) * H * PART_STRIDE,
-                          parts, H, smem_u32(merge_buf), p.rotation_t, warp, lane, 0, WARPS * 32, out_row, out_row_f32,
-                          WARPS == 16 ? hb : 0, WARPS == 16 ? min(hb + 16, H) : H, p.rotated_out != 0);
+    merge_sequence<8>(p.partials + (size_t)layer * (size_t)p.part_layer_stride + (size_t)(first_w + g) * H * PART_STRIDE,
+                      parts, H, smem_u32(merge_buf), p.rotation_t, warp, lane, 0, 256, out_row, out_row_f32, 0, H, p.rotated_out != 0);
+}
+
+// The merge of one layer's partials (mode 1), the tail of that layer: bound by latency.  One CTA per (sequence, 8 heads), a warp per
+// head, its parts' loads in flight together.  Under the attention's last tiles, before the wait: R's fragments and which workers had
+// a part, from the positions (which that launch does not write; what came before it has finished when this one starts).
+struct MergeLayerParams {
+    const float* partials;       // [workers + G][H][PART_STRIDE]
+    const int* positions;        // device [G] or null: pos_value
+    const __half* rotation_t;
+    __half* out;                 // [G][q_dim]
+    float* out_f32;              // optional [G][H][128]
+    int pos_value, G, H, q_dim;
+    int workers;                 // workers of the attention launch
+};
+constexpr int MERGE_HEADS = 8;
+__global__ void __launch_bounds__(MERGE_HEADS * 32) merge_layer_kernel(const MergeLayerParams p) {
+    __shared__ __align__(16) __half a_op[2 * MERGE_HEADS * MERGE_ROW];  // rows 0-7: high parts, 8-15: low parts
+    __shared__ int sums[2][MERGE_HEADS];
+    pdl_launch_dependents();
+    const int g = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane >> 2, t4 = lane & 3;
+    const int h = MERGE_HEADS * (int)blockIdx.y + warp;
+    // out[h][d] = sum_k a[h][k] R[k][d]: B fragments of the column blocks `warp` and `warp + 8`
+    uint4 bf[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int m = 0; m < 4; ++m)  // (step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3, on both sides)
+            bf[i][m] = ldg128_now(reinterpret_cast<const uint4*>(p.rotation_t + (size_t)(8 * (warp + MERGE_HEADS * i) + gl) * HEAD_DIM) + t4 + 4 * m);
+    auto tiles_of = [&](int i) {
+        const int pos = p.positions ? p.positions[i] : p.pos_value;
+        return ((pos < 0 ? 0 : pos) + TILE_TOKENS) / TILE_TOKENS;
+    };
+    int before = 0, all = 0;  // tiles before sequence g, of all sequences
+    for (int i = threadIdx.x; i < p.G; i += MERGE_HEADS * 32) {
+        const int n = tiles_of(i);
+        all += n;
+        before += i < g ? n : 0;
+    }
+    const int own = tiles_of(g);
+    all = __reduce_add_sync(0xffffffffu, all);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+        sums[0][warp] = all;
+        sums[1][warp] = before;
+    }
+    __syncthreads();
+    all = before = 0;
+#pragma unroll
+    for (int w = 0; w < MERGE_HEADS; ++w) {
+        all += sums[0][w];
+        before += sums[1][w];
+    }
+    // owners of the sequence's first and last tile, as in the attention kernel's cut of the list
+    const long long W = attention_workers(p.workers, all, p.G);
+    const int first_w = (int)(((long long)(before + 1) * W - 1) / all);
+    const int parts = (int)(((long long)(before + own) * W - 1) / all) - first_w + 1;
+    const float* const part0 = p.partials + ((size_t)(first_w + g) * p.H + h) * PART_STRIDE;
+    const size_t pstride = (size_t)p.H * PART_STRIDE;
+    pdl_wait();
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (h < p.H) {
+        constexpr int FLIGHT = 16;
+        float M = -1e30f, Z = 0.0f;
+        for (int j0 = 0; j0 < parts; j0 += FLIGHT) {
+            const int n = parts - j0;
+            float2 ml = make_float2(-1e30f, 0.0f);
+            if (lane < FLIGHT && lane < n) ml = __ldcg(reinterpret_cast<const float2*>(part0 + (size_t)(j0 + lane) * pstride + HEAD_DIM));
+            float4 v[FLIGHT];
+#pragma unroll
+            for (int j = 0; j < FLIGHT; ++j)
+                v[j] = j < n ? __ldcg(reinterpret_cast<const float4*>(part0 + (size_t)(j0 + j) * pstride) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float Mn = ml.x;
+#pragma unroll
+            for (int o = FLIGHT / 2; o > 0; o >>= 1) Mn = fmaxf(Mn, __shfl_xor_sync(0xffffffffu, Mn, o));
+            Mn = fmaxf(M, __shfl_sync(0xffffffffu, Mn, 0));
+            const float e = lane < FLIGHT && lane < n ? ex2_approx(ml.x - Mn) : 0.0f, f = ex2_approx(M - Mn);
+            float z = ml.y * e;
+#pragma unroll
+            for (int o = FLIGHT / 2; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+            Z = Z * f + __shfl_sync(0xffffffffu, z, 0);
+            M = Mn;
+            a.x *= f; a.y *= f; a.z *= f; a.w *= f;
+#pragma unroll
+            for (int j = 0; j < FLIGHT; ++j) {
+                const float wj = __shfl_sync(0xffffffffu, e, j);
+                a.x = fmaf(wj, v[j].x, a.x); a.y = fmaf(wj, v[j].y, a.y);
+                a.z = fmaf(wj, v[j].z, a.z); a.w = fmaf(wj, v[j].w, a.w);
+            }
+        }
+        const float inv = 1.0f / (Z + 1e-8f);
+        a.x *= inv; a.y *= inv; a.z *= inv; a.w *= inv;
+    }
+    *reinterpret_cast<uint2*>(a_op + warp * MERGE_ROW + 4 * lane) = make_uint2(pack_half2(a.x, a.y), pack_half2(a.z, a.w));
+    *reinterpret_cast<uint2*>(a_op + (warp + MERGE_HEADS) * MERGE_ROW + 4 * lane) = make_uint2(pack_low_half2(a.x, a.y), pack_low_half2(a.z, a.w));
+    __syncthreads();
+    float c[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[i][0][e] = c[i][1][e] = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const uint4 hi = *reinterpret_cast<const uint4*>(a_op + gl * MERGE_ROW + 32 * m + 8 * t4);
+        const uint4 lo = *reinterpret_cast<const uint4*>(a_op + (gl + MERGE_HEADS) * MERGE_ROW + 32 * m + 8 * t4);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mma16816(c[i][0], hi.x, lo.x, hi.y, lo.y, bf[i][m].x, bf[i][m].y);
+            mma16816(c[i][1], hi.z, lo.z, hi.w, lo.w, bf[i][m].z, bf[i][m].w);
+        }
+    }
+    const int ho = MERGE_HEADS * (int)blockIdx.y + gl;
+    if (ho >= p.H) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float o0 = (c[i][0][0] + c[i][1][0]) + (c[i][0][2] + c[i][1][2]), o1 = (c[i][0][1] + c[i][1][1]) + (c[i][0][3] + c[i][1][3]);
+        const size_t at = (size_t)ho * HEAD_DIM + 8 * (warp + MERGE_HEADS * i) + 2 * t4;
+        *reinterpret_cast<__half2*>(p.out + (size_t)g * p.q_dim + at) = __floats2half2_rn(o0, o1);
+        if (p.out_f32) *reinterpret_cast<float2*>(p.out_f32 + (size_t)g * p.H * HEAD_DIM + at) = make_float2(o0, o1);
+    }
 }
 
 }  // namespace tq

@@ -289,23 +289,28 @@ int tq_append_decode(uint8_t* ck_q, void* k_norms, uint8_t* cv_q, void* v_norms,
                        workspace_bytes, true, cs(s));
 }
 
-// Inputs of the fused per-layer launch (append + query rotation + attention in one kernel).
-struct FusedInputs {
+// Inputs of the layer form: layer_prep_kernel (append, query rotation), the attention, its merge.
+struct LayerInputs {
     const void* q;
-    const void* k;
+    const void* k;              // null: nothing is appended
     const void* v;
-    const void* rotation;
+    const void* rotation;       // R row-major, rot_copies copies back to back
     int rot_copies;
-    int early;
-    const int* seq_capacity;  // ragged slots: per-sequence row limits (device), or null
+    int static_rotation;        // R is not written by any kernel of the stream
+    void* rotation_t;           // where R transposed is to go, or null (the caller has it)
+    const int* seq_capacity;    // ragged slots: per-sequence row limits (device), or null
 };
+// (it moves the vectors 16 bytes at a time)
+static bool layer_form_ok(const void* q, const void* k, const void* v, int q_dim) {
+    return (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15u) == 0 && q_dim % 8 == 0;
+}
 
 static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& tmV, const void* ck_q, const void* cv_q,
                           const void* k_norms, const void* v_norms,
                           const void* rotation_t, const int* positions, int pos_value, const long long* row_base,
                           long long total_rows, int max_seq_len, int G, int num_heads, int num_kv_heads, int q_dim,
                           int bits, void* workspace, size_t workspace_bytes, cudaStream_t s, bool pdl = false,
-                          const FusedInputs* fused = nullptr, float* out_f32 = nullptr,
+                          const LayerInputs* layer = nullptr, float* out_f32 = nullptr,
                           const long long* prefix_base = nullptr, const int* prefix_tiles = nullptr) {
     FullWorkspace fw = carve_full(workspace, G, num_heads);
     if (fw.bytes > workspace_bytes) return TQ_ERR_WORKSPACE;
@@ -330,32 +335,32 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
 #endif
     static const int l2_ahead = getenv("TQ_ATTN_L2_AHEAD") ? atoi(getenv("TQ_ATTN_L2_AHEAD")) : ATTN_L2_AHEAD;
     p.l2_ahead = l2_ahead > 0 ? l2_ahead : (1 << 28);  // 0 switches the prefetch off
-    if (fused) {
-        p.new_k = (const __half*)fused->k; p.new_v = (const __half*)fused->v; p.new_q = (const __half*)fused->q;
-        p.rotation = (const __half*)fused->rotation;
-        p.rot_copies = fused->rot_copies;
-        p.early = fused->early;
-        // what the append of one token costs its worker, in 32-token tiles (measured; TQ_FUSED_WEIGHT overrides)
-        static const int app_weight = getenv("TQ_FUSED_WEIGHT") ? atoi(getenv("TQ_FUSED_WEIGHT")) : 7;
-        p.app_weight = (!fused->k || app_weight < 0) ? 0 : app_weight;  // nothing to weigh without an append
-        p.kv_dim = num_kv_heads * HEAD_DIM; p.capacity_rows = max_seq_len;
-        p.seq_capacity = fused->seq_capacity;
-    }
     const int ctas = attention_ctas(G, max_seq_len);
-    if (!fused) return launch_attention(bits, tmK, tmV, p, ctas, s, pdl, 0);
-    // The merge inside the kernel (by the last worker to arrive at a sequence, under the others' last tiles and the next layer's
-    // start) or as a launch of its own: with more than 16 heads (two rounds) or few sequences, cut into many parts, that
-    // worker is a layer's tail of ten microseconds and more.  Measured per layer, in the kernel / as a launch: 4-bit 16 heads
-    // 64 x 4096 80 / 84 us, 4 x 16384 61 / 42, 1 x 16384 38 / 30, 18 ragged x 6395 28 / 30; 32 heads 16 x 1500 34 / 26, 64 x 1500 41 / 40,
-    // 96 x 1500 61 / 64; over 4 KV heads, whose workers have four warps for the merge, 16 x 1500 38 / 22, 128 x 1500 62 / 59.
-    const bool separate = num_heads > 16 ? num_kv_heads == 4 || 2 * ctas * ATTN_GROUPS > 7 * G : ctas * ATTN_GROUPS > 36 * G;
-    p.table_out = fw.w.tile_start;
-    const int r = launch_attention(bits, tmK, tmV, p, ctas, s, pdl, separate ? 3 : 1);
-    if (r != TQ_OK || !separate) return r;
-    MergeParams m{};
-    m.partials = p.partials; m.table = p.table_out; m.rotation_t = p.rotation_t; m.out = p.out; m.out_f32 = out_f32;
-    m.G = G; m.H = num_heads; m.q_dim = q_dim; m.app_weight = p.app_weight;
-    return launch_kernel(merge_partials_kernel<16>, dim3((unsigned)G, 1u, (unsigned)((num_heads + 15) / 16)), dim3(512), 0, s, use_pdl(), m);
+    if (!layer) return launch_attention(bits, tmK, tmV, p, ctas, s, pdl, 0);
+    LayerPrepParams lp{};
+    lp.ck = (uint8_t*)const_cast<void*>(ck_q); lp.cv = (uint8_t*)const_cast<void*>(cv_q);
+    lp.kn = (__half*)const_cast<void*>(k_norms); lp.vn = (__half*)const_cast<void*>(v_norms);
+    lp.new_k = (const __half*)layer->k; lp.new_v = (const __half*)layer->v; lp.q = (const __half*)layer->q;
+    lp.rotation = (const __half*)layer->rotation; lp.rot_copies = layer->rot_copies; lp.static_rotation = layer->static_rotation;
+    lp.rotation_t = (__half*)layer->rotation_t;
+    // The 2-bit scores' 16-bit queries come from fp32 ones where a sequence's block of them fits the kernel's area (16 heads).
+    const bool wide = bits == 2 && num_kv_heads == 8 && num_heads <= 16;
+    if (wide) lp.q_rot32 = fw.w.q_rot;
+    else lp.q_rot16 = (__half*)fw.w.q_rot;
+    lp.positions = positions; lp.row_base = row_base; lp.seq_capacity = layer->seq_capacity; lp.status = p.status;
+    lp.pos_value = pos_value; lp.max_seq_len = max_seq_len; lp.capacity_rows = max_seq_len;
+    lp.G = G; lp.H = num_heads; lp.Hkv = num_kv_heads; lp.q_dim = q_dim;
+    int r = launch_layer_prep(bits, lp, s, use_pdl());
+    if (r != TQ_OK) return r;
+    p.appends = layer->k ? 1 : 0;
+    p.q_rot16 = lp.q_rot16; p.q_rot32 = lp.q_rot32;
+    p.n_layers = 1;
+    r = launch_attention(bits, tmK, tmV, p, ctas, s, use_pdl(), 1);
+    if (r != TQ_OK) return r;
+    MergeLayerParams m{};
+    m.partials = p.partials; m.positions = positions; m.pos_value = pos_value; m.rotation_t = p.rotation_t; m.out = p.out; m.out_f32 = out_f32;
+    m.G = G; m.H = num_heads; m.q_dim = q_dim; m.workers = ctas * ATTN_GROUPS;
+    return launch_kernel(merge_layer_kernel, dim3((unsigned)G, (unsigned)((num_heads + MERGE_HEADS - 1) / MERGE_HEADS)), dim3(MERGE_HEADS * 32), 0, s, use_pdl(), m);
 }
 
 int tq_decode_attention(void* out, const uint8_t* ck_q, const uint8_t* cv_q, const void* k_norms, const void* v_norms,
@@ -610,9 +615,8 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
         need = carve_full(nullptr, G, num_heads).bytes;
         r = compat_workspace(need, &ws, cs(s));
     }
-    if (r == TQ_OK && one_launch && G <= FUSED_MAX_G && pos) {
-        // one launch: the attention kernel builds its tile table and rotates the queries itself (its fused form without
-        // an append); only the transpose of R for the merge precedes it
+    if (r == TQ_OK && one_launch && G <= FUSED_MAX_G && pos && layer_form_ok(q, nullptr, nullptr, q_dim)) {
+        // the layer form without an append
         if (!q || !out || !ck_q || !cv_q || !k_norms || !v_norms || !rotation) r = TQ_ERR_ARG;
         FullWorkspace fw = carve_full(ws, G, num_heads);
         CUtensorMap tmK, tmV;
@@ -620,12 +624,7 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
         if (r == TQ_OK) r = cached_code_map(&tmK, ck_q, (long long)G * msl, kvp);
         if (r == TQ_OK) r = cached_code_map(&tmV, cv_q, (long long)G * msl, kvp);
         if (r == TQ_OK) {
-            // (the shared workspace is carved per call: whatever an earlier call left where the tickets now live goes)
-            transpose_rotation_kernel<<<16, 256, 0, cs(s)>>>(fw.rot_t, (const __half*)rotation, fw.w.tickets, G);
-            r = cuda_status(cudaGetLastError());
-        }
-        if (r == TQ_OK) {
-            FusedInputs in{q, nullptr, nullptr, rotation, 1, 0, nullptr};
+            LayerInputs in{q, nullptr, nullptr, rotation, 1, 0, fw.rot_t, nullptr};
             r = attention_impl(out, tmK, tmV, ck_q, cv_q, k_norms, v_norms, fw.rot_t, pos, -1, nullptr, (long long)G * msl, msl, G,
                                num_heads, num_kv_heads, q_dim, bits, ws, need, cs(s), false, &in);
         }
@@ -1409,10 +1408,9 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
         return generic_attention(out, q, L.k, L.v, L.kn, L.vn, e->d_rotation, e->d_positions, -1, e->rb(), e->msl, e->G, H,
                                         Hkv, e->q_dim(), e->kv_bits, cs(s));
     }
-    // One launch per layer when the batch fits the kernel's shared-memory tile table (tq_engine_set_fused).
-    if (e->fused && e->G <= FUSED_MAX_G) {
-        const int early = engine_reads_early(e, chained, cs(s)) ? 1 : 0;
-        FusedInputs in{q, k, v, e->d_rotation_rep, ROT_COPIES, early, e->caps()};
+    // The layer form when the batch fits the kernel's shared-memory tile table (tq_engine_set_fused).
+    if (e->fused && e->G <= FUSED_MAX_G && layer_form_ok(q, k, v, e->q_dim())) {
+        LayerInputs in{q, k, v, e->d_rotation_rep, ROT_COPIES, 1, nullptr, e->caps()};
         const int r = attention_impl(out, L.tmK, L.tmV, L.k, L.v, L.kn, L.vn, e->d_rotation_t, e->d_positions, -1, e->rb(),
                                      e->total_rows, e->msl, e->G, H, Hkv, e->q_dim(), e->kv_bits, e->workspace, e->ws_bytes,
                                      cs(s), use_pdl(), &in, f32, e->shared_active ? e->d_prefix_base : nullptr,
@@ -1614,13 +1612,10 @@ static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* 
     p.status = fw.w.status;
     p.total_rows = e->total_rows; p.pos_value = -1; p.max_seq_len = e->msl;
     p.G = G; p.H = H; p.Hkv = Hkv; p.q_dim = e->q_dim();
-    p.new_q = (const __half*)q; p.rotation = (const __half*)e->d_rotation_rep; p.rot_copies = ROT_COPIES;
-    p.kv_dim = e->kv_dim(); p.capacity_rows = e->msl;
     static const int l2_ahead = getenv("TQ_ATTN_L2_AHEAD") ? atoi(getenv("TQ_ATTN_L2_AHEAD")) : ATTN_L2_AHEAD;
     p.l2_ahead = l2_ahead > 0 ? l2_ahead : (1 << 28);  // 0 switches the prefetch off
     p.layer0 = l0; p.n_layers = n;
     p.norm_layer_stride = (long long)(e->norm_layer_stride / 2);
-    p.q_layer_stride = (long long)G * e->q_dim();
     p.part_layer_stride = (long long)e->step_part_stride;
     p.table_out = e->step_table;
     p.q_rot16 = (const __half*)e->step_qrot + (size_t)l0 * G * H * HEAD_DIM;
@@ -1648,7 +1643,7 @@ static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* 
     MergeParams m{};
     m.partials = p.partials; m.table = e->step_table; m.rotation_t = (const __half*)e->d_rotation_t;
     m.out = (__half*)out; m.out_f32 = e->out_f32 ? e->out_f32 + (size_t)l0 * G * H * HEAD_DIM : nullptr;
-    m.part_layer_stride = p.part_layer_stride; m.q_layer_stride = p.q_layer_stride;
+    m.part_layer_stride = p.part_layer_stride; m.q_layer_stride = (long long)G * e->q_dim();
     m.G = G; m.H = H; m.q_dim = e->q_dim();
     m.rotated_out = (prod && prod->rotated_output) ? 1 : 0;
 #ifdef TQ_TIMING_SWITCHES
@@ -1662,7 +1657,7 @@ static int engine_step_attend(tq_engine* e, int l0, int n, const void* q, void* 
                 n, h[0] / w, h[1] / w, h[2] / w, h[3] / w, h[4] / w, h[5] / w, h[6] / w, h[8] / w, h[9] / w, h[10] / w, h[11] / w, h[12] / w, w);
     }
 #endif
-    return launch_kernel(merge_partials_kernel<8>, dim3(G, n), dim3(256), 0, s, use_pdl(), m);
+    return launch_kernel(merge_partials_kernel, dim3(G, n), dim3(256), 0, s, use_pdl(), m);
 }
 
 int tq_engine_time_attention(tq_engine* e, int enable) {

@@ -22,6 +22,7 @@
 #include "tq_decode_cluster.cuh"
 #include "tq_fp16.cuh"
 #include "tq_fp16_tc.cuh"
+#include "tq_layer_prep.cuh"
 #include "tq_qrot.cuh"
 #include "tq_generic.cuh"
 #include "tq_prefill_fa.cuh"
@@ -353,7 +354,7 @@ inline int launch_attention_t(const CUtensorMap& tmK, const CUtensorMap& tmV, co
                               bool pdl) {
     int ar = ensure_dynamic_smem((const void*)decode_attention_kernel<BITS, HKV, MODE>, ATTN_DYN_SMEM);
     if (ar != TQ_OK) return ar;
-    if constexpr (MODE == 2 && HKV == 8) {
+    if constexpr ((MODE == 1 || MODE == 2) && HKV == 8) {
         // the register split inside the kernel draws on what the launch brings: never launch with less
         static const int regs = [] {
             cudaFuncAttributes f{};
@@ -374,9 +375,9 @@ inline int launch_attention_t(const CUtensorMap& tmK, const CUtensorMap& tmV, co
     return cuda_status(cudaLaunchKernelEx(&cfg, decode_attention_kernel<BITS, HKV, MODE>, tmK, tmV, p));
 }
 
-// mode 0: after append_rotate_kernel (rotated queries and tile table in the workspace); 1: one launch per layer and step
-// (table, query rotation, optional append and merge in the kernel); 2: whole-step form over AttnParams::n_layers layers; 3: as 1
-// with the merge left to merge_partials_kernel; 4: as 2 without the copy warps (8 KV heads only).
+// mode 0: after append_rotate_kernel (rotated queries and tile table in the workspace, merge in the kernel); 1: one layer, after
+// layer_prep_kernel, the merge left to merge_layer_kernel; 2: whole-step form over AttnParams::n_layers layers; 4: as 2 without the
+// copy warps (8 KV heads only).
 inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnParams& p, int ctas,
                             cudaStream_t s, bool pdl = false, int mode = 0) {
     if (p.Hkv != 8 && p.Hkv != 4) return TQ_ERR_UNSUPPORTED;
@@ -388,10 +389,17 @@ inline int launch_attention(int bits, const CUtensorMap& tmK, const CUtensorMap&
                      : launch_attention_t<2, 4, MODE>(tmK, tmV, p, ctas, s, pdl);
     if (mode == 4) return bits == 4 ? launch_attention_t<4, 8, 4>(tmK, tmV, p, ctas, s, pdl) : launch_attention_t<2, 8, 4>(tmK, tmV, p, ctas, s, pdl);
     if (mode == 2) { TQ_ATTN_DISPATCH(2) }
-    if (mode == 3) { TQ_ATTN_DISPATCH(3) }
     if (mode == 1) { TQ_ATTN_DISPATCH(1) }
     TQ_ATTN_DISPATCH(0)
 #undef TQ_ATTN_DISPATCH
+}
+
+// Two CTAs per SM at most: each fetches R once and loops.
+inline int launch_layer_prep(int bits, const LayerPrepParams& p, cudaStream_t s, bool pdl) {
+    const long long items = (p.new_k ? p.G : 0) + ((long long)p.G * p.H + 15) / 16;
+    const dim3 grid((unsigned)std::min(items, 2ll * device_props().sm_count));
+    return bits == 4 ? launch_kernel(layer_prep_kernel<4>, grid, dim3(PREP_THREADS), 0, s, pdl, p)
+                     : launch_kernel(layer_prep_kernel<2>, grid, dim3(PREP_THREADS), 0, s, pdl, p);
 }
 
 // One cluster per (sequence, KV head, block of 8 query heads): tq_decode_cluster.cuh.  `max_tokens`: rows a sequence may hold.
@@ -485,14 +493,12 @@ inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int lay
                                              : launch_cluster_decode_e<HOST, true>(bits, p, layers, split_layers, max_tokens, s, pdl);
 }
 
-__global__ void transpose_rotation_kernel(__half* dst, const __half* src, int* tickets = nullptr, int n_tickets = 0) {
+__global__ void transpose_rotation_kernel(__half* dst, const __half* src) {
     // dst[d][k] = src[k][d]; one block per 32x32 tile would be overkill for 32 KB: a plain strided copy
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < HEAD_DIM * HEAD_DIM; i += gridDim.x * blockDim.x) {
         const int d = i >> 7, k = i & 127;
         dst[i] = src[k * HEAD_DIM + d];
     }
-    // optionally also clears the per-sequence tickets for a launch that is not preceded by the append kernel
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_tickets; i += gridDim.x * blockDim.x) tickets[i] = 0;
 }
 
 // Tensor-core form of the twin (tq_fp16_tc.cuh): every query head of a KV head from one pass, whatever their number.
