@@ -456,6 +456,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     if (TQ_DBG(32)) { pdl_wait(); pdl_launch_dependents(); return; }
     const int G = p.G;
 
+    // (layer form: the first positions are on their way while the look-up table is written)
+    int first_pos = p.pos_value;
+    if (LAYER && p.positions && tid < G) asm volatile("ld.global.u32 %0, [%1];" : "=r"(first_pos) : "l"(p.positions + tid));
     // ---- byte -> centroid table, one column per lane ----
     if (TQ_DBG(16)) {
     } else if (BITS == 4) {
@@ -502,7 +505,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             const int gq = base + tid;
             int n = 0;
             if (gq < G) {
-                int pos = p.positions ? p.positions[gq] : p.pos_value;
+                int pos = LAYER && base == 0 ? first_pos : p.positions ? p.positions[gq] : p.pos_value;
                 if (pos < 0) pos = 0;
                 n = (pos + TILE_TOKENS) / TILE_TOKENS;
             }
@@ -536,7 +539,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         ts = p.tile_start;
     }
     __syncthreads();
-    const long long N = ts[G];
+    const int N = ts[G];  // (the host refuses caches of 2^31 rows or more)
 
     // ---- work slice of this worker ----
     // At most min(workers, N) workers take part, so that every participant owns at least one tile: the ticket
@@ -546,11 +549,12 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     const int wid = blockIdx.x * ATTN_GROUPS + group;
     if (PERSIST && blockIdx.x == 0 && tid == 0) {
         p.table_out[G + 1] = W;
-        p.table_out[G + 2] = (int)N;
+        p.table_out[G + 2] = N;
     }
     if (wid >= W && !copier) return;  // uniform for the worker; no CTA-wide barrier follows
     // Worker w takes the tiles [w * N / W, (w + 1) * N / W).
-    const long long lo = (long long)wid * N / W, hi = (long long)(wid + 1) * N / W;
+    const int n_each = N / W, n_over = N - n_each * W;  // (N < 2^26, W <= 1024)
+    const int lo = wid * n_each + wid * n_over / W, hi = (wid + 1) * n_each + (wid + 1) * n_over / W;
     int g;  // first sequence of the slice: largest g with tile_start[g] <= lo
     if (!PUBLISH && p.worker_g && !TQ_DBG_FACTOR) {
         g = p.worker_g[wid];
@@ -558,7 +562,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         int a = 0, b = G;  // invariant: tile_start[a] <= lo < tile_start[b]
         while (b - a > 1) {
             int mid = (a + b) >> 1;
-            if ((long long)ts[mid] <= lo) a = mid; else b = mid;
+            if (ts[mid] <= lo) a = mid; else b = mid;
         }
         g = a;
     }
@@ -567,7 +571,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     if (idle) g = 0;
     // ---- load cursor over the flat tile list (warp-uniform, advanced in step by every warp of the worker) ----
     // Tile counts and row numbers fit 32 bits (the host refuses caches of 2^31 rows or more).
-    const int lo_i = idle ? 0 : (int)lo, hi_i = idle ? 0 : (int)hi;
+    const int lo_i = idle ? 0 : lo, hi_i = idle ? 0 : hi;
     int cl_tile = lo_i;                         // next tile to load into shared memory
     int cl_g = g;
     int cl_gend = ts[g + 1];

@@ -31,10 +31,11 @@ static inline bool cluster_on() {
     static const bool on = !(getenv("TQ_CLUSTER") && atoi(getenv("TQ_CLUSTER")) == 0);
     return on;
 }
-// Calls without an engine: the streaming kernels' rotated queries, table and clears are launches of their own there (packed 9 us,
-// fp16 3).
+// Calls without an engine: the streaming kernels' clears and writes are launches of their own there for fp16 rows (3 us); packed, the
+// layer form has the same three, and the cluster form, which cannot start under the appends, is 3 us ahead in 2-bit only (2-bit
+// 32/4 heads 128 x 600 tokens 38.9 us a layer with the appends, streaming 40.9; 4-bit 32/4 48 x 2500 58.9 / 36.3, 16/8 64 x 1500 64.7 / 44.4).
 static inline bool compat_cluster_size(int bits, int G, int H, int Hkv, int max_tokens) {
-    return cluster_on() && cluster_layer_faster(bits, G, Hkv, H / Hkv, (long long)G * max_tokens, max_tokens, bits ? 9.0 : 3.0);
+    return cluster_on() && cluster_layer_faster(bits, G, Hkv, H / Hkv, (long long)G * max_tokens, max_tokens, bits == 4 ? 0.0 : 3.0);
 }
 
 extern "C" {
@@ -586,6 +587,22 @@ static int compat_cluster_attention(void* out, const void* q, const void* ck, co
     return launch_cluster_decode(bits, p, 1, 1, pos ? msl : pos_value + 1, s, use_pdl());
 }
 
+// The others with a streaming layout: the layer form without an append.
+static int compat_layer_attention(void* out, const void* q, const uint8_t* ck, const uint8_t* cv, const void* k_norms, const void* v_norms,
+                                  const void* rotation, const int* pos, int pos_value, int msl, int G, int H, int Hkv, int q_dim, int bits, void* ws,
+                                  size_t ws_bytes, cudaStream_t s) {
+    if (!q || !out || !ck || !cv || !k_norms || !v_norms || !rotation) return TQ_ERR_ARG;
+    FullWorkspace fw = carve_full(ws, G, H);
+    CUtensorMap tmK, tmV;
+    const int kvp = Hkv * (bits == 4 ? 64 : 32);
+    int r = cached_code_map(&tmK, ck, (long long)G * msl, kvp);
+    if (r == TQ_OK) r = cached_code_map(&tmV, cv, (long long)G * msl, kvp);
+    if (r != TQ_OK) return r;
+    LayerInputs in{q, nullptr, nullptr, rotation, 1, 0, fw.rot_t, nullptr};
+    return attention_impl(out, tmK, tmV, ck, cv, k_norms, v_norms, fw.rot_t, pos, pos_value, nullptr, (long long)G * msl, msl, G, H, Hkv, q_dim, bits,
+                          ws, ws_bytes, s, false, &in);
+}
+
 void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* ck_q, const uint8_t* cv_q,
                                       const void* k_norms, const void* v_norms, const void* rotation, float* as,
                                       const int* pos, int msl, int G, int num_heads, int num_kv_heads, int head_dim,
@@ -616,19 +633,8 @@ void launch_turbo_gqa_attention_batch(void* out, const void* q, const uint8_t* c
         r = compat_workspace(need, &ws, cs(s));
     }
     if (r == TQ_OK && one_launch && G <= FUSED_MAX_G && pos && layer_form_ok(q, nullptr, nullptr, q_dim)) {
-        // the layer form without an append
-        if (!q || !out || !ck_q || !cv_q || !k_norms || !v_norms || !rotation) r = TQ_ERR_ARG;
-        FullWorkspace fw = carve_full(ws, G, num_heads);
-        CUtensorMap tmK, tmV;
-        const int kvp = num_kv_heads * (bits == 4 ? 64 : 32);
-        if (r == TQ_OK) r = cached_code_map(&tmK, ck_q, (long long)G * msl, kvp);
-        if (r == TQ_OK) r = cached_code_map(&tmV, cv_q, (long long)G * msl, kvp);
-        if (r == TQ_OK) {
-            LayerInputs in{q, nullptr, nullptr, rotation, 1, 0, fw.rot_t, nullptr};
-            r = attention_impl(out, tmK, tmV, ck_q, cv_q, k_norms, v_norms, fw.rot_t, pos, -1, nullptr, (long long)G * msl, msl, G,
-                               num_heads, num_kv_heads, q_dim, bits, ws, need, cs(s), false, &in);
-        }
-        g_compat_status = r;
+        g_compat_status = compat_layer_attention(out, q, ck_q, cv_q, k_norms, v_norms, rotation, pos, -1, msl, G, num_heads, num_kv_heads, q_dim,
+                                                 bits, ws, need, cs(s));
         return;
     }
     if (r == TQ_OK)
@@ -667,6 +673,12 @@ void launch_turbo_gqa_attention(const void* q, const uint8_t* ck_q, const uint8_
     if (r == TQ_OK) {
         need = carve_full(nullptr, 1, num_heads).bytes;
         r = compat_workspace(need, &ws, cs(s));
+    }
+    static const bool layer_form = !(getenv("TQ_FUSED") && atoi(getenv("TQ_FUSED")) == 0);
+    if (r == TQ_OK && layer_form && layer_form_ok(q, nullptr, nullptr, q_dim)) {
+        g_compat_status = compat_layer_attention(output, q, ck_q, cv_q, k_norms, v_norms, rotation, nullptr, pos, msl, 1, num_heads, num_kv_heads,
+                                                 q_dim, bits, ws, need, cs(s));
+        return;
     }
     if (r == TQ_OK)
         r = append_impl(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, q, rotation, nullptr, pos, nullptr, 0, 0,
@@ -1492,7 +1504,7 @@ static bool engine_step_small(const tq_engine* e, StepInputs inputs) {
     if (!fast_shape(H, Hkv, e->kv_bits != 0)) return true;
     if (!cluster_on()) return false;
     const long long clusters = (long long)e->G * Hkv * NL;
-    const int S = cluster_split(e->kv_bits, clusters, heads, e->msl);
+    const int S = cluster_split(e->kv_bits, clusters, heads, e->msl, false);
     if (e->kv_bits == 0) {
         const double tiles = ((e->msl + 15) / 16) / (double)(CD_WARPS * S);
         return 600.0 * tiles + 2.0 * clusters + 0.002 * (double)e->total_rows * Hkv * NL < 2000.0 + 10000.0 * NL;

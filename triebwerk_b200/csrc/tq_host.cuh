@@ -440,9 +440,11 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
 // hides the latency of the first one's loads: above 12 tiles 0.6 to 0.95 of the time (4 x 8192 tokens, 8 KV heads, 44 -> 28 us),
 // above 4 for fp16, whose rows are four times as long.  Not with more than 4 query heads per cluster in a packed mode: the warps'
 // partial results leave room for one CTA per SM there.
-inline int cluster_split(int bits, long long clusters, int heads, int max_tokens) {
+// Where those are one layer's (`layer`) and 4-bit, the next layer's clusters of 8 and 16 find no room either beside this one's: as many
+// as leave it half of the SMs (32/4 heads, 2 x 4000 tokens 17.1 -> 10.0 us, 2 x 8000 21.1 -> 13.9, 4 x 4000 20.1 -> 15.4).
+inline int cluster_split(int bits, long long clusters, int heads, int max_tokens, bool layer) {
     const long long sms = device_props().sm_count, blocks = (max_tokens + 15) / 16;
-    auto fit = [&](int n) { return sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
+    auto fit = [&](int n) { return n >= 8 && layer && bits == 4 && heads > 4 ? (sms - 20) / 2 : sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
     int S = 1;
     auto longer = [&](int n) { return n == 8 ? 2 * n * CD_WARPS <= blocks : n * CD_WARPS < blocks; };
     while (S < CD_MAX_CLUSTER && longer(S) && clusters * S * 2 <= fit(2 * S)) S *= 2;
@@ -454,8 +456,10 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
 // Is one layer faster in the cluster form than in the streaming one?  Both times, in us, are lines in what bounds them, measured
 // over 1 to 128 sequences of 64 to 16384 tokens, equal and ragged, and 8 KV heads of 2 and 4 query heads, 4 of 8.  Packed: the
 // cluster form 4.6 + 0.4 per tile of its longest warp + 0.3 more per turn of the SMs + 0.023 per 1000 rows and KV heads + 0.007 to
-// 0.009 per cluster, the streaming form 17.7 + 0.030 per 1000 rows and KV heads + 0.4 per 1000 tokens of the longest sequence;
-// where the two are within 3 us it is the streaming form.  fp16: a tile costs the cluster form 1 us more than the streaming form's
+// 0.009 per cluster, the streaming form 14.6 + 0.030 per 1000 rows and KV heads + 0.4 per 1000 tokens of the longest sequence.  Long
+// chains of tiles cost the cluster form more than those lines say, and with 8 heads in 4-bit, one CTA per SM, more turns: 12 tiles at
+// most, with many rows a few more (cluster / streaming: 4-bit 32/8 heads 8 x 8000 39.4 / 29.7 us, 2-bit 32/4 8 x 8000 29.3 / 21.4, 4-bit
+// 32/4 48 x 1023 26.0 / 21.5, 2 x 16000 23.3 / 21.5, 96 x 600 31.8 / 26.7, 24 x 1500 17.2 / 17.6).  fp16: a tile costs the cluster form 1 us more than the streaming form's
 // share of it where there is one turn, less with more turns and with 8 query heads,
 // and that form starts 7 us later.  Above 640 clusters their number counts for more than in the lines fitted below it (128 x 64
 // tokens, 16/8 heads, 4-bit 25.7 / 19.7 us, 96 x 64 19.8 / 19.0, 64 x 64 13.5 / 17.2; 32/8 heads 128 x 64 26.8 / 24.9, 96 x 64 20 / 23;
@@ -463,17 +467,18 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
 // `extra`: us the streaming form's launches cost on top.
 inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, double extra) {
     const long long clusters = (long long)G * Hkv, sms = device_props().sm_count;
-    const int S = cluster_split(bits, clusters, heads, max_tokens);
+    const int S = cluster_split(bits, clusters, heads, max_tokens, true);
     const double chain = ((max_tokens + 15) / 16) / (double)(S * CD_WARPS), turns = (double)((clusters * S + sms - 1) / sms);
     if (bits == 0) return (heads > 4 ? 0.5 : 1.0) * chain < 7.0 + 1.5 * turns + extra && !(clusters > 768 && chain > 2.0);
     const double many = heads > 2 ? 0.0015 * std::max(0ll, clusters - 800) : 0.02 * std::max(0ll, clusters - 640);
+    if (bits == 4 && heads > 4 ? chain * turns > 12.0 : chain > 12.0 + 5e-6 * (double)rows * Hkv) return false;
     return 0.4 * chain + 0.3 * chain * turns + 0.009 * clusters + many < 10.0 + 7e-6 * (double)rows * Hkv + 0.0004 * max_tokens + extra;
 }
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
 inline int cluster_launch_split(int bits, int G, int split_layers, int H, int Hkv, int max_tokens) {
     const int head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
     const bool one_per_sm = bits != 0 && !fast_shape(H, Hkv, true);  // (EXACT, packed: as with 8 heads)
-    return cluster_split(bits, (long long)G * split_layers * Hkv * head_blocks, one_per_sm ? CD_HEADS : std::min(CD_HEADS, H / Hkv), max_tokens);
+    return cluster_split(bits, (long long)G * split_layers * Hkv * head_blocks, one_per_sm ? CD_HEADS : std::min(CD_HEADS, H / Hkv), max_tokens, split_layers == 1);
 }
 template <bool HOST, bool EXACT>
 inline int launch_cluster_decode_e(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {

@@ -177,30 +177,48 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) layer_prep_kernel(const Layer
         }
         if (tid == 0 && !ok) atomicMax(p.status, ST_BAD_POSITION);
         __syncthreads();
-        // the code: how many bounds the coordinate has reached (NaN: as the reference's comparisons fall out)
-        auto search = [&](float y) -> uint32_t {
-            int n = 0;
+        // the codes: how many bounds a coordinate has reached (NaN: as the reference's comparisons fall out); value 4 r + e: row gl + 8 r,
+        // block e >> 1, coordinate 2 t4 + (e & 1) of it.  (All eight a step at a time: their look-ups are in flight together.)
+        auto search = [&](const float* y, auto count, uint32_t* n) {
+            constexpr int C = decltype(count)::value;
 #pragma unroll
-            for (int step = (NBND + 1) / 2; step > 0; step >>= 1)
-                if (y >= bound_s[n + step]) n += step;
-            return BITS == 4 && y != y ? 15u : (uint32_t)n;
+            for (int i = 0; i < C; ++i) n[i] = 0u;
+#pragma unroll
+            for (uint32_t step = (NBND + 1) / 2; step > 0; step >>= 1) {
+                float b[C];
+#pragma unroll
+                for (int i = 0; i < C; ++i) b[i] = bound_s[n[i] + step];
+#pragma unroll
+                for (int i = 0; i < C; ++i) n[i] += y[i] >= b[i] ? step : 0u;
+            }
+            if (BITS == 4) {
+#pragma unroll
+                for (int i = 0; i < C; ++i) n[i] = y[i] != y[i] ? 15u : n[i];
+            }
         };
-        uint32_t codes = 0u, near = 0u;  // nibble (bit) 4 r + e: row gl + 8 r, block e >> 1, coordinate 2 t4 + (e & 1) of it
+        float x[8];
+        uint32_t n8[8], codes = 0u, near = 0u, zeros = 0u;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const float inv = inv_s[gl + 8 * r], ss = ss_s[gl + 8 * r];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
+                const int i = 4 * r + e;
                 const float rot = c[e >> 1][0][2 * r + (e & 1)] + c[e >> 1][1][2 * r + (e & 1)];
-                float x = mul_ftz(rot, inv);
-                if (!(add_ftz(ss, 1e-12f) < 3.0e38f)) x = __int_as_float(0x7fc00000);  // an infinity or a NaN among the inputs: NaN everywhere, as in the reference
+                x[i] = mul_ftz(rot, inv);
+                if (!(add_ftz(ss, 1e-12f) < 3.0e38f)) x[i] = __int_as_float(0x7fc00000);  // an infinity or a NaN among the inputs: NaN everywhere, as in the reference
                 const bool zero = ss == 0.0f && rot == 0.0f;  // all zero: every coordinate is 0, on a bound but exact
-                if (zero) x = 0.0f;
-                const uint32_t n = search(x);
-                codes |= n << (4 * (4 * r + e));
-                if (!zero && fminf(x - bound_s[n], bound_s[n + 1] - x) < PREP_MARGIN && gl + 8 * r < nvec) near |= 1u << (4 * r + e);
+                if (zero) x[i] = 0.0f;
+                if (zero || gl + 8 * r >= nvec) zeros |= 1u << i;
             }
         }
+        search(x, std::integral_constant<int, 8>(), n8);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            codes |= n8[i] << (4 * i);
+            near |= fminf(x[i] - bound_s[n8[i]], bound_s[n8[i] + 1] - x[i]) < PREP_MARGIN ? 1u << i : 0u;
+        }
+        near &= ~zeros;
         while (near) {  // about 1 coordinate in 700: the reference's k-ascending chain
             const int at = __ffs((int)near) - 1, v = gl + 8 * (at >> 2), d = 8 * (2 * warp + ((at >> 1) & 1)) + 2 * t4 + (at & 1);
             near &= near - 1u;
@@ -218,7 +236,9 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) layer_prep_kernel(const Layer
                     acc = fma_ftz(rf.y, mul_ftz(xf.y, inv), acc);
                 }
             }
-            codes = (codes & ~(15u << (4 * at))) | search(acc) << (4 * at);
+            uint32_t n;
+            search(&acc, std::integral_constant<int, 1>(), &n);
+            codes = (codes & ~(15u << (4 * at))) | n << (4 * at);
         }
         __syncwarp();
 #pragma unroll
