@@ -305,6 +305,10 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         }
     };
 
+    auto ready = [&](uint32_t bar, uint32_t parity) {  // (two blocks: most waits are over when they are asked for)
+        if (MT == 1 || !mbar_try_wait(bar, parity)) wait_bar(bar, parity);
+    };
+
     // ---- once: tensor memory, barriers, table, queries, R ----
     if (warp == 0) {
         tmem_alloc(ctrl + 128u, 512u);
@@ -474,10 +478,16 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       } else if (warp == MMA_WARP) {
         // ================= one thread issues every product =================
         if (lane == 0) {
+            // (Two blocks: the products follow each other closely and this thread's own time counts: a wait on a barrier that is complete
+            // costs it 100 cycles and more, in which they run out.  So a slot's turn waits for K and V ahead of its weights, and the second
+            // slot, which shares them, does not: 8192 tokens, 32 heads, fp16 503 -> 478 us a layer, 4-bit 629 -> 607.  With one block a slot's next
+            // tile is two further on and not to be waited for before the values.)
             auto issue_scores = [&](int s, int i) {
                 const int j = tile_of(s, i), st = j % STAGES;
-                if (!DIRECT) wait_bar(bar_kfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
-                tc_fence_after();
+                if (MT == 1) {
+                    if (!DIRECT) wait_bar(bar_kfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
+                    tc_fence_after();
+                }
                 if (dead) return;
                 const uint32_t a = pft_lo_k(sb + PftSmem::Q + (MT == 2 ? s * PFT_TILE : 0u)), b = pft_lo_k(sb + PftSmem::K + st * PFT_TILE);
 #pragma unroll
@@ -494,9 +504,11 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             };
             auto issue_values = [&](int s, int i) {
                 const int j = tile_of(s, i), st = j % STAGES;
-                if (!DIRECT) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
-                wait_bar(bar_pfull + 8u * s, (uint32_t)(i & 1));
-                tc_fence_after();
+                if (MT == 1) {
+                    if (!DIRECT) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));
+                    wait_bar(bar_pfull + 8u * s, (uint32_t)(i & 1));
+                    tc_fence_after();
+                }
                 if (dead) return;
                 const uint32_t b = pft_lo_mn(sb + PftSmem::V + st * PFT_TILE);
 #pragma unroll
@@ -512,8 +524,31 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 if (MT == 1 || s == (j < n1 ? 1 : 0)) umma_commit(bar_vfree + 8u * (j & 1));
             };
             if (!PACKED) wait_bar(bar_q, 0u);
+            if (MT == 2) {  // (the first block has tiles)
+                if (!DIRECT) ready(bar_kfull, 0u);
+                tc_fence_after();
+            }
             if (n0 > 0) issue_scores(0, 0);
             if (n1 > 0) issue_scores(1, 0);
+            if constexpr (MT == 2) {
+                auto turn = [&](int s, int i, int n) {
+                    if (i >= n) return;
+                    if (!DIRECT && (s == 0 || i >= n0)) {
+                        ready(bar_vfull + 8u * (i & 1), (uint32_t)((i >> 1) & 1));
+                        if (i + 1 < n) ready(bar_kfull + 8u * ((i + 1) & 1), (uint32_t)(((i + 1) >> 1) & 1));
+                    } else if (!DIRECT && i + 1 < n && i + 1 >= n0) {  // (the first block ends here)
+                        ready(bar_kfull + 8u * ((i + 1) & 1), (uint32_t)(((i + 1) >> 1) & 1));
+                    }
+                    ready(bar_pfull + 8u * s, (uint32_t)(i & 1));
+                    tc_fence_after();
+                    issue_values(s, i);
+                    if (i + 1 < n) issue_scores(s, i + 1);
+                };
+                for (int i = 0; i < max(n0, n1); ++i) {
+                    turn(0, i, n0);
+                    turn(1, i, n1);
+                }
+            } else
             for (int i = 0; i < max(n0, n1); ++i) {
                 if (i < n0) {
                     issue_values(0, i);
@@ -554,8 +589,8 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};  // (sums: of this thread's columns)
         for (int i = 0; i < nt; ++i) {
             const int j = tile_of(slot, i), st = j % STAGES, col0 = j * PFT_KT;
-            if (PACKED && !DIRECT) wait_bar(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
-            wait_bar(bar_sfull + 8u * slot, (uint32_t)(i & 1));
+            if (PACKED && !DIRECT) ready(bar_vfull + 8u * (j & 1), (uint32_t)((j >> 1) & 1));  // (for the tile's norms)
+            ready(bar_sfull + 8u * slot, (uint32_t)(i & 1));
             tc_fence_after();
             const bool diagonal = col0 + PFT_KT - 1 > my_first;  // (uniform for the slot)
             const float2* const nrm = reinterpret_cast<const float2*>(gb + PftSmem::NORM + (uint32_t)st * PFT_NORM_BYTES) + t4;
