@@ -205,6 +205,11 @@ __device__ __forceinline__ void tmem_st_pack32(uint32_t taddr, const uint32_t (&
                  "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                  : "memory");
 }
+// Four 8 x 8 matrices of halves to shared memory: lane l holds (row l / 4, columns 2 (l % 4), + 1) of each and names the address of row
+// l % 8 of matrix l / 8 (16 bytes).
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // The same products with the descriptors as their low words; the high word is common to all operand tiles of this kernel (groups
 // of 8 rows 1024 bytes apart, descriptor version, 128-byte swizzle).  Few registers, few instructions: the thread that issues
@@ -356,11 +361,25 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     // softmax warps: slot, 16 score rows (= tensor-memory lanes) row0 ..; a thread's rows row0 + g and row0 + g + 8
     const int slot = (warp >> 2) & 1, row0 = 32 * (warp & 3) + 16 * (warp >> 3), g = lane >> 2, t4 = lane & 3;
     const int my_first = q0 + (MT == 2 ? slot * QT : 0);
-    auto token_of = [&](int row) { return row / GRP < QT ? my_first + row / GRP : p.T; };  // (p.T: a row of no query)
+    // row / GRP by a multiplication, exact below 128; (made anew where it is used: not live through the tiles)
+    auto make_by_grp = [&]() {
+        uint32_t d = (uint32_t)GRP;
+        asm volatile("" : "+r"(d));
+        return (65536u + d - 1u) / d;
+    };
+    auto token_in = [&](int row, uint32_t by_grp) { return (int)(((uint32_t)row * by_grp) >> 16); };
+    auto token_of = [&](int row, uint32_t by_grp) { return token_in(row, by_grp) < QT ? my_first + token_in(row, by_grp) : p.T; };  // (p.T: a row of no query)
     const uint32_t my_lanes = tmem + ((uint32_t)row0 << 16);
-    // a pair of columns (c, c + 1) of a row of an operand tile
-    auto put_pair = [&](uint32_t tile, int row, int c, float x, float y) {
-        *reinterpret_cast<uint32_t*>(gb + tile + pft_chunk(row, c >> 3) + (uint32_t)(c & 7) * 2u) = pack_half2(x, y);
+    // the warp's rows, columns c0 .. c0 + 63, of an operand tile from a 64-column fragment.  (Pair by pair, with 32 columns of
+    // tensor memory at a time and a division per stored row, the way from the last tile to the end took 3.4 us.)
+    auto put_frag = [&](uint32_t tile, int c0, const float (&y)[32]) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                auto two = [&](int b) { return pack_half2(y[4 * b + 2 * h], y[4 * b + 2 * h + 1]); };
+                stmatrix_x4(sb + tile + pft_chunk(row0 + 8 * h + (lane & 7), (c0 >> 3) + j + (lane >> 3)), two(j), two(j + 1), two(j + 2), two(j + 3));
+            }
     };
     // in the products before and after the tiles a warp takes 128 columns of its slot's rows, or with one query block, whose rows
     // both slots' warps share, 64
@@ -417,19 +436,19 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             wait_bar(bar_rot, 0u);
             tc_fence_after();
 #pragma unroll 1
-            for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 32) {
-                uint32_t r[16];
-                tmem_ld_frag32(my_lanes + 128u * pslot + (uint32_t)c0, r);
+            for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 64) {
+                uint32_t r[32];
+                tmem_ld_frag64(my_lanes + 128u * pslot + (uint32_t)c0, r);
                 tmem_ld_wait();
+                float y[32];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int e = 0; e < 32; ++e) y[e] = __uint_as_float(r[e]) * PFT_SCALE;
+                put_frag(PftSmem::Q + pslot * PFT_TILE, c0, y);
+                if (LOW) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float q0 = __uint_as_float(r[4 * j + 2 * h]) * PFT_SCALE, q1 = __uint_as_float(r[4 * j + 2 * h + 1]) * PFT_SCALE;
-                        put_pair(PftSmem::Q + pslot * PFT_TILE, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, q0, q1);
-                        if (LOW)
-                            put_pair(PftSmem::Q + PFT_TILE, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, low_part(q0), low_part(q1));
-                    }
+                    for (int e = 0; e < 32; ++e) y[e] = low_part(y[e]);
+                    put_frag(PftSmem::Q + PFT_TILE, c0, y);
+                }
             }
         }
         if (warp < PFT_SOFT_WARPS || warp == MMA_WARP) {  // the rotated queries are in place (the copies of the first tiles are on their way already)
@@ -585,7 +604,8 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         regs_inc<PFT_REGS_SOFT>();
         const uint32_t s_col = my_lanes + 128u * slot, o_col = my_lanes + 256u + 128u * slot;
         const int nt = slot ? n1 : n0;
-        const int tok0 = token_of(row0 + g), tok1 = token_of(row0 + g + 8);
+        const uint32_t by_grp0 = make_by_grp();
+        const int tok0 = token_of(row0 + g, by_grp0), tok1 = token_of(row0 + g + 8, by_grp0);
         float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.0f, 0.0f};  // (sums: of this thread's columns)
         for (int i = 0; i < nt; ++i) {
             const int j = tile_of(slot, i), st = j % STAGES, col0 = j * PFT_KT;
@@ -729,36 +749,30 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             for (int h = 0; h < 2; ++h) w0[h] = 1.0f / (l_run[h] + 1e-8f);
         }
         const bool has_rows = MT == 1 || nt > 0;
-        auto result = [&](int c0, float (&y)[16]) {  // columns c0 .. c0 + 31, normalised, in fragment order
-            uint32_t r[16];
-            tmem_ld_frag32((MT == 2 ? o_col : my_lanes + 256u) + (uint32_t)c0, r);
+        auto result = [&](int c0, float (&y)[32]) {  // columns c0 .. c0 + 63, normalised, in fragment order
+            uint32_t r[32];
+            tmem_ld_frag64((MT == 2 ? o_col : my_lanes + 256u) + (uint32_t)c0, r);
             tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(r[e]) * w0[(e >> 1) & 1];
+            for (int e = 0; e < 32; ++e) y[e] = __uint_as_float(r[e]) * w0[(e >> 1) & 1];
             if (MT == 1 && n1 > 0) {
-                tmem_ld_frag32(my_lanes + 384u + (uint32_t)c0, r);
+                tmem_ld_frag64(my_lanes + 384u + (uint32_t)c0, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 16; ++e) y[e] = fmaf(__uint_as_float(r[e]), w1[(e >> 1) & 1], y[e]);
+                for (int e = 0; e < 32; ++e) y[e] = fmaf(__uint_as_float(r[e]), w1[(e >> 1) & 1], y[e]);
             }
-        };
-        auto put_frag = [&](uint32_t tile, int c0, const float (&y)[16]) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) put_pair(tile, row0 + g + 8 * h, c0 + 8 * j + 2 * t4, y[4 * j + 2 * h], y[4 * j + 2 * h + 1]);
         };
         const uint32_t qtile = PftSmem::Q + pslot * PFT_TILE, ktile = PftSmem::K + pslot * PFT_TILE;
         if constexpr (PACKED) {
             // out[d] = sum_k R[k][d] * acc[k]: the normalised rows, split into fp16 high and low parts, over the Q and K tiles
             if (has_rows) {
 #pragma unroll 1
-                for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 32) {
-                    float y[16];
+                for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 64) {
+                    float y[32];
                     result(c0, y);
                     put_frag(qtile, c0, y);
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) y[e] = low_part(y[e]);
+                    for (int e = 0; e < 32; ++e) y[e] = low_part(y[e]);
                     put_frag(ktile, c0, y);
                 }
             }
@@ -771,14 +785,14 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         if (has_rows) {
             // the finished values as fp16 through the (consumed) query tile, so that 16 lanes store 256 contiguous bytes of a row
 #pragma unroll 1
-            for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 32) {
-                float y[16];
+            for (int c0 = pcol0; c0 < pcol0 + PCOLS; c0 += 64) {
+                float y[32];
                 if constexpr (PACKED) {
-                    uint32_t r[16];
-                    tmem_ld_frag32(my_lanes + 128u * pslot + (uint32_t)c0, r);
+                    uint32_t r[32];
+                    tmem_ld_frag64(my_lanes + 128u * pslot + (uint32_t)c0, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(r[e]);
+                    for (int e = 0; e < 32; ++e) y[e] = __uint_as_float(r[e]);
                 } else {
                     result(c0, y);
                 }
@@ -786,12 +800,13 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             }
             __syncwarp();
             constexpr int CH = PCOLS / 8;  // 16-byte pieces per row
+            const uint32_t by_grp = make_by_grp();
 #pragma unroll
             for (int k = 0; k < CH / 2; ++k) {
-                const int at = 32 * k + lane, row = row0 + at / CH, ch = (pcol0 >> 3) + at % CH, tok = token_of(row);
+                const int at = 32 * k + lane, row = row0 + at / CH, ch = (pcol0 >> 3) + at % CH, tok = token_of(row, by_grp);
                 if (tok < p.T) {
                     const uint4 u = *reinterpret_cast<const uint4*>(gb + qtile + pft_chunk(row, ch));
-                    *(reinterpret_cast<uint4*>(out_seq + (size_t)tok * p.q_dim + (size_t)(kvh * GRP + row % GRP) * HEAD_DIM) + ch) = u;
+                    *(reinterpret_cast<uint4*>(out_seq + (size_t)tok * p.q_dim + (size_t)(kvh * GRP + row - token_in(row, by_grp) * GRP) * HEAD_DIM) + ch) = u;
                 }
             }
         }
