@@ -400,6 +400,24 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
 
     // The reference's k-ascending fp32 chain for coordinate d of one vector (x: its 128 fp16 inputs in global memory),
     // by one thread; R comes from the operand tile in shared memory.
+    // chain_in_tile: the vector too, which is row `row` there.
+    auto chain_in_tile = [&](int row, float inv, int d) -> int {
+        float acc = 0.0f;
+#pragma unroll 4
+        for (int j = 0; j < 16; ++j) {
+            const uint4 xv = *reinterpret_cast<const uint4*>(gbase + tc_operand_addr(TcSmem::A_X, row, 8 * j));
+            const uint4 rv = *reinterpret_cast<const uint4*>(gbase + tc_operand_addr(TcSmem::B_R, d, 8 * j));
+            const __half2* xh = reinterpret_cast<const __half2*>(&xv);
+            const __half2* rh = reinterpret_cast<const __half2*>(&rv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 xf = __half22float2(xh[e]), rf = __half22float2(rh[e]);
+                acc = fma_ftz(rf.x, mul_ftz(xf.x, inv), acc);
+                acc = fma_ftz(rf.y, mul_ftz(xf.y, inv), acc);
+            }
+        }
+        return quantize_code(acc, bits);
+    };
     auto exact_code = [&](const __half* x, float inv, int d) -> int {
         const uint4* src = reinterpret_cast<const uint4*>(x);
         float acc = 0.0f;
@@ -459,7 +477,8 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                 const uint32_t item = list_s[i];
                 const int v = (int)(item >> 8), d = (int)(item & 255u);
                 const long long dst = dst_s[v];
-                if (dst >= 0) patch(cq + dst, d, exact_code(vector_input(kind, vec0 + v), inv_s[v], d));
+                // (a CTA's last tile stays in the operand tile: its chains, the tail of a prompt of a few tiles, need no trip to memory)
+                if (dst >= 0) patch(cq + dst, d, tile + (int)gridDim.x >= total_tiles ? chain_in_tile(v, inv_s[v], d) : exact_code(vector_input(kind, vec0 + v), inv_s[v], d));
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty + 8u * (uint32_t)b);
