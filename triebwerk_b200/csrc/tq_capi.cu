@@ -1790,7 +1790,7 @@ int tq_fold_rotation_into_projection(void* w_out, const void* w_in, const void* 
 // Prompts of n_seq consecutive sequences (first_seq ..), all T tokens long and all at positions first_pos ..; inputs
 // [n_seq][T][kv_dim].  One launch.
 static int engine_prefill_impl(tq_engine* e, int layer, int first_seq, int n_seq, const void* k, const void* v, int first_pos,
-                               int T, tq_stream_t s) {
+                               int T, tq_stream_t s, PrefillRows* rows = nullptr) {
     if (e) e->chain_ok = false;  // not a fused decode launch: the next one reads nothing early
     if (!e || layer < 0 || layer >= e->shape.num_layers || !k || !v || T <= 0 || first_pos < 0 || n_seq <= 0) return TQ_ERR_ARG;
     if (e->asleep || !e->arena || e->G == 0 || !engine_on_its_device(e)) return TQ_ERR_STATE;
@@ -1839,10 +1839,26 @@ static int engine_prefill_impl(tq_engine* e, int layer, int first_seq, int n_seq
     p.max_seq_len = e->msl; p.capacity_rows = cap;
     p.n_src = T; p.H = e->shape.num_heads; p.Hkv = e->shape.num_kv_heads; p.q_dim = e->q_dim(); p.kv_dim = e->kv_dim();
     p.bits = e->kv_bits; p.pos_value = first_pos;
-    if (n_seq == 1) return launch_append(p, cs(s), use_pdl());
+    if (n_seq == 1) return launch_append(p, cs(s), use_pdl(), rows);
     if ((long long)n_seq * T * p.Hkv >= (1ll << 31)) return TQ_ERR_CAPACITY;
     // several sequences: the tensor-core kernel takes them in one launch (whatever their number of head vectors)
-    return launch_prefill_tc(p, cs(s), use_pdl(), n_seq, e->msl, e->rb() ? e->rb() + first_seq : nullptr);
+    return launch_prefill_tc(p, cs(s), use_pdl(), n_seq, e->msl, e->rb() ? e->rb() + first_seq : nullptr, rows);
+}
+
+// May the append of these prompts make the attention's rows as well?  They fit the scratch as a whole, a tile of the append (128 / Hkv
+// tokens) is of one prompt, and the attention takes the call and is not the one that converts codes itself.  Up to 4096 tokens of 8 KV
+// heads, where the launch in between and its wait count for more than the append's slower stores (16/8 heads, 4-bit, with the rows made in a
+// launch of their own / by the append: 300 tokens 22.9 / 21.5 us a layer, 777 29.9 / 28.3, 1200 35.3 / 32.8, 2048 51.4 / 48.5, 4 x 1024 62.1 / 60.7; 2-bit 8 x 1024
+// 114 / 116, 32/8 8192 621 / 619).
+static bool engine_prefill_makes_rows(const tq_engine* e, int first_seq, int n_seq, const void* q, const void* out, int T, int q_stride) {
+    const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
+    if (first_seq < 0 || n_seq <= 0 || first_seq + n_seq > e->G) return false;
+    for (int i = 0; i < n_seq; ++i)
+        if (e->prefix_tokens[first_seq + i] > 0) return false;
+    return e->kv_bits != 0 && !e->asleep && e->arena && e->prefill_scratch && T > PFT_KT && 8 % Hkv == 0 && prefill_tc_on() &&
+           (n_seq == 1 || T % (TC_TILE / Hkv) == 0) && !prefill_exact(e->kv_bits, H, Hkv) && prefill_attn_shape(H, Hkv) &&
+           (((uintptr_t)q | (uintptr_t)out) & 15u) == 0 && q_stride >= H * HEAD_DIM && (q_stride & 7) == 0 &&
+           (long long)n_seq * T * Hkv <= 32768 && (size_t)n_seq <= e->prefill_scratch_bytes / prefill_scratch_bytes(T, Hkv, false);
 }
 
 // A prompt of T tokens shared by the sequences first_seq .. first_seq + n_seq - 1 (rollouts of one prompt: the
@@ -1915,7 +1931,39 @@ int tq_engine_prefill_append_batch(tq_engine* e, int layer, int first_seq, int n
 int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_seq, const void* q, const void* k, const void* v,
                                   void* out, int T, int q_stride, tq_stream_t s) {
     if (!e || !q || !out) return TQ_ERR_ARG;
-    int r = engine_prefill_impl(e, layer, first_seq, n_seq, k, v, 0, T, s);
+    // calls on several streams take turns in the engine's scratch
+    std::unique_lock<std::mutex> lock(e->prefill_mutex, std::defer_lock);
+    bool ordered = false;
+    unsigned long long id = 0;
+    auto take_scratch = [&]() -> int {
+        lock.lock();
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        TQ_CUDA(cudaStreamIsCapturing(cs(s), &capture));
+        ordered = capture == cudaStreamCaptureStatusNone;  // (a captured call runs when its graph does: the caller orders that)
+        if (ordered) {
+            TQ_CUDA(cudaStreamGetId(cs(s), &id));
+            if (!e->ev_prefill) TQ_CUDA(cudaEventCreateWithFlags(&e->ev_prefill, cudaEventDisableTiming));
+            if (e->prefill_stream_id != 0 && e->prefill_stream_id != id) TQ_CUDA(cudaStreamWaitEvent(cs(s), e->ev_prefill, 0));
+        }
+        return TQ_OK;
+    };
+    auto leave_scratch = [&]() -> int {
+        if (ordered) {
+            TQ_CUDA(cudaEventRecord(e->ev_prefill, cs(s)));
+            e->prefill_stream_id = id;
+        }
+        return TQ_OK;
+    };
+    PrefillRows rows{};
+    int r = TQ_OK;
+    const bool makes_rows = engine_on_its_device(e) && engine_prefill_makes_rows(e, first_seq, n_seq, q, out, T, q_stride);
+    if (makes_rows) {
+        const PrefillScratch c = prefill_rows_in(e->prefill_scratch, n_seq, T, e->shape.num_kv_heads, false);
+        rows.k16 = c.k16; rows.v16 = c.v16; rows.norms = c.norms; rows.tiles = prefill_tiles(T);
+        r = take_scratch();
+        if (r != TQ_OK) return r;
+    }
+    r = engine_prefill_impl(e, layer, first_seq, n_seq, k, v, 0, T, s, makes_rows ? &rows : nullptr);
     if (r != TQ_OK) return r;
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
     if (q_stride < H * HEAD_DIM || (q_stride & 7) != 0) return TQ_ERR_ARG;
@@ -1972,22 +2020,13 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
         return r != TQ_OK ? r : launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, ws, least, cs(s));
     }
     if (e->kv_bits == 0) return launch_prefill_attention(0, ap, e->total_rows - row0, nullptr, 0, cs(s));
-    std::lock_guard<std::mutex> lock(e->prefill_mutex);
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    TQ_CUDA(cudaStreamIsCapturing(cs(s), &capture));
-    const bool ordered = capture == cudaStreamCaptureStatusNone;  // (a captured call runs when its graph does: the caller orders that)
-    unsigned long long id = 0;
-    if (ordered) {
-        TQ_CUDA(cudaStreamGetId(cs(s), &id));
-        if (!e->ev_prefill) TQ_CUDA(cudaEventCreateWithFlags(&e->ev_prefill, cudaEventDisableTiming));
-        if (e->prefill_stream_id != 0 && e->prefill_stream_id != id) TQ_CUDA(cudaStreamWaitEvent(cs(s), e->ev_prefill, 0));
+    if (!makes_rows) {
+        r = take_scratch();
+        if (r != TQ_OK) return r;
     }
-    r = launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s));
-    if (ordered) {
-        TQ_CUDA(cudaEventRecord(e->ev_prefill, cs(s)));
-        e->prefill_stream_id = id;
-    }
-    return r;
+    r = launch_prefill_attention(e->kv_bits, ap, e->total_rows - row0, e->prefill_scratch, e->prefill_scratch_bytes, cs(s), rows.made);
+    const int left = leave_scratch();
+    return r != TQ_OK ? r : left;
 }
 
 int tq_engine_prefill_layer(tq_engine* e, int layer, int seq, const void* q, const void* k, const void* v, void* out, int T,

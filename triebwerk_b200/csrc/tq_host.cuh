@@ -237,7 +237,8 @@ inline int launch_append_t(const AppendParams& p, dim3 grid, cudaStream_t s, boo
 // Whole prompts (token form, K and/or V, no queries) go to the tensor-core kernel; TQ_PREFILL_TC=0 keeps them on
 // the fp32-chain kernel.  Both store the same bytes.
 // producer: the form that applies QK-norm and rotary embedding to the K vectors on the way in (PrefillTcParams)
-inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bool pdl, bool producer = false) {
+// rows_made: set where the launch makes the rows and norms that t.k16 asks for as well (ROWS16)
+inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bool pdl, bool producer = false, bool* rows_made = nullptr) {
     const long long tokens = (long long)t.n_seq * t.T;
     const long long tiles = ((tokens * t.Hkv + TC_TILE - 1) / TC_TILE) * ((t.k_buf ? 1 : 0) + (t.v_buf ? 1 : 0));
     long long grid = (long long)(producer ? 2 : TC_CTAS_PER_SM) * device_props().sm_count;
@@ -250,11 +251,16 @@ inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bo
     bool tma = !producer && tma_allowed;
     if (tma && t.k_buf) tma = make_append_input_map(&tmk, t.k_buf, tokens, t.Hkv, t.kv_dim) == TQ_OK;
     if (tma && t.v_buf) tma = make_append_input_map(&tmv, t.v_buf, tokens, t.Hkv, t.kv_dim) == TQ_OK;
-    const void* kernel = producer ? (const void*)prefill_append_tc_kernel<true, false>
-                                  : (tma ? (const void*)prefill_append_tc_kernel<false, true> : (const void*)prefill_append_tc_kernel<false, false>);
-    int ar = ensure_dynamic_smem(kernel, TC_DYN_SMEM);
-    if (ar != TQ_OK) return ar;
     PrefillTcParams ts = t;
+    const bool rows16 = tma && rows_made && t.k16;
+    if (rows_made) *rows_made = rows16;
+    if (rows16) grid = std::min<long long>(tiles, 2ll * device_props().sm_count);
+    const size_t smem = rows16 ? (size_t)TC_ROWS_END : TC_DYN_SMEM;
+    const void* kernel = producer ? (const void*)prefill_append_tc_kernel<true, false>
+                         : rows16 ? (const void*)prefill_append_tc_kernel<false, true, true>
+                                  : (tma ? (const void*)prefill_append_tc_kernel<false, true> : (const void*)prefill_append_tc_kernel<false, false>);
+    int ar = ensure_dynamic_smem(kernel, smem);
+    if (ar != TQ_OK) return ar;
 #ifdef TQ_TIMING_SWITCHES
     static unsigned long long* d_stamps = nullptr;
     static int stamp_calls = 0;
@@ -266,7 +272,7 @@ inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bo
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = TC_DYN_SMEM;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -275,6 +281,7 @@ inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bo
     cfg.numAttrs = pdl ? 1 : 0;
     cudaError_t le;
     if (producer) le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<true, false>, tmk, tmv, ts);
+    else if (rows16) le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<false, true, true>, tmk, tmv, ts);
     else if (tma) le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<false, true>, tmk, tmv, ts);
     else le = cudaLaunchKernelEx(&cfg, prefill_append_tc_kernel<false, false>, tmk, tmv, ts);
     if (le != cudaSuccess) return (int)le;
@@ -295,8 +302,16 @@ inline int launch_prefill_tc_params(const PrefillTcParams& t, cudaStream_t s, bo
     return cuda_status(cudaGetLastError());
 }
 
+// Where a packed prompt's rows as fp16 and its norms go (PrefillTcParams), and whether the append made them.
+struct PrefillRows {
+    __half* k16;
+    __half* v16;
+    float* norms;
+    int tiles;
+    bool made;
+};
 inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, bool pdl, int n_seq = 1, long long seq_stride_rows = 0,
-                             const long long* seq_row_base = nullptr) {
+                             const long long* seq_row_base = nullptr, PrefillRows* rows = nullptr) {
     PrefillTcParams t{};
     t.ck = p.ck; t.kn = p.kn; t.cv = p.cv; t.vn = p.vn;
     t.k_buf = p.k_buf; t.v_buf = p.v_buf; t.rotation = p.rotation; t.positions = p.positions; t.pos_value = p.pos_value; t.status = p.status;
@@ -304,16 +319,21 @@ inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, bool pdl, in
     t.seq_stride_rows = seq_stride_rows; t.row_base = seq_row_base; t.n_seq = n_seq;
     t.T = p.n_src; t.Hkv = p.Hkv; t.kv_dim = p.kv_dim; t.bits = p.bits;
     t.static_rotation = p.rot_prep ? 1 : 0;  // (the engine's own R)
-    return launch_prefill_tc_params(t, s, pdl);
+    if (rows) { t.k16 = rows->k16; t.v16 = rows->v16; t.norms = rows->norms; t.norm_tiles = rows->tiles; }
+    return launch_prefill_tc_params(t, s, pdl, false, rows ? &rows->made : nullptr);
 }
 
-inline int launch_append(const AppendParams& p, cudaStream_t s, bool pdl = false) {
-    static const bool prefill_tc = !(getenv("TQ_PREFILL_TC") && atoi(getenv("TQ_PREFILL_TC")) == 0);
+inline bool prefill_tc_on() {
+    static const bool on = !(getenv("TQ_PREFILL_TC") && atoi(getenv("TQ_PREFILL_TC")) == 0);
+    return on;
+}
+inline int launch_append(const AppendParams& p, cudaStream_t s, bool pdl = false, PrefillRows* rows = nullptr) {
+    const bool prefill_tc = prefill_tc_on();
     // (the tensor-core kernel moves 16 bytes at a time: every array it touches has to be 16-byte aligned)
     const uintptr_t align_or = (uintptr_t)p.k_buf | (uintptr_t)p.v_buf | (uintptr_t)p.ck | (uintptr_t)p.cv | (uintptr_t)p.rotation;
     if (prefill_tc && p.token_mode && !p.q && (p.k_buf || p.v_buf) && (align_or & 15u) == 0 &&
         p.kv_dim == p.Hkv * HEAD_DIM && (long long)p.n_src * p.Hkv >= 4 * TC_TILE && (long long)p.n_src * p.Hkv < (1ll << 31))
-        return launch_prefill_tc(p, s, pdl);
+        return launch_prefill_tc(p, s, pdl, 1, 0, nullptr, rows);
     const int nk = p.k_buf ? p.Hkv : 0, nv = p.v_buf ? p.Hkv : 0, nq = p.q ? p.H : 0;
     const long long total = (long long)p.n_src * (nk + nv + nq);
     const bool tables = p.tile_start != nullptr && !p.token_mode;
@@ -594,7 +614,21 @@ inline size_t prefill_scratch_bytes(int T, int Hkv, bool exact) {
 // Causal prefill attention.  `total_rows`: rows of the arrays ck and cv point into (from where they point); `scratch`: packed
 // modes, device memory for at least one KV head of one prompt (prompts go through it in groups; one that is too long for it as a
 // whole, some of its KV heads at a time).  Prompts of one tile need none: their blocks convert the codes themselves.
-inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long total_rows, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+// rows_made: the append has left the rows and norms of all prompts in the scratch (prefill_rows_in).
+struct PrefillScratch {
+    __half* k16;
+    __half* v16;
+    float* norms;
+    long long rows;  // of each array, low parts included
+};
+inline PrefillScratch prefill_rows_in(void* scratch, int n_seq, int T, int Hkv, bool low) {
+    PrefillScratch c{};
+    c.rows = (long long)n_seq * T * (low ? 2 : 1);
+    const size_t bytes = align_up((size_t)c.rows * Hkv * HEAD_DIM * sizeof(__half), 256);
+    c.k16 = (__half*)scratch; c.v16 = (__half*)((char*)scratch + bytes); c.norms = (float*)((char*)scratch + 2 * bytes);
+    return c;
+}
+inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long total_rows, void* scratch, size_t scratch_bytes, cudaStream_t s, bool rows_made = false) {
     p.grp = p.H / p.Hkv;
     const bool exact = prefill_exact(bits, p.H, p.Hkv), low = exact && bits != 0;
     if (p.n_seq <= 0) p.n_seq = 1;
@@ -635,15 +669,17 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
                 d.kn = p.kn + rows * p.Hkv + h0; d.vn = p.vn + rows * p.Hkv + h0;
                 d.row_base = p.row_base ? p.row_base + s0 : nullptr;
                 d.seq_rows = p.seq_rows; d.T = p.T; d.tiles = prefill_tiles(p.T); d.Hkv = a.Hkv; d.row_heads = p.Hkv;
-                const long long rows_hi = (long long)a.n_seq * p.T, rows_all = low ? 2 * rows_hi : rows_hi;  // the low parts behind the high ones
-                const size_t rows16 = align_up((size_t)rows_all * kv_dim * sizeof(__half), 256);
+                const long long rows_hi = (long long)a.n_seq * p.T;  // the low parts behind the high ones
+                const PrefillScratch c = prefill_rows_in(scratch, a.n_seq, p.T, a.Hkv, low);
+                const long long rows_all = c.rows;
                 d.low = rows_hi * kv_dim;
-                d.k16 = (__half*)scratch; d.v16 = (__half*)((char*)scratch + rows16); d.norms = (float*)((char*)scratch + 2 * rows16);
+                d.k16 = c.k16; d.v16 = c.v16; d.norms = c.norms;
                 const long long pieces = 2ll * p.T * a.Hkv * 16;
                 d.code_blocks = (int)std::min<long long>((pieces + 1023) / 1024, 8ll * device_props().sm_count);
                 const int norm_blocks = (int)std::min<long long>(((long long)a.Hkv * d.tiles + 7) / 8, device_props().sm_count);
                 const dim3 grid((unsigned)(d.code_blocks + norm_blocks), (unsigned)a.n_seq);
-                if (low) r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4, true>, grid, dim3(256), 0, s, true, d)
+                if (rows_made) r = TQ_OK;
+                else if (low) r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4, true>, grid, dim3(256), 0, s, true, d)
                                        : launch_kernel(dequantize_rows_kernel<2, true>, grid, dim3(256), 0, s, true, d);
                 else r = bits == 4 ? launch_kernel(dequantize_rows_kernel<4, false>, grid, dim3(256), 0, s, true, d)
                                    : launch_kernel(dequantize_rows_kernel<2, false>, grid, dim3(256), 0, s, true, d);

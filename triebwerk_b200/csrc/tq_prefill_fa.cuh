@@ -38,11 +38,9 @@
 namespace tq {
 
 constexpr int PFT_ROWS = 128;     // score rows of a slot
-constexpr int PFT_KT = 128;       // cache rows per tile
 constexpr float PFT_SLACK = 4.0f;
 constexpr float PFT_SCALE = 0.12751743074602467f;  // log2(e) / sqrt(128); packed forms: carried by the rotated queries
 constexpr uint32_t PFT_TILE = 32768u;  // an operand tile: [2 halves of the coordinates][128 rows][128 B]
-constexpr int PFT_NORMS = 2 * PFT_KT + 4;  // floats per tile of a packed cache: K norms, V norms, the largest V norm, padding to 16 bytes
 constexpr uint32_t PFT_NORM_BYTES = PFT_NORMS * 4u;
 
 constexpr int PFT_SOFT_WARPS = 16;
@@ -134,7 +132,8 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const DequantParam
                 top = max(top, __float_as_uint(vn));
             }
             top = __reduce_max_sync(0xffffffffu, top);
-            if (lane == 0) dst[2 * PFT_KT] = __uint_as_float(top);
+            // (as a half, exactly; what is not a number stays above the infinity)
+            if (lane == 0) *reinterpret_cast<uint4*>(dst + 2 * PFT_KT) = make_uint4(__half_as_ushort(__float2half_rn(__uint_as_float(top))), 0u, 0u, 0u);
         }
         return;
     }
@@ -614,7 +613,14 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             tc_fence_after();
             const bool diagonal = col0 + PFT_KT - 1 > my_first;  // (uniform for the slot)
             const float2* const nrm = reinterpret_cast<const float2*>(gb + PftSmem::NORM + (uint32_t)st * PFT_NORM_BYTES) + t4;
-            const float v_top = PACKED ? *reinterpret_cast<const float*>(gb + PftSmem::NORM + (uint32_t)st * PFT_NORM_BYTES + 8u * PFT_KT) : 0.0f;
+            float v_top = 0.0f;  // the tile's largest V norm: one word, or the largest of eight halves
+            if constexpr (DIRECT != 0) {
+                v_top = *reinterpret_cast<const float*>(gb + PftSmem::NORM + 8u * PFT_KT);
+            } else if constexpr (PACKED) {
+                const uint4 u = *reinterpret_cast<const uint4*>(gb + PftSmem::NORM + (uint32_t)st * PFT_NORM_BYTES + 8u * PFT_KT);
+                const uint32_t m = __vmaxu2(__vmaxu2(u.x, u.y), __vmaxu2(u.z, u.w));
+                v_top = __half2float(__ushort_as_half((unsigned short)max(m & 0xffffu, m >> 16)));
+            }
             // ---- scores, scaled (packed: by the K norms), masked; row maxima ----
             uint32_t sr[2][32];
             tmem_ld_frag64(s_col, sr[0]);

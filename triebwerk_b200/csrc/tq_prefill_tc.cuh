@@ -70,9 +70,17 @@ struct TcSmem {
     static constexpr uint32_t END = LIST1 + 4 * TC_LIST_CAP;
 };
 static_assert(TcSmem::CTRL + 64 <= TcSmem::GRID, "control words run into the bucket table");
+// ROWS16 (below): byte (4-bit) or nibble (2-bit) -> two centroids, eight copies; the largest V norm of each head in the tile
+constexpr uint32_t TC_ROWS_LUT = 0x13000, TC_ROWS_TOP = TC_ROWS_LUT + 8192, TC_ROWS_END = TC_ROWS_TOP + 32;
+static_assert(TcSmem::END <= TC_ROWS_LUT, "the rows' table runs into the queues");
 constexpr size_t TC_DYN_SMEM = TcSmem::END;  // enough wherever the dynamic shared memory starts at or below TcSmem::DST0
 constexpr int TC_CTAS_PER_SM = 3;
 static_assert(TC_CTAS_PER_SM * (TC_DYN_SMEM + 1024) <= 228 * 1024, "three CTAs of the tensor-core append must fit one SM");
+
+// Norms of a packed prompt for the prefill attention (tq_prefill_fa.cuh), by KV head and tile of 128 tokens: K norms, V norms (zero behind
+// the prompt) as floats, then eight halves, the largest of which is the tile's largest V norm.
+constexpr int PFT_KT = 128;                // cache rows per tile
+constexpr int PFT_NORMS = 2 * PFT_KT + 4;  // floats per tile
 
 struct PrefillTcParams {
     uint8_t* ck;
@@ -114,6 +122,12 @@ struct PrefillTcParams {
 #ifdef TQ_TIMING_SWITCHES
     unsigned long long* stamps;  // timing-experiment builds only: [2][16] summed clock deltas of a tile's sections (warps 0, 7)
 #endif
+    // ROWS16: what dequantize_rows_kernel would make of the prompts afterwards: fp16 centroids [n_seq][T][kv_dim] and norms
+    // [n_seq][Hkv][norm_tiles][PFT_NORMS]
+    __half* k16;
+    __half* v16;
+    float* norms;
+    int norm_tiles;
     __half* k_post;            // [vectors][128] like k_buf: receives the produced K vectors (what the reference's k buffer
                                // holds after its two kernels); the exact chains of near-bound coordinates re-read them
 };
@@ -270,14 +284,18 @@ __device__ __forceinline__ uint32_t tc_operand_addr(uint32_t tile, int row, int 
 // TMA_IN: the tile's 128 vectors reach the operand tile by ONE tensor-map copy (issued while the previous tile is being
 // quantised) instead of through registers; the sums of squares are then taken from shared memory while the tensor core
 // already rotates.  Needs a tensor map over the input (make_append_input_map) and Hkv dividing 128; never with PRODUCER.
-template <bool PRODUCER, bool TMA_IN>
-__global__ void __launch_bounds__(TC_THREADS, PRODUCER ? 2 : TC_CTAS_PER_SM)  // (the producer form needs more registers)
+// ROWS16: the prompt's rows as fp16 centroids and its norms as floats too, for the attention behind this launch: one launch and one
+// pass over the codes less where the prompt is short enough for those to count (whole prompts from position 0; Hkv divides 8, a
+// tile's tokens are of one prompt).
+template <bool PRODUCER, bool TMA_IN, bool ROWS16 = false>
+__global__ void __launch_bounds__(TC_THREADS, PRODUCER || ROWS16 ? 2 : TC_CTAS_PER_SM)  // (these need more registers, shared memory)
 prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __grid_constant__ CUtensorMap tm_v_in, const PrefillTcParams p) {
+    static_assert(!ROWS16 || TMA_IN, "a tile of whole tokens");
     static_assert(!(PRODUCER && TMA_IN), "the producer form computes its K vectors: they cannot come by a bulk copy");
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t dyn_base = smem_u32(tc_smem);
-    if (dyn_base > TcSmem::DST0 || dyn_base + (uint32_t)TC_DYN_SMEM < TcSmem::END) {  // (uniform over the CTA)
+    if (dyn_base > TcSmem::DST0 || dyn_base + (ROWS16 ? TC_ROWS_END : (uint32_t)TC_DYN_SMEM) < (ROWS16 ? TC_ROWS_END : TcSmem::END)) {  // (uniform over the CTA)
         if (tid == 0) atomicMax(p.status, ST_SMEM_LAYOUT);
         return;
     }
@@ -353,6 +371,15 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
             }
         }
         grid_s[i] = amb >= 0 ? ((__float_as_uint(ambv) & ~15u) | (uint32_t)amb) : (0x7f000000u | (uint32_t)code);
+    }
+    uint32_t* const rows_lut = reinterpret_cast<uint32_t*>(gbase + TC_ROWS_LUT);
+    uint32_t* const rows_top = reinterpret_cast<uint32_t*>(gbase + TC_ROWS_TOP);
+    if constexpr (ROWS16) {
+        if (tid < 8) rows_top[tid] = 0u;
+        for (int i = tid; i < (bits == 4 ? 256 : 16) * 8; i += TC_THREADS) {
+            const int e = i >> 3;
+            rows_lut[i] = bits == 4 ? pack_half2(kCent4[e & 15], kCent4[e >> 4]) : pack_half2(kCent2[e & 3], kCent2[(e >> 2) & 3]);
+        }
     }
     // (divisions and what else depends on the parameters alone: before the wait)
     const int vec_per_seq = p.T * p.Hkv;
@@ -449,6 +476,9 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         atomicAnd(w, ~m);
         atomicOr(w, (uint32_t)code << sh);
     };
+    auto patch_row = [&](int kind, int vid, int d, int code) {
+        if constexpr (ROWS16) (kind == 0 ? p.k16 : p.v16)[(size_t)vid * HEAD_DIM + d] = __float2half_rn(bits == 4 ? kCent4[code] : kCent2[code]);
+    };
     auto vector_input = [&](int kind, int vid) -> const __half* {  // the 128 inputs of vector vid of a kind, as rotated
         const int tok = fastdiv(vid, div_hkv), head = vid - tok * p.Hkv;
         const __half* buf = kind == 0 ? (PRODUCER ? p.k_post : p.k_buf) : p.v_buf;
@@ -478,7 +508,11 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                 const int v = (int)(item >> 8), d = (int)(item & 255u);
                 const long long dst = dst_s[v];
                 // (a CTA's last tile stays in the operand tile: its chains, the tail of a prompt of a few tiles, need no trip to memory)
-                if (dst >= 0) patch(cq + dst, d, tile + (int)gridDim.x >= total_tiles ? chain_in_tile(v, inv_s[v], d) : exact_code(vector_input(kind, vec0 + v), inv_s[v], d));
+                if (dst >= 0) {
+                    const int code = tile + (int)gridDim.x >= total_tiles ? chain_in_tile(v, inv_s[v], d) : exact_code(vector_input(kind, vec0 + v), inv_s[v], d);
+                    patch(cq + dst, d, code);
+                    patch_row(kind, vec0 + v, d, code);
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty + 8u * (uint32_t)b);
@@ -773,6 +807,12 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         if (settle_v >= 0) {  // settle the vector: norm out, 1/norm, where its codes go
             const bool abnormal = !(my_tt < 3.0e38f);  // an infinity or a NaN among the inputs: every coordinate is a NaN
             if (my_dst >= 0) cn[my_norm] = __float2half_rn(sqrt_approx_ftz(my_tt));
+            if constexpr (ROWS16) {
+                const __half n = vec0 + settle_v < vec_per_kind ? __float2half_rn(sqrt_approx_ftz(my_tt)) : __ushort_as_half((unsigned short)0);
+                const int t = t0 + dtok;
+                p.norms[(((long long)seq0 * p.Hkv + dhead) * p.norm_tiles + (t >> 7)) * PFT_NORMS + kind * PFT_KT + (t & (PFT_KT - 1))] = __half2float(n);
+                if (kind == 1) atomicMax(&rows_top[dhead], (uint32_t)__half_as_ushort(n));
+            }
             dst_s[settle_v] = my_dst;
             // (an all-zero vector -- padding, say -- has every coordinate ON the bound 0: 128 exact chains, all with the result
             //  +0; it gets its constant codes directly instead.  The sum of squares of any other fp16 vector is at least 3.6e-15.)
@@ -791,6 +831,22 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
         }
         TC_STAMP(6);
 
+        if constexpr (ROWS16) {
+            // the largest V norm of each head among this tile's tokens; behind a prompt's last token: zero
+            const int part = (t0 & (PFT_KT - 1)) / TPT;
+            auto tops = [&](int head) { return reinterpret_cast<unsigned short*>(p.norms + (((long long)seq0 * p.Hkv + head) * p.norm_tiles + (t0 >> 7)) * PFT_NORMS + 2 * PFT_KT); };
+            const int left = t0 + TPT >= p.T ? PFT_KT - (t0 & (PFT_KT - 1)) - TPT : 0;  // tokens of the last tile nobody brings
+            if (kind == 1 && tid < p.Hkv) {
+                tops(tid)[part] = (unsigned short)rows_top[tid];
+                rows_top[tid] = 0u;
+                for (int i = p.Hkv; part == 0 && i < 8; ++i) tops(tid)[i] = 0;
+                for (int i = part + 1; left > 0 && i < p.Hkv; ++i) tops(tid)[i] = 0;
+            }
+            for (int i = tid; i < left * p.Hkv; i += TC_WORKERS) {
+                const int tl = i / p.Hkv, head = i - tl * p.Hkv;
+                p.norms[(((long long)seq0 * p.Hkv + head) * p.norm_tiles + (t0 >> 7)) * PFT_NORMS + kind * PFT_KT + PFT_KT - left + tl] = 0.0f;
+            }
+        }
         // ---- 3. accumulators -> codes.  A warp reaches the 32 TMEM lanes (vectors) of its rank modulo 4; warps w and
         //         w + 4 share those vectors and take 64 of the 128 coordinates (two blocks of 32 columns) each ----
         uint32_t own0 = 0u, own1 = 0u;  // near-bound coordinates (of this thread's two blocks) that did not fit the shared queue
@@ -845,6 +901,21 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                     words[0] = words[1] = words[2] = words[3] = inv == -2.0f ? zero_codes : (bits == 4 ? 0xffffffffu : 0u);
                     near_mask = 0u;
                 }
+                if constexpr (ROWS16) {
+                    if (vec0 + ev < vec_per_kind) {
+                        __half* const dst = (kind == 0 ? p.k16 : p.v16) + (size_t)(vec0 + ev) * HEAD_DIM + 32 * cc;
+                        const uint32_t* const lut = rows_lut + (lane & 7);
+#pragma unroll
+                        for (int j = 0; j < 4; j += 2) {  // 16 coordinates: a whole sector at a time
+                            uint32_t u[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                u[i] = lut[bits == 4 ? ((words[j + (i >> 2)] >> (8 * (i & 3))) & 0xffu) * 8 : ((words[j >> 1] >> (4 * i)) & 0xfu) * 8];
+                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 8 * j), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]),
+                                         "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]) : "memory");
+                        }
+                    }
+                }
                 if (ev_dst < 0) near_mask = 0u;  // (a vector past the end of the input is all zeros: every coordinate ON a bound)
                 while (near_mask) {
                     const int i = __ffs(near_mask) - 1;
@@ -877,7 +948,9 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                 while (m) {
                     const int i = __ffs(m) - 1;
                     m &= m - 1;
-                    patch(cq + ev_dst_keep, 32 * (cc0 + k) + i, exact_code(x, inv, 32 * (cc0 + k) + i));
+                    const int code = exact_code(x, inv, 32 * (cc0 + k) + i);
+                    patch(cq + ev_dst_keep, 32 * (cc0 + k) + i, code);
+                    patch_row(kind, vec0 + ev, 32 * (cc0 + k) + i, code);
                 }
             }
         }
