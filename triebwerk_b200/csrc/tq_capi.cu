@@ -496,10 +496,11 @@ int tq_fp16_append_decode(void* ck, void* cv, const void* k_buf, const void* v_b
     return cuda_status(cudaGetLastError());
 }
 
-int tq_fp16_decode_attention(void* out, const void* q, const void* ck, const void* cv, const int* positions,
-                             int pos_value, const long long* row_base, long long total_rows, int max_seq_len, int G,
-                             int num_heads, int num_kv_heads, int head_dim, int q_dim, int kv_dim, void* workspace,
-                             size_t workspace_bytes, tq_stream_t s) {
+// behind_write: directly behind an fp16_cache_write_kernel that has cleared the tickets
+static int fp16_attention(void* out, const void* q, const void* ck, const void* cv, const int* positions,
+                          int pos_value, const long long* row_base, long long total_rows, int max_seq_len, int G,
+                          int num_heads, int num_kv_heads, int head_dim, int q_dim, int kv_dim, void* workspace,
+                          size_t workspace_bytes, tq_stream_t s, bool behind_write) {
     int r = check_shape(G, num_heads, num_kv_heads, head_dim, q_dim, kv_dim, 0, false);
     if (r != TQ_OK) return r;
     if (!out || !q || !ck || !cv) return TQ_ERR_ARG;
@@ -521,7 +522,7 @@ int tq_fp16_decode_attention(void* out, const void* q, const void* ck, const voi
     p.pos_value = pos_value; p.max_seq_len = max_seq_len;
     p.nchunk_max = (max_seq_len + FP16_CHUNK - 1) / FP16_CHUNK;
     p.G = G; p.H = num_heads; p.Hkv = num_kv_heads; p.q_dim = q_dim; p.kv_dim = kv_dim;
-    TQ_CUDA(cudaMemsetAsync(p.tickets, 0, (size_t)G * num_heads * sizeof(int), cs(s)));
+    if (!behind_write) TQ_CUDA(cudaMemsetAsync(p.tickets, 0, (size_t)G * num_heads * sizeof(int), cs(s)));
     // The tensor-core form by default (with four or eight query heads per KV head the fp32-FMA form is bound by its FMAs).
     // TQ_FP16_TC=0 keeps everything on the FMA form, TQ_FP16_TC=1 only one and two heads per KV head.
     static const int tc_mode = getenv("TQ_FP16_TC") ? atoi(getenv("TQ_FP16_TC")) : 2;
@@ -535,9 +536,17 @@ int tq_fp16_decode_attention(void* out, const void* q, const void* ck, const voi
             r2 = cached_fp16_map(&tmK, ck, total_rows, kv_dim);
             if (r2 == TQ_OK) r2 = cached_fp16_map(&tmV, cv, total_rows, kv_dim);
         }
-        if (r2 == TQ_OK) return launch_fp16_tc_attention(tmK, tmV, p, cs(s));
+        if (r2 == TQ_OK) return launch_fp16_tc_attention(tmK, tmV, p, cs(s), behind_write && use_pdl());
     }
     return launch_fp16_attention(p, cs(s));
+}
+
+int tq_fp16_decode_attention(void* out, const void* q, const void* ck, const void* cv, const int* positions,
+                             int pos_value, const long long* row_base, long long total_rows, int max_seq_len, int G,
+                             int num_heads, int num_kv_heads, int head_dim, int q_dim, int kv_dim, void* workspace,
+                             size_t workspace_bytes, tq_stream_t s) {
+    return fp16_attention(out, q, ck, cv, positions, pos_value, row_base, total_rows, max_seq_len, G, num_heads, num_kv_heads, head_dim, q_dim,
+                          kv_dim, workspace, workspace_bytes, s, false);
 }
 
 static size_t fp16_workspace_bytes(int G, int H, int Hkv, int max_seq_len) {
@@ -1402,13 +1411,22 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
         (!fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, 0.0))))
         return engine_cluster_layers(e, layer, 1, 1, q, k, v, out, chained, cs(s));
     if (e->kv_bits == 0) {
-        fp16_cache_write_kernel<<<e->G, 128, 0, cs(s)>>>((__half*)L.k, (__half*)L.v, (const __half*)k, (const __half*)v,
-                                                         e->d_positions, e->rb(), e->msl, e->msl, e->G,
-                                                         e->kv_dim(), (int*)e->workspace, e->caps());
-        int r = cuda_status(cudaGetLastError());
+        // (the write clears the attention's tickets, which then starts under it)
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)e->G);
+        cfg.blockDim = dim3(128);
+        cfg.stream = cs(s);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = use_pdl() ? 1 : 0;
+        int r = cuda_status(cudaLaunchKernelEx(&cfg, fp16_cache_write_kernel, (__half*)L.k, (__half*)L.v, (const __half*)k, (const __half*)v,
+                                               (const int*)e->d_positions, (const long long*)e->rb(), e->msl, e->msl, e->G, e->kv_dim(),
+                                               (int*)e->workspace, (const int*)e->caps(), (int*)((char*)e->workspace + 256), H));
         if (r != TQ_OK) return r;
-        return tq_fp16_decode_attention(out, q, L.k, L.v, e->d_positions, -1, e->rb(), e->total_rows, e->msl, e->G,
-                                        H, Hkv, D, e->q_dim(), e->kv_dim(), e->workspace, e->ws_bytes, s);
+        return fp16_attention(out, q, L.k, L.v, e->d_positions, -1, e->rb(), e->total_rows, e->msl, e->G,
+                              H, Hkv, D, e->q_dim(), e->kv_dim(), e->workspace, e->ws_bytes, s, fast_shape(H, Hkv, false));
     }
     if (!fast_shape(H, Hkv, true)) {
         // a head layout outside the streaming kernel's: append with the chain kernel, attend with the generic one

@@ -43,9 +43,12 @@ struct Fp16AttnParams {
 
 __global__ void fp16_cache_write_kernel(__half* ck, __half* cv, const __half* k, const __half* v, const int* positions,
                                         const long long* row_base, int max_seq_len, int capacity_rows, int G,
-                                        int kv_dim, int* status, const int* seq_capacity = nullptr) {
+                                        int kv_dim, int* status, const int* seq_capacity = nullptr, int* tickets = nullptr, int n_tickets = 0) {
     const int g = blockIdx.x;
+    pdl_wait();
+    pdl_launch_dependents();  // (what came before this launch has finished: the attention behind it reads all but the rows written here)
     if (g >= G) return;
+    for (int i = threadIdx.x; i < n_tickets; i += blockDim.x) tickets[g * n_tickets + i] = 0;  // of the attention behind it
     const int pos = positions[g];
     if (seq_capacity) capacity_rows = seq_capacity[g];  // ragged slots: every sequence has its own limit
     if (pos < 0 || (capacity_rows > 0 && pos >= capacity_rows)) {

@@ -35,6 +35,9 @@ __global__ void __launch_bounds__(FP16TC_WARPS * 32)
 fp16_tc_decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                                 const Fp16AttnParams p) {
     extern __shared__ __align__(1024) uint8_t tc16_smem[];
+    // In a launch that may start under its predecessor, the write of the new rows (fp16_cache_write_kernel), all but those rows and the
+    // tickets is there already.
+    pdl_launch_dependents();
     const int kvh = blockIdx.x, chunk = blockIdx.y, g = blockIdx.z;
     const int pos = p.positions ? p.positions[g] : p.pos_value;
     const int L = (pos < 0 ? 0 : pos) + 1;
@@ -76,6 +79,7 @@ fp16_tc_decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const _
         const int tok = t_first + i * step;
         const uint32_t dst = ring + (uint32_t)(i % FP16TC_STAGES) * FP16TC_STAGE_BYTES;
         const uint32_t bar = bars + 8u * (uint32_t)(i % FP16TC_STAGES);
+        if (tok + FP16TC_BLOCK >= L) pdl_wait();  // the new token's rows
         mbar_arrive_expect_tx(bar, FP16TC_STAGE_BYTES);  // a box always delivers its full size (rows past the array end: zeros)
         tma_load_3d(dst, &tmK, bar, 0, (int)(row0 + tok), 2 * kvh);
         tma_load_3d(dst + FP16TC_ARRAY_BYTES, &tmV, bar, 0, (int)(row0 + tok), 2 * kvh);
@@ -240,6 +244,7 @@ fp16_tc_decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const _
         }
     }
     if (nparts == 1) return;
+    pdl_wait();  // the tickets are clear
     __threadfence();
     __syncthreads();
     if (tid == 0) {

@@ -528,19 +528,28 @@ __global__ void transpose_rotation_kernel(__half* dst, const __half* src) {
 
 // Tensor-core form of the twin (tq_fp16_tc.cuh): every query head of a KV head from one pass, whatever their number.
 template <int GRP>
-inline int launch_fp16_tc_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const Fp16AttnParams& p, cudaStream_t s) {
+inline int launch_fp16_tc_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const Fp16AttnParams& p, cudaStream_t s, bool pdl) {
     int ar = ensure_dynamic_smem((const void*)fp16_tc_decode_attention_kernel<GRP>, FP16TC_SMEM);
     if (ar != TQ_OK) return ar;
     dim3 grid(p.Hkv, p.nchunk_max, p.G);
-    fp16_tc_decode_attention_kernel<GRP><<<grid, FP16TC_WARPS * 32, FP16TC_SMEM, s>>>(tmK, tmV, p);
-    return cuda_status(cudaGetLastError());
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(FP16TC_WARPS * 32);
+    cfg.dynamicSmemBytes = FP16TC_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cuda_status(cudaLaunchKernelEx(&cfg, fp16_tc_decode_attention_kernel<GRP>, tmK, tmV, p));
 }
-inline int launch_fp16_tc_attention(const CUtensorMap& tmK, const CUtensorMap& tmV, const Fp16AttnParams& p, cudaStream_t s) {
+inline int launch_fp16_tc_attention(const CUtensorMap& tmK, const CUtensorMap& tmV, const Fp16AttnParams& p, cudaStream_t s, bool pdl) {
     switch (p.H / p.Hkv) {
-        case 1: return launch_fp16_tc_t<1>(tmK, tmV, p, s);
-        case 2: return launch_fp16_tc_t<2>(tmK, tmV, p, s);
-        case 4: return launch_fp16_tc_t<4>(tmK, tmV, p, s);
-        case 8: return launch_fp16_tc_t<8>(tmK, tmV, p, s);
+        case 1: return launch_fp16_tc_t<1>(tmK, tmV, p, s, pdl);
+        case 2: return launch_fp16_tc_t<2>(tmK, tmV, p, s, pdl);
+        case 4: return launch_fp16_tc_t<4>(tmK, tmV, p, s, pdl);
+        case 8: return launch_fp16_tc_t<8>(tmK, tmV, p, s, pdl);
         default: return TQ_ERR_UNSUPPORTED;
     }
 }
