@@ -484,11 +484,16 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
 // and that form starts 7 us later.  Above 640 clusters their number counts for more than in the lines fitted below it (128 x 64
 // tokens, 16/8 heads, 4-bit 25.7 / 19.7 us, 96 x 64 19.8 / 19.0, 64 x 64 13.5 / 17.2; 32/8 heads 128 x 64 26.8 / 24.9, 96 x 64 20 / 23;
 // fp16 128 x 300 43.0 / 39.1, 96 x 300 32.6 / 33.2).
+// fp16 slots of one chunk of the streaming form, which has nothing to merge there and starts under the write of the new rows, go to it
+// where the cluster form has one CTA per sequence and KV head (cluster / streaming: 16/8 heads 12 x 500 tokens 11.9 / 9.8 us, 48 x 300 21.6 /
+// 17.1, 96 x 500 44.6 / 37.4, 32/8 24 x 500 14.8 / 13.4), unless those just fill two CTAs per SM (32/8 32 x 300 11.4 / 11.9).
 // `extra`: us the streaming form's launches cost on top.
 inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, double extra) {
     const long long clusters = (long long)G * Hkv, sms = device_props().sm_count;
     const int S = cluster_split(bits, clusters, heads, max_tokens, true);
     const double chain = ((max_tokens + 15) / 16) / (double)(S * CD_WARPS), turns = (double)((clusters * S + sms - 1) / sms);
+    if (bits == 0 && extra == 0.0 && S == 1 && heads <= 4 && max_tokens <= FP16_CHUNK && max_tokens > FP16_CHUNK / 2 && (2 * clusters <= 3 * sms || clusters > 2 * sms))
+        return false;
     if (bits == 0) return (heads > 4 ? 0.5 : 1.0) * chain < 7.0 + 1.5 * turns + extra && !(clusters > 768 && chain > 2.0);
     const double many = heads > 2 ? 0.0015 * std::max(0ll, clusters - 800) : 0.02 * std::max(0ll, clusters - 640);
     if (bits == 4 && heads > 4 ? chain * turns > 12.0 : chain > 12.0 + 5e-6 * (double)rows * Hkv) return false;
