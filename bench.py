@@ -397,6 +397,8 @@ def prefill_launches(bits, batch, T, Hkv):
     131072 rows of a KV head at a time, some prompts or some KV heads of one."""
     if bits == 0 or T <= 128:
         return (1 if batch else 0) + 1
+    if batch and 8 % Hkv == 0 and batch * T * Hkv <= 32768 and (batch == 1 or T % (128 // Hkv) == 0):
+        return 2   # the cache write makes them
     prompts = max(1, 131072 // (T * Hkv))
     return (1 if batch else 0) + 2 * -(-(batch or 1) // prompts) * -(-T * Hkv // 131072)
 
@@ -773,10 +775,10 @@ def run_ours(args, w, rank, world, local_rank):
                 "h2d_bytes_per_step": int(world * NL * G * (q_dim + 2 * kv_dim) * 2),
                 "d2h_bytes_per_step": int(world * NL * G * q_dim * 2)},
         # kernels of this library launched inside the timed region (none of anybody else's but NCCL's at N > 1)
-        "gpu_launches": int(steps * ((4 if world == 1 else 2 + 2 * len(sharded_groups(NL, world))) if whole else NL * (1 if fused else 2))),
+        "gpu_launches": int(steps * ((4 if world == 1 else 2 + 2 * len(sharded_groups(NL, world))) if whole else NL * (3 if fused else 2))),
         "roofline": {"kernel": "fp16_cache_write_kernel + fp16_decode_attention_kernel" if bits == 0 else
                      f"decode_attention_kernel<{bits}>" + (" (whole-step form: one launch streams all layers; per layer)" if whole else
-                                                           " (one launch per layer: append + query rotation + attention)" if fused else ""),
+                                                           " (layer form: append + query rotation, attention, merge; per layer)" if fused else ""),
                      "bound": "hbm", "achieved": achieved, "peak": peak, "timed_by": timed_by,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind, "frac_of_8TBs": achieved / 8000.0,
                      "us_per_launch": attn_ms * 1e3 * (NL if whole else 1), "us_per_layer": attn_ms * 1e3,

@@ -210,9 +210,9 @@ int tq_engine_create(const tq_model_shape* shape, int max_seq_len, int kv_bits, 
 void tq_engine_destroy(tq_engine* e);
 int tq_engine_kv_bits(const tq_engine* e);
 
-/* Packed modes: choose between ONE launch per layer and step (on = 1, the default: the attention kernel also appends
- * the new token and rotates the queries) and the two-launch form (on = 0: append kernel, then attention kernel).
- * Both store identical bytes.  Returns the previous setting, or a negative status.  The environment variable
+/* Packed modes: choose between the layer form (on = 1, the default: a launch that appends the new token and rotates the queries on
+ * the tensor cores, the attention, the merge of its parts, each starting under the one before) and the two-launch form (on = 0: append
+ * kernel, then attention kernel).  Both store identical bytes.  Returns the previous setting, or a negative status.  The environment variable
  * TQ_FUSED=0 makes the two-launch form the default of new engines.  No counterpart in the reference. */
 int tq_engine_set_fused(tq_engine* e, int on);
 

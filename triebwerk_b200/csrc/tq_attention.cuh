@@ -20,7 +20,7 @@
 //     contiguous bulk copies; completion on one mbarrier per stage.  (An optional cp.async.bulk.prefetch.L2 of tiles
 //     further ahead exists, TQ_ATTN_L2_AHEAD; it is off by default because it did not pay on B200.)  The last warp of the
 //     worker to finish a stage (one shared-memory atomic per warp and tile) re-arms it: nobody waits for a slower
-//     warp.  In the whole-step form a copy warp does, which the warps tell through a barrier per part: without the list's
+//     warp.  In the layer form and in whole steps of enough tiles a copy warp does, which the warps tell through a barrier per part: without the list's
 //     cursor, the atomics and the fences 664 -> 630 warp instructions per warp and tile (28 layers of 64 x 4096 tokens
 //     2007 -> 1863 us, ragged 128 sequences 2319 -> 2135; shared memory 74 % busy, issue slots 64 %, and
 //     with two stages the time from hand-back to copy counts: a thread that polls and sleeps 64 ns, 4 layers 2-bit 64 x 3000
@@ -38,14 +38,18 @@
 //   * 2-bit scores need no table there (PLANES): a centroid is affine in its code's two bits, so every bit of the code bytes,
 //     masked in place, is an operand of mma.sync.m16n8k32 (u8 x s8) against 16-bit fixed-point queries; one mask per four
 //     codes and plane, as many products as before.  The table look-ups of K were 64 of a tile's 176 shared-memory wavefronts: that
-//     pipe 67 -> 49 % busy, 550 -> 484 warp instructions, 8 layers of 64 x 4096 tokens (32/8 heads) 456 -> 423 us in the whole-step form, 32 x 8192 one launch per
-//     layer 73.5 -> 69.7 us.  What is left is instruction issue (65 %) and the ALU (56 %).  V keeps the table: its operand is the weights, whose
+//     pipe 67 -> 49 % busy, 550 -> 484 warp instructions, 8 layers of 64 x 4096 tokens (32/8 heads) 456 -> 423 us in the whole-step form.
+//     What is left is instruction issue (65 %) and the ALU (56 %).  V keeps the table: its operand is the weights, whose
 //     range fixed point does not cover.  Scalar fp32 FMAs cannot
 //     keep up with HBM3e on this path: 512 FMAs per 132-byte row is more than the SMs can issue.
-//   * A worker that finishes its part of a sequence writes (acc[128], m, l) per query head to the workspace
-//     and takes a ticket; the last arrival merges all parts, and multiplies by R^T on the tensor cores
-//     (normalised accumulators split into fp16 high + low parts as the A operand, R^T as B).  Nobody spins on
-//     anybody: the ticket is a single atomicAdd.
+//   * A worker that finishes its part of a sequence writes (acc[128], m, l) per query head to the workspace.  A kernel behind
+//     this one merges the parts and multiplies by R^T on the tensor cores (normalised accumulators split into fp16
+//     high + low parts as the A operand, R^T as B); in MODE 0 the last worker to arrive does, found by a ticket: a single
+//     atomicAdd, nobody spins on anybody.
+//   * Layer form (MODE 1): append and query rotation in a launch before (tq_layer_prep.cuh), merge in one behind, so that a tile loop with
+//     copy warps and nothing else is left, which starts with table and ring ready.  With all of it in one launch a tile took
+//     1.76 us for 1.47 and the first one began 4 us later: 32 x 8192 tokens 2-bit, 32/8 heads 69.6 -> 57.9 us a layer (issue
+//     slots 51 -> 64 % busy, DRAM 24 -> 32 %), 4-bit 32 x 4096 49.8 -> 41.8, 128 x 64 18.7 -> 17.0.
 #pragma once
 
 #include <type_traits>
@@ -1334,6 +1338,7 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const MergeParams p
 // The merge of one layer's partials (mode 1), the tail of that layer: bound by latency.  One CTA per (sequence, 8 heads), a warp per
 // head, its parts' loads in flight together.  Under the attention's last tiles, before the wait: R's fragments and which workers had
 // a part, from the positions (which that launch does not write; what came before it has finished when this one starts).
+// From the wait to the end 2.4 to 3.1 us (32 x 8192 tokens, 32 heads); by the last arriving worker inside the attention 5.6.
 struct MergeLayerParams {
     const float* partials;       // [workers + G][H][PART_STRIDE]
     const int* positions;        // device [G] or null: pos_value

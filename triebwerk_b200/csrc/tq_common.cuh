@@ -34,7 +34,7 @@ enum : int {
 // ---- workspace layout ---------------------------------------------------------------------------------------
 // [0,256)                       header: int status; int total_tiles; ...
 // q_rot      float [G][H][128]  pre-rotated queries, already multiplied by log2(e)/sqrt(128)
-// tile_start int   [G+4]        exclusive prefix of ceil(L_g / TILE_TOKENS); one-launch form: then workers, total tiles
+// tile_start int   [G+4]        exclusive prefix of ceil(L_g / TILE_TOKENS)
 // tickets    int   [G]          arrivals per sequence (zeroed by the append/rotate kernel)
 // worker_g   int   [MAX_WORKERS] first sequence of each attention worker's slice
 // partials   float [W+G][H][PART_STRIDE]  acc[128], m, l, pad

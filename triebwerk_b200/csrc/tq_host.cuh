@@ -852,7 +852,7 @@ struct tq_engine {
     // launch saw them, so the next fused launch may read them before it has seen its predecessor finish.
     bool chain_ok = false;
     cudaStream_t chain_stream = nullptr;
-    bool fused = !(getenv("TQ_FUSED") && atoi(getenv("TQ_FUSED")) == 0);  // one launch per layer-step (packed modes)
+    bool fused = !(getenv("TQ_FUSED") && atoi(getenv("TQ_FUSED")) == 0);  // the layer form, not the two-launch form (packed modes)
 
     // current carving
     int G = 0;

@@ -10,7 +10,7 @@
 // Tiles are 128 cache rows.  K lies in shared memory as [coordinate half][128 rows][128 B] (K-major B operand of S = Q K^T),
 // V in the same form, read as an MN-major B operand of O += P V: no transposition anywhere, both arrive by one tensor-map
 // copy.  Packed caches are turned into fp16 centroids (unscaled: the same operands as ever) and fp32 norms by
-// dequantize_rows_kernel first, once per prompt and layer instead of once per query block: done by producer warps inside
+// dequantize_rows_kernel (short prompts: by the append, tq_prefill_tc.cuh) first, once per prompt and layer instead of once per query block: done by producer warps inside
 // this kernel the table look-ups and operand stores took as much of the shared-memory pipe as the products themselves (8192
 // tokens, 16/8 heads, 4-bit, eight softmax warps: 617 us against 439).  Prompts of a single tile are the exception (DIRECT).  P (times the V norm, fp16) replaces S in tensor memory and is read from
 // there as the A operand.
@@ -28,9 +28,8 @@
 // Every wait on a barrier is bounded; a wait that runs out raises the status word and the kernel runs to its end.
 // Bound by the softmax threads (exponentials, tensor-memory loads) against the tensor core at long prompts, by the chain copy ->
 // S -> softmax -> O of a single block at short ones.  Per layer, 8 KV heads, cache write included, the one-block kernel with V
-// transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 507 us in runs of a few milliseconds (1080 TFLOP/s
-// of causal arithmetic), 590 (930) under the power cap of longer ones; 4-bit 8192 tokens 16 heads 763 -> 343 to 361 us, 777 tokens
-// 43.7 -> 32.5.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
+// transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 478 us in runs of a few milliseconds (1150 TFLOP/s
+// of causal arithmetic), 557 (987) under the power cap of longer ones; 4-bit 777 tokens 16 heads 43.7 -> 28.3.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
 #pragma once
 
 #include "tq_prefill_tc.cuh"

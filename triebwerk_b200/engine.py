@@ -175,7 +175,7 @@ class Engine:
 
     def step_prepare(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
         """First phase of decode_step: every layer's append and query rotation.  False when the engine cannot split the
-        step (fp16 cache, one launch per layer): use decode_layers then."""
+        step (fp16 cache, launches per layer): use decode_layers then."""
         for t in (q, k, v):
             assert t.is_cuda and t.is_contiguous() and t.dtype == torch.float16 and t.shape[0] == self.shape.num_layers
         r = lib().tq_engine_step_prepare(self._h, q.data_ptr(), k.data_ptr(), v.data_ptr(), self._stream())
