@@ -70,3 +70,30 @@ def test_several_prompts(bits, H, Hkv, T, n):
     assert eng.status() == 0
     for i in range(n):
         hp.assert_attention_close(out[i].cpu().numpy(), _launcher(eng, 0, 1 + i, q[i], msl, H, Hkv, bits), H, D, f"prompt {i}")
+
+
+@pytest.mark.parametrize("bits,H,Hkv,T,n", [(4, 16, 8, 33, 1), (4, 16, 8, 64, 1), (2, 32, 8, 128, 1), (4, 16, 8, 100, 16), (4, 16, 8, 129, 1), (2, 32, 4, 777, 1),
+                                            (4, 40, 8, 300, 1), (4, 16, 8, 2500, 2)])
+def test_queries_that_are_the_layer_befores_result(bits, H, Hkv, T, n):
+    """The attention reads its queries under the append; they are what the launch before that wrote, or a kernel of another library."""
+    NL, msl = 4, -(-T // 32) * 32
+    rng = np.random.default_rng(T)
+    eng = tq.Engine(msl, bits, num_layers=NL, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(n, msl)
+    k, v, q = _draw(rng, NL, n, T, Hkv * D), _draw(rng, NL, n, T, Hkv * D), _draw(rng, n, T, H * D)
+
+    def chain(settle):
+        x = q.clone()
+        for layer in range(NL):
+            out = torch.full_like(x, float("nan"))
+            settle()
+            eng.prefill_layer_batch(layer, 0, x, k[layer], v[layer], out)
+            settle()
+            x = out * 4 if layer == 1 else out
+            settle()
+        return x.cpu().numpy().view(np.uint16)
+
+    want = chain(torch.cuda.synchronize)
+    for _ in range(3):
+        assert np.array_equal(chain(lambda: None), want)
+    assert eng.status() == 0

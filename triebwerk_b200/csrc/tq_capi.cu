@@ -1981,7 +1981,7 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
         r = take_scratch();
         if (r != TQ_OK) return r;
     }
-    r = engine_prefill_impl(e, layer, first_seq, n_seq, k, v, 0, T, s, makes_rows ? &rows : nullptr);
+    r = engine_prefill_impl(e, layer, first_seq, n_seq, k, v, 0, T, s, &rows);
     if (r != TQ_OK) return r;
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
     if (q_stride < H * HEAD_DIM || (q_stride & 7) != 0) return TQ_ERR_ARG;
@@ -2029,6 +2029,7 @@ int tq_engine_prefill_layer_batch(tq_engine* e, int layer, int first_seq, int n_
         ap.vn = (const __half*)L.vn + (size_t)row0 * Hkv;
         ap.rotation = (const __half*)e->d_rotation;
     }
+    ap.early = rows.behind && use_pdl() ? 1 : 0;
     ap.status = (int*)e->workspace;
     const size_t least = e->kv_bits ? prefill_scratch_bytes(T, 1, prefill_exact(e->kv_bits, H, Hkv)) : 0;
     if (least > e->prefill_scratch_bytes) {  // not even one KV head of such a prompt fits

@@ -309,6 +309,7 @@ struct PrefillRows {
     float* norms;
     int tiles;
     bool made;
+    bool behind;  // the append was the tensor-core kernel: what comes next may read everything before it at once
 };
 inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, bool pdl, int n_seq = 1, long long seq_stride_rows = 0,
                              const long long* seq_row_base = nullptr, PrefillRows* rows = nullptr) {
@@ -320,6 +321,7 @@ inline int launch_prefill_tc(const AppendParams& p, cudaStream_t s, bool pdl, in
     t.T = p.n_src; t.Hkv = p.Hkv; t.kv_dim = p.kv_dim; t.bits = p.bits;
     t.static_rotation = p.rot_prep ? 1 : 0;  // (the engine's own R)
     if (rows) { t.k16 = rows->k16; t.v16 = rows->v16; t.norms = rows->norms; t.norm_tiles = rows->tiles; }
+    if (rows) rows->behind = true;
     return launch_prefill_tc_params(t, s, pdl, false, rows ? &rows->made : nullptr);
 }
 
@@ -592,15 +594,15 @@ inline int make_prefill_query_map(CUtensorMap* m, const void* base, long long to
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TQ_OK : TQ_ERR_ARG;
 }
-template <bool PACKED, int MT, bool EXACT = false, int DIRECT = 0>
+template <bool PACKED, int MT, bool EXACT = false, int DIRECT = 0, bool EARLY = false>
 inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ, const CUtensorMap& tmR, const PrefillAttnParams& p,
                                dim3 grid, cudaStream_t s) {
-    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT>, PftSmem::BYTES);
+    int r = ensure_dynamic_smem((const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT, EARLY>, PftSmem::BYTES);
     if (r != TQ_OK) return r;
     // the register split inside the kernel draws on what the launch brings: never launch with less
     static const int regs = [] {
         cudaFuncAttributes a{};
-        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT>) == cudaSuccess ? a.numRegs : 0;
+        return cudaFuncGetAttributes(&a, (const void*)prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT, EARLY>) == cudaSuccess ? a.numRegs : 0;
     }();
     if (regs < PFT_REGS_LAUNCH) return TQ_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg{};
@@ -613,7 +615,7 @@ inline int launch_prefill_fa_t(const CUtensorMap& tmK, const CUtensorMap& tmV, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT>, tmK, tmV, tmQ, tmR, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, prefill_attention_fa_kernel<PACKED, MT, EXACT, DIRECT, EARLY>, tmK, tmV, tmQ, tmR, p));
 }
 // Which layouts keep fp32's precision (tq_prefill_fa.cuh): those that neither this kernel's predecessor nor the streaming kernels took.
 inline bool prefill_exact(int bits, int H, int Hkv) {
@@ -719,7 +721,11 @@ inline int launch_prefill_attention(int bits, PrefillAttnParams p, long long tot
             const long long blocks = mt == 2 ? blocks2 : blocks1;
             if (cols > 2147483647ll || blocks > 65535) return TQ_ERR_CAPACITY;
             dim3 grid((unsigned)cols, (unsigned)blocks);
-            if (direct) r = bits == 4 ? (mt == 2 ? launch_prefill_fa_t<true, 2, false, 4>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1, false, 4>(tmK, tmV, tmQ, tmR, a, grid, s))
+            // Where the blocks convert the codes themselves, that comes behind the rotation in the early form: taken where append and attention
+            // fit the GPU side by side (28 layers, 2-bit, 120 tokens 435 -> 407 us, 64 4-bit 400 -> 390, but 8 of 16 x 100 188 -> 191).
+            const bool early = direct && a.early && mt == 1 && cols * blocks + 2ll * a.n_seq * p.T * a.Hkv / TC_TILE <= sms;
+            if (early) r = bits == 4 ? launch_prefill_fa_t<true, 1, false, 4, true>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1, false, 2, true>(tmK, tmV, tmQ, tmR, a, grid, s);
+            else if (direct) r = bits == 4 ? (mt == 2 ? launch_prefill_fa_t<true, 2, false, 4>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1, false, 4>(tmK, tmV, tmQ, tmR, a, grid, s))
                                       : (mt == 2 ? launch_prefill_fa_t<true, 2, false, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1, false, 2>(tmK, tmV, tmQ, tmR, a, grid, s));
             else if (low) r = launch_prefill_fa_t<true, 1, true>(tmK, tmV, tmQ, tmR, a, grid, s);
             else if (bits != 0) r = mt == 2 ? launch_prefill_fa_t<true, 2>(tmK, tmV, tmQ, tmR, a, grid, s) : launch_prefill_fa_t<true, 1>(tmK, tmV, tmQ, tmR, a, grid, s);

@@ -24,12 +24,14 @@
 // Numbers of query heads per KV head other than 1, 2, 4, 8 and 16 took a kernel with fp32 queries, centroids and weights.  Here they
 // are fp16 high + low parts (EXACT: three products for one, two for fp16 caches): the results' error is that kernel's.  With the high
 // parts alone it was 2.4 (4-bit), 2.9 (2-bit) and 1.2 (fp16) times as large.
-// Packed forms: Q R^T at the start and (O / l) R at the end (fp16 high + low parts) are tcgen05 products too.
+// Packed forms: Q R^T at the start and (O / l) R at the end (fp16 high + low parts) are tcgen05 products too.  Behind the append the first of
+// them is done before the wait: the append lets this launch start when everything before it has finished, and its own stores have nothing
+// to do with queries and R.  Per layer, 16/8 heads, 4-bit: 300 tokens 21.6 -> 20.1 us, 777 28.4 -> 27.0, 16 x 256 50.2 -> 47.1.
 // Every wait on a barrier is bounded; a wait that runs out raises the status word and the kernel runs to its end.
 // Bound by the softmax threads (exponentials, tensor-memory loads) against the tensor core at long prompts, by the chain copy ->
 // S -> softmax -> O of a single block at short ones.  Per layer, 8 KV heads, cache write included, the one-block kernel with V
 // transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 478 us in runs of a few milliseconds (1150 TFLOP/s
-// of causal arithmetic), 557 (987) under the power cap of longer ones; 4-bit 777 tokens 16 heads 43.7 -> 28.3.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
+// of causal arithmetic), 557 (987) under the power cap of longer ones; 4-bit 777 tokens 16 heads 43.7 -> 27.0.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
 #pragma once
 
 #include "tq_prefill_tc.cuh"
@@ -56,6 +58,8 @@ struct PrefillAttnParams {
     const uint8_t* cv;
     const __half* kn;         // [rows][Hkv], packed caches (read by DIRECT)
     const __half* vn;
+    int early;                // packed, behind prefill_append_tc_kernel (or a launch behind it), which lets its successor start once all before it
+                              // has finished: queries and R may be read and rotated before the wait
     const __half* rotation;   // packed: R row-major [128][128]
     int low_row;              // packed, EXACT: rows from the high parts to the low parts of ck, cv
     const float* norms;       // packed: fp32 [n_seq][Hkv][tiles][PFT_NORMS] (dequantize_rows_kernel)
@@ -260,7 +264,8 @@ __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.a
 // DIRECT (4 or 2 bits, prompts of one tile): the softmax warps turn the tile's codes into centroids themselves, while the queries arrive
 // and are rotated.  Every query block of a head repeats that, but dequantize_rows_kernel's launch is saved: a layer of 35 tokens,
 // 16/8 heads, 4-bit 20.4 -> 15.5 us, 16 prompts of 32 tokens, 2-bit 24.9 -> 19.9, 16 of 128, 4-bit 33.0 -> 25.8.
-template <bool PACKED, int MT, bool EXACT, int DIRECT>
+// EARLY (DIRECT only; elsewhere p.early says it): queries and R before the wait, the codes behind the rotation.
+template <bool PACKED, int MT, bool EXACT, int DIRECT, bool EARLY = false>
 __global__ void __launch_bounds__(PFT_THREADS, 1)
 prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ,
                             const __grid_constant__ CUtensorMap tmR, const PrefillAttnParams p) {
@@ -274,6 +279,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     constexpr int COPY_WARP = PFT_SOFT_WARPS, MMA_WARP = PFT_SOFT_WARPS + 1;
     constexpr bool LOW = PACKED && EXACT;  // low parts of the operands in shared memory
     static_assert(!LOW || MT == 1, "the second query block's places hold the low parts");
+    static_assert(!EARLY || DIRECT, "decided by p.early");
     static_assert(!DIRECT || (PACKED && !EXACT), "a packed form");
     // DIRECT: byte (4-bit) or nibble (2-bit) -> two centroids, eight copies, in the idle second stage of K
     constexpr int CODES = DIRECT == 4 ? 256 : 16;
@@ -343,8 +349,11 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_wait();
-    pdl_launch_dependents();  // (the next launch waits for this one's end before it reads or writes anything of the caller's)
+    const bool early = DIRECT ? EARLY : PACKED && p.early != 0;
+    if (!early) {
+        pdl_wait();
+        pdl_launch_dependents();  // (the next launch waits for this one's end before it reads or writes anything of the caller's)
+    }
     // this block's queries, row (token, head), and R: one copy each (rows behind GRP * QT and tokens past the prompt: whatever comes
     // -- a row's garbage stays in that row and is never stored)
     if (tid == 32 * COPY_WARP) {
@@ -396,7 +405,7 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     umma_lo(tmem + 128u * m, pft_lo_k(sb + PftSmem::Q + m * PFT_TILE) + pft_kstep(ks), pft_lo_k(sb + PftSmem::R) + pft_kstep(ks), PFT_IDESC_K, ks != 0);
             umma_commit(bar_rot);
         }
-        if (DIRECT && warp < PFT_SOFT_WARPS) {
+        auto make_operands = [&]() {
             constexpr int PIECES = 2 * PFT_KT * 16 / (32 * PFT_SOFT_WARPS);  // of 8 codes per thread: K rows, then V rows
             uint32_t c[PIECES];
             const size_t head0 = ((size_t)seq_row0 * p.Hkv + kvh) * 16;
@@ -429,8 +438,9 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 }
                 *reinterpret_cast<uint4*>(gb + (i < PIECES / 2 ? PftSmem::K : PftSmem::V) + pft_chunk(row, tid & 15)) = u;
             }
-        }
+        };
         if (warp < PFT_SOFT_WARPS) {
+            if constexpr (DIRECT && !EARLY) make_operands();
             wait_bar(bar_rot, 0u);
             tc_fence_after();
 #pragma unroll 1
@@ -448,6 +458,10 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     put_frag(PftSmem::Q + PFT_TILE, c0, y);
                 }
             }
+            if constexpr (EARLY) {
+                pdl_wait();
+                make_operands();
+            }
         }
         if (warp < PFT_SOFT_WARPS || warp == MMA_WARP) {  // the rotated queries are in place (the copies of the first tiles are on their way already)
             fence_proxy_async_smem();
@@ -460,6 +474,10 @@ prefill_attention_fa_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     if (warp >= PFT_SOFT_WARPS) {
       regs_dec<PFT_REGS_REST>();
       if (warp == COPY_WARP) {
+        if (early) {  // (every other warp gets what the launches before this one made from this one's copies)
+            pdl_wait();
+            pdl_launch_dependents();
+        }
         // ================= the copies of every tile =================
         // (fp16 caches, the prompt's last tile: rows past the prompt may hold anything, and 0 x NaN is NaN, so its V rows are blanked)
         const int x_row = (int)seq_row0;
