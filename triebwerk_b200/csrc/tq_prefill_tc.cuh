@@ -71,7 +71,7 @@ struct TcSmem {
 };
 static_assert(TcSmem::CTRL + 64 <= TcSmem::GRID, "control words run into the bucket table");
 // ROWS16 (below): byte (4-bit) or nibble (2-bit) -> two centroids, eight copies; the largest V norm of each head in the tile
-constexpr uint32_t TC_ROWS_LUT = 0x13000, TC_ROWS_TOP = TC_ROWS_LUT + 8192, TC_ROWS_END = TC_ROWS_TOP + 32;
+constexpr uint32_t TC_ROWS_LUT = 0x13000, TC_ROWS_TOP = TC_ROWS_LUT + 32768, TC_ROWS_END = TC_ROWS_TOP + 32;
 static_assert(TcSmem::END <= TC_ROWS_LUT, "the rows' table runs into the queues");
 constexpr size_t TC_DYN_SMEM = TcSmem::END;  // enough wherever the dynamic shared memory starts at or below TcSmem::DST0
 constexpr int TC_CTAS_PER_SM = 3;
@@ -376,9 +376,10 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
     uint32_t* const rows_top = reinterpret_cast<uint32_t*>(gbase + TC_ROWS_TOP);
     if constexpr (ROWS16) {
         if (tid < 8) rows_top[tid] = 0u;
-        for (int i = tid; i < (bits == 4 ? 256 : 16) * 8; i += TC_THREADS) {
+        for (int i = tid; i < (bits == 4 ? 256 : 16) * 8; i += TC_THREADS) {  // (a copy for every lane)
             const int e = i >> 3;
-            rows_lut[i] = bits == 4 ? pack_half2(kCent4[e & 15], kCent4[e >> 4]) : pack_half2(kCent2[e & 3], kCent2[(e >> 2) & 3]);
+            const uint32_t u = bits == 4 ? pack_half2(kCent4[e & 15], kCent4[e >> 4]) : pack_half2(kCent2[e & 3], kCent2[(e >> 2) & 3]);
+            reinterpret_cast<uint4*>(rows_lut)[i] = make_uint4(u, u, u, u);
         }
     }
     // (divisions and what else depends on the parameters alone: before the wait)
@@ -904,13 +905,13 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                 if constexpr (ROWS16) {
                     if (vec0 + ev < vec_per_kind) {
                         __half* const dst = (kind == 0 ? p.k16 : p.v16) + (size_t)(vec0 + ev) * HEAD_DIM + 32 * cc;
-                        const uint32_t* const lut = rows_lut + (lane & 7);
+                        const uint32_t* const lut = rows_lut + lane;
 #pragma unroll
                         for (int j = 0; j < 4; j += 2) {  // 16 coordinates: a whole sector at a time
                             uint32_t u[8];
 #pragma unroll
                             for (int i = 0; i < 8; ++i)
-                                u[i] = lut[bits == 4 ? ((words[j + (i >> 2)] >> (8 * (i & 3))) & 0xffu) * 8 : ((words[j >> 1] >> (4 * i)) & 0xfu) * 8];
+                                u[i] = lut[bits == 4 ? ((words[j + (i >> 2)] >> (8 * (i & 3))) & 0xffu) * 32 : ((words[j >> 1] >> (4 * i)) & 0xfu) * 32];
                             asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 8 * j), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]),
                                          "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]) : "memory");
                         }
