@@ -903,18 +903,27 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                     near_mask = 0u;
                 }
                 if constexpr (ROWS16) {
-                    if (vec0 + ev < vec_per_kind) {
-                        __half* const dst = (kind == 0 ? p.k16 : p.v16) + (size_t)(vec0 + ev) * HEAD_DIM + 32 * cc;
-                        const uint32_t* const lut = rows_lut + lane;
+                    // 32 coordinates are two sectors: two lanes exchange halves, so that a store takes both sectors of a row next to each other
+                    const uint32_t* const lut = rows_lut + lane;
+                    uint32_t u[2][8];
 #pragma unroll
-                        for (int j = 0; j < 4; j += 2) {  // 16 coordinates: a whole sector at a time
-                            uint32_t u[8];
+                    for (int j = 0; j < 2; ++j)
 #pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                u[i] = lut[bits == 4 ? ((words[j + (i >> 2)] >> (8 * (i & 3))) & 0xffu) * 32 : ((words[j >> 1] >> (4 * i)) & 0xfu) * 32];
-                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 8 * j), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]),
-                                         "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]) : "memory");
-                        }
+                        for (int i = 0; i < 8; ++i)
+                            u[j][i] = lut[bits == 4 ? ((words[2 * j + (i >> 2)] >> (8 * (i & 3))) & 0xffu) * 32 : ((words[j] >> (4 * i)) & 0xfu) * 32];
+                    const int odd = lane & 1;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t y = __shfl_xor_sync(0xffffffffu, odd ? u[0][i] : u[1][i], 1);
+                        if (odd) u[0][i] = y;
+                        else u[1][i] = y;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {  // the even lane's row, then the odd lane's
+                        const int row = vec0 + (ev & ~1) + j;
+                        if (row < vec_per_kind)
+                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"((kind == 0 ? p.k16 : p.v16) + (size_t)row * HEAD_DIM + 32 * cc + 16 * odd),
+                                         "r"(u[j][0]), "r"(u[j][1]), "r"(u[j][2]), "r"(u[j][3]), "r"(u[j][4]), "r"(u[j][5]), "r"(u[j][6]), "r"(u[j][7]) : "memory");
                     }
                 }
                 if (ev_dst < 0) near_mask = 0u;  // (a vector past the end of the input is all zeros: every coordinate ON a bound)
