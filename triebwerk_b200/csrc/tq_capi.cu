@@ -1866,7 +1866,7 @@ static int engine_prefill_impl(tq_engine* e, int layer, int first_seq, int n_seq
 // May the append of these prompts make the attention's rows as well?  They fit the scratch as a whole, a tile of the append (128 / Hkv
 // tokens) is of one prompt, and the attention takes the call and is not the one that converts codes itself.  Up to 4096 tokens of 8 KV
 // heads, where the launch in between and its wait count for more than the append's slower stores (16/8 heads, 4-bit, with the rows made in a
-// launch of their own / by the append: 300 tokens 22.9 / 21.5 us a layer, 777 29.9 / 28.3, 1200 35.3 / 32.8, 2048 51.4 / 48.5, 4 x 1024 62.1 / 60.7; 2-bit 8 x 1024
+// launch of their own / by the append, before the steps that only the append's form gained from: 300 tokens 22.9 / 21.5 us a layer, 777 29.9 / 28.3, 1200 35.3 / 32.8, 2048 51.4 / 48.5, 4 x 1024 62.1 / 60.7; 2-bit 8 x 1024
 // 114 / 116, 32/8 8192 621 / 619).
 static bool engine_prefill_makes_rows(const tq_engine* e, int first_seq, int n_seq, const void* q, const void* out, int T, int q_stride) {
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;

@@ -31,7 +31,7 @@
 // Bound by the softmax threads (exponentials, tensor-memory loads) against the tensor core at long prompts, by the chain copy ->
 // S -> softmax -> O of a single block at short ones.  Per layer, 8 KV heads, cache write included, the one-block kernel with V
 // transposed through shared memory -> this one: fp16 8192 tokens 32 heads 2811 -> 478 us in runs of a few milliseconds (1150 TFLOP/s
-// of causal arithmetic), 557 (987) under the power cap of longer ones; 4-bit 777 tokens 16 heads 43.7 -> 27.0.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
+// of causal arithmetic), 557 (987) under the power cap of longer ones; 4-bit 777 tokens 16 heads 43.7 -> 26.3.  (With one thread per row, eight softmax warps, S read twice: 530, 379, 34.2.)
 #pragma once
 
 #include "tq_prefill_tc.cuh"

@@ -70,7 +70,8 @@ struct TcSmem {
     static constexpr uint32_t END = LIST1 + 4 * TC_LIST_CAP;
 };
 static_assert(TcSmem::CTRL + 64 <= TcSmem::GRID, "control words run into the bucket table");
-// ROWS16 (below): byte (4-bit) or nibble (2-bit) -> two centroids, eight copies; the largest V norm of each head in the tile
+// ROWS16 (below): byte (4-bit) or nibble (2-bit) -> two centroids, a copy per lane (eight, with four lanes on a bank: 777 tokens
+// 757 -> 748 us for 28 layers); the largest V norm of each head in the tile
 constexpr uint32_t TC_ROWS_LUT = 0x13000, TC_ROWS_TOP = TC_ROWS_LUT + 32768, TC_ROWS_END = TC_ROWS_TOP + 32;
 static_assert(TcSmem::END <= TC_ROWS_LUT, "the rows' table runs into the queues");
 constexpr size_t TC_DYN_SMEM = TcSmem::END;  // enough wherever the dynamic shared memory starts at or below TcSmem::DST0
@@ -903,7 +904,8 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                     near_mask = 0u;
                 }
                 if constexpr (ROWS16) {
-                    // 32 coordinates are two sectors: two lanes exchange halves, so that a store takes both sectors of a row next to each other
+                    // 32 coordinates are two sectors: two lanes exchange halves, so that a store takes both sectors of a row side by side
+                    // (16 rows of 256 bytes instead of 32: 777 tokens 749 -> 736 us for 28 layers)
                     const uint32_t* const lut = rows_lut + lane;
                     uint32_t u[2][8];
 #pragma unroll
