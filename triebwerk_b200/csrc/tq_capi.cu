@@ -300,6 +300,7 @@ struct LayerInputs {
     int static_rotation;        // R is not written by any kernel of the stream
     void* rotation_t;           // where R transposed is to go, or null (the caller has it)
     const int* seq_capacity;    // ragged slots: per-sequence row limits (device), or null
+    void* q_rot;                // where the rotated queries go: [G][H][128] as fp16, or as fp32 (attention_impl)
 };
 // (it moves the vectors 16 bytes at a time)
 static bool layer_form_ok(const void* q, const void* k, const void* v, int q_dim) {
@@ -346,8 +347,8 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
     lp.rotation_t = (__half*)layer->rotation_t;
     // The 2-bit scores' 16-bit queries come from fp32 ones where a sequence's block of them fits the kernel's area (16 heads).
     const bool wide = bits == 2 && num_kv_heads == 8 && num_heads <= 16;
-    if (wide) lp.q_rot32 = fw.w.q_rot;
-    else lp.q_rot16 = (__half*)fw.w.q_rot;
+    if (wide) lp.q_rot32 = (float*)layer->q_rot;
+    else lp.q_rot16 = (__half*)layer->q_rot;
     lp.positions = positions; lp.row_base = row_base; lp.seq_capacity = layer->seq_capacity; lp.status = p.status;
     lp.pos_value = pos_value; lp.max_seq_len = max_seq_len; lp.capacity_rows = max_seq_len;
     lp.G = G; lp.H = num_heads; lp.Hkv = num_kv_heads; lp.q_dim = q_dim;
@@ -607,7 +608,7 @@ static int compat_layer_attention(void* out, const void* q, const uint8_t* ck, c
     int r = cached_code_map(&tmK, ck, (long long)G * msl, kvp);
     if (r == TQ_OK) r = cached_code_map(&tmV, cv, (long long)G * msl, kvp);
     if (r != TQ_OK) return r;
-    LayerInputs in{q, nullptr, nullptr, rotation, 1, 0, fw.rot_t, nullptr};
+    LayerInputs in{q, nullptr, nullptr, rotation, 1, 0, fw.rot_t, nullptr, fw.w.q_rot};
     return attention_impl(out, tmK, tmV, ck, cv, k_norms, v_norms, fw.rot_t, pos, pos_value, nullptr, (long long)G * msl, msl, G, H, Hkv, q_dim, bits,
                           ws, ws_bytes, s, false, &in);
 }
@@ -1440,7 +1441,9 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     }
     // The layer form when the batch fits the kernel's shared-memory tile table (tq_engine_set_fused).
     if (e->fused && e->G <= FUSED_MAX_G && layer_form_ok(q, k, v, e->q_dim())) {
-        LayerInputs in{q, k, v, e->d_rotation_rep, ROT_COPIES, 1, nullptr, e->caps()};
+        // The rotated queries go where the whole-step form has its parts (132 floats per head and worker or sequence): the workspace's own
+        // area holds those of the two-launch form, which tq_engine_attend_layer reads.
+        LayerInputs in{q, k, v, e->d_rotation_rep, ROT_COPIES, 1, nullptr, e->caps(), e->step_partials};
         const int r = attention_impl(out, L.tmK, L.tmV, L.k, L.v, L.kn, L.vn, e->d_rotation_t, e->d_positions, -1, e->rb(),
                                      e->total_rows, e->msl, e->G, H, Hkv, e->q_dim(), e->kv_bits, e->workspace, e->ws_bytes,
                                      cs(s), use_pdl(), &in, f32, e->shared_active ? e->d_prefix_base : nullptr,
