@@ -90,6 +90,44 @@ def test_queries_with_one_large_coordinate():
         assert np.isnan(step[layer, beyond]).all()
 
 
+# the same through one layer's calls with more than 16 query heads: fp32 up to the fixed point, so finite where fp16 is not
+@pytest.mark.parametrize("H", [24, 32])
+def test_layer_calls_take_queries_beyond_fp16(H):
+    rng = np.random.default_rng(H)
+    G, msl = 216, 96  # (so many that the batch launcher streams too)
+    R = ops.rotation_matrix().numpy()
+    eng = tq.Engine(msl, 2, num_layers=1, num_heads=H, num_kv_heads=HKV, head_dim=D)
+    eng.alloc_batch(G, msl)
+    eng.reset()
+    assert tq.lib().tq_engine_decode_form(eng._h, 0) == 0
+    k, v = (rng.standard_normal((G, msl, HKV * D), dtype=np.float32).astype(np.float16) for _ in range(2))
+    eng.prefill_append_batch(0, 0, gu.dev(k[:, :msl - 1]), gu.dev(v[:, :msl - 1]))
+    pos = np.where(np.arange(G) < 108, 95, 0).astype(np.int32)
+    eng.set_positions(pos)
+    Rf, at = R.astype(np.float32), np.arange(G)
+    q = rng.standard_normal((G, H, D), dtype=np.float32)
+    q[:108] += 8 * Rf[at[:108] % D][:, None]
+    q[108:] = 65504 * np.where(Rf[at[108:] % D] < 0, -1, 1)[:, None]
+    assert (np.abs(q[108:, 0] @ Rf.T * 0.12751743).max(1) > 65520).sum() >= 36
+    q = q.astype(np.float16).reshape(G, H * D)
+    layer = gu.host(eng.decode_layer(0, gu.dev(q), gu.dev(k[at, pos]), gu.dev(v[at, pos])))
+    ck, cv, kn, vn = (gu.host(t) for t in eng.layer_cache(0))
+    ref, _ = tqo.attention_batch(q, ck, cv, kn, vn, R, pos, msl, H, HKV, D, 2)
+    hp.assert_attention_close(layer, ref, H, D, "decode_layer")
+    hp.assert_attention_close(gu.gpu_attention_batch(q, ck, cv, kn, vn, R, pos, msl, H, HKV, D, 2), ref, H, D, "batch launcher")
+    # one long sequence; one token, with codes that go with the rotated query's signs and the largest norm, has all the weight
+    n, j = 40000, 12345
+    ck, cv = (rng.integers(0, 256, (n, HKV * D // 4), dtype=np.uint8) for _ in range(2))
+    kn, vn = (rng.uniform(0.5, 1.0, (n, HKV)).astype(np.float16) for _ in range(2))
+    big = (65504 * np.where(Rf[7] < 0, -1, 1)).astype(np.float16)
+    ck[j] = np.tile(hp.pack_codes(np.where(big.astype(np.float32) @ Rf.T > 0, 3, 0), 2), HKV)
+    kn[j] = 4.0
+    q = np.tile(big, H)
+    ref, _ = tqo.attention_batch(q[None], ck, cv, kn, vn, R, np.array([n - 1], np.int32), n, H, HKV, D, 2)
+    hp.assert_attention_close(gu.gpu_attention_single(q, ck, cv, kn, vn, R, n - 1, n, H, HKV, D, 2)[None], ref, H, D, "single launcher")
+    assert eng.status() == 0
+
+
 # a slot that 8 CTAs serve with more than one block per warp; the launchers' clusters of one and two CTAs, one per SM
 @pytest.mark.parametrize("bits,H,msl,lengths,ctas", [(4, 16, 1536, [1500], 8), (2, 32, 2032, [2032], 8), (2, 32, 1024, [1023] * 8, 2), (4, 16, 512, [300, 512] * 8, 1)])
 def test_cluster_sizes_and_the_launchers(bits, H, msl, lengths, ctas):

@@ -95,7 +95,9 @@ struct AttnParams {
     // layer form (MODE 1): after layer_prep_kernel (tq_layer_prep.cuh), whose predecessors have finished when this kernel starts:
     // positions and cache rows are read before that launch has, but for the tiles it writes the new tokens to
     int appends;               // 1: layer_prep_kernel appends, to the last tile of every sequence
-    const float* q_rot32;      // rotated queries as fp32 [G][H][128] instead of q_rot16 (2-bit with eight KV heads, up to 16 heads)
+    const float* q_rot32;      // rotated queries as fp32 [G][H][128] instead of q_rot16 (2-bit with eight KV heads, for the planes), coordinate
+                               // 32 a + 4 b + c at 16 b + 4 a + c: what the four lanes of a head load together lies side by side (in the
+                               // order of the coordinates their loads met on one bank: 32 x 8192, 32 heads, 58.9 us a layer)
     int l2_ahead;              // tiles prefetched into L2 beyond the shared-memory ring
     // whole-step form (MODE 2): ONE launch streams the layers [layer0, layer0 + n_layers) back to back -- every worker
     // walks its slice of the tile list once per layer, its ring of stages never drains in between -- and only PUBLISHES its
@@ -138,10 +140,11 @@ struct RegionA {
     static constexpr uint32_t MERGE_OFF = 512;   // per group: hi + lo [16][MERGE_ROW] halves
     static constexpr uint32_t MERGE_GROUP_BYTES = 2 * 16 * MERGE_ROW * 2;  // 8704
     static constexpr uint32_t BLOCKS_OFF = MERGE_OFF + ATTN_GROUPS * MERGE_GROUP_BYTES;
-    // layer and whole-step form: tile table of the launch
-    static constexpr uint32_t FUSED_SCAN_OFF = BLOCKS_OFF;           // 32 ints of scan scratch
-    static constexpr uint32_t FUSED_TS_OFF = FUSED_SCAN_OFF + 128;   // tile_start[G + 1], G <= FUSED_MAX_G
-    static constexpr uint32_t FUSED_BLOCKS_OFF = FUSED_TS_OFF + 4096;
+    static constexpr uint32_t Q32_GROUP_BYTES = ATTN_MAX_HEADS * HEAD_DIM * 4;  // in the merge operands' place: a sequence's fp32 queries
+    // layer and whole-step form, `area` bytes per group in that place: tile table of the launch, then the stage blocks
+    __host__ __device__ static constexpr uint32_t scan_off(uint32_t area) { return MERGE_OFF + ATTN_GROUPS * area; }   // 32 ints of scan scratch
+    __host__ __device__ static constexpr uint32_t ts_off(uint32_t area) { return scan_off(area) + 128; }               // tile_start[G + 1], G <= FUSED_MAX_G
+    __host__ __device__ static constexpr uint32_t blocks_off(uint32_t area) { return ts_off(area) + 4096; }
 };
 constexpr int FUSED_MAX_G = 1023;
 
@@ -429,7 +432,9 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     // ---- shared memory map (absolute shared addresses) ----
     const uint32_t dyn_base = smem_u32(dyn_smem);
     const uint32_t a_base = (dyn_base + 1023u) & ~1023u;
-    const uint32_t blocks_a = (a_base + (PUBLISH ? RegionA::FUSED_BLOCKS_OFF : RegionA::BLOCKS_OFF) + 1023u) & ~1023u;
+    constexpr bool Q_WIDE = LAYER && PLANES;  // rotated queries as fp32 (two groups' areas still leave room for three stages)
+    constexpr uint32_t MERGE_AREA = Q_WIDE ? RegionA::Q32_GROUP_BYTES : RegionA::MERGE_GROUP_BYTES;
+    const uint32_t blocks_a = (a_base + (PUBLISH ? RegionA::blocks_off(MERGE_AREA) : RegionA::BLOCKS_OFF) + 1023u) & ~1023u;
     const uint32_t n_a = blocks_a < LUT_ABS ? (LUT_ABS - blocks_a) / stage_bytes : 0u;
     const uint32_t dyn_end = dyn_base + (uint32_t)ATTN_DYN_SMEM;
     const uint32_t n_b = dyn_end > REGION_B_ABS ? (dyn_end - REGION_B_ABS) / stage_bytes : 0u;
@@ -453,7 +458,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     const uint32_t cnt0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 8u);
     const uint32_t ebar0 = a_base + RegionA::CNT_OFF + (uint32_t)group * (ATTN_MAX_STAGES * 16u);  // copy warps: "part handed back" barriers
     const uint32_t ctrl_s = a_base + RegionA::CTRL_OFF + (uint32_t)group * 16u;
-    const uint32_t merge_s = a_base + RegionA::MERGE_OFF + (uint32_t)group * RegionA::MERGE_GROUP_BYTES;
+    const uint32_t merge_s = a_base + RegionA::MERGE_OFF + (uint32_t)group * MERGE_AREA;
 
     // (modes with a table of their own let their successor start only once they have themselves seen their predecessor finish)
     if (!PUBLISH) pdl_launch_dependents();
@@ -502,8 +507,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     // append kernel left in the workspace.
     const int* ts;
     if constexpr (PUBLISH) {
-        int* ts_s = reinterpret_cast<int*>(dyn_smem + (a_base - dyn_base) + RegionA::FUSED_TS_OFF);
-        int* scan_s = reinterpret_cast<int*>(dyn_smem + (a_base - dyn_base) + RegionA::FUSED_SCAN_OFF);
+        int* ts_s = reinterpret_cast<int*>(dyn_smem + (a_base - dyn_base) + RegionA::ts_off(MERGE_AREA));
+        int* scan_s = reinterpret_cast<int*>(dyn_smem + (a_base - dyn_base) + RegionA::scan_off(MERGE_AREA));
         int carry = 0;
         for (int base = 0; base < G; base += (int)blockDim.x) {
             const int gq = base + tid;
@@ -614,12 +619,11 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     // area of the worker, completion on a barrier of their own; the copy for the next segment goes out as soon as every
     // warp has taken its fragments of the current one
     const uint32_t qbar = a_base + 320u + 8u * (uint32_t)group;
-    const bool q_wide = LAYER && PLANES && p.q_rot32 != nullptr;
-    const uint32_t q_block_bytes = (uint32_t)p.H * HEAD_DIM * (q_wide ? 4u : 2u);
+    const uint32_t q_block_bytes = (uint32_t)p.H * HEAD_DIM * (Q_WIDE ? 4u : 2u);
     uint32_t q_par = 0;
     auto issue_queries = [&](int layer, int gq) {
         mbar_arrive_expect_tx(qbar, q_block_bytes);
-        const char* const src = q_wide ? reinterpret_cast<const char*>(p.q_rot32) : reinterpret_cast<const char*>(p.q_rot16);
+        const char* const src = Q_WIDE ? reinterpret_cast<const char*>(p.q_rot32) : reinterpret_cast<const char*>(p.q_rot16);
         bulk_load(merge_s, src + ((size_t)layer * p.G + (size_t)gq) * q_block_bytes, q_block_bytes, qbar);
     };
     int consumed = 0;
@@ -776,7 +780,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         // a byte's coordinate j is worth 2^(2 j + b) where it stands: the query of that plane is divided by it (by 2^(2 (j mod 2) + b): the
         // coordinates 0, 1 and 2, 3 have sums of their own, 16 apart).  The sum's offset is minus half the sum with all bits set.
         // Rounding: half a weight (1 and 4, 2 and 8) of the 32639 C_b / C0 steps to the largest coordinate: 1.5e-5 to 6.6e-5 of it at most.
-        // Queries with an infinity (rotated and scaled they do not fit fp16, in the whole-step form) give NaN.
+        // The queries are fp32, but in the whole-step form, which holds them as fp16: there up to 4.9e-4 of every coordinate on top, and
+        // queries that do not fit fp16 rotated and scaled, infinities here, give NaN.
         auto make_planes = [&](const float (&x)[32]) {
             constexpr float C0 = 0.13351f - 0.04003f, C1 = 0.13351f + 0.04003f;
             uint32_t top = 0u;  // of the magnitudes' bits: an infinity or a NaN comes out on top
@@ -818,12 +823,12 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         // lane (gl, t4): the 32 coordinates 32*t4 .. of its head from the merge area, rows `pitch` bytes apart
         auto take_fragments = [&]() {
             constexpr uint32_t pitch = HEAD_DIM * 2u;
-            if (q_wide) {
+            if constexpr (Q_WIDE) {
                 float x[32];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                    if (q_on && !dead) u = ldsv128(merge_s + (uint32_t)(head * grp + q_col) * (HEAD_DIM * 4u) + (uint32_t)(32 * t4 + 4 * i) * 4u);
+                    if (q_on && !dead) u = ldsv128(merge_s + (uint32_t)(head * grp + q_col) * (HEAD_DIM * 4u) + (uint32_t)(4 * i + t4) * 16u);
                     x[4 * i] = __uint_as_float(u.x); x[4 * i + 1] = __uint_as_float(u.y);
                     x[4 * i + 2] = __uint_as_float(u.z); x[4 * i + 3] = __uint_as_float(u.w);
                 }

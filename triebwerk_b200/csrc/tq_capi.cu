@@ -345,9 +345,8 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
     lp.new_k = (const __half*)layer->k; lp.new_v = (const __half*)layer->v; lp.q = (const __half*)layer->q;
     lp.rotation = (const __half*)layer->rotation; lp.rot_copies = layer->rot_copies; lp.static_rotation = layer->static_rotation;
     lp.rotation_t = (__half*)layer->rotation_t;
-    // The 2-bit scores' 16-bit queries come from fp32 ones where a sequence's block of them fits the kernel's area (16 heads).
-    const bool wide = bits == 2 && num_kv_heads == 8 && num_heads <= 16;
-    if (wide) lp.q_rot32 = (float*)layer->q_rot;
+    // (the 2-bit scores' fixed-point queries, eight KV heads, come from fp32 ones)
+    if (bits == 2 && num_kv_heads == 8) lp.q_rot32 = (float*)layer->q_rot;
     else lp.q_rot16 = (__half*)layer->q_rot;
     lp.positions = positions; lp.row_base = row_base; lp.seq_capacity = layer->seq_capacity; lp.status = p.status;
     lp.pos_value = pos_value; lp.max_seq_len = max_seq_len; lp.capacity_rows = max_seq_len;

@@ -33,7 +33,7 @@ struct LayerPrepParams {
     int rot_copies;              // CTA b reads copy b % rot_copies: all of them fetch the same 32 KB at once
     int static_rotation;         // R is not written by any kernel of the stream: fetched before the wait
     __half* q_rot16;             // [G][H][128], or as fp32:
-    float* q_rot32;
+    float* q_rot32;              // (in AttnParams::q_rot32's order)
     __half* rotation_t;          // or null: R transposed goes here, for the merge
     const int* positions;        // device [G] or null: pos_value
     const long long* row_base;   // [G] or null: g * max_seq_len
@@ -146,10 +146,10 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) layer_prep_kernel(const Layer
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const float y0 = (c[i][0][2 * r] + c[i][1][2 * r]) * sc, y1 = (c[i][0][2 * r + 1] + c[i][1][2 * r + 1]) * sc;
-                    const size_t at = (size_t)((item - n_app) * 16 + gl + 8 * r) * HEAD_DIM + 8 * (2 * warp + i) + 2 * t4;
+                    const size_t vec = (size_t)((item - n_app) * 16 + gl + 8 * r) * HEAD_DIM;
                     if (!on[r]) continue;
-                    if (p.q_rot32) *reinterpret_cast<float2*>(p.q_rot32 + at) = make_float2(y0, y1);
-                    else *reinterpret_cast<__half2*>(p.q_rot16 + at) = __floats2half2_rn(y0, y1);
+                    if (p.q_rot32) *reinterpret_cast<float2*>(p.q_rot32 + vec + 16 * (4 * (warp & 1) + 2 * i + (t4 >> 1)) + 4 * (warp >> 1) + 2 * (t4 & 1)) = make_float2(y0, y1);
+                    else *reinterpret_cast<__half2*>(p.q_rot16 + vec + 8 * (2 * warp + i) + 2 * t4) = __floats2half2_rn(y0, y1);
                 }
             continue;
         }
