@@ -1344,6 +1344,8 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const MergeParams p
 // head, its parts' loads in flight together.  Under the attention's last tiles, before the wait: R's fragments and which workers had
 // a part, from the positions (which that launch does not write; what came before it has finished when this one starts).
 // From the wait to the end 2.4 to 3.1 us (32 x 8192 tokens, 32 heads); by the last arriving worker inside the attention 5.6.
+// At least two CTAs per SM: at 141 registers, one, the merge was longer than the attention where there are many sequences (2-bit, 32/8
+// heads, 1000 x 100 tokens 73 us of a layer's 140.6; with two 113.1 a layer; 128 x 300 32.6 -> 29.2).
 struct MergeLayerParams {
     const float* partials;       // [workers + G][H][PART_STRIDE]
     const int* positions;        // device [G] or null: pos_value
@@ -1354,7 +1356,7 @@ struct MergeLayerParams {
     int workers;                 // workers of the attention launch
 };
 constexpr int MERGE_HEADS = 8;
-__global__ void __launch_bounds__(MERGE_HEADS * 32) merge_layer_kernel(const MergeLayerParams p) {
+__global__ void __launch_bounds__(MERGE_HEADS * 32, 2) merge_layer_kernel(const MergeLayerParams p) {
     __shared__ __align__(16) __half a_op[2 * MERGE_HEADS * MERGE_ROW];  // rows 0-7: high parts, 8-15: low parts
     __shared__ int sums[2][MERGE_HEADS];
     pdl_launch_dependents();
