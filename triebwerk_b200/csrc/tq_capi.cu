@@ -31,11 +31,8 @@ static inline bool cluster_on() {
     static const bool on = !(getenv("TQ_CLUSTER") && atoi(getenv("TQ_CLUSTER")) == 0);
     return on;
 }
-// Calls without an engine: the streaming kernels' clears and writes are launches of their own there for fp16 rows (3 us); packed, the
-// layer form has the same three, and the cluster form, which cannot start under the appends, is 3 us ahead in 2-bit only (2-bit
-// 32/4 heads 128 x 600 tokens 38.9 us a layer with the appends, streaming 40.9; 4-bit 32/4 48 x 2500 58.9 / 36.3, 16/8 64 x 1500 64.7 / 44.4).
 static inline bool compat_cluster_size(int bits, int G, int H, int Hkv, int max_tokens) {
-    return cluster_on() && cluster_layer_faster(bits, G, Hkv, H / Hkv, (long long)G * max_tokens, max_tokens, bits == 4 ? 0.0 : 3.0);
+    return cluster_on() && cluster_layer_faster(bits, G, Hkv, H / Hkv, (long long)G * max_tokens, max_tokens, LayerCaller::Launchers);
 }
 
 extern "C" {
@@ -1408,7 +1405,7 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
     float* const f32 = e->out_f32 ? e->out_f32 + (size_t)layer * e->G * H * HEAD_DIM : nullptr;
     // Head layouts outside the streaming kernels', and small batches of any layout: the cluster form, one launch.
     if (engine_cluster_ok(e, q, k, v, out) &&
-        (!fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, 0.0))))
+        (!fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, LayerCaller::Engine))))
         return engine_cluster_layers(e, layer, 1, 1, q, k, v, out, chained, cs(s));
     if (e->kv_bits == 0) {
         // (the write clears the attention's tickets, which then starts under it)
@@ -1552,7 +1549,7 @@ static bool engine_step_small(const tq_engine* e, StepInputs inputs) {
 int tq_engine_decode_form(const tq_engine* e, int whole_step) {
     if (!e || !e->arena || e->G == 0) return TQ_ERR_STATE;
     const int H = e->shape.num_heads, Hkv = e->shape.num_kv_heads;
-    const bool layer = !fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, 0.0));
+    const bool layer = !fast_shape(H, Hkv, e->kv_bits != 0) || (cluster_on() && cluster_layer_faster(e->kv_bits, e->G, Hkv, H / Hkv, e->total_rows, e->msl, LayerCaller::Engine));
     if (!e->fused || !(whole_step ? engine_step_small(e, StepInputs::Plain) : layer)) return 0;
     return cluster_launch_split(e->kv_bits, e->G, whole_step ? e->shape.num_layers : 1, H, Hkv, e->msl);
 }

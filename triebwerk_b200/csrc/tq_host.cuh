@@ -486,15 +486,22 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
 // and that form starts 7 us later.  Above 640 clusters their number counts for more than in the lines fitted below it (128 x 64
 // tokens, 16/8 heads, 4-bit 25.7 / 19.7 us, 96 x 64 19.8 / 19.0, 64 x 64 13.5 / 17.2; 32/8 heads 128 x 64 26.8 / 24.9, 96 x 64 20 / 23;
 // fp16 128 x 300 43.0 / 39.1, 96 x 300 32.6 / 33.2).
-// fp16 slots of one chunk of the streaming form, which has nothing to merge there and starts under the write of the new rows, go to it
-// where the cluster form has one CTA per sequence and KV head (cluster / streaming: 16/8 heads 12 x 500 tokens 11.9 / 9.8 us, 48 x 300 21.6 /
-// 17.1, 96 x 500 44.6 / 37.4, 32/8 24 x 500 14.8 / 13.4), unless those just fill two CTAs per SM (32/8 32 x 300 11.4 / 11.9).
-// `extra`: us the streaming form's launches cost on top.
-inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, double extra) {
+// fp16 slots of one chunk of the streaming form, which has nothing to merge there and in an engine starts under the write of the new rows, go
+// to it where the cluster form has one CTA per sequence and KV head and its warps enough tiles (cluster / streaming, slots of 288, 352, 416 and
+// 512 rows: 16/8 heads 96 clusters 5.9 / 6.7, 7.1 / 7.2, 8.9 / 7.9, 11.7 / 9.3 us, 160 7.5 / 8.0, 10.5 / 10.0, 13.0 / 10.9, 14.4 / 11.8, 384 18.2 / 16.6,
+// 22.3 / 18.5, 26.5 / 20.3, 29.7 / 23.0; 8/8 96 5.6 / 7.3, 6.9 / 7.9, 8.5 / 8.6, 11.3 / 10.0, 512 18.3 / 19.2, 22.4 / 21.1), unless those just
+// fill two CTAs per SM (16/8 296 10.1 / 11.9, 12.1 / 13.0, 14.3 / 14.7, 16.1 / 17.0).
+// Launchers: their streaming fp16 form has its clears and writes in launches of their own (3 us); packed, the layer form has the same
+// three launches, and the cluster form, which cannot start under the appends, is 3 us ahead in 2-bit only (2-bit 32/4 heads 128 x 600
+// tokens 38.9 us a layer with the appends, streaming 40.9; 4-bit 32/4 48 x 2500 58.9 / 36.3, 16/8 64 x 1500 64.7 / 44.4).
+enum class LayerCaller { Engine, Launchers };
+inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, LayerCaller caller) {
     const long long clusters = (long long)G * Hkv, sms = device_props().sm_count;
     const int S = cluster_split(bits, clusters, heads, max_tokens, true);
     const double chain = ((max_tokens + 15) / 16) / (double)(S * CD_WARPS), turns = (double)((clusters * S + sms - 1) / sms);
-    if (bits == 0 && extra == 0.0 && S == 1 && heads <= 4 && max_tokens <= FP16_CHUNK && max_tokens > FP16_CHUNK / 2 && (2 * clusters <= 3 * sms || clusters > 2 * sms))
+    const double extra = caller == LayerCaller::Launchers && bits != 4 ? 3.0 : 0.0;  // us the streaming form's launches cost on top
+    if (bits == 0 && caller == LayerCaller::Engine && S == 1 && heads <= 4 && max_tokens <= FP16_CHUNK && (2 * clusters <= 3 * sms || clusters > 2 * sms) &&
+        chain > (clusters > 2 * sms ? 2.2 : 4 * clusters > 3 * sms ? 2.5 : 2.8))
         return false;
     if (bits == 0) return (heads > 4 ? 0.5 : 1.0) * chain < 7.0 + 1.5 * turns + extra && !(clusters > 768 && chain > 2.0);
     const double many = heads > 2 ? 0.0015 * std::max(0ll, clusters - 800) : 0.02 * std::max(0ll, clusters - 640);
