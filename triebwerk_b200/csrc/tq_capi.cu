@@ -1521,7 +1521,7 @@ static bool engine_step_small(const tq_engine* e, StepInputs inputs) {
     if (!fast_shape(H, Hkv, e->kv_bits != 0)) return true;
     if (!cluster_on()) return false;
     const long long clusters = (long long)e->G * Hkv * NL;
-    const int S = cluster_split(e->kv_bits, clusters, heads, e->msl, false);
+    const int S = cluster_split(e->kv_bits, clusters, heads, e->msl, false, true);
     if (e->kv_bits == 0) {
         const double tiles = ((e->msl + 15) / 16) / (double)(CD_WARPS * S);
         return 600.0 * tiles + 2.0 * clusters + 0.002 * (double)e->total_rows * Hkv * NL < 2000.0 + 10000.0 * NL;

@@ -463,10 +463,14 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
 // above 4 for fp16, whose rows are four times as long.  Not with more than 4 query heads per cluster in a packed mode: the warps'
 // partial results leave room for one CTA per SM there.
 // Where those are one layer's (`layer`) and 4-bit, the next layer's clusters of 8 and 16 find no room either beside this one's: as many
-// as leave it half of the SMs (32/4 heads, 2 x 4000 tokens 17.1 -> 10.0 us, 2 x 8000 21.1 -> 13.9, 4 x 4000 20.1 -> 15.4).
-inline int cluster_split(int bits, long long clusters, int heads, int max_tokens, bool layer) {
+// as leave it half of the SMs (32/4 heads, 2 x 4000 tokens 17.1 -> 10.0 us, 2 x 8000 21.1 -> 13.9, 4 x 4000 20.1 -> 15.4).  Layouts without a
+// streaming form (`streams` false) keep clusters of 8 where 4 would have chains of more than 20 tiles (40/8 heads, 16 -> 8 CTAs: one sequence
+// of 2048 tokens 13.8 -> 8.3 us, 12000 25.6 -> 20.4, 32000 52.1 -> 49.0; 8 -> 4: two of 520 11.5 -> 5.9, 6000 25.2 -> 22.1, 10000 37.5 -> 37.0, 12000
+// 43.1 -> 44.0, 16000 53.0 -> 56.5).
+inline int cluster_split(int bits, long long clusters, int heads, int max_tokens, bool layer, bool streams) {
     const long long sms = device_props().sm_count, blocks = (max_tokens + 15) / 16;
-    auto fit = [&](int n) { return n >= 8 && layer && bits == 4 && heads > 4 ? (sms - 20) / 2 : sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
+    auto half = [&](int n) { return n >= 8 && layer && bits == 4 && heads > 4 && (streams || n > 8 || blocks <= 20 * 4 * CD_WARPS); };
+    auto fit = [&](int n) { return half(n) ? (sms - 20) / 2 : sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
     int S = 1;
     auto longer = [&](int n) { return n == 8 ? 2 * n * CD_WARPS <= blocks : n * CD_WARPS < blocks; };
     while (S < CD_MAX_CLUSTER && longer(S) && clusters * S * 2 <= fit(2 * S)) S *= 2;
@@ -497,7 +501,7 @@ inline int cluster_split(int bits, long long clusters, int heads, int max_tokens
 enum class LayerCaller { Engine, Launchers };
 inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long rows, int max_tokens, LayerCaller caller) {
     const long long clusters = (long long)G * Hkv, sms = device_props().sm_count;
-    const int S = cluster_split(bits, clusters, heads, max_tokens, true);
+    const int S = cluster_split(bits, clusters, heads, max_tokens, true, true);
     const double chain = ((max_tokens + 15) / 16) / (double)(S * CD_WARPS), turns = (double)((clusters * S + sms - 1) / sms);
     const double extra = caller == LayerCaller::Launchers && bits != 4 ? 3.0 : 0.0;  // us the streaming form's launches cost on top
     if (bits == 0 && caller == LayerCaller::Engine && S == 1 && heads <= 4 && max_tokens <= FP16_CHUNK && (2 * clusters <= 3 * sms || clusters > 2 * sms) &&
@@ -511,8 +515,8 @@ inline bool cluster_layer_faster(int bits, int G, int Hkv, int heads, long long 
 // split_layers: the number of layers the cut of the work is made for (a step's layers give the same bits in one launch or several)
 inline int cluster_launch_split(int bits, int G, int split_layers, int H, int Hkv, int max_tokens) {
     const int head_blocks = (H / Hkv + CD_HEADS - 1) / CD_HEADS;
-    const bool one_per_sm = bits != 0 && !fast_shape(H, Hkv, true);  // (EXACT, packed: as with 8 heads)
-    return cluster_split(bits, (long long)G * split_layers * Hkv * head_blocks, one_per_sm ? CD_HEADS : std::min(CD_HEADS, H / Hkv), max_tokens, split_layers == 1);
+    const bool streams = fast_shape(H, Hkv, bits != 0), one_per_sm = bits != 0 && !streams;  // (EXACT, packed: as with 8 heads)
+    return cluster_split(bits, (long long)G * split_layers * Hkv * head_blocks, one_per_sm ? CD_HEADS : std::min(CD_HEADS, H / Hkv), max_tokens, split_layers == 1, streams);
 }
 template <bool HOST, bool EXACT>
 inline int launch_cluster_decode_e(int bits, const ClusterDecodeParams& p, int layers, int split_layers, int max_tokens, cudaStream_t s, bool pdl) {
