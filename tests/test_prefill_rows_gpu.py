@@ -44,6 +44,26 @@ def test_rows_made_by_the_append_equal_those_made_from_the_cache(bits, H, Hkv, T
     assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("bits,H,Hkv,T", [(4, 16, 8, 4095), (2, 32, 4, 8190)])
+def test_rows_of_more_tiles_than_ctas(bits, H, Hkv, T):
+    """A CTA of the append has two tiles: the largest V norms of the first, far above or below the second's, are the first's alone."""
+    rng = np.random.default_rng(T)
+    msl = -(-T // 32) * 32
+    eng = tq.Engine(msl, bits, num_layers=1, num_heads=H, num_kv_heads=Hkv, head_dim=D)
+    eng.alloc_batch(1, msl)
+    k, v, q = _draw(rng, T, Hkv * D), _draw(rng, T, Hkv * D), _draw(rng, T, H * D)
+    v *= torch.exp2(torch.from_numpy(rng.integers(-6, 10, -(-T // 16))).cuda().half().repeat_interleave(16)[:T, None])
+    out = torch.empty_like(q)
+    want = None
+    for _ in range(3):
+        eng.prefill_layer(0, 0, q, k, v, out)
+        assert eng.status() == 0
+        got = out.cpu().numpy()
+        if want is None: want = _launcher(eng, 0, 0, q, msl, H, Hkv, bits)
+        assert np.isfinite(got).all()
+        assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+
+
 def test_values_that_are_not_numbers_reach_no_earlier_query():
     bits, H, Hkv, T, msl = 4, 16, 8, 300, 512
     rng = np.random.default_rng(3)

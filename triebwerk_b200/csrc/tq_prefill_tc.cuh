@@ -71,8 +71,9 @@ struct TcSmem {
 };
 static_assert(TcSmem::CTRL + 64 <= TcSmem::GRID, "control words run into the bucket table");
 // ROWS16 (below): byte (4-bit) or nibble (2-bit) -> two centroids, a copy per lane (eight, with four lanes on a bank: 777 tokens
-// 757 -> 748 us for 28 layers); the largest V norm of each head in the tile
-constexpr uint32_t TC_ROWS_LUT = 0x13000, TC_ROWS_TOP = TC_ROWS_LUT + 32768, TC_ROWS_END = TC_ROWS_TOP + 32;
+// 757 -> 748 us for 28 layers); the largest V norm of each head in the tile, for tiles of either parity: a warp may be at the next tile's
+// norms while another still has this tile's to read
+constexpr uint32_t TC_ROWS_LUT = 0x13000, TC_ROWS_TOP = TC_ROWS_LUT + 32768, TC_ROWS_END = TC_ROWS_TOP + 64;
 static_assert(TcSmem::END <= TC_ROWS_LUT, "the rows' table runs into the queues");
 constexpr size_t TC_DYN_SMEM = TcSmem::END;  // enough wherever the dynamic shared memory starts at or below TcSmem::DST0
 constexpr int TC_CTAS_PER_SM = 3;
@@ -376,7 +377,7 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
     uint32_t* const rows_lut = reinterpret_cast<uint32_t*>(gbase + TC_ROWS_LUT);
     uint32_t* const rows_top = reinterpret_cast<uint32_t*>(gbase + TC_ROWS_TOP);
     if constexpr (ROWS16) {
-        if (tid < 8) rows_top[tid] = 0u;
+        if (tid < 16) rows_top[tid] = 0u;
         for (int i = tid; i < (bits == 4 ? 256 : 16) * 8; i += TC_THREADS) {  // (a copy for every lane)
             const int e = i >> 3;
             const uint32_t u = bits == 4 ? pack_half2(kCent4[e & 15], kCent4[e >> 4]) : pack_half2(kCent2[e & 3], kCent2[(e >> 2) & 3]);
@@ -813,7 +814,7 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
                 const __half n = vec0 + settle_v < vec_per_kind ? __float2half_rn(sqrt_approx_ftz(my_tt)) : __ushort_as_half((unsigned short)0);
                 const int t = t0 + dtok;
                 p.norms[(((long long)seq0 * p.Hkv + dhead) * p.norm_tiles + (t >> 7)) * PFT_NORMS + kind * PFT_KT + (t & (PFT_KT - 1))] = __half2float(n);
-                if (kind == 1) atomicMax(&rows_top[dhead], (uint32_t)__half_as_ushort(n));
+                if (kind == 1) atomicMax(&rows_top[8 * b + dhead], (uint32_t)__half_as_ushort(n));
             }
             dst_s[settle_v] = my_dst;
             // (an all-zero vector -- padding, say -- has every coordinate ON the bound 0: 128 exact chains, all with the result
@@ -839,8 +840,8 @@ prefill_append_tc_kernel(const __grid_constant__ CUtensorMap tm_k_in, const __gr
             auto tops = [&](int head) { return reinterpret_cast<unsigned short*>(p.norms + (((long long)seq0 * p.Hkv + head) * p.norm_tiles + (t0 >> 7)) * PFT_NORMS + 2 * PFT_KT); };
             const int left = t0 + TPT >= p.T ? PFT_KT - (t0 & (PFT_KT - 1)) - TPT : 0;  // tokens of the last tile nobody brings
             if (kind == 1 && tid < p.Hkv) {
-                tops(tid)[part] = (unsigned short)rows_top[tid];
-                rows_top[tid] = 0u;
+                tops(tid)[part] = (unsigned short)rows_top[8 * b + tid];
+                rows_top[8 * b + tid] = 0u;  // (used again by the tile after the next, behind that one's barrier)
                 for (int i = p.Hkv; part == 0 && i < 8; ++i) tops(tid)[i] = 0;
                 for (int i = part + 1; left > 0 && i < p.Hkv; ++i) tops(tid)[i] = 0;
             }
