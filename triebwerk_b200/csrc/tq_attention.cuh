@@ -207,6 +207,18 @@ __device__ __forceinline__ uint4 ldg128_now(const void* src) {
     asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(src));
     return r;
 }
+// The same, and a word, past L1: for what an earlier kernel of the stream has written that is known to have finished, though this launch has
+// not waited yet.
+__device__ __forceinline__ uint4 ldg128_l2(const void* src) {
+    uint4 r;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(src));
+    return r;
+}
+__device__ __forceinline__ int ldg32_l2(const int* src) {
+    int r;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(r) : "l"(src));
+    return r;
+}
 __device__ __forceinline__ float ldsp_h2f(uint32_t addr) {  // one fp16 from shared memory as float
     unsigned short h;
     asm("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(addr));
@@ -467,7 +479,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 
     // (layer form: the first positions are on their way while the look-up table is written)
     int first_pos = p.pos_value;
-    if (LAYER && p.positions && tid < G) asm volatile("ld.global.u32 %0, [%1];" : "=r"(first_pos) : "l"(p.positions + tid));
+    if (LAYER && p.positions && tid < G) first_pos = ldg32_l2(p.positions + tid);
     // ---- byte -> centroid table, one column per lane ----
     if (TQ_DBG(16)) {
     } else if (BITS == 4) {
@@ -514,7 +526,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             const int gq = base + tid;
             int n = 0;
             if (gq < G) {
-                int pos = LAYER && base == 0 ? first_pos : p.positions ? p.positions[gq] : p.pos_value;
+                int pos = LAYER && base == 0 ? first_pos : p.positions ? __ldcg(p.positions + gq) : p.pos_value;
                 if (pos < 0) pos = 0;
                 n = (pos + TILE_TOKENS) / TILE_TOKENS;
             }
@@ -1342,7 +1354,9 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const MergeParams p
 
 // The merge of one layer's partials (mode 1), the tail of that layer: bound by latency.  One CTA per (sequence, 8 heads), a warp per
 // head, its parts' loads in flight together.  Under the attention's last tiles, before the wait: R's fragments and which workers had
-// a part, from the positions (which that launch does not write; what came before it has finished when this one starts).
+// a part, from the positions (which that launch does not write).  Both may be the work of a launch shortly before: the attention lets this one
+// start behind its own wait, when layer_prep_kernel, which transposes a caller's R, and all before that have finished; the loads pass
+// by L1, in which an SM may still have what it read in the layer before.
 // From the wait to the end 2.4 to 3.1 us (32 x 8192 tokens, 32 heads); by the last arriving worker inside the attention 5.6.
 // At least two CTAs per SM: at 141 registers, one, the merge was longer than the attention where there are many sequences (2-bit, 32/8
 // heads, 1000 x 100 tokens 73 us of a layer's 140.6; with two 113.1 a layer; 128 x 300 32.6 -> 29.2).
@@ -1368,9 +1382,9 @@ __global__ void __launch_bounds__(MERGE_HEADS * 32, 2) merge_layer_kernel(const 
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int m = 0; m < 4; ++m)  // (step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3, on both sides)
-            bf[i][m] = ldg128_now(reinterpret_cast<const uint4*>(p.rotation_t + (size_t)(8 * (warp + MERGE_HEADS * i) + gl) * HEAD_DIM) + t4 + 4 * m);
+            bf[i][m] = ldg128_l2(reinterpret_cast<const uint4*>(p.rotation_t + (size_t)(8 * (warp + MERGE_HEADS * i) + gl) * HEAD_DIM) + t4 + 4 * m);
     auto tiles_of = [&](int i) {
-        const int pos = p.positions ? p.positions[i] : p.pos_value;
+        const int pos = p.positions ? __ldcg(p.positions + i) : p.pos_value;
         return ((pos < 0 ? 0 : pos) + TILE_TOKENS) / TILE_TOKENS;
     };
     int before = 0, all = 0;  // tiles before sequence g, of all sequences
