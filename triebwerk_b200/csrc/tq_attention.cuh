@@ -1369,26 +1369,33 @@ struct MergeLayerParams {
     int pos_value, G, H, q_dim;
     int workers;                 // workers of the attention launch
 };
-constexpr int MERGE_HEADS = 8;
-__global__ void __launch_bounds__(MERGE_HEADS * 32, 2) merge_layer_kernel(const MergeLayerParams p) {
-    __shared__ __align__(16) __half a_op[2 * MERGE_HEADS * MERGE_ROW];  // rows 0-7: high parts, 8-15: low parts
-    __shared__ int sums[2][MERGE_HEADS];
+// HEADS = 1: a CTA per (sequence, head) instead, an eighth of its parts for every warp: for few sequences, which are cut into many parts
+// each (launch_merge_layer, tq_host.cuh).
+constexpr int MERGE_WARPS = 8;
+template <int HEADS>
+__global__ void __launch_bounds__(MERGE_WARPS * 32, 2) merge_layer_kernel(const MergeLayerParams p) {
+    static_assert(HEADS == 1 || HEADS == MERGE_WARPS, "a warp per head, or all warps for one");
+    constexpr bool SPLIT = HEADS == 1;
+    __shared__ __align__(16) __half a_op[2 * MERGE_WARPS * MERGE_ROW];  // rows 0-7: high parts, 8-15: low parts (SPLIT: rows 0 and 8 alone are used)
+    __shared__ int sums[2][MERGE_WARPS];
+    __shared__ float4 acc_s[SPLIT ? MERGE_WARPS : 1][32];
+    __shared__ float2 ml_s[SPLIT ? MERGE_WARPS : 1];
     pdl_launch_dependents();
     const int g = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane >> 2, t4 = lane & 3;
-    const int h = MERGE_HEADS * (int)blockIdx.y + warp;
+    const int h = HEADS * (int)blockIdx.y + (SPLIT ? 0 : warp);
     // out[h][d] = sum_k a[h][k] R[k][d]: B fragments of the column blocks `warp` and `warp + 8`
     uint4 bf[2][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int m = 0; m < 4; ++m)  // (step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3, on both sides)
-            bf[i][m] = ldg128_l2(reinterpret_cast<const uint4*>(p.rotation_t + (size_t)(8 * (warp + MERGE_HEADS * i) + gl) * HEAD_DIM) + t4 + 4 * m);
+            bf[i][m] = ldg128_l2(reinterpret_cast<const uint4*>(p.rotation_t + (size_t)(8 * (warp + MERGE_WARPS * i) + gl) * HEAD_DIM) + t4 + 4 * m);
     auto tiles_of = [&](int i) {
         const int pos = p.positions ? __ldcg(p.positions + i) : p.pos_value;
         return ((pos < 0 ? 0 : pos) + TILE_TOKENS) / TILE_TOKENS;
     };
     int before = 0, all = 0;  // tiles before sequence g, of all sequences
-    for (int i = threadIdx.x; i < p.G; i += MERGE_HEADS * 32) {
+    for (int i = threadIdx.x; i < p.G; i += MERGE_WARPS * 32) {
         const int n = tiles_of(i);
         all += n;
         before += i < g ? n : 0;
@@ -1403,16 +1410,17 @@ __global__ void __launch_bounds__(MERGE_HEADS * 32, 2) merge_layer_kernel(const 
     __syncthreads();
     all = before = 0;
 #pragma unroll
-    for (int w = 0; w < MERGE_HEADS; ++w) {
+    for (int w = 0; w < MERGE_WARPS; ++w) {
         all += sums[0][w];
         before += sums[1][w];
     }
     // owners of the sequence's first and last tile, as in the attention kernel's cut of the list
     const long long W = attention_workers(p.workers, all, p.G);
     const int first_w = (int)(((long long)(before + 1) * W - 1) / all);
-    const int parts = (int)(((long long)(before + own) * W - 1) / all) - first_w + 1;
-    const float* const part0 = p.partials + ((size_t)(first_w + g) * p.H + h) * PART_STRIDE;
+    const int all_parts = (int)(((long long)(before + own) * W - 1) / all) - first_w + 1;
+    const int part_lo = SPLIT ? all_parts * warp / MERGE_WARPS : 0, parts = SPLIT ? all_parts * (warp + 1) / MERGE_WARPS - part_lo : all_parts;
     const size_t pstride = (size_t)p.H * PART_STRIDE;
+    const float* const part0 = p.partials + ((size_t)(first_w + g) * p.H + h) * PART_STRIDE + (size_t)part_lo * pstride;
     pdl_wait();
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     if (h < p.H) {
@@ -1444,11 +1452,30 @@ __global__ void __launch_bounds__(MERGE_HEADS * 32, 2) merge_layer_kernel(const 
                 a.z = fmaf(wj, v[j].z, a.z); a.w = fmaf(wj, v[j].w, a.w);
             }
         }
+        if constexpr (SPLIT) {  // the warps' shares meet in shared memory, in their order
+            acc_s[warp][lane] = a;
+            if (lane == 0) ml_s[warp] = make_float2(M, Z);
+            __syncthreads();
+            M = ml_s[0].x;
+#pragma unroll
+            for (int w = 1; w < MERGE_WARPS; ++w) M = fmaxf(M, ml_s[w].x);
+            a = make_float4(0.f, 0.f, 0.f, 0.f);
+            Z = 0.0f;
+#pragma unroll
+            for (int w = 0; w < MERGE_WARPS; ++w) {
+                const float f = ex2_approx(ml_s[w].x - M);
+                const float4 v = acc_s[w][lane];
+                Z = fmaf(ml_s[w].y, f, Z);
+                a.x = fmaf(v.x, f, a.x); a.y = fmaf(v.y, f, a.y); a.z = fmaf(v.z, f, a.z); a.w = fmaf(v.w, f, a.w);
+            }
+        }
         const float inv = 1.0f / (Z + 1e-8f);
         a.x *= inv; a.y *= inv; a.z *= inv; a.w *= inv;
     }
-    *reinterpret_cast<uint2*>(a_op + warp * MERGE_ROW + 4 * lane) = make_uint2(pack_half2(a.x, a.y), pack_half2(a.z, a.w));
-    *reinterpret_cast<uint2*>(a_op + (warp + MERGE_HEADS) * MERGE_ROW + 4 * lane) = make_uint2(pack_low_half2(a.x, a.y), pack_low_half2(a.z, a.w));
+    if (!SPLIT || warp == 0) {
+        *reinterpret_cast<uint2*>(a_op + warp * MERGE_ROW + 4 * lane) = make_uint2(pack_half2(a.x, a.y), pack_half2(a.z, a.w));
+        *reinterpret_cast<uint2*>(a_op + (warp + MERGE_WARPS) * MERGE_ROW + 4 * lane) = make_uint2(pack_low_half2(a.x, a.y), pack_low_half2(a.z, a.w));
+    }
     __syncthreads();
     float c[2][2][4];
 #pragma unroll
@@ -1458,19 +1485,19 @@ __global__ void __launch_bounds__(MERGE_HEADS * 32, 2) merge_layer_kernel(const 
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
         const uint4 hi = *reinterpret_cast<const uint4*>(a_op + gl * MERGE_ROW + 32 * m + 8 * t4);
-        const uint4 lo = *reinterpret_cast<const uint4*>(a_op + (gl + MERGE_HEADS) * MERGE_ROW + 32 * m + 8 * t4);
+        const uint4 lo = *reinterpret_cast<const uint4*>(a_op + (gl + MERGE_WARPS) * MERGE_ROW + 32 * m + 8 * t4);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             mma16816(c[i][0], hi.x, lo.x, hi.y, lo.y, bf[i][m].x, bf[i][m].y);
             mma16816(c[i][1], hi.z, lo.z, hi.w, lo.w, bf[i][m].z, bf[i][m].w);
         }
     }
-    const int ho = MERGE_HEADS * (int)blockIdx.y + gl;
-    if (ho >= p.H) return;
+    const int ho = HEADS * (int)blockIdx.y + gl;
+    if (gl >= HEADS || ho >= p.H) return;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const float o0 = (c[i][0][0] + c[i][1][0]) + (c[i][0][2] + c[i][1][2]), o1 = (c[i][0][1] + c[i][1][1]) + (c[i][0][3] + c[i][1][3]);
-        const size_t at = (size_t)ho * HEAD_DIM + 8 * (warp + MERGE_HEADS * i) + 2 * t4;
+        const size_t at = (size_t)ho * HEAD_DIM + 8 * (warp + MERGE_WARPS * i) + 2 * t4;
         *reinterpret_cast<__half2*>(p.out + (size_t)g * p.q_dim + at) = __floats2half2_rn(o0, o1);
         if (p.out_f32) *reinterpret_cast<float2*>(p.out_f32 + (size_t)g * p.H * HEAD_DIM + at) = make_float2(o0, o1);
     }

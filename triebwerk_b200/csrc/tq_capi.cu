@@ -358,7 +358,7 @@ static int attention_impl(void* out, const CUtensorMap& tmK, const CUtensorMap& 
     MergeLayerParams m{};
     m.partials = p.partials; m.positions = positions; m.pos_value = pos_value; m.rotation_t = p.rotation_t; m.out = p.out; m.out_f32 = out_f32;
     m.G = G; m.H = num_heads; m.q_dim = q_dim; m.workers = ctas * ATTN_GROUPS;
-    return launch_kernel(merge_layer_kernel, dim3((unsigned)G, (unsigned)((num_heads + MERGE_HEADS - 1) / MERGE_HEADS)), dim3(MERGE_HEADS * 32), 0, s, use_pdl(), m);
+    return launch_merge_layer(m, s, use_pdl());
 }
 
 int tq_decode_attention(void* out, const uint8_t* ck_q, const uint8_t* cv_q, const void* k_norms, const void* v_norms,

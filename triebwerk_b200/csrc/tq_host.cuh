@@ -536,6 +536,16 @@ inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int lay
                                              : launch_cluster_decode_e<HOST, true>(bits, p, layers, split_layers, max_tokens, s, pdl);
 }
 
+// Merge of a layer's partials.  Few sequences are cut into many parts each, and a warp that adds up a head's alone, 16 in flight, was up to
+// half of the layer: from 14 workers per sequence on, and while two CTAs per SM hold all of them, a CTA per head (eight heads / one, 4-bit 16/8 heads
+// 3 x 30000 tokens 51.3 / 34.4 us a layer, 5 x 16384 40.7 / 31.7, 10 x 8192 35.0 / 31.3, 18 x 6000 38.9 / 38.1; 2-bit 32/8 9 x 8000 30.5 / 28.9, 12 x 8000, 384
+// heads, 32.8 / 34.5; nine parts: 8/8 36 x 2000 28.9 / 30.3, 4/4 37 x 3000 24.9 / 26.2).
+inline int launch_merge_layer(const MergeLayerParams& p, cudaStream_t s, bool pdl) {
+    if (p.workers >= 14 * p.G && (long long)p.G * p.H <= 2ll * device_props().sm_count)
+        return launch_kernel(merge_layer_kernel<1>, dim3((unsigned)p.G, (unsigned)p.H), dim3(MERGE_WARPS * 32), 0, s, pdl, p);
+    return launch_kernel(merge_layer_kernel<MERGE_WARPS>, dim3((unsigned)p.G, (unsigned)((p.H + MERGE_WARPS - 1) / MERGE_WARPS)), dim3(MERGE_WARPS * 32), 0, s, pdl, p);
+}
+
 __global__ void transpose_rotation_kernel(__half* dst, const __half* src) {
     // dst[d][k] = src[k][d]; one block per 32x32 tile would be overkill for 32 KB: a plain strided copy
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < HEAD_DIM * HEAD_DIM; i += gridDim.x * blockDim.x) {
