@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("bits,H,Hkv,G,slot,form", [
     # fp16 slots of one chunk: few tiles per warp stay in the cluster form
     (0, 8, 8, 12, 288, 1), (0, 8, 8, 12, 352, 1), (0, 16, 8, 12, 416, 0), (0, 16, 4, 32, 288, 1), (0, 16, 4, 32, 352, 0), (0, 16, 8, 48, 288, 0), (0, 16, 8, 37, 512, 1),
-    # packed layouts outside the streaming kernels', 4-bit: clusters that leave the next layer's half of the SMs, unless the chains get long
+    # 4-bit clusters that would fill the GPU leave the next layer's half of it, unless there is no streaming form and the chains get long; smaller ones only
+    # where slots are short
+    (4, 32, 4, 2, 4000, 8), (4, 32, 4, 3, 1024, 4), (4, 32, 4, 3, 1056, 8), (4, 32, 4, 3, 6016, 8), (4, 40, 5, 1, 4000, 16), (4, 56, 7, 2, 2048, 8),
     (4, 40, 8, 1, 4000, 8), (4, 40, 8, 2, 1504, 4), (4, 40, 8, 4, 1504, 4), (2, 40, 8, 1, 4000, 16), (4, 24, 2, 2, 4000, 8), (4, 40, 8, 2, 10240, 4), (4, 40, 8, 2, 10272, 8),
     (4, 40, 8, 1, 32000, 8), (4, 24, 2, 4, 16000, 8),
 ])

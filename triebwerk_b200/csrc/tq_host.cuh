@@ -462,14 +462,18 @@ inline int launch_cluster_decode_t(const ClusterDecodeParams& p, int S, int laye
 // hides the latency of the first one's loads: above 12 tiles 0.6 to 0.95 of the time (4 x 8192 tokens, 8 KV heads, 44 -> 28 us),
 // above 4 for fp16, whose rows are four times as long.  Not with more than 4 query heads per cluster in a packed mode: the warps'
 // partial results leave room for one CTA per SM there.
-// Where those are one layer's (`layer`) and 4-bit, the next layer's clusters of 8 and 16 find no room either beside this one's: as many
-// as leave it half of the SMs (32/4 heads, 2 x 4000 tokens 17.1 -> 10.0 us, 2 x 8000 21.1 -> 13.9, 4 x 4000 20.1 -> 15.4).  Layouts without a
-// streaming form (`streams` false) keep clusters of 8 where 4 would have chains of more than 20 tiles (40/8 heads, 16 -> 8 CTAs: one sequence
-// of 2048 tokens 13.8 -> 8.3 us, 12000 25.6 -> 20.4, 32000 52.1 -> 49.0; 8 -> 4: two of 520 11.5 -> 5.9, 6000 25.2 -> 22.1, 10000 37.5 -> 37.0, 12000
-// 43.1 -> 44.0, 16000 53.0 -> 56.5).
+// Where those are one layer's (`layer`), 4-bit, and as many as fit, the next layer's clusters of 8 and 16 find no room beside this one's: they are
+// halved (32/4 heads 2 x 4000 tokens 17.1 -> 10.1 us, 2 x 8000 20.9 -> 13.8, 4 x 4000 19.9 -> 14.5; 40/8 1 x 2048 13.8 -> 8.3, 1 x 12000 25.6 -> 20.4,
+// 1 x 32000 52.1 -> 49.0, 2 x 520 11.5 -> 5.9, 2 x 6000 25.2 -> 22.1).  Layouts without a streaming form (`streams` false) keep clusters of 8 where 4
+// would have chains of more than 20 tiles (40/8 2 x 10000 37.5 -> 37.0, 2 x 12000 43.1 -> 44.0, 2 x 16000 53.0 -> 56.5).  With a cluster's room and more to
+// spare only short slots are, where the shorter exchange pays (full / halved: 32/4 3 x 700 7.2 / 6.2, 3 x 1300 7.7 / 7.7, 3 x 4000 10.8 / 14.4, 3 x 8000 14.4 /
+// 23.0; 8 heads over 5, 6 and 7 KV heads, 80 to 120 CTAs: 700 tokens 1.05 to 1.18 of the time, 1300 0.87 to 0.99, 4000 0.67 to 0.73; 16 CTAs from 2100 on 0.98 to 1.1).
 inline int cluster_split(int bits, long long clusters, int heads, int max_tokens, bool layer, bool streams) {
     const long long sms = device_props().sm_count, blocks = (max_tokens + 15) / 16;
-    auto half = [&](int n) { return n >= 8 && layer && bits == 4 && heads > 4 && (streams || n > 8 || blocks <= 20 * 4 * CD_WARPS); };
+    auto half = [&](int n) {
+        if (n < 8 || !layer || bits != 4 || heads <= 4) return false;
+        return clusters * n > sms - 28 ? streams || n > 8 || blocks <= 20 * 4 * CD_WARPS : blocks <= n * CD_WARPS;
+    };
     auto fit = [&](int n) { return half(n) ? (sms - 20) / 2 : sms - (n >= 8 ? 20 : n >= 4 ? 12 : 0); };
     int S = 1;
     auto longer = [&](int n) { return n == 8 ? 2 * n * CD_WARPS <= blocks : n * CD_WARPS < blocks; };
