@@ -50,10 +50,13 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) layer_prep_kernel(const Layer
     __shared__ float inv_s[16], ss_s[16];
     __shared__ float bound_s[17];  // decision bounds between -inf and +inf
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gl = lane >> 2, t4 = lane & 3;
+    const long long n_vec = (long long)p.G * p.H;
+    const long long n_app = p.new_k ? p.G : 0, n_items = n_app + (n_vec + 15) / 16;
     const __half* const R = p.rotation + (size_t)(blockIdx.x % p.rot_copies) * (HEAD_DIM * HEAD_DIM);
     // B fragments of the coordinate blocks 2 warp and 2 warp + 1; step (m, e) of lane t4 covers k = 32m + 8*t4 + 4e .. +3, on both sides
     uint4 bf[2][4];
     auto fetch_rotation = [&]() {
+        if (blockIdx.x >= n_items) return;  // (a CTA that only helps with the transposition)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -82,8 +85,6 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) layer_prep_kernel(const Layer
     if (p.rotation_t)
         for (int i = (int)blockIdx.x * PREP_THREADS + tid; i < HEAD_DIM * HEAD_DIM; i += (int)gridDim.x * PREP_THREADS)
             p.rotation_t[i] = R[(i & (HEAD_DIM - 1)) * HEAD_DIM + (i >> 7)];
-    const long long n_vec = (long long)p.G * p.H;
-    const long long n_app = p.new_k ? p.G : 0, n_items = n_app + (n_vec + 15) / 16;
     const int nvec = 2 * p.Hkv;
     for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
         const bool app = item < n_app;
