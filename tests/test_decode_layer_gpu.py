@@ -20,7 +20,8 @@ pytestmark = pytest.mark.gpu
     (2, 4, 4, [31, 32, 33, 40000]),
     (4, 32, 4, [30000, 63, 64, 65]),
     (4, 16, 8, [33000] + [5] * 25),  # many parts of one sequence, one warp per head
-    (2, 32, 8, [9000] * 9), (4, 32, 8, [9000] * 10),  # the last batch that is merged by a CTA per head, and the first that is not
+    (2, 32, 8, [9000] * 8), (4, 32, 8, [9000] * 9),  # the last batch that is merged by a CTA per head, and the first that is not
+    (4, 16, 8, [3000] * 80),  # more CTAs than SMs in the merge
 ])
 def test_layer_form_equals_two_launch_form(bits, H, Hkv, lengths):
     D, G = 128, len(lengths)

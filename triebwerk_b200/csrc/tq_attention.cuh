@@ -1358,8 +1358,9 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const MergeParams p
 // start behind its own wait, when layer_prep_kernel, which transposes a caller's R, and all before that have finished; the loads pass
 // by L1, in which an SM may still have what it read in the layer before.
 // From the wait to the end 2.4 to 3.1 us (32 x 8192 tokens, 32 heads); by the last arriving worker inside the attention 5.6.
-// At least two CTAs per SM: at 141 registers, one, the merge was longer than the attention where there are many sequences (2-bit, 32/8
-// heads, 1000 x 100 tokens 73 us of a layer's 140.6; with two 113.1 a layer; 128 x 300 32.6 -> 29.2).
+// PER_SM: with 141 registers one CTA fills an SM, which is the fastest where that is enough (32 x 8192 tokens, 2-bit, 58.3 us a layer, with 128
+// registers 59.1) and a queue where there are many sequences: longer than the attention at 1000 x 100 tokens, 73 us of a layer's 140.6;
+// with room for two 113.1, 128 x 300 32.6 -> 29.2.
 struct MergeLayerParams {
     const float* partials;       // [workers + G][H][PART_STRIDE]
     const int* positions;        // device [G] or null: pos_value
@@ -1372,8 +1373,8 @@ struct MergeLayerParams {
 // HEADS = 1: a CTA per (sequence, head) instead, an eighth of its parts for every warp: for few sequences, which are cut into many parts
 // each (launch_merge_layer, tq_host.cuh).
 constexpr int MERGE_WARPS = 8;
-template <int HEADS>
-__global__ void __launch_bounds__(MERGE_WARPS * 32, 2) merge_layer_kernel(const MergeLayerParams p) {
+template <int HEADS, int PER_SM>
+__global__ void __launch_bounds__(MERGE_WARPS * 32, PER_SM) merge_layer_kernel(const MergeLayerParams p) {
     static_assert(HEADS == 1 || HEADS == MERGE_WARPS, "a warp per head, or all warps for one");
     constexpr bool SPLIT = HEADS == 1;
     __shared__ __align__(16) __half a_op[2 * MERGE_WARPS * MERGE_ROW];  // rows 0-7: high parts, 8-15: low parts (SPLIT: rows 0 and 8 alone are used)

@@ -542,13 +542,19 @@ inline int launch_cluster_decode(int bits, const ClusterDecodeParams& p, int lay
 }
 
 // Merge of a layer's partials.  Few sequences are cut into many parts each, and a warp that adds up a head's alone, 16 in flight, was up to
-// half of the layer: from 14 workers per sequence on, and while two CTAs per SM hold all of them, a CTA per head (eight heads / one, 4-bit 16/8 heads
-// 3 x 30000 tokens 51.3 / 34.4 us a layer, 5 x 16384 40.7 / 31.7, 10 x 8192 35.0 / 31.3, 18 x 6000 38.9 / 38.1; 2-bit 32/8 9 x 8000 30.5 / 28.9, 12 x 8000, 384
-// heads, 32.8 / 34.5; nine parts: 8/8 36 x 2000 28.9 / 30.3, 4/4 37 x 3000 24.9 / 26.2).
+// half of the layer: from 14 workers per sequence on, a CTA per head, while these are not many more than the SMs (eight heads per CTA / one, 4-bit
+// 16/8 heads 3 x 30000 tokens 51.3 / 34.4 us a layer, 5 x 16384 40.7 / 31.7, 10 x 8192 35.0 / 31.3, 2-bit 32/8 8 x 8000 29.0 / 26.0; 288 heads: 9 x 8000 28.3 /
+// 28.7, 4-bit 16/8 18 x 6000 37.2 / 38.0; nine parts: 8/8 36 x 2000 27.7 / 30.3).
 inline int launch_merge_layer(const MergeLayerParams& p, cudaStream_t s, bool pdl) {
-    if (p.workers >= 14 * p.G && (long long)p.G * p.H <= 2ll * device_props().sm_count)
-        return launch_kernel(merge_layer_kernel<1>, dim3((unsigned)p.G, (unsigned)p.H), dim3(MERGE_WARPS * 32), 0, s, pdl, p);
-    return launch_kernel(merge_layer_kernel<MERGE_WARPS>, dim3((unsigned)p.G, (unsigned)((p.H + MERGE_WARPS - 1) / MERGE_WARPS)), dim3(MERGE_WARPS * 32), 0, s, pdl, p);
+    const long long sms = device_props().sm_count, each = (long long)p.G * p.H;
+    const dim3 threads(MERGE_WARPS * 32);
+    if (p.workers >= 14 * p.G && 4 * each <= 7 * sms) {
+        const dim3 grid((unsigned)p.G, (unsigned)p.H);
+        return each <= sms ? launch_kernel(merge_layer_kernel<1, 1>, grid, threads, 0, s, pdl, p) : launch_kernel(merge_layer_kernel<1, 2>, grid, threads, 0, s, pdl, p);
+    }
+    const dim3 grid((unsigned)p.G, (unsigned)((p.H + MERGE_WARPS - 1) / MERGE_WARPS));
+    return (long long)grid.x * grid.y <= sms ? launch_kernel(merge_layer_kernel<MERGE_WARPS, 1>, grid, threads, 0, s, pdl, p)
+                                             : launch_kernel(merge_layer_kernel<MERGE_WARPS, 2>, grid, threads, 0, s, pdl, p);
 }
 
 __global__ void transpose_rotation_kernel(__half* dst, const __half* src) {
