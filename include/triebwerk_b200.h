@@ -284,8 +284,8 @@ int tq_engine_decode_layer(tq_engine* e, int layer, const void* q, const void* k
                            tq_stream_t s);
 
 /* The attention over the current positions alone, on whatever rotated queries the engine's workspace holds (those
- * of the last two-launch tq_engine_decode_layer, zeros before; packed modes only).  Used to time the attention
- * kernel by itself. */
+ * of the last tq_engine_decode_layer in the two-launch form, zeros before; the other forms leave them alone; packed modes
+ * only).  Used to time the attention kernel by itself. */
 int tq_engine_attend_layer(tq_engine* e, int layer, void* out, tq_stream_t s);
 
 /* tq_engine_attend_layer for every layer in turn: out [layers][G][q_dim] on the device. */

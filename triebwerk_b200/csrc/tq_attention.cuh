@@ -233,10 +233,10 @@ __device__ __forceinline__ float ldsp_h2f(uint32_t addr) {  // one fp16 from sha
 template <int NW, typename OutRow, typename OutRowF32>
 __device__ __forceinline__ void merge_sequence(const float* part0, int parts, int H, uint32_t merge_s, const __half* rotation_t,
                                                int head, int lane, int bar_group, int nthreads, OutRow out_row,
-                                               OutRowF32 out_row_f32, int hb_begin, int hb_end, bool rotated_out = false) {
+                                               OutRowF32 out_row_f32, bool rotated_out = false) {
     const int gl = lane >> 2, t4 = lane & 3;
     constexpr int RH = 2, FLIGHT = 16 / RH;  // heads per warp at a time, parts whose loads are in flight together
-    for (int hb = hb_begin; hb < hb_end; hb += 16) {
+    for (int hb = 0; hb < H; hb += 16) {
         // ---- phase A: heads hb .. hb+15, two heads per warp at a time with all their loads in flight
         //      together: combine the parts, normalise, split into fp16 high + low, store as the A operand
         //      [16][MERGE_ROW]
@@ -1291,7 +1291,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 return p.out_f32 + ((size_t)g * H + (size_t)vh) * HEAD_DIM;
             };
             merge_sequence<Hkv>(p.partials + (size_t)(first_w + g) * H * PART_STRIDE, parts, H, merge_s, p.rotation_t, head, lane,
-                                group, gthreads, out_row, out_row_f32, 0, H);
+                                group, gthreads, out_row, out_row_f32);
         }
         ++g;
     }
@@ -1349,7 +1349,7 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const MergeParams p
         return p.out_f32 + (((size_t)layer * p.G + (size_t)g) * H + (size_t)vh) * HEAD_DIM;
     };
     merge_sequence<8>(p.partials + (size_t)layer * (size_t)p.part_layer_stride + (size_t)(first_w + g) * H * PART_STRIDE,
-                      parts, H, smem_u32(merge_buf), p.rotation_t, warp, lane, 0, 256, out_row, out_row_f32, 0, H, p.rotated_out != 0);
+                      parts, H, smem_u32(merge_buf), p.rotation_t, warp, lane, 0, 256, out_row, out_row_f32, p.rotated_out != 0);
 }
 
 // The merge of one layer's partials (mode 1), the tail of that layer: bound by latency.  One CTA per (sequence, 8 heads), a warp per

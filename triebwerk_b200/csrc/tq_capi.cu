@@ -853,8 +853,8 @@ static int engine_upload_rotation(tq_engine* e, cudaStream_t s) {
             prep[((size_t)(k / 4) * HEAD_DIM + d) * 4 + (k % 4)] = __half2float(__half(raw));
         }
     TQ_CUDA(cudaMemcpyAsync(e->d_rotation_prep, prep.data(), prep.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-    // For the fused kernel: ROT_COPIES copies of R back to back.  Every worker of the kernel reads all of R at the same
-    // moment; with one copy those reads queue up on the same L2 lines.
+    // For layer_prep_kernel: ROT_COPIES copies of R back to back.  Every CTA reads all of R at the same moment; with one copy those
+    // reads queue up on the same L2 lines.
     if (!e->d_rotation_rep) TQ_CUDA(cudaMalloc(&e->d_rotation_rep, bytes * ROT_COPIES));
     for (int c = 0; c < ROT_COPIES; ++c)
         TQ_CUDA(cudaMemcpyAsync((char*)e->d_rotation_rep + bytes * c, e->h_rotation.data(), bytes, cudaMemcpyHostToDevice, s));
@@ -1535,7 +1535,8 @@ static bool engine_step_small(const tq_engine* e, StepInputs inputs) {
     double four = 26.0 + layers + cached;
     switch (inputs) {
         // (since the table is written four columns at a time the four launches are 3 % faster, 4-bit ones with 8 KV heads 5 to 10: 28 layers, 16/8
-        // heads, one launch / four: 24 x 300 tokens 191 / 145, 32 x 128 184 / 141, 16 x 2019 370 / 306, 8 x 4000 338 / 295)
+        // heads, one launch / four: 24 x 300 tokens 191 / 145, 32 x 128 184 / 141, 16 x 2019 370 / 306, 8 x 4000 338 / 295; the other inputs keep the line
+        // they were fitted with)
         case StepInputs::Plain:
             if (b4 && Hkv == 8) four = 24.0 + 0.8 * layers + 0.95 * cached;
             break;

@@ -33,7 +33,8 @@ enum : int {
 
 // ---- workspace layout ---------------------------------------------------------------------------------------
 // [0,256)                       header: int status; int total_tiles; ...
-// q_rot      float [G][H][128]  pre-rotated queries, already multiplied by log2(e)/sqrt(128)
+// q_rot      float [G][H][128]  pre-rotated queries, already multiplied by log2(e)/sqrt(128) (the launchers' layer form: as fp16, or in
+//                               AttnParams::q_rot32's order; an engine's layer form has its own elsewhere)
 // tile_start int   [G+4]        exclusive prefix of ceil(L_g / TILE_TOKENS)
 // tickets    int   [G]          arrivals per sequence (zeroed by the append/rotate kernel)
 // worker_g   int   [MAX_WORKERS] first sequence of each attention worker's slice

@@ -959,7 +959,7 @@ struct tq_engine {
     void* d_rotation = nullptr;
     void* d_rotation_t = nullptr;
     float* d_rotation_prep = nullptr;  // fp32, in the append kernel's shared-memory order
-    void* d_rotation_rep = nullptr;    // R row-major, several copies, for the fused kernel's query rotation
+    void* d_rotation_rep = nullptr;    // R row-major, several copies, for layer_prep_kernel
 
     // sleep that keeps the sequences: every sequence's written rows as a blob in host memory (see tq_engine_export_sequence)
     struct Kept {

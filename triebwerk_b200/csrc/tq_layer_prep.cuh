@@ -10,7 +10,7 @@
 // the previous layer's end and its first tile, a few workers had the append on top, and its warps the registers of all that
 // in their tile loop, without copy warps.
 // From the wait on (32 x 8192 tokens, 2-bit, 32/8 heads): rotated queries stored after 2.1 us, the appends after 2.8 to 4.3; inside the
-// attention kernel 3.7 and 7.  A piece of 16 vectors per CTA up to the number of SMs: more per CTA is a longer chain.
+// attention kernel 3.7 and 7.  A piece of 16 vectors per CTA while two CTAs per SM hold all pieces; beyond that CTAs loop.
 #pragma once
 
 #include "tq_attention.cuh"
@@ -18,7 +18,11 @@
 namespace tq {
 
 constexpr int PREP_THREADS = 256;
-constexpr float PREP_MARGIN = 1.7e-5f;  // see tq_prefill_tc.cuh
+// Twice the bound on either sum's rounding, 128 terms whose magnitudes sum to 1 at most (7.7e-6 each), and 1.5e-6 for the norm's two places: on
+// every term in the exact chain, on the sum here.  The two chains of products here round less often than that; largest difference measured to the exact
+// chain 8.4e-7 (1.9e9 coordinates: normal, heavy-tailed, all terms of one sign, 1e-5 to 65504).  Bytes against the two-launch form's: 2.15e9
+// coordinates of those kinds, none differ.
+constexpr float PREP_MARGIN = 1.7e-5f;
 constexpr int PREP_ROW = HEAD_DIM + 8;  // halves per row of R in shared memory
 
 struct LayerPrepParams {

@@ -46,7 +46,7 @@ class Engine:
         return int(lib().tq_engine_kv_bits(self._h))
 
     def set_fused(self, on: bool) -> bool:
-        """One launch per layer and step (default) or the two-launch form; returns the previous setting."""
+        """The layer form (default) or the two-launch form; returns the previous setting."""
         r = int(lib().tq_engine_set_fused(self._h, int(bool(on))))
         check(min(r, 0), "set_fused")
         return bool(r)
@@ -135,7 +135,7 @@ class Engine:
         return out
 
     def attend_layer(self, layer: int, out: torch.Tensor) -> torch.Tensor:
-        """Attention only, on the queries rotated by the last decode_layer call (packed modes)."""
+        """Attention only, on the queries rotated by the last decode_layer call in the two-launch form, zeros before (packed modes)."""
         check(lib().tq_engine_attend_layer(self._h, layer, out.data_ptr(), self._stream()), "attend_layer")
         return out
 
